@@ -21,6 +21,7 @@
 #include "decode_ll.cuh"
 #include "gdn.cuh"
 #include "gemm.cuh"
+#include "tc.cuh"
 #include "json_min.h"
 #include "prefill.cuh"
 #include "quant.cuh"
@@ -353,6 +354,8 @@ struct crane_b200_model {
     size_t last_decode_steps = 0;
     uint64_t launches = 0;
     uint64_t graph_launches[2][5] = {};
+    unsigned char* xqr_buf = nullptr;  // activation rows quantised for the tensor-core linears (qrows_at), xqr_rows of them
+    int xqr_rows = 0, xqr_mode_last = -1;
     unsigned char* xq_buf = nullptr;   // activations quantised for the quantised GEMVs (xquant_launch)
     int xq_mode_last = -1;
     // Split precision (default): every bf16 activation operand / KV page has a low-order plane (x = hi + lo) so the prefill
@@ -1007,11 +1010,23 @@ void crane_b200_model::linear_decode(int epi, bool norm, const bf16* w, const un
 }
 
 // Prefill through a quantised linear: candle's `QMatMul::forward` quantises every activation ROW to Q8_K / Q8_0 blocks and takes
-// ggml integer dots whatever the number of rows (crane-core/src/ops/linear.rs:23-48), so S > 1 runs the same xquant + qgemv
-// kernels as decode, four rows per pass over the quantised weights.  (A tensor-core formulation would have to reproduce the
-// per-block integer dots exactly; the decode kernels already do.)
+// ggml integer dots whatever the number of rows (crane-core/src/ops/linear.rs:23-48).  From QROWS_MIN rows on the integer dots run on the
+// tensor cores (qgemm.cu); fewer rows go through the decode kernels, up to four per pass over the quantised weights.
+// `reuse_xq`: the rows were quantised by the previous call (same input, same norm) -- still checked against the block rule it used.
 void crane_b200_model::qlinear_rows(int epi, const unsigned char* qw, int qt, int N, int K, const float* xin, int ldx, const float* norm_w,
                                     float* y, int ldy, int S, bool reuse_xq) {
+    if (S >= QROWS_MIN) {
+        const int mode = xq_mode_for(qt);
+        const QRows xr = qrows_at(xqr_buf, xqr_rows, K);
+        if (!reuse_xq || mode != xqr_mode_last) {
+            LAUNCH_OK(xquant_rows_launch(stream, S, xin, ldx, K, norm_w, eps, mode, xr, use_pdl));
+            xqr_mode_last = mode;
+            ++launches;
+        }
+        LAUNCH_OK(qgemm_launch(stream, qt, qw, xr, S, N, K, epi, y, ldy, use_pdl));
+        ++launches;
+        return;
+    }
     for (int s0 = 0; s0 < S;) {
         const int B = (S - s0 >= 4) ? 4 : (S - s0 >= 2) ? 2 : 1;
         linear_decode(epi, norm_w != nullptr, nullptr, qw, qt, N, K, xin + (size_t)s0 * ldx, ldx, norm_w, y + (size_t)s0 * ldy, ldy, nullptr, B,
@@ -1184,7 +1199,7 @@ void crane_b200_model::ensure_prefill_ws(int S) {
     if (S <= ws_S) return;
     CUDA_OK(cudaStreamSynchronize(stream));
     for (void* p : {(void*)x, (void*)qkv, (void*)xn, (void*)q_bf, (void*)attn_bf, (void*)act_bf, (void*)ids_dev, (void*)pos3_dev,
-                    (void*)rows_dev, (void*)embeds_in, (void*)rows_f32, (void*)g_proj, (void*)g_conv, (void*)g_qn, (void*)g_kn, (void*)g_gb, (void*)g_y, (void*)g_gl, (void*)g_chunk})
+                    (void*)rows_dev, (void*)embeds_in, (void*)rows_f32, (void*)xqr_buf, (void*)g_proj, (void*)g_conv, (void*)g_qn, (void*)g_kn, (void*)g_gb, (void*)g_y, (void*)g_gl, (void*)g_chunk})
         dfree(p);
     const int cap = (S + 127) / 128 * 128;
     x = dalloc<float>((size_t)cap * H);
@@ -1212,6 +1227,8 @@ void crane_b200_model::ensure_prefill_ws(int S) {
     rows_dev = dalloc<int>(cap);
     embeds_in = dalloc<float>((size_t)cap * H);
     rows_f32 = any_quant ? dalloc<float>((size_t)cap * std::max(I, q_dim())) : nullptr;
+    xqr_buf = any_quant ? dalloc<unsigned char>(qrows_bytes(cap, std::max(std::max(H, I), q_dim()))) : nullptr;
+    xqr_rows = cap;
     ws_S = cap;
 }
 
@@ -1453,6 +1470,7 @@ void crane_b200_model::ll_err_fetch() {
     if (ll_err) CUDA_OK(cudaMemcpyAsync(h_ll_err, ll_err, sizeof(unsigned int), cudaMemcpyDeviceToHost, stream));
 }
 void crane_b200_model::ll_err_verify() {
+    if (tc_take_wait_error(stream)) fail(CRANE_B200_CUDA_ERROR, "a tensor-core kernel's wait ran out (results discarded)");
     if (!ll_err || *h_ll_err == 0) return;
     std::vector<unsigned int> d(16 + num_sms * LL_WARPS);
     CUDA_OK(cudaMemcpy(d.data(), ll_err, d.size() * sizeof(unsigned int), cudaMemcpyDeviceToHost));
@@ -1525,13 +1543,13 @@ void crane_b200_model::prefill(const uint32_t* ids, const float* embeds, size_t 
             spans.mark(SP_ATTN_QKV);
             if (q_qkv) {   // GGUF keeps q / k / v separate and quantised (qwen3/modeling.rs:252-255): integer-dot rows, 4 at a time
                 const int qs = nh * q_stride(), kvd = nkv * D;
-                for (int s0 = 0; s0 < S;) {
-                    const int B = (S - s0 >= 4) ? 4 : (S - s0 >= 2) ? 2 : 1;
+                for (int s0 = 0; s0 < S;) {               // (a few rows: groups that share their codes)
+                    const int left = S - s0, B = left >= QROWS_MIN ? left : left >= 4 ? 4 : left >= 2 ? 2 : 1;
                     const float* xr = x + (size_t)s0 * H;
                     float* yr = qkv + (size_t)s0 * qkv_dim();
-                    linear_decode(GEMV_STORE, true, nullptr, l.q_wq, l.qt_q, qs, H, xr, H, l.ln1, yr, qkv_dim(), nullptr, B);
-                    linear_decode(GEMV_STORE, true, nullptr, l.q_wk, l.qt_k, kvd, H, xr, H, l.ln1, yr + qs, qkv_dim(), nullptr, B, true);
-                    linear_decode(GEMV_STORE, true, nullptr, l.q_wv, l.qt_v, kvd, H, xr, H, l.ln1, yr + qs + kvd, qkv_dim(), nullptr, B, true);
+                    qlinear_rows(GEMV_STORE, l.q_wq, l.qt_q, qs, H, xr, H, l.ln1, yr, qkv_dim(), B);
+                    qlinear_rows(GEMV_STORE, l.q_wk, l.qt_k, kvd, H, xr, H, l.ln1, yr + qs, qkv_dim(), B, true);
+                    qlinear_rows(GEMV_STORE, l.q_wv, l.qt_v, kvd, H, xr, H, l.ln1, yr + qs + kvd, qkv_dim(), B, true);
                     s0 += B;
                 }
             } else {
@@ -2610,7 +2628,7 @@ int crane_b200_op_qlinear(int device, const float* x, size_t m, size_t k, const 
     if (cudaSetDevice(device) != cudaSuccess) return CRANE_B200_CUDA_ERROR;
     int rc = CRANE_B200_OK;
     float *dx = nullptr, *dy = nullptr, *dn = nullptr;
-    unsigned char *dw = nullptr, *dxq = nullptr;
+    unsigned char *dw = nullptr, *dxq = nullptr, *dxr = nullptr;
     try {
         cudaDeviceProp prop;
         CUDA_OK(cudaGetDeviceProperties(&prop, device));
@@ -2623,7 +2641,12 @@ int crane_b200_op_qlinear(int device, const float* x, size_t m, size_t k, const 
         CUDA_OK(cudaMemcpy(dw, packed.data(), packed.size(), cudaMemcpyHostToDevice));
         CUDA_OK(cudaMemset(dy, 0, m * n * 4));
         if (norm_w) { CUDA_OK(cudaMalloc((void**)&dn, k * 4)); CUDA_OK(cudaMemcpy(dn, norm_w, k * 4, cudaMemcpyHostToDevice)); }
-        for (size_t s0 = 0; s0 < m;) {
+        if (m >= (size_t)QROWS_MIN) {
+            CUDA_OK(cudaMalloc((void**)&dxr, qrows_bytes((int)m, (int)k)));
+            const QRows xr = qrows_at(dxr, (int)m, (int)k);
+            LAUNCH_OK(xquant_rows_launch(nullptr, (int)m, dx, (int)k, (int)k, dn, eps, xq_mode_for(ggml_type), xr, false));
+            LAUNCH_OK(qgemm_launch(nullptr, ggml_type, dw, xr, (int)m, (int)n, (int)k, GEMV_STORE, dy, (int)n, false));
+        } else for (size_t s0 = 0; s0 < m;) {
             const int B = (m - s0 >= 4) ? 4 : (m - s0 >= 2) ? 2 : 1;
             LAUNCH_OK(xquant_launch(nullptr, B, dx + s0 * k, (int)k, (int)k, dn, eps, xq_mode_for(ggml_type), dxq, false));
             QGemvArgs qa = {};
@@ -2633,12 +2656,13 @@ int crane_b200_op_qlinear(int device, const float* x, size_t m, size_t k, const 
             s0 += B;
         }
         CUDA_OK(cudaDeviceSynchronize());
+        if (tc_take_wait_error(nullptr)) fail(CRANE_B200_CUDA_ERROR, "a tensor-core kernel's wait ran out (results discarded)");
         CUDA_OK(cudaMemcpy(y, dy, m * n * 4, cudaMemcpyDeviceToHost));
     } catch (const EngineError& e) {
         g_create_error = e.msg;
         rc = e.code;
     }
-    for (void* p : {(void*)dx, (void*)dy, (void*)dn, (void*)dw, (void*)dxq}) if (p) cudaFree(p);
+    for (void* p : {(void*)dx, (void*)dy, (void*)dn, (void*)dw, (void*)dxq, (void*)dxr}) if (p) cudaFree(p);
     return rc;
 }
 

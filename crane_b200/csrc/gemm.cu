@@ -1,80 +1,16 @@
 // tcgen05 + TMA GEMM for the prefill / ViT path.  See gemm.cuh for the design notes.
 #include "gemm.cuh"
+#include "tc.cuh"
 
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
-#include <mutex>
-#include <unordered_map>
 
 namespace cb {
 
 // CRANE_B200_GEMM_BN=64|128|256 pins the tile width (sweeps).  (Round 1 also had 2x2 TMA-multicast clusters; measured on B200 they
 // did not pay -- the L2 already merges concurrent requests for a line from a few CTAs -- and they are gone.)
 static const int g_gemm_bn = [] { const char* e = getenv("CRANE_B200_GEMM_BN"); return e ? atoi(e) : 0; }();
-
-// =====================================================================================
-// PTX wrappers (sm_100a)
-// =====================================================================================
-__device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-        ::"r"(smem_u32(smem_dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1) : "memory");
-}
-__device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
-    asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t ncols) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(ncols) : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish() {
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
-// Arrives on `bar` when every tcgen05.mma issued so far by this thread has completed.
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* v) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
-          "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
-          "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-        : "r"(taddr) : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-// K-major, SWIZZLE_128B shared-memory matrix descriptor (cute::UMMA::SmemDescriptor layout):
-// start address >> 4 in [0,14), LBO(=1, ignored for swizzled K-major) in [16,30),
-// SBO = 1024 B (8 rows x 128 B) >> 4 in [32,46), version = 1 in [46,48), layout SWIZZLE_128B = 2 in [61,64).
-__device__ __forceinline__ uint64_t make_smem_desc_sw128(uint32_t smem_addr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((smem_addr & 0x3FFFFu) >> 4);
-    d |= (uint64_t)1 << 16;
-    d |= (uint64_t)(1024 >> 4) << 32;
-    d |= (uint64_t)1 << 46;
-    d |= (uint64_t)2 << 61;
-    return d;
-}
-// Instruction descriptor (cute::UMMA::InstrDescriptor): D=f32, A=B=bf16, both K-major, M x N.
-__host__ __device__ constexpr uint32_t make_idesc_bf16(int M, int N) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
-}
 
 // =====================================================================================
 // Fused epilogue of one warp: a 32-row x 32-column accumulator block (lane = row, as tcgen05.ld delivers it).
@@ -204,20 +140,6 @@ constexpr int GEMM_BK = 64;
 constexpr int GEMM_STAGE_BUDGET = 192 * 1024;
 constexpr int GEMM_MAX_CTAS = 160;                 // workspace slots: two partial tiles per CTA
 
-struct GemmSched {
-    int tiles_m, tiles_n, KB;      // output tiles and k-steps per tile; tile t = n_tile * tiles_m + m_tile (the CTAs working at the
-                                   // same time share their weight rows: the L2 merges those requests)
-    int G, unit, base, rem;        // G CTAs; CTA c owns iterations [unit * (c * base + min(c, rem)), ...): base or base + 1 units of
-                                   // `unit` k-steps -- unit = KB deals out whole tiles (nothing is split), unit = 1 is stream-K
-    float* ws;                     // [2 * G][128 * BN] partial tiles
-    int* counters;                 // [tiles] arrivals per tile, zero between launches (the finisher resets its tile)
-};
-__host__ __device__ inline int sched_start(const GemmSched& s, int c) { return s.unit * (c * s.base + (c < s.rem ? c : s.rem)); }
-__host__ __device__ inline int sched_owner(const GemmSched& s, int it) {       // CTA whose range holds iteration `it`
-    const int u = it / s.unit, big = s.rem * (s.base + 1);
-    return u < big ? u / (s.base + 1) : s.rem + (u - big) / s.base;
-}
-
 template <int BN, bool SPLIT>
 struct GemmCfg {
     static constexpr int A_BYTES = GEMM_BM * GEMM_BK * 2;
@@ -234,7 +156,7 @@ struct GemmCfg {
 template <int BN, int MODE, bool SPLIT>
 __global__ void __launch_bounds__(256, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmAlo, const __grid_constant__ CUtensorMap tmB,
-               GemmEpi ep, int M, int N, int K, GemmSched sc) {
+               GemmEpi ep, int M, int N, int K, TcSched sc) {
     using Cfg = GemmCfg<BN, SPLIT>;
     constexpr int STAGES = Cfg::STAGES;
     extern __shared__ uint8_t smem_raw[];
@@ -484,98 +406,6 @@ gemm_simt_kernel(const bf16* __restrict__ A, const bf16* __restrict__ A_lo, int 
 // =====================================================================================
 // Host side
 // =====================================================================================
-typedef CUresult (*PFN_encodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                    const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                    CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static PFN_encodeTiled get_encode_fn() {
-    static PFN_encodeTiled fn = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qres) == cudaSuccess &&
-            qres == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<PFN_encodeTiled>(p);
-    });
-    return fn;
-}
-
-// 2-D bf16 row-major [rows, cols] with `ld` elements between rows; box = [box_rows, 64 cols], SWIZZLE_128B.
-// Encoding a map costs a few microseconds of host time -- as much as a small GEMM runs -- and a prefill pass issues the same
-// few hundred (buffer, shape) pairs on every request, so encoded maps are cached by their defining tuple.
-struct TmapKey {
-    const void* base; uint64_t rows, cols, ld; uint32_t box_rows;
-    bool operator==(const TmapKey& o) const { return base == o.base && rows == o.rows && cols == o.cols && ld == o.ld && box_rows == o.box_rows; }
-};
-struct TmapKeyHash {
-    size_t operator()(const TmapKey& k) const {
-        size_t h = std::hash<const void*>()(k.base);
-        for (uint64_t v : {k.rows, k.cols, k.ld, (uint64_t)k.box_rows}) h = h * 1000003u ^ std::hash<uint64_t>()(v);
-        return h;
-    }
-};
-static bool make_tmap_bf16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows) {
-    static std::unordered_map<TmapKey, CUtensorMap, TmapKeyHash> cache;
-    static std::mutex mu;
-    const TmapKey key{base, rows, cols, ld, box_rows};
-    {
-        std::lock_guard<std::mutex> g(mu);
-        auto it = cache.find(key);
-        if (it != cache.end()) { *map = it->second; return true; }
-    }
-    PFN_encodeTiled enc = get_encode_fn();
-    if (!enc) return false;
-    cuuint64_t dims[2] = {cols, rows};
-    cuuint64_t strides[1] = {ld * 2};
-    cuuint32_t box[2] = {(cuuint32_t)GEMM_BK, box_rows};
-    cuuint32_t estr[2] = {1, 1};
-    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return false;
-    std::lock_guard<std::mutex> g(mu);
-    if (cache.size() > 8192) cache.clear();
-    cache.emplace(key, *map);
-    return true;
-}
-
-// Per-stream stream-K scratch: partial tiles + arrival counters.  GEMMs on one stream are ordered (and a programmatic dependent only
-// touches the scratch after its dependency wait), so one set per stream is enough; gemm_release_stream frees it with the stream.
-struct GemmScratch { float* ws = nullptr; int* counters = nullptr; size_t ws_floats = 0; int n_counters = 0; };
-static std::mutex g_scratch_mu;
-static std::unordered_map<uint64_t, GemmScratch> g_scratch;
-static uint64_t scratch_key(cudaStream_t st) { int dev = 0; cudaGetDevice(&dev); return ((uint64_t)(uintptr_t)st << 6) ^ (uint64_t)dev; }
-
-static int scratch_get(cudaStream_t st, size_t ws_floats, int n_counters, GemmScratch* out) {
-    std::lock_guard<std::mutex> g(g_scratch_mu);
-    GemmScratch& sc = g_scratch[scratch_key(st)];
-    if (sc.ws_floats < ws_floats || sc.n_counters < n_counters) {
-        // (growing: the old buffers may still be in use by kernels in flight on this stream)
-        if (sc.ws || sc.counters) { cudaStreamSynchronize(st); cudaFree(sc.ws); cudaFree(sc.counters); }
-        sc.ws_floats = std::max(ws_floats, sc.ws_floats);
-        sc.n_counters = std::max(n_counters, std::max(sc.n_counters, 4096));
-        if (cudaMalloc(&sc.ws, sc.ws_floats * sizeof(float)) != cudaSuccess) { sc = GemmScratch{}; return (int)cudaErrorMemoryAllocation; }
-        if (cudaMalloc(&sc.counters, (size_t)sc.n_counters * sizeof(int)) != cudaSuccess) { cudaFree(sc.ws); sc = GemmScratch{}; return (int)cudaErrorMemoryAllocation; }
-        if (cudaMemsetAsync(sc.counters, 0, (size_t)sc.n_counters * sizeof(int), st) != cudaSuccess) return (int)cudaGetLastError();
-    }
-    *out = sc;
-    return 0;
-}
-void gemm_release_stream(cudaStream_t st) {
-    std::lock_guard<std::mutex> g(g_scratch_mu);
-    auto it = g_scratch.find(scratch_key(st));
-    if (it == g_scratch.end()) return;
-    cudaFree(it->second.ws); cudaFree(it->second.counters);
-    g_scratch.erase(it);
-}
-static int device_sms() {
-    static int sms[CB_MAX_DEV] = {};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= CB_MAX_DEV) return 148;
-    if (!sms[dev]) { int v = 0; cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev); sms[dev] = v > 0 ? v : 148; }
-    return sms[dev];
-}
 // CRANE_B200_GEMM_MINIT: fewest k-steps worth giving a CTA (below that the fixed cost of a CTA -- setup, first operand latency,
 // parking and re-reading partial tiles -- outweighs the parallelism)
 static const int g_gemm_minit = [] { const char* e = getenv("CRANE_B200_GEMM_MINIT"); const int v = e ? atoi(e) : 0; return v > 0 ? v : 8; }();
@@ -585,25 +415,25 @@ static int launch_tc(cudaStream_t stream, const bf16* A, const bf16* A_lo, int l
                      bool stream_k) {
     using Cfg = GemmCfg<BN, SPLIT>;
     CUtensorMap tmA, tmAlo, tmB;
-    if (!make_tmap_bf16(&tmA, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, GEMM_BM)) return -1001;
-    if (!make_tmap_bf16(&tmAlo, SPLIT ? A_lo : A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, GEMM_BM)) return -1001;
-    if (!make_tmap_bf16(&tmB, W, (uint64_t)N, (uint64_t)K, (uint64_t)K, BN)) return -1001;
+    if (!tc_tmap_bf16(&tmA, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, GEMM_BM)) return -1001;
+    if (!tc_tmap_bf16(&tmAlo, SPLIT ? A_lo : A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, GEMM_BM)) return -1001;
+    if (!tc_tmap_bf16(&tmB, W, (uint64_t)N, (uint64_t)K, (uint64_t)K, BN)) return -1001;
     static SmemOptIn seen;
     if (const int e = ensure_dyn_smem(gemm_tc_kernel<BN, MODE, SPLIT>, (size_t)Cfg::SMEM_BYTES, seen)) return e;
-    GemmSched sc = {};
+    TcSched sc = {};
     sc.tiles_m = (M + GEMM_BM - 1) / GEMM_BM;
     sc.tiles_n = (N + BN - 1) / BN;
     sc.KB = K / GEMM_BK;
     const long long tiles = (long long)sc.tiles_m * sc.tiles_n, iters = tiles * sc.KB;
     if (iters > 0x7fffffffLL) return -1000;
-    const int cap = std::min(device_sms(), GEMM_MAX_CTAS);
+    const int cap = std::min(tc_device_sms(), GEMM_MAX_CTAS);
     sc.unit = stream_k ? 1 : sc.KB;
     const long long units = iters / sc.unit;
     sc.G = (int)std::max<long long>(1, std::min<long long>(cap, stream_k ? iters / g_gemm_minit : tiles));
     sc.base = (int)(units / sc.G);
     sc.rem = (int)(units % sc.G);
-    GemmScratch scratch;
-    if (const int e = scratch_get(stream, (size_t)2 * GEMM_MAX_CTAS * GEMM_BM * 256, (int)std::max<long long>(tiles, 1), &scratch)) return e;
+    TcScratch scratch;
+    if (const int e = tc_scratch_get(stream, (size_t)2 * GEMM_MAX_CTAS * GEMM_BM * 256, (int)std::max<long long>(tiles, 1), &scratch)) return e;
     sc.ws = scratch.ws;
     sc.counters = scratch.counters;
     cudaLaunchConfig_t cfg = {};
@@ -661,7 +491,7 @@ static int launch_mode(cudaStream_t stream, const bf16* A, const bf16* A_lo, int
         gemm_simt_kernel<MODE><<<grid, 128, 0, stream>>>(A, A_lo, lda, W, epi, M, N, K);
         return (int)cudaGetLastError();
     }
-    const GemmPlan p = gemm_plan(M, N, K, A_lo != nullptr, std::min(device_sms(), GEMM_MAX_CTAS));
+    const GemmPlan p = gemm_plan(M, N, K, A_lo != nullptr, std::min(tc_device_sms(), GEMM_MAX_CTAS));
     if (A_lo != nullptr) {
         switch (p.bn) {
             case 256: return launch_tc<256, MODE, true>(stream, A, A_lo, lda, W, M, N, K, epi, p.stream_k);

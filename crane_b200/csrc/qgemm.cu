@@ -1,0 +1,500 @@
+// GGUF-quantised linears for many activation rows on the tensor cores: y[m, n] = epilogue(sum_k W[n, k] . xq[m, k]), with the integer dots of
+// candle's CPU `QMatMul::forward` (crane-core/src/ops/linear.rs:23-48) kept exact.
+//
+// Exactness.  Activations are int8 codes (xquant_kernel<true>), weights are small integers times block scales.  Both sides go through
+// tcgen05.mma kind::f16 as f16 INTEGERS, so every product is exact and the f32 accumulator holds the block's integer sum:
+//   Q4_K  A = sc_j * q (<= 63 * 15: 10 bits), one accumulator per 256-element super-block; a second one takes sum_j m_j * bsum_j, the offsets'
+//         share, as a K = 16 product of [m_j | 64 m_j] and [bsum mod 64 | bsum div 64]
+//   Q6_K  A = sc * (q - 32) needs 12 bits, so it is two f16 planes, sc * ql / 4 and 4 * sc * (qh - 2), accumulated into the same columns
+//   Q8_0  A = q, one accumulator per 32-element block (both sides have a scale per 32)
+// and the block scales are applied in f32 when the accumulator is read, once per block: acc += (d_w D - dmin_w D2) d_x.
+//
+// The weight rows are the MMA's M = 128 rows and the activation rows its N (NT = 16 .. 128), so a decode batch pays for the columns it has.
+//
+// What bounds it: at few rows the quantised bytes (decode), at many the MMAs and, nearly as much, the instructions that turn nibbles into
+// f16 (about 1.2 per weight) and scale accumulators.  Hence the split of a CTA into roles that overlap: one or four warps that copy raw blocks into a
+// ring, eight that unpack them into swizzled f16 tiles, one TMA producer for the activation codes, one MMA issuer, four or eight warps that
+// read accumulators.  Stream-K over (128 x NT tile, super-block): every SM has the same number of super-blocks whatever the shape; partial
+// tiles are added in contributor order by the last to arrive, so a result does not depend on who that was.
+#include "quant.cuh"
+#include "tc.cuh"
+
+#include <cuda_fp16.h>
+
+#include <algorithm>
+
+namespace cb {
+
+constexpr int QT_MAX_CTAS = 160;
+constexpr int DEQ_WARPS = 8;                                    // two on each of a super-block's four 64-wide steps, 64 weight rows each
+
+template <int QT, int NT>
+struct QCfg {
+    static constexpr int SB = QT == QT_Q4_K ? 144 : QT == QT_Q6_K ? 224 : 272;
+    static constexpr int PLANES = QT == QT_Q6_K ? 2 : 1;
+    static constexpr int A_BYTES = 128 * 128 * PLANES;          // one 64-wide step of the unpacked weights
+    static constexpr int B_BYTES = NT * 128;                    // ... of the activation codes
+    static constexpr int RAW_BYTES = 128 * SB;
+    static constexpr int NA = QT == QT_Q6_K ? (NT > 64 ? 3 : 4) : QT == QT_Q4_K && NT <= 32 ? 6 : 4;
+    static constexpr int NB = QT == QT_Q8_0 && NT > 64 ? 3 : 4;
+    static constexpr int NR = NT > 64 ? (QT == QT_Q4_K ? 3 : 2) : QT == QT_Q4_K ? 5 : QT == QT_Q8_0 || NT <= 16 ? 3 : 2;
+    static constexpr int GROUPS = QT == QT_Q8_0 ? 8 : 1;        // accumulators per super-block
+    static constexpr int ND = QT == QT_Q8_0 ? 4 : 2;            // accumulator ring
+    static constexpr bool MINS = QT == QT_Q4_K;
+    static constexpr int D_COLS = (MINS ? 2 : 1) * NT;
+    static constexpr int TMEM_COLS = ND * D_COLS <= 32 ? 32 : ND * D_COLS <= 64 ? 64 : ND * D_COLS <= 128 ? 128 : ND * D_COLS <= 256 ? 256 : 512;
+    static constexpr int NS = 4;                                // ring of scales (see the note at their writers)
+    static constexpr int SCW_BYTES = GROUPS * 128 * (MINS ? 8 : 4);
+    static constexpr int DX_BYTES = GROUPS * NT * 4;
+    static constexpr int A2_BYTES = MINS ? 128 * 32 : 0, B2_BYTES = MINS ? NT * 32 : 0;
+    static constexpr int EPI_WARPS = NT > 32 ? 8 : 4;
+    static constexpr int ACC = NT / (EPI_WARPS / 4);            // columns per epilogue thread
+    static constexpr int RAW_WARPS = NT > 32 ? 1 : 4;            // (few rows: bound by these copies; many: registers are dearer)
+    static constexpr int THREADS = (EPI_WARPS + DEQ_WARPS + 2 + RAW_WARPS) * 32;
+    // offsets from a 1024-byte boundary; the swizzled tiles first
+    static constexpr int OFF_A = 0, OFF_B = OFF_A + NA * A_BYTES, OFF_A2 = OFF_B + NB * B_BYTES, OFF_B2 = OFF_A2 + 2 * A2_BYTES,
+                         OFF_RAW = OFF_B2 + 2 * B2_BYTES, OFF_SCW = OFF_RAW + NR * RAW_BYTES, OFF_DX = OFF_SCW + NS * SCW_BYTES,
+                         OFF_BAR = OFF_DX + NS * DX_BYTES, SMEM = OFF_BAR + 512 + 1024;
+    static_assert(SMEM <= 227 * 1024, "tile rings do not fit");
+    static_assert(OFF_A2 % 1024 == 0 && OFF_RAW % 128 == 0 && OFF_DX % 16 == 0 && OFF_BAR % 8 == 0, "alignment");
+};
+
+struct QGemmArgs {
+    const unsigned char* w;        // [N, K / 256] blocks
+    int M, N, K, epi;              // activation rows, weight rows
+    float* y; int ldy;             // [M, ldy] (GEMV_SILU_MUL: [M, N / 2])
+    const float* dx;               // [GROUPS * K / 256][ldd] activation scales
+    int ldd;
+    TcSched sc;
+    int* err;
+};
+
+__device__ __forceinline__ uint32_t h2_fma(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t d;
+    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
+__device__ __forceinline__ uint32_t h2_add(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+__device__ __forceinline__ uint32_t h2_mul(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+__host__ __device__ constexpr uint32_t h2_const(uint32_t bits) { return bits | (bits << 16); }
+// a small unsigned integer as a pair of f16: 0x6400 is 1024, one unit per mantissa bit
+__device__ __forceinline__ uint32_t h2_int(uint32_t v) { return h2_add(v * 0x00010001u + 0x64006400u, h2_const(0xE400)); }
+// ... a signed byte (v + 128 is unsigned)
+__device__ __forceinline__ uint32_t h2_byte(uint32_t v) { return h2_add(((v ^ 0x80u) & 0xffu) * 0x00010001u + 0x64006400u, h2_const(0xE480)); }
+
+template <int QT, int NT>
+__global__ void __launch_bounds__(QCfg<QT, NT>::THREADS, 1)
+qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmS, QGemmArgs a) {
+    using C = QCfg<QT, NT>;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sm + C::OFF_BAR);
+    uint64_t *raw_full = bars, *raw_empty = raw_full + C::NR, *a_full = raw_empty + C::NR, *a_empty = a_full + C::NA, *b_full = a_empty + C::NA,
+             *b_empty = b_full + C::NB, *dx_full = b_empty + C::NB, *d_full = dx_full + C::NS, *d_empty = d_full + C::ND;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(d_empty + C::ND);
+    int* last_flag = reinterpret_cast<int*>(tmem_slot + 1);
+    int* gave_up = last_flag + 1;
+    static_assert((2 * C::NR + 2 * C::NA + 2 * C::NB + C::NS + 2 * C::ND) * 8 + 12 <= 512, "barrier area");
+    const TcWait wait{gave_up, a.err};
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int W_DEQ = C::EPI_WARPS, W_TMA = W_DEQ + DEQ_WARPS, W_MMA = W_TMA + 1, W_RAW = W_MMA + 1;
+    const int KB = a.sc.KB, it_begin = sched_start(a.sc, blockIdx.x), it_end = sched_start(a.sc, blockIdx.x + 1);
+
+    if (threadIdx.x == 0) {
+        *gave_up = 0;
+        for (int i = 0; i < C::NR; ++i) { mbar_init(&raw_full[i], C::RAW_WARPS * 32); mbar_init(&raw_empty[i], DEQ_WARPS); }
+        for (int i = 0; i < C::NA; ++i) { mbar_init(&a_full[i], DEQ_WARPS / 4); mbar_init(&a_empty[i], 1); }
+        for (int i = 0; i < C::NB; ++i) { mbar_init(&b_full[i], 1); mbar_init(&b_empty[i], 1); }
+        for (int i = 0; i < C::NS; ++i) mbar_init(&dx_full[i], 1);
+        for (int i = 0; i < C::ND; ++i) { mbar_init(&d_full[i], 1); mbar_init(&d_empty[i], C::EPI_WARPS); }
+        fence_barrier_init();
+    }
+    if (warp == W_MMA) { tmem_alloc(tmem_slot, C::TMEM_COLS); tmem_relinquish(); }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    pdl_launch_dependents();
+
+    // ------------------------------------------------------------------------------------------------ raw weights: 16-byte asynchronous copies
+    if (warp >= W_RAW) {           // (the weights do not depend on the kernel ahead: no dependency wait)
+        const int t = threadIdx.x - W_RAW * 32;
+        constexpr uint32_t CPB = C::SB / 16;
+        const size_t row_bytes = (size_t)KB * C::SB;
+        int rs = 0; uint32_t rph = 0;
+        for (int it = it_begin; it < it_end; ++it) {
+            wait(&raw_empty[rs], rph ^ 1);
+            const int n0 = (it / KB / a.sc.tiles_m) * 128;
+            const uint8_t* src = a.w + (size_t)n0 * row_bytes + (size_t)(it % KB) * C::SB;
+            const uint32_t dst = smem_u32(sm + C::OFF_RAW + rs * C::RAW_BYTES) + t * 16;
+#pragma unroll
+            for (uint32_t j = 0; j < CPB * 4 / C::RAW_WARPS; ++j) {
+                const uint32_t q = j * (C::RAW_WARPS * 32) + (uint32_t)t, r = q / CPB, c = q - r * CPB;
+                const bool in = n0 + (int)r < a.N;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + j * (C::RAW_WARPS * 512)), "l"(src + (in ? r * row_bytes + c * 16 : 0)), "r"(in ? 16 : 0) : "memory");
+            }
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&raw_full[rs])) : "memory");
+            if (++rs == C::NR) { rs = 0; rph ^= 1; }
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    // ------------------------------------------------------------------------------------------------ activation codes and their scales by TMA
+    } else if (warp == W_TMA) {
+        if (lane == 0) {
+            tma_prefetch_desc(&tmX);
+            pdl_wait();
+            int bs = 0, ds = 0; uint32_t bph = 0;
+            for (int it = it_begin; it < it_end; ++it) {
+                const int kb = it % KB, m0 = (it / KB % a.sc.tiles_m) * NT;
+                // Slot ds of the scales was last read for super-block it - 4.  Its successor's data may go in once step 0 of `it` has its place: that is
+                // the place of a step of it - 1, and the accumulator ring kept the MMAs of it - 1 behind the readers of it - 3.
+                for (int g = 0; g < 4; ++g) {
+                    wait(&b_empty[bs], bph ^ 1);
+                    if (g == 0) {
+                        mbar_arrive_expect_tx(&dx_full[ds], C::DX_BYTES);
+#pragma unroll
+                        for (int q = 0; q < C::GROUPS; ++q)
+                            bulk_load(sm + C::OFF_DX + ds * C::DX_BYTES + q * NT * 4, a.dx + (size_t)(kb * C::GROUPS + q) * a.ldd + m0, NT * 4, &dx_full[ds]);
+                        if (++ds == C::NS) ds = 0;
+                    }
+                    const bool mins = C::MINS && g == 3;
+                    mbar_arrive_expect_tx(&b_full[bs], C::B_BYTES + (mins ? C::B2_BYTES : 0));
+                    tma_load_2d(sm + C::OFF_B + bs * C::B_BYTES, &tmX, &b_full[bs], kb * 256 + g * 64, m0);
+                    if (mins) tma_load_2d(sm + C::OFF_B2 + (it & 1) * C::B2_BYTES, &tmS, &b_full[bs], kb * 16, m0);
+                    if (++bs == C::NB) { bs = 0; bph ^= 1; }
+                }
+            }
+            wait.drain();
+        }
+    // ------------------------------------------------------------------------------------------------ MMA issuer
+    } else if (warp == W_MMA) {
+        if (lane == 0) {
+            constexpr uint32_t idesc = make_idesc_f16(128, NT);
+            int as = 0, bs = 0, ds = 0; uint32_t aph = 0, bph = 0, dph = 0;
+            for (int it = it_begin; it < it_end; ++it) {
+                for (int g = 0; g < 4; ++g) {
+                    if (QT != QT_Q8_0 && g == 0) { wait(&d_empty[ds], dph ^ 1); tc_fence_after(); }
+                    wait(&a_full[as], aph);
+                    wait(&b_full[bs], bph);
+                    tc_fence_after();
+                    const uint32_t aa = smem_u32(sm + C::OFF_A + as * C::A_BYTES), ba = smem_u32(sm + C::OFF_B + bs * C::B_BYTES);
+                    const uint64_t ad = make_smem_desc_sw128(aa), ad2 = make_smem_desc_sw128(aa + 16384), bd = make_smem_desc_sw128(ba);
+                    if constexpr (QT == QT_Q8_0) {
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            wait(&d_empty[ds], dph ^ 1);
+                            tc_fence_after();
+                            const uint32_t d = tmem + (uint32_t)(ds * C::D_COLS);
+                            umma_bf16(d, ad + 4 * h, bd + 4 * h, idesc, 0u);
+                            umma_bf16(d, ad + 4 * h + 2, bd + 4 * h + 2, idesc, 1u);
+                            umma_commit(&d_full[ds]);
+                            if (++ds == C::ND) { ds = 0; dph ^= 1; }
+                        }
+                    } else {
+                        const uint32_t d = tmem + (uint32_t)(ds * C::D_COLS);
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            umma_bf16(d, ad + 2 * k, bd + 2 * k, idesc, (uint32_t)((g | k) != 0));
+                            if (C::PLANES == 2) umma_bf16(d, ad2 + 2 * k, bd + 2 * k, idesc, 1u);
+                        }
+                        if (C::MINS && g == 3)
+                            umma_bf16(d + NT, make_smem_desc_sw32(smem_u32(sm + C::OFF_A2 + (it & 1) * C::A2_BYTES)),
+                                      make_smem_desc_sw32(smem_u32(sm + C::OFF_B2 + (it & 1) * C::B2_BYTES)), idesc, 0u);
+                    }
+                    umma_commit(&a_empty[as]);
+                    umma_commit(&b_empty[bs]);
+                    if (++as == C::NA) { as = 0; aph ^= 1; }
+                    if (++bs == C::NB) { bs = 0; bph ^= 1; }
+                }
+                if constexpr (QT != QT_Q8_0) {
+                    umma_commit(&d_full[ds]);
+                    if (++ds == C::ND) { ds = 0; dph ^= 1; }
+                }
+            }
+        }
+    // ------------------------------------------------------------------------------------------------ weights: blocks -> f16 integers
+    } else if (warp >= W_DEQ) {
+        // A warp always works on the same one of a super-block's four 64-wide steps: one wait and one proxy fence per super-block and warp, and 128
+        // independent elements per lane.
+        const int dw = warp - W_DEQ, g = dw & 3, row0 = (dw >> 2) * 64 + lane;
+        int rs = 0; uint32_t rph = 0, seq = (uint32_t)g;
+        for (int it = it_begin; it < it_end; ++it, seq += 4) {
+            const uint32_t as = seq % C::NA, aph = (seq / C::NA) & 1;
+            wait(&raw_full[rs], rph);
+            // With four places or more a warp's next place cannot be two uses ahead of it (the MMAs take the steps in order); with three it can, so
+            // there the warp follows every step's place and a parity never stands for the wrong use.
+            if constexpr (C::NA < 4) {
+                for (uint32_t u = seq - (uint32_t)g; u < seq; ++u) wait(&a_empty[u % C::NA], ((u / C::NA) & 1) ^ 1);
+            }
+            wait(&a_empty[as], aph ^ 1);
+            uint8_t* A = sm + C::OFF_A + as * C::A_BYTES;
+            uint8_t* scw = sm + C::OFF_SCW + (it & (C::NS - 1)) * C::SCW_BYTES;
+#pragma unroll
+            for (int rr = 0; rr < 2; ++rr) {
+                const int row = row0 + 32 * rr;
+                const uint8_t* sb = sm + C::OFF_RAW + rs * C::RAW_BYTES + row * C::SB;
+                if constexpr (QT == QT_Q4_K) {
+                    const uint4 hdr = *reinterpret_cast<const uint4*>(sb);
+                    const uint4 w0 = *reinterpret_cast<const uint4*>(sb + 16 + 32 * g), w1 = *reinterpret_cast<const uint4*>(sb + 32 + 32 * g);
+                    // scales of sub-blocks 2g (low nibbles) and 2g + 1 (high): ggml get_scale_min_k4
+                    const int sh = 16 * (g & 1);
+                    const uint32_t y = hdr.y >> sh, z = hdr.w >> sh;
+                    const uint32_t sa = g < 2 ? y & 63 : (z & 0xF) | (((y >> 6) & 3) << 4), sb2 = g < 2 ? (y >> 8) & 63 : ((z >> 8) & 0xF) | (((y >> 14) & 3) << 4);
+                    const uint32_t s_lo = h2_int(sa), o_lo = h2_mul(s_lo, h2_const(0xE400)), t = h2_int(sb2), s_hi = h2_mul(t, h2_const(0x2C00)), o_hi = h2_mul(t, h2_const(0xD400));
+                    const uint32_t ww[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {          // (1024 + q) * s - 1024 * s and (1024 + 16 q) * s / 16 - 64 * s: one rounding, exact
+                        uint32_t lo[4], hi[4];
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) {
+                            const uint32_t v = ww[2 * c + i], v8 = v >> 8;
+                            lo[2 * i] = h2_fma((v & 0x000F000Fu) | 0x64006400u, s_lo, o_lo);
+                            lo[2 * i + 1] = h2_fma((v8 & 0x000F000Fu) | 0x64006400u, s_lo, o_lo);
+                            hi[2 * i] = h2_fma((v & 0x00F000F0u) | 0x64006400u, s_hi, o_hi);
+                            hi[2 * i + 1] = h2_fma((v8 & 0x00F000F0u) | 0x64006400u, s_hi, o_hi);
+                        }
+                        *reinterpret_cast<uint4*>(A + sw128_off(row, c)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                        *reinterpret_cast<uint4*>(A + sw128_off(row, 4 + c)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                    }
+                    if (g == 3) {                          // offsets m_0 .. m_7, 64 times them; d and dmin for the accumulators' readers
+                        uint32_t m[4], m64[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            uint32_t mj[2];
+#pragma unroll
+                            for (int e = 0; e < 2; ++e) {
+                                const int q = 2 * j + e, b = 8 * (q & 3);
+                                mj[e] = q < 4 ? (hdr.z >> b) & 63 : ((hdr.w >> (b + 4)) & 0xF) | (((hdr.z >> (b + 6)) & 3) << 4);
+                            }
+                            m[j] = h2_add((mj[0] | (mj[1] << 16)) + 0x64006400u, h2_const(0xE400));
+                            m64[j] = h2_mul(m[j], h2_const(0x5400));
+                        }
+                        uint8_t* a2 = sm + C::OFF_A2 + (it & 1) * C::A2_BYTES + row * 32;
+                        const int sw = ((row >> 2) & 1) << 4;
+                        *reinterpret_cast<uint4*>(a2 + sw) = make_uint4(m[0], m[1], m[2], m[3]);
+                        *reinterpret_cast<uint4*>(a2 + (sw ^ 16)) = make_uint4(m64[0], m64[1], m64[2], m64[3]);
+                        reinterpret_cast<float2*>(scw)[row] = make_float2(__half2float(__ushort_as_half((unsigned short)(hdr.x & 0xffffu))), __half2float(__ushort_as_half((unsigned short)(hdr.x >> 16))));
+                    }
+                } else if constexpr (QT == QT_Q6_K) {
+                    const int h = g >> 1, p = g & 1;       // p = 0: low nibbles, quarters q1 | q2 of half h; p = 1: high nibbles, q3 | q4
+                    if (g == 0) reinterpret_cast<float*>(scw)[row] = 4.f * __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short*>(sb + 208)));
+                    const uint32_t sw = *reinterpret_cast<const uint32_t*>(sb + 192 + 8 * h + 4 * p);       // scales: byte 2 * quarter + (element / 16)
+                    const uint32_t lmul = p ? h2_const(0x2400) : h2_const(0x3400), lofs = p ? h2_const(0xCC00) : h2_const(0xDC00);    // 1/64, 1/4; -16, -256
+                    const uint32_t lm = p ? 0x00F000F0u : 0x000F000Fu;
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {          // e: elements [16 e, 16 e + 16) of a quarter
+                        const uint4 qh = *reinterpret_cast<const uint4*>(sb + 128 + 32 * h + 16 * e);
+                        const uint32_t wh[4] = {qh.x >> (4 * p), qh.y >> (4 * p), qh.z >> (4 * p), qh.w >> (4 * p)};
+#pragma unroll
+                        for (int q = 0; q < 2; ++q) {      // q: which of the two quarters, elements [32 q, 32 q + 32) of the step
+                            const uint4 ql = *reinterpret_cast<const uint4*>(sb + 64 * h + 32 * q + 16 * e);
+                            const uint32_t f = h2_byte(sw >> (16 * q + 8 * e)), ls = h2_mul(f, lmul), lo_o = h2_mul(f, lofs);
+                            // high plane: two bits at 2 q (after the shift by 4 p): (1024 + 4^q v - 1024 - 2 * 4^q) * 4 f / 4^q
+                            const uint32_t hm = q ? 0x000C000Cu : 0x00030003u, hsub = q ? h2_const(0xE408) : h2_const(0xE402), hs = q ? f : h2_mul(f, h2_const(0x4400));
+                            const uint32_t wl[4] = {ql.x, ql.y, ql.z, ql.w};
+                            uint32_t lo[8], hi[8];
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                const uint32_t v = wl[i], v8 = v >> 8, u = wh[i], u8 = u >> 8;
+                                lo[2 * i] = h2_fma((v & lm) | 0x64006400u, ls, lo_o);
+                                lo[2 * i + 1] = h2_fma((v8 & lm) | 0x64006400u, ls, lo_o);
+                                hi[2 * i] = h2_mul(h2_add((u & hm) | 0x64006400u, hsub), hs);
+                                hi[2 * i + 1] = h2_mul(h2_add((u8 & hm) | 0x64006400u, hsub), hs);
+                            }
+#pragma unroll
+                            for (int c = 0; c < 2; ++c) {
+                                const uint32_t off = sw128_off(row, 4 * q + 2 * e + c);
+                                *reinterpret_cast<uint4*>(A + off) = make_uint4(lo[4 * c], lo[4 * c + 1], lo[4 * c + 2], lo[4 * c + 3]);
+                                *reinterpret_cast<uint4*>(A + 16384 + off) = make_uint4(hi[4 * c], hi[4 * c + 1], hi[4 * c + 2], hi[4 * c + 3]);
+                            }
+                        }
+                    }
+                } else {
+                    const uint32_t d2 = *reinterpret_cast<const uint32_t*>(sb + 256 + 4 * g);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const uint4 qv = *reinterpret_cast<const uint4*>(sb + 64 * g + 16 * c);
+                        const uint32_t ww[4] = {qv.x ^ 0x80808080u, qv.y ^ 0x80808080u, qv.z ^ 0x80808080u, qv.w ^ 0x80808080u};   // + 128: 0 .. 255
+                        uint32_t o[8];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            o[2 * i] = h2_add((ww[i] & 0x00FF00FFu) | 0x64006400u, h2_const(0xE480));
+                            o[2 * i + 1] = h2_add(((ww[i] >> 8) & 0x00FF00FFu) | 0x64006400u, h2_const(0xE480));
+                        }
+                        *reinterpret_cast<uint4*>(A + sw128_off(row, 2 * c)) = make_uint4(o[0], o[1], o[2], o[3]);
+                        *reinterpret_cast<uint4*>(A + sw128_off(row, 2 * c + 1)) = make_uint4(o[4], o[5], o[6], o[7]);
+                    }
+                    reinterpret_cast<float*>(scw)[(2 * g) * 128 + row] = __half2float(__ushort_as_half((unsigned short)(d2 & 0xffffu)));
+                    reinterpret_cast<float*>(scw)[(2 * g + 1) * 128 + row] = __half2float(__ushort_as_half((unsigned short)(d2 >> 16)));
+                }
+            }
+            fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) { mbar_arrive(&a_full[as]); mbar_arrive(&raw_empty[rs]); }
+            if constexpr (C::NA < 4) {
+                for (uint32_t u = seq + 1; (u & 3) != 0; ++u) wait(&a_empty[u % C::NA], ((u / C::NA) & 1) ^ 1);
+            }
+            if (++rs == C::NR) { rs = 0; rph ^= 1; }
+        }
+    // ------------------------------------------------------------------------------------------------ accumulators -> f32 sums -> epilogue
+    } else {
+        pdl_wait();
+        const int q = warp & 3, col0 = (warp >> 2) * C::ACC, row = q * 32 + lane;
+        constexpr size_t TILE_F = (size_t)128 * NT;
+        constexpr int CH = NT > 64 ? 8 : 16;                        // columns per read: what the registers leave room for
+        int ds = 0, xs = 0; uint32_t dph = 0, xph = 0;
+        for (int it = it_begin; it < it_end;) {
+            const int seg_end = min(it_end, (it / KB + 1) * KB), t = it / KB;
+            const int n0 = (t / a.sc.tiles_m) * 128, m0 = (t % a.sc.tiles_m) * NT;
+            const bool sole = it % KB == 0 && seg_end - it == KB, head = it == it_begin;
+            float acc[C::ACC];
+#pragma unroll
+            for (int j = 0; j < C::ACC; ++j) acc[j] = 0.f;
+            for (; it < seg_end; ++it) {
+                const uint8_t* scw = sm + C::OFF_SCW + (it & (C::NS - 1)) * C::SCW_BYTES;
+                wait(&dx_full[xs], xph);
+                const float* dx = reinterpret_cast<const float*>(sm + C::OFF_DX + xs * C::DX_BYTES) + col0;
+#pragma unroll 1
+                for (int g = 0; g < C::GROUPS; ++g) {
+                    wait(&d_full[ds], dph);
+                    tc_fence_after();
+                    float dw, dm = 0.f;
+                    if constexpr (C::MINS) { const float2 s = reinterpret_cast<const float2*>(scw)[row]; dw = s.x; dm = s.y; }
+                    else dw = reinterpret_cast<const float*>(scw)[g * 128 + row];
+                    const uint32_t d = tmem + (uint32_t)(ds * C::D_COLS + col0) + ((uint32_t)(q * 32) << 16);
+#pragma unroll
+                    for (int c = 0; c < C::ACC; c += CH) {
+                        uint32_t r[CH], s[CH];
+                        if constexpr (CH == 16) { tmem_ld16_async(d + c, r); if (C::MINS) tmem_ld16_async(d + NT + c, s); }
+                        else { tmem_ld8_async(d + c, r); if (C::MINS) tmem_ld8_async(d + NT + c, s); }
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < CH; j += 4) {
+                            const float4 x = *reinterpret_cast<const float4*>(dx + g * NT + c + j);
+                            const float xv[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                float v = dw * __uint_as_float(r[j + e]);
+                                if (C::MINS) v = fmaf(-dm, __uint_as_float(s[j + e]), v);
+                                acc[c + j + e] = fmaf(v, xv[e], acc[c + j + e]);
+                            }
+                        }
+                    }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&d_empty[ds]);
+                    if (++ds == C::ND) { ds = 0; dph ^= 1; }
+                }
+                if (++xs == C::NS) { xs = 0; xph ^= 1; }
+            }
+            bool finish = sole;
+            if (!sole) {      // park the partial tile (column by column: a warp's store is 128 contiguous bytes); the last contributor adds them in order
+                float* mine = a.sc.ws + (size_t)(2 * blockIdx.x + (head ? 0 : 1)) * TILE_F + (size_t)col0 * 128 + row;
+#pragma unroll
+                for (int j = 0; j < C::ACC; ++j) mine[j * 128] = acc[j];
+                __threadfence();
+                named_bar_sync(1, C::EPI_WARPS * 32);
+                const int c_first = sched_owner(a.sc, t * KB), c_last = sched_owner(a.sc, t * KB + KB - 1);
+                if (threadIdx.x == 0) *last_flag = atomicAdd(&a.sc.counters[t], 1) == c_last - c_first;
+                named_bar_sync(1, C::EPI_WARPS * 32);
+                finish = *last_flag != 0;
+                if (finish) {
+                    __threadfence();
+#pragma unroll
+                    for (int j = 0; j < C::ACC; ++j) acc[j] = 0.f;
+                    for (int cc = c_first; cc <= c_last; ++cc) {
+                        const float* p = a.sc.ws + (size_t)(2 * cc + (sched_start(a.sc, cc) < t * KB ? 1 : 0)) * TILE_F + (size_t)col0 * 128 + row;
+#pragma unroll
+                        for (int j = 0; j < C::ACC; ++j) {
+                            acc[j] += __ldcg(p + j * 128);
+                            if ((j & 15) == 15) asm volatile("" ::: "memory");     // 16 loads in flight, not all: registers
+                        }
+                    }
+                    if (threadIdx.x == 0) a.sc.counters[t] = 0;
+                }
+                named_bar_sync(1, C::EPI_WARPS * 32);              // last_flag is rewritten by the next segment
+            }
+            if (finish) {
+                const int n = n0 + row, cols = min(C::ACC, a.M - m0 - col0);
+                if (a.epi == GEMV_SILU_MUL) {                       // rows interleaved (gate_j, up_j): neighbouring lanes
+                    float* y = a.y + (size_t)(m0 + col0) * a.ldy + (n >> 1);
+                    const bool mine = !(lane & 1) && n < a.N;
+#pragma unroll
+                    for (int j = 0; j < C::ACC; ++j, y += a.ldy) {
+                        const float up = __shfl_xor_sync(0xffffffffu, acc[j], 1);
+                        if (mine && j < cols) *y = silu_f(acc[j]) * up;
+                    }
+                } else if (n < a.N) {
+                    float* y = a.y + (size_t)(m0 + col0) * a.ldy + n;
+                    if (a.epi == GEMV_RESID) {
+#pragma unroll
+                        for (int c = 0; c < C::ACC; c += 8, y += (size_t)8 * a.ldy) {
+                            float o[8];
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) o[j] = c + j < cols ? y[(size_t)j * a.ldy] : 0.f;
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) if (c + j < cols) y[(size_t)j * a.ldy] = o[j] + acc[c + j];
+                        }
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < C::ACC; ++j, y += a.ldy) if (j < cols) *y = acc[j];
+                    }
+                }
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == W_MMA) { tc_fence_after(); tmem_dealloc(tmem, C::TMEM_COLS); }
+}
+
+template <int QT, int NT>
+static int qgemm_launch_t(cudaStream_t st, const unsigned char* w, const QRows& x, int M, int N, int K, int epi, float* y, int ldy, bool pdl) {
+    using C = QCfg<QT, NT>;
+    CUtensorMap tmX, tmS;
+    if (!tc_tmap_16(&tmX, x.codes, (uint64_t)M, (uint64_t)K, (uint64_t)K, NT, 64, CU_TENSOR_MAP_SWIZZLE_128B)) return -1001;
+    if (!tc_tmap_16(&tmS, x.bsum, (uint64_t)M, (uint64_t)K / 16, (uint64_t)K / 16, NT, 16, CU_TENSOR_MAP_SWIZZLE_32B)) return -1001;
+    static SmemOptIn seen;
+    if (const int e = ensure_dyn_smem(qgemm_kernel<QT, NT>, (size_t)C::SMEM, seen)) return e;
+    QGemmArgs a = {};
+    a.w = w; a.M = M; a.N = N; a.K = K; a.epi = epi; a.y = y; a.ldy = ldy; a.dx = x.dx; a.ldd = x.ldd;
+    TcSched& sc = a.sc;
+    sc.tiles_m = (M + NT - 1) / NT; sc.tiles_n = (N + 127) / 128; sc.KB = K / 256;
+    const long long tiles = (long long)sc.tiles_m * sc.tiles_n, iters = tiles * sc.KB;
+    if (iters > 0x7fffffffLL) return -1000;
+    sc.unit = 1;
+    sc.G = (int)std::max<long long>(1, std::min<long long>(std::min(tc_device_sms(), QT_MAX_CTAS), iters / 2));     // two super-blocks pay for a CTA's setup
+    sc.base = (int)(iters / sc.G); sc.rem = (int)(iters % sc.G);
+    TcScratch s;
+    if (const int e = tc_scratch_get(st, TC_WS_FLOATS, (int)std::max<long long>(tiles, 1), &s)) return e;
+    sc.ws = s.ws; sc.counters = s.counters; a.err = s.err;
+    return launch_k(qgemm_kernel<QT, NT>, dim3(sc.G), dim3(C::THREADS), C::SMEM, st, pdl, tmX, tmS, a);
+}
+
+template <int QT>
+static int qgemm_launch_q(cudaStream_t st, const unsigned char* w, const QRows& x, int M, int N, int K, int epi, float* y, int ldy, bool pdl) {
+    if (M <= 16) return qgemm_launch_t<QT, 16>(st, w, x, M, N, K, epi, y, ldy, pdl);
+    if (M <= 32) return qgemm_launch_t<QT, 32>(st, w, x, M, N, K, epi, y, ldy, pdl);
+    if (M <= 64) return qgemm_launch_t<QT, 64>(st, w, x, M, N, K, epi, y, ldy, pdl);
+    return qgemm_launch_t<QT, 128>(st, w, x, M, N, K, epi, y, ldy, pdl);
+}
+
+int qgemm_launch(cudaStream_t st, int qt, const unsigned char* w, const QRows& x, int M, int N, int K, int epi, float* y, int ldy, bool pdl) {
+    if (M <= 0 || N <= 0 || K <= 0 || (K % 256) != 0 || (epi == GEMV_SILU_MUL && (N % 2) != 0) || M > x.ldd) return -1000;
+    switch (qt) {
+        case QT_Q4_K: return qgemm_launch_q<QT_Q4_K>(st, w, x, M, N, K, epi, y, ldy, pdl);
+        case QT_Q6_K: return qgemm_launch_q<QT_Q6_K>(st, w, x, M, N, K, epi, y, ldy, pdl);
+        case QT_Q8_0: return qgemm_launch_q<QT_Q8_0>(st, w, x, M, N, K, epi, y, ldy, pdl);
+        default: return -1000;
+    }
+}
+
+}  // namespace cb

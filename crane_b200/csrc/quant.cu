@@ -205,8 +205,10 @@ __device__ __forceinline__ void warp_reduce_scatter(float (&v)[N], int lane, int
 constexpr int XQ_THREADS = 1024;
 __host__ __device__ inline size_t xq_seq_bytes(int K) { return (size_t)K + (size_t)(K / 32) * 8 + (size_t)(K / 16) * 4; }
 
+// ROWS: the codes leave as f16 rows for the tensor cores (quant.cuh, QRows) instead of the GEMV's shared-memory image
+template <bool ROWS>
 __global__ void __launch_bounds__(XQ_THREADS, 1)
-xquant_kernel(const float* __restrict__ x, int ldx, int K, const float* __restrict__ norm_w, float eps, int B, int mode, unsigned char* __restrict__ out) {
+xquant_kernel(const float* __restrict__ x, int ldx, int K, const float* __restrict__ norm_w, float eps, int B, int mode, unsigned char* __restrict__ out, QRows rows) {
     __shared__ float red[32];
     const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     unsigned char* xq = out + (size_t)b * xq_seq_bytes(K);
@@ -271,6 +273,24 @@ xquant_kernel(const float* __restrict__ x, int ldx, int K, const float* __restri
             for (int j = 0; j < 8; ++j) q[j] = (int)roundf(v[j] * id);
             d = __half2float(__float2half_rn(df));
         }
+        if constexpr (ROWS) {
+            auto pair = [&](int i, int j) { return (uint32_t)__half_as_ushort(__int2half_rn(q[i])) | ((uint32_t)__half_as_ushort(__int2half_rn(q[j])) << 16); };
+            *reinterpret_cast<uint4*>(rows.codes + (size_t)b * K + e) = make_uint4(pair(0, 2), pair(1, 3), pair(4, 6), pair(5, 7));
+            int s32 = q[0] + q[1] + q[2] + q[3] + q[4] + q[5] + q[6] + q[7];
+            s32 += __shfl_xor_sync(0xffffffffu, s32, 1);
+            s32 += __shfl_xor_sync(0xffffffffu, s32, 2);
+            if (mode == XQ_Q8_K) {
+                if (lane == 0) rows.dx[(size_t)g * rows.ldd + b] = d;
+                if ((lane & 3) == 0) {
+                    unsigned short* bs = rows.bsum + (size_t)b * (K / 16) + g * 16 + (lane >> 2);
+                    bs[0] = __half_as_ushort(__int2half_rn(s32 & 63));
+                    bs[8] = __half_as_ushort(__int2half_rn(s32 >> 6));
+                }
+            } else if ((lane & 3) == 0) {
+                rows.dx[(size_t)(e >> 5) * rows.ldd + b] = d;
+            }
+            continue;
+        }
         const uint32_t p0 = (uint32_t)(q[0] & 0xff) | ((uint32_t)(q[1] & 0xff) << 8) | ((uint32_t)(q[2] & 0xff) << 16) | ((uint32_t)(q[3] & 0xff) << 24);
         const uint32_t p1 = (uint32_t)(q[4] & 0xff) | ((uint32_t)(q[5] & 0xff) << 8) | ((uint32_t)(q[6] & 0xff) << 16) | ((uint32_t)(q[7] & 0xff) << 24);
         *reinterpret_cast<uint2*>(xq + xq_swz(e)) = make_uint2(p0, p1);
@@ -280,7 +300,7 @@ xquant_kernel(const float* __restrict__ x, int ldx, int K, const float* __restri
         if ((lane & 1) == 0) isp[e >> 4] = s16;
         if ((lane & 3) == 0) dsp[e >> 5] = make_float2(d, d * (float)s32);
     }
-    if (tid == 0) reinterpret_cast<float*>(out + (size_t)B * xq_seq_bytes(K))[b] = 1.f;      // the rows are already normalised
+    if (!ROWS && tid == 0) reinterpret_cast<float*>(out + (size_t)B * xq_seq_bytes(K))[b] = 1.f;      // the rows are already normalised
 }
 
 size_t xquant_bytes(int B, int K) { return (size_t)B * xq_seq_bytes(K) + 16; }
@@ -296,7 +316,24 @@ int xquant_launch(cudaStream_t st, int B, const float* x, int ldx, int K, const 
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
-    return (int)cudaLaunchKernelEx(&cfg, xquant_kernel, x, ldx, K, norm_w, eps, B, mode, out);
+    return (int)cudaLaunchKernelEx(&cfg, xquant_kernel<false>, x, ldx, K, norm_w, eps, B, mode, out, QRows{});
+}
+
+// the scales' rows are read 128 columns at a time whatever the number of rows
+static size_t qrows_pad(int rows) { return (size_t)(rows + 127) / 128 * 128; }
+size_t qrows_bytes(int rows, int K) { return qrows_pad(rows) * ((size_t)K * 2 + (size_t)(K / 16) * 2 + (size_t)(K / 32) * 4); }
+QRows qrows_at(unsigned char* buf, int rows, int K) {
+    const size_t r = qrows_pad(rows);
+    QRows q;
+    q.codes = reinterpret_cast<unsigned short*>(buf);
+    q.bsum = reinterpret_cast<unsigned short*>(buf + r * K * 2);
+    q.dx = reinterpret_cast<float*>(buf + r * ((size_t)K * 2 + (size_t)(K / 16) * 2));
+    q.ldd = (int)r;
+    return q;
+}
+int xquant_rows_launch(cudaStream_t st, int M, const float* x, int ldx, int K, const float* norm_w, float eps, int mode, const QRows& out, bool pdl) {
+    if ((K % 256) != 0 || M < 1 || M > out.ldd || (ldx % 4) != 0) return -1000;
+    return launch_k(xquant_kernel<true>, dim3(M), dim3(XQ_THREADS), 0, st, pdl, x, ldx, K, norm_w, eps, M, mode, (unsigned char*)nullptr, out);
 }
 
 #ifndef QG_R_DEF                    // tools/qgemv_bench.cu sweeps these

@@ -37,6 +37,18 @@ size_t xquant_bytes(int B, int K);
 int xquant_launch(cudaStream_t st, int B, const float* x, int ldx, int K, const float* norm_w, float eps, int mode, unsigned char* out, bool pdl);
 
 int qgemv_launch(cudaStream_t st, int B, const QGemvArgs& a, int num_sms, bool pdl);
+
+// ---- many rows (qgemm.cu): the same codes as f16 integers, for the tensor cores ----
+// `rows` (a capacity) activation rows of up to K columns.  codes [rows, K] f16, elements of every group of four in the order 0, 2, 1, 3 (the order
+// in which the weights' bytes unpack in pairs); dx [blocks][ldd] the blocks' scales (256 or 32 elements); bsum [rows, K / 16] f16, per super-block
+// the eight 32-element sums mod 64 and their quotients by 64 (Q8_K codes only)
+constexpr int QROWS_MIN = 5;
+struct QRows { unsigned short* codes; float* dx; unsigned short* bsum; int ldd; };
+size_t qrows_bytes(int rows, int K);
+QRows qrows_at(unsigned char* buf, int rows, int K);
+int xquant_rows_launch(cudaStream_t st, int M, const float* x, int ldx, int K, const float* norm_w, float eps, int mode, const QRows& out, bool pdl);
+// y[m, n] = epi(sum_k W[n, k] x[m, k]); epi: GEMV_STORE, GEMV_RESID or GEMV_SILU_MUL (rows of W interleaved); x quantised for W's type
+int qgemm_launch(cudaStream_t st, int qt, const unsigned char* w, const QRows& x, int M, int N, int K, int epi, float* y, int ldy, bool pdl);
 // rows x K quantised -> bf16 row-major
 int q_dequant_bf16_launch(cudaStream_t st, int qt, const unsigned char* w, size_t rows, int K, bf16* out);
 // gather + dequantise rows of a quantised embedding table to f32: ids[rows] (prefill) or, with ids == nullptr, state[r].token

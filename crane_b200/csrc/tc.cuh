@@ -1,0 +1,170 @@
+// tcgen05 / TMA / mbarrier wrappers shared by the tensor-core kernels, and the host side they share: encoded tensor maps, per-stream
+// scratch, and the bounded waits' error flag.
+#pragma once
+
+#include <cuda.h>
+#include "common.cuh"
+
+namespace cb {
+
+// ---- bounded waits ---------------------------------------------------------------------
+// A wait that runs out (4 s at 1.9 GHz: a wait in these kernels is for a copy or an MMA of its own CTA, or for the end of the kernel ahead)
+// raises the CTA's `gave_up` word in shared memory and the stream's error word in pinned host memory; every later wait of the CTA
+// returns at once, the kernel runs to its end with its results discarded, and the host reports the error at its next read of a result.
+constexpr long long TC_WAIT_CYCLES = 8000000000LL;
+struct TcWait {
+    volatile int* gave_up;      // shared memory, zeroed before the first wait
+    int* err;                   // pinned host memory (TcScratch::err), written only when a wait runs out
+    __device__ __forceinline__ void operator()(uint64_t* bar, uint32_t parity) const {
+        const uint32_t addr = smem_u32(bar);
+        long long t0 = 0;
+        for (uint32_t n = 0;; ++n) {
+            uint32_t ok;
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t"
+                "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                "selp.u32 %0, 1, 0, p;\n\t}"
+                : "=r"(ok) : "r"(addr), "r"(parity) : "memory");
+            if (ok) return;
+            if ((n & 255u) == 255u) {
+                if (*gave_up) return;
+                if (!t0) t0 = clock64();
+                else if (clock64() - t0 > TC_WAIT_CYCLES) { *gave_up = 1; *reinterpret_cast<volatile int*>(err) = 1; return; }
+            }
+        }
+    }
+    // the issuing thread's last act when a wait ran out: copies still in flight must not land in a successor's shared memory
+    __device__ __forceinline__ void drain() const {
+        if (!*gave_up) return;
+        const long long t0 = clock64();
+        while (clock64() - t0 < 20000000LL) {}
+    }
+};
+// generic-proxy writes to shared memory (st.shared) become visible to tcgen05.mma / TMA
+__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+// ---- PTX wrappers (sm_100a) --------------------------------------------------------------
+__device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+        ::"r"(smem_u32(smem_dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1) : "memory");
+}
+__device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
+}
+__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t ncols) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(ncols) : "memory");
+}
+__device__ __forceinline__ void tmem_relinquish() {
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+// Arrives on `bar` when every tcgen05.mma issued so far by this thread has completed.
+__device__ __forceinline__ void umma_commit(uint64_t* bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* v) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
+          "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
+          "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+        : "r"(taddr) : "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+// 16 / 8 columns, without the wait: several loads in flight, then one tmem_ld_wait() before their registers are read
+__device__ __forceinline__ void tmem_ld16_async(uint32_t taddr, uint32_t* v) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_ld8_async(uint32_t taddr, uint32_t* v) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+        : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+// K-major, SWIZZLE_128B shared-memory matrix descriptor (cute::UMMA::SmemDescriptor layout):
+// start address >> 4 in [0,14), LBO(=1, ignored for swizzled K-major) in [16,30),
+// SBO = 1024 B (8 rows x 128 B) >> 4 in [32,46), version = 1 in [46,48), layout SWIZZLE_128B = 2 in [61,64).
+__device__ __forceinline__ uint64_t make_smem_desc_sw128(uint32_t smem_addr) {
+    uint64_t d = 0;
+    d |= (uint64_t)((smem_addr & 0x3FFFFu) >> 4);
+    d |= (uint64_t)1 << 16;
+    d |= (uint64_t)(1024 >> 4) << 32;
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)2 << 61;
+    return d;
+}
+// Instruction descriptor (cute::UMMA::InstrDescriptor): D=f32, A=B=bf16, both K-major, M x N.
+__host__ __device__ constexpr uint32_t make_idesc_bf16(int M, int N) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+}
+// The same for 32-byte rows (16 f16 / bf16): SWIZZLE_32B = 6, SBO = 8 rows x 32 B; the 16-byte half c of row r sits at half c ^ ((r >> 2) & 1).
+__device__ __forceinline__ uint64_t make_smem_desc_sw32(uint32_t smem_addr) {
+    uint64_t d = 0;
+    d |= (uint64_t)((smem_addr & 0x3FFFFu) >> 4);
+    d |= (uint64_t)1 << 16;
+    d |= (uint64_t)(256 >> 4) << 32;
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)6 << 61;
+    return d;
+}
+// A, B = f16 instead of bf16
+__host__ __device__ constexpr uint32_t make_idesc_f16(int M, int N) { return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24); }
+// 128-byte rows: byte offset of the 16-byte piece c of row r
+__device__ __forceinline__ uint32_t sw128_off(int r, int c) { return (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4)); }
+
+// ---- host side (tc.cu) ---------------------------------------------------------------------
+// 2-D row-major [rows, cols] of 16-bit elements with `ld` elements between rows; box = [box_rows, box_cols].  Encoded maps are cached by
+// their defining tuple: encoding costs a few microseconds of host time, as much as a small kernel runs.
+bool tc_tmap_16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows, uint32_t box_cols, CUtensorMapSwizzle swizzle);
+// ... of bf16 in boxes of 64 columns, SWIZZLE_128B
+inline bool tc_tmap_bf16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows) {
+    return tc_tmap_16(map, base, rows, cols, ld, box_rows, 64, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+// Per-stream scratch: partial tiles, arrival counters (zero between launches) and the bounded waits' error word.  Kernels on one stream
+// are ordered (and a programmatic dependent only touches the scratch after its dependency wait), so one set per stream is enough;
+// gemm_release_stream (gemm.cuh) frees it with the stream.
+struct TcScratch { float* ws = nullptr; int* counters = nullptr; int* err = nullptr; size_t ws_floats = 0; int n_counters = 0; };
+int tc_scratch_get(cudaStream_t st, size_t ws_floats, int n_counters, TcScratch* out);
+constexpr size_t TC_WS_FLOATS = (size_t)2 * 160 * 128 * 256;     // what every user asks for: two partial 128 x 256 tiles per CTA
+// true once if a wait of a kernel on `st` ran out since the last call (read after a synchronisation of the stream)
+bool tc_take_wait_error(cudaStream_t st);
+int tc_device_sms();
+
+// ---- work dealt out along K ------------------------------------------------------------------
+// G CTAs share tiles x KB iterations; CTA c owns the iterations [unit * (c * base + min(c, rem)), ...): base or base + 1 units of `unit`
+// iterations -- unit = KB deals out whole tiles (nothing is split), unit = 1 is stream-K
+struct TcSched {
+    int tiles_m, tiles_n, KB;      // output tiles and iterations per tile; tile t = n_tile * tiles_m + m_tile (the CTAs working at the
+                                   // same time share their weight rows: the L2 merges those requests)
+    int G, unit, base, rem;
+    float* ws;                     // [2 * G] partial tiles
+    int* counters;                 // [tiles] arrivals per tile, zero between launches (the finisher resets its tile)
+};
+__host__ __device__ inline int sched_start(const TcSched& s, int c) { return s.unit * (c * s.base + (c < s.rem ? c : s.rem)); }
+__host__ __device__ inline int sched_owner(const TcSched& s, int it) {       // CTA whose range holds iteration `it`
+    const int u = it / s.unit, big = s.rem * (s.base + 1);
+    return u < big ? u / (s.base + 1) : s.rem + (u - big) / s.base;
+}
+
+}  // namespace cb
