@@ -26,37 +26,41 @@
 namespace cb {
 
 constexpr int QT_MAX_CTAS = 160;
-constexpr int DEQ_WARPS = 8;                                    // two on each of a super-block's four 64-wide steps, 64 weight rows each
+constexpr int DEQ_WARPS = 8;
 
+// What paces the issuing warp (measured on B200, one CTA): an MMA of up to 64 columns 40 - 47 cycles, 128 columns 64; a wait that succeeds at once
+// 160 - 200; a commit 46.  So a stage carries eight MMAs, weights and activations arrive on ONE barrier and leave on one, and accumulators
+// change hands once per super-block (Q8_0: per stage).  (Stages of four MMAs with barriers of their own for either operand cost 2.1 us per
+// super-block whatever the copies and the unpacking did: 54 us for 4096 x 24576 at 8 rows.)
 template <int QT, int NT>
 struct QCfg {
     static constexpr int SB = QT == QT_Q4_K ? 144 : QT == QT_Q6_K ? 224 : 272;
     static constexpr int PLANES = QT == QT_Q6_K ? 2 : 1;
-    static constexpr int A_BYTES = 128 * 128 * PLANES;          // one 64-wide step of the unpacked weights
-    static constexpr int B_BYTES = NT * 128;                    // ... of the activation codes
+    static constexpr int CH64 = QT == QT_Q6_K || (QT == QT_Q8_0 && NT > 64) ? 1 : 2;      // 64-wide tiles of each operand per stage
+    static constexpr int SPS = 4 / CH64;                        // stages per super-block
+    static constexpr int A_BYTES = 128 * 128 * PLANES * CH64, B_BYTES = NT * 128 * CH64, STG_BYTES = A_BYTES + B_BYTES;
     static constexpr int RAW_BYTES = 128 * SB;
-    static constexpr int NA = QT == QT_Q6_K ? (NT > 64 ? 3 : 4) : QT == QT_Q4_K && NT <= 32 ? 6 : 4;
-    static constexpr int NB = QT == QT_Q8_0 && NT > 64 ? 3 : 4;
-    static constexpr int NR = NT > 64 ? (QT == QT_Q4_K ? 3 : 2) : QT == QT_Q4_K ? 5 : QT == QT_Q8_0 || NT <= 16 ? 3 : 2;
+    static constexpr int NSTG = QT == QT_Q4_K ? (NT > 64 ? 2 : 3) : QT == QT_Q6_K ? (NT > 64 ? 3 : 4) : (NT > 64 ? 3 : 2);
+    static constexpr int NR = QT == QT_Q4_K ? (NT > 64 ? 4 : NT > 32 ? 3 : NT > 16 ? 4 : 5) : QT == QT_Q6_K ? (NT > 16 ? 2 : 3) : (NT > 64 ? 2 : 3);
     static constexpr int GROUPS = QT == QT_Q8_0 ? 8 : 1;        // accumulators per super-block
-    static constexpr int ND = QT == QT_Q8_0 ? 4 : 2;            // accumulator ring
+    static constexpr int DG = QT == QT_Q8_0 ? 2 * CH64 : 1;     // ... that change hands together
     static constexpr bool MINS = QT == QT_Q4_K;
-    static constexpr int D_COLS = (MINS ? 2 : 1) * NT;
-    static constexpr int TMEM_COLS = ND * D_COLS <= 32 ? 32 : ND * D_COLS <= 64 ? 64 : ND * D_COLS <= 128 ? 128 : ND * D_COLS <= 256 ? 256 : 512;
+    static constexpr int D_COLS = (MINS ? 2 : DG) * NT;         // two such sets
+    static constexpr int TMEM_COLS = 2 * D_COLS <= 32 ? 32 : 2 * D_COLS <= 64 ? 64 : 2 * D_COLS <= 128 ? 128 : 2 * D_COLS <= 256 ? 256 : 512;
     static constexpr int NS = 4;                                // ring of scales (see the note at their writers)
     static constexpr int SCW_BYTES = GROUPS * 128 * (MINS ? 8 : 4);
     static constexpr int DX_BYTES = GROUPS * NT * 4;
     static constexpr int A2_BYTES = MINS ? 128 * 32 : 0, B2_BYTES = MINS ? NT * 32 : 0;
     static constexpr int EPI_WARPS = NT > 32 ? 8 : 4;
     static constexpr int ACC = NT / (EPI_WARPS / 4);            // columns per epilogue thread
-    static constexpr int RAW_WARPS = NT > 32 ? 1 : 4;            // (few rows: bound by these copies; many: registers are dearer)
+    static constexpr int RAW_WARPS = NT > 32 ? 1 : 4;           // (few rows: bound by these copies; many: registers are dearer)
     static constexpr int THREADS = (EPI_WARPS + DEQ_WARPS + 2 + RAW_WARPS) * 32;
     // offsets from a 1024-byte boundary; the swizzled tiles first
-    static constexpr int OFF_A = 0, OFF_B = OFF_A + NA * A_BYTES, OFF_A2 = OFF_B + NB * B_BYTES, OFF_B2 = OFF_A2 + 2 * A2_BYTES,
+    static constexpr int OFF_A2 = NSTG * STG_BYTES, OFF_B2 = OFF_A2 + 2 * A2_BYTES,
                          OFF_RAW = OFF_B2 + 2 * B2_BYTES, OFF_SCW = OFF_RAW + NR * RAW_BYTES, OFF_DX = OFF_SCW + NS * SCW_BYTES,
                          OFF_BAR = OFF_DX + NS * DX_BYTES, SMEM = OFF_BAR + 512 + 1024;
     static_assert(SMEM <= 227 * 1024, "tile rings do not fit");
-    static_assert(OFF_A2 % 1024 == 0 && OFF_RAW % 128 == 0 && OFF_DX % 16 == 0 && OFF_BAR % 8 == 0, "alignment");
+    static_assert(STG_BYTES % 1024 == 0 && OFF_A2 % 1024 == 0 && OFF_RAW % 128 == 0 && OFF_DX % 16 == 0 && OFF_BAR % 8 == 0, "alignment");
 };
 
 struct QGemmArgs {
@@ -97,12 +101,12 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint64_t* bars = reinterpret_cast<uint64_t*>(sm + C::OFF_BAR);
-    uint64_t *raw_full = bars, *raw_empty = raw_full + C::NR, *a_full = raw_empty + C::NR, *a_empty = a_full + C::NA, *b_full = a_empty + C::NA,
-             *b_empty = b_full + C::NB, *dx_full = b_empty + C::NB, *d_full = dx_full + C::NS, *d_empty = d_full + C::ND;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(d_empty + C::ND);
+    uint64_t *raw_full = bars, *raw_empty = raw_full + C::NR, *full = raw_empty + C::NR, *empty = full + C::NSTG, *dx_full = empty + C::NSTG,
+             *d_full = dx_full + C::NS, *d_empty = d_full + 2;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(d_empty + 2);
     int* last_flag = reinterpret_cast<int*>(tmem_slot + 1);
     int* gave_up = last_flag + 1;
-    static_assert((2 * C::NR + 2 * C::NA + 2 * C::NB + C::NS + 2 * C::ND) * 8 + 12 <= 512, "barrier area");
+    static_assert((2 * C::NR + 2 * C::NSTG + C::NS + 4) * 8 + 12 <= 512, "barrier area");
     const TcWait wait{gave_up, a.err};
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -112,10 +116,9 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
     if (threadIdx.x == 0) {
         *gave_up = 0;
         for (int i = 0; i < C::NR; ++i) { mbar_init(&raw_full[i], C::RAW_WARPS * 32); mbar_init(&raw_empty[i], DEQ_WARPS); }
-        for (int i = 0; i < C::NA; ++i) { mbar_init(&a_full[i], DEQ_WARPS / 4); mbar_init(&a_empty[i], 1); }
-        for (int i = 0; i < C::NB; ++i) { mbar_init(&b_full[i], 1); mbar_init(&b_empty[i], 1); }
+        for (int i = 0; i < C::NSTG; ++i) { mbar_init(&full[i], DEQ_WARPS / C::SPS + 1); mbar_init(&empty[i], 1); }
         for (int i = 0; i < C::NS; ++i) mbar_init(&dx_full[i], 1);
-        for (int i = 0; i < C::ND; ++i) { mbar_init(&d_full[i], 1); mbar_init(&d_empty[i], C::EPI_WARPS); }
+        for (int i = 0; i < 2; ++i) { mbar_init(&d_full[i], 1); mbar_init(&d_empty[i], C::EPI_WARPS); }
         fence_barrier_init();
     }
     if (warp == W_MMA) { tmem_alloc(tmem_slot, C::TMEM_COLS); tmem_relinquish(); }
@@ -151,13 +154,13 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
         if (lane == 0) {
             tma_prefetch_desc(&tmX);
             pdl_wait();
-            int bs = 0, ds = 0; uint32_t bph = 0;
+            int st = 0, ds = 0; uint32_t ph = 0;
             for (int it = it_begin; it < it_end; ++it) {
                 const int kb = it % KB, m0 = (it / KB % a.sc.tiles_m) * NT;
-                // Slot ds of the scales was last read for super-block it - 4.  Its successor's data may go in once step 0 of `it` has its place: that is
-                // the place of a step of it - 1, and the accumulator ring kept the MMAs of it - 1 behind the readers of it - 3.
-                for (int g = 0; g < 4; ++g) {
-                    wait(&b_empty[bs], bph ^ 1);
+                // Slot ds of the scales was last read for super-block it - 4.  Its successor's data may go in once the first stage of `it` is free: a stage
+                // at most two super-blocks back has been multiplied then, and the accumulators kept that one behind the readers of it - 4.
+                for (int g = 0; g < C::SPS; ++g) {
+                    wait(&empty[st], ph ^ 1);
                     if (g == 0) {
                         mbar_arrive_expect_tx(&dx_full[ds], C::DX_BYTES);
 #pragma unroll
@@ -165,81 +168,69 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                             bulk_load(sm + C::OFF_DX + ds * C::DX_BYTES + q * NT * 4, a.dx + (size_t)(kb * C::GROUPS + q) * a.ldd + m0, NT * 4, &dx_full[ds]);
                         if (++ds == C::NS) ds = 0;
                     }
-                    const bool mins = C::MINS && g == 3;
-                    mbar_arrive_expect_tx(&b_full[bs], C::B_BYTES + (mins ? C::B2_BYTES : 0));
-                    tma_load_2d(sm + C::OFF_B + bs * C::B_BYTES, &tmX, &b_full[bs], kb * 256 + g * 64, m0);
-                    if (mins) tma_load_2d(sm + C::OFF_B2 + (it & 1) * C::B2_BYTES, &tmS, &b_full[bs], kb * 16, m0);
-                    if (++bs == C::NB) { bs = 0; bph ^= 1; }
+                    const bool mins = C::MINS && g == C::SPS - 1;
+                    mbar_arrive_expect_tx(&full[st], C::B_BYTES + (mins ? C::B2_BYTES : 0));
+#pragma unroll
+                    for (int c = 0; c < C::CH64; ++c)
+                        tma_load_2d(sm + st * C::STG_BYTES + C::A_BYTES + c * NT * 128, &tmX, &full[st], kb * 256 + (g * C::CH64 + c) * 64, m0);
+                    if (mins) tma_load_2d(sm + C::OFF_B2 + (it & 1) * C::B2_BYTES, &tmS, &full[st], kb * 16, m0);
+                    if (++st == C::NSTG) { st = 0; ph ^= 1; }
                 }
             }
             wait.drain();
         }
-    // ------------------------------------------------------------------------------------------------ MMA issuer
+    // ------------------------------------------------------------------------------------------------ MMA issuer (the whole warp runs the loop)
     } else if (warp == W_MMA) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = make_idesc_f16(128, NT);
-            int as = 0, bs = 0, ds = 0; uint32_t aph = 0, bph = 0, dph = 0;
-            for (int it = it_begin; it < it_end; ++it) {
-                for (int g = 0; g < 4; ++g) {
-                    if (QT != QT_Q8_0 && g == 0) { wait(&d_empty[ds], dph ^ 1); tc_fence_after(); }
-                    wait(&a_full[as], aph);
-                    wait(&b_full[bs], bph);
-                    tc_fence_after();
-                    const uint32_t aa = smem_u32(sm + C::OFF_A + as * C::A_BYTES), ba = smem_u32(sm + C::OFF_B + bs * C::B_BYTES);
-                    const uint64_t ad = make_smem_desc_sw128(aa), ad2 = make_smem_desc_sw128(aa + 16384), bd = make_smem_desc_sw128(ba);
-                    if constexpr (QT == QT_Q8_0) {
+        constexpr uint32_t idesc = make_idesc_f16(128, NT);
+        int st = 0, ds = 0; uint32_t ph = 0, dph = 0;
+        for (int it = it_begin; it < it_end; ++it) {
+            for (int g = 0; g < C::SPS; ++g) {
+                if (QT == QT_Q8_0 || g == 0) { wait(&d_empty[ds], dph ^ 1); tc_fence_after(); }
+                wait(&full[st], ph);
+                tc_fence_after();
+                const uint32_t aa = smem_u32(sm + st * C::STG_BYTES), d = tmem + (uint32_t)(ds * C::D_COLS);
+                const uint64_t ad = make_smem_desc_sw128(aa), bd = make_smem_desc_sw128(aa + C::A_BYTES);
+                if (elect_one()) {
 #pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            wait(&d_empty[ds], dph ^ 1);
-                            tc_fence_after();
-                            const uint32_t d = tmem + (uint32_t)(ds * C::D_COLS);
-                            umma_bf16(d, ad + 4 * h, bd + 4 * h, idesc, 0u);
-                            umma_bf16(d, ad + 4 * h + 2, bd + 4 * h + 2, idesc, 1u);
-                            umma_commit(&d_full[ds]);
-                            if (++ds == C::ND) { ds = 0; dph ^= 1; }
-                        }
-                    } else {
-                        const uint32_t d = tmem + (uint32_t)(ds * C::D_COLS);
+                    for (int c = 0; c < C::CH64; ++c)
 #pragma unroll
                         for (int k = 0; k < 4; ++k) {
-                            umma_bf16(d, ad + 2 * k, bd + 2 * k, idesc, (uint32_t)((g | k) != 0));
-                            if (C::PLANES == 2) umma_bf16(d, ad2 + 2 * k, bd + 2 * k, idesc, 1u);
+                            const uint64_t aw = ad + (uint64_t)(c * C::PLANES * 1024 + 2 * k), bw = bd + (uint64_t)(c * NT * 8 + 2 * k);
+                            if constexpr (QT == QT_Q8_0) umma_bf16(d + (2 * c + (k >> 1)) * NT, aw, bw, idesc, (uint32_t)(k & 1));
+                            else umma_bf16(d, aw, bw, idesc, (uint32_t)((g | c | k) != 0));
+                            if (C::PLANES == 2) umma_bf16(d, aw + 1024, bw, idesc, 1u);
                         }
-                        if (C::MINS && g == 3)
-                            umma_bf16(d + NT, make_smem_desc_sw32(smem_u32(sm + C::OFF_A2 + (it & 1) * C::A2_BYTES)),
-                                      make_smem_desc_sw32(smem_u32(sm + C::OFF_B2 + (it & 1) * C::B2_BYTES)), idesc, 0u);
-                    }
-                    umma_commit(&a_empty[as]);
-                    umma_commit(&b_empty[bs]);
-                    if (++as == C::NA) { as = 0; aph ^= 1; }
-                    if (++bs == C::NB) { bs = 0; bph ^= 1; }
+                    if (C::MINS && g == C::SPS - 1)
+                        umma_bf16(d + NT, make_smem_desc_sw32(smem_u32(sm + C::OFF_A2 + (it & 1) * C::A2_BYTES)),
+                                  make_smem_desc_sw32(smem_u32(sm + C::OFF_B2 + (it & 1) * C::B2_BYTES)), idesc, 0u);
+                    umma_commit(&empty[st]);
+                    if (QT == QT_Q8_0 || g == C::SPS - 1) umma_commit(&d_full[ds]);
                 }
-                if constexpr (QT != QT_Q8_0) {
-                    umma_commit(&d_full[ds]);
-                    if (++ds == C::ND) { ds = 0; dph ^= 1; }
-                }
+                __syncwarp();
+                if (++st == C::NSTG) { st = 0; ph ^= 1; }
+                if (QT == QT_Q8_0 || g == C::SPS - 1) { if (++ds == 2) { ds = 0; dph ^= 1; } }
             }
         }
     // ------------------------------------------------------------------------------------------------ weights: blocks -> f16 integers
     } else if (warp >= W_DEQ) {
-        // A warp always works on the same one of a super-block's four 64-wide steps: one wait and one proxy fence per super-block and warp, and 128
-        // independent elements per lane.
-        const int dw = warp - W_DEQ, g = dw & 3, row0 = (dw >> 2) * 64 + lane;
-        int rs = 0; uint32_t rph = 0, seq = (uint32_t)g;
-        for (int it = it_begin; it < it_end; ++it, seq += 4) {
-            const uint32_t as = seq % C::NA, aph = (seq / C::NA) & 1;
+        // A warp always works on the same one of a super-block's stages, 64 rows of a 64-wide tile or 32 rows of two: 128 independent elements per lane
+        // between one pair of waits and one proxy fence.
+        const int dw = warp - W_DEQ, stage = dw % C::SPS, row0 = (dw / C::SPS) * (64 / C::CH64) + lane;
+        int rs = 0; uint32_t rph = 0, seq = (uint32_t)stage;
+        for (int it = it_begin; it < it_end; ++it, seq += C::SPS) {
+            const uint32_t st = seq % C::NSTG, ph = (seq / C::NSTG) & 1;
             wait(&raw_full[rs], rph);
-            // With four places or more a warp's next place cannot be two uses ahead of it (the MMAs take the steps in order); with three it can, so
-            // there the warp follows every step's place and a parity never stands for the wrong use.
-            if constexpr (C::NA < 4) {
-                for (uint32_t u = seq - (uint32_t)g; u < seq; ++u) wait(&a_empty[u % C::NA], ((u / C::NA) & 1) ^ 1);
+            // With as many places as a super-block has stages, a warp's next place cannot be two uses ahead of it (the MMAs take the stages in
+            // order); with fewer it can, so there the warp follows every stage's place and a parity never stands for the wrong use.
+            if constexpr (C::NSTG < C::SPS) {
+                for (uint32_t u = seq - (uint32_t)stage; u < seq; ++u) wait(&empty[u % C::NSTG], ((u / C::NSTG) & 1) ^ 1);
             }
-            wait(&a_empty[as], aph ^ 1);
-            uint8_t* A = sm + C::OFF_A + as * C::A_BYTES;
+            wait(&empty[st], ph ^ 1);
             uint8_t* scw = sm + C::OFF_SCW + (it & (C::NS - 1)) * C::SCW_BYTES;
 #pragma unroll
             for (int rr = 0; rr < 2; ++rr) {
-                const int row = row0 + 32 * rr;
+                const int row = C::CH64 == 2 ? row0 : row0 + 32 * rr, g = C::CH64 == 2 ? 2 * stage + rr : stage;        // g: which 64 of the 256 elements
+                uint8_t* A = sm + st * C::STG_BYTES + (C::CH64 == 2 ? rr * 16384 : 0);
                 const uint8_t* sb = sm + C::OFF_RAW + rs * C::RAW_BYTES + row * C::SB;
                 if constexpr (QT == QT_Q4_K) {
                     const uint4 hdr = *reinterpret_cast<const uint4*>(sb);
@@ -338,9 +329,9 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
             }
             fence_proxy_async();
             __syncwarp();
-            if (lane == 0) { mbar_arrive(&a_full[as]); mbar_arrive(&raw_empty[rs]); }
-            if constexpr (C::NA < 4) {
-                for (uint32_t u = seq + 1; (u & 3) != 0; ++u) wait(&a_empty[u % C::NA], ((u / C::NA) & 1) ^ 1);
+            if (lane == 0) { mbar_arrive(&full[st]); mbar_arrive(&raw_empty[rs]); }
+            if constexpr (C::NSTG < C::SPS) {
+                for (uint32_t u = seq + 1; u % C::SPS != 0; ++u) wait(&empty[u % C::NSTG], ((u / C::NSTG) & 1) ^ 1);
             }
             if (++rs == C::NR) { rs = 0; rph ^= 1; }
         }
@@ -364,12 +355,11 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                 const float* dx = reinterpret_cast<const float*>(sm + C::OFF_DX + xs * C::DX_BYTES) + col0;
 #pragma unroll 1
                 for (int g = 0; g < C::GROUPS; ++g) {
-                    wait(&d_full[ds], dph);
-                    tc_fence_after();
+                    if (g % C::DG == 0) { wait(&d_full[ds], dph); tc_fence_after(); }
                     float dw, dm = 0.f;
                     if constexpr (C::MINS) { const float2 s = reinterpret_cast<const float2*>(scw)[row]; dw = s.x; dm = s.y; }
                     else dw = reinterpret_cast<const float*>(scw)[g * 128 + row];
-                    const uint32_t d = tmem + (uint32_t)(ds * C::D_COLS + col0) + ((uint32_t)(q * 32) << 16);
+                    const uint32_t d = tmem + (uint32_t)(ds * C::D_COLS + (g % C::DG) * NT + col0) + ((uint32_t)(q * 32) << 16);
 #pragma unroll
                     for (int c = 0; c < C::ACC; c += CH) {
                         uint32_t r[CH], s[CH];
@@ -388,10 +378,12 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                             }
                         }
                     }
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&d_empty[ds]);
-                    if (++ds == C::ND) { ds = 0; dph ^= 1; }
+                    if (g % C::DG == C::DG - 1) {
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&d_empty[ds]);
+                        if (++ds == 2) { ds = 0; dph ^= 1; }
+                    }
                 }
                 if (++xs == C::NS) { xs = 0; xph ^= 1; }
             }
