@@ -414,6 +414,71 @@ embed_decode_kernel(const bf16* __restrict__ embed, int H, const SeqState* __res
     for (int i = threadIdx.x; i < H; i += blockDim.x) x[(size_t)b * H + i] = __bfloat162float(row[i]);
 }
 
+// =====================================================================================
+// Greedy argmax of a batch's logits rows (two launches: parts of every row, then one block per row)
+// =====================================================================================
+__device__ __forceinline__ void arg_better(float& bv, int& bi, float v, int i) {
+    if (v > bv || (v == bv && i < bi)) { bv = v; bi = i; }
+}
+__device__ __forceinline__ void arg_warp(float& bv, int& bi) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+        arg_better(bv, bi, ov, oi);
+    }
+}
+__global__ void __launch_bounds__(256)
+argmax_row_parts_kernel(const float* __restrict__ logits, int V, float* __restrict__ pv, int* __restrict__ pi) {
+    pdl_wait();
+    pdl_launch_dependents();
+    __shared__ float sv[8];
+    __shared__ int si[8];
+    const int b = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const float* row = logits + (size_t)b * V;
+    const int per = (V + ARGMAX_ROW_PARTS - 1) / ARGMAX_ROW_PARTS, lo = blockIdx.x * per, hi = min(V, lo + per);
+    float bv = -INFINITY; int bi = 0x7fffffff;
+    for (int i = lo + threadIdx.x; i < hi; i += 256) if (row[i] > bv) { bv = row[i]; bi = i; }
+    arg_warp(bv, bi);
+    if (lane == 0) { sv[warp] = bv; si[warp] = bi; }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) arg_better(bv, bi, sv[w], si[w]);
+        pv[b * ARGMAX_ROW_PARTS + blockIdx.x] = bv; pi[b * ARGMAX_ROW_PARTS + blockIdx.x] = bi;
+    }
+}
+__global__ void __launch_bounds__(256)
+argmax_row_finish_kernel(const float* __restrict__ pv, const int* __restrict__ pi, SeqState* state, uint32_t* out_tokens, int out_stride,
+                         const bf16* __restrict__ embed, float* __restrict__ x_next, int H, int V, int advance) {
+    pdl_wait();
+    pdl_launch_dependents();
+    __shared__ uint32_t tok_s;
+    const int b = blockIdx.x;
+    if (threadIdx.x < 32) {
+        float bv = pv[b * ARGMAX_ROW_PARTS + threadIdx.x]; int bi = pi[b * ARGMAX_ROW_PARTS + threadIdx.x];
+        arg_warp(bv, bi);
+        if ((unsigned)bi >= (unsigned)V) bi = 0;             // an all-NaN row has no maximum: never gather from an out-of-range id
+        if (threadIdx.x == 0) {
+            SeqState* s = state + b;
+            out_tokens[(size_t)b * out_stride + s->step] = (uint32_t)bi;
+            const uint32_t fed = advance == 2 ? s->token : (uint32_t)bi;
+            tok_s = fed;
+            if (advance) { s->token = fed; s->kv_len += 1; s->pos[0] += 1; s->pos[1] += 1; s->pos[2] += 1; }
+            s->step += 1;
+        }
+    }
+    __syncthreads();
+    if (advance && embed != nullptr) {
+        const bf16* row = embed + (size_t)tok_s * H;
+        for (int i = threadIdx.x; i < H; i += 256) x_next[(size_t)b * H + i] = __bfloat162float(row[i]);
+    }
+}
+int argmax_rows_launch(cudaStream_t st, int B, const float* logits, int V, float* part_val, int* part_idx, SeqState* state, uint32_t* out_tokens, int out_stride,
+                       const bf16* embed, float* x_next, int H, int advance, bool pdl) {
+    if (const int e = launch_k(argmax_row_parts_kernel, dim3(ARGMAX_ROW_PARTS, B), dim3(256), 0, st, pdl, logits, V, part_val, part_idx)) return e;
+    return launch_k(argmax_row_finish_kernel, dim3(B), dim3(256), 0, st, pdl, part_val, part_idx, state, out_tokens, out_stride, embed, x_next, H, V, advance);
+}
+
 int embed_decode_launch(cudaStream_t st, int B, const bf16* embed, int H, const SeqState* state, float* x, bool pdl) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(B);

@@ -19,7 +19,6 @@ namespace cb {
 
 constexpr int KV_PAGE = 64;        // tokens per KV page
 constexpr int ATTN_NSPLIT = 8;     // split-KV factor == thread-block cluster size (static grid: the step lives in a CUDA graph)
-constexpr int MAX_BATCH = 8;
 
 // Device-resident per-sequence decode state (lets a whole decode step replay as a CUDA graph).
 struct SeqState {
@@ -106,6 +105,12 @@ int gemv_max_group(int K, int N, int num_sms);
 // (norm with a.fs_x set: the parallel-streams form)
 int gemv_launch(cudaStream_t st, int B, int epi, bool norm, const GemvArgs& a, int num_sms, bool pdl);
 int attn_decode_launch(cudaStream_t st, int B, int D, const AttnDecArgs& a, bool pdl);
+// Greedy choice of B logits rows and what follows it, as the GEMV's GEMV_LOGITS_ARGMAX epilogue does for up to four: (value, lowest index) maximum,
+// out_tokens[b * out_stride + step], step + 1; advance == 1 feeds the token back, 2 keeps the state's own, and either moves the positions on and
+// gathers the next input row from `embed` (nullable).  part_* [B, ARGMAX_ROW_PARTS].
+constexpr int ARGMAX_ROW_PARTS = 32;
+int argmax_rows_launch(cudaStream_t st, int B, const float* logits, int V, float* part_val, int* part_idx, SeqState* state, uint32_t* out_tokens, int out_stride,
+                       const bf16* embed, float* x_next, int H, int advance, bool pdl);
 int embed_decode_launch(cudaStream_t st, int B, const bf16* embed, int H, const SeqState* state, float* x, bool pdl);
 
 }  // namespace cb

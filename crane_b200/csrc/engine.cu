@@ -189,6 +189,21 @@ struct FosovikModel;   // layer-list models (engine_fosovik.inc)
 #include "engine_sampler.inc"
 
 struct crane_b200_model {
+    // A decode batch shares one pass over the weights: up to four sequences through the GEMVs, from wide_min on all of them (up to 64) through the
+    // tensor-core linears of few rows (gemm_rows.cu, qgemm.cu).
+    static constexpr int DECODE_GROUP_MAX = 64;
+    bool wide_ok = false;                   // ... built for this handle
+    int wide_min = 5;
+    bool wide(int B) const { return wide_ok && B >= wide_min; }
+    int decode_group(size_t left) const;    // sequences of the next group when `left` remain
+    bf16* w3_buf = nullptr;                 // three bf16 planes of a group's activations, w3_plane elements apart
+    size_t w3_plane = 0;
+    unsigned char* xqd_buf = nullptr;       // ... quantised (qrows_at, wide_rows rows)
+    int wide_rows = 0, wide_xq_mode = -1;
+    float* am_val = nullptr; int* am_idx = nullptr;
+    void linear_wide(int epi, const bf16* w, const unsigned char* qw, int qt, int N, int K, const float* xin, int ldx, const float* norm_w, float* y, int ldy,
+                     int B, bool same_input = false);
+    void enqueue_wide_step(int advance, int B);
     // ---- configuration ----
     int device = 0, num_sms = 148;
     FosovikModel* fsv = nullptr;            // "architecture": "Fosovik", "Gavipel", "Nifarax", "Puzonex", "Suvapel" or "Rupulix" -- the handle then runs ragged-batch steps (engine_fosovik.inc)
@@ -216,6 +231,7 @@ struct crane_b200_model {
     unsigned long long* ll_trace = nullptr;   // CRANE_B200_LL_TRACE=<file>: event trace of one step (tools/ll_trace.py)
     void ll_err_fetch();                   // enqueue the D2H copy of the flag (before a stream sync the caller does anyway)
     void ll_err_verify();                  // after that sync
+    void wait_verify();
     // vision
     int v_depth = 0, v_H = 0, v_I = 0, v_nh = 0, v_hd = 0, v_patch = 16, v_merge = 2, v_tpatch = 2, v_in = 3, v_out = 0,
         v_npos = 0, v_side = 0;
@@ -287,8 +303,9 @@ struct crane_b200_model {
     // Sequence state travels host -> device through a ring of pinned snapshots, one per call: the ABI hands out stream-ordered
     // results, so a caller may issue the next call before the previous upload has run, and a single staging slot would be
     // overwritten under it.  A slot is reused only after its own upload has completed (its event).
-    static constexpr int STATE_RING = 16, STATE_GROUP = 4;
-    SeqState* h_state_ring = nullptr; // pinned [STATE_RING][STATE_GROUP]
+    static constexpr int STATE_RING = 16;
+    int state_group = 4;              // sequences per snapshot
+    SeqState* h_state_ring = nullptr; // pinned [STATE_RING][state_group]
     cudaEvent_t h_state_ev[STATE_RING] = {};
     bool h_state_used[STATE_RING] = {};
     int h_state_next = 0;
@@ -296,7 +313,7 @@ struct crane_b200_model {
     SeqState* stage_state() {
         const int i = h_state_next;
         if (h_state_used[i]) CUDA_OK(cudaEventSynchronize(h_state_ev[i]));
-        h_state = h_state_ring + (size_t)i * STATE_GROUP;
+        h_state = h_state_ring + (size_t)i * state_group;
         return h_state;
     }
     void push_state(int nseq) {       // upload the staged snapshot(s) to the device-resident state
@@ -346,14 +363,14 @@ struct crane_b200_model {
     void park_gdn_state(int slot);         // working recurrent / conv state -> the slot's store (hybrid models)
     void fork_seq(int src, int dst);
     const int* bt_cur() const { return block_table + (size_t)cur * max_pages; }
-    cudaGraphExec_t graph_step[2][5] = {};   // [advance][sequences in the group: 1, 2, 4]
+    cudaGraphExec_t graph_step[2][DECODE_GROUP_MAX + 1] = {};   // [advance][sequences in the group]
     bool graph_failed = false;
     cudaEvent_t pev0 = nullptr, pev1 = nullptr, dev0 = nullptr, dev1 = nullptr;
     bool pev0_armed = false;
     float last_prefill_ms = 0.f, last_decode_ms = 0.f;
     size_t last_decode_steps = 0;
     uint64_t launches = 0;
-    uint64_t graph_launches[2][5] = {};
+    uint64_t graph_launches[2][DECODE_GROUP_MAX + 1] = {};
     unsigned char* xqr_buf = nullptr;  // activation rows quantised for the tensor-core linears (qrows_at), xqr_rows of them
     int xqr_rows = 0, xqr_mode_last = -1;
     unsigned char* xq_buf = nullptr;   // activations quantised for the quantised GEMVs (xquant_launch)
@@ -440,6 +457,7 @@ struct crane_b200_model {
     // forward paths
     void arm_state(uint32_t token, size_t start_pos, int p0, int p1, int p2);
     void enqueue_decode_step(int advance, bool with_embed, int B = 1);
+    void attn_decode(LayerW& l, int B);
     void decode_step_graphed(int advance, int B = 1);
     void decode_steps(int n_steps, int advance);
     void prefill(const uint32_t* ids, const float* embeds, size_t S, const uint32_t* pos3_host, size_t start_pos,
@@ -1145,7 +1163,23 @@ void crane_b200_model::finalize() {
     seq_kv.assign(max_batch, 0); seq_pos.assign(max_batch, 0); seq_used.assign(max_batch, 0);
     seq_used[0] = 1;
 
-    const int B = std::min(max_batch, 4);   // decode batches run in groups of <= 4 sequences per weight pass
+    wide_ok = !hybrid && !is_tts && owns_stream && !use_simt && max_batch > 1;
+    const int B = std::min(max_batch, wide_ok ? (int)DECODE_GROUP_MAX : 4);   // sequences per weight pass
+    state_group = B;
+    if (wide_ok) {
+        const int kmax = std::max(std::max(H, I), q_dim());
+        wide_rows = B;
+        w3_plane = (size_t)B * kmax;
+        w3_buf = dalloc<bf16>(3 * w3_plane);
+        if (any_quant) xqd_buf = dalloc<unsigned char>(qrows_bytes(B, kmax));
+        am_val = dalloc<float>((size_t)B * ARGMAX_ROW_PARTS); am_idx = dalloc<int>((size_t)B * ARGMAX_ROW_PARTS);
+        // (the scratch of the tensor-core linears: here, not under a graph capture)
+        TcScratch sc;
+        LAUNCH_OK(tc_scratch_get(stream, TC_WS_FLOATS, 4096, &sc));
+        wide_ok = (std::max(std::max(V, 2 * I), qkv_dim()) + 127) / 128 <= 4096;
+        // below wide_min the GEMVs (up to four sequences per pass) are as fast or faster
+        wide_min = any_quant ? 5 : 3;
+    }
     x_dec = dalloc<float>((size_t)B * H);
     qkv_dec = dalloc<float>((size_t)B * qkv_dim());
     attn_dec = dalloc<float>((size_t)B * q_dim());
@@ -1183,7 +1217,7 @@ void crane_b200_model::finalize() {
         if (getenv("CRANE_B200_PROF")) { ll_prof = dalloc<unsigned long long>(16); CUDA_OK(cudaMemset(ll_prof, 0, 128)); }
         if (getenv("CRANE_B200_LL_TRACE")) ll_trace = dalloc<unsigned long long>((size_t)6 * LL_TRACE_CAP * 2);
     }
-    CUDA_OK(cudaMallocHost((void**)&h_state_ring, sizeof(SeqState) * STATE_RING * STATE_GROUP));
+    CUDA_OK(cudaMallocHost((void**)&h_state_ring, sizeof(SeqState) * STATE_RING * state_group));
     for (auto& e : h_state_ev) CUDA_OK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     CUDA_OK(cudaMallocHost((void**)&h_tokens, sizeof(uint32_t) * out_cap));
     CUDA_OK(cudaEventCreate(&pev0));
@@ -1252,7 +1286,24 @@ void crane_b200_model::embed_step_input(int B) {
     ++launches;
 }
 
+void crane_b200_model::attn_decode(LayerW& l, int B) {
+    AttnDecArgs a = {};
+    a.qkv = qkv_dec; a.q_stride = q_stride(); a.gated = hybrid ? 1 : 0; a.rot_half = rot_half;
+    a.q_norm_w = l.qn; a.k_norm_w = l.kn; a.eps = eps; a.cos_tab = cos_tab; a.sin_tab = sin_tab; a.axis_of = axis_of;
+    a.state = state; a.block_table = block_table; a.max_pages = max_pages; a.k_pool = l.k_pool; a.v_pool = l.v_pool;
+    a.nh = nh; a.nkv = nkv; a.scale = 1.0f / std::sqrt((float)D);
+    a.out = attn_dec; a.kv_lo_off = kv_bits ? 0 : lo_kv;
+    a.kv_bits = kv_bits; a.kv_split = split ? 1 : 0; a.k_codes = l.k_codes; a.v_codes = l.v_codes; a.k_scale = l.k_scale; a.v_scale = l.v_scale;
+    LAUNCH_OK(attn_decode_launch(stream, B, D, a, use_pdl));
+    ++launches;   // attention
+}
+
 void crane_b200_model::enqueue_decode_step(int advance, bool with_embed, int B) {
+    if (wide(B)) {
+        if (with_embed) embed_step_input(B);
+        enqueue_wide_step(advance, B);
+        return;
+    }
     const bool pdl = use_pdl;
     if (with_embed) embed_step_input(B);
     for (int li = 0; li < L; ++li) {
@@ -1266,15 +1317,7 @@ void crane_b200_model::enqueue_decode_step(int advance, bool with_embed, int B) 
             } else {
                 linear_decode(GEMV_STORE, true, l.wqkv, nullptr, 0, qkv_dim(), H, x_dec, H, l.ln1, qkv_dec, qkv_dim(), nullptr, B);
             }
-            AttnDecArgs a = {};
-            a.qkv = qkv_dec; a.q_stride = q_stride(); a.gated = hybrid ? 1 : 0; a.rot_half = rot_half;
-            a.q_norm_w = l.qn; a.k_norm_w = l.kn; a.eps = eps; a.cos_tab = cos_tab; a.sin_tab = sin_tab; a.axis_of = axis_of;
-            a.state = state; a.block_table = block_table; a.max_pages = max_pages; a.k_pool = l.k_pool; a.v_pool = l.v_pool;
-            a.nh = nh; a.nkv = nkv; a.scale = 1.0f / std::sqrt((float)D);
-            a.out = attn_dec; a.kv_lo_off = kv_bits ? 0 : lo_kv;
-            a.kv_bits = kv_bits; a.kv_split = split ? 1 : 0; a.k_codes = l.k_codes; a.v_codes = l.v_codes; a.k_scale = l.k_scale; a.v_scale = l.v_scale;
-            LAUNCH_OK(attn_decode_launch(stream, B, D, a, pdl));
-            ++launches;   // attention
+            attn_decode(l, B);
             linear_decode(GEMV_RESID, false, l.wo, l.q_wo, l.qt_o, H, q_dim(), attn_dec, q_dim(), nullptr, x_dec, H, nullptr, B);
         } else {   // Gated-Delta-Net token mixer (ops/gdn/layer.rs:122-163), S = 1
             GemvArgs g = {};
@@ -1381,6 +1424,61 @@ void crane_b200_model::lm_head_last_row(const float* xrow, int advance, int B) {
     if (advance && q_embed && !hov.gather_set) embed_step_input(B);
 }
 
+int crane_b200_model::decode_group(size_t left) const {
+    if (wide_ok && left >= (size_t)wide_min) return (int)std::min<size_t>(left, DECODE_GROUP_MAX);
+    int maxg = 4;
+    if (!any_quant)
+        for (int K : {H, I, q_dim()}) maxg = std::min(maxg, gemv_max_group(K, V, num_sms));
+    return std::min(maxg, left >= 4 ? 4 : left >= 2 ? 2 : 1);
+}
+
+// y = epi(W x) of a group's rows, f32 in and out: the rows as three bf16 planes (24 bits), or as Q8 codes in front of a quantised matrix.
+// `same_input`: the rows are as the previous call left them (same input and norm) -- still checked against the block rule it used.
+void crane_b200_model::linear_wide(int epi, const bf16* w, const unsigned char* qw, int qt, int N, int K, const float* xin, int ldx, const float* norm_w,
+                                   float* y, int ldy, int B, bool same_input) {
+    if (qt) {
+        const int mode = xq_mode_for(qt);
+        const QRows xr = qrows_at(xqd_buf, wide_rows, K);
+        if (!same_input || mode != wide_xq_mode) {
+            LAUNCH_OK(xquant_rows_launch(stream, B, xin, ldx, K, norm_w, eps, mode, xr, use_pdl));
+            wide_xq_mode = mode;
+            ++launches;
+        }
+        LAUNCH_OK(qgemm_launch(stream, qt, qw, xr, B, N, K, epi, y, ldy, use_pdl));
+    } else {
+        if (!same_input) {
+            LAUNCH_OK(rows_split3_launch(stream, xin, ldx, B, K, norm_w, eps, w3_buf, (long long)w3_plane, use_pdl));
+            ++launches;
+        }
+        const bf16* planes[3] = {w3_buf, w3_buf + w3_plane, w3_buf + 2 * w3_plane};
+        GemmEpi ep{y, nullptr, ldy, nullptr, epi == GEMV_RESID ? EPI_RESID_F32 : epi == GEMV_SILU_MUL ? EPI_SILU_MUL_F32 : EPI_STORE_F32};
+        LAUNCH_OK(gemm_rows_launch(stream, planes, 3, K, w, B, N, K, ep, use_pdl));
+    }
+    ++launches;
+}
+
+void crane_b200_model::enqueue_wide_step(int advance, int B) {
+    for (int li = 0; li < L; ++li) {
+        LayerW& l = layers[li];
+        if (l.qt_q) {
+            const int qs = nh * q_stride(), kvd = nkv * D;
+            linear_wide(GEMV_STORE, nullptr, l.q_wq, l.qt_q, qs, H, x_dec, H, l.ln1, qkv_dec, qkv_dim(), B);
+            linear_wide(GEMV_STORE, nullptr, l.q_wk, l.qt_k, kvd, H, x_dec, H, l.ln1, qkv_dec + qs, qkv_dim(), B, true);
+            linear_wide(GEMV_STORE, nullptr, l.q_wv, l.qt_v, kvd, H, x_dec, H, l.ln1, qkv_dec + qs + kvd, qkv_dim(), B, true);
+        } else {
+            linear_wide(GEMV_STORE, l.wqkv, nullptr, 0, qkv_dim(), H, x_dec, H, l.ln1, qkv_dec, qkv_dim(), B);
+        }
+        attn_decode(l, B);
+        linear_wide(GEMV_RESID, l.wo, l.q_wo, l.qt_o, H, q_dim(), attn_dec, q_dim(), nullptr, x_dec, H, B);
+        linear_wide(GEMV_SILU_MUL, l.wgu, l.q_wgu, l.qt_gu, 2 * I, H, x_dec, H, l.ln2, act_dec, I, B);
+        linear_wide(GEMV_RESID, l.wdown, l.q_wdown, l.qt_down, H, I, act_dec, I, nullptr, x_dec, H, B);
+    }
+    linear_wide(GEMV_STORE, lm_head, q_lm_head, qt_lm, V, H, x_dec, H, final_norm, logits, V, B);
+    LAUNCH_OK(argmax_rows_launch(stream, B, logits, V, am_val, am_idx, state, out_tokens, out_cap, q_embed ? nullptr : embed, x_dec, H, advance, use_pdl));
+    launches += 2;
+    if (advance && q_embed) embed_step_input(B);
+}
+
 // One decode step (layers + lm_head), replayed from a CUDA graph when capture is available.
 void crane_b200_model::decode_step_graphed(int advance, int B) {
     cudaGraphExec_t& ge = graph_step[advance][B];
@@ -1465,12 +1563,16 @@ void crane_b200_model::decode_steps(int n_steps, int advance) {
     for (int i = 0; i < n_steps; ++i) decode_step_graphed(advance);
 }
 
+// The tensor-core kernels bound theirs too (tc.cuh): read after a synchronisation of the stream.
+void crane_b200_model::wait_verify() {
+    if (tc_take_wait_error(stream)) fail(CRANE_B200_CUDA_ERROR, "a tensor-core kernel's wait ran out (results discarded)");
+}
 // The persistent kernel bounds every wait; a wait that gave up leaves garbage behind and raises this flag (read at sync points).
 void crane_b200_model::ll_err_fetch() {
     if (ll_err) CUDA_OK(cudaMemcpyAsync(h_ll_err, ll_err, sizeof(unsigned int), cudaMemcpyDeviceToHost, stream));
 }
 void crane_b200_model::ll_err_verify() {
-    if (tc_take_wait_error(stream)) fail(CRANE_B200_CUDA_ERROR, "a tensor-core kernel's wait ran out (results discarded)");
+    wait_verify();
     if (!ll_err || *h_ll_err == 0) return;
     std::vector<unsigned int> d(16 + num_sms * LL_WARPS);
     CUDA_OK(cudaMemcpy(d.data(), ll_err, d.size() * sizeof(unsigned int), cudaMemcpyDeviceToHost));
@@ -2469,13 +2571,9 @@ int crane_b200_decode_batch(crane_b200_model* m, const int* seqs, const uint32_t
         if (m->seq_kv[s] + n_steps > (size_t)m->max_seq) fail(CRANE_B200_OOM, "sequence %d would exceed max_seq_len %d", s, m->max_seq);
     }
     CUDA_OK(cudaEventRecord(m->dev0, m->stream));
-    // groups of 4 / 2 / 1 sequences share one pass over the weights (cb::gemv_kernel<B>)
-    int maxg = 4;
-    if (!m->any_quant)
-        for (int K : {m->H, m->I, m->q_dim()}) maxg = std::min(maxg, gemv_max_group(K, m->V, m->num_sms));
     size_t done = 0;
     while (done < n) {
-        const int B = std::min(maxg, (n - done >= 4) ? 4 : (n - done >= 2) ? 2 : 1);
+        const int B = m->decode_group(n - done);
         m->stage_state();
         for (int b = 0; b < B; ++b) {
             const int s = seqs[done + b];
@@ -2489,12 +2587,15 @@ int crane_b200_decode_batch(crane_b200_model* m, const int* seqs, const uint32_t
         m->push_state(B);
         m->embed_step_input(B);
         for (size_t t = 0; t < n_steps; ++t) m->decode_step_graphed(1, B);
-        for (int b = 0; b < B; ++b)
-            CUDA_OK(cudaMemcpyAsync(tokens_out + (done + b) * n_steps, m->out_tokens + (size_t)b * m->out_cap, n_steps * sizeof(uint32_t),
-                                    cudaMemcpyDeviceToHost, m->stream));
+        // (through pinned memory while they fit: B copies into the caller's pageable rows cost more than a step)
+        const bool pinned = (size_t)B * n_steps <= (size_t)m->out_cap;
+        CUDA_OK(cudaMemcpy2DAsync(pinned ? m->h_tokens : tokens_out + done * n_steps, n_steps * sizeof(uint32_t), m->out_tokens, (size_t)m->out_cap * sizeof(uint32_t),
+                                  n_steps * sizeof(uint32_t), B, cudaMemcpyDeviceToHost, m->stream));
         if (logits_host)
             CUDA_OK(cudaMemcpyAsync(logits_host + done * (size_t)m->V, m->logits, (size_t)B * m->V * sizeof(float), cudaMemcpyDeviceToHost, m->stream));
         CUDA_OK(cudaStreamSynchronize(m->stream));     // tokens_out / logits_host are the caller's memory: complete before returning
+        m->wait_verify();
+        if (pinned) std::memcpy(tokens_out + done * n_steps, m->h_tokens, (size_t)B * n_steps * sizeof(uint32_t));
         for (int b = 0; b < B; ++b) {
             const int s = seqs[done + b];
             m->seq_kv[s] += n_steps;
@@ -2589,12 +2690,9 @@ int crane_b200_decode_batch_sample(crane_b200_model* m, const int* seqs, const u
         if (tokens[i] >= (uint32_t)m->V) fail(CRANE_B200_INVALID_ARG, "token id %u >= vocab %d", tokens[i], m->V);
         if (m->seq_kv[s] + 1 > (size_t)m->max_seq) fail(CRANE_B200_OOM, "sequence %d would exceed max_seq_len %d", s, m->max_seq);
     }
-    int maxg = 4;
-    if (!m->any_quant)
-        for (int K : {m->H, m->I, m->q_dim()}) maxg = std::min(maxg, gemv_max_group(K, m->V, m->num_sms));
     size_t done = 0;
     while (done < n) {
-        const int B = std::min(maxg, (n - done >= 4) ? 4 : (n - done >= 2) ? 2 : 1);
+        const int B = m->decode_group(n - done);
         m->stage_state();
         for (int b = 0; b < B; ++b) {
             const int s = seqs[done + b];

@@ -483,6 +483,9 @@ static GemmPlan gemm_plan(int M, int N, int K, bool split, int sms) {
     return best;
 }
 
+// Up to this many rows (one 128-row tile) the weights are the tile and the rows its columns: gemm_rows.cu.
+constexpr int GEMM_ROWS_MAX = 128;
+
 template <int MODE>
 static int launch_mode(cudaStream_t stream, const bf16* A, const bf16* A_lo, int lda, const bf16* W, int M, int N, int K,
                        const GemmEpi& epi, bool use_simt) {
@@ -509,6 +512,10 @@ static int launch_mode(cudaStream_t stream, const bf16* A, const bf16* A_lo, int
 int gemm_bf16_launch(cudaStream_t stream, const bf16* A, const bf16* A_lo, int lda, const bf16* W, int M, int N, int K,
                      const GemmEpi& epi, bool use_simt) {
     if (M <= 0 || N <= 0 || K <= 0 || (K % GEMM_BK) != 0 || (N % 32) != 0 || (lda % 8) != 0) return -1000;
+    if (!use_simt && M <= GEMM_ROWS_MAX && epi.prof == nullptr) {
+        const bf16* planes[3] = {A, A_lo, nullptr};
+        return gemm_rows_launch(stream, planes, A_lo ? 2 : 1, lda, W, M, N, K, epi, prefill_pdl());
+    }
     switch (epi.mode) {
         case EPI_STORE_F32:      return launch_mode<EPI_STORE_F32>(stream, A, A_lo, lda, W, M, N, K, epi, use_simt);
         case EPI_STORE_BF16:     return launch_mode<EPI_STORE_BF16>(stream, A, A_lo, lda, W, M, N, K, epi, use_simt);

@@ -24,7 +24,8 @@ enum GemmEpiMode : int {
                            // the clamped unit instead: g = min(acc[2j], L), u = clamp(acc[2j+1], -L, L), out = g * sigmoid(1.702 g) * (u + 1)
     EPI_GELU_ERF_BF16 = 4, // out bf16 = gelu_erf(acc + bias)
     EPI_GELU_TANH_BF16 = 5, // out bf16 = gelu_tanh(acc + bias)
-    EPI_RELU2_BF16 = 6     // out bf16 = max(acc + bias, 0)^2
+    EPI_RELU2_BF16 = 6,    // out bf16 = max(acc + bias, 0)^2
+    EPI_SILU_MUL_F32 = 7   // as EPI_SILU_MUL_BF16 with an f32 output (gemm_rows_launch with three planes only)
 };
 
 struct GemmEpi {
@@ -48,6 +49,11 @@ struct TmaEncoder;  // host: resolves cuTensorMapEncodeTiled once
 // `A_lo` (nullable): low-order plane of a split-precision activation operand, same shape/stride as A (see gemm.cu).
 int gemm_bf16_launch(cudaStream_t stream, const bf16* A, const bf16* A_lo, int lda, const bf16* W, int M, int N, int K,
                      const GemmEpi& epi, bool use_simt);
+// Few activation rows, 1 .. 3 bf16 planes (gemm_rows.cu); planes share lda.  gemm_bf16_launch comes here by itself where it pays.
+bool gemm_rows_fits(int planes, int M);
+int gemm_rows_launch(cudaStream_t stream, const bf16* const* planes, int n_planes, int lda, const bf16* W, int M, int N, int K, const GemmEpi& epi, bool pdl);
+// f32 rows -> three bf16 planes `plane` elements apart, rows of K; RMS-normalised first when norm_w is set
+int rows_split3_launch(cudaStream_t stream, const float* x, int ldx, int M, int K, const float* norm_w, float eps, bf16* out, long long plane, bool pdl);
 // Frees the stream-K scratch (partial tiles, arrival counters) kept for `stream`; call before destroying the stream.
 void gemm_release_stream(cudaStream_t stream);
 

@@ -1,0 +1,362 @@
+// Linears of few activation rows (M <= 128):  C[M, N] (+)= (A_0 + .. + A_{P-1})[M, K] x W[N, K]^T, the activations as P = 1 .. 3 bf16 planes.
+//
+// What bounds it is the weight bytes, which pass once whatever M is, so the tile is the weights': 128 weight rows are the MMA's M, and the planes of all
+// activation rows side by side are its N (P x M rounded up to 16 columns: a batch of 32 in three planes is one MMA of 96 columns); every plane has
+// accumulator columns of its own, added when they are read.  Three planes carry all 24 bits of an f32 activation (a decode batch keeps the
+// accuracy of the f32 GEMV it replaces), two the split-precision operands of the prefill, one plain bf16.
+//
+// A stage is 128 weight rows x 128 columns and the planes beside it: eight MMAs per wait and commit, because a wait costs the issuing warp as much as
+// four MMAs of these widths (tc.cuh, elect_one; gemm_tc_kernel's 64-wide stages of four take 0.33 us each whatever their width: 20 us for
+// 2048 x 2048 at 77 rows on 32 CTAs).  Stream-K over (128-row tile, 128-wide step) puts the same number of steps on every SM; partial tiles
+// are added in contributor order by the last to arrive, so the result does not depend on who that was.
+#include "gemm.cuh"
+#include "tc.cuh"
+
+#include <algorithm>
+
+namespace cb {
+
+constexpr int GR_MAX_CTAS = 160;
+constexpr int GR_W_BYTES = 128 * 256;             // weights of a stage: two 64-wide tiles
+constexpr int GR_BUDGET = 208 * 1024;
+
+struct GemmRowsArgs {
+    GemmEpi ep;
+    int M, Mp, N, KB, nstg;        // Mp: M rounded up to 16; KB: 128-wide steps
+    TcSched sc;
+    int* err;
+};
+
+// one chunk of 16 activation rows m0 .. m0 + 15 of this lane's weight row n
+template <int MODE>
+__device__ __forceinline__ void rows_epi16(const GemmEpi& ep, int M, int N, int m0, int n, float* v, int lane) {
+    const bool in = n < N;
+    const int rows = min(16, M - m0);
+    if (ep.bias && in) {
+        const float b = ep.bias[n];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] += b;
+    }
+    if (ep.col_scale && in) {
+        const float c = ep.col_scale[n];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] *= c;
+    }
+    if (ep.gate && in) {
+        const float gb = ep.gate_bias ? ep.gate_bias[n] : 0.f;
+        const float* g = ep.gate + (size_t)m0 * ep.ldg + n;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) if (j < rows) v[j] *= 1.f / (1.f + expf(-(g[(size_t)j * ep.ldg] + gb)));
+    }
+    if constexpr (MODE == EPI_STORE_F32 || MODE == EPI_RESID_F32) {
+        if (!in) return;
+        float* o = reinterpret_cast<float*>(ep.out) + (size_t)m0 * ep.ldo + n;
+        if constexpr (MODE == EPI_RESID_F32) {
+            float x[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) x[j] = j < rows ? o[(size_t)j * ep.ldo] : 0.f;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] += x[j];
+        }
+#pragma unroll
+        for (int j = 0; j < 16; ++j) if (j < rows) o[(size_t)j * ep.ldo] = v[j];
+    } else if constexpr (MODE == EPI_SILU_MUL_F32 || MODE == EPI_SILU_MUL_BF16) {
+        // rows interleaved (gate_j, up_j): an even lane has the gate, its neighbour the up; pairs of results to every fourth lane for 4-byte stores
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            const float up = __shfl_xor_sync(0xffffffffu, v[j], 1), g = glu_pair_f(v[j], up, ep.glu_limit);
+            if constexpr (MODE == EPI_SILU_MUL_F32) {
+                if (!(lane & 1) && in && j < rows) reinterpret_cast<float*>(ep.out)[(size_t)(m0 + j) * ep.ldo + (n >> 1)] = g;
+            } else {
+                const float g2 = __shfl_xor_sync(0xffffffffu, g, 2);
+                if (!(lane & 3) && in && j < rows) {
+                    uint32_t hi, lo;
+                    split_bf16x2(g, g2, hi, lo);
+                    const size_t off = (size_t)(m0 + j) * ep.ldo + (n >> 1);
+                    *reinterpret_cast<uint32_t*>(reinterpret_cast<bf16*>(ep.out) + off) = hi;
+                    if (ep.out_lo) *reinterpret_cast<uint32_t*>(reinterpret_cast<bf16*>(ep.out_lo) + off) = lo;
+                }
+            }
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            float a = v[j];
+            if constexpr (MODE == EPI_GELU_ERF_BF16) a = gelu_erf_f(a);
+            else if constexpr (MODE == EPI_GELU_TANH_BF16) a = gelu_tanh_f(a);
+            else if constexpr (MODE == EPI_RELU2_BF16) { a = fmaxf(a, 0.f); a *= a; }
+            const float b = __shfl_xor_sync(0xffffffffu, a, 1);
+            if (!(lane & 1) && in && j < rows) {
+                uint32_t hi, lo;
+                split_bf16x2(a, b, hi, lo);
+                const size_t off = (size_t)(m0 + j) * ep.ldo + n;
+                *reinterpret_cast<uint32_t*>(reinterpret_cast<bf16*>(ep.out) + off) = hi;
+                if (ep.out_lo) *reinterpret_cast<uint32_t*>(reinterpret_cast<bf16*>(ep.out_lo) + off) = lo;
+            }
+        }
+    }
+}
+
+//   warp 0: TMA producer    warp 1: MMA issuer    warp 2: TMEM allocator    warps 4 - 7: epilogue (TMEM lanes 32 (warp % 4) ..)
+template <int P, int MODE>
+__global__ void __launch_bounds__(256, 1)
+gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmA1,
+                 const __grid_constant__ CUtensorMap tmA2, GemmRowsArgs a) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    __shared__ uint64_t full[8], empty[8], d_full[2], d_empty[2];
+    __shared__ uint32_t tmem_slot;
+    __shared__ int last_flag, gave_up;
+    const TcWait wait{&gave_up, a.err};
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int Mp = a.Mp, KB = a.KB, nstg = a.nstg, cols = P * Mp, stg_bytes = GR_W_BYTES + cols * 256;
+    const int it_begin = sched_start(a.sc, blockIdx.x), it_end = sched_start(a.sc, blockIdx.x + 1);
+
+    if (threadIdx.x == 0) {
+        gave_up = 0;
+        for (int i = 0; i < nstg; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
+        for (int i = 0; i < 2; ++i) { mbar_init(&d_full[i], 1); mbar_init(&d_empty[i], 4); }
+        fence_barrier_init();
+    }
+    if (warp == 2) { tmem_alloc(&tmem_slot, 512); tmem_relinquish(); }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+    pdl_launch_dependents();
+
+    if (warp == 0) {
+        if (lane == 0) {
+            tma_prefetch_desc(&tmW); tma_prefetch_desc(&tmA0);
+            auto weights = [&](int it, int st) {
+                mbar_arrive_expect_tx(&full[st], stg_bytes);
+                const int n0 = it / KB * 128, k0 = it % KB * 128;
+                tma_load_2d(sm + st * stg_bytes, &tmW, &full[st], k0, n0);
+                tma_load_2d(sm + st * stg_bytes + GR_W_BYTES / 2, &tmW, &full[st], k0 + 64, n0);
+            };
+            // weights do not depend on the predecessor kernel: the first stages' go out before the dependency wait
+            const int npre = a.ep.w_dynamic ? 0 : min(it_end - it_begin, nstg);
+            for (int i = 0; i < npre; ++i) weights(it_begin + i, i);
+            pdl_wait();
+            int st = 0; uint32_t ph = 0;
+            for (int it = it_begin; it < it_end; ++it) {
+                if (it - it_begin >= npre) { wait(&empty[st], ph ^ 1); weights(it, st); }
+                const int k0 = it % KB * 128;
+                uint8_t* b = sm + st * stg_bytes + GR_W_BYTES;
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    tma_load_2d(b + c * cols * 128, &tmA0, &full[st], k0 + 64 * c, 0);
+                    if (P > 1) tma_load_2d(b + c * cols * 128 + Mp * 128, &tmA1, &full[st], k0 + 64 * c, 0);
+                    if (P > 2) tma_load_2d(b + c * cols * 128 + 2 * Mp * 128, &tmA2, &full[st], k0 + 64 * c, 0);
+                }
+                if (++st == nstg) { st = 0; ph ^= 1; }
+            }
+            wait.drain();
+        }
+    } else if (warp == 1) {
+        const uint32_t idesc = make_idesc_bf16(128, cols);
+        int st = 0, seg = 0; uint32_t ph = 0;
+        for (int it = it_begin; it < it_end; ++seg) {
+            const int seg_end = min(it_end, (it / KB + 1) * KB), b = seg & 1;
+            wait(&d_empty[b], ((seg >> 1) & 1) ^ 1);
+            tc_fence_after();
+            const uint32_t d = tmem + (uint32_t)(b * 256);
+            for (int i = it; i < seg_end; ++i) {
+                wait(&full[st], ph);
+                tc_fence_after();
+                const uint32_t wa = smem_u32(sm + st * stg_bytes);
+                const uint64_t wd = make_smem_desc_sw128(wa), ad = make_smem_desc_sw128(wa + GR_W_BYTES);
+                if (elect_one()) {
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)
+                        umma_bf16(d, wd + (uint64_t)((k >> 2) * (GR_W_BYTES / 32) + 2 * (k & 3)), ad + (uint64_t)((k >> 2) * cols * 8 + 2 * (k & 3)), idesc,
+                                  (uint32_t)((i != it) | (k != 0)));
+                    umma_commit(&empty[st]);
+                    if (i == seg_end - 1) umma_commit(&d_full[b]);
+                }
+                __syncwarp();
+                if (++st == nstg) { st = 0; ph ^= 1; }
+            }
+            it = seg_end;
+        }
+    } else if (warp >= 4) {
+        pdl_wait();                                 // (reads / overwrites activations of the predecessor too)
+        const int q = warp & 3, row = q * 32 + lane;
+        const size_t tile_f = (size_t)128 * Mp;
+        int seg = 0;
+        for (int it = it_begin; it < it_end; ++seg) {
+            const int seg_end = min(it_end, (it / KB + 1) * KB), t = it / KB, n = t * 128 + row, b = seg & 1;
+            const bool sole = it % KB == 0 && seg_end - it == KB;
+            const uint32_t d = tmem + (uint32_t)(b * 256) + ((uint32_t)(q * 32) << 16);
+            wait(&d_full[b], (seg >> 1) & 1);
+            tc_fence_after();
+            float* mine = a.sc.ws + (size_t)(2 * blockIdx.x + (it == it_begin ? 0 : 1)) * tile_f + row;
+#pragma unroll 1
+            for (int c = 0; c < Mp; c += 16) {
+                uint32_t r0[16], r1[16], r2[16];
+                tmem_ld16_async(d + c, r0);
+                if (P > 1) tmem_ld16_async(d + Mp + c, r1);
+                if (P > 2) tmem_ld16_async(d + 2 * Mp + c, r2);
+                tmem_ld_wait();
+                float v[16];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {      // small terms first
+                    v[j] = __uint_as_float(r0[j]);
+                    if (P == 2) v[j] += __uint_as_float(r1[j]);
+                    if (P == 3) v[j] += __uint_as_float(r1[j]) + __uint_as_float(r2[j]);
+                }
+                if (sole) rows_epi16<MODE>(a.ep, a.M, a.N, c, n, v, lane);
+                else {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) mine[(size_t)(c + j) * 128] = v[j];
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&d_empty[b]);
+            if (!sole) {                            // arrive at the tile; the last of its contributors adds them in order and finishes it
+                __threadfence();
+                named_bar_sync(1, 128);
+                const int c_first = sched_owner(a.sc, t * KB), c_last = sched_owner(a.sc, t * KB + KB - 1);
+                if (threadIdx.x == 128) last_flag = atomicAdd(&a.sc.counters[t], 1) == c_last - c_first;
+                named_bar_sync(1, 128);
+                if (last_flag) {
+                    __threadfence();
+#pragma unroll 1
+                    for (int c = 0; c < Mp; c += 16) {
+                        float v[16];
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) v[j] = 0.f;
+                        for (int cc = c_first; cc <= c_last; cc += 2) {           // two contributors' loads in flight; the additions stay in order
+                            const float* p0 = a.sc.ws + (size_t)(2 * cc + (sched_start(a.sc, cc) < t * KB ? 1 : 0)) * tile_f + (size_t)c * 128 + row;
+                            const bool two = cc < c_last;
+                            const float* p1 = two ? a.sc.ws + (size_t)(2 * (cc + 1) + (sched_start(a.sc, cc + 1) < t * KB ? 1 : 0)) * tile_f + (size_t)c * 128 + row : p0;
+                            float x0[16], x1[16];
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) x0[j] = __ldcg(p0 + j * 128);
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) x1[j] = two ? __ldcg(p1 + j * 128) : 0.f;
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) v[j] += x0[j];
+                            if (two) {
+#pragma unroll
+                                for (int j = 0; j < 16; ++j) v[j] += x1[j];
+                            }
+                        }
+                        rows_epi16<MODE>(a.ep, a.M, a.N, c, n, v, lane);
+                    }
+                    if (threadIdx.x == 128) a.sc.counters[t] = 0;
+                }
+                named_bar_sync(1, 128);             // last_flag is rewritten by the next segment
+            }
+            it = seg_end;
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 2) { tc_fence_after(); tmem_dealloc(tmem, 512); }
+}
+
+template <int P, int MODE>
+static int rows_launch_t(cudaStream_t st, const bf16* const* A, int lda, const bf16* W, int M, int N, int K, const GemmEpi& ep, bool pdl) {
+    GemmRowsArgs a = {};
+    a.ep = ep; a.M = M; a.Mp = (M + 15) / 16 * 16; a.N = N; a.KB = (K + 127) / 128;
+    CUtensorMap tmW, tm[3];
+    if (!tc_tmap_bf16(&tmW, W, (uint64_t)N, (uint64_t)K, (uint64_t)K, 128)) return -1001;
+    for (int p = 0; p < 3; ++p)
+        if (!tc_tmap_bf16(&tm[p], A[p < P ? p : 0], (uint64_t)M, (uint64_t)K, (uint64_t)lda, (uint32_t)a.Mp)) return -1001;
+    const int stg = GR_W_BYTES + P * a.Mp * 256;
+    a.nstg = std::min(6, GR_BUDGET / stg);
+    static SmemOptIn seen;
+    const size_t smem = (size_t)a.nstg * stg + 1024;
+    if (const int e = ensure_dyn_smem(gemm_rows_kernel<P, MODE>, smem, seen)) return e;
+    TcSched& sc = a.sc;
+    sc.tiles_m = 1; sc.tiles_n = (N + 127) / 128; sc.KB = a.KB;
+    const long long iters = (long long)sc.tiles_n * a.KB;
+    if (iters > 0x7fffffffLL) return -1000;
+    sc.unit = 1;
+    sc.G = (int)std::max<long long>(1, std::min<long long>(std::min(tc_device_sms(), GR_MAX_CTAS), iters / 3));     // three steps pay for a CTA's setup
+    sc.base = (int)(iters / sc.G); sc.rem = (int)(iters % sc.G);
+    TcScratch s;
+    if (const int e = tc_scratch_get(st, TC_WS_FLOATS, sc.tiles_n, &s)) return e;
+    sc.ws = s.ws; sc.counters = s.counters; a.err = s.err;
+    return launch_k(gemm_rows_kernel<P, MODE>, dim3(sc.G), dim3(256), smem, st, pdl, tmW, tm[0], tm[1], tm[2], a);
+}
+
+template <int MODE>
+static int rows_launch_m(cudaStream_t st, const bf16* const* A, int P, int lda, const bf16* W, int M, int N, int K, const GemmEpi& ep, bool pdl) {
+    switch (P) {
+        case 1: return rows_launch_t<1, MODE>(st, A, lda, W, M, N, K, ep, pdl);
+        case 2: return rows_launch_t<2, MODE>(st, A, lda, W, M, N, K, ep, pdl);
+        default: return -1000;
+    }
+}
+
+bool gemm_rows_fits(int P, int M) { return M >= 1 && P * ((M + 15) / 16 * 16) <= 256; }
+
+int gemm_rows_launch(cudaStream_t st, const bf16* const* A, int P, int lda, const bf16* W, int M, int N, int K, const GemmEpi& ep, bool pdl) {
+    if (!gemm_rows_fits(P, M) || N <= 0 || K <= 0 || (K % 8) != 0 || (N % 4) != 0 || (lda % 8) != 0) return -1000;
+    if (P == 3) {                                   // the decode batch's epilogues
+        switch (ep.mode) {
+            case EPI_STORE_F32:    return rows_launch_t<3, EPI_STORE_F32>(st, A, lda, W, M, N, K, ep, pdl);
+            case EPI_RESID_F32:    return rows_launch_t<3, EPI_RESID_F32>(st, A, lda, W, M, N, K, ep, pdl);
+            case EPI_SILU_MUL_F32: return rows_launch_t<3, EPI_SILU_MUL_F32>(st, A, lda, W, M, N, K, ep, pdl);
+            default: return -1000;
+        }
+    }
+    switch (ep.mode) {
+        case EPI_STORE_F32:      return rows_launch_m<EPI_STORE_F32>(st, A, P, lda, W, M, N, K, ep, pdl);
+        case EPI_STORE_BF16:     return rows_launch_m<EPI_STORE_BF16>(st, A, P, lda, W, M, N, K, ep, pdl);
+        case EPI_RESID_F32:      return rows_launch_m<EPI_RESID_F32>(st, A, P, lda, W, M, N, K, ep, pdl);
+        case EPI_SILU_MUL_BF16:  return rows_launch_m<EPI_SILU_MUL_BF16>(st, A, P, lda, W, M, N, K, ep, pdl);
+        case EPI_GELU_ERF_BF16:  return rows_launch_m<EPI_GELU_ERF_BF16>(st, A, P, lda, W, M, N, K, ep, pdl);
+        case EPI_GELU_TANH_BF16: return rows_launch_m<EPI_GELU_TANH_BF16>(st, A, P, lda, W, M, N, K, ep, pdl);
+        case EPI_RELU2_BF16:     return rows_launch_m<EPI_RELU2_BF16>(st, A, P, lda, W, M, N, K, ep, pdl);
+        default: return -1000;
+    }
+}
+
+// f32 rows -> three bf16 planes (hi, mid, lo: all 24 bits), RMS-normalised first when norm_w is set.  One CTA per row; a few microseconds of latency.
+__global__ void __launch_bounds__(256)
+rows_split3_kernel(const float* __restrict__ x, int ldx, int K, const float* __restrict__ norm_w, float eps, bf16* __restrict__ out, long long plane) {
+    pdl_wait();
+    pdl_launch_dependents();
+    __shared__ float red[32];
+    const float* xr = x + (size_t)blockIdx.x * ldx;
+    float rstd = 1.f;
+    if (norm_w) {
+        float ssq = 0.f;
+        for (int i = threadIdx.x * 4; i < K; i += 1024) {
+            const float4 v = *reinterpret_cast<const float4*>(xr + i);
+            ssq += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+        }
+        rstd = rsqrtf(block_sum(ssq, red) / (float)K + eps);
+    }
+    bf16* o = out + (size_t)blockIdx.x * K;
+    for (int i = threadIdx.x * 4; i < K; i += 1024) {
+        float4 v = *reinterpret_cast<const float4*>(xr + i);
+        if (norm_w) {
+            const float4 g = *reinterpret_cast<const float4*>(norm_w + i);
+            v.x = v.x * rstd * g.x; v.y = v.y * rstd * g.y; v.z = v.z * rstd * g.z; v.w = v.w * rstd * g.w;
+        }
+        uint32_t h[2], m[2], l[2];
+        const float e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const float a = e[2 * k], b = e[2 * k + 1];
+            h[k] = pack_bf16(a, b);
+            const float ra = a - bf16lo(h[k]), rb = b - bf16hi(h[k]);
+            m[k] = pack_bf16(ra, rb);
+            l[k] = pack_bf16(ra - bf16lo(m[k]), rb - bf16hi(m[k]));
+        }
+        *reinterpret_cast<uint2*>(o + i) = make_uint2(h[0], h[1]);
+        *reinterpret_cast<uint2*>(o + plane + i) = make_uint2(m[0], m[1]);
+        *reinterpret_cast<uint2*>(o + 2 * plane + i) = make_uint2(l[0], l[1]);
+    }
+}
+int rows_split3_launch(cudaStream_t st, const float* x, int ldx, int M, int K, const float* norm_w, float eps, bf16* out, long long plane, bool pdl) {
+    if ((K % 4) != 0 || (ldx % 4) != 0 || M < 1) return -1000;
+    return launch_k(rows_split3_kernel, dim3(M), dim3(256), 0, st, pdl, x, ldx, K, norm_w, eps, out, plane);
+}
+
+}  // namespace cb

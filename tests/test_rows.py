@@ -1,0 +1,108 @@
+"""Linears of few rows (csrc/gemm_rows.cu) and decode batches that share one pass over the weights, at the edges of their tiles."""
+import numpy as np
+import pytest
+
+from crane_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+def planes(x):
+    hi = synth.bf16_round(x)
+    return hi, synth.bf16_round(x - hi)
+
+
+# f32 accumulation over K terms of either sign: under sqrt(K) * 2^-24 of the largest sum (4e-6 at K = 4096), eight-fold; a bf16 output adds half a unit, 2^-9
+@pytest.mark.parametrize("split", [False, True])
+@pytest.mark.parametrize("m,n,k", [(1, 32, 64), (15, 96, 192), (16, 160, 256), (17, 128, 2048), (77, 4096, 320), (113, 2080, 1024), (128, 384, 4096)])
+def test_few_rows(m, n, k, split):
+    import crane_b200 as cb
+    rng = np.random.default_rng(m * 7 + n + k)
+    hi, lo = planes(rng.standard_normal((m, k)).astype(np.float32))
+    w = synth.bf16_round((rng.standard_normal((n, k)) / np.sqrt(k)).astype(np.float32))
+    bias, init = rng.standard_normal(n).astype(np.float32), rng.standard_normal((m, n)).astype(np.float32)
+    a, al, wb = synth.f32_to_bf16_bits(hi), synth.f32_to_bf16_bits(lo) if split else None, synth.f32_to_bf16_bits(w)
+    ref = (hi.astype(np.float64) + (lo.astype(np.float64) if split else 0.0)) @ w.astype(np.float64).T
+    f32 = 8 * np.sqrt(k) * 2.0 ** -24
+
+    def close(got, want, rel):
+        assert np.abs(got - want).max() <= rel * np.abs(want).max()
+    close(cb.op_gemm(a, wb, cb.EPI_STORE_F32, bias=bias, a_lo_bits=al), ref + bias, f32)
+    out = cb.op_gemm(a, wb, cb.EPI_RESID_F32, out_init=init, a_lo_bits=al)
+    close(out, ref + init, f32)
+    assert np.array_equal(out, cb.op_gemm(a, wb, cb.EPI_RESID_F32, out_init=init, a_lo_bits=al))       # the same bits whoever came last
+    g, u = ref[:, 0::2], ref[:, 1::2]
+    close(synth.bf16_bits_to_f32(cb.op_gemm(a, wb, cb.EPI_SILU_MUL_BF16, a_lo_bits=al)), g / (1 + np.exp(-g)) * u, 2.0 ** -8)
+    close(synth.bf16_bits_to_f32(cb.op_gemm(a, wb, cb.EPI_STORE_BF16, bias=bias, a_lo_bits=al)), ref + bias, 2.0 ** -8)
+
+
+@pytest.mark.parametrize("n", [2, 3, 5, 16, 33, 64])
+@pytest.mark.parametrize("kv", ["", "int8"])
+def test_decode_batch_against_single_steps(n, kv):
+    """Rounds of a batch against the same tokens fed to every sequence by itself; the two differ by rounding alone (24-bit activations on either side,
+    KV rows rounded alike), 1e-5 over three layers; int8 pages turn that into a code here and there."""
+    import crane_b200
+    cfg = synth.TINY_QWEN3_UNTIED
+    m = crane_b200.Qwen3Model(cfg, max_seq_len=128, max_batch=64, **({"kv_cache": kv} if kv else {}))
+    m.load_checkpoint(synth.synth_checkpoint(cfg))
+    slots = [0] + [m.seq_create() for _ in range(n - 1)]
+    ids = {s: synth.synth_token_ids(5 + (7 * s) % 60, cfg["vocab_size"], f"rows-{s}") for s in slots}
+    forced = [synth.synth_token_ids(n, cfg["vocab_size"], f"rows-forced-{r}") for r in range(3)]
+    want = []
+    for j, s in enumerate(slots):
+        m.seq_select(s)
+        m.forward_step(ids[s], 0)
+        want.append([m.forward_step([int(f[j])], len(ids[s]) + r) for r, f in enumerate(forced)])
+        m.set_kv_caches([], len(ids[s]))
+    for r, f in enumerate(forced):
+        toks, got = m.decode_batch(slots, f, 1, want_logits=True)
+        ref = np.stack([w[r] for w in want])
+        assert np.abs(got - ref).max() <= (2e-2 if kv else 3e-5) * np.abs(ref).max()
+        assert np.array_equal(toks[:, 0], got.argmax(1))
+    # greedy rounds on the device: what one round chooses is what the next one reads
+    for s in slots:
+        m.seq_select(s)
+        m.set_kv_caches([], len(ids[s]))
+    three, _ = m.decode_batch(slots, forced[0], 3)
+    for s in slots:
+        m.seq_select(s)
+        m.set_kv_caches([], len(ids[s]))
+    one = np.asarray(forced[0])
+    for r in range(3):
+        one = m.decode_batch(slots, one, 1)[0][:, 0]
+        assert np.array_equal(one, three[:, r])
+    m.close()
+
+
+@pytest.mark.parametrize("recipe", ["Q4_K", "Q8_0"])
+def test_quantised_decode_batch(recipe):
+    """A batch of nine in one pass against the same in passes of up to four: the same codes and integer dots, so a one-layer model differs by f32 rounding
+    until a code sits on a border (one in 128 of its block's largest value: 1e-2 of an output of K = 256 terms)."""
+    import crane_b200
+    from oracle import ggml_quant as gq
+    cfg = dict(synth.TINY_QWEN3_UNTIED, num_hidden_layers=1)
+    m = crane_b200.Qwen3Model(cfg, max_seq_len=64, max_batch=16)
+    for name, shape, kind in synth.tensor_specs(cfg):
+        t = synth.make_tensor(name, shape, kind)
+        if "proj" in name or name == "lm_head.weight":
+            m.load_tensor_ggml(name, gq.GGML_TYPE_ID[recipe], t.shape, gq.quantize(t, recipe))
+        else:
+            m.load_tensor(name, t)
+    m.finalize()
+    slots = [0] + [m.seq_create() for _ in range(8)]
+    for s in slots:
+        m.seq_select(s)
+        m.forward_step(synth.synth_token_ids(4 + s, cfg["vocab_size"], f"q{s}"), 0)
+    tok = synth.synth_token_ids(9, cfg["vocab_size"], "qt")
+
+    def back():
+        for s in slots:
+            m.seq_select(s)
+            m.set_kv_caches([], 4 + s)
+    back()
+    _, nine = m.decode_batch(slots, tok, 1, want_logits=True)
+    back()
+    four = np.concatenate([m.decode_batch(slots[i: i + 4], tok[i: i + 4], 1, want_logits=True)[1] for i in (0, 4, 8)])
+    err = np.abs(nine - four).max(1) / np.abs(four).max()
+    assert err.max() < 3e-2 and np.median(err) < 1e-2
+    m.close()
