@@ -494,14 +494,19 @@ int embed_decode_launch(cudaStream_t st, int B, const bf16* embed, int H, const 
 
 // =====================================================================================
 // Decode attention: QK-norm + (M)RoPE + KV-page append + split-KV GQA attention + in-cluster split merge
-//   grid (nkv * ATTN_NSPLIT, B), 256 threads, thread-block CLUSTER of ATTN_NSPLIT CTAs per KV head.
-//   * every CTA first pulls its token range of the K/V pages into shared memory with cp.async -- BEFORE
-//     griddepcontrol.wait: cached K/V and the sequence state were written at least two kernels ago, so the whole
-//     KV read overlaps the QKV GEMV that precedes this kernel;
+//   grid (nkv * nsplit, B), 256 threads, thread-block CLUSTER of nsplit (1 .. 8) CTAs per KV head and sequence.
+//   * the K/V rows are requested BEFORE griddepcontrol.wait: cached K/V and the sequence state were written at least two kernels ago,
+//     so (the first part of) the KV read overlaps the QKV linear that precedes this kernel;
+//   * RING (bf16 pages): every lane streams its own 16-byte pieces through a private ring of ATTN_DEPTH places -- it copies what it
+//     reads itself, so nothing but its own copies is waited for -- and 96 KB per CTA keep two CTAs on an SM.  (Tiles of 128 KB shared by the CTA,
+//     one CTA per SM, load and compute in turn: 171 us for 32 sequences of 135 .. 900 tokens, 8 KV heads; the bytes take 23.)
+//     Quantised pages are dequantised into shared tiles instead;
 //   * all NREP query heads of the KV group share every K/V byte (read once per group, 16-byte vectors);
 //   * the split partials are merged through distributed shared memory (no global round trip, no atomics).
 // =====================================================================================
-template <int D, int NREP>
+constexpr int ATTN_DEPTH = 6;
+
+template <int D, int NREP, bool RING>
 __global__ void __launch_bounds__(256)
 attn_decode_kernel(AttnDecArgs a) {
     namespace cg = cooperative_groups;
@@ -529,7 +534,7 @@ attn_decode_kernel(AttnDecArgs a) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // a KV head whose query group is wider than NREP is served by `groups` CTA clusters of NREP query heads each (6 = 2 x 3,
     // 8 = 2 x 4, ...): kvv numbers those sub-groups, query head = kvv * NREP + h; only sub-group 0 appends the new K/V row
-    const int kvv = blockIdx.x / ATTN_NSPLIT, split = blockIdx.x % ATTN_NSPLIT;
+    const int ns = a.nsplit, kvv = blockIdx.x / ns, split = blockIdx.x % ns;
     const int kvh = kvv / a.groups, sub = kvv % a.groups;
     const int b = blockIdx.y;
     const int q_dim = a.nh * D, kv_dim = a.nkv * D;
@@ -538,7 +543,7 @@ attn_decode_kernel(AttnDecArgs a) {
     // ---- token range of this split, then start the K/V copy (independent of the previous kernel) ----
     const SeqState st = a.state[b];
     const int T = st.kv_len + 1;                      // including the token being decoded
-    int chunk = (T + ATTN_NSPLIT - 1) / ATTN_NSPLIT;
+    int chunk = (T + ns - 1) / ns;
     chunk = (chunk + 7) & ~7;
     const int t0 = split * chunk;
     const int t1 = min(T, t0 + chunk);
@@ -597,7 +602,31 @@ attn_decode_kernel(AttnDecArgs a) {
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    if (t0 < t_end) load_tile(t0);
+    // RING: token groups r0 = t0 + warp * TPW + i * NW * TPW of this warp; a lane's place holds its pieces of K hi, V hi, K lo, V lo, 512 bytes apart
+    const int grp = lane / LPT, gl = lane % LPT;        // token group inside the warp, lane inside the group
+    const int w0 = t0 + warp * TPW, n_it = max(0, (t_end - w0 + NW * TPW - 1) / (NW * TPW));
+    unsigned char* ring = asm_ + (size_t)warp * ATTN_DEPTH * 2048 + lane * 16;
+    const uint32_t ring_u32 = smem_u32(ring);
+    auto ring_issue = [&](int i) {
+        const int t = w0 + i * NW * TPW + grp;
+        if (i < n_it && t < t_end) {
+            const size_t off = (((size_t)bt[t / KV_PAGE] * a.nkv + kvh) * KV_PAGE + (t % KV_PAGE)) * D + gl * EPL;
+            const uint32_t dst = ring_u32 + (uint32_t)(i % ATTN_DEPTH) * 2048;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(a.k_pool + off) : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 512), "l"(a.v_pool + off) : "memory");
+            if (split_kv) {
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 1024), "l"(a.k_pool + a.kv_lo_off + off) : "memory");
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 1536), "l"(a.v_pool + a.kv_lo_off + off) : "memory");
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if constexpr (RING) {
+#pragma unroll
+        for (int i = 0; i < ATTN_DEPTH; ++i) ring_issue(i);
+    } else {
+        if (t0 < t_end) load_tile(t0);
+    }
 
     // norm weights and this position's cos/sin depend only on immutable data and the sequence state: fetch them before
     // the dependency wait too (lane l owns elements l + 32 j, so a rotary pair is lane-local)
@@ -696,7 +725,6 @@ attn_decode_kernel(AttnDecArgs a) {
     }
 
     // ---- the cached tokens of this split, tile by tile out of shared memory ----
-    const int grp = lane / LPT, gl = lane % LPT;        // token group inside the warp, lane inside the group
     float qr[NREP][EPL];
 #pragma unroll
     for (int h = 0; h < NREP; ++h)
@@ -709,49 +737,61 @@ attn_decode_kernel(AttnDecArgs a) {
 #pragma unroll
         for (int j = 0; j < EPL; ++j) o[h][j] = 0.f;
     }
-    for (int tb = t0; tb < t_end; tb += TILE) {
-        if (tb != t0) { __syncthreads(); load_tile(tb); }
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();
-        const int n = min(TILE, t_end - tb);
-        for (int r0 = warp * TPW; r0 < n; r0 += NW * TPW) {
-            const int r = r0 + grp;
-            const bool valid = r < n;
-            float kf[EPL], vf[EPL];
-            if (valid) {
-                const uint4 kr = *reinterpret_cast<const uint4*>(k_t + r * D + gl * EPL);
-                const uint4 vr = *reinterpret_cast<const uint4*>(v_t + r * D + gl * EPL);
-                kf[0] = bf16lo(kr.x); kf[1] = bf16hi(kr.x); kf[2] = bf16lo(kr.y); kf[3] = bf16hi(kr.y);
-                kf[4] = bf16lo(kr.z); kf[5] = bf16hi(kr.z); kf[6] = bf16lo(kr.w); kf[7] = bf16hi(kr.w);
-                vf[0] = bf16lo(vr.x); vf[1] = bf16hi(vr.x); vf[2] = bf16lo(vr.y); vf[3] = bf16hi(vr.y);
-                vf[4] = bf16lo(vr.z); vf[5] = bf16hi(vr.z); vf[6] = bf16lo(vr.w); vf[7] = bf16hi(vr.w);
-                if (split_kv) {
-                    const uint4 kl = *reinterpret_cast<const uint4*>(kl_t + r * D + gl * EPL);
-                    const uint4 vl = *reinterpret_cast<const uint4*>(vl_t + r * D + gl * EPL);
-                    kf[0] += bf16lo(kl.x); kf[1] += bf16hi(kl.x); kf[2] += bf16lo(kl.y); kf[3] += bf16hi(kl.y);
-                    kf[4] += bf16lo(kl.z); kf[5] += bf16hi(kl.z); kf[6] += bf16lo(kl.w); kf[7] += bf16hi(kl.w);
-                    vf[0] += bf16lo(vl.x); vf[1] += bf16hi(vl.x); vf[2] += bf16lo(vl.y); vf[3] += bf16hi(vl.y);
-                    vf[4] += bf16lo(vl.z); vf[5] += bf16hi(vl.z); vf[6] += bf16lo(vl.w); vf[7] += bf16hi(vl.w);
-                }
-            } else {
-#pragma unroll
-                for (int j = 0; j < EPL; ++j) { kf[j] = 0.f; vf[j] = 0.f; }
+    auto attend = [&](bool valid, const void* kp, const void* vp, const void* klp, const void* vlp) {
+        float kf[EPL], vf[EPL];
+        if (valid) {
+            const uint4 kr = *reinterpret_cast<const uint4*>(kp);
+            const uint4 vr = *reinterpret_cast<const uint4*>(vp);
+            kf[0] = bf16lo(kr.x); kf[1] = bf16hi(kr.x); kf[2] = bf16lo(kr.y); kf[3] = bf16hi(kr.y);
+            kf[4] = bf16lo(kr.z); kf[5] = bf16hi(kr.z); kf[6] = bf16lo(kr.w); kf[7] = bf16hi(kr.w);
+            vf[0] = bf16lo(vr.x); vf[1] = bf16hi(vr.x); vf[2] = bf16lo(vr.y); vf[3] = bf16hi(vr.y);
+            vf[4] = bf16lo(vr.z); vf[5] = bf16hi(vr.z); vf[6] = bf16lo(vr.w); vf[7] = bf16hi(vr.w);
+            if (split_kv) {
+                const uint4 kl = *reinterpret_cast<const uint4*>(klp);
+                const uint4 vl = *reinterpret_cast<const uint4*>(vlp);
+                kf[0] += bf16lo(kl.x); kf[1] += bf16hi(kl.x); kf[2] += bf16lo(kl.y); kf[3] += bf16hi(kl.y);
+                kf[4] += bf16lo(kl.z); kf[5] += bf16hi(kl.z); kf[6] += bf16lo(kl.w); kf[7] += bf16hi(kl.w);
+                vf[0] += bf16lo(vl.x); vf[1] += bf16hi(vl.x); vf[2] += bf16lo(vl.y); vf[3] += bf16hi(vl.y);
+                vf[4] += bf16lo(vl.z); vf[5] += bf16hi(vl.z); vf[6] += bf16lo(vl.w); vf[7] += bf16hi(vl.w);
             }
+        } else {
 #pragma unroll
-            for (int h = 0; h < NREP; ++h) {
-                float s = 0.f;
+            for (int j = 0; j < EPL; ++j) { kf[j] = 0.f; vf[j] = 0.f; }
+        }
 #pragma unroll
-                for (int j = 0; j < EPL; ++j) s = fmaf(qr[h][j], kf[j], s);
+        for (int h = 0; h < NREP; ++h) {
+            float s = 0.f;
 #pragma unroll
-                for (int ofs = LPT / 2; ofs > 0; ofs >>= 1) s += __shfl_xor_sync(0xffffffffu, s, ofs);
-                if (valid) {
-                    const float mn = fmaxf(m[h], s);
-                    const float corr = __expf(m[h] - mn), p = __expf(s - mn);
-                    l[h] = l[h] * corr + p;
+            for (int j = 0; j < EPL; ++j) s = fmaf(qr[h][j], kf[j], s);
 #pragma unroll
-                    for (int j = 0; j < EPL; ++j) o[h][j] = o[h][j] * corr + p * vf[j];
-                    m[h] = mn;
-                }
+            for (int ofs = LPT / 2; ofs > 0; ofs >>= 1) s += __shfl_xor_sync(0xffffffffu, s, ofs);
+            if (valid) {
+                const float mn = fmaxf(m[h], s);
+                const float corr = __expf(m[h] - mn), p = __expf(s - mn);
+                l[h] = l[h] * corr + p;
+#pragma unroll
+                for (int j = 0; j < EPL; ++j) o[h][j] = o[h][j] * corr + p * vf[j];
+                m[h] = mn;
+            }
+        }
+    };
+    if constexpr (RING) {
+        for (int i = 0; i < n_it; ++i) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(ATTN_DEPTH - 1) : "memory");
+            const unsigned char* p = ring + (i % ATTN_DEPTH) * 2048;
+            attend(w0 + i * NW * TPW + grp < t_end, p, p + 512, p + 1024, p + 1536);
+            ring_issue(i + ATTN_DEPTH);
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+    } else {
+        for (int tb = t0; tb < t_end; tb += TILE) {
+            if (tb != t0) { __syncthreads(); load_tile(tb); }
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncthreads();
+            const int n = min(TILE, t_end - tb);
+            for (int r0 = warp * TPW; r0 < n; r0 += NW * TPW) {
+                const int o_ = (r0 + grp) * D + gl * EPL;
+                attend(r0 + grp < n, k_t + o_, v_t + o_, kl_t + o_, vl_t + o_);
             }
         }
     }
@@ -818,12 +858,13 @@ attn_decode_kernel(AttnDecArgs a) {
     }
     // ---- merge the splits of this KV group through distributed shared memory ----
     cluster.sync();
-    for (int idx = split * 256 + tid; idx < NREP * D; idx += ATTN_NSPLIT * 256) {
+    for (int idx = split * 256 + tid; idx < NREP * D; idx += ns * 256) {
         const int h = idx / D, i = idx % D;
         float ms[ATTN_NSPLIT];
         float M = -INFINITY;
 #pragma unroll
         for (int s = 0; s < ATTN_NSPLIT; ++s) {
+            if (s >= ns) break;
             const float* rml = cluster.map_shared_rank(&cta_ml[0][0], s);
             ms[s] = rml[h * 2];
             M = fmaxf(M, ms[s]);
@@ -831,6 +872,7 @@ attn_decode_kernel(AttnDecArgs a) {
         float L = 0.f, O = 0.f;
 #pragma unroll
         for (int s = 0; s < ATTN_NSPLIT; ++s) {
+            if (s >= ns) break;
             const float c = (ms[s] == -INFINITY) ? 0.f : __expf(ms[s] - M);
             const float* rml = cluster.map_shared_rank(&cta_ml[0][0], s);
             const float* ro = cluster.map_shared_rank(&cta_o[0][0], s);
@@ -845,24 +887,30 @@ attn_decode_kernel(AttnDecArgs a) {
     cluster.sync();                                      // nobody exits while its shared memory is still being read
 }
 
-template <int D, int NREP>
+template <int D, int NREP, bool RING>
 static int attn_decode_launch_t(cudaStream_t st, int B, const AttnDecArgs& a, bool pdl) {
-    const int SMEM = (a.kv_bits ? a.kv_split : (a.kv_lo_off != 0)) ? 131072 : 65536;
+    const int SMEM = RING ? 8 * ATTN_DEPTH * 2048 : (a.kv_bits ? a.kv_split : (a.kv_lo_off != 0)) ? 131072 : 65536;
     static SmemOptIn seen;
-    if (const int e = ensure_dyn_smem(attn_decode_kernel<D, NREP>, (size_t)SMEM, seen)) return e;
+    if (const int e = ensure_dyn_smem(attn_decode_kernel<D, NREP, RING>, (size_t)SMEM, seen)) return e;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(a.nkv * a.groups * ATTN_NSPLIT, B);
+    cfg.gridDim = dim3(a.nkv * a.groups * a.nsplit, B);
     cfg.blockDim = dim3(256);
     cfg.dynamicSmemBytes = SMEM;
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = ATTN_NSPLIT; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[0].val.clusterDim.x = a.nsplit; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 2 : 1;
-    return (int)cudaLaunchKernelEx(&cfg, attn_decode_kernel<D, NREP>, a);
+    return (int)cudaLaunchKernelEx(&cfg, attn_decode_kernel<D, NREP, RING>, a);
+}
+template <int D, int NREP>
+static int attn_decode_launch_r(cudaStream_t st, int B, const AttnDecArgs& a, bool pdl) {
+    // (a few sequences: the whole range of a CTA fits its tile, requested ahead of the dependency wait -- 20 us for one sequence of 1000 tokens,
+    // D = 256, where the rings take 26)
+    return a.kv_bits || B <= 4 ? attn_decode_launch_t<D, NREP, false>(st, B, a, pdl) : attn_decode_launch_t<D, NREP, true>(st, B, a, pdl);
 }
 
 int attn_decode_launch(cudaStream_t st, int B, int D, const AttnDecArgs& a_in, bool pdl) {
@@ -873,19 +921,23 @@ int attn_decode_launch(cudaStream_t st, int B, int D, const AttnDecArgs& a_in, b
     // any group width: the widest instantiated sub-group (4, 3, 2, 1 query heads) that divides it
     const int sub = nrep % 4 == 0 ? 4 : nrep % 3 == 0 ? 3 : nrep % 2 == 0 ? 2 : 1;
     a.groups = nrep / sub;
+    // splits per (sequence, KV group): all eight while they leave SMs idle, fewer as the batch itself fills the chip (two CTAs per SM)
+    const int pairs = B * a.nkv * a.groups;
+    a.nsplit = pairs <= 37 ? 8 : pairs <= 148 ? 4 : pairs <= 512 ? 2 : 1;
+    if (B <= 4) a.nsplit = ATTN_NSPLIT;
     if (D == 128) {
         switch (sub) {
-            case 1: return attn_decode_launch_t<128, 1>(st, B, a, pdl);
-            case 2: return attn_decode_launch_t<128, 2>(st, B, a, pdl);
-            case 3: return attn_decode_launch_t<128, 3>(st, B, a, pdl);
-            case 4: return attn_decode_launch_t<128, 4>(st, B, a, pdl);
+            case 1: return attn_decode_launch_r<128, 1>(st, B, a, pdl);
+            case 2: return attn_decode_launch_r<128, 2>(st, B, a, pdl);
+            case 3: return attn_decode_launch_r<128, 3>(st, B, a, pdl);
+            case 4: return attn_decode_launch_r<128, 4>(st, B, a, pdl);
         }
     } else if (D == 256) {
         switch (sub) {
-            case 1: return attn_decode_launch_t<256, 1>(st, B, a, pdl);
-            case 2: return attn_decode_launch_t<256, 2>(st, B, a, pdl);
-            case 3: return attn_decode_launch_t<256, 3>(st, B, a, pdl);
-            case 4: return attn_decode_launch_t<256, 4>(st, B, a, pdl);
+            case 1: return attn_decode_launch_r<256, 1>(st, B, a, pdl);
+            case 2: return attn_decode_launch_r<256, 2>(st, B, a, pdl);
+            case 3: return attn_decode_launch_r<256, 3>(st, B, a, pdl);
+            case 4: return attn_decode_launch_r<256, 4>(st, B, a, pdl);
         }
     }
     return -1000;

@@ -18,7 +18,7 @@
 namespace cb {
 
 constexpr int KV_PAGE = 64;        // tokens per KV page
-constexpr int ATTN_NSPLIT = 8;     // split-KV factor == thread-block cluster size (static grid: the step lives in a CUDA graph)
+constexpr int ATTN_NSPLIT = 8;     // largest split-KV factor == thread-block cluster size (static grid: the step lives in a CUDA graph)
 
 // Device-resident per-sequence decode state (lets a whole decode step replay as a CUDA graph).
 struct SeqState {
@@ -98,6 +98,7 @@ struct AttnDecArgs {
     int kv_split = 0;        // kv_bits != 0: stage the dequantised value as hi + lo bf16 planes (the parity mode) or hi only
     unsigned char *k_codes = nullptr, *v_codes = nullptr;
     float *k_scale = nullptr, *v_scale = nullptr;
+    int nsplit = 8;          // set by attn_decode_launch: CTAs per sequence and KV group (cluster size)
     int groups = 1;          // set by attn_decode_launch: CTA clusters per KV head (query group width / kernel sub-group width)
 };
 

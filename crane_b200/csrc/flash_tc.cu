@@ -1,0 +1,398 @@
+// Flash attention forward on tcgen05 (prefill and vision tower): 128 query rows x one head per CTA, 64-key tiles, scores and output in TMEM.
+//
+// What bounds it: in split precision (hi + lo bf16 planes, three products kept of each) the MMAs -- per 64 keys at D = 128 24 of 64 columns for the scores
+// and 12 of 128 for the output, 1.9 k cycles -- and, just below, the 64 KB of K / V planes a tile brings from L2 (64 KB per us and SM).  The
+// softmax of a tile, one row per thread, is 1 k cycles and runs under the MMAs of the next scores.  mma.sync (flash.cuh) takes 1.69 ms
+// for 4096 rows x 32 heads, D = 128, causal, split.
+//
+// One TMA producer, one MMA issuer, four softmax / epilogue warps (TMEM lane = query row = thread).  K and V stream through ONE ring of 16 KB slots in
+// the order the MMAs take them -- K of tile i + 1 ahead of V of tile i -- so a slot is refilled as soon as its dozen MMAs are done, whatever
+// the tile: K slots are [64 keys x 64 columns] per plane, V slots [R keys x all columns] per plane, read as an MN-major operand.
+// P goes from registers to TMEM as the A operand of P V.  The output is rescaled only when a row's maximum has grown by more than 2^8
+// since the last time (any reference works as long as sums and output share it).  Heads vary fastest and query tiles run from
+// the last (longest) to the first, so the tail of a causal launch is short work.
+#include "prefill.cuh"
+#include "tc.cuh"
+
+#include <algorithm>
+
+namespace cb {
+
+template <int D, bool SPLIT>
+struct FtcCfg {
+    static constexpr int P = SPLIT ? 2 : 1;
+    static constexpr int KC = (P == 1 && D >= 128) ? 2 : 1;         // 64-wide column tiles per K slot
+    static constexpr int SLOT = KC * P * 8192;
+    static constexpr int R = SLOT / (D * 2 * P) < 64 ? SLOT / (D * 2 * P) : 64;      // keys per V slot
+    static constexpr int NKS = D / 64 / KC, NVS = 64 / R;           // slots per 64-key tile
+    static constexpr int Q_BYTES = P * 128 * D * 2;
+    static constexpr int NSLOT = (208 * 1024 - Q_BYTES) / SLOT;
+    static constexpr int SMEM = Q_BYTES + NSLOT * SLOT + 1024;
+    static constexpr int C_S = D, C_P = D + 128;                    // TMEM columns: O [0, D), two score buffers of 64, P planes of 32
+    static_assert(NVS * R == 64 && R >= 16 && NSLOT >= 4 && C_P + 32 * P <= 512, "");
+};
+
+__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {     // A from TMEM
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                 ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* v) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
+        ::"r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
+          "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// MN-major operand, SWIZZLE_128B: 64 columns (128 B) x 8 keys per 1 KB atom; `lbo` bytes between 64-column groups, 1 KB between groups of 8 keys
+__device__ __forceinline__ uint64_t make_smem_desc_mn128(uint32_t smem_addr, uint32_t lbo) {
+    uint64_t d = 0;
+    d |= (uint64_t)((smem_addr & 0x3FFFFu) >> 4);
+    d |= (uint64_t)(lbo >> 4) << 16;
+    d |= (uint64_t)(1024 >> 4) << 32;
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)2 << 61;
+    return d;
+}
+
+struct FtcMaps { CUtensorMap k[2], v[2]; };
+
+template <int D, bool SPLIT, bool CAUSAL, bool PAGED>
+__global__ void __launch_bounds__(256, 1)
+flash_tc_kernel(const __grid_constant__ FtcMaps maps, FlashArgs a, int* err) {
+    using C = FtcCfg<D, SPLIT>;
+    constexpr int P = C::P;
+    const int head = blockIdx.x, z = blockIdx.z, q0 = (CAUSAL ? gridDim.y - 1 - blockIdx.y : blockIdx.y) * 128;
+    pdl_wait();                                       // (sequence bounds of a ragged batch come from the kernel ahead)
+    pdl_launch_dependents();
+    const int row0 = a.seq_start ? a.seq_start[z] : 0, S = a.seq_len ? a.seq_len[z] : a.S;
+    if (q0 >= S) return;
+    const int kv_off = CAUSAL ? (a.seq_kv_offset ? a.seq_kv_offset[z] : a.kv_offset) : 0;
+    const int T = CAUSAL ? kv_off + S : S, kvh = head / (a.nh / a.nkv);
+    const int* btab = (PAGED && a.seq_slot) ? a.block_table + (size_t)a.seq_slot[z] * a.bt_stride : a.block_table;
+    const int n_tiles = CAUSAL ? (kv_off + min(q0 + 127, S - 1)) / 64 + 1 : (T + 63) / 64;
+    // sliding window: the first query row of the tile reaches furthest back; the tiles of the kept first keys that the window does not reach come first
+    const int t_first = (CAUSAL && a.window > 0) ? max(0, kv_off + q0 - a.window + 1) / 64 : 0;
+    const int keep = (CAUSAL && a.window > 0) ? a.keep_first : 0, n_keep = min((keep + 63) / 64, t_first), n_walk = n_keep + n_tiles - t_first;
+    auto tile_at = [&](int i) { return i < n_keep ? i : t_first + i - n_keep; };
+
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t* ring = sm + C::Q_BYTES;
+    __shared__ uint64_t full[C::NSLOT], empty[C::NSLOT], q_full, s_full[2], s_empty[2], p_full, pv_done;
+    __shared__ uint32_t tmem_slot;
+    __shared__ int gave_up;
+    const TcWait wait{&gave_up, err};
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        gave_up = 0;
+        for (int i = 0; i < C::NSLOT; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
+        mbar_init(&q_full, 128); mbar_init(&p_full, 128); mbar_init(&pv_done, 1);
+        for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&s_empty[i], 128); }
+        fence_barrier_init();
+    }
+    if (warp == 2) { tmem_alloc(&tmem_slot, 512); tmem_relinquish(); }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            int st = 0; uint32_t ph = 0;
+            auto next = [&]() {
+                wait(&empty[st], ph ^ 1);
+                mbar_arrive_expect_tx(&full[st], C::SLOT);
+            };
+            auto step = [&]() { if (++st == C::NSLOT) { st = 0; ph ^= 1; } };
+            auto origin = [&](int tile) { return PAGED ? (btab[tile] * a.nkv + kvh) * 64 : row0 + tile * 64; };       // first row of the tile
+            const int x0 = PAGED ? 0 : kvh * D;
+            auto load_k = [&](int y) {
+                for (int s = 0; s < C::NKS; ++s) {
+                    next();
+#pragma unroll
+                    for (int kc = 0; kc < C::KC; ++kc)
+#pragma unroll
+                        for (int p = 0; p < P; ++p)
+                            tma_load_2d(ring + st * C::SLOT + (kc * P + p) * 8192, &maps.k[p], &full[st], x0 + (s * C::KC + kc) * 64, y);
+                    step();
+                }
+            };
+            auto load_v = [&](int y) {
+                for (int s = 0; s < C::NVS; ++s) {
+                    next();
+#pragma unroll
+                    for (int p = 0; p < P; ++p)
+#pragma unroll
+                        for (int c = 0; c < D / 64; ++c)
+                            tma_load_2d(ring + st * C::SLOT + (p * (D / 64) + c) * (C::R * 128), &maps.v[p], &full[st], x0 + c * 64, y + s * C::R);
+                    step();
+                }
+            };
+            int y = origin(tile_at(0));
+            load_k(y);
+            for (int i = 0; i < n_walk; ++i) {
+                int yn = 0;
+                if (i + 1 < n_walk) { yn = origin(tile_at(i + 1)); load_k(yn); }
+                load_v(y);
+                y = yn;
+            }
+            wait.drain();
+        }
+    } else if (warp == 1) {
+        constexpr uint32_t id_s = make_idesc_bf16(128, 64), id_o = make_idesc_bf16(128, D) | (1u << 16);      // (B of P V: MN-major)
+        const uint64_t qd = make_smem_desc_sw128(smem_u32(sm));
+        int st = 0; uint32_t ph = 0;
+        wait(&q_full, 0);
+        auto scores = [&](int i) {
+            const uint32_t d = tmem + C::C_S + (uint32_t)(i & 1) * 64;
+            wait(&s_empty[i & 1], ((i >> 1) & 1) ^ 1);
+            tc_fence_after();
+            for (int s = 0; s < C::NKS; ++s) {
+                wait(&full[st], ph);
+                const uint64_t kd = make_smem_desc_sw128(smem_u32(ring + st * C::SLOT));
+                if (elect_one()) {
+#pragma unroll
+                    for (int kc = 0; kc < C::KC; ++kc)
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            const uint64_t qa = qd + (uint64_t)((s * C::KC + kc) * 1024 + 2 * k), kb = kd + (uint64_t)(kc * P * 512 + 2 * k);
+                            constexpr uint64_t QLO = (uint64_t)(128 * D * 2) >> 4;
+                            const uint32_t acc = (uint32_t)((s | kc | k) != 0);
+                            if constexpr (SPLIT) {                     // small terms first
+                                umma_bf16(d, qa + QLO, kb, id_s, acc);
+                                umma_bf16(d, qa, kb + 512, id_s, 1u);
+                                umma_bf16(d, qa, kb, id_s, 1u);
+                            } else umma_bf16(d, qa, kb, id_s, acc);
+                        }
+                    umma_commit(&empty[st]);
+                    if (s == C::NKS - 1) umma_commit(&s_full[i & 1]);
+                }
+                __syncwarp();
+                if (++st == C::NSLOT) { st = 0; ph ^= 1; }
+            }
+        };
+        scores(0);
+        for (int i = 0; i < n_walk; ++i) {
+            if (i + 1 < n_walk) scores(i + 1);
+            wait(&p_full, i & 1);
+            tc_fence_after();
+            for (int s = 0; s < C::NVS; ++s) {
+                wait(&full[st], ph);
+                const uint32_t va = smem_u32(ring + st * C::SLOT);
+                const uint64_t vd = make_smem_desc_mn128(va, C::R * 128), vl = make_smem_desc_mn128(va + (P - 1) * (C::SLOT / P), C::R * 128);
+                if (elect_one()) {
+#pragma unroll
+                    for (int k = 0; k < C::R / 16; ++k) {
+                        const uint32_t pa = tmem + C::C_P + (uint32_t)(s * (C::R / 2) + k * 8);
+                        const uint32_t acc = (uint32_t)((i | s | k) != 0);
+                        if constexpr (SPLIT) {
+                            umma_ts(tmem, pa + 32, vd + (uint64_t)(k * 128), id_o, acc);
+                            umma_ts(tmem, pa, vl + (uint64_t)(k * 128), id_o, 1u);
+                            umma_ts(tmem, pa, vd + (uint64_t)(k * 128), id_o, 1u);
+                        } else umma_ts(tmem, pa, vd + (uint64_t)(k * 128), id_o, acc);
+                    }
+                    umma_commit(&empty[st]);
+                    if (s == C::NVS - 1) umma_commit(&pv_done);
+                }
+                __syncwarp();
+                if (++st == C::NSLOT) { st = 0; ph ^= 1; }
+            }
+        }
+    } else if (warp >= 4) {
+        const int q = warp & 3, r = q * 32 + lane, qrow = q0 + r, qpos = kv_off + qrow;
+        const uint32_t lanes = (uint32_t)(q * 32) << 16;
+        // ---- the Q tile: swizzled [128 rows x 64 columns] tiles per plane, rows past S zero; a warp copies whole rows ----
+        for (int rr = q * 32; rr < q * 32 + 32; ++rr) {
+            const bool in = q0 + rr < S;
+            const bf16* src = a.q + (size_t)(row0 + min(q0 + rr, S - 1)) * a.q_stride + head * D;
+#pragma unroll
+            for (int e = lane; e < P * (D / 8); e += 32) {
+                const int p = e / (D / 8), ch = e % (D / 8);
+                const uint4 v = in ? *reinterpret_cast<const uint4*>(src + (p ? a.q_lo_off : 0) + ch * 8) : make_uint4(0, 0, 0, 0);
+                *reinterpret_cast<uint4*>(sm + p * (128 * D * 2) + (ch >> 3) * 16384 + sw128_off(rr, ch & 7)) = v;
+            }
+        }
+        fence_proxy_async();
+        mbar_arrive(&q_full);
+
+        const float sl2 = a.scale * 1.4426950408889634f;
+        const bool mods = CAUSAL && (a.softcap > 0.f || a.dist_r1 || a.dist_table);
+        const float inv_cap = a.softcap > 0.f ? 1.f / a.softcap : 0.f;
+        const float dr1 = (CAUSAL && a.dist_r1) ? a.dist_r1[head] : 0.f, dr2 = (CAUSAL && a.dist_r1) ? a.dist_r2[head] : 0.f;
+        const float* dtab = (CAUSAL && a.dist_table) ? a.dist_table + (size_t)head * a.dist_rows : nullptr;
+        float m = -INFINITY, l = 0.f;                 // reference of the exponentials (not always the running maximum), sum
+        for (int i = 0; i < n_walk; ++i) {
+            const int kv0 = tile_at(i) * 64;
+            wait(&s_full[i & 1], (i >> 1) & 1);
+            tc_fence_after();
+            uint32_t u[64];
+            const uint32_t sa = tmem + lanes + C::C_S + (uint32_t)(i & 1) * 64;
+#pragma unroll
+            for (int c = 0; c < 64; c += 16) tmem_ld16_async(sa + c, u + c);
+            tmem_ld_wait();
+            tc_fence_before();
+            mbar_arrive(&s_empty[i & 1]);
+            float* s = reinterpret_cast<float*>(u);
+            // every key of the tile visible to every row of this warp?  (the warp's first row sees the fewest new keys, its last the fewest old ones)
+            const bool whole = kv0 + 64 <= T && (!CAUSAL || (kv0 + 63 <= kv_off + q0 + q * 32 && (a.window <= 0 || kv_off + q0 + q * 32 + 31 - kv0 < a.window)));
+            float mx = -INFINITY;
+            if (whole && !mods) {
+#pragma unroll
+                for (int c = 0; c < 64; ++c) { s[c] *= sl2; mx = fmaxf(mx, s[c]); }
+            } else {
+#pragma unroll
+                for (int c = 0; c < 64; ++c) {
+                    const int col = kv0 + c, dist = qpos - col;
+                    const bool vis = col < T && (!CAUSAL || (dist >= 0 && (a.window <= 0 || dist < a.window || col < keep)));
+                    float v = s[c] * sl2;
+                    if (mods && vis) {          // cap, then the distance terms, in f32 on the scaled score
+                        float sc = s[c] * a.scale;
+                        if (a.softcap > 0.f) {            // tanh(x) = 1 - 2 / (e^{2x} + 1)
+                            const float t = __expf(fminf(2.f * sc * inv_cap, 40.f));
+                            sc = a.softcap * (1.f - __fdividef(2.f, t + 1.f));
+                        }
+                        if (a.dist_r1) sc -= dr1 * log1pf(dr2 * (float)dist);
+                        if (dtab) sc += dtab[min(dist, a.dist_rows - 1)];
+                        v = sc * 1.4426950408889634f;
+                    }
+                    s[c] = vis ? v : -INFINITY;
+                    mx = fmaxf(mx, s[c]);
+                }
+            }
+            if (i > 0) { wait(&pv_done, (i - 1) & 1); tc_fence_after(); }      // O is whole and the P columns are free
+            const bool grow = mx > m + 8.f || (m == -INFINITY && mx > -INFINITY);
+            if (__any_sync(0xffffffffu, grow)) {
+                const float mn = fmaxf(m, mx), f = m == -INFINITY ? 0.f : exp2f(m - mn);
+                l *= f;
+                m = mn;
+                if (i > 0) {
+#pragma unroll 1
+                    for (int c = 0; c < D; c += 16) {
+                        uint32_t o[16];
+                        tmem_ld16_async(tmem + lanes + c, o);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * f);
+                        tmem_st16(tmem + lanes + c, o);
+                    }
+                }
+            }
+            const float ref = m == -INFINITY ? 0.f : m;
+            float sum = 0.f;
+#pragma unroll
+            for (int c = 0; c < 64; c += 32) {
+                uint32_t hi[16], lo[16];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    const float p0 = exp2f(s[c + 2 * j] - ref), p1 = exp2f(s[c + 2 * j + 1] - ref);
+                    sum += p0 + p1;
+                    split_bf16x2(p0, p1, hi[j], lo[j]);
+                }
+                tmem_st16(tmem + lanes + C::C_P + c / 2, hi);
+                if (SPLIT) tmem_st16(tmem + lanes + C::C_P + 32 + c / 2, lo);
+            }
+            l += sum;
+            tmem_st_wait();
+            tc_fence_before();
+            if (PAGED && kv0 + 64 > T) {       // the rest of the last page was never written: zero times whatever is there must stay zero
+                const int seq = n_walk * C::NKS + (n_walk - 1) * C::NVS;
+                for (int j = 0; j < C::NVS; ++j) {
+                    const int slot = (seq + j) % C::NSLOT, lo_r = max(0, T - kv0 - j * C::R);
+                    if (lo_r >= C::R) continue;
+                    wait(&full[slot], ((seq + j) / C::NSLOT) & 1);
+                    const int per = (C::R - lo_r) * 8;          // 16-byte pieces per tile
+                    for (int e = threadIdx.x - 128; e < P * (D / 64) * per; e += 128)
+                        *reinterpret_cast<uint4*>(ring + slot * C::SLOT + (e / per) * (C::R * 128) + lo_r * 128 + (e % per) * 16) = make_uint4(0, 0, 0, 0);
+                }
+                fence_proxy_async();
+            }
+            mbar_arrive(&p_full);
+        }
+        wait(&pv_done, (n_walk - 1) & 1);
+        tc_fence_after();
+        // ---- normalise and store ----
+        float inv = 1.f / l;
+        if (a.sink) {        // the sink joins the denominator only: rescale to the larger of the reference and the sink
+            const float s2 = a.sink[head] * 1.4426950408889634f, mn = fmaxf(m, s2), c = exp2f(m - mn);
+            inv = c / (l * c + exp2f(s2 - mn));
+        }
+        inv *= a.out_mult;
+        const bool in = qrow < S;
+        const size_t orow = (size_t)(row0 + qrow);
+        if (in && a.gate && a.gate_heads) inv *= 1.f / (1.f + __expf(-a.gate[orow * a.g_stride + head]));
+        bf16* o = a.out + orow * a.o_stride + head * D;
+        const float* gt = (a.gate && !a.gate_heads) ? a.gate + orow * a.g_stride + head * D : nullptr;
+#pragma unroll 1
+        for (int c = 0; c < D; c += 16) {
+            uint32_t w[16];
+            tmem_ld16_async(tmem + lanes + c, w);
+            tmem_ld_wait();
+            if (in) {
+                uint32_t hi[8], lo[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    float o0 = __uint_as_float(w[2 * j]) * inv, o1 = __uint_as_float(w[2 * j + 1]) * inv;
+                    if (gt) {
+                        const float2 g = *reinterpret_cast<const float2*>(gt + c + 2 * j);
+                        o0 *= 1.f / (1.f + __expf(-g.x)); o1 *= 1.f / (1.f + __expf(-g.y));
+                    }
+                    split_bf16x2(o0, o1, hi[j], lo[j]);
+                }
+                *reinterpret_cast<uint4*>(o + c) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                *reinterpret_cast<uint4*>(o + c + 8) = make_uint4(hi[4], hi[5], hi[6], hi[7]);
+                if (SPLIT) {
+                    *reinterpret_cast<uint4*>(o + a.out_lo_off + c) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                    *reinterpret_cast<uint4*>(o + a.out_lo_off + c + 8) = make_uint4(lo[4], lo[5], lo[6], lo[7]);
+                }
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 2) { tc_fence_after(); tmem_dealloc(tmem, 512); }
+}
+
+template <int D, bool SPLIT, bool CAUSAL, bool PAGED>
+static int ftc_launch_t(cudaStream_t st, const FlashArgs& a) {
+    using C = FtcCfg<D, SPLIT>;
+    FtcMaps m;
+    // (a pool's rows are addressed through its pages, always inside it: the map's row count only has to reach that far)
+    const bf16 *k = PAGED ? a.k_pool : a.k, *v = PAGED ? a.v_pool : a.v;
+    const uint64_t rows = PAGED ? (uint64_t)1 << 28 : (uint64_t)a.kv_rows, cols = PAGED ? D : (uint64_t)a.nkv * D, ld = PAGED ? D : (uint64_t)a.kv_stride;
+    for (int p = 0; p < 2; ++p) {
+        const long long off = p && SPLIT ? a.kv_lo_off : 0;
+        if (!tc_tmap_16(&m.k[p], k + off, rows, cols, ld, 64, 64, CU_TENSOR_MAP_SWIZZLE_128B)) return -1001;
+        if (!tc_tmap_16(&m.v[p], v + off, rows, cols, ld, C::R, 64, CU_TENSOR_MAP_SWIZZLE_128B)) return -1001;
+    }
+    static SmemOptIn seen;
+    if (const int e = ensure_dyn_smem(flash_tc_kernel<D, SPLIT, CAUSAL, PAGED>, (size_t)C::SMEM, seen)) return e;
+    TcScratch s;
+    if (const int e = tc_scratch_get(st, TC_WS_FLOATS, 4096, &s)) return e;
+    const int max_len = a.seq_len ? a.max_len : a.S;
+    return launch_k(flash_tc_kernel<D, SPLIT, CAUSAL, PAGED>, dim3(a.nh, (max_len + 127) / 128, a.seq_len ? a.nseq : 1), dim3(256), C::SMEM, st, prefill_pdl(), m, a, s.err);
+}
+
+bool flash_tc_fits(int D, bool causal, bool paged, const FlashArgs& a) {
+    if (causal != paged || (!paged && a.kv_rows <= 0) || (D != 64 && D != 128 && !(D == 256 && causal))) return false;
+    const long long al = (long long)a.q_stride | a.o_stride | (paged ? 0 : a.kv_stride) | a.q_lo_off | a.kv_lo_off | a.out_lo_off;
+    const uintptr_t ptr = (uintptr_t)a.q | (uintptr_t)a.out | (uintptr_t)(paged ? a.k_pool : a.k) | (uintptr_t)(paged ? a.v_pool : a.v);
+    return (al & 7) == 0 && (ptr & 15) == 0 && (!a.gate || a.gate_heads || (a.g_stride & 1) == 0);
+}
+int flash_tc_launch(cudaStream_t st, int D, bool causal, const FlashArgs& a) {
+    const bool split = a.q_lo_off != 0;
+    if (causal) {
+        switch (D) {
+            case 64:  return split ? ftc_launch_t<64, true, true, true>(st, a) : ftc_launch_t<64, false, true, true>(st, a);
+            case 128: return split ? ftc_launch_t<128, true, true, true>(st, a) : ftc_launch_t<128, false, true, true>(st, a);
+            case 256: return split ? ftc_launch_t<256, true, true, true>(st, a) : ftc_launch_t<256, false, true, true>(st, a);
+        }
+    } else {
+        switch (D) {
+            case 64:  return split ? ftc_launch_t<64, true, false, false>(st, a) : ftc_launch_t<64, false, false, false>(st, a);
+            case 128: return split ? ftc_launch_t<128, true, false, false>(st, a) : ftc_launch_t<128, false, false, false>(st, a);
+        }
+    }
+    return -1000;
+}
+
+}  // namespace cb

@@ -5,24 +5,32 @@
 // accumulator columns of its own, added when they are read.  Three planes carry all 24 bits of an f32 activation (a decode batch keeps the
 // accuracy of the f32 GEMV it replaces), two the split-precision operands of the prefill, one plain bf16.
 //
-// A stage is 128 weight rows x 128 columns and the planes beside it: eight MMAs per wait and commit, because a wait costs the issuing warp as much as
-// four MMAs of these widths (tc.cuh, elect_one; gemm_tc_kernel's 64-wide stages of four take 0.33 us each whatever their width: 20 us for
-// 2048 x 2048 at 77 rows on 32 CTAs).  Stream-K over (128-row tile, 128-wide step) puts the same number of steps on every SM; partial tiles
-// are added in contributor order by the last to arrive, so the result does not depend on who that was.
+// A stage is 128 weight rows x 64 CH columns and the planes beside it.  CH = 2, eight MMAs per wait and commit, while three such stages fit (a wait costs
+// the issuing warp as much as four MMAs of these widths: tc.cuh, elect_one); CH = 1 for wider activations, whose MMAs take longer anyway:
+// with two stages in flight instead of five, 12288 x 2048 at 77 rows in two planes took 43 us.  
+//
+// Fewer tiles than SMs (N < 19 000): a cluster of up to eight CTAs shares a tile along K and adds its partial tiles through distributed shared memory,
+// every CTA finishing its share of the columns.  More: stream-K over (tile, step), the same number of steps on every SM; partial tiles
+// go through global memory and the last contributor to arrive adds them, in contributor order either way.
 #include "gemm.cuh"
 #include "tc.cuh"
 
+#include <cooperative_groups.h>
+
 #include <algorithm>
+#include <mutex>
 
 namespace cb {
+namespace cg = cooperative_groups;
 
 constexpr int GR_MAX_CTAS = 160;
-constexpr int GR_W_BYTES = 128 * 256;             // weights of a stage: two 64-wide tiles
+constexpr int GR_TILE = 128 * 128;                // one 64-wide tile of the weights
 constexpr int GR_BUDGET = 208 * 1024;
 
 struct GemmRowsArgs {
     GemmEpi ep;
-    int M, Mp, N, KB, nstg;        // Mp: M rounded up to 16; KB: 128-wide steps
+    int M, Mp, N, KB, nstg;        // Mp: M rounded up to 16; KB: steps of 64 CH columns
+    int cl;                        // CTAs per tile (a cluster; 1: none), 0: stream-K
     TcSched sc;
     int* err;
 };
@@ -98,7 +106,7 @@ __device__ __forceinline__ void rows_epi16(const GemmEpi& ep, int M, int N, int 
 }
 
 //   warp 0: TMA producer    warp 1: MMA issuer    warp 2: TMEM allocator    warps 4 - 7: epilogue (TMEM lanes 32 (warp % 4) ..)
-template <int P, int MODE>
+template <int P, int MODE, int CH>
 __global__ void __launch_bounds__(256, 1)
 gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmA1,
                  const __grid_constant__ CUtensorMap tmA2, GemmRowsArgs a) {
@@ -109,8 +117,9 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     __shared__ int last_flag, gave_up;
     const TcWait wait{&gave_up, a.err};
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int Mp = a.Mp, KB = a.KB, nstg = a.nstg, cols = P * Mp, stg_bytes = GR_W_BYTES + cols * 256;
-    const int it_begin = sched_start(a.sc, blockIdx.x), it_end = sched_start(a.sc, blockIdx.x + 1);
+    const int Mp = a.Mp, KB = a.KB, nstg = a.nstg, cols = P * Mp, stg_bytes = CH * (GR_TILE + cols * 128);
+    const int rank = a.cl > 1 ? blockIdx.x % a.cl : 0, t0 = a.cl ? blockIdx.x / a.cl * KB : 0;
+    const int it_begin = a.cl ? t0 + rank * KB / a.cl : sched_start(a.sc, blockIdx.x), it_end = a.cl ? t0 + (rank + 1) * KB / a.cl : sched_start(a.sc, blockIdx.x + 1);
 
     if (threadIdx.x == 0) {
         gave_up = 0;
@@ -130,9 +139,9 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
             tma_prefetch_desc(&tmW); tma_prefetch_desc(&tmA0);
             auto weights = [&](int it, int st) {
                 mbar_arrive_expect_tx(&full[st], stg_bytes);
-                const int n0 = it / KB * 128, k0 = it % KB * 128;
-                tma_load_2d(sm + st * stg_bytes, &tmW, &full[st], k0, n0);
-                tma_load_2d(sm + st * stg_bytes + GR_W_BYTES / 2, &tmW, &full[st], k0 + 64, n0);
+                const int n0 = it / KB * 128, k0 = it % KB * (64 * CH);
+#pragma unroll
+                for (int c = 0; c < CH; ++c) tma_load_2d(sm + st * stg_bytes + c * GR_TILE, &tmW, &full[st], k0 + 64 * c, n0);
             };
             // weights do not depend on the predecessor kernel: the first stages' go out before the dependency wait
             const int npre = a.ep.w_dynamic ? 0 : min(it_end - it_begin, nstg);
@@ -141,10 +150,10 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
             int st = 0; uint32_t ph = 0;
             for (int it = it_begin; it < it_end; ++it) {
                 if (it - it_begin >= npre) { wait(&empty[st], ph ^ 1); weights(it, st); }
-                const int k0 = it % KB * 128;
-                uint8_t* b = sm + st * stg_bytes + GR_W_BYTES;
+                const int k0 = it % KB * (64 * CH);
+                uint8_t* b = sm + st * stg_bytes + CH * GR_TILE;
 #pragma unroll
-                for (int c = 0; c < 2; ++c) {
+                for (int c = 0; c < CH; ++c) {
                     tma_load_2d(b + c * cols * 128, &tmA0, &full[st], k0 + 64 * c, 0);
                     if (P > 1) tma_load_2d(b + c * cols * 128 + Mp * 128, &tmA1, &full[st], k0 + 64 * c, 0);
                     if (P > 2) tma_load_2d(b + c * cols * 128 + 2 * Mp * 128, &tmA2, &full[st], k0 + 64 * c, 0);
@@ -165,11 +174,11 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
                 wait(&full[st], ph);
                 tc_fence_after();
                 const uint32_t wa = smem_u32(sm + st * stg_bytes);
-                const uint64_t wd = make_smem_desc_sw128(wa), ad = make_smem_desc_sw128(wa + GR_W_BYTES);
+                const uint64_t wd = make_smem_desc_sw128(wa), ad = make_smem_desc_sw128(wa + CH * GR_TILE);
                 if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < 8; ++k)
-                        umma_bf16(d, wd + (uint64_t)((k >> 2) * (GR_W_BYTES / 32) + 2 * (k & 3)), ad + (uint64_t)((k >> 2) * cols * 8 + 2 * (k & 3)), idesc,
+                    for (int k = 0; k < 4 * CH; ++k)
+                        umma_bf16(d, wd + (uint64_t)((k >> 2) * (GR_TILE / 16) + 2 * (k & 3)), ad + (uint64_t)((k >> 2) * cols * 8 + 2 * (k & 3)), idesc,
                                   (uint32_t)((i != it) | (k != 0)));
                     umma_commit(&empty[st]);
                     if (i == seg_end - 1) umma_commit(&d_full[b]);
@@ -190,7 +199,8 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
             const uint32_t d = tmem + (uint32_t)(b * 256) + ((uint32_t)(q * 32) << 16);
             wait(&d_full[b], (seg >> 1) & 1);
             tc_fence_after();
-            float* mine = a.sc.ws + (size_t)(2 * blockIdx.x + (it == it_begin ? 0 : 1)) * tile_f + row;
+            // a cluster's partial tile stays in shared memory, in place of the operands (every MMA of this CTA has read its own)
+            float* mine = a.cl > 1 ? reinterpret_cast<float*>(sm) + row : a.sc.ws + (size_t)(2 * blockIdx.x + (it == it_begin ? 0 : 1)) * tile_f + row;
 #pragma unroll 1
             for (int c = 0; c < Mp; c += 16) {
                 uint32_t r0[16], r1[16], r2[16];
@@ -214,7 +224,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&d_empty[b]);
-            if (!sole) {                            // arrive at the tile; the last of its contributors adds them in order and finishes it
+            if (!sole && a.cl == 0) {               // arrive at the tile; the last of its contributors adds them in order and finishes it
                 __threadfence();
                 named_bar_sync(1, 128);
                 const int c_first = sched_owner(a.sc, t * KB), c_last = sched_owner(a.sc, t * KB + KB - 1);
@@ -252,35 +262,108 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
             it = seg_end;
         }
     }
+    if (a.cl > 1) {
+        cg::cluster_group cluster = cg::this_cluster();
+        cluster.sync();
+        if (warp >= 4) {
+            const int row = (warp & 3) * 32 + lane, n = it_begin / KB * 128 + row;
+#pragma unroll 1
+            for (int c = rank * 16; c < Mp; c += 16 * a.cl) {
+                float v[16];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) v[j] = 0.f;
+                for (int r = 0; r < a.cl; ++r) {
+                    const float* p = cluster.map_shared_rank(reinterpret_cast<float*>(sm), r) + (size_t)c * 128 + row;
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) v[j] += p[j * 128];
+                }
+                rows_epi16<MODE>(a.ep, a.M, a.N, c, n, v, lane);
+            }
+        }
+        cluster.sync();                              // nobody leaves while its shared memory is still being read
+    }
     tc_fence_before();
     __syncthreads();
     if (warp == 2) { tc_fence_after(); tmem_dealloc(tmem, 512); }
 }
 
-template <int P, int MODE>
-static int rows_launch_t(cudaStream_t st, const bf16* const* A, int lda, const bf16* W, int M, int N, int K, const GemmEpi& ep, bool pdl) {
+// clusters of `cl` CTAs, one CTA per SM, that the device runs at the same time
+static int rows_max_clusters(int cl) {
+    static std::mutex mu;
+    static int known[CB_MAX_DEV][9] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= CB_MAX_DEV) return 0;
+    std::lock_guard<std::mutex> g(mu);
+    if (!known[dev][cl]) {
+        const auto kernel = gemm_rows_kernel<1, EPI_STORE_F32, 2>;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(cl); cfg.blockDim = dim3(256); cfg.dynamicSmemBytes = GR_BUDGET;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = cl; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr; cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GR_BUDGET + 1024) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
+        known[dev][cl] = n + 1;
+    }
+    return known[dev][cl] - 1;
+}
+
+template <int P, int MODE, int CH>
+static int rows_launch_c(cudaStream_t st, const bf16* const* A, int lda, const bf16* W, int M, int N, int K, const GemmEpi& ep, bool pdl) {
     GemmRowsArgs a = {};
-    a.ep = ep; a.M = M; a.Mp = (M + 15) / 16 * 16; a.N = N; a.KB = (K + 127) / 128;
+    a.ep = ep; a.M = M; a.Mp = (M + 15) / 16 * 16; a.N = N; a.KB = (K + 64 * CH - 1) / (64 * CH);
     CUtensorMap tmW, tm[3];
     if (!tc_tmap_bf16(&tmW, W, (uint64_t)N, (uint64_t)K, (uint64_t)K, 128)) return -1001;
     for (int p = 0; p < 3; ++p)
         if (!tc_tmap_bf16(&tm[p], A[p < P ? p : 0], (uint64_t)M, (uint64_t)K, (uint64_t)lda, (uint32_t)a.Mp)) return -1001;
-    const int stg = GR_W_BYTES + P * a.Mp * 256;
-    a.nstg = std::min(6, GR_BUDGET / stg);
+    const int stg = CH * (GR_TILE + P * a.Mp * 128);
+    a.nstg = std::min(8, GR_BUDGET / stg);
     static SmemOptIn seen;
     const size_t smem = (size_t)a.nstg * stg + 1024;
-    if (const int e = ensure_dyn_smem(gemm_rows_kernel<P, MODE>, smem, seen)) return e;
+    if (const int e = ensure_dyn_smem(gemm_rows_kernel<P, MODE, CH>, smem, seen)) return e;
     TcSched& sc = a.sc;
     sc.tiles_m = 1; sc.tiles_n = (N + 127) / 128; sc.KB = a.KB;
     const long long iters = (long long)sc.tiles_n * a.KB;
     if (iters > 0x7fffffffLL) return -1000;
-    sc.unit = 1;
-    sc.G = (int)std::max<long long>(1, std::min<long long>(std::min(tc_device_sms(), GR_MAX_CTAS), iters / 3));     // three steps pay for a CTA's setup
-    sc.base = (int)(iters / sc.G); sc.rem = (int)(iters % sc.G);
+    const int sms = std::min(tc_device_sms(), GR_MAX_CTAS);
     TcScratch s;
     if (const int e = tc_scratch_get(st, TC_WS_FLOATS, sc.tiles_n, &s)) return e;
     sc.ws = s.ws; sc.counters = s.counters; a.err = s.err;
-    return launch_k(gemm_rows_kernel<P, MODE>, dim3(sc.G), dim3(256), smem, st, pdl, tmW, tm[0], tm[1], tm[2], a);
+    int grid;
+    if (sc.tiles_n <= sms) {
+        // as many CTAs per tile as the chip has room for at once (clusters live inside a GPC: sixteen of eight CTAs do not fit, and a second wave
+        // doubled 2048 x 6144 at 77 rows to 37 us), each with at least 256 columns of K
+        a.cl = std::max(1, std::min(std::min(8, sms / sc.tiles_n), a.KB * CH / 4));
+        while (a.cl > 1 && rows_max_clusters(a.cl) < sc.tiles_n) --a.cl;
+        grid = sc.tiles_n * a.cl;
+    } else {
+        sc.unit = 1; sc.G = sms;
+        sc.base = (int)(iters / sc.G); sc.rem = (int)(iters % sc.G);
+        grid = sc.G;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid); cfg.blockDim = dim3(256); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    int na = 0;
+    if (a.cl > 1) {
+        attr[na].id = cudaLaunchAttributeClusterDimension;
+        attr[na].val.clusterDim.x = a.cl; attr[na].val.clusterDim.y = 1; attr[na].val.clusterDim.z = 1;
+        ++na;
+    }
+    if (pdl) {
+        attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[na].val.programmaticStreamSerializationAllowed = 1;
+        ++na;
+    }
+    cfg.attrs = attr; cfg.numAttrs = na;
+    return (int)cudaLaunchKernelEx(&cfg, gemm_rows_kernel<P, MODE, CH>, tmW, tm[0], tm[1], tm[2], a);
+}
+
+template <int P, int MODE>
+static int rows_launch_t(cudaStream_t st, const bf16* const* A, int lda, const bf16* W, int M, int N, int K, const GemmEpi& ep, bool pdl) {
+    return P * ((M + 15) / 16 * 16) <= 96 ? rows_launch_c<P, MODE, 2>(st, A, lda, W, M, N, K, ep, pdl) : rows_launch_c<P, MODE, 1>(st, A, lda, W, M, N, K, ep, pdl);
 }
 
 template <int MODE>

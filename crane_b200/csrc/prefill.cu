@@ -209,6 +209,7 @@ int rope_append_launch(cudaStream_t st, int D, const RopeAppendArgs& a) {
 int flash_prefill_launch(cudaStream_t st, int D, bool causal, bool paged, const FlashArgs& a, int DV) {
     const bool split = a.q_lo_off != 0;
     if (split && (a.kv_lo_off == 0 || a.out_lo_off == 0)) return -1000;
+    if ((DV == 0 || DV == D) && flash_tc_fits(D, causal, paged, a)) return flash_tc_launch(st, D, causal, a);
     if (DV != 0 && DV != D) {
         if (!causal || !paged) return -1000;
         if (D == 64 && DV == 128) return split ? flash_launch_t<64, 128, true, true, true>(st, a) : flash_launch_t<64, 128, true, true, false>(st, a);

@@ -42,6 +42,7 @@ struct FlashArgs {
     const int* block_table;
     int nh, nkv;
     bf16* out;       int o_stride;      // out[(row) * o_stride + head * D + d]
+    int kv_rows = 0;                    // contiguous mode: rows of the buffer k and v point into (0: unknown, the tensor-memory-access kernel is not used)
     const int* seq_start;               // [nseq] first row of each sequence (nullptr: single sequence at row 0)
     const int* seq_len;                 // [nseq] query rows per sequence
     int S;                              // single-sequence mode: query rows
@@ -93,6 +94,9 @@ int layernorm_rows_launch(cudaStream_t st, const float* x, int rows, int W, cons
 int rope_append_launch(cudaStream_t st, int D, const RopeAppendArgs& a);
 // D: key width; DV: value width (0: equal).  Widths that differ: paged causal launches with (64, 128) or (128, 64); flash_widths_fit tells.
 int flash_prefill_launch(cudaStream_t st, int D, bool causal, bool paged, const FlashArgs& a, int DV = 0);
+// ... on tcgen05 (flash_tc.cu), where operands and widths allow it
+bool flash_tc_fits(int D, bool causal, bool paged, const FlashArgs& a);
+int flash_tc_launch(cudaStream_t st, int D, bool causal, const FlashArgs& a);
 inline bool flash_widths_fit(int D, int DV) { return (D == DV && (D == 64 || D == 128 || D == 256)) || (D == 64 && DV == 128) || (D == 128 && DV == 64); }
 // Ragged causal launches over paged caches with any widths (FlashArgs::k_w, v_w, dv): the tile is the next larger one the kernel is compiled for.
 int flash_ragged_launch(cudaStream_t st, const FlashArgs& a);

@@ -1,0 +1,65 @@
+"""Prefill attention on tcgen05 (csrc/flash_tc.cu) through one-layer models, at the edges of its tiles: 128 query rows, 64 keys, a last page that was never
+written to its end, cached prefixes; the oracle in f32."""
+import numpy as np
+import pytest
+
+from crane_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+# split precision keeps 16 bits of every operand (2^-17 each): 3e-5 of the largest logit over a layer, four-fold; plain bf16 2^-9: 2e-2
+@pytest.mark.parametrize("rows,past", [(2, 0), (63, 0), (64, 1), (65, 63), (127, 0), (128, 64), (129, 7), (300, 0), (37, 200), (513, 130)])
+@pytest.mark.parametrize("precision", ["split", "bf16"])
+def test_dense_prefill(rows, past, precision):
+    import crane_b200
+    from oracle.qwen3 import Qwen3Oracle
+    cfg = dict(synth.TINY_QWEN3_UNTIED, num_hidden_layers=1)
+    w = dict(synth.synth_checkpoint(cfg))
+    m = crane_b200.Qwen3Model(cfg, max_seq_len=704, precision=precision)
+    m.load_checkpoint(w.items())
+    orc = Qwen3Oracle(cfg, w)
+    ids = synth.synth_token_ids(past + rows, cfg["vocab_size"], f"ftc-{rows}-{past}")
+    if past:
+        orc.forward(ids[:past], 0)
+        m.forward_step(ids[:past], 0)
+    ref, got = orc.forward(ids[past:], past).numpy(), m.forward_step(ids[past:], past)
+    assert np.abs(got - ref).max() <= (1.2e-4 if precision == "split" else 2e-2) * np.abs(ref).max()
+    m.close()
+
+
+@pytest.mark.parametrize("rows,past", [(70, 0), (129, 90), (260, 0)])
+def test_hybrid_prefill(rows, past):
+    """D = 256, output gate applied behind it."""
+    import crane_b200
+    from oracle.qwen3_5 import Qwen3_5Oracle
+    cfg = synth.TINY_QWEN3_5
+    w = dict(synth.synth_checkpoint(cfg))
+    m = crane_b200.Qwen3_5Model(cfg, max_seq_len=512)
+    m.load_checkpoint(w.items())
+    orc = Qwen3_5Oracle(cfg, w)
+    ids = synth.synth_token_ids(past + rows, cfg["vocab_size"], f"ftch-{rows}")
+    if past:
+        orc.forward(ids[:past], 0)
+        m.forward_step(ids[:past], 0)
+    ref, got = orc.forward(ids[past:], past).numpy(), m.forward_step(ids[past:], past)
+    assert np.abs(got - ref).max() <= 1.2e-4 * np.abs(ref).max()
+    m.close()
+
+
+@pytest.mark.parametrize("grids", [[(1, 2, 2)], [(1, 8, 18)], [(1, 16, 16), (1, 4, 6), (2, 6, 10)]])
+def test_vision(grids):
+    """Strided keys, no mask, several images in one call."""
+    import crane_b200
+    from oracle.qwen3_vl import VisionOracle
+    cfg = synth.TINY_QWEN3_VL
+    w = dict(synth.synth_checkpoint(cfg))
+    m = crane_b200.Qwen3VLModel(cfg, max_seq_len=64)
+    m.load_checkpoint(w.items())
+    n = sum(t * h * x for t, h, x in grids)
+    pv = np.random.default_rng(n).uniform(-1, 1, (n, 1536)).astype(np.float32)
+    ref, deep = VisionOracle(cfg["vision_config"], w).forward(pv, grids)
+    got, ds = m.encode_images(pv, grids, want_deepstack=3)
+    for g, r in [(got, ref)] + list(zip(ds, deep)):
+        assert np.abs(g - r.numpy()).max() <= 1.2e-4 * np.abs(r.numpy()).max()
+    m.close()
