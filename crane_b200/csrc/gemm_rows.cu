@@ -18,7 +18,6 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
-#include <mutex>
 
 namespace cb {
 namespace cg = cooperative_groups;
@@ -287,29 +286,6 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     if (warp == 2) { tc_fence_after(); tmem_dealloc(tmem, 512); }
 }
 
-// clusters of `cl` CTAs, one CTA per SM, that the device runs at the same time
-static int rows_max_clusters(int cl) {
-    static std::mutex mu;
-    static int known[CB_MAX_DEV][9] = {};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= CB_MAX_DEV) return 0;
-    std::lock_guard<std::mutex> g(mu);
-    if (!known[dev][cl]) {
-        const auto kernel = gemm_rows_kernel<1, EPI_STORE_F32, 2>;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(cl); cfg.blockDim = dim3(256); cfg.dynamicSmemBytes = GR_BUDGET;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = cl; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr; cfg.numAttrs = 1;
-        int n = 0;
-        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GR_BUDGET + 1024) != cudaSuccess ||
-            cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
-        known[dev][cl] = n + 1;
-    }
-    return known[dev][cl] - 1;
-}
-
 template <int P, int MODE, int CH>
 static int rows_launch_c(cudaStream_t st, const bf16* const* A, int lda, const bf16* W, int M, int N, int K, const GemmEpi& ep, bool pdl) {
     GemmRowsArgs a = {};
@@ -336,7 +312,7 @@ static int rows_launch_c(cudaStream_t st, const bf16* const* A, int lda, const b
         // as many CTAs per tile as the chip has room for at once (clusters live inside a GPC: sixteen of eight CTAs do not fit, and a second wave
         // doubled 2048 x 6144 at 77 rows to 37 us), each with at least 256 columns of K
         a.cl = std::max(1, std::min(std::min(8, sms / sc.tiles_n), a.KB * CH / 4));
-        while (a.cl > 1 && rows_max_clusters(a.cl) < sc.tiles_n) --a.cl;
+        while (a.cl > 1 && tc_max_clusters(a.cl) < sc.tiles_n) --a.cl;
         grid = sc.tiles_n * a.cl;
     } else {
         sc.unit = 1; sc.G = sms;

@@ -36,12 +36,12 @@ template <int QT, int NT>
 struct QCfg {
     static constexpr int SB = QT == QT_Q4_K ? 144 : QT == QT_Q6_K ? 224 : 272;
     static constexpr int PLANES = QT == QT_Q6_K ? 2 : 1;
-    static constexpr int CH64 = QT == QT_Q6_K || (QT == QT_Q8_0 && NT > 64) ? 1 : 2;      // 64-wide tiles of each operand per stage
+    static constexpr int CH64 = QT == QT_Q6_K ? 1 : 2;      // 64-wide tiles of each operand per stage
     static constexpr int SPS = 4 / CH64;                        // stages per super-block
     static constexpr int A_BYTES = 128 * 128 * PLANES * CH64, B_BYTES = NT * 128 * CH64, STG_BYTES = A_BYTES + B_BYTES;
     static constexpr int RAW_BYTES = 128 * SB;
-    static constexpr int NSTG = QT == QT_Q4_K ? (NT > 64 ? 2 : 3) : QT == QT_Q6_K ? (NT > 64 ? 3 : 4) : (NT > 64 ? 3 : 2);
-    static constexpr int NR = QT == QT_Q4_K ? (NT > 64 ? 4 : NT > 32 ? 3 : NT > 16 ? 4 : 5) : QT == QT_Q6_K ? (NT > 16 ? 2 : 3) : (NT > 64 ? 2 : 3);
+    static constexpr int NSTG = QT == QT_Q4_K ? (NT > 64 ? 2 : 3) : QT == QT_Q6_K ? (NT > 64 ? 3 : 4) : 2;
+    static constexpr int NR = QT == QT_Q4_K ? (NT > 64 ? 4 : NT > 32 ? 3 : NT > 16 ? 4 : 5) : QT == QT_Q6_K ? (NT > 16 ? 2 : 3) : 3;
     static constexpr int GROUPS = QT == QT_Q8_0 ? 8 : 1;        // accumulators per super-block
     static constexpr int DG = QT == QT_Q8_0 ? 2 * CH64 : 1;     // ... that change hands together
     static constexpr bool MINS = QT == QT_Q4_K;
@@ -475,8 +475,12 @@ template <int QT>
 static int qgemm_launch_q(cudaStream_t st, const unsigned char* w, const QRows& x, int M, int N, int K, int epi, float* y, int ldy, bool pdl) {
     if (M <= 16) return qgemm_launch_t<QT, 16>(st, w, x, M, N, K, epi, y, ldy, pdl);
     if (M <= 32) return qgemm_launch_t<QT, 32>(st, w, x, M, N, K, epi, y, ldy, pdl);
-    if (M <= 64) return qgemm_launch_t<QT, 64>(st, w, x, M, N, K, epi, y, ldy, pdl);
-    return qgemm_launch_t<QT, 128>(st, w, x, M, N, K, epi, y, ldy, pdl);
+    // Two 64-column tiles against one of 128, per layer at width 4096: K-quants 128 rows 398 / 480 us, 512 rows 947 / 817 (the wider tile unpacks the weights
+    // half as often, but has two stages for its operands instead of three); Q8_0, which reads an accumulator per 32 elements, 475 / 655 and 1224 / 1328.
+    if constexpr (QT != QT_Q8_0) {
+        if (M > 192) return qgemm_launch_t<QT, 128>(st, w, x, M, N, K, epi, y, ldy, pdl);
+    }
+    return qgemm_launch_t<QT, 64>(st, w, x, M, N, K, epi, y, ldy, pdl);
 }
 
 int qgemm_launch(cudaStream_t st, int qt, const unsigned char* w, const QRows& x, int M, int N, int K, int epi, float* y, int ldy, bool pdl) {

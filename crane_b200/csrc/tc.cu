@@ -112,4 +112,27 @@ int tc_device_sms() {
     return sms[dev];
 }
 
+__global__ void __launch_bounds__(256, 1) cluster_probe_kernel() {}
+int tc_max_clusters(int cl) {
+    static std::mutex mu;
+    static int known[CB_MAX_DEV][9] = {};
+    int dev = 0;
+    if (cl < 2 || cl > 8 || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= CB_MAX_DEV) return 0;
+    std::lock_guard<std::mutex> g(mu);
+    if (!known[dev][cl]) {
+        constexpr int SMEM = 208 * 1024;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(cl); cfg.blockDim = dim3(256); cfg.dynamicSmemBytes = SMEM;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = cl; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr; cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaFuncSetAttribute(cluster_probe_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, cluster_probe_kernel, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
+        known[dev][cl] = n + 1;
+    }
+    return known[dev][cl] - 1;
+}
+
 }  // namespace cb

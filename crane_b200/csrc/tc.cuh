@@ -157,6 +157,8 @@ constexpr size_t TC_WS_FLOATS = (size_t)2 * 160 * 128 * 256;     // what every u
 // true once if a wait of a kernel on `st` ran out since the last call (read after a synchronisation of the stream)
 bool tc_take_wait_error(cudaStream_t st);
 int tc_device_sms();
+// clusters of `cl` (2 .. 8) CTAs that the device runs at the same time when a CTA takes a whole SM
+int tc_max_clusters(int cl);
 
 // ---- work dealt out along K ------------------------------------------------------------------
 // G CTAs share tiles x KB iterations; CTA c owns the iterations [unit * (c * base + min(c, rem)), ...): base or base + 1 units of `unit`

@@ -9,7 +9,7 @@ pytestmark = pytest.mark.gpu
 
 
 # split precision keeps 16 bits of every operand (2^-17 each): 3e-5 of the largest logit over a layer, four-fold; plain bf16 2^-9: 2e-2
-@pytest.mark.parametrize("rows,past", [(2, 0), (63, 0), (64, 1), (65, 63), (127, 0), (128, 64), (129, 7), (300, 0), (37, 200), (513, 130)])
+@pytest.mark.parametrize("rows,past", [(2, 0), (63, 0), (64, 1), (65, 63), (127, 0), (128, 64), (129, 7), (300, 0), (37, 200), (513, 130), (70, 600), (16, 640)])
 @pytest.mark.parametrize("precision", ["split", "bf16"])
 def test_dense_prefill(rows, past, precision):
     import crane_b200
