@@ -534,7 +534,7 @@ attn_decode_kernel(AttnDecArgs a) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // a KV head whose query group is wider than NREP is served by `groups` CTA clusters of NREP query heads each (6 = 2 x 3,
     // 8 = 2 x 4, ...): kvv numbers those sub-groups, query head = kvv * NREP + h; only sub-group 0 appends the new K/V row
-    const int ns = a.nsplit, kvv = blockIdx.x / ns, split = blockIdx.x % ns;
+    const int ns = RING ? a.nsplit : ATTN_NSPLIT, kvv = blockIdx.x / ns, split = blockIdx.x % ns;
     const int kvh = kvv / a.groups, sub = kvv % a.groups;
     const int b = blockIdx.y;
     const int q_dim = a.nh * D, kv_dim = a.nkv * D;
@@ -737,7 +737,7 @@ attn_decode_kernel(AttnDecArgs a) {
 #pragma unroll
         for (int j = 0; j < EPL; ++j) o[h][j] = 0.f;
     }
-    auto attend = [&](bool valid, const void* kp, const void* vp, const void* klp, const void* vlp) {
+    auto attend = [&](bool valid, const bf16* kp, const bf16* vp, const bf16* klp, const bf16* vlp) __attribute__((always_inline)) {
         float kf[EPL], vf[EPL];
         if (valid) {
             const uint4 kr = *reinterpret_cast<const uint4*>(kp);
@@ -778,8 +778,8 @@ attn_decode_kernel(AttnDecArgs a) {
     if constexpr (RING) {
         for (int i = 0; i < n_it; ++i) {
             asm volatile("cp.async.wait_group %0;" ::"n"(ATTN_DEPTH - 1) : "memory");
-            const unsigned char* p = ring + (i % ATTN_DEPTH) * 2048;
-            attend(w0 + i * NW * TPW + grp < t_end, p, p + 512, p + 1024, p + 1536);
+            const bf16* p = reinterpret_cast<const bf16*>(ring + (i % ATTN_DEPTH) * 2048);
+            attend(w0 + i * NW * TPW + grp < t_end, p, p + 256, p + 512, p + 768);
             ring_issue(i + ATTN_DEPTH);
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -863,19 +863,18 @@ attn_decode_kernel(AttnDecArgs a) {
         float ms[ATTN_NSPLIT];
         float M = -INFINITY;
 #pragma unroll
-        for (int s = 0; s < ATTN_NSPLIT; ++s) {
-            if (s >= ns) break;
-            const float* rml = cluster.map_shared_rank(&cta_ml[0][0], s);
-            ms[s] = rml[h * 2];
+        for (int s = 0; s < ATTN_NSPLIT; ++s) {       // (every load issued, splits that are not there masked: a loop with an early end serialised them, 1.3 us)
+            const float* rml = cluster.map_shared_rank(&cta_ml[0][0], RING ? min(s, ns - 1) : s);
+            ms[s] = RING && s >= ns ? -INFINITY : rml[h * 2];
             M = fmaxf(M, ms[s]);
         }
         float L = 0.f, O = 0.f;
 #pragma unroll
         for (int s = 0; s < ATTN_NSPLIT; ++s) {
-            if (s >= ns) break;
+            const int rs = RING ? min(s, ns - 1) : s;
             const float c = (ms[s] == -INFINITY) ? 0.f : __expf(ms[s] - M);
-            const float* rml = cluster.map_shared_rank(&cta_ml[0][0], s);
-            const float* ro = cluster.map_shared_rank(&cta_o[0][0], s);
+            const float* rml = cluster.map_shared_rank(&cta_ml[0][0], rs);
+            const float* ro = cluster.map_shared_rank(&cta_o[0][0], rs);
             L += rml[h * 2 + 1] * c;
             O += ro[h * D + i] * c;
         }
@@ -924,7 +923,7 @@ int attn_decode_launch(cudaStream_t st, int B, int D, const AttnDecArgs& a_in, b
     // splits per (sequence, KV group): all eight while they leave SMs idle, fewer as the batch itself fills the chip (two CTAs per SM)
     const int pairs = B * a.nkv * a.groups;
     a.nsplit = pairs <= 37 ? 8 : pairs <= 148 ? 4 : pairs <= 512 ? 2 : 1;
-    if (B <= 4) a.nsplit = ATTN_NSPLIT;
+    if (B <= 4 || a.kv_bits) a.nsplit = ATTN_NSPLIT;      // (the tile form's split is fixed)
     if (D == 128) {
         switch (sub) {
             case 1: return attn_decode_launch_r<128, 1>(st, B, a, pdl);
