@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <mutex>
 #include <unordered_map>
+#include <vector>
 
 namespace cb {
 
@@ -67,12 +68,26 @@ static std::mutex g_scratch_mu;
 static std::unordered_map<uint64_t, TcScratch> g_scratch;
 static uint64_t scratch_key(cudaStream_t st) { int dev = 0; cudaGetDevice(&dev); return ((uint64_t)(uintptr_t)st << 6) ^ (uint64_t)dev; }
 
+// Error words of streams: blocks of 1024 in pinned memory, handed out and taken back under g_scratch_mu (pinning a page per stream costs a handle's
+// first call milliseconds, giving it back a device synchronisation)
+static std::vector<int*> g_err_free;
+static int* take_err_word() {
+    if (g_err_free.empty()) {
+        int* block = nullptr;
+        if (cudaHostAlloc((void**)&block, 1024 * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+        for (int i = 1023; i >= 0; --i) { block[i] = 0; g_err_free.push_back(block + i); }
+    }
+    int* w = g_err_free.back();
+    g_err_free.pop_back();
+    return w;
+}
+
 int tc_scratch_get(cudaStream_t st, size_t ws_floats, int n_counters, TcScratch* out) {
     std::lock_guard<std::mutex> g(g_scratch_mu);
     TcScratch& sc = g_scratch[scratch_key(st)];
     if (!sc.err) {
-        if (cudaHostAlloc((void**)&sc.err, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) { sc.err = nullptr; return (int)cudaErrorMemoryAllocation; }
-        *sc.err = 0;
+        sc.err = take_err_word();
+        if (!sc.err) return (int)cudaErrorMemoryAllocation;
     }
     if (sc.ws_floats < ws_floats || sc.n_counters < n_counters) {
         // (growing: the old buffers may still be in use by kernels in flight on this stream)
@@ -101,7 +116,7 @@ void gemm_release_stream(cudaStream_t st) {
     auto it = g_scratch.find(scratch_key(st));
     if (it == g_scratch.end()) return;
     cudaFree(it->second.ws); cudaFree(it->second.counters);
-    if (it->second.err) cudaFreeHost(it->second.err);
+    if (it->second.err) { *it->second.err = 0; g_err_free.push_back(it->second.err); }
     g_scratch.erase(it);
 }
 int tc_device_sms() {
