@@ -1077,7 +1077,7 @@ void crane_b200_model::finalize() {
             if (l.qt_down) mx = std::max(mx, (size_t)H * I);
         }
         (void)mx;
-        xq_buf = dalloc<unsigned char>(xquant_bytes(4, std::max(std::max(H, I), q_dim())));      // groups of <= 4 rows / sequences
+        xq_buf = dalloc<unsigned char>(xquant_bytes(4, std::max(std::max(H, I), q_dim())));      // calls of up to four rows / sequences
     }
     for (int i = 0; i < L; ++i) {
         // full: q,k,v,o (1|2|4|8) gate,up,down (16|32|64) ln1,ln2 (128|256) q_norm,k_norm (512|1024)

@@ -1,5 +1,5 @@
-// GGUF-quantised linear layers (Q4_K / Q6_K / Q8_0): decode GEMV on the quantised bytes + dequantise-to-bf16 for prefill.
-// See quant.cu.
+// GGUF-quantised linear layers (Q4_K / Q6_K / Q8_0): GEMV on the quantised bytes for up to four rows (quant.cu),
+// integer dots on the tensor cores for more (qgemm.cu), expansion of blocks to bf16.
 #pragma once
 
 #include "decode.cuh"

@@ -180,8 +180,8 @@ CRANE_B200_API int crane_b200_seq_free(crane_b200_model* m, int seq);
 CRANE_B200_API int crane_b200_seq_select(crane_b200_model* m, int seq);
 /* `n_steps` greedy decode rounds for `n` sequences at once: replaces setup_batch_decode + step_batch_decode x rounds +
  * extract_batch_kv (crane-core/src/models/qwen3/modeling.rs:1141-1277, crane-serve/src/engine/mod.rs:822-1062).  No left-padding,
- * mask or KV copy: each sequence attends over its own pages with its own length and position; groups of up to 4 sequences share
- * one pass over the weights.  tokens[i] is consumed by seqs[i] at its cached length; tokens_out is [n, n_steps];
+ * mask or KV copy: each sequence attends over its own pages with its own length and position; groups of up to 64 sequences (4 in
+ * the hybrid and TTS models) share one pass over the weights.  tokens[i] is consumed by seqs[i] at its cached length; tokens_out is [n, n_steps];
  * logits_host (optional) receives the [n, vocab] f32 logits of the LAST round. */
 CRANE_B200_API int crane_b200_decode_batch(crane_b200_model* m, const int* seqs, const uint32_t* tokens, size_t n, size_t n_steps,
                                            uint32_t* tokens_out, float* logits_host);
@@ -318,7 +318,7 @@ CRANE_B200_API int crane_b200_decode_path(const crane_b200_model* m);
 CRANE_B200_API int crane_b200_op_gemm(int device, const uint16_t* a, const uint16_t* a_lo, const uint16_t* w, int M, int N, int K, int mode,
                        const float* bias, void* out_inout, int use_simt);
 
-/* y[m, n] = quantised linear of x[m, k] (host f32) through the decode kernels (xquant + qgemv, rows in groups of <= 4): `raw` = n rows
+/* y[m, n] = quantised linear of x[m, k] (host f32) through the engine's kernels (xquant + qgemv up to 4 rows, qgemm above): `raw` = n rows
  * of ggml blocks (ggml_type 8 / 12 / 14), optional RMSNorm weight norm_w[k] applied first (eps).  = candle's CPU `QMatMul::forward`
  * (crane-core/src/ops/linear.rs:23-48). */
 CRANE_B200_API int crane_b200_op_qlinear(int device, const float* x, size_t m, size_t k, const void* raw, size_t raw_bytes, int ggml_type, size_t n,
