@@ -1173,10 +1173,8 @@ void crane_b200_model::finalize() {
         w3_buf = dalloc<bf16>(3 * w3_plane);
         if (any_quant) xqd_buf = dalloc<unsigned char>(qrows_bytes(B, kmax));
         am_val = dalloc<float>((size_t)B * ARGMAX_ROW_PARTS); am_idx = dalloc<int>((size_t)B * ARGMAX_ROW_PARTS);
-        // (the scratch of the tensor-core linears: here, not under a graph capture)
-        TcScratch sc;
-        LAUNCH_OK(tc_scratch_get(stream, TC_WS_FLOATS, 4096, &sc));
-        wide_ok = (std::max(std::max(V, 2 * I), qkv_dim()) + 127) / 128 <= 4096;
+        TcScratch sc;                               // (taken here, not by the first decode step)
+        LAUNCH_OK(tc_scratch_get(stream, (std::max(std::max(V, 2 * I), qkv_dim()) + 127) / 128, &sc));
         // below wide_min the GEMVs (up to four sequences per pass) are as fast or faster
         wide_min = any_quant ? 5 : 3;
     }
@@ -2041,8 +2039,7 @@ void crane_b200_destroy(crane_b200_model* m) {
     m->sampler.release();
     m->spans.release();
     for (cudaEvent_t e : {m->pev0, m->pev1, m->dev0, m->dev1}) if (e) cudaEventDestroy(e);
-    if (m->stream) gemm_release_stream(m->stream);
-    if (m->stream && m->owns_stream) cudaStreamDestroy(m->stream);
+    if (m->stream && m->owns_stream) { tc_scratch_release(m->stream); cudaStreamDestroy(m->stream); }
     delete m;
 }
 

@@ -455,8 +455,8 @@ static int ftc_launch_t(cudaStream_t st, const FlashArgs& a) {
     }
     static SmemOptIn seen;
     if (const int e = ensure_dyn_smem(flash_tc_kernel<D, SPLIT, CAUSAL, PAGED>, (size_t)C::SMEM, seen)) return e;
-    TcScratch s;
-    if (const int e = tc_scratch_get(st, TC_WS_FLOATS, 4096, &s)) return e;
+    int* err = nullptr;
+    if (const int e = tc_err_word(st, &err)) return e;
     const int max_len = a.seq_len ? a.max_len : a.S, qt = (max_len + 127) / 128;
     // too few query tiles for the chip (a short turn behind a long cached prefix): clusters share their keys, at least two tiles each
     int ns = 1;
@@ -480,7 +480,7 @@ static int ftc_launch_t(cudaStream_t st, const FlashArgs& a) {
         ++na;
     }
     cfg.attrs = attr; cfg.numAttrs = na;
-    return (int)cudaLaunchKernelEx(&cfg, flash_tc_kernel<D, SPLIT, CAUSAL, PAGED>, m, a, ns, s.err);
+    return (int)cudaLaunchKernelEx(&cfg, flash_tc_kernel<D, SPLIT, CAUSAL, PAGED>, m, a, ns, err);
 }
 
 bool flash_tc_fits(int D, bool causal, bool paged, const FlashArgs& a) {

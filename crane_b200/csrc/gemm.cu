@@ -432,10 +432,12 @@ static int launch_tc(cudaStream_t stream, const bf16* A, const bf16* A_lo, int l
     sc.G = (int)std::max<long long>(1, std::min<long long>(cap, stream_k ? iters / g_gemm_minit : tiles));
     sc.base = (int)(units / sc.G);
     sc.rem = (int)(units % sc.G);
-    TcScratch scratch;
-    if (const int e = tc_scratch_get(stream, (size_t)2 * GEMM_MAX_CTAS * GEMM_BM * 256, (int)std::max<long long>(tiles, 1), &scratch)) return e;
-    sc.ws = scratch.ws;
-    sc.counters = scratch.counters;
+    if (sc.unit != sc.KB) {                          // (whole tiles dealt out: none is shared)
+        TcScratch scratch;
+        if (const int e = tc_scratch_get(stream, (int)tiles, &scratch)) return e;
+        sc.ws = scratch.ws;
+        sc.counters = scratch.counters;
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(sc.G);
     cfg.blockDim = dim3(256);

@@ -54,7 +54,5 @@ bool gemm_rows_fits(int planes, int M);
 int gemm_rows_launch(cudaStream_t stream, const bf16* const* planes, int n_planes, int lda, const bf16* W, int M, int N, int K, const GemmEpi& epi, bool pdl);
 // f32 rows -> three bf16 planes `plane` elements apart, rows of K; RMS-normalised first when norm_w is set
 int rows_split3_launch(cudaStream_t stream, const float* x, int ldx, int M, int K, const float* norm_w, float eps, bf16* out, long long plane, bool pdl);
-// Frees the stream-K scratch (partial tiles, arrival counters) kept for `stream`; call before destroying the stream.
-void gemm_release_stream(cudaStream_t stream);
 
 }  // namespace cb

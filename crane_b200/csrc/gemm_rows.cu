@@ -304,9 +304,6 @@ static int rows_launch_c(cudaStream_t st, const bf16* const* A, int lda, const b
     const long long iters = (long long)sc.tiles_n * a.KB;
     if (iters > 0x7fffffffLL) return -1000;
     const int sms = std::min(tc_device_sms(), GR_MAX_CTAS);
-    TcScratch s;
-    if (const int e = tc_scratch_get(st, TC_WS_FLOATS, sc.tiles_n, &s)) return e;
-    sc.ws = s.ws; sc.counters = s.counters; a.err = s.err;
     int grid;
     if (sc.tiles_n <= sms) {
         // as many CTAs per tile as the chip has room for at once (clusters live inside a GPC: sixteen of eight CTAs do not fit, and a second wave
@@ -314,7 +311,11 @@ static int rows_launch_c(cudaStream_t st, const bf16* const* A, int lda, const b
         a.cl = std::max(1, std::min(std::min(8, sms / sc.tiles_n), a.KB * CH / 4));
         while (a.cl > 1 && tc_max_clusters(a.cl) < sc.tiles_n) --a.cl;
         grid = sc.tiles_n * a.cl;
+        if (const int e = tc_err_word(st, &a.err)) return e;
     } else {
+        TcScratch s;
+        if (const int e = tc_scratch_get(st, sc.tiles_n, &s)) return e;
+        sc.ws = s.ws; sc.counters = s.counters; a.err = s.err;
         sc.unit = 1; sc.G = sms;
         sc.base = (int)(iters / sc.G); sc.rem = (int)(iters % sc.G);
         grid = sc.G;

@@ -466,7 +466,7 @@ static int qgemm_launch_t(cudaStream_t st, const unsigned char* w, const QRows& 
     sc.G = (int)std::max<long long>(1, std::min<long long>(std::min(tc_device_sms(), QT_MAX_CTAS), iters / 2));     // two super-blocks pay for a CTA's setup
     sc.base = (int)(iters / sc.G); sc.rem = (int)(iters % sc.G);
     TcScratch s;
-    if (const int e = tc_scratch_get(st, TC_WS_FLOATS, (int)std::max<long long>(tiles, 1), &s)) return e;
+    if (const int e = tc_scratch_get(st, (int)tiles, &s)) return e;
     sc.ws = s.ws; sc.counters = s.counters; a.err = s.err;
     return launch_k(qgemm_kernel<QT, NT>, dim3(sc.G), dim3(C::THREADS), C::SMEM, st, pdl, tmX, tmS, a);
 }

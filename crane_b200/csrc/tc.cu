@@ -1,11 +1,8 @@
 // Host side of the tensor-core kernels.  See tc.cuh.
 #include "tc.cuh"
-#include "gemm.cuh"
 
-#include <algorithm>
 #include <mutex>
 #include <unordered_map>
-#include <vector>
 
 namespace cb {
 
@@ -64,61 +61,6 @@ bool tc_tmap_16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols
     return true;
 }
 
-static std::mutex g_scratch_mu;
-static std::unordered_map<uint64_t, TcScratch> g_scratch;
-static uint64_t scratch_key(cudaStream_t st) { int dev = 0; cudaGetDevice(&dev); return ((uint64_t)(uintptr_t)st << 6) ^ (uint64_t)dev; }
-
-// Error words of streams: blocks of 1024 in pinned memory, handed out and taken back under g_scratch_mu (pinning a page per stream costs a handle's
-// first call milliseconds, giving it back a device synchronisation)
-static std::vector<int*> g_err_free;
-static int* take_err_word() {
-    if (g_err_free.empty()) {
-        int* block = nullptr;
-        if (cudaHostAlloc((void**)&block, 1024 * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) { cudaGetLastError(); return nullptr; }
-        for (int i = 1023; i >= 0; --i) { block[i] = 0; g_err_free.push_back(block + i); }
-    }
-    int* w = g_err_free.back();
-    g_err_free.pop_back();
-    return w;
-}
-
-int tc_scratch_get(cudaStream_t st, size_t ws_floats, int n_counters, TcScratch* out) {
-    std::lock_guard<std::mutex> g(g_scratch_mu);
-    TcScratch& sc = g_scratch[scratch_key(st)];
-    if (!sc.err) {
-        sc.err = take_err_word();
-        if (!sc.err) return (int)cudaErrorMemoryAllocation;
-    }
-    if (sc.ws_floats < ws_floats || sc.n_counters < n_counters) {
-        // (growing: the old buffers may still be in use by kernels in flight on this stream)
-        if (sc.ws || sc.counters) { cudaStreamSynchronize(st); cudaFree(sc.ws); cudaFree(sc.counters); }
-        sc.ws = nullptr; sc.counters = nullptr;
-        const size_t want = std::max(ws_floats, sc.ws_floats);
-        const int wantc = std::max(n_counters, std::max(sc.n_counters, 4096));
-        sc.ws_floats = 0; sc.n_counters = 0;
-        if (cudaMalloc(&sc.ws, want * sizeof(float)) != cudaSuccess) { sc.ws = nullptr; return (int)cudaErrorMemoryAllocation; }
-        if (cudaMalloc(&sc.counters, (size_t)wantc * sizeof(int)) != cudaSuccess) { cudaFree(sc.ws); sc.ws = nullptr; sc.counters = nullptr; return (int)cudaErrorMemoryAllocation; }
-        sc.ws_floats = want; sc.n_counters = wantc;
-        if (cudaMemsetAsync(sc.counters, 0, (size_t)sc.n_counters * sizeof(int), st) != cudaSuccess) return (int)cudaGetLastError();
-    }
-    *out = sc;
-    return 0;
-}
-bool tc_take_wait_error(cudaStream_t st) {
-    std::lock_guard<std::mutex> g(g_scratch_mu);
-    auto it = g_scratch.find(scratch_key(st));
-    if (it == g_scratch.end() || !it->second.err || !*reinterpret_cast<volatile int*>(it->second.err)) return false;
-    *it->second.err = 0;
-    return true;
-}
-void gemm_release_stream(cudaStream_t st) {
-    std::lock_guard<std::mutex> g(g_scratch_mu);
-    auto it = g_scratch.find(scratch_key(st));
-    if (it == g_scratch.end()) return;
-    cudaFree(it->second.ws); cudaFree(it->second.counters);
-    if (it->second.err) { *it->second.err = 0; g_err_free.push_back(it->second.err); }
-    g_scratch.erase(it);
-}
 int tc_device_sms() {
     static int sms[CB_MAX_DEV] = {};
     int dev = 0;

@@ -1,9 +1,10 @@
-// tcgen05 / TMA / mbarrier wrappers shared by the tensor-core kernels, and the host side they share: encoded tensor maps, per-stream
-// scratch, and the bounded waits' error flag.
+// tcgen05 / TMA / mbarrier wrappers shared by the tensor-core kernels, and the host side they share: encoded tensor maps and the per-stream
+// scratch (tc_scratch.h).
 #pragma once
 
 #include <cuda.h>
 #include "common.cuh"
+#include "tc_scratch.h"
 
 namespace cb {
 
@@ -14,7 +15,7 @@ namespace cb {
 constexpr long long TC_WAIT_CYCLES = 8000000000LL;
 struct TcWait {
     volatile int* gave_up;      // shared memory, zeroed before the first wait
-    int* err;                   // pinned host memory (TcScratch::err), written only when a wait runs out
+    int* err;                   // pinned host memory (tc_err_word), written only when a wait runs out
     __device__ __forceinline__ void operator()(uint64_t* bar, uint32_t parity) const {
         const uint32_t addr = smem_u32(bar);
         long long t0 = 0;
@@ -148,14 +149,6 @@ bool tc_tmap_16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols
 inline bool tc_tmap_bf16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows) {
     return tc_tmap_16(map, base, rows, cols, ld, box_rows, 64, CU_TENSOR_MAP_SWIZZLE_128B);
 }
-// Per-stream scratch: partial tiles, arrival counters (zero between launches) and the bounded waits' error word.  Kernels on one stream
-// are ordered (and a programmatic dependent only touches the scratch after its dependency wait), so one set per stream is enough;
-// gemm_release_stream (gemm.cuh) frees it with the stream.
-struct TcScratch { float* ws = nullptr; int* counters = nullptr; int* err = nullptr; size_t ws_floats = 0; int n_counters = 0; };
-int tc_scratch_get(cudaStream_t st, size_t ws_floats, int n_counters, TcScratch* out);
-constexpr size_t TC_WS_FLOATS = (size_t)2 * 160 * 128 * 256;     // what every user asks for: two partial 128 x 256 tiles per CTA
-// true once if a wait of a kernel on `st` ran out since the last call (read after a synchronisation of the stream)
-bool tc_take_wait_error(cudaStream_t st);
 int tc_device_sms();
 // clusters of `cl` (2 .. 8) CTAs that the device runs at the same time when a CTA takes a whole SM
 int tc_max_clusters(int cl);

@@ -106,3 +106,40 @@ def test_quantised_decode_batch(recipe):
     err = np.abs(nine - four).max(1) / np.abs(four).max()
     assert err.max() < 3e-2 and np.median(err) < 1e-2
     m.close()
+
+
+@pytest.mark.parametrize("recipe", ["", "Q8_0"])
+def test_batch_after_a_long_prompt(recipe):
+    """A captured batch step, a prompt whose linears have more tiles than any call before it (Q8_0: 64 rows x 128 columns, 33 x 128 of them), the same
+    step replayed: the same bits."""
+    import crane_b200
+    from oracle import ggml_quant as gq
+    cfg = dict(synth.TINY_QWEN3_UNTIED, num_hidden_layers=1, hidden_size=256, intermediate_size=8192)
+    m = crane_b200.Qwen3Model(cfg, max_seq_len=2176, max_batch=8)
+    for name, shape, kind in synth.tensor_specs(cfg):
+        t = synth.make_tensor(name, shape, kind)
+        if recipe and "proj" in name:
+            m.load_tensor_ggml(name, gq.GGML_TYPE_ID[recipe], t.shape, gq.quantize(t, recipe))
+        else:
+            m.load_tensor(name, t)
+    m.finalize()
+    slots = [0] + [m.seq_create() for _ in range(5)]
+    extra = m.seq_create()
+    for s in slots:
+        m.seq_select(s)
+        m.forward_step(synth.synth_token_ids(9 + s, cfg["vocab_size"], f"lp{s}"), 0)
+    tok = synth.synth_token_ids(6, cfg["vocab_size"], "lpt")
+
+    def batch():
+        for s in slots:
+            m.seq_select(s)
+            m.set_kv_caches([], 9 + s)
+        return m.decode_batch(slots, tok, 2, want_logits=True)
+    toks, want = batch()
+    for rows in (700, 2112, 2170):
+        m.seq_select(extra)
+        m.set_kv_caches([], 0)
+        m.forward_step(synth.synth_token_ids(rows, cfg["vocab_size"], f"lpp{rows}"), 0)
+        again, got = batch()
+        assert np.array_equal(again, toks) and np.array_equal(got, want)
+    m.close()
