@@ -143,3 +143,32 @@ def test_batch_after_a_long_prompt(recipe):
         again, got = batch()
         assert np.array_equal(again, toks) and np.array_equal(got, want)
     m.close()
+
+
+@pytest.mark.parametrize("vocab", [997, 998, 999])
+def test_decode_batch_of_any_vocabulary(vocab):
+    """Vocabularies that are not a multiple of four rows, against single steps (bounds as in test_decode_batch_against_single_steps)."""
+    import crane_b200
+    cfg = dict(synth.TINY_QWEN3_UNTIED, vocab_size=vocab)
+    m = crane_b200.Qwen3Model(cfg, max_seq_len=64, max_batch=33)
+    m.load_checkpoint(synth.synth_checkpoint(cfg))
+    slots = [0] + [m.seq_create() for _ in range(32)]
+    tok = synth.synth_token_ids(33, vocab, "anyv")
+    want = []
+    for s in slots:
+        m.seq_select(s)
+        m.forward_step(synth.synth_token_ids(3 + s, vocab, f"anyv{s}"), 0)
+        want.append(m.forward_step([int(tok[s])], 3 + s))
+    want = np.stack(want)
+    for n in (2, 3, 5, 33):
+        for s in slots[:n]:
+            m.seq_select(s)
+            m.set_kv_caches([], 3 + s)
+        toks, got = m.decode_batch(slots[:n], tok[:n], 1, want_logits=True)
+        assert np.abs(got - want[:n]).max() <= 3e-5 * np.abs(want).max()
+        assert np.array_equal(toks[:, 0], got.argmax(1))
+    for s in slots:
+        m.seq_select(s)
+        m.set_kv_caches([], 3 + s)
+    assert np.array_equal(m.decode_batch_sample(slots, tok, [dict(temperature=0.0)] * 33), toks[:, 0])
+    m.close()
