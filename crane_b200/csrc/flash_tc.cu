@@ -375,7 +375,7 @@ flash_tc_kernel(const __grid_constant__ FtcMaps maps, FlashArgs a, int ns, int* 
             l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
             tmem_st_wait();
             tc_fence_before();
-            if (PAGED && kv0 + BN > T) {       // the rest of the last page was never written: zero times whatever is there must stay zero
+            if (kv0 + BN > T) {       // the rows behind the last key are a page's never written rest or the next sequence's: zero times whatever is there must stay zero
                 const int seq = n_walk * C::NKS + (n_walk - 1) * C::NVS;
                 for (int j = 0; j < C::NVS; ++j) {
                     const int slot = (seq + j) % C::NSLOT, lo_r = max(0, T - kv0 - j * C::R);

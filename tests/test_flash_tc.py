@@ -63,3 +63,23 @@ def test_vision(grids):
     for g, r in [(got, ref)] + list(zip(ds, deep)):
         assert np.abs(g - r.numpy()).max() <= 1.2e-4 * np.abs(r.numpy()).max()
     m.close()
+
+
+@pytest.mark.parametrize("grid", [(1, 2, 2), (1, 8, 18), (1, 20, 20), (1, 16, 24)])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_image_beside_one_that_is_not_finite(grid, bad):
+    """The keys behind an image's last one are the next image's: whatever it holds, the first image's features are the same bits."""
+    import crane_b200
+    cfg = synth.TINY_QWEN3_VL
+    m = crane_b200.Qwen3VLModel(cfg, max_seq_len=64)
+    m.load_checkpoint(synth.synth_checkpoint(cfg))
+    grids = [grid, (1, 12, 14)]
+    n = grid[1] * grid[2]
+    pv = np.random.default_rng(n).uniform(-1, 1, (n + 168, 1536)).astype(np.float32)
+    clean, clean_ds = m.encode_images(pv, grids, want_deepstack=3)
+    pv[n:, ::7] = bad
+    got, ds = m.encode_images(pv, grids, want_deepstack=3)
+    assert not np.isfinite(got[n // 4:]).any()
+    for g, c in [(got, clean)] + list(zip(ds, clean_ds)):
+        assert np.array_equal(g[: n // 4], c[: n // 4])
+    m.close()
