@@ -60,6 +60,16 @@ struct EngineError {
                            r__ > 0 ? cudaGetErrorString((cudaError_t)r__) : "", __FILE__, __LINE__);          \
     } while (0)
 
+// Results leave for the caller: the tensor-core kernels bound their waits (tc.cuh), and a kernel that gave one up has left garbage behind.
+// Called on an idle stream, ahead of everything that a good result is followed by (a sequence's length, a return code).
+void check_waits(cudaStream_t st) {
+    if (tc_take_wait_error(st)) fail(CRANE_B200_CUDA_ERROR, "a tensor-core kernel's wait ran out (results discarded)");
+}
+void sync_results(cudaStream_t st) {
+    CUDA_OK(cudaStreamSynchronize(st));
+    check_waits(st);
+}
+
 std::string g_create_error;
 
 // ---- host dtype conversion ---------------------------------------------------------------------
@@ -231,7 +241,6 @@ struct crane_b200_model {
     unsigned long long* ll_trace = nullptr;   // CRANE_B200_LL_TRACE=<file>: event trace of one step (tools/ll_trace.py)
     void ll_err_fetch();                   // enqueue the D2H copy of the flag (before a stream sync the caller does anyway)
     void ll_err_verify();                  // after that sync
-    void wait_verify();
     // vision
     int v_depth = 0, v_H = 0, v_I = 0, v_nh = 0, v_hd = 0, v_patch = 16, v_merge = 2, v_tpatch = 2, v_in = 3, v_out = 0,
         v_npos = 0, v_side = 0;
@@ -1561,16 +1570,12 @@ void crane_b200_model::decode_steps(int n_steps, int advance) {
     for (int i = 0; i < n_steps; ++i) decode_step_graphed(advance);
 }
 
-// The tensor-core kernels bound theirs too (tc.cuh): read after a synchronisation of the stream.
-void crane_b200_model::wait_verify() {
-    if (tc_take_wait_error(stream)) fail(CRANE_B200_CUDA_ERROR, "a tensor-core kernel's wait ran out (results discarded)");
-}
 // The persistent kernel bounds every wait; a wait that gave up leaves garbage behind and raises this flag (read at sync points).
 void crane_b200_model::ll_err_fetch() {
     if (ll_err) CUDA_OK(cudaMemcpyAsync(h_ll_err, ll_err, sizeof(unsigned int), cudaMemcpyDeviceToHost, stream));
 }
 void crane_b200_model::ll_err_verify() {
-    wait_verify();
+    check_waits(stream);
     if (!ll_err || *h_ll_err == 0) return;
     std::vector<unsigned int> d(16 + num_sms * LL_WARPS);
     CUDA_OK(cudaMemcpy(d.data(), ll_err, d.size() * sizeof(unsigned int), cudaMemcpyDeviceToHost));
@@ -2165,6 +2170,7 @@ int crane_b200_warmup(crane_b200_model* m) {
         CUDA_OK(cudaStreamSynchronize(m->stream));
         m->fsv->seq_free(m->cur);
         m->kv_len = 0;
+        check_waits(m->stream);
         return CRANE_B200_OK;
     }
     uint32_t ids[4] = {0, 1 % (uint32_t)m->V, 2 % (uint32_t)m->V, 3 % (uint32_t)m->V};
@@ -2175,6 +2181,7 @@ int crane_b200_warmup(crane_b200_model* m) {
     m->kv_len = 0;
     m->next_mrope_pos = saved_pos;
     if (m->hybrid) m->reset_recurrent_state();
+    check_waits(m->stream);
     API_END(m)
 }
 
@@ -2290,7 +2297,7 @@ int crane_b200_encode_images(crane_b200_model* m, const float* pixel_values, con
     if (image_embeds_out) CUDA_OK(cudaMemcpyAsync(image_embeds_out, m->img_embeds, n * sizeof(float), cudaMemcpyDeviceToHost, m->stream));
     if (deepstack_out && !m->v_deepstack.empty())
         CUDA_OK(cudaMemcpyAsync(deepstack_out, m->ds_embeds, m->v_deepstack.size() * n * sizeof(float), cudaMemcpyDeviceToHost, m->stream));
-    CUDA_OK(cudaStreamSynchronize(m->stream));
+    sync_results(m->stream);
     API_END(m)
 }
 
@@ -2425,7 +2432,7 @@ int crane_b200_kv_export(crane_b200_model* m, int layer, float* k_out, float* v_
             if (capacity_floats < std::max(cs, rs)) fail(CRANE_B200_INVALID_ARG, "kv_export: GDN layer needs %zu floats", std::max(cs, rs));
             if (k_out) CUDA_OK(cudaMemcpyAsync(k_out, l.conv_state, cs * sizeof(float), cudaMemcpyDeviceToHost, m->stream));
             if (v_out) CUDA_OK(cudaMemcpyAsync(v_out, l.rec_state, rs * sizeof(float), cudaMemcpyDeviceToHost, m->stream));
-            CUDA_OK(cudaStreamSynchronize(m->stream));
+            sync_results(m->stream);
         }
     } else {
         *n_tokens = T;
@@ -2445,6 +2452,7 @@ int crane_b200_kv_export(crane_b200_model* m, int layer, float* k_out, float* v_
                 cudaStreamSynchronize(m->stream);
             }
             cudaFree(tmp);
+            check_waits(m->stream);
         }
     }
     API_END(m)
@@ -2551,7 +2559,7 @@ int crane_b200_decode_batch(crane_b200_model* m, const int* seqs, const uint32_t
         m->logits = m->fsv->logits; m->launches = m->fsv->launches;
         if (logits_host) {
             CUDA_OK(cudaMemcpyAsync(logits_host, m->logits, n * (size_t)m->V * sizeof(float), cudaMemcpyDeviceToHost, m->stream));
-            CUDA_OK(cudaStreamSynchronize(m->stream));
+            sync_results(m->stream);
         }
         for (int i = 0; i < m->max_batch; ++i) m->seq_kv[i] = (size_t)m->fsv->seqs[i].len;
         m->kv_len = m->seq_kv[m->cur];
@@ -2590,8 +2598,7 @@ int crane_b200_decode_batch(crane_b200_model* m, const int* seqs, const uint32_t
                                   n_steps * sizeof(uint32_t), B, cudaMemcpyDeviceToHost, m->stream));
         if (logits_host)
             CUDA_OK(cudaMemcpyAsync(logits_host + done * (size_t)m->V, m->logits, (size_t)B * m->V * sizeof(float), cudaMemcpyDeviceToHost, m->stream));
-        CUDA_OK(cudaStreamSynchronize(m->stream));     // tokens_out / logits_host are the caller's memory: complete before returning
-        m->wait_verify();
+        sync_results(m->stream);                       // tokens_out / logits_host are the caller's memory: complete before returning
         if (pinned) std::memcpy(tokens_out + done * n_steps, m->h_tokens, (size_t)B * n_steps * sizeof(uint32_t));
         for (int b = 0; b < B; ++b) {
             const int s = seqs[done + b];
@@ -2661,7 +2668,7 @@ int crane_b200_topk(crane_b200_model* m, size_t k, uint32_t* idx_out, float* val
     LAUNCH_OK(sampler_topk_launch(m->stream, m->logits, m->V, 1, (int)k, m->sampler.tk_idx, m->sampler.tk_val));
     CUDA_OK(cudaMemcpyAsync(idx_out, m->sampler.tk_idx, k * sizeof(uint32_t), cudaMemcpyDeviceToHost, m->stream));
     if (vals_out) CUDA_OK(cudaMemcpyAsync(vals_out, m->sampler.tk_val, k * sizeof(float), cudaMemcpyDeviceToHost, m->stream));
-    CUDA_OK(cudaStreamSynchronize(m->stream));
+    sync_results(m->stream);
     API_END(m)
 }
 
@@ -2751,7 +2758,7 @@ int crane_b200_op_qlinear(int device, const float* x, size_t m, size_t k, const 
             s0 += B;
         }
         CUDA_OK(cudaDeviceSynchronize());
-        if (tc_take_wait_error(nullptr)) fail(CRANE_B200_CUDA_ERROR, "a tensor-core kernel's wait ran out (results discarded)");
+        check_waits(nullptr);
         CUDA_OK(cudaMemcpy(y, dy, m * n * 4, cudaMemcpyDeviceToHost));
     } catch (const EngineError& e) {
         g_create_error = e.msg;
@@ -2768,9 +2775,16 @@ extern "C" CRANE_B200_API int crane_b200_debug_peek(crane_b200_model* m, int whi
     need_ready(m);
     const float* src = which == 0 ? m->x : which == 1 ? m->qkv : m->rows_f32;
     if (!src || !out) fail(CRANE_B200_INVALID_ARG, "debug_peek: buffer %d does not exist", which);
-    CUDA_OK(cudaStreamSynchronize(m->stream));
+    sync_results(m->stream);
     CUDA_OK(cudaMemcpy(out, src, n_floats * sizeof(float), cudaMemcpyDeviceToHost));
     API_END(m)
+}
+
+/* debugging aid (not in the public header): a kernel on the handle's stream (nullptr: the current device's default stream) whose wait, for a barrier that nothing arrives at,
+ * runs out after about a millisecond -- what the host then reads is what it reads when a wait of a tensor-core kernel runs out */
+extern "C" CRANE_B200_API int crane_b200_debug_expire_wait(crane_b200_model* m) {
+    if (m) cudaSetDevice(m->device);
+    return tc_expire_wait(m ? m->stream : nullptr) == 0 ? CRANE_B200_OK : CRANE_B200_CUDA_ERROR;
 }
 
 static int op_sampler(int device, const float* logits, size_t vocab, size_t k, const crane_b200_sampling* p, uint32_t* out, float* logits_after) {
@@ -2842,7 +2856,9 @@ int crane_b200_op_gemm(int device, const uint16_t* a, const uint16_t* a_lo, cons
         GemmEpi ep{dout, nullptr, out_cols, db, mode};
         const int r = gemm_bf16_launch(nullptr, da, a_lo ? da + (size_t)M * K : nullptr, K, dw, M, N, K, ep, use_simt != 0);
         if (r == -1000) rc = CRANE_B200_UNSUPPORTED;
-        else if (r == 0 && cudaDeviceSynchronize() == cudaSuccess) {
+        else if (const bool done = r == 0 && cudaDeviceSynchronize() == cudaSuccess; done && tc_take_wait_error(nullptr)) {
+            g_create_error = "op_gemm: a tensor-core kernel's wait ran out (results discarded)";
+        } else if (done) {
             cudaMemcpy(out_inout, dout, out_bytes, cudaMemcpyDeviceToHost);
             rc = CRANE_B200_OK;
             if (getenv("CRANE_B200_GEMM_PROF") && !use_simt) {      // tile timeline + event timing of this shape (tools/gemm_probe.py)

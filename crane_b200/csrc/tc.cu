@@ -69,6 +69,23 @@ int tc_device_sms() {
     return sms[dev];
 }
 
+__global__ void expire_wait_kernel(int* err) {
+    __shared__ uint64_t bar;
+    __shared__ int gave_up;
+    gave_up = 0;
+    mbar_init(&bar, 1);
+    fence_barrier_init();
+    const TcWaitT<2000000> wait{&gave_up, err};
+    wait(&bar, 0);
+    wait(&bar, 0);                  // (given up: returns at once)
+}
+int tc_expire_wait(cudaStream_t st) {
+    int* err = nullptr;
+    if (const int e = tc_err_word(st, &err)) return e;
+    expire_wait_kernel<<<1, 1, 0, st>>>(err);
+    return (int)cudaGetLastError();
+}
+
 __global__ void __launch_bounds__(256, 1) cluster_probe_kernel() {}
 int tc_max_clusters(int cl) {
     static std::mutex mu;

@@ -11,9 +11,11 @@ namespace cb {
 // ---- bounded waits ---------------------------------------------------------------------
 // A wait that runs out (4 s at 1.9 GHz: a wait in these kernels is for a copy or an MMA of its own CTA, or for the end of the kernel ahead)
 // raises the CTA's `gave_up` word in shared memory and the stream's error word in pinned host memory; every later wait of the CTA
-// returns at once, the kernel runs to its end with its results discarded, and the host reports the error at its next read of a result.
+// returns at once, the kernel runs to its end with its results discarded, and every call that hands results to the caller reads the word first
+// (sync_results in engine.cu) and reports the error.  Results that are left on the device are covered by the call that reads them.
 constexpr long long TC_WAIT_CYCLES = 8000000000LL;
-struct TcWait {
+template <long long LIMIT>
+struct TcWaitT {
     volatile int* gave_up;      // shared memory, zeroed before the first wait
     int* err;                   // pinned host memory (tc_err_word), written only when a wait runs out
     __device__ __forceinline__ void operator()(uint64_t* bar, uint32_t parity) const {
@@ -30,7 +32,7 @@ struct TcWait {
             if ((n & 255u) == 255u) {
                 if (*gave_up) return;
                 if (!t0) t0 = clock64();
-                else if (clock64() - t0 > TC_WAIT_CYCLES) { *gave_up = 1; *reinterpret_cast<volatile int*>(err) = 1; return; }
+                else if (clock64() - t0 > LIMIT) { *gave_up = 1; *reinterpret_cast<volatile int*>(err) = 1; return; }
             }
         }
     }
@@ -41,6 +43,7 @@ struct TcWait {
         while (clock64() - t0 < 20000000LL) {}
     }
 };
+using TcWait = TcWaitT<TC_WAIT_CYCLES>;
 // One lane of a converged warp.  An issuing warp runs its loop as a whole and only its tcgen05 / TMA instructions under this: addresses and descriptors
 // stay in uniform registers (measured, 128 x 16 MMAs: 40 cycles each, 52 when a single lane runs the loop).
 __device__ __forceinline__ bool elect_one() {
@@ -149,6 +152,8 @@ bool tc_tmap_16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols
 inline bool tc_tmap_bf16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows) {
     return tc_tmap_16(map, base, rows, cols, ld, box_rows, 64, CU_TENSOR_MAP_SWIZZLE_128B);
 }
+// launches a kernel whose wait runs out after about a millisecond (for tests of what follows)
+int tc_expire_wait(cudaStream_t st);
 int tc_device_sms();
 // clusters of `cl` (2 .. 8) CTAs that the device runs at the same time when a CTA takes a whole SM
 int tc_max_clusters(int cl);
