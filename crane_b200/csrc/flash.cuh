@@ -9,8 +9,8 @@ namespace cb {
 // Flash attention forward (prefill + ViT): 64 query rows x one head per CTA, 64-key tiles,
 // bf16 mma.sync m16n8k16 with f32 accumulation and an online (base-2) softmax.
 // Keys/values come either from KV pages (one tile == one page) or from a strided buffer.
-// Runs where key and value widths differ, on ragged widths, and where an address or stride is not a multiple of 16 bytes;
-// equal widths otherwise go through flash_tc.cu.
+// Runs where key and value widths differ, on ragged widths, on few keys (flash_few_keys in prefill.cu has the lines), and where an address or
+// stride is not a multiple of 16 bytes; equal widths otherwise go through flash_tc.cu.
 // -------------------------------------------------------------------------------------
 __device__ __forceinline__ void ldmatrix_x4(uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3, uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(addr));

@@ -9,6 +9,7 @@
 //   splice / DeepStack .............. qwen3_5/vlm.rs:433-468 ; qwen3_vl/text.rs:280-333
 #include "prefill.cuh"
 #include "flash.cuh"
+#include "tc.cuh"
 
 namespace cb {
 
@@ -206,10 +207,25 @@ int rope_append_launch(cudaStream_t st, int D, const RopeAppendArgs& a) {
     return -1000;
 }
 
+// Few keys: flash.cuh's 64-row tiles beat the 128 x 128 ones of flash_tc.cu, whose setup (TMEM, barriers, a query tile of 128 rows) and first tile take 9 - 13 us
+// whatever they hold, as long as those tiles fit the chip at once.  us, flash.cuh / flash_tc.cu, one sequence:
+//   D = 128 causal, split (16 heads)   2 rows 6.6 / 12.8, 64 9.5 / 12.1, 100 12.1 / 12.0, 192 16.3 / 13.7; 16 rows behind 64 cached 11.5 / 11.6
+//   D = 128 causal, plain              128 rows 8.0 / 8.7, 129 10.0 / 11.0, 192 11.0 / 10.5
+//   D = 256 causal, split (8 heads)    16 rows 12.0 / 13.4, 33 13.6 / 12.9
+//   D = 64 causal, split (16 heads)    64 rows 6.9 / 9.7, 129 9.9 / 11.8, 192 11.6 / 11.5
+//   D = 64 contiguous, split           64 rows 5.5 / 8.4, 256 10.0 / 10.2, 320 11.5 / 11.7, 400 14.0 / 13.5; four images of 160: 11.7 / 11.1 (192 tiles of 64 rows)
+//   D = 64 contiguous, plain           224 rows 6.4 / 8.2, 512 9.6 / 10.2, 1024 23.8 / 14.7
+//   D = 128 contiguous, split          64 rows 8.6 / 10.0, 224 15.7 / 12.7
+static bool flash_few_keys(int D, bool causal, bool split, const FlashArgs& a) {
+    const int rows = a.seq_len ? a.max_len : a.S, keys = a.seq_len ? (causal ? a.max_kv : a.max_len) : (causal ? a.kv_offset : 0) + a.S;
+    const int most = D == 256 ? 32 : D == 128 ? (split ? 96 : 160) : causal ? 160 : split ? 320 : 512;
+    return keys > 0 && keys <= most && (long long)((rows + 63) / 64) * a.nh * (a.seq_len ? a.nseq : 1) <= tc_device_sms();
+}
+
 int flash_prefill_launch(cudaStream_t st, int D, bool causal, bool paged, const FlashArgs& a, int DV) {
     const bool split = a.q_lo_off != 0;
     if (split && (a.kv_lo_off == 0 || a.out_lo_off == 0)) return -1000;
-    if ((DV == 0 || DV == D) && flash_tc_fits(D, causal, paged, a)) return flash_tc_launch(st, D, causal, a);
+    if ((DV == 0 || DV == D) && flash_tc_fits(D, causal, paged, a) && !flash_few_keys(D, causal, split, a)) return flash_tc_launch(st, D, causal, a);
     if (DV != 0 && DV != D) {
         if (!causal || !paged) return -1000;
         if (D == 64 && DV == 128) return split ? flash_launch_t<64, 128, true, true, true>(st, a) : flash_launch_t<64, 128, true, true, false>(st, a);

@@ -50,6 +50,7 @@ struct FlashArgs {
     float scale;
     int nseq;
     int max_len;                        // max query rows over sequences (grid sizing)
+    int max_kv = 0;                     // causal, seq_len given: no sequence sees more keys than this (0: unknown); it only chooses the kernel
     // split precision (x = hi + lo, both bf16): element offsets of the low-order planes, 0 = plain bf16
     long long q_lo_off, kv_lo_off, out_lo_off;
     // ragged batches over paged caches (seq_start / seq_len set): sequence z reads block_table + seq_slot[z] * bt_stride and sees

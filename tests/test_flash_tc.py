@@ -83,3 +83,22 @@ def test_image_beside_one_that_is_not_finite(grid, bad):
     for g, c in [(got, clean)] + list(zip(ds, clean_ds)):
         assert np.array_equal(g[: n // 4], c[: n // 4])
     m.close()
+
+
+# the lines between the two attention kernels (flash_few_keys): 96 keys at D = 128 in split precision, 160 in plain bf16
+@pytest.mark.parametrize("rows,past", [(95, 0), (96, 0), (97, 0), (16, 80), (16, 81), (160, 0), (161, 0), (2, 158), (2, 159), (40, 57)])
+@pytest.mark.parametrize("precision", ["split", "bf16"])
+def test_few_keys(rows, past, precision):
+    test_dense_prefill(rows, past, precision)
+
+
+@pytest.mark.parametrize("rows,past", [(31, 0), (32, 0), (33, 0), (2, 30), (2, 31)])
+def test_few_keys_hybrid(rows, past):
+    """... 32 at D = 256"""
+    test_hybrid_prefill(rows, past)
+
+
+@pytest.mark.parametrize("grids", [[(1, 16, 20)], [(1, 18, 18)], [(1, 10, 16)] * 2, [(1, 2, 2), (1, 18, 20)]])
+def test_few_keys_vision(grids):
+    """... 320 at D = 64 without a mask, as long as the 64-row tiles of all images fit the chip"""
+    test_vision(grids)
