@@ -374,6 +374,14 @@ struct crane_b200_model {
     const int* bt_cur() const { return block_table + (size_t)cur * max_pages; }
     cudaGraphExec_t graph_step[2][DECODE_GROUP_MAX + 1] = {};   // [advance][sequences in the group]
     bool graph_failed = false;
+    // A step of a wide group runs as fast launched kernel by kernel (28 layers of width 1024, 8 sequences: 1357 us, replayed 1337; 36 Q4_K_M layers 2377 and
+    // 2307) and a capture costs 1 - 2 ms, so a server whose batch grows and shrinks through every size must not capture each at sight: a size is
+    // captured once GRAPH_AFTER steps of it have run, and the GRAPH_KEEP sizes last used are kept.
+    static constexpr uint32_t GRAPH_AFTER = 16;
+    static constexpr int GRAPH_KEEP = 16;
+    uint32_t graph_uses[2][DECODE_GROUP_MAX + 1] = {};
+    uint64_t graph_last[2][DECODE_GROUP_MAX + 1] = {}, graph_tick = 0;
+    void drop_oldest_wide_graph();
     cudaEvent_t pev0 = nullptr, pev1 = nullptr, dev0 = nullptr, dev1 = nullptr;
     bool pev0_armed = false;
     float last_prefill_ms = 0.f, last_decode_ms = 0.f;
@@ -1486,10 +1494,29 @@ void crane_b200_model::enqueue_wide_step(int advance, int B) {
     if (advance && q_embed) embed_step_input(B);
 }
 
+// Leaves room for one more captured wide step.
+void crane_b200_model::drop_oldest_wide_graph() {
+    int held = 0, oa = 0, ob = 0;
+    for (int a = 0; a < 2; ++a)
+        for (int b = wide_min; b <= DECODE_GROUP_MAX; ++b)
+            if (graph_step[a][b] && (++held == 1 || graph_last[a][b] < graph_last[oa][ob])) { oa = a; ob = b; }
+    if (held < GRAPH_KEEP) return;
+    CUDA_OK(cudaStreamSynchronize(stream));             // (a replay of it may still be running)
+    CUDA_OK(cudaGraphExecDestroy(graph_step[oa][ob]));
+    graph_step[oa][ob] = nullptr;
+    graph_uses[oa][ob] = 0;
+}
+
 // One decode step (layers + lm_head), replayed from a CUDA graph when capture is available.
 void crane_b200_model::decode_step_graphed(int advance, int B) {
     cudaGraphExec_t& ge = graph_step[advance][B];
-    if (use_graphs && !graph_failed && ge == nullptr) {
+    bool capture = use_graphs && !graph_failed && ge == nullptr;
+    if (wide(B)) {
+        graph_last[advance][B] = ++graph_tick;
+        if (capture && graph_uses[advance][B] < GRAPH_AFTER) { ++graph_uses[advance][B]; capture = false; }
+        if (capture) drop_oldest_wide_graph();
+    }
+    if (capture) {
         cudaGraph_t g = nullptr;
         const uint64_t before = launches;
         cudaError_t e = cudaStreamBeginCapture(stream, cudaStreamCaptureModeRelaxed);

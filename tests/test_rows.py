@@ -172,3 +172,29 @@ def test_decode_batch_of_any_vocabulary(vocab):
         m.set_kv_caches([], 3 + s)
     assert np.array_equal(m.decode_batch_sample(slots, tok, [dict(temperature=0.0)] * 33), toks[:, 0])
     m.close()
+
+
+def test_batches_of_many_sizes():
+    """Steps launched kernel by kernel, captured after a while, replayed, dropped for other sizes' captures and captured again: the same bits as without graphs."""
+    import crane_b200
+    cfg = dict(synth.TINY_QWEN3_UNTIED, num_hidden_layers=1)
+    out = []
+    for graphs in (True, False):
+        m = crane_b200.Qwen3Model(cfg, max_seq_len=64, max_batch=24, graphs=graphs)
+        m.load_checkpoint(synth.synth_checkpoint(cfg))
+        slots = [0] + [m.seq_create() for _ in range(23)]
+        for s in slots:
+            m.seq_select(s)
+            m.forward_step(synth.synth_token_ids(5 + s, cfg["vocab_size"], f"ms{s}"), 0)
+        tok = synth.synth_token_ids(24, cfg["vocab_size"], "mst")
+        got = []
+        for n in list(range(2, 25)) * 2 + [3, 24, 3]:
+            for s in slots[:n]:
+                m.seq_select(s)
+                m.set_kv_caches([], 5 + s)
+            got += m.decode_batch(slots[:n], tok[:n], 20, want_logits=True)
+            got.append(m.decode_batch(slots[:n], tok[:n], 1)[0])
+        out.append(got)
+        m.close()
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
