@@ -1,4 +1,4 @@
-"""Prefill attention on tcgen05 (csrc/flash_tc.cu) through one-layer models, at the edges of its tiles: 128 query rows, 64 keys, a last page that was never
+"""Prefill attention on tcgen05 (csrc/flash_tc.cu) through one-layer models, at the edges of its tiles: 128 query rows, 128 keys (64 at D = 256), a last page that was never
 written to its end, cached prefixes; the oracle in f32."""
 import numpy as np
 import pytest
@@ -102,3 +102,57 @@ def test_few_keys_hybrid(rows, past):
 def test_few_keys_vision(grids):
     """... 320 at D = 64 without a mask, as long as the 64-row tiles of all images fit the chip"""
     test_vision(grids)
+
+
+# a cluster of CTAs shares the keys of a query tile: one of them has none (the first query tile has one key tile), and clusters of eight
+@pytest.mark.parametrize("family,rows,past", [("dense", 700, 0), ("dense", 70, 2100), ("hybrid", 90, 1100)])
+def test_shared_keys(family, rows, past):
+    import crane_b200
+    from oracle.qwen3 import Qwen3Oracle
+    from oracle.qwen3_5 import Qwen3_5Oracle
+    cfg = dict(synth.TINY_QWEN3_UNTIED, num_hidden_layers=1) if family == "dense" else synth.TINY_QWEN3_5
+    w = dict(synth.synth_checkpoint(cfg))
+    m = (crane_b200.Qwen3Model if family == "dense" else crane_b200.Qwen3_5Model)(cfg, max_seq_len=past + rows + 64)
+    m.load_checkpoint(w.items())
+    orc = (Qwen3Oracle if family == "dense" else Qwen3_5Oracle)(cfg, w)
+    ids = synth.synth_token_ids(past + rows, cfg["vocab_size"], f"ftsk-{rows}-{past}")
+    if past:
+        orc.forward(ids[:past], 0)
+        m.forward_step(ids[:past], 0)
+    ref, got = orc.forward(ids[past:], past).numpy(), m.forward_step(ids[past:], past)
+    assert np.abs(got - ref).max() <= 1.2e-4 * np.abs(ref).max()
+    m.close()
+
+
+def modified(which):
+    """Layer lists whose attention has 128-wide heads and, between them, every score modifier and mask; windows at the edges of the 128-key tiles."""
+    import test_gavipel as g
+    import test_puzonex as p
+    import test_suvapel as s
+    wide = dict(width=256, vocab=300)
+    if which == "window, gate, sink":
+        return g, g.config([g.layer(g.mixer(heads=4, kv_heads=2, dim=128, vdim=128, scale=0.08, window=128, rot_dims=64), None),
+                            g.layer(g.mixer(heads=4, kv_heads=2, dim=128, vdim=128, scale=0.08, window=0, rot_dims=64), None)], loop=(0, 1, 1), **wide)
+    if which == "cap, distance":
+        return p, p.config([p.layer(p.attention(heads=4, kv_heads=2, dim=128, vdim=128, window=129, scale=0.09), None),
+                            p.layer(p.attention(heads=4, kv_heads=4, dim=128, vdim=128, window=0, scale=0.09), None)], **wide)
+    if which == "cap, table":
+        return p, p.config([p.layer(p.parallel(heads=2, kv_heads=1, dim=128, window=150, scale=0.09, rheads=2, rdim=64, rvdim=64), None)], **wide)
+    return s, s.config([s.layer(s.parallel(heads=4, kv_heads=2, dim=128, vdim=128, size=127, keep=130, scale=0.09, right=s.rule(heads=2, kv_heads=1, dim=64, vdim=64, conv=3)), None)], side=40, **wide)
+
+
+@pytest.mark.parametrize("which", ["window, gate, sink", "cap, distance", "cap, table", "window, kept first keys"])
+def test_modifiers_in_a_ragged_batch(which):
+    """Unequal prompts side by side, then their next portions, in 128-row tiles: every row against the oracle in f64."""
+    mod, cfg = modified(which)
+    m, w = mod.make(cfg, 21, precision="split", max_tokens=2048)
+    lens, more = (400, 129, 257), (70, 128, 3)
+    slots = [0, m.seq_create(), m.seq_create()]
+    ids = [mod.tokens(a + b, cfg["vocab"], 30 + i) for i, (a, b) in enumerate(zip(lens, more))]
+    first = m.step_batch([(s, t[:a], mod.all_rows(a)) for s, t, a in zip(slots, ids, lens)])
+    second = m.step_batch([(s, t[a:], mod.all_rows(b)) for s, t, a, b in zip(slots, ids, lens, more)])
+    fa, fb = np.cumsum((0,) + lens), np.cumsum((0,) + more)
+    for i in range(3):
+        got = np.concatenate([first[fa[i]: fa[i + 1]], second[fb[i]: fb[i + 1]]])
+        assert mod.rel(got, mod.oracle_logits(cfg, w, ids[i])) < mod.SPLIT_TOL
+    m.close()

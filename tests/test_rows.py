@@ -198,3 +198,40 @@ def test_batches_of_many_sizes():
         m.close()
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("recipe", ["Q4_K", "Q6_K", "Q8_0"])
+def test_quantised_decode_batch_against_the_oracle(recipe):
+    """Nine sequences in one pass, each row against the oracle's integer dots.  The same codes give the same sums: rows whose activations avoid the border of
+    two codes agree to f32 rounding, a code on a border moves an output by up to 1e-2 (one in 128 of its block's largest value)."""
+    import crane_b200
+    from oracle import ggml_quant as gq
+    from oracle.qwen3 import Qwen3Oracle
+    cfg = dict(synth.TINY_QWEN3_UNTIED, num_hidden_layers=1)
+    m = crane_b200.Qwen3Model(cfg, max_seq_len=64, max_batch=16)
+    w, qd = {}, {}
+    for name, t in synth.synth_checkpoint(cfg):
+        if "proj" in name or name == "lm_head.weight":
+            raw = gq.quantize(t, recipe)
+            m.load_tensor_ggml(name, gq.GGML_TYPE_ID[recipe], t.shape, raw)
+            w[name], qd[name] = gq.dequantize(raw, recipe, t.shape[1]), (raw, recipe)
+        else:
+            m.load_tensor(name, t)
+            w[name] = t
+    m.finalize()
+    slots = [0] + [m.seq_create() for _ in range(8)]
+    ids = synth.synth_token_ids(18, cfg["vocab_size"], "qo")
+    orc = Qwen3Oracle(cfg, w, quantised=qd)
+    want = []
+    for s in slots:
+        m.seq_select(s)
+        m.forward_step(ids[s: s + 1], 0)
+        orc.clear_kv_cache()
+        orc.forward(ids[s: s + 1], 0)
+        want.append(orc.forward(ids[9 + s: 10 + s], 1).numpy().ravel())
+    want = np.stack(want)
+    _, got = m.decode_batch(slots, ids[9:], 1, want_logits=True)
+    err = np.abs(got - want).max(1) / np.abs(want).max(1)
+    print(recipe, " ".join(f"{e:.1e}" for e in err))
+    assert (err < 2e-5).sum() >= 3 and err.max() < 3e-2
+    m.close()
