@@ -1,8 +1,10 @@
 // GGUF-quantised linears for many activation rows on the tensor cores: y[m, n] = epilogue(sum_k W[n, k] . xq[m, k]), with the integer dots of
-// candle's CPU `QMatMul::forward` (crane-core/src/ops/linear.rs:23-48) kept exact.
+// candle's CPU `QMatMul::forward` (crane-core/src/ops/linear.rs:23-48).
 //
 // Exactness.  Activations are int8 codes (xquant_kernel<true>), weights are small integers times block scales.  Both sides go through
-// tcgen05.mma kind::f16 as f16 INTEGERS, so every product is exact and the f32 accumulator holds the block's integer sum:
+// tcgen05.mma kind::f16 as f16 INTEGERS, so every product is exact and the f32 accumulator holds the block's integer sum, exactly
+// while it stays under 2^24 (a block of one sign near the ends of its ranges can reach 3.1e7 in Q4_K and 1.3e8 quarters in Q6_K: there the accumulator
+// rounds each of its 16 to 32 steps, some 1e-7 of the block):
 //   Q4_K  A = sc_j * q (<= 63 * 15: 10 bits), one accumulator per 256-element super-block; a second one takes sum_j m_j * bsum_j, the offsets'
 //         share, as a K = 16 product of [m_j | 64 m_j] and [bsum mod 64 | bsum div 64]
 //   Q6_K  A = sc * (q - 32) needs 12 bits, so it is two f16 planes, sc * ql / 4 and 4 * sc * (qh - 2), accumulated into the same columns

@@ -34,3 +34,29 @@ def test_rows_against_integer_dots(qt, m, n, k):
     assert not got[0].any()
     again = crane_b200.op_qlinear(x, raw, gq.GGML_TYPE_ID[qt], n)
     assert np.array_equal(got, again)                   # contributor order, whoever came last
+
+
+@pytest.mark.parametrize("qt", ["Q4_K", "Q6_K"])
+@pytest.mark.parametrize("m", [5, 40, 130])
+def test_sums_above_24_bits(qt, m):
+    """Scales, weights and activations of one sign near the ends of their ranges: a super-block's sum passes 2^24 (Q4_K up to 3.1e7, Q6_K 1.3e8 in the units it is
+    summed in), where the accumulator rounds instead of counting.  Sixteen to 32 partial sums of at most a unit in the last place (2^-23) each, the f32
+    terms beside them: under 40 * 2^-23 of a result that has no cancellation."""
+    import crane_b200
+    rng = np.random.default_rng(m)
+    n, k = 130, 512
+    nb = k // 256
+    half = np.frombuffer(np.float16(0.01).tobytes(), np.uint8)
+    if qt == "Q4_K":
+        sc = rng.integers(48, 64, (n, nb, 8)).astype(np.uint8)
+        head = np.concatenate([sc[..., :4] | ((sc[..., 4:] >> 4) << 6), np.zeros((n, nb, 4), np.uint8), sc[..., 4:] & 15], -1)
+        qs = (rng.integers(11, 16, (n, nb, 128)) | (rng.integers(11, 16, (n, nb, 128)) << 4)).astype(np.uint8)
+        raw = np.concatenate([np.broadcast_to(half, (n, nb, 2)), np.zeros((n, nb, 2), np.uint8), head, qs], -1)
+    else:
+        raw = np.concatenate([rng.integers(0, 256, (n, nb, 128)).astype(np.uint8), np.full((n, nb, 64), 255, np.uint8), rng.integers(96, 128, (n, nb, 16)).astype(np.uint8),
+                              np.broadcast_to(half, (n, nb, 2))], -1)
+    raw = np.ascontiguousarray(raw.reshape(n, -1))
+    x = rng.uniform(0.8, 1.0, (m, k)).astype(np.float32)
+    want = gq.qmatmul(x, raw, qt)
+    got = crane_b200.op_qlinear(x, raw, gq.GGML_TYPE_ID[qt], n)
+    assert (np.abs(got - want) <= 40 * 2.0 ** -23 * np.abs(want)).all()
