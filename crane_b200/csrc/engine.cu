@@ -1180,6 +1180,8 @@ void crane_b200_model::finalize() {
     seq_kv.assign(max_batch, 0); seq_pos.assign(max_batch, 0); seq_used.assign(max_batch, 0);
     seq_used[0] = 1;
 
+    // (hybrid models have no decode batches; a TTS model's head also leaves its normalised input row for the code predictor (GemvArgs::norm_out),
+    // which the wide head does not write)
     wide_ok = !hybrid && !is_tts && owns_stream && !use_simt && max_batch > 1;
     const int B = std::min(max_batch, wide_ok ? (int)DECODE_GROUP_MAX : 4);   // sequences per weight pass
     state_group = B;
@@ -1673,7 +1675,7 @@ void crane_b200_model::prefill(const uint32_t* ids, const float* embeds, size_t 
         if (!q_qkv) LAUNCH_OK(rmsnorm_rows_launch(stream, x, S, H, l.ln1, eps, xn, lo_xn));
         if (l.full) {
             spans.mark(SP_ATTN_QKV);
-            if (q_qkv) {   // GGUF keeps q / k / v separate and quantised (qwen3/modeling.rs:252-255): integer-dot rows, 4 at a time
+            if (q_qkv) {   // GGUF keeps q / k / v separate and quantised (qwen3/modeling.rs:252-255): integer dots
                 const int qs = nh * q_stride(), kvd = nkv * D;
                 for (int s0 = 0; s0 < S;) {               // (a few rows: groups that share their codes)
                     const int left = S - s0, B = left >= QROWS_MIN ? left : left >= 4 ? 4 : left >= 2 ? 2 : 1;

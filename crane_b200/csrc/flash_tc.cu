@@ -49,7 +49,7 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* v) {
           "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(taddr) : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// 2^x; results under 2^-126 are zero (probabilities against a largest of 2^-8 .. 1)
+// 2^x; results under 2^-126 are zero (the reference trails the running maximum by up to 8, so a row's largest probability is 1 .. 2^8)
 __device__ __forceinline__ float ex2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

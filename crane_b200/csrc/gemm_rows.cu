@@ -352,12 +352,10 @@ static int rows_launch_m(cudaStream_t st, const bf16* const* A, int P, int lda, 
     }
 }
 
-bool gemm_rows_fits(int P, int M) { return M >= 1 && P * ((M + 15) / 16 * 16) <= 256; }
-
 int gemm_rows_launch(cudaStream_t st, const bf16* const* A, int P, int lda, const bf16* W, int M, int N, int K, const GemmEpi& ep, bool pdl) {
     // f32 results leave one by one, bf16 ones in pairs of columns; of SiLU's (gate, up) rows a result takes two
     const int unit = ep.mode == EPI_STORE_F32 || ep.mode == EPI_RESID_F32 ? 1 : ep.mode == EPI_SILU_MUL_BF16 ? 4 : 2;
-    if (!gemm_rows_fits(P, M) || N <= 0 || K <= 0 || (K % 8) != 0 || (N % unit) != 0 || (lda % 8) != 0) return -1000;
+    if (M < 1 || P * ((M + 15) / 16 * 16) > 256 || N <= 0 || K <= 0 || (K % 8) != 0 || (N % unit) != 0 || (lda % 8) != 0) return -1000;
     if (P == 3) {                                   // the decode batch's epilogues
         switch (ep.mode) {
             case EPI_STORE_F32:    return rows_launch_t<3, EPI_STORE_F32>(st, A, lda, W, M, N, K, ep, pdl);

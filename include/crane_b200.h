@@ -181,7 +181,7 @@ CRANE_B200_API int crane_b200_seq_select(crane_b200_model* m, int seq);
 /* `n_steps` greedy decode rounds for `n` sequences at once: replaces setup_batch_decode + step_batch_decode x rounds +
  * extract_batch_kv (crane-core/src/models/qwen3/modeling.rs:1141-1277, crane-serve/src/engine/mod.rs:822-1062).  No left-padding,
  * mask or KV copy: each sequence attends over its own pages with its own length and position; groups of up to 64 sequences (4 in
- * the hybrid and TTS models) share one pass over the weights.  tokens[i] is consumed by seqs[i] at its cached length; tokens_out is [n, n_steps];
+ * TTS models) share one pass over the weights; hybrid models are refused.  tokens[i] is consumed by seqs[i] at its cached length; tokens_out is [n, n_steps];
  * logits_host (optional) receives the [n, vocab] f32 logits of the LAST round. */
 CRANE_B200_API int crane_b200_decode_batch(crane_b200_model* m, const int* seqs, const uint32_t* tokens, size_t n, size_t n_steps,
                                            uint32_t* tokens_out, float* logits_host);
