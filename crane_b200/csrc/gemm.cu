@@ -485,10 +485,6 @@ static GemmPlan gemm_plan(int M, int N, int K, bool split, int sms) {
     return best;
 }
 
-// Up to this many rows (one 128-row tile) the weights are the tile and the rows its columns: gemm_rows.cu.  Past 96 columns only where a cluster can
-// share a tile: 12288 x 2048 at 77 rows in two planes takes 35 us on 96 lone CTAs there, 27 with the 128-wide tiles here; 4096 x 2048 14 and 18.
-constexpr int GEMM_ROWS_MAX = 128;
-
 template <int MODE>
 static int launch_mode(cudaStream_t stream, const bf16* A, const bf16* A_lo, int lda, const bf16* W, int M, int N, int K,
                        const GemmEpi& epi, bool use_simt) {
@@ -515,10 +511,10 @@ static int launch_mode(cudaStream_t stream, const bf16* A, const bf16* A_lo, int
 int gemm_bf16_launch(cudaStream_t stream, const bf16* A, const bf16* A_lo, int lda, const bf16* W, int M, int N, int K,
                      const GemmEpi& epi, bool use_simt) {
     if (M <= 0 || N <= 0 || K <= 0 || (K % GEMM_BK) != 0 || (N % 32) != 0 || (lda % 8) != 0) return -1000;
-    const int cols = (A_lo ? 2 : 1) * ((M + 15) / 16 * 16);
-    if (!use_simt && M <= GEMM_ROWS_MAX && epi.prof == nullptr && (N <= 64 * tc_device_sms() || cols <= 96)) {
+    const int P = A_lo ? 2 : 1;
+    if (!use_simt && epi.prof == nullptr && gemm_rows_pays(epi.mode, P, M, N, K)) {       // the weights are the tile and the rows its columns
         const bf16* planes[3] = {A, A_lo, nullptr};
-        return gemm_rows_launch(stream, planes, A_lo ? 2 : 1, lda, W, M, N, K, epi, prefill_pdl());
+        return gemm_rows_launch(stream, planes, P, lda, W, M, N, K, epi, prefill_pdl());
     }
     switch (epi.mode) {
         case EPI_STORE_F32:      return launch_mode<EPI_STORE_F32>(stream, A, A_lo, lda, W, M, N, K, epi, use_simt);

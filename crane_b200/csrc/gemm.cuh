@@ -49,7 +49,8 @@ struct TmaEncoder;  // host: resolves cuTensorMapEncodeTiled once
 // `A_lo` (nullable): low-order plane of a split-precision activation operand, same shape/stride as A (see gemm.cu).
 int gemm_bf16_launch(cudaStream_t stream, const bf16* A, const bf16* A_lo, int lda, const bf16* W, int M, int N, int K,
                      const GemmEpi& epi, bool use_simt);
-// Few activation rows, 1 .. 3 bf16 planes (gemm_rows.cu); planes share lda.  gemm_bf16_launch comes here by itself where it pays.
+// Few activation rows, 1 .. 3 bf16 planes (gemm_rows.cu); planes share lda.  gemm_bf16_launch comes here by itself where gemm_rows_pays.
+bool gemm_rows_pays(int mode, int planes, int M, int N, int K);
 int gemm_rows_launch(cudaStream_t stream, const bf16* const* planes, int n_planes, int lda, const bf16* W, int M, int N, int K, const GemmEpi& epi, bool pdl);
 // f32 rows -> three bf16 planes `plane` elements apart, rows of K; RMS-normalised first when norm_w is set
 int rows_split3_launch(cudaStream_t stream, const float* x, int ldx, int M, int K, const float* norm_w, float eps, bf16* out, long long plane, bool pdl);

@@ -286,6 +286,33 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     if (warp == 2) { tc_fence_after(); tmem_dealloc(tmem, 512); }
 }
 
+// CTAs per tile: as many as the chip has room for at once (clusters live inside a GPC: sixteen of eight CTAs do not fit, and a second wave
+// doubled 2048 x 6144 at 77 rows to 37 us), each with at least 256 columns of K (`steps` of 64)
+static int rows_cluster(int tiles_n, int steps, int sms) {
+    int cl = std::max(1, std::min(std::min(8, sms / tiles_n), steps / 4));
+    while (cl > 1 && tc_max_clusters(cl) < tiles_n) --cl;
+    return cl;
+}
+
+// Is this kernel the faster one of the two for up to 128 rows?  Both stream the weights at about the same rate; the tiles of gemm.cu pay for 128 rows whatever M
+// is, while here a CTA finishes 16 rows after 16 rows, f32 results 0.4 us each, bf16 ones with or without a unary function 1.5, gate and up 5, shared by the
+// CTAs of a cluster.  us, here / gemm.cu (planes x rows: weights):
+//   f32, a cluster per tile    always, but for 1 x 97 - 128: 4096 x 1024 9.6 / 8.9 (4096 x 2048 11.4 / 14.2; 2 x 128: 4096 x 1024 10.2 / 10.5)
+//   f32, one CTA per tile      1 x 64: 12288 x 2048 13.2 / 15.4, 24576 x 4096 41.3 / 41.8; 1 x 96: 14.5 / 15.5, 46.4 / 42.5; 2 x 64: 18.0 / 18.2, 46.0 / 49.6; 2 x 96: 16384 x 2048 20.0 / 19.5
+//   others, one CTA per tile   1 x 48: gate / up 12288 x 2048 25.6 / 28.0, 24576 x 4096 65.1 / 65.5; bf16 12288 x 2048 15.1 / 14.7; 1 x 64: 30.1 / 27.8, 75.8 / 65.8, 16.2 / 14.9;
+//                              2 x 48: 26.8 / 30.7, 66.8 / 73.6, 15.9 / 18.3; 2 x 64: 35.0 / 30.6, 81.1 / 73.7, 21.0 / 18.8
+//   others, a cluster          by 16-row pieces per CTA.  One: gate / up 6144 x 1024 11.3 / 15.8, bf16 4096 x 1024 8.5 / 8.4; two: 6144 x 1024 16.3 / 15.5, 4096 x 1024
+//                              10.2 / 8.4, but 4096 x 2048 20.0 / 20.6, 8192 x 2048 13.7 / 14.2; three: 9472 x 4096 32.2 / 32.5; four: 38.6 / 32.4
+bool gemm_rows_pays(int mode, int P, int M, int N, int K) {
+    if (M > 128) return false;
+    const bool f32 = mode == EPI_STORE_F32 || mode == EPI_RESID_F32;
+    const int tiles_n = (N + 127) / 128, sms = std::min(tc_device_sms(), GR_MAX_CTAS), cl = tiles_n <= sms ? rows_cluster(tiles_n, K / 64, sms) : 1;
+    if (cl == 1) return M <= (!f32 ? 48 : P == 1 ? 80 : 64);
+    if (f32) return M <= 96 || P > 1 || K > 1024;
+    const int pieces = ((M + 15) / 16 + cl - 1) / cl;
+    return pieces <= std::max(1, std::min(3, K / 1024));
+}
+
 template <int P, int MODE, int CH>
 static int rows_launch_c(cudaStream_t st, const bf16* const* A, int lda, const bf16* W, int M, int N, int K, const GemmEpi& ep, bool pdl) {
     GemmRowsArgs a = {};
@@ -306,10 +333,7 @@ static int rows_launch_c(cudaStream_t st, const bf16* const* A, int lda, const b
     const int sms = std::min(tc_device_sms(), GR_MAX_CTAS);
     int grid;
     if (sc.tiles_n <= sms) {
-        // as many CTAs per tile as the chip has room for at once (clusters live inside a GPC: sixteen of eight CTAs do not fit, and a second wave
-        // doubled 2048 x 6144 at 77 rows to 37 us), each with at least 256 columns of K
-        a.cl = std::max(1, std::min(std::min(8, sms / sc.tiles_n), a.KB * CH / 4));
-        while (a.cl > 1 && tc_max_clusters(a.cl) < sc.tiles_n) --a.cl;
+        a.cl = rows_cluster(sc.tiles_n, a.KB * CH, sms);
         grid = sc.tiles_n * a.cl;
         if (const int e = tc_err_word(st, &a.err)) return e;
     } else {

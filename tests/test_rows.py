@@ -235,3 +235,11 @@ def test_quantised_decode_batch_against_the_oracle(recipe):
     print(recipe, " ".join(f"{e:.1e}" for e in err))
     assert (err < 2e-5).sum() >= 3 and err.max() < 3e-2
     m.close()
+
+
+# both sides of the lines between few-row tiles and 128-row tiles (gemm_rows_pays): one CTA per tile (75 tiles and more) and clusters
+@pytest.mark.parametrize("split", [False, True])
+@pytest.mark.parametrize("m,n,k", [(48, 9600, 64), (49, 9600, 64), (64, 9600, 128), (65, 9600, 128), (80, 9600, 64), (81, 9600, 64), (64, 2048, 1024), (65, 2048, 1024), (96, 2048, 1024),
+                                   (97, 2048, 1024), (128, 2048, 2048), (128, 1024, 1088), (5, 19008, 64)])
+def test_few_rows_at_the_lines(m, n, k, split):
+    test_few_rows(m, n, k, split)
