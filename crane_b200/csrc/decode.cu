@@ -1,5 +1,6 @@
 // Decode-path kernels.  See decode.cuh for the design.
 #include "decode.cuh"
+#include "tc.cuh"
 
 #include <cooperative_groups.h>
 
@@ -905,11 +906,17 @@ static int attn_decode_launch_t(cudaStream_t st, int B, const AttnDecArgs& a, bo
     cfg.numAttrs = pdl ? 2 : 1;
     return (int)cudaLaunchKernelEx(&cfg, attn_decode_kernel<D, NREP, RING>, a);
 }
+// Tile form (a CTA requests its whole range ahead of the dependency wait) while its clusters of eight, one per (sequence, KV group), run at once: in split
+// precision a tile takes an SM, in plain bf16 a third of one.  Rings beyond.  us, tile / rings, contexts of 1000 tokens:
+//   split, D = 128, 8 KV heads   1 sequence 8.6 / 8.6, 2 16.8 / 9.7, 4 25.5 / 11.5         2 KV groups of 2   3 sequences (12 clusters) 11.8 / 11.7, 4 (16) 22.1 / 13.4
+//   split, D = 256, 2 KV heads   1 sequence 13.6 / 19.1, 5 14.5 / 19.4, 8 28.1 / 23.1      8 KV heads         1 sequence 12.8 / 14.3, 2 24.7 / 17.0
+//   plain, D = 128, 8 KV heads   4 sequences 11.0 / 10.3, in groups of two (64 heads) 2 sequences (32 clusters) 13.3 / 13.9, 3 (48) 24.8 / 20.7
+//   plain, D = 256               2 KV heads, 8 sequences 17.5 / 21.6; 8 KV heads, 4 17.2 / 17.2
+static bool attn_tile_form(const AttnDecArgs& a, int pairs) { return a.kv_bits || pairs <= (a.kv_lo_off ? tc_max_clusters(ATTN_NSPLIT) : 32); }
+
 template <int D, int NREP>
 static int attn_decode_launch_r(cudaStream_t st, int B, const AttnDecArgs& a, bool pdl) {
-    // (a few sequences: the whole range of a CTA fits its tile, requested ahead of the dependency wait -- 20 us for one sequence of 1000 tokens,
-    // D = 256, where the rings take 26)
-    return a.kv_bits || B <= 4 ? attn_decode_launch_t<D, NREP, false>(st, B, a, pdl) : attn_decode_launch_t<D, NREP, true>(st, B, a, pdl);
+    return attn_tile_form(a, B * a.nkv * a.groups) ? attn_decode_launch_t<D, NREP, false>(st, B, a, pdl) : attn_decode_launch_t<D, NREP, true>(st, B, a, pdl);
 }
 
 int attn_decode_launch(cudaStream_t st, int B, int D, const AttnDecArgs& a_in, bool pdl) {
@@ -923,7 +930,7 @@ int attn_decode_launch(cudaStream_t st, int B, int D, const AttnDecArgs& a_in, b
     // splits per (sequence, KV group): all eight while they leave SMs idle, fewer as the batch itself fills the chip (two CTAs per SM)
     const int pairs = B * a.nkv * a.groups;
     a.nsplit = pairs <= 37 ? 8 : pairs <= 148 ? 4 : pairs <= 512 ? 2 : 1;
-    if (B <= 4 || a.kv_bits) a.nsplit = ATTN_NSPLIT;      // (the tile form's split is fixed)
+    if (attn_tile_form(a, pairs)) a.nsplit = ATTN_NSPLIT;      // (its split is fixed)
     if (D == 128) {
         switch (sub) {
             case 1: return attn_decode_launch_r<128, 1>(st, B, a, pdl);
