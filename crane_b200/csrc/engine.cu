@@ -199,12 +199,15 @@ struct FosovikModel;   // layer-list models (engine_fosovik.inc)
 #include "engine_sampler.inc"
 
 struct crane_b200_model {
-    // A decode batch shares one pass over the weights: up to four sequences through the GEMVs, from wide_min on all of them (up to 64) through the
-    // tensor-core linears of few rows (gemm_rows.cu, qgemm.cu).
+    // A decode batch shares one pass over the weights: 1, 2 or 4 sequences through the GEMVs, other numbers (up to 64) through the tensor-core linears of few
+    // rows (gemm_rows.cu, qgemm.cu), dense models from three on.  us per two rounds, one pass here / GEMVs (three as 2 + 1, five as 4 + 1), 4 dense or 2
+    // quantised layers of width 1024 and 4096:
+    //   dense   2: 501 / 356, 1032 / 955   3: 508 / 628, 1040 / 1666   4: 558 / 514, 1085 / 1849 (width 2048: 658 / 727)   5: 540 / 817, 1074 / 2642
+    //   Q4_K_M  2: 379 / 280, 650 / 498    3: 398 / 509, 664 / 810     4: 408 / 337, 696 / 548                             5: 405 / 578, 680 / 925
+    //   Q8_0    2: 409 / 270, 746 / 419    3: 413 / 482, 754 / 799     4: 439 / 313, 794 / 510                             5: 439 / 540, 774 / 893
     static constexpr int DECODE_GROUP_MAX = 64;
     bool wide_ok = false;                   // ... built for this handle
-    int wide_min = 5;
-    bool wide(int B) const { return wide_ok && B >= wide_min; }
+    bool wide(int B) const { return wide_ok && B >= 3 && !(any_quant && B == 4); }
     int decode_group(size_t left) const;    // sequences of the next group when `left` remain
     bf16* w3_buf = nullptr;                 // three bf16 planes of a group's activations, w3_plane elements apart
     size_t w3_plane = 0;
@@ -1194,8 +1197,6 @@ void crane_b200_model::finalize() {
         am_val = dalloc<float>((size_t)B * ARGMAX_ROW_PARTS); am_idx = dalloc<int>((size_t)B * ARGMAX_ROW_PARTS);
         TcScratch sc;                               // (taken here, not by the first decode step)
         LAUNCH_OK(tc_scratch_get(stream, (std::max(std::max(V, 2 * I), qkv_dim()) + 127) / 128, &sc));
-        // below wide_min the GEMVs (up to four sequences per pass) are as fast or faster
-        wide_min = any_quant ? 5 : 3;
     }
     x_dec = dalloc<float>((size_t)B * H);
     qkv_dec = dalloc<float>((size_t)B * qkv_dim());
@@ -1442,7 +1443,7 @@ void crane_b200_model::lm_head_last_row(const float* xrow, int advance, int B) {
 }
 
 int crane_b200_model::decode_group(size_t left) const {
-    if (wide_ok && left >= (size_t)wide_min) return (int)std::min<size_t>(left, DECODE_GROUP_MAX);
+    if (const int all = (int)std::min<size_t>(left, DECODE_GROUP_MAX); wide(all)) return all;
     int maxg = 4;
     if (!any_quant)
         for (int K : {H, I, q_dim()}) maxg = std::min(maxg, gemv_max_group(K, V, num_sms));
@@ -1500,8 +1501,8 @@ void crane_b200_model::enqueue_wide_step(int advance, int B) {
 void crane_b200_model::drop_oldest_wide_graph() {
     int held = 0, oa = 0, ob = 0;
     for (int a = 0; a < 2; ++a)
-        for (int b = wide_min; b <= DECODE_GROUP_MAX; ++b)
-            if (graph_step[a][b] && (++held == 1 || graph_last[a][b] < graph_last[oa][ob])) { oa = a; ob = b; }
+        for (int b = 3; b <= DECODE_GROUP_MAX; ++b)
+            if (wide(b) && graph_step[a][b] && (++held == 1 || graph_last[a][b] < graph_last[oa][ob])) { oa = a; ob = b; }
     if (held < GRAPH_KEEP) return;
     CUDA_OK(cudaStreamSynchronize(stream));             // (a replay of it may still be running)
     CUDA_OK(cudaGraphExecDestroy(graph_step[oa][ob]));
