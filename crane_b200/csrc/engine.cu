@@ -1048,12 +1048,12 @@ void crane_b200_model::linear_decode(int epi, bool norm, const bf16* w, const un
 }
 
 // Prefill through a quantised linear: candle's `QMatMul::forward` quantises every activation ROW to Q8_K / Q8_0 blocks and takes
-// ggml integer dots whatever the number of rows (crane-core/src/ops/linear.rs:23-48).  From QROWS_MIN rows on the integer dots run on the
+// ggml integer dots whatever the number of rows (crane-core/src/ops/linear.rs:23-48).  From qrows_min rows on the integer dots run on the
 // tensor cores (qgemm.cu); fewer rows go through the decode kernels, up to four per pass over the quantised weights.
 // `reuse_xq`: the rows were quantised by the previous call (same input, same norm) -- still checked against the block rule it used.
 void crane_b200_model::qlinear_rows(int epi, const unsigned char* qw, int qt, int N, int K, const float* xin, int ldx, const float* norm_w,
                                     float* y, int ldy, int S, bool reuse_xq) {
-    if (S >= QROWS_MIN) {
+    if (S >= qrows_min(qt)) {
         const int mode = xq_mode_for(qt);
         const QRows xr = qrows_at(xqr_buf, xqr_rows, K);
         if (!reuse_xq || mode != xqr_mode_last) {
@@ -1678,8 +1678,9 @@ void crane_b200_model::prefill(const uint32_t* ids, const float* embeds, size_t 
             spans.mark(SP_ATTN_QKV);
             if (q_qkv) {   // GGUF keeps q / k / v separate and quantised (qwen3/modeling.rs:252-255): integer dots
                 const int qs = nh * q_stride(), kvd = nkv * D;
-                for (int s0 = 0; s0 < S;) {               // (a few rows: groups that share their codes)
-                    const int left = S - s0, B = left >= QROWS_MIN ? left : left >= 4 ? 4 : left >= 2 ? 2 : 1;
+                const bool all = S >= std::max(qrows_min(l.qt_q), std::max(qrows_min(l.qt_k), qrows_min(l.qt_v)));
+                for (int s0 = 0; s0 < S;) {               // (a few rows: groups of up to four, the three linears of a group share their codes)
+                    const int left = S - s0, B = all ? left : left >= 4 ? 4 : left >= 2 ? 2 : 1;
                     const float* xr = x + (size_t)s0 * H;
                     float* yr = qkv + (size_t)s0 * qkv_dim();
                     qlinear_rows(GEMV_STORE, l.q_wq, l.qt_q, qs, H, xr, H, l.ln1, yr, qkv_dim(), B);
@@ -2773,7 +2774,7 @@ int crane_b200_op_qlinear(int device, const float* x, size_t m, size_t k, const 
         CUDA_OK(cudaMemcpy(dw, packed.data(), packed.size(), cudaMemcpyHostToDevice));
         CUDA_OK(cudaMemset(dy, 0, m * n * 4));
         if (norm_w) { CUDA_OK(cudaMalloc((void**)&dn, k * 4)); CUDA_OK(cudaMemcpy(dn, norm_w, k * 4, cudaMemcpyHostToDevice)); }
-        if (m >= (size_t)QROWS_MIN) {
+        if (m >= (size_t)qrows_min(ggml_type)) {
             CUDA_OK(cudaMalloc((void**)&dxr, qrows_bytes((int)m, (int)k)));
             const QRows xr = qrows_at(dxr, (int)m, (int)k);
             LAUNCH_OK(xquant_rows_launch(nullptr, (int)m, dx, (int)k, (int)k, dn, eps, xq_mode_for(ggml_type), xr, false));

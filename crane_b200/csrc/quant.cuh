@@ -39,10 +39,13 @@ int xquant_launch(cudaStream_t st, int B, const float* x, int ldx, int K, const 
 int qgemv_launch(cudaStream_t st, int B, const QGemvArgs& a, int num_sms, bool pdl);
 
 // ---- many rows (qgemm.cu): the same codes as f16 integers, for the tensor cores ----
+// From this many rows on: five are 4 + 1 through the GEMVs, six 4 + 2.  us per call of two layers, here / GEMVs, widths 1024, 2048, 4096:
+//   Q4_K_M  5 rows 207 / 222, 230 / 257, 325 / 372
+//   Q8_0    5 rows 213 / 210, 250 / 241, 377 / 356   6 213 / 217, 249 / 245, 374 / 366   7 214 / 277, 250 / 316, 375 / 476
+constexpr int qrows_min(int qt) { return qt == QT_Q8_0 ? 7 : 5; }
 // `rows` (a capacity) activation rows of up to K columns.  codes [rows, K] f16, elements of every group of four in the order 0, 2, 1, 3 (the order
 // in which the weights' bytes unpack in pairs); dx [blocks][ldd] the blocks' scales (256 or 32 elements); bsum [rows, K / 16] f16, per super-block
 // the eight 32-element sums mod 64 and their quotients by 64 (Q8_K codes only)
-constexpr int QROWS_MIN = 5;
 struct QRows { unsigned short* codes; float* dx; unsigned short* bsum; int ldd; };
 size_t qrows_bytes(int rows, int K);
 QRows qrows_at(unsigned char* buf, int rows, int K);

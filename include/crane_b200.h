@@ -318,7 +318,7 @@ CRANE_B200_API int crane_b200_decode_path(const crane_b200_model* m);
 CRANE_B200_API int crane_b200_op_gemm(int device, const uint16_t* a, const uint16_t* a_lo, const uint16_t* w, int M, int N, int K, int mode,
                        const float* bias, void* out_inout, int use_simt);
 
-/* y[m, n] = quantised linear of x[m, k] (host f32) through the engine's kernels (xquant + qgemv up to 4 rows, qgemm above): `raw` = n rows
+/* y[m, n] = quantised linear of x[m, k] (host f32) through the engine's kernels (xquant + qgemv up to 4 rows, Q8_0 6, qgemm above): `raw` = n rows
  * of ggml blocks (ggml_type 8 / 12 / 14), optional RMSNorm weight norm_w[k] applied first (eps).  = candle's CPU `QMatMul::forward`
  * (crane-core/src/ops/linear.rs:23-48). */
 CRANE_B200_API int crane_b200_op_qlinear(int device, const float* x, size_t m, size_t k, const void* raw, size_t raw_bytes, int ggml_type, size_t n,

@@ -60,3 +60,37 @@ def test_sums_above_24_bits(qt, m):
     want = gq.qmatmul(x, raw, qt)
     got = crane_b200.op_qlinear(x, raw, gq.GGML_TYPE_ID[qt], n)
     assert (np.abs(got - want) <= 40 * 2.0 ** -23 * np.abs(want)).all()
+
+
+@pytest.mark.parametrize("recipe", [("Q8_0", "Q8_0"), ("Q4_K", "Q8_0"), ("Q4_K", "Q6_K")])
+def test_prompts_at_the_line(recipe):
+    """Prompts of 4 to 8 tokens, where GEMVs and tensor-core linears meet (7 rows for Q8_0, 5 for K-quants), with value projections of another type than the
+    queries': each row count against the oracle; a code on the border of two moves a one-layer model's logits by up to 1e-2."""
+    import crane_b200
+    from crane_b200 import synth
+    from oracle.qwen3 import Qwen3Oracle
+    cfg = dict(synth.TINY_QWEN3_UNTIED, num_hidden_layers=1)
+    m = crane_b200.Qwen3Model(cfg, max_seq_len=64)
+    w, qd = {}, {}
+    for name, t in synth.synth_checkpoint(cfg):
+        if "proj" in name or name == "lm_head.weight":
+            qt = recipe["v_proj" in name or "down" in name]
+            raw = gq.quantize(t, qt)
+            m.load_tensor_ggml(name, gq.GGML_TYPE_ID[qt], t.shape, raw)
+            w[name], qd[name] = gq.dequantize(raw, qt, t.shape[1]), (raw, qt)
+        else:
+            m.load_tensor(name, t)
+            w[name] = t
+    m.finalize()
+    orc = Qwen3Oracle(cfg, w, quantised=qd)
+    err = []
+    for rows in (4, 5, 6, 7, 8):
+        for seed in range(3):
+            ids = synth.synth_token_ids(rows, cfg["vocab_size"], f"ql{seed}")
+            orc.clear_kv_cache()
+            m.clear_kv_cache()
+            want = orc.forward(ids, 0).numpy().ravel()
+            err.append(np.abs(m.forward_step(ids, 0).ravel() - want).max() / np.abs(want).max())
+    print(recipe, " ".join(f"{e:.1e}" for e in err))
+    assert max(err) < 3e-2 and min(err) < 1e-4
+    m.close()
