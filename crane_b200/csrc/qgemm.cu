@@ -473,14 +473,27 @@ static int qgemm_launch_t(cudaStream_t st, const unsigned char* w, const QRows& 
     return launch_k(qgemm_kernel<QT, NT>, dim3(sc.G), dim3(C::THREADS), C::SMEM, st, pdl, tmX, tmS, a);
 }
 
+// Above 32 rows: tiles of 64 activation rows, or of 128 (K-quants only), which unpack a block of weights half as often but have two stages for their operands
+// instead of three and twice the partial tile to park and add for every CTA that shares one.  Estimated us of either: super-blocks on the busiest CTA,
+// CTAs per tile, a constant; fitted to 7 linears x 14 row counts (33 .. 512) at widths 1024, 2048, 4096, within 16 % (Q4_K) and 9 % (Q6_K) of each time.
+// us, 64 / 128 wide:
+//   Q4_K  6144 x 1024   128 rows 13.3 / 16.4, 256 17.7 / 21.5, 512 27.9 / 26.3    2048 x 2048   256 14.9 / 22.3, 512 21.3 / 27.0
+//         12288 x 2048  128 27.5 / 28.8, 192 36.8 / 37.0, 256 47.4 / 37.5          24576 x 4096  64 46.6 / 58.4, 65 86.1 / 58.3, 512 325 / 198
+//   Q6_K  2048 x 6144   256 35.1 / 55.9, 512 58.6 / 63.2                           4096 x 12288  192 85.4 / 101, 256 111 / 101, 512 212 / 175
+// (Q8_0 reads an accumulator per 32 elements; at width 4096 a layer took 475 us at 128 rows and 1224 at 512 with 64, 655 and 1328 with 128.)
+static float qgemm_estimate(int qt, int nt, int M, int N, int K) {
+    const long long iters = (long long)((M + nt - 1) / nt) * ((N + 127) / 128) * (K / 256), G = std::max<long long>(1, std::min<long long>(tc_device_sms(), iters / 2));
+    const float most = (float)((iters + G - 1) / G), sharing = (float)(K / 256) * (float)G / (float)iters;
+    if (qt == QT_Q4_K) return nt == 64 ? 2.0f * most + 0.7f * sharing + 4.6f : 2.5f * most + 2.8f * sharing + 6.2f;
+    return nt == 64 ? 2.5f * most + 0.9f * sharing + 4.6f : 4.3f * most + 6.5f * sharing - 3.6f;
+}
+
 template <int QT>
 static int qgemm_launch_q(cudaStream_t st, const unsigned char* w, const QRows& x, int M, int N, int K, int epi, float* y, int ldy, bool pdl) {
     if (M <= 16) return qgemm_launch_t<QT, 16>(st, w, x, M, N, K, epi, y, ldy, pdl);
     if (M <= 32) return qgemm_launch_t<QT, 32>(st, w, x, M, N, K, epi, y, ldy, pdl);
-    // Two 64-column tiles against one of 128, per layer at width 4096: K-quants 128 rows 398 / 480 us, 512 rows 947 / 817 (the wider tile unpacks the weights
-    // half as often, but has two stages for its operands instead of three); Q8_0, which reads an accumulator per 32 elements, 475 / 655 and 1224 / 1328.
     if constexpr (QT != QT_Q8_0) {
-        if (M > 192) return qgemm_launch_t<QT, 128>(st, w, x, M, N, K, epi, y, ldy, pdl);
+        if (qgemm_estimate(QT, 128, M, N, K) < qgemm_estimate(QT, 64, M, N, K)) return qgemm_launch_t<QT, 128>(st, w, x, M, N, K, epi, y, ldy, pdl);
     }
     return qgemm_launch_t<QT, 64>(st, w, x, M, N, K, epi, y, ldy, pdl);
 }

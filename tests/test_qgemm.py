@@ -94,3 +94,10 @@ def test_prompts_at_the_line(recipe):
     print(recipe, " ".join(f"{e:.1e}" for e in err))
     assert max(err) < 3e-2 and min(err) < 1e-4
     m.close()
+
+
+@pytest.mark.parametrize("qt", ["Q4_K", "Q6_K"])
+@pytest.mark.parametrize("m,n,k", [(200, 12288, 512), (257, 12160, 512)])
+def test_wide_row_tiles(qt, m, n, k):
+    """Enough work for every block that tiles of 128 rows are taken."""
+    test_rows_against_integer_dots(qt, m, n, k)
