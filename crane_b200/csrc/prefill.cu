@@ -208,17 +208,18 @@ int rope_append_launch(cudaStream_t st, int D, const RopeAppendArgs& a) {
 }
 
 // Few keys: flash.cuh's 64-row tiles beat the 128 x 128 ones of flash_tc.cu, whose setup (TMEM, barriers, a query tile of 128 rows) and first tile take 9 - 13 us
-// whatever they hold, as long as those tiles fit the chip at once.  us, flash.cuh / flash_tc.cu, one sequence:
-//   D = 128 causal, split (16 heads)   2 rows 6.6 / 12.8, 64 9.5 / 12.1, 100 12.1 / 12.0, 192 16.3 / 13.7; 16 rows behind 64 cached 11.5 / 11.6
-//   D = 128 causal, plain              128 rows 8.0 / 8.7, 129 10.0 / 11.0, 192 11.0 / 10.5
-//   D = 256 causal, split (8 heads)    16 rows 12.0 / 13.4, 33 13.6 / 12.9
-//   D = 64 causal, split (16 heads)    64 rows 6.9 / 9.7, 129 9.9 / 11.8, 192 11.6 / 11.5
-//   D = 64 contiguous, split           64 rows 5.5 / 8.4, 256 10.0 / 10.2, 320 11.5 / 11.7, 400 14.0 / 13.5; four images of 160: 11.7 / 11.1 (192 tiles of 64 rows)
-//   D = 64 contiguous, plain           224 rows 6.4 / 8.2, 512 9.6 / 10.2, 1024 23.8 / 14.7
-//   D = 128 contiguous, split          64 rows 8.6 / 10.0, 224 15.7 / 12.7
+// whatever they hold, as long as those tiles fit the chip at once.  The lines are from whole calls, both kernels in turn on one state (a launch timed
+// by itself, after its like, flatters flash.cuh in plain bf16 and flash_tc.cu in split precision).  us, flash.cuh / flash_tc.cu:
+//   D = 128 causal, split   prompt of 2 rows, 2 layers of width 2048 195 / 219, 64 242 / 254, 128 262 / 276, 160 329 / 331, 176 334 / 332; 8 rows behind 150 210 / 222
+//   D = 128 causal, plain   2 rows 198 / 205, 4 behind 60 206 / 206, 16 213 / 207, 64 234 / 223, 128 265 / 244
+//   D = 256 causal, split   4 hybrid layers, 3 rows 311 / 316, 16 339 / 333, 64 442 / 432
+//   D = 64 causal           2 layers, split 64 rows 189 / 198, 160 236 / 242, 192 239 / 240, 256 242 / 240; plain 64 191 / 194, 256 215 / 218
+//   D = 64 contiguous       vision tower, split 64 patches 1564 / 1682, 320 2657 / 2728, 360 2713 / 2740, 396 3060 / 2951; 3 images of 168 2795 / 2794; plain 320 2208 / 2301,
+//                           360 2302 / 2368, 440 2562 / 2568
+//   D = 128 contiguous      (a launch by itself, split) 64 rows 8.6 / 10.0, 224 15.7 / 12.7
 static bool flash_few_keys(int D, bool causal, bool split, const FlashArgs& a) {
     const int rows = a.seq_len ? a.max_len : a.S, keys = a.seq_len ? (causal ? a.max_kv : a.max_len) : (causal ? a.kv_offset : 0) + a.S;
-    const int most = D == 256 ? 32 : D == 128 ? (split ? 96 : 160) : causal ? 160 : split ? 320 : 512;
+    const int most = D == 64 ? (causal ? (split ? 192 : 256) : (split ? 360 : 440)) : D == 128 ? (!split ? 8 : causal ? 160 : 96) : 8;
     return keys > 0 && keys <= most && (long long)((rows + 63) / 64) * a.nh * (a.seq_len ? a.nseq : 1) <= tc_device_sms();
 }
 
