@@ -1158,7 +1158,7 @@ def main():
         return
 
     peaks = load_peaks()
-    traffic = None           # DRAM bytes of one decode launch measured by ncu (tools/profile.sh + tools/summarize_ncu.py traffic)
+    traffic = None           # DRAM bytes of one decode launch measured by ncu (tools/summarize_ncu.py traffic)
     for tf in ("r02_traffic.json", "r01_traffic.json"):
         try:
             traffic = json.load(open(os.path.join(ROOT, "profiles", tf)))

@@ -1,5 +1,4 @@
-"""GPU, world_size 2 (needs two devices: `gpurun --gpus 2 -- python -m pytest tests/test_multi_gpu.py -m gpu`; skipped on a one-GPU
-box): config 4's data path -- sequences sharded over ranks, one handle per GPU, NCCL all-gather of every round's logits and tokens
+"""GPU, world_size 2 (skipped where there are not two devices): config 4's data path -- sequences sharded over ranks, one handle per GPU, NCCL all-gather of every round's logits and tokens
 through crane_b200_comm_init / crane_b200_decode_batch_gather -- against the CPU oracle run sequence by sequence."""
 import numpy as np
 import pytest

@@ -1,5 +1,5 @@
 // Standalone GEMV micro-benchmark (compiled ON the GPU box so pipeline parameters can be swept in one call):
-//   nvcc -gencode arch=compute_100a,code=sm_100a -O3 -std=c++17 -DGV_WARPS=8 -DGV_DEPTH=5 tools/gemv_bench.cu -o /tmp/gb && /tmp/gb
+//   nvcc -gencode arch=compute_100a,code=sm_100a -O3 -std=c++17 -DGV_WARPS=8 -DGV_DEPTH=5 tools/gemv_bench.cu crane_b200/csrc/tc.cu crane_b200/csrc/tc_scratch.cu -o /tmp/gb && /tmp/gb
 // 1) isolated kernels per shape (weights rotated through > L2 worth of copies), 2) the PDL-chained weight stream of a whole
 // Qwen3-VL-2B decode step (28 x [qkv, o, gate_up, down] + lm_head, attention omitted).
 #include "../crane_b200/csrc/decode.cu"

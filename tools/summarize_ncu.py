@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Turn ncu outputs brought back in gpurun_out/ into the small tracked summaries under profiles/.
+"""Turn ncu outputs into the small tracked summaries under profiles/.
   launches CSV (gpu__time_duration per launch)  -> per-kernel totals / shares
   .ncu-rep (ncu --set full)                     -> selected raw metrics per captured launch"""
 import collections
@@ -68,13 +68,13 @@ def _bytes(d, key):
 
 
 def traffic(prefix, dst):
-    """DRAM bytes of one decode step from the full captures prof_gemv_/prof_lmhead_/prof_attn_<tag>.ncu-rep:
+    """DRAM bytes of one decode step from the full captures prof_gemv_/prof_lmhead_/prof_attn_<tag>.ncu-rep in the working folder:
     28 x (qkv + o + gate_up + down GEMV + attention) + lm_head, each = dram__bytes_read.sum + dram__bytes_write.sum of its launch."""
     import json
     tag = prefix
-    gemv = _raw(f"gpurun_out/prof_gemv_{tag}.ncu-rep")
-    head = _raw(f"gpurun_out/prof_lmhead_{tag}.ncu-rep")
-    attn = _raw(f"gpurun_out/prof_attn_{tag}.ncu-rep")
+    gemv = _raw(f"prof_gemv_{tag}.ncu-rep")
+    head = _raw(f"prof_lmhead_{tag}.ncu-rep")
+    attn = _raw(f"prof_attn_{tag}.ncu-rep")
     per = lambda d: _bytes(d, "dram__bytes_read.sum") + _bytes(d, "dram__bytes_write.sum")
     names = [d["Kernel Name"][0] for d in gemv]
     layer = sum(per(d) for d in gemv[:4])                      # four consecutive GEMVs of a layer (any rotation of qkv, o, gate_up, down)
