@@ -60,7 +60,8 @@ struct EngineError {
                            r__ > 0 ? cudaGetErrorString((cudaError_t)r__) : "", __FILE__, __LINE__);          \
     } while (0)
 
-// Results leave for the caller: the tensor-core kernels bound their waits (tc.cuh), and a kernel that gave one up has left garbage behind.
+// Results leave for the caller: attention, few-row and quantised linears on the tensor cores bound their waits (TcWait, tc.cuh), and a kernel that gave one up
+// has left garbage behind.
 // Called on an idle stream, ahead of everything that a good result is followed by (a sequence's length, a return code).
 void check_waits(cudaStream_t st) {
     if (tc_take_wait_error(st)) fail(CRANE_B200_CUDA_ERROR, "a tensor-core kernel's wait ran out (results discarded)");
