@@ -13,20 +13,18 @@ namespace cb {
 static const int g_gemm_bn = [] { const char* e = getenv("CRANE_B200_GEMM_BN"); return e ? atoi(e) : 0; }();
 
 // =====================================================================================
-// Fused epilogue of one warp: a 32-row x 32-column accumulator block (lane = row, as tcgen05.ld delivers it).
-// The arithmetic (bias / activation / SiLU*up / bf16 split) runs on the lane's own row; the results are then transposed
-// through a 32 x 144 B shared-memory patch so that every global store (and the residual read) covers whole 128-byte rows --
-// row-per-lane stores cost 32 LSU wavefronts per instruction and made the epilogue as long as the main loop.
+// Row-per-lane stores of 32 finished columns (bias already added), for the SIMT debugging kernel.
 // =====================================================================================
-// Row-per-lane stores of 32 finished columns (bias already added): the bf16 modes of the tcgen05 epilogue and every mode of the
-// SIMT debugging kernel.
 template <int MODE>
 __device__ __forceinline__ void epi_store32(const GemmEpi& ep, int m, int n, float* v, bool ok) {
     if (!ok) return;
     if constexpr (MODE == EPI_STORE_F32 || MODE == EPI_RESID_F32) {
-        float* o = reinterpret_cast<float*>(ep.out) + (size_t)m * ep.ldo + n;
+        float4* o = reinterpret_cast<float4*>(reinterpret_cast<float*>(ep.out) + (size_t)m * ep.ldo + n);
+        float4 x[8];
 #pragma unroll
-        for (int j = 0; j < 32; ++j) o[j] = (MODE == EPI_RESID_F32 ? o[j] : 0.f) + v[j];
+        for (int j = 0; j < 8; ++j) x[j] = MODE == EPI_RESID_F32 ? o[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] = make_float4(x[j].x + v[4 * j], x[j].y + v[4 * j + 1], x[j].z + v[4 * j + 2], x[j].w + v[4 * j + 3]);
     } else if constexpr (MODE == EPI_SILU_MUL_BF16) {
         const size_t off = (size_t)m * ep.ldo + (n >> 1);
         uint32_t p[8], q[8];
@@ -61,11 +59,23 @@ __device__ __forceinline__ void epi_store32(const GemmEpi& ep, int m, int n, flo
     }
 }
 
-constexpr int EPI_PITCH = 144;                     // bytes per staged row (128 B payload + 16 B skew)
-constexpr int EPI_WARP_BYTES = 32 * EPI_PITCH;
+// =====================================================================================
+// Fused epilogue of one warp: 32 rows x 32 accumulator columns at a time (lane = row, as tcgen05.ld delivers them).  The arithmetic (bias, scale, gate,
+// activation, bf16 split) runs on the lane's own row; the results go to 2 KB patches of shared memory in TMA's swizzled order without bank
+// conflicts, and leave as TMA stores, the residual's as TMA adds: the old values never pass through the SM, rows and columns outside the matrix are dropped by the
+// copy engine.  (Row-per-lane stores cost 32 LSU wavefronts per instruction, and reading the residual first put a round trip to the L2 into every
+// block of columns.)
+// A turn of the loop is 32 columns and is not unrolled further: a CTA with one tile runs this code once or twice, out of a cold instruction cache (64 unrolled
+// columns: gate / up of a 77-row turn 26.9 us instead of 25.1), while a turn's own chain (TMEM load, proxy fence, store) is too long for 16
+// (784 x 4096 with GELU: 25.5 us, 21.6 with 32).
+// A warp has one patch of its own.  The epilogue of a CTA's last segment, which nothing runs beside, has four in the operand ring, free by
+// then.  32 KB of own patches instead of 16 measured slower (320 x 6144 x 4096 34.9 us, 32.3 with 16): the kernels before and after a linear want the
+// rest of the shared memory.
+// =====================================================================================
+constexpr int EPI_WARPS = 8;
+constexpr int EPI_PATCH = 2048;
 
-template <int MODE>
-__device__ __forceinline__ void epi_block(const GemmEpi& ep, uint8_t* stg, int m_base, int M, int n, float* v, int lane) {
+__device__ __forceinline__ void epi_linear(const GemmEpi& ep, int m, int M, int n, float* v) {
     if (ep.bias != nullptr) {
 #pragma unroll
         for (int j = 0; j < 32; j += 4) {
@@ -80,8 +90,8 @@ __device__ __forceinline__ void epi_block(const GemmEpi& ep, uint8_t* stg, int m
             v[j] *= c.x; v[j + 1] *= c.y; v[j + 2] *= c.z; v[j + 3] *= c.w;
         }
     }
-    if (ep.gate != nullptr && m_base + lane < M) {      // a lane holds 32 neighbouring columns of its own row
-        const float* g = ep.gate + (size_t)(m_base + lane) * ep.ldg + n;
+    if (ep.gate != nullptr && m < M) {                  // a lane holds 32 neighbouring columns of its own row
+        const float* g = ep.gate + (size_t)m * ep.ldg + n;
 #pragma unroll
         for (int j = 0; j < 32; j += 4) {
             float4 z = *reinterpret_cast<const float4*>(g + j);
@@ -89,47 +99,112 @@ __device__ __forceinline__ void epi_block(const GemmEpi& ep, uint8_t* stg, int m
             v[j] *= 1.f / (1.f + expf(-z.x)); v[j + 1] *= 1.f / (1.f + expf(-z.y)); v[j + 2] *= 1.f / (1.f + expf(-z.z)); v[j + 3] *= 1.f / (1.f + expf(-z.w));
         }
     }
-    if constexpr (MODE == EPI_STORE_F32 || MODE == EPI_RESID_F32) {
-        uint8_t* mine = stg + lane * EPI_PITCH;
-        // the residual rows first (independent loads, all in flight together), then the transpose
-        float4 y[8];
-        if constexpr (MODE == EPI_RESID_F32) {
-#pragma unroll
-            for (int it = 0; it < 8; ++it) {
-                const int m = m_base + it * 4 + (lane >> 3);
-                y[it] = (m < M) ? *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(ep.out) + (size_t)m * ep.ldo + n + (lane & 7) * 4)
-                                : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(mine + j * 4) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+}
+
+struct EpiPatch {
+    uint8_t* base;
+    bool ring;          // four patches, else one
+    int n = 0;          // stores so far
+    // the next patch, its last store's reads done
+    __device__ __forceinline__ uint8_t* take(int lane) const {
+        if (lane == 0) { if (ring) tma_store_wait_read<3>(); else tma_store_wait_read<0>(); }
         __syncwarp();
+        return base + (ring ? (n & 3) * EPI_PATCH : 0);
+    }
+    // written by every lane: lane 0 may hand it to the copy engine
+    __device__ __forceinline__ void ready() {
+        fence_proxy_async();
+        __syncwarp();
+        ++n;
+    }
+};
+// BN accumulator columns of rows m0 .. m0 + 31, shared by the row quarter's warps (`part` of EPI_WARPS / 4); load(c, v) gives columns 32 c .. 32 c + 31.
+// A patch is 16 f32 columns, 32 columns of one bf16 plane, or (gate / up, whose 32 columns are 16 results) 16 of both planes.
+template <int MODE, int BN, typename Load>
+__device__ __forceinline__ void epi_rows(const GemmEpi& ep, const CUtensorMap& tmO, const CUtensorMap& tmOlo, EpiPatch& patch, int m0, int M, int n0, int N, int part,
+                                         int lane, Load&& load) {
+    constexpr bool F32 = MODE == EPI_STORE_F32 || MODE == EPI_RESID_F32, GLU = MODE == EPI_SILU_MUL_BF16;
+#pragma unroll 1
+    for (int c = part; c < BN / 32; c += EPI_WARPS / 4) {
+        const int n = n0 + 32 * c;
+        if (n >= N) break;
+        float v[32];
+        load(c, v);
+        epi_linear(ep, m0 + lane, M, n, v);
+        if constexpr (F32) {
 #pragma unroll
-        for (int it = 0; it < 8; ++it) {           // 4 rows x 128 B per instruction
-            const int r = it * 4 + (lane >> 3), c4 = lane & 7;
-            const int m = m_base + r;
-            if (m < M) {
-                float4 x = *reinterpret_cast<const float4*>(stg + r * EPI_PITCH + c4 * 16);
-                if constexpr (MODE == EPI_RESID_F32) { x.x += y[it].x; x.y += y[it].y; x.z += y[it].z; x.w += y[it].w; }
-                *reinterpret_cast<float4*>(reinterpret_cast<float*>(ep.out) + (size_t)m * ep.ldo + n + c4 * 4) = x;
+            for (int g = 0; g < 2; ++g) {
+                uint8_t* p = patch.take(lane);
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    *reinterpret_cast<float4*>(p + sw64_off(lane, j)) = make_float4(v[16 * g + 4 * j], v[16 * g + 4 * j + 1], v[16 * g + 4 * j + 2], v[16 * g + 4 * j + 3]);
+                patch.ready();
+                if (lane == 0) {
+                    if constexpr (MODE == EPI_RESID_F32) tma_add_2d(&tmO, p, n + 16 * g, m0);
+                    else tma_store_2d(&tmO, p, n + 16 * g, m0);
+                    tma_store_commit();
+                }
+            }
+        } else if constexpr (GLU) {
+            if (m0 + lane >= M) {                       // rows behind the last are zeros, which the division takes 100 cycles each for
+#pragma unroll
+                for (int j = 0; j < 32; j += 2) v[j] = 1.f;
+            }
+            if (ep.glu_limit == 0.f) {                  // (outside the loop: sixteen independent exponentials and divisions)
+#pragma unroll
+                for (int j = 0; j < 16; ++j) v[j] = silu_f(v[2 * j]) * v[2 * j + 1];
+            } else {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) v[j] = glu_pair_f(v[2 * j], v[2 * j + 1], ep.glu_limit);
+            }
+            uint32_t hi[8], lo[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) split_bf16x2(v[2 * j], v[2 * j + 1], hi[j], lo[j]);
+            uint8_t* p = patch.take(lane);
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                *reinterpret_cast<uint4*>(p + sw32_off(lane, j)) = make_uint4(hi[4 * j], hi[4 * j + 1], hi[4 * j + 2], hi[4 * j + 3]);
+                *reinterpret_cast<uint4*>(p + EPI_PATCH / 2 + sw32_off(lane, j)) = make_uint4(lo[4 * j], lo[4 * j + 1], lo[4 * j + 2], lo[4 * j + 3]);
+            }
+            patch.ready();
+            if (lane == 0) {
+                tma_store_2d(&tmO, p, n / 2, m0);
+                if (ep.out_lo != nullptr) tma_store_2d(&tmOlo, p + EPI_PATCH / 2, n / 2, m0);
+                tma_store_commit();
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+                if constexpr (MODE == EPI_GELU_ERF_BF16) v[j] = gelu_erf_f(v[j]);
+                else if constexpr (MODE == EPI_GELU_TANH_BF16) v[j] = gelu_tanh_f(v[j]);
+                else if constexpr (MODE == EPI_RELU2_BF16) { v[j] = fmaxf(v[j], 0.f); v[j] *= v[j]; }
+            }
+            uint32_t hi[16], lo[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) split_bf16x2(v[2 * j], v[2 * j + 1], hi[j], lo[j]);
+            uint8_t* p = patch.take(lane);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(p + sw64_off(lane, j)) = make_uint4(hi[4 * j], hi[4 * j + 1], hi[4 * j + 2], hi[4 * j + 3]);
+            patch.ready();
+            if (lane == 0) { tma_store_2d(&tmO, p, n, m0); tma_store_commit(); }
+            if (ep.out_lo != nullptr) {
+                p = patch.take(lane);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(p + sw64_off(lane, j)) = make_uint4(lo[4 * j], lo[4 * j + 1], lo[4 * j + 2], lo[4 * j + 3]);
+                patch.ready();
+                if (lane == 0) { tma_store_2d(&tmOlo, p, n, m0); tma_store_commit(); }
             }
         }
-        __syncwarp();                              // the patch is rewritten by the next block
-    } else {
-        // bf16 outputs: a lane's 32 (16) values are 64 (32) contiguous bytes = whole sectors already -- stored straight from registers
-        epi_store32<MODE>(ep, m_base + lane, n, v, m_base + lane < M);
     }
 }
 
 // =====================================================================================
-// tcgen05 kernel: persistent, stream-K over (tile, k-step) iterations, 256 threads per CTA, one CTA per SM
+// tcgen05 kernel: persistent, stream-K over (tile, k-step) iterations, 384 threads per CTA, one CTA per SM
 //   warp 0 : TMA producer (one elected lane)       warp 1 : MMA issuer (one elected lane)
-//   warp 2 : TMEM allocator / deallocator           warps 4-7 : epilogue (TMEM lane quadrant = warp % 4)
+//   warp 2 : TMEM allocator / deallocator           warps 4-11 : epilogue (TMEM lane quadrant = warp % 4, two warps share its columns)
 //
 // Why stream-K.  At the prefill shapes of this engine (M = 454 text rows, 784 patches) a 128 x BN grid of output tiles is either too
-// few CTAs (BN = 256: 32-64 tiles for N = 2048-4096) or, with narrow tiles, bound by L2 -> SM operand traffic: measured (tools/
-// gemm_probe.py) a k-step costs ~325 ns whether BN is 64, 128 or 256, i.e. the ~12 TB/s the L2 can hand out, while the tensor pipe
-// needs 32 / 64 / 128 cycles per MMA.  Only BN = 256 tiles are MMA-bound, so the work is cut the other way: the iteration space
+// few CTAs (BN = 256: 32-64 tiles for N = 2048-4096) or, with narrow tiles, bound by operand traffic; so the work can be cut the other way: the iteration space
 // tiles x k-steps is dealt out evenly, in order, to min(#SMs, ...) CTAs; a CTA whose range starts or ends inside a tile owns a
 // PARTIAL sum of that tile.  Partials go to a workspace; the contributor that arrives last adds them IN CONTRIBUTOR ORDER (so the
 // result does not depend on who was last: bitwise reproducible) and runs the fused epilogue.  Nobody ever waits for another CTA.
@@ -146,17 +221,18 @@ struct GemmCfg {
     static constexpr int B_BYTES = BN * GEMM_BK * 2;
     static constexpr int STAGE_BYTES = A_BYTES * (SPLIT ? 2 : 1) + B_BYTES;     // [A hi | A lo (SPLIT) | B]
     static constexpr int STAGES = (GEMM_STAGE_BUDGET / STAGE_BYTES) < 8 ? (GEMM_STAGE_BUDGET / STAGE_BYTES) : 8;
-    static constexpr int EPI_BYTES = 4 * EPI_WARP_BYTES;                        // transpose patches of the four epilogue warps
+    static constexpr int EPI_BYTES = EPI_WARPS * EPI_PATCH;                     // store patches of the epilogue warps
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_BYTES + 1024 /*align*/ + 256 /*barriers*/;
     static constexpr int TMEM_COLS = 2 * BN;
 };
 
 // SPLIT: the activation operand comes as two bf16 planes A = hi + lo (lo = bf16(x - hi), ~16 mantissa bits together); the
 // weight tile is fetched once and multiplied by both, accumulating into the same TMEM columns: D = hi.W^T + lo.W^T.
+// (Bounds: 384 threads, but no more registers than 512 would leave each: the row kernels beside a linear need some too.)
 template <int BN, int MODE, bool SPLIT>
-__global__ void __launch_bounds__(256, 1)
+__global__ void __launch_bounds__(512, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmAlo, const __grid_constant__ CUtensorMap tmB,
-               GemmEpi ep, int M, int N, int K, TcSched sc) {
+               const __grid_constant__ CUtensorMap tmO, const __grid_constant__ CUtensorMap tmOlo, GemmEpi ep, int M, int N, int K, TcSched sc, int* err) {
     using Cfg = GemmCfg<BN, SPLIT>;
     constexpr int STAGES = Cfg::STAGES;
     extern __shared__ uint8_t smem_raw[];
@@ -165,9 +241,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     uint64_t* full_bar = reinterpret_cast<uint64_t*>(epi_smem + Cfg::EPI_BYTES);
     uint64_t* empty_bar = full_bar + STAGES;
     uint64_t* tmem_full_bar = empty_bar + STAGES;      // [2] accumulator b complete
-    uint64_t* tmem_empty_bar = tmem_full_bar + 2;      // [2] accumulator b drained by the four epilogue warps
+    uint64_t* tmem_empty_bar = tmem_full_bar + 2;      // [2] accumulator b drained by the epilogue warps
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty_bar + 2);
     int* last_flag = reinterpret_cast<int*>(tmem_slot + 1);
+    int* gave_up = last_flag + 1;
+    const TcWait wait{gave_up, err};
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int cta = blockIdx.x;
@@ -185,7 +263,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         if (SPLIT) tma_prefetch_desc(&tmAlo);
         tma_prefetch_desc(&tmB);
         for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(&tmem_full_bar[b], 1); mbar_init(&tmem_empty_bar[b], 4); }
+        for (int b = 0; b < 2; ++b) { mbar_init(&tmem_full_bar[b], 1); mbar_init(&tmem_empty_bar[b], EPI_WARPS); }
+        *gave_up = 0;
         fence_barrier_init();
     }
     if (warp == 2) { tmem_alloc(tmem_slot, Cfg::TMEM_COLS); tmem_relinquish(); }
@@ -196,166 +275,160 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     if (threadIdx.x == 0) stamp(1);                 // setup done
 
     pdl_launch_dependents();                        // the next kernel may begin its own setup / weight prefetch now
-    auto tile_origin = [&](int it, int& m0, int& n0) {
-        const int t = it / KB;
-        m0 = (t % sc.tiles_m) * GEMM_BM;
-        n0 = (t / sc.tiles_m) * BN;
-    };
     if (warp == 0) {
         if (lane == 0) {
+            // A step takes the tensor pipe 130 to 530 ns and the issuing thread should take far less: the tile's coordinates are divided out once per
+            // segment, not per step.  (Four integer divisions a step made a step cost 325 - 420 ns whatever the tile's width: 1111 x 2048 x 6144 in
+            // plain bf16 took 39.9 us, 31.2 without them.)
+            constexpr int B_OFF = Cfg::A_BYTES * (SPLIT ? 2 : 1);
             // weights do not depend on the predecessor kernel: their first tiles go out before the dependency wait
             const int npre = ep.w_dynamic ? 0 : min(it_end - it_begin, STAGES);
+            int t = it_begin / KB, kb = it_begin - t * KB, n0 = t / sc.tiles_m * BN;
             for (int i = 0; i < npre; ++i) {
-                int m0, n0;
-                tile_origin(it_begin + i, m0, n0);
-                uint8_t* st = smem + i * Cfg::STAGE_BYTES;
                 mbar_arrive_expect_tx(&full_bar[i], Cfg::STAGE_BYTES);
-                tma_load_2d(st + Cfg::A_BYTES * (SPLIT ? 2 : 1), &tmB, &full_bar[i], ((it_begin + i) % KB) * GEMM_BK, n0);
+                tma_load_2d(smem + i * Cfg::STAGE_BYTES + B_OFF, &tmB, &full_bar[i], kb * GEMM_BK, n0);
+                if (++kb == KB) { kb = 0; ++t; n0 = t / sc.tiles_m * BN; }
             }
             pdl_wait();
-            int s = 0; uint32_t ph = 0;
-            for (int it = it_begin; it < it_end; ++it) {
-                int m0, n0;
-                tile_origin(it, m0, n0);
-                const int kc = (it % KB) * GEMM_BK;
-                uint8_t* a_dst = smem + s * Cfg::STAGE_BYTES;
-                const bool pre = it - it_begin < npre;
-                if (!pre) {
-                    mbar_wait(&empty_bar[s], ph ^ 1);
-                    mbar_arrive_expect_tx(&full_bar[s], Cfg::STAGE_BYTES);
-                    tma_load_2d(a_dst + Cfg::A_BYTES * (SPLIT ? 2 : 1), &tmB, &full_bar[s], kc, n0);
+            int s = 0, left = npre; uint32_t ph = 0;
+            for (int it = it_begin; it < it_end;) {
+                t = it / KB;
+                const int seg_end = min(it_end, (t + 1) * KB), nt = t / sc.tiles_m, m0 = (t - nt * sc.tiles_m) * GEMM_BM;
+                n0 = nt * BN;
+                int kc = (it - t * KB) * GEMM_BK;
+                for (; it < seg_end; ++it, kc += GEMM_BK) {
+                    uint8_t* a_dst = smem + s * Cfg::STAGE_BYTES;
+                    if (left > 0) --left;
+                    else {
+                        wait(&empty_bar[s], ph ^ 1);
+                        mbar_arrive_expect_tx(&full_bar[s], Cfg::STAGE_BYTES);
+                        tma_load_2d(a_dst + B_OFF, &tmB, &full_bar[s], kc, n0);
+                    }
+                    tma_load_2d(a_dst, &tmA, &full_bar[s], kc, m0);
+                    if (SPLIT) tma_load_2d(a_dst + Cfg::A_BYTES, &tmAlo, &full_bar[s], kc, m0);
+                    if (++s == STAGES) { s = 0; ph ^= 1; }
                 }
-                tma_load_2d(a_dst, &tmA, &full_bar[s], kc, m0);
-                if (SPLIT) tma_load_2d(a_dst + Cfg::A_BYTES, &tmAlo, &full_bar[s], kc, m0);
-                if (++s == STAGES) { s = 0; ph ^= 1; }
             }
+            wait.drain();
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = make_idesc_bf16(GEMM_BM, BN);
-            int s = 0; uint32_t ph = 0;
-            int seg = 0;
-            for (int it = it_begin; it < it_end; ++seg) {
-                const int seg_end = min(it_end, (it / KB + 1) * KB);
-                const int b = seg & 1;
-                mbar_wait(&tmem_empty_bar[b], ((seg >> 1) & 1) ^ 1);      // the epilogue has drained this accumulator (first two: free)
+        constexpr uint32_t idesc = make_idesc_bf16(GEMM_BM, BN);
+        int s = 0; uint32_t ph = 0;
+        int seg = 0;
+        for (int it = it_begin; it < it_end; ++seg) {
+            const int seg_end = min(it_end, (it / KB + 1) * KB);
+            const int b = seg & 1;
+            wait(&tmem_empty_bar[b], ((seg >> 1) & 1) ^ 1);           // the epilogue has drained this accumulator (first two: free)
+            tc_fence_after();
+            const uint32_t acc = tmem_base + (uint32_t)(b * BN);
+            for (int i = it; i < seg_end; ++i) {
+                wait(&full_bar[s], ph);
                 tc_fence_after();
-                const uint32_t acc = tmem_base + (uint32_t)(b * BN);
-                for (int i = it; i < seg_end; ++i) {
-                    mbar_wait(&full_bar[s], ph);
-                    tc_fence_after();
-                    if (i == it_begin) stamp(2);        // first operands landed
-                    const uint32_t a_addr = smem_u32(smem + s * Cfg::STAGE_BYTES);
-                    const uint64_t adesc = make_smem_desc_sw128(a_addr);
-                    const uint64_t aldesc = make_smem_desc_sw128(a_addr + Cfg::A_BYTES);
-                    const uint64_t bdesc = make_smem_desc_sw128(a_addr + Cfg::A_BYTES * (SPLIT ? 2 : 1));
+                if (lane == 0 && i == it_begin) stamp(2);             // first operands landed
+                const uint32_t a_addr = smem_u32(smem + s * Cfg::STAGE_BYTES);
+                const uint64_t adesc = make_smem_desc_sw128(a_addr);
+                const uint64_t aldesc = make_smem_desc_sw128(a_addr + Cfg::A_BYTES);
+                const uint64_t bdesc = make_smem_desc_sw128(a_addr + Cfg::A_BYTES * (SPLIT ? 2 : 1));
+                if (elect_one()) {
 #pragma unroll
                     for (int k = 0; k < GEMM_BK / 16; ++k) {
                         // +32 B per K=16 step inside the 128 B swizzle atom -> +2 in the >>4-encoded start address
                         umma_bf16(acc, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc, (uint32_t)((i != it) | (k != 0)));
                         if (SPLIT) umma_bf16(acc, aldesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc, 1u);
                     }
-                    umma_commit(&empty_bar[s]);         // frees the smem stage once these MMAs retire
-                    if (++s == STAGES) { s = 0; ph ^= 1; }
+                    umma_commit(&empty_bar[s]);                       // frees the smem stage once these MMAs retire
+                    if (i == seg_end - 1) umma_commit(&tmem_full_bar[b]);         // this segment's accumulator is complete
                 }
-                umma_commit(&tmem_full_bar[b]);         // this segment's accumulator is complete
-                it = seg_end;
+                __syncwarp();
+                if (++s == STAGES) { s = 0; ph ^= 1; }
             }
-            stamp(3);                                   // last MMA issued
+            it = seg_end;
         }
+        if (lane == 0) stamp(3);                                      // last MMA issued
     } else if (warp >= 4) {
+        if (threadIdx.x == 128) { tma_prefetch_desc(&tmO); tma_prefetch_desc(&tmOlo); }
         pdl_wait();                                 // the epilogue reads / overwrites activations of the predecessor too
-        const int q = warp & 3;
-        uint8_t* stg = epi_smem + q * EPI_WARP_BYTES;
+        const int q = warp & 3, part = (warp - 4) >> 2;
+        EpiPatch patch{epi_smem + (warp - 4) * EPI_PATCH, false};
         constexpr int CHUNKS = BN / 32;
         constexpr size_t TILE_F = (size_t)GEMM_BM * BN;
         int seg = 0;
         for (int it = it_begin; it < it_end; ++seg) {
             const int seg_end = min(it_end, (it / KB + 1) * KB);
             const int t = it / KB, kb0 = it % KB, kb1 = kb0 + (seg_end - it);
-            const int m0 = (t % sc.tiles_m) * GEMM_BM, n0 = (t / sc.tiles_m) * BN;
+            const int m0 = (t % sc.tiles_m) * GEMM_BM + q * 32, n0 = (t / sc.tiles_m) * BN;
             const int b = seg & 1;
             const uint32_t acc = tmem_base + (uint32_t)(b * BN) + ((uint32_t)(q * 32) << 16);
             const bool sole = kb0 == 0 && kb1 == KB;
-            mbar_wait(&tmem_full_bar[b], (seg >> 1) & 1);
+            const int c_first = sched_owner(sc, t * KB), c_last = sched_owner(sc, t * KB + KB - 1);
+            // a shared tile whose other contributors have all arrived already is finished without parking this part (read while the MMAs run)
+            if (!sole && threadIdx.x == 128) *last_flag = ld_acquire(&sc.counters[t]) == c_last - c_first;
+            wait(&tmem_full_bar[b], (seg >> 1) & 1);
             tc_fence_after();
             if (threadIdx.x == 128 && seg == 0) stamp(4);   // first accumulator ready
-            if (sole) {
+            bool finish = sole;
+            if (!sole) {
+                named_bar_sync(1, 32 * EPI_WARPS);
+                finish = *last_flag;
+                if (!finish) {
+                    // park it.  A 32 x 32 block of (row = lane, column j) is stored as 8 rows of 32 float4: the float4
+                    // of lane l in row k holds columns 4k .. 4k+3 of row l, so every store / reload instruction moves 512 contiguous bytes
+                    float* mine = sc.ws + (size_t)(2 * cta + (it == it_begin ? 0 : 1)) * TILE_F + (size_t)q * CHUNKS * 1024;
 #pragma unroll 1
-                for (int c = 0; c < CHUNKS; ++c) {
-                    uint32_t r[32];
-                    tmem_ld32(acc + (uint32_t)(c * 32), r);
-                    const int n = n0 + c * 32;
-                    if (n < N) {                            // warp-uniform
-                        float v[32];
+                    for (int c = part; c < CHUNKS; c += EPI_WARPS / 4) {
+                        uint32_t r[32];
+                        tmem_ld32(acc + (uint32_t)(c * 32), r);
+                        float4* dst = reinterpret_cast<float4*>(mine + c * 1024) + lane;
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
-                        epi_block<MODE>(ep, stg, m0 + q * 32, M, n, v, lane);
+                        for (int k = 0; k < 8; ++k)
+                            dst[k * 32] = make_float4(__uint_as_float(r[4 * k]), __uint_as_float(r[4 * k + 1]), __uint_as_float(r[4 * k + 2]), __uint_as_float(r[4 * k + 3]));
                     }
-                }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&tmem_empty_bar[b]);
-            } else {
-                // partial sum of tile t: park it.  A 32 x 32 block of (row = lane, column j) is stored as 8 rows of 32 float4: the float4
-                // of lane l in row k holds columns 4k .. 4k+3 of row l, so every store / reload instruction moves 512 contiguous bytes
-                float* mine = sc.ws + (size_t)(2 * cta + (it == it_begin ? 0 : 1)) * TILE_F + (size_t)q * CHUNKS * 1024;
-#pragma unroll 1
-                for (int c = 0; c < CHUNKS; ++c) {
-                    uint32_t r[32];
-                    tmem_ld32(acc + (uint32_t)(c * 32), r);
-                    float4* dst = reinterpret_cast<float4*>(mine + c * 1024) + lane;
-#pragma unroll
-                    for (int k = 0; k < 8; ++k)
-                        dst[k * 32] = make_float4(__uint_as_float(r[4 * k]), __uint_as_float(r[4 * k + 1]), __uint_as_float(r[4 * k + 2]), __uint_as_float(r[4 * k + 3]));
-                }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&tmem_empty_bar[b]);
-                // arrive at the tile; the last of its contributors finishes it
-                __threadfence();
-                asm volatile("bar.sync 1, 128;" ::: "memory");
-                const int c_first = sched_owner(sc, t * KB), c_last = sched_owner(sc, t * KB + KB - 1);
-                if (threadIdx.x == 128) *last_flag = atomicAdd(&sc.counters[t], 1) == c_last - c_first;
-                asm volatile("bar.sync 1, 128;" ::: "memory");
-                if (*last_flag) {
+                    // arrive at the tile; the last of its contributors finishes it
                     __threadfence();
-#pragma unroll 1
-                    for (int c = 0; c < CHUNKS; ++c) {
-                        const int n = n0 + c * 32;
-                        if (n >= N) break;
-                        float v[32];
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) v[j] = 0.f;
-                        auto part = [&](int cc) {
-                            return reinterpret_cast<const float4*>(sc.ws + (size_t)(2 * cc + (sched_start(sc, cc) < t * KB ? 1 : 0)) * TILE_F +
-                                                                   (size_t)(q * CHUNKS + c) * 1024) + lane;
-                        };
-                        // contributor order, whoever came last; two contributors' loads in flight together (the additions stay in order)
-                        for (int cc = c_first; cc <= c_last; cc += 2) {
-                            const bool two = cc + 1 <= c_last;
-                            const float4* p0 = part(cc);
-                            const float4* p1 = part(two ? cc + 1 : cc);
-                            float4 x0[8], x1[8];
-#pragma unroll
-                            for (int k = 0; k < 8; ++k) x0[k] = __ldcg(p0 + k * 32);
-#pragma unroll
-                            for (int k = 0; k < 8; ++k) x1[k] = two ? __ldcg(p1 + k * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-                            for (int k = 0; k < 8; ++k) { v[4 * k] += x0[k].x; v[4 * k + 1] += x0[k].y; v[4 * k + 2] += x0[k].z; v[4 * k + 3] += x0[k].w; }
-                            if (two) {
-#pragma unroll
-                                for (int k = 0; k < 8; ++k) { v[4 * k] += x1[k].x; v[4 * k + 1] += x1[k].y; v[4 * k + 2] += x1[k].z; v[4 * k + 3] += x1[k].w; }
-                            }
-                        }
-                        epi_block<MODE>(ep, stg, m0 + q * 32, M, n, v, lane);
-                    }
+                    named_bar_sync(1, 32 * EPI_WARPS);
+                    if (threadIdx.x == 128) *last_flag = atomicAdd(&sc.counters[t], 1) == c_last - c_first;
+                    named_bar_sync(1, 32 * EPI_WARPS);
+                    finish = *last_flag;
+                }
+                if (finish) {
+                    __threadfence();
                     if (threadIdx.x == 128) sc.counters[t] = 0;       // clean for the next launch on this stream
                 }
-                asm volatile("bar.sync 1, 128;" ::: "memory");           // last_flag is rewritten by the next segment
             }
+            if (seg_end == it_end) { patch.base = smem + (warp - 4) * 4 * EPI_PATCH; patch.ring = true; }      // every MMA of this CTA has read its operands
+            if (finish && m0 < M)
+                epi_rows<MODE, BN>(ep, tmO, tmOlo, patch, m0, M, n0, N, part, lane, [&](int c, float* v) {
+                    tmem_ld32(acc + (uint32_t)(c * 32), reinterpret_cast<uint32_t*>(v));
+                    if (sole) return;
+                    // a shared tile: contributor order, whoever came last
+                    float sum[32];
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) sum[j] = 0.f;
+#pragma unroll 1
+                    for (int cc = c_first; cc <= c_last; ++cc) {
+                        if (cc == cta) {
+#pragma unroll
+                            for (int j = 0; j < 32; ++j) sum[j] += v[j];
+                            continue;
+                        }
+                        const float4* p = reinterpret_cast<const float4*>(sc.ws + (size_t)(2 * cc + (sched_start(sc, cc) < t * KB ? 1 : 0)) * TILE_F +
+                                                                          (size_t)(q * CHUNKS + c) * 1024) + lane;
+                        float4 x[8];
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) x[k] = __ldcg(p + k * 32);
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) { sum[4 * k] += x[k].x; sum[4 * k + 1] += x[k].y; sum[4 * k + 2] += x[k].z; sum[4 * k + 3] += x[k].w; }
+                    }
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) v[j] = sum[j];
+                });
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&tmem_empty_bar[b]);
+            if (!sole) named_bar_sync(1, 32 * EPI_WARPS);             // last_flag is rewritten by the next segment
             it = seg_end;
         }
+        if (lane == 0) tma_store_wait_read<0>();        // (the writes themselves are complete when the grid is)
         if (threadIdx.x == 128) stamp(5);               // this CTA's rows stored
     }
     tc_fence_before();
@@ -418,6 +491,16 @@ static int launch_tc(cudaStream_t stream, const bf16* A, const bf16* A_lo, int l
     if (!tc_tmap_bf16(&tmA, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, GEMM_BM)) return -1001;
     if (!tc_tmap_bf16(&tmAlo, SPLIT ? A_lo : A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, GEMM_BM)) return -1001;
     if (!tc_tmap_bf16(&tmB, W, (uint64_t)N, (uint64_t)K, (uint64_t)K, BN)) return -1001;
+    constexpr bool F32 = MODE == EPI_STORE_F32 || MODE == EPI_RESID_F32;
+    CUtensorMap tmO, tmOlo;
+    const uint64_t out_cols = MODE == EPI_SILU_MUL_BF16 ? N / 2 : N;
+    const CUtensorMapDataType ot = F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+    constexpr bool GLU = MODE == EPI_SILU_MUL_BF16;
+    constexpr CUtensorMapSwizzle osw = GLU ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B;
+    if (!tc_tmap(&tmO, epi.out, ot, (uint64_t)M, out_cols, (uint64_t)epi.ldo, 32, F32 || GLU ? 16 : 32, osw)) return -1001;
+    if (!tc_tmap(&tmOlo, !F32 && epi.out_lo ? epi.out_lo : epi.out, ot, (uint64_t)M, out_cols, (uint64_t)epi.ldo, 32, F32 || GLU ? 16 : 32, osw)) return -1001;
+    int* err = nullptr;
+    if (const int e = tc_err_word(stream, &err)) return e;
     static SmemOptIn seen;
     if (const int e = ensure_dyn_smem(gemm_tc_kernel<BN, MODE, SPLIT>, (size_t)Cfg::SMEM_BYTES, seen)) return e;
     TcSched sc = {};
@@ -440,7 +523,7 @@ static int launch_tc(cudaStream_t stream, const bf16* A, const bf16* A_lo, int l
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(sc.G);
-    cfg.blockDim = dim3(256);
+    cfg.blockDim = dim3(128 + 32 * EPI_WARPS);
     cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
@@ -452,32 +535,32 @@ static int launch_tc(cudaStream_t stream, const bf16* A, const bf16* A_lo, int l
     }
     cfg.attrs = attr;
     cfg.numAttrs = na;
-    return (int)cudaLaunchKernelEx(&cfg, gemm_tc_kernel<BN, MODE, SPLIT>, tmA, tmAlo, tmB, epi, M, N, K, sc);
+    return (int)cudaLaunchKernelEx(&cfg, gemm_tc_kernel<BN, MODE, SPLIT>, tmA, tmAlo, tmB, tmO, tmOlo, epi, M, N, K, sc, err);
 }
 
-// Tile width and schedule from a cost model fitted to tools/gemm_probe.py on B200 (microseconds):
-//   a k-step costs t_k(BN): the L2 hands a CTA its operands at ~0.33 us per k-step whatever the tile width (0.46 with the second
-//   activation plane), only the 128 x 256 tile is slower than that because its MMAs are (0.34 / 0.60);
+// Tile width and schedule from a cost model fitted on B200 (microseconds; 42 shapes of 77 - 4096 rows, every width and schedule):
+//   a k-step costs t_k: 64- and 128-wide tiles wait for their operands, 128 x 256 ones for shared memory, which MMAs read at 96 bytes a cycle while TMA writes
+//   64 (two planes) or 96 (one) into it: 128 is the limit;
 //   whole tiles: each CTA runs ceil(tiles / CTAs) tiles, the epilogue of all but the last hidden under the next tile's MMAs;
-//   stream-K:    tiles x k-steps dealt evenly to all SMs, plus parking a partial tile and the last contributor re-reading c of them.
+//   stream-K:    tiles x k-steps dealt evenly to all SMs, and the last of a tile's c contributors adding the others' parts.
 struct GemmPlan { int bn; bool stream_k; double cost; };
-static GemmPlan gemm_plan(int M, int N, int K, bool split, int sms) {
+static GemmPlan gemm_plan(int mode, int M, int N, int K, bool split, int sms) {
     static const int g_mode = [] { const char* e = getenv("CRANE_B200_GEMM_SCHED"); return e ? atoi(e) : 0; }();   // 1: whole tiles, 2: stream-K
     const int tm = (M + GEMM_BM - 1) / GEMM_BM, KB = K / GEMM_BK;
+    const bool light = mode == EPI_STORE_F32 || mode == EPI_RESID_F32 || mode == EPI_STORE_BF16 || mode == EPI_RELU2_BF16;
     GemmPlan best{64, false, 1e30};
     for (int bn : {256, 128, 64}) {
         if (g_gemm_bn && bn != g_gemm_bn) continue;
         if (!g_gemm_bn && bn > 64 && N < bn) continue;
         const long long tiles = (long long)tm * ((N + bn - 1) / bn);
-        const bool busy = tiles >= sms - 20;                                  // (nearly) every SM pulling operands: the L2 is the limit
-        const double tk = split ? (bn == 256 ? (busy ? 0.68 : 0.60) : 0.46) : (bn == 256 ? 0.34 : 0.33);
-        const double epi = 6.0 * bn / 256.0;
         const long long per = (tiles + std::min<long long>(tiles, sms) - 1) / std::min<long long>(tiles, sms);
-        const double whole = 1.5 + (double)per * KB * tk + epi;
-        const double it = (double)tiles * KB / sms;
-        const double contrib = std::ceil((double)KB / std::max(it, 1.0)) + 1.0;
-        const double tks = split ? (bn == 256 ? 0.68 : 0.46) : (bn == 256 ? 0.36 : 0.33);
-        const double sk = it < g_gemm_minit ? 1e30 : 1.5 + it * tks + 1.6 * epi + contrib * 6.0 * bn / 256.0;
+        const double tk = split ? (bn == 256 ? (per > 1 ? 0.66 : tiles > 96 ? 0.60 : 0.565) : bn == 128 ? 0.405 : 0.35)
+                                : (bn == 256 ? (per > 1 ? 0.42 : 0.34) : bn == 128 ? 0.267 : 0.25);
+        const double fixed = 3.7 + (light ? 2.7 : 5.5) * bn / 256.0;
+        const double whole = fixed + (double)per * KB * tk;
+        const double it = std::max((double)tiles * KB / sms, (double)g_gemm_minit);
+        const double contrib = KB / it + 1.0;
+        const double sk = fixed + it * (split && bn == 256 ? 0.66 : tk) + contrib * (bn == 256 ? 2.3 : bn == 128 ? 1.9 : 1.3);
         if (g_mode != 2 && whole < best.cost) best = GemmPlan{bn, false, whole};
         // stream-K only below one wave of whole tiles: above it the extra partial-tile traffic costs more than the idle SMs
         if (g_mode != 1 && (tiles < sms || g_mode == 2) && tiles * KB >= 2LL * sms && sk < best.cost) best = GemmPlan{bn, true, sk};
@@ -493,7 +576,7 @@ static int launch_mode(cudaStream_t stream, const bf16* A, const bf16* A_lo, int
         gemm_simt_kernel<MODE><<<grid, 128, 0, stream>>>(A, A_lo, lda, W, epi, M, N, K);
         return (int)cudaGetLastError();
     }
-    const GemmPlan p = gemm_plan(M, N, K, A_lo != nullptr, std::min(tc_device_sms(), GEMM_MAX_CTAS));
+    const GemmPlan p = gemm_plan(MODE, M, N, K, A_lo != nullptr, std::min(tc_device_sms(), GEMM_MAX_CTAS));
     if (A_lo != nullptr) {
         switch (p.bn) {
             case 256: return launch_tc<256, MODE, true>(stream, A, A_lo, lda, W, M, N, K, epi, p.stream_k);

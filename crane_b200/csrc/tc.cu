@@ -24,22 +24,23 @@ static PFN_encodeTiled get_encode_fn() {
 }
 
 struct TmapKey {
-    const void* base; uint64_t rows, cols, ld; uint32_t box_rows, box_cols; int swizzle;
+    const void* base; uint64_t rows, cols, ld; uint32_t box_rows, box_cols; int swizzle, type;
     bool operator==(const TmapKey& o) const {
-        return base == o.base && rows == o.rows && cols == o.cols && ld == o.ld && box_rows == o.box_rows && box_cols == o.box_cols && swizzle == o.swizzle;
+        return base == o.base && rows == o.rows && cols == o.cols && ld == o.ld && box_rows == o.box_rows && box_cols == o.box_cols && swizzle == o.swizzle && type == o.type;
     }
 };
 struct TmapKeyHash {
     size_t operator()(const TmapKey& k) const {
         size_t h = std::hash<const void*>()(k.base);
-        for (uint64_t v : {k.rows, k.cols, k.ld, (uint64_t)k.box_rows, (uint64_t)k.box_cols, (uint64_t)k.swizzle}) h = h * 1000003u ^ std::hash<uint64_t>()(v);
+        for (uint64_t v : {k.rows, k.cols, k.ld, (uint64_t)k.box_rows, (uint64_t)k.box_cols, (uint64_t)(k.swizzle * 64 + k.type)}) h = h * 1000003u ^ std::hash<uint64_t>()(v);
         return h;
     }
 };
-bool tc_tmap_16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows, uint32_t box_cols, CUtensorMapSwizzle swizzle) {
+bool tc_tmap(CUtensorMap* map, const void* base, CUtensorMapDataType type, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows, uint32_t box_cols,
+             CUtensorMapSwizzle swizzle) {
     static std::unordered_map<TmapKey, CUtensorMap, TmapKeyHash> cache;
     static std::mutex mu;
-    const TmapKey key{base, rows, cols, ld, box_rows, box_cols, (int)swizzle};
+    const TmapKey key{base, rows, cols, ld, box_rows, box_cols, (int)swizzle, (int)type};
     {
         std::lock_guard<std::mutex> g(mu);
         auto it = cache.find(key);
@@ -48,10 +49,10 @@ bool tc_tmap_16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols
     PFN_encodeTiled enc = get_encode_fn();
     if (!enc) return false;
     cuuint64_t dims[2] = {cols, rows};
-    cuuint64_t strides[1] = {ld * 2};
+    cuuint64_t strides[1] = {ld * (type == CU_TENSOR_MAP_DATA_TYPE_FLOAT32 ? 4 : 2)};
     cuuint32_t box[2] = {box_cols, box_rows};
     cuuint32_t estr[2] = {1, 1};
-    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+    CUresult r = enc(map, type, 2, const_cast<void*>(base), dims, strides, box, estr,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return false;

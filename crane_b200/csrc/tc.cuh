@@ -44,6 +44,7 @@ struct TcWaitT {
     }
 };
 using TcWait = TcWaitT<TC_WAIT_CYCLES>;
+__device__ __forceinline__ int ld_acquire(const int* p) { int v; asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory"); return v; }
 // One lane of a converged warp.  An issuing warp runs its loop as a whole and only its tcgen05 / TMA instructions under this: addresses and descriptors
 // stay in uniform registers (measured, 128 x 16 MMAs: 40 cycles each, 52 when a single lane runs the loop).
 __device__ __forceinline__ bool elect_one() {
@@ -60,6 +61,17 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
         ::"r"(smem_u32(smem_dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1) : "memory");
 }
+// shared -> global, rows and columns outside the tensor are dropped; and the same with the old values added (f32, in the L2).  One thread issues and commits.
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, const void* smem_src, int c0, int c1) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(map), "r"(smem_u32(smem_src)), "r"(c0), "r"(c1) : "memory");
+}
+__device__ __forceinline__ void tma_add_2d(const CUtensorMap* map, const void* smem_src, int c0, int c1) {
+    asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];"
+                 ::"l"(map), "r"(smem_u32(smem_src)), "r"(c0), "r"(c1) : "memory");
+}
+__device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+template <int N>      // the sources of all but the last N stores may be rewritten
+__device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
 }
@@ -143,11 +155,18 @@ __device__ __forceinline__ uint64_t make_smem_desc_sw32(uint32_t smem_addr) {
 __host__ __device__ constexpr uint32_t make_idesc_f16(int M, int N) { return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24); }
 // 128-byte rows: byte offset of the 16-byte piece c of row r
 __device__ __forceinline__ uint32_t sw128_off(int r, int c) { return (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4)); }
+// 64- and 32-byte rows
+__device__ __forceinline__ uint32_t sw32_off(int r, int c) { return (uint32_t)(r * 32 + ((c ^ ((r >> 2) & 1)) << 4)); }
+__device__ __forceinline__ uint32_t sw64_off(int r, int c) { return (uint32_t)(r * 64 + ((c ^ ((r >> 1) & 3)) << 4)); }
 
 // ---- host side (tc.cu) ---------------------------------------------------------------------
-// 2-D row-major [rows, cols] of 16-bit elements with `ld` elements between rows; box = [box_rows, box_cols].  Encoded maps are cached by
+// 2-D row-major [rows, cols] of 16- or 32-bit elements with `ld` elements between rows; box = [box_rows, box_cols].  Encoded maps are cached by
 // their defining tuple: encoding costs a few microseconds of host time, as much as a small kernel runs.
-bool tc_tmap_16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows, uint32_t box_cols, CUtensorMapSwizzle swizzle);
+bool tc_tmap(CUtensorMap* map, const void* base, CUtensorMapDataType type, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows, uint32_t box_cols,
+             CUtensorMapSwizzle swizzle);
+inline bool tc_tmap_16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows, uint32_t box_cols, CUtensorMapSwizzle swizzle) {
+    return tc_tmap(map, base, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rows, cols, ld, box_rows, box_cols, swizzle);
+}
 // ... of bf16 in boxes of 64 columns, SWIZZLE_128B
 inline bool tc_tmap_bf16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows) {
     return tc_tmap_16(map, base, rows, cols, ld, box_rows, 64, CU_TENSOR_MAP_SWIZZLE_128B);
