@@ -25,6 +25,7 @@ namespace cg = cooperative_groups;
 constexpr int GR_MAX_CTAS = 160;
 constexpr int GR_TILE = 128 * 128;                // one 64-wide tile of the weights
 constexpr int GR_BUDGET = 208 * 1024;
+constexpr int GR_EPI = 8;                         // epilogue warps: two take turns at a quarter's chunks of 16 rows
 
 struct GemmRowsArgs {
     GemmEpi ep;
@@ -68,18 +69,41 @@ __device__ __forceinline__ void rows_epi16(const GemmEpi& ep, int M, int N, int 
 #pragma unroll
         for (int j = 0; j < 16; ++j) if (j < rows) o[(size_t)j * ep.ldo] = v[j];
     } else if constexpr (MODE == EPI_SILU_MUL_F32 || MODE == EPI_SILU_MUL_BF16) {
-        // rows interleaved (gate_j, up_j): an even lane has the gate, its neighbour the up; pairs of results to every fourth lane for 4-byte stores
+        // rows interleaved (gate_j, up_j): an even lane has the gates of a column's 16 rows, its neighbour the ups.  They trade halves: the even lane finishes rows
+        // 0 - 7, the odd one 8 - 15, eight independent exponentials and divisions each.
+        const bool odd = lane & 1;
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            const float up = __shfl_xor_sync(0xffffffffu, v[j], 1), g = glu_pair_f(v[j], up, ep.glu_limit);
-            if constexpr (MODE == EPI_SILU_MUL_F32) {
-                if (!(lane & 1) && in && j < rows) reinterpret_cast<float*>(ep.out)[(size_t)(m0 + j) * ep.ldo + (n >> 1)] = g;
-            } else {
-                const float g2 = __shfl_xor_sync(0xffffffffu, g, 2);
-                if (!(lane & 3) && in && j < rows) {
+        for (int j = 0; j < 16; ++j) v[j] = j < rows ? v[j] : 1.f;       // rows behind the last are zeros, which the division takes 100 cycles each for
+        float r[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const float x = __shfl_xor_sync(0xffffffffu, odd ? v[j] : v[j + 8], 1);
+            r[j] = odd ? x : v[j];
+            v[j] = odd ? v[j + 8] : x;
+        }
+        if (ep.glu_limit == 0.f) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) r[j] = silu_f(r[j]) * v[j];
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) r[j] = glu_pair_f(r[j], v[j], ep.glu_limit);
+        }
+        const int mo = m0 + (odd ? 8 : 0);
+        if constexpr (MODE == EPI_SILU_MUL_F32) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) if (in && mo + j < M) reinterpret_cast<float*>(ep.out)[(size_t)(mo + j) * ep.ldo + (n >> 1)] = r[j];
+        } else {
+            // neighbouring columns (lanes two apart) as 4-byte stores: the lower lane takes the first four of the rows, the upper the last
+            const bool up = lane & 2;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float x = __shfl_xor_sync(0xffffffffu, up ? r[j] : r[j + 4], 2);
+                const float a = up ? x : r[j], b = up ? r[j + 4] : x;
+                const int m = mo + (up ? 4 : 0) + j;
+                if (in && m < M) {
                     uint32_t hi, lo;
-                    split_bf16x2(g, g2, hi, lo);
-                    const size_t off = (size_t)(m0 + j) * ep.ldo + (n >> 1);
+                    split_bf16x2(a, b, hi, lo);
+                    const size_t off = (size_t)m * ep.ldo + ((n >> 1) & ~1);
                     *reinterpret_cast<uint32_t*>(reinterpret_cast<bf16*>(ep.out) + off) = hi;
                     if (ep.out_lo) *reinterpret_cast<uint32_t*>(reinterpret_cast<bf16*>(ep.out_lo) + off) = lo;
                 }
@@ -88,15 +112,21 @@ __device__ __forceinline__ void rows_epi16(const GemmEpi& ep, int M, int N, int 
     } else {
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
-            float a = v[j];
-            if constexpr (MODE == EPI_GELU_ERF_BF16) a = gelu_erf_f(a);
-            else if constexpr (MODE == EPI_GELU_TANH_BF16) a = gelu_tanh_f(a);
-            else if constexpr (MODE == EPI_RELU2_BF16) { a = fmaxf(a, 0.f); a *= a; }
-            const float b = __shfl_xor_sync(0xffffffffu, a, 1);
-            if (!(lane & 1) && in && j < rows) {
+            if constexpr (MODE == EPI_GELU_ERF_BF16) v[j] = gelu_erf_f(v[j]);
+            else if constexpr (MODE == EPI_GELU_TANH_BF16) v[j] = gelu_tanh_f(v[j]);
+            else if constexpr (MODE == EPI_RELU2_BF16) { v[j] = fmaxf(v[j], 0.f); v[j] *= v[j]; }
+        }
+        // neighbouring columns as 4-byte stores: the even lane takes rows 0 - 7, the odd one 8 - 15
+        const bool odd = lane & 1;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const float x = __shfl_xor_sync(0xffffffffu, odd ? v[j] : v[j + 8], 1);
+            const float a = odd ? x : v[j], b = odd ? v[j + 8] : x;
+            const int jj = j + (odd ? 8 : 0);
+            if (in && jj < rows) {
                 uint32_t hi, lo;
                 split_bf16x2(a, b, hi, lo);
-                const size_t off = (size_t)(m0 + j) * ep.ldo + n;
+                const size_t off = (size_t)(m0 + jj) * ep.ldo + (n & ~1);
                 *reinterpret_cast<uint32_t*>(reinterpret_cast<bf16*>(ep.out) + off) = hi;
                 if (ep.out_lo) *reinterpret_cast<uint32_t*>(reinterpret_cast<bf16*>(ep.out_lo) + off) = lo;
             }
@@ -104,9 +134,9 @@ __device__ __forceinline__ void rows_epi16(const GemmEpi& ep, int M, int N, int 
     }
 }
 
-//   warp 0: TMA producer    warp 1: MMA issuer    warp 2: TMEM allocator    warps 4 - 7: epilogue (TMEM lanes 32 (warp % 4) ..)
+//   warp 0: TMA producer    warp 1: MMA issuer    warp 2: TMEM allocator    warps 4 - 11: epilogue (TMEM lanes 32 (warp % 4) .., every other 16 rows)
 template <int P, int MODE, int CH>
-__global__ void __launch_bounds__(256, 1)
+__global__ void __launch_bounds__(128 + 32 * GR_EPI, 1)
 gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmA1,
                  const __grid_constant__ CUtensorMap tmA2, GemmRowsArgs a) {
     extern __shared__ uint8_t smem_raw[];
@@ -123,7 +153,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     if (threadIdx.x == 0) {
         gave_up = 0;
         for (int i = 0; i < nstg; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
-        for (int i = 0; i < 2; ++i) { mbar_init(&d_full[i], 1); mbar_init(&d_empty[i], 4); }
+        for (int i = 0; i < 2; ++i) { mbar_init(&d_full[i], 1); mbar_init(&d_empty[i], GR_EPI); }
         fence_barrier_init();
     }
     if (warp == 2) { tmem_alloc(&tmem_slot, 512); tmem_relinquish(); }
@@ -189,7 +219,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         }
     } else if (warp >= 4) {
         pdl_wait();                                 // (reads / overwrites activations of the predecessor too)
-        const int q = warp & 3, row = q * 32 + lane;
+        const int q = warp & 3, part = (warp - 4) >> 2, row = q * 32 + lane;
         const size_t tile_f = (size_t)128 * Mp;
         int seg = 0;
         for (int it = it_begin; it < it_end; ++seg) {
@@ -201,7 +231,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
             // a cluster's partial tile stays in shared memory, in place of the operands (every MMA of this CTA has read its own)
             float* mine = a.cl > 1 ? reinterpret_cast<float*>(sm) + row : a.sc.ws + (size_t)(2 * blockIdx.x + (it == it_begin ? 0 : 1)) * tile_f + row;
 #pragma unroll 1
-            for (int c = 0; c < Mp; c += 16) {
+            for (int c = 16 * part; c < Mp; c += 4 * GR_EPI) {
                 uint32_t r0[16], r1[16], r2[16];
                 tmem_ld16_async(d + c, r0);
                 if (P > 1) tmem_ld16_async(d + Mp + c, r1);
@@ -225,14 +255,14 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
             if (lane == 0) mbar_arrive(&d_empty[b]);
             if (!sole && a.cl == 0) {               // arrive at the tile; the last of its contributors adds them in order and finishes it
                 __threadfence();
-                named_bar_sync(1, 128);
+                named_bar_sync(1, 32 * GR_EPI);
                 const int c_first = sched_owner(a.sc, t * KB), c_last = sched_owner(a.sc, t * KB + KB - 1);
                 if (threadIdx.x == 128) last_flag = atomicAdd(&a.sc.counters[t], 1) == c_last - c_first;
-                named_bar_sync(1, 128);
+                named_bar_sync(1, 32 * GR_EPI);
                 if (last_flag) {
                     __threadfence();
 #pragma unroll 1
-                    for (int c = 0; c < Mp; c += 16) {
+                    for (int c = 16 * part; c < Mp; c += 4 * GR_EPI) {
                         float v[16];
 #pragma unroll
                         for (int j = 0; j < 16; ++j) v[j] = 0.f;
@@ -256,7 +286,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
                     }
                     if (threadIdx.x == 128) a.sc.counters[t] = 0;
                 }
-                named_bar_sync(1, 128);             // last_flag is rewritten by the next segment
+                named_bar_sync(1, 32 * GR_EPI);             // last_flag is rewritten by the next segment
             }
             it = seg_end;
         }
@@ -267,7 +297,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         if (warp >= 4) {
             const int row = (warp & 3) * 32 + lane, n = it_begin / KB * 128 + row;
 #pragma unroll 1
-            for (int c = rank * 16; c < Mp; c += 16 * a.cl) {
+            for (int c = (rank + ((warp - 4) >> 2) * a.cl) * 16; c < Mp; c += 4 * GR_EPI * a.cl) {
                 float v[16];
 #pragma unroll
                 for (int j = 0; j < 16; ++j) v[j] = 0.f;
@@ -295,22 +325,21 @@ static int rows_cluster(int tiles_n, int steps, int sms) {
 }
 
 // Is this kernel the faster one of the two for up to 128 rows?  Both stream the weights at about the same rate; the tiles of gemm.cu pay for 128 rows whatever M
-// is, while here a CTA finishes 16 rows after 16 rows, f32 results 0.4 us each, bf16 ones with or without a unary function 1.5, gate and up 5, shared by the
-// CTAs of a cluster.  us, here / gemm.cu (planes x rows: weights):
-//   f32, a cluster per tile    always, but for 1 x 97 - 128: 4096 x 1024 9.6 / 8.9 (4096 x 2048 11.4 / 14.2; 2 x 128: 4096 x 1024 10.2 / 10.5)
+// is, while here the activations' traffic and the epilogue grow with the rows.  us, here / gemm.cu (planes x rows: weights):
+//   f32, a cluster per tile    always, but for 1 x 96 - 128 of K = 1024: 4096 x 1024 8.3 / 8.0 (1 x 77: 8.0 / 7.9; 4096 x 2048 11.3 / 12.0; 2 x 128: 4096 x 1024 10.0 / 10.2)
 //   f32, one CTA per tile      1 x 64: 12288 x 2048 13.2 / 15.4, 24576 x 4096 41.3 / 41.8; 1 x 96: 14.5 / 15.5, 46.4 / 42.5; 2 x 64: 18.0 / 18.2, 46.0 / 49.6; 2 x 96: 16384 x 2048 20.0 / 19.5
-//   others, one CTA per tile   1 x 48: gate / up 12288 x 2048 25.6 / 28.0, 24576 x 4096 65.1 / 65.5; bf16 12288 x 2048 15.1 / 14.7; 1 x 64: 30.1 / 27.8, 75.8 / 65.8, 16.2 / 14.9;
-//                              2 x 48: 26.8 / 30.7, 66.8 / 73.6, 15.9 / 18.3; 2 x 64: 35.0 / 30.6, 81.1 / 73.7, 21.0 / 18.8
-//   others, a cluster          by 16-row pieces per CTA.  One: gate / up 6144 x 1024 11.3 / 15.8, bf16 4096 x 1024 8.5 / 8.4; two: 6144 x 1024 16.3 / 15.5, 4096 x 1024
-//                              10.2 / 8.4, but 4096 x 2048 20.0 / 20.6, 8192 x 2048 13.7 / 14.2; three: 9472 x 4096 32.2 / 32.5; four: 38.6 / 32.4
+//   gate / up, one plane       a cluster: 64 rows 6144 x 1024 7.9 / 9.0, 7168 x 1024 8.4 / 9.4; 77: 9.3 / 9.0, 10.0 / 10.1.  One CTA: 77 12288 x 2048 14.7 / 16.1, 24576 x 4096
+//                              43.2 / 44.4; 96: 15.4 / 16.2, 45.5 / 45.0
+//   gate / up, two planes      96 rows: 6144 x 1024 11.0 / 11.1, 12288 x 2048 19.9 / 20.6; 112: 11.6 / 11.2, 21.2 / 20.7; more tiles than SMs: 128 24576 x 4096 63.2 / 63.9
+//   other bf16 results         a cluster: 1 x 96 4096 x 1024 9.3 / 9.5, 112 10.2 / 9.6, 128 4096 x 2048 11.9 / 12.2; 2 x 128: 4096 x 1024 11.8 / 12.5
+//                              one CTA: 1 x 48: 12288 x 2048 15.1 / 14.7; 2 x 48: 15.9 / 18.3; 2 x 64: 21.0 / 18.8
 bool gemm_rows_pays(int mode, int P, int M, int N, int K) {
     if (M > 128) return false;
-    const bool f32 = mode == EPI_STORE_F32 || mode == EPI_RESID_F32;
+    const bool f32 = mode == EPI_STORE_F32 || mode == EPI_RESID_F32, glu = mode == EPI_SILU_MUL_BF16;
     const int tiles_n = (N + 127) / 128, sms = std::min(tc_device_sms(), GR_MAX_CTAS), cl = tiles_n <= sms ? rows_cluster(tiles_n, K / 64, sms) : 1;
+    if (glu) return M <= (P == 1 ? (cl > 1 ? 64 : 80) : tiles_n <= sms ? 96 : 128);
     if (cl == 1) return M <= (!f32 ? 48 : P == 1 ? 80 : 64);
-    if (f32) return M <= 96 || P > 1 || K > 1024;
-    const int pieces = ((M + 15) / 16 + cl - 1) / cl;
-    return pieces <= std::max(1, std::min(3, K / 1024));
+    return P > 1 || K > 1024 || M <= (f32 ? 80 : 96);
 }
 
 template <int P, int MODE, int CH>
@@ -345,7 +374,7 @@ static int rows_launch_c(cudaStream_t st, const bf16* const* A, int lda, const b
         grid = sc.G;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid); cfg.blockDim = dim3(256); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    cfg.gridDim = dim3(grid); cfg.blockDim = dim3(128 + 32 * GR_EPI); cfg.dynamicSmemBytes = smem; cfg.stream = st;
     cudaLaunchAttribute attr[2];
     int na = 0;
     if (a.cl > 1) {
