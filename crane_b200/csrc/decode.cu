@@ -4,6 +4,8 @@
 
 #include <cooperative_groups.h>
 
+#include <algorithm>
+
 namespace cb {
 
 // =====================================================================================
@@ -413,6 +415,46 @@ embed_decode_kernel(const bf16* __restrict__ embed, int H, const SeqState* __res
     const int b = blockIdx.x;
     const bf16* row = embed + (size_t)state[b].token * H;
     for (int i = threadIdx.x; i < H; i += blockDim.x) x[(size_t)b * H + i] = __bfloat162float(row[i]);
+}
+
+__global__ void __launch_bounds__(SEQ_PACK)
+set_state_kernel(SeqState* __restrict__ state, const __grid_constant__ SeqPack pack, int n) {
+    pdl_launch_dependents();
+    if ((int)threadIdx.x < n) state[threadIdx.x] = pack.s[threadIdx.x];
+}
+int set_state_launch(cudaStream_t st, SeqState* state, const SeqState* snapshots, int n) {
+    if (n < 1 || n > SEQ_PACK) return -1000;
+    SeqPack pack = {};
+    for (int i = 0; i < n; ++i) pack.s[i] = snapshots[i];
+    return launch_k(set_state_kernel, dim3(1), dim3(SEQ_PACK), 0, st, false, state, pack, n);
+}
+
+// blockIdx.y: segment.  Bound by HBM for long segments (four 16-byte loads in flight per thread), by the launch for short ones.
+__global__ void __launch_bounds__(256)
+copy_list_kernel(const __grid_constant__ CopyList list) {
+    const CopySeg g = list.s[blockIdx.y];
+    const size_t n = g.bytes / 16, step = (size_t)gridDim.x * 256;
+    uint4* d = reinterpret_cast<uint4*>(g.dst);
+    const uint4* s = reinterpret_cast<const uint4*>(g.src);
+    uint4* k = reinterpret_cast<uint4*>(g.park);
+    for (size_t i = blockIdx.x * (size_t)256 + threadIdx.x; i < n; i += 4 * step) {
+        uint4 v[4], o[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (i + j * step < n) { v[j] = s[i + j * step]; if (k) o[j] = d[i + j * step]; }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (i + j * step < n) { if (k) k[i + j * step] = o[j]; d[i + j * step] = v[j]; }
+    }
+}
+int copy_list_launch(cudaStream_t st, const CopyList& list) {
+    if (list.n < 0 || list.n > COPY_LIST) return -1000;
+    if (list.n == 0) return 0;
+    size_t most = 0;
+    for (int i = 0; i < list.n; ++i) most = std::max(most, list.s[i].bytes);
+    const size_t blocks = (most / 16 + 1023) / 1024;
+    copy_list_kernel<<<dim3((unsigned)std::max<size_t>(1, std::min<size_t>(blocks, 64)), list.n), 256, 0, st>>>(list);
+    return (int)cudaGetLastError();
 }
 
 // =====================================================================================

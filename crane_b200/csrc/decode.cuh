@@ -112,6 +112,16 @@ int attn_decode_launch(cudaStream_t st, int B, int D, const AttnDecArgs& a, bool
 constexpr int ARGMAX_ROW_PARTS = 32;
 int argmax_rows_launch(cudaStream_t st, int B, const float* logits, int V, float* part_val, int* part_idx, SeqState* state, uint32_t* out_tokens, int out_stride,
                        const bf16* embed, float* x_next, int H, int advance, bool pdl);
+// state[0 .. n) <- the snapshots, which travel as launch parameters: an upload of 32 bytes per sequence by the copy engine put 8 us between two kernels.
+constexpr int SEQ_PACK = 64;
+struct SeqPack { SeqState s[SEQ_PACK]; };
+int set_state_launch(cudaStream_t st, SeqState* state, const SeqState* snapshots, int n);
+// Device copies of one call, a launch for up to COPY_LIST of them (56 copies of a fork took 250 us one by one: 4 us each, whatever their size).
+// dst[i] <- src[i]; with `park`, park[i] <- the old dst[i] first (src and park may be the same memory only if dst is another).  Pointers and bytes in units of 16.
+constexpr int COPY_LIST = 64;
+struct CopySeg { void* dst; const void* src; void* park; size_t bytes; };
+struct CopyList { CopySeg s[COPY_LIST]; int n; };
+int copy_list_launch(cudaStream_t st, const CopyList& list);
 int embed_decode_launch(cudaStream_t st, int B, const bf16* embed, int H, const SeqState* state, float* x, bool pdl);
 
 }  // namespace cb

@@ -313,27 +313,12 @@ struct crane_b200_model {
     void tts_frame(float rep_penalty, bool forced, int frame);
     const bf16** tts_tables_dev = nullptr;
     int* block_table = nullptr;
-    // Sequence state travels host -> device through a ring of pinned snapshots, one per call: the ABI hands out stream-ordered
-    // results, so a caller may issue the next call before the previous upload has run, and a single staging slot would be
-    // overwritten under it.  A slot is reused only after its own upload has completed (its event).
-    static constexpr int STATE_RING = 16;
-    int state_group = 4;              // sequences per snapshot
-    SeqState* h_state_ring = nullptr; // pinned [STATE_RING][state_group]
-    cudaEvent_t h_state_ev[STATE_RING] = {};
-    bool h_state_used[STATE_RING] = {};
-    int h_state_next = 0;
-    SeqState* h_state = nullptr;      // the slot being filled (stage_state)
-    SeqState* stage_state() {
-        const int i = h_state_next;
-        if (h_state_used[i]) CUDA_OK(cudaEventSynchronize(h_state_ev[i]));
-        h_state = h_state_ring + (size_t)i * state_group;
-        return h_state;
-    }
-    void push_state(int nseq) {       // upload the staged snapshot(s) to the device-resident state
-        CUDA_OK(cudaMemcpyAsync(state, h_state, sizeof(SeqState) * nseq, cudaMemcpyHostToDevice, stream));
-        CUDA_OK(cudaEventRecord(h_state_ev[h_state_next], stream));
-        h_state_used[h_state_next] = true;
-        h_state_next = (h_state_next + 1) % STATE_RING;
+    // Sequence state travels host -> device in the parameters of a launch: the ABI hands out stream-ordered results, so a caller may issue the next call
+    // before this one has run, and parameters are the launch's own.
+    SeqState h_state[SEQ_PACK] = {};  // the snapshot being filled
+    void push_state(int nseq) {       // the staged snapshot(s) to the device-resident state
+        LAUNCH_OK(set_state_launch(stream, state, h_state, nseq));
+        ++launches;
     }
     uint32_t* h_tokens = nullptr;     // pinned
     // prefill workspaces (grown on demand)
@@ -373,7 +358,6 @@ struct crane_b200_model {
     std::vector<uint32_t> seq_pos;
     std::vector<char> seq_used;
     void select_seq(int s);               // parks the current slot's view (and GDN state) and brings slot s in
-    void park_gdn_state(int slot);         // working recurrent / conv state -> the slot's store (hybrid models)
     void fork_seq(int src, int dst);
     const int* bt_cur() const { return block_table + (size_t)cur * max_pages; }
     cudaGraphExec_t graph_step[2][DECODE_GROUP_MAX + 1] = {};   // [advance][sequences in the group]
@@ -1188,7 +1172,6 @@ void crane_b200_model::finalize() {
     // which the wide head does not write)
     wide_ok = !hybrid && !is_tts && owns_stream && !use_simt && max_batch > 1;
     const int B = std::min(max_batch, wide_ok ? (int)DECODE_GROUP_MAX : 4);   // sequences per weight pass
-    state_group = B;
     if (wide_ok) {
         const int kmax = std::max(std::max(H, I), q_dim());
         wide_rows = B;
@@ -1236,8 +1219,6 @@ void crane_b200_model::finalize() {
         if (getenv("CRANE_B200_PROF")) { ll_prof = dalloc<unsigned long long>(16); CUDA_OK(cudaMemset(ll_prof, 0, 128)); }
         if (getenv("CRANE_B200_LL_TRACE")) ll_trace = dalloc<unsigned long long>((size_t)6 * LL_TRACE_CAP * 2);
     }
-    CUDA_OK(cudaMallocHost((void**)&h_state_ring, sizeof(SeqState) * STATE_RING * state_group));
-    for (auto& e : h_state_ev) CUDA_OK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     CUDA_OK(cudaMallocHost((void**)&h_tokens, sizeof(uint32_t) * out_cap));
     CUDA_OK(cudaEventCreate(&pev0));
     CUDA_OK(cudaEventCreate(&pev1));
@@ -1289,7 +1270,6 @@ void crane_b200_model::ensure_prefill_ws(int S) {
 // decode step
 // =================================================================================================
 void crane_b200_model::arm_state(uint32_t token, size_t start_pos, int p0, int p1, int p2) {
-    stage_state();
     h_state[0].kv_len = (int)start_pos;
     h_state[0].pos[0] = p0; h_state[0].pos[1] = p1; h_state[0].pos[2] = p2;
     h_state[0].token = token;
@@ -1300,8 +1280,8 @@ void crane_b200_model::arm_state(uint32_t token, size_t start_pos, int p0, int p
 
 // x_dec <- the embedding rows of state[b].token (bf16 table, or rows dequantised out of a quantised table)
 void crane_b200_model::embed_step_input(int B) {
-    if (q_embed) LAUNCH_OK(embed_rows_q_launch(stream, qt_embed, q_embed, H, nullptr, state, B, x_dec, false));
-    else LAUNCH_OK(embed_decode_launch(stream, B, embed, H, state, x_dec, false));
+    if (q_embed) LAUNCH_OK(embed_rows_q_launch(stream, qt_embed, q_embed, H, nullptr, state, B, x_dec, use_pdl));
+    else LAUNCH_OK(embed_decode_launch(stream, B, embed, H, state, x_dec, use_pdl));
     ++launches;
 }
 
@@ -1365,62 +1345,71 @@ void crane_b200_model::gdn_args(GdnArgs& g, const LayerW& l, int S, const float*
     g.rec_state = l.rec_state; g.conv_out = conv; g.qn = qn; g.kn = kn; g.gb = gb; g.y = y;
 }
 
-void crane_b200_model::park_gdn_state(int slot) {
-    if (!hybrid || max_batch <= 1) return;
-    const size_t cs = (size_t)conv_dim() * ck, rs = (size_t)nv * dk * dv;
-    for (auto& l : layers)
-        if (!l.full) {
-            CUDA_OK(cudaMemcpyAsync(l.conv_slots + slot * cs, l.conv_state, cs * sizeof(float), cudaMemcpyDeviceToDevice, stream));
-            CUDA_OK(cudaMemcpyAsync(l.rec_slots + slot * rs, l.rec_state, rs * sizeof(float), cudaMemcpyDeviceToDevice, stream));
+// Copies of one call: pieces of 16 bytes go on the list, others (odd sizes of small models) one by one.
+struct SegList {
+    cudaStream_t stream;
+    CopyList l = {};
+    void add(void* dst, const void* src, size_t bytes, void* park = nullptr) {
+        if (((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(park) | bytes) & 15) != 0) {
+            if (park) CUDA_OK(cudaMemcpyAsync(park, dst, bytes, cudaMemcpyDeviceToDevice, stream));
+            CUDA_OK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, stream));
+            return;
         }
-}
+        if (l.n == COPY_LIST) flush();
+        l.s[l.n++] = CopySeg{dst, src, park, bytes};
+    }
+    void flush() {
+        LAUNCH_OK(copy_list_launch(stream, l));
+        l.n = 0;
+    }
+};
 
 void crane_b200_model::select_seq(int s) {
     if (s == cur) return;
     seq_kv[cur] = kv_len; seq_pos[cur] = next_mrope_pos;
-    park_gdn_state(cur);
-    cur = s;
-    kv_len = seq_kv[s]; next_mrope_pos = seq_pos[s];
-    if (hybrid && max_batch > 1) {
+    if (hybrid && max_batch > 1) {              // the live state is parked as the other sequence's takes its place
         const size_t cs = (size_t)conv_dim() * ck, rs = (size_t)nv * dk * dv;
+        SegList c{stream};
         for (auto& l : layers)
             if (!l.full) {
-                CUDA_OK(cudaMemcpyAsync(l.conv_state, l.conv_slots + s * cs, cs * sizeof(float), cudaMemcpyDeviceToDevice, stream));
-                CUDA_OK(cudaMemcpyAsync(l.rec_state, l.rec_slots + s * rs, rs * sizeof(float), cudaMemcpyDeviceToDevice, stream));
+                c.add(l.conv_state, l.conv_slots + s * cs, cs * sizeof(float), l.conv_slots + cur * cs);
+                c.add(l.rec_state, l.rec_slots + s * rs, rs * sizeof(float), l.rec_slots + cur * rs);
             }
+        c.flush();
     }
+    cur = s;
+    kv_len = seq_kv[s]; next_mrope_pos = seq_pos[s];
 }
 
-// dst becomes a copy of src: the used KV pages of every attention layer (both precision planes) and the parked GDN state.
+// dst becomes a copy of src: the used KV pages of every attention layer (both precision planes) and the GDN state (the live one, when src is current).
 // Pages are statically owned by their slot, so a fork copies bytes; it is O(context), device to device, on the engine stream.
 void crane_b200_model::fork_seq(int src, int dst) {
     seq_kv[cur] = kv_len; seq_pos[cur] = next_mrope_pos;
-    if (src == cur) park_gdn_state(cur);
     const size_t len = seq_kv[src];
     const size_t pages = (len + KV_PAGE - 1) / KV_PAGE;
     const size_t page_elems = (size_t)nkv * KV_PAGE * D;
     const size_t so = (size_t)src * max_pages * page_elems, dofs = (size_t)dst * max_pages * page_elems, n = pages * page_elems;
     const size_t cs = hybrid ? (size_t)conv_dim() * ck : 0, rs = hybrid ? (size_t)nv * dk * dv : 0;
+    SegList c{stream};
     for (auto& l : layers) {
         if (l.full && kv_bits) {
             if (!pages) continue;
             const size_t rows = pages * nkv * KV_PAGE, rs0 = (size_t)src * max_pages * nkv * KV_PAGE, rd0 = (size_t)dst * max_pages * nkv * KV_PAGE;
             const size_t cb = (size_t)D * kv_bits / 8;
-            for (unsigned char* c : {l.k_codes, l.v_codes})
-                CUDA_OK(cudaMemcpyAsync(c + rd0 * cb, c + rs0 * cb, rows * cb, cudaMemcpyDeviceToDevice, stream));
-            for (float* sc : {l.k_scale, l.v_scale})
-                CUDA_OK(cudaMemcpyAsync(sc + rd0, sc + rs0, rows * sizeof(float), cudaMemcpyDeviceToDevice, stream));
+            for (unsigned char* p : {l.k_codes, l.v_codes}) c.add(p + rd0 * cb, p + rs0 * cb, rows * cb);
+            for (float* sc : {l.k_scale, l.v_scale}) c.add(sc + rd0, sc + rs0, rows * sizeof(float));
         } else if (l.full) {
             if (!n) continue;
             for (bf16* pool : {l.k_pool, l.v_pool}) {
-                CUDA_OK(cudaMemcpyAsync(pool + dofs, pool + so, n * sizeof(bf16), cudaMemcpyDeviceToDevice, stream));
-                if (lo_kv) CUDA_OK(cudaMemcpyAsync(pool + lo_kv + dofs, pool + lo_kv + so, n * sizeof(bf16), cudaMemcpyDeviceToDevice, stream));
+                c.add(pool + dofs, pool + so, n * sizeof(bf16));
+                if (lo_kv) c.add(pool + lo_kv + dofs, pool + lo_kv + so, n * sizeof(bf16));
             }
         } else if (max_batch > 1) {
-            CUDA_OK(cudaMemcpyAsync(l.conv_slots + dst * cs, l.conv_slots + src * cs, cs * sizeof(float), cudaMemcpyDeviceToDevice, stream));
-            CUDA_OK(cudaMemcpyAsync(l.rec_slots + dst * rs, l.rec_slots + src * rs, rs * sizeof(float), cudaMemcpyDeviceToDevice, stream));
+            c.add(l.conv_slots + dst * cs, src == cur ? l.conv_state : l.conv_slots + src * cs, cs * sizeof(float));
+            c.add(l.rec_slots + dst * rs, src == cur ? l.rec_state : l.rec_slots + src * rs, rs * sizeof(float));
         }
     }
+    c.flush();
     seq_kv[dst] = len; seq_pos[dst] = seq_pos[src];
 }
 
@@ -1754,7 +1743,6 @@ void crane_b200_model::prefill(const uint32_t* ids, const float* embeds, size_t 
     }
     // state for the last-row lm_head / a following on-device decode loop
     spans.mark(SP_HEAD);
-    stage_state();
     h_state[0].kv_len = (int)(start_pos + S - 1);   // lm_head(advance) bumps it to start_pos + S
     h_state[0].pos[0] = h_state[0].pos[1] = h_state[0].pos[2] = (int)next_mrope_pos - 1;
     h_state[0].token = 0;
@@ -2066,8 +2054,6 @@ void crane_b200_destroy(crane_b200_model* m) {
     for (auto& ga : m->graph_step) for (auto& g : ga) if (g) cudaGraphExecDestroy(g);
     for (void* p : m->allocs) cudaFree(p);
     if (m->fsv) { m->fsv->release(); delete m->fsv; m->fsv = nullptr; }
-    if (m->h_state_ring) cudaFreeHost(m->h_state_ring);
-    for (cudaEvent_t e : m->h_state_ev) if (e) cudaEventDestroy(e);
     if (m->h_tokens) cudaFreeHost(m->h_tokens);
     if (m->h_ll_err) cudaFreeHost(m->h_ll_err);
     if (m->h_stage) cudaFreeHost(m->h_stage);
@@ -2611,7 +2597,6 @@ int crane_b200_decode_batch(crane_b200_model* m, const int* seqs, const uint32_t
     size_t done = 0;
     while (done < n) {
         const int B = m->decode_group(n - done);
-        m->stage_state();
         for (int b = 0; b < B; ++b) {
             const int s = seqs[done + b];
             SeqState& st = m->h_state[b];
@@ -2729,7 +2714,6 @@ int crane_b200_decode_batch_sample(crane_b200_model* m, const int* seqs, const u
     size_t done = 0;
     while (done < n) {
         const int B = m->decode_group(n - done);
-        m->stage_state();
         for (int b = 0; b < B; ++b) {
             const int s = seqs[done + b];
             SeqState& st = m->h_state[b];
