@@ -11,29 +11,22 @@ namespace cb {
 // =====================================================================================
 // Weight-streaming GEMV:  y[b, n] = epilogue( sum_k W[n, k] * x[b, k] )          (B <= 4 sequences)
 //
-// grid = #SMs; CTA c owns the contiguous row block [c*rpc, (c+1)*rpc) of W -- one contiguous byte slab -- and splits it
-// into GV_WARPS contiguous sub-slabs, one per warp.  Every warp runs its own private, barrier-free pipeline:
-// GV_DEPTH x 2 KB shared-memory slots filled by cp.async (LDGSTS, 16 B per lane, L1-bypassing) and drained with 16-byte
-// LDS (conflict-free) into f32 FMAs -- 80 KB of weight bytes in flight per SM, no cross-warp synchronisation in the
-// streaming loop.  Weights do not depend on the previous kernel, so the pipelines are primed BEFORE griddepcontrol.wait:
-// with programmatic dependent launch the next kernel's CTAs sit next to this kernel's on the SM (2 x 104 KB shared
-// memory) and the HBM pipe stays busy across the kernel boundary.  Activations are staged once per CTA as f32 (RMSNorm
-// folded in).  Rows are flushed to a shared accumulator (shuffle reduce + one shared atomic per row change per warp).
+// grid = #SMs; CTA c owns the contiguous rows [c*rpc, (c+1)*rpc) of W.  A unit of work is four rows x one of `ns` slices of K (gemv_slices): a warp takes
+// every GV_WARPS-th unit and runs its own, barrier-free pipeline: slots of 4 rows x 256 columns (2 KB) filled by cp.async (16 B per lane, L1-bypassing),
+// every lane reading back what it copied itself, into f32 FMAs.  Four rows share each read of the activations (f32 in shared memory, RMSNorm folded in):
+// row by row they were two thirds of the shared-memory traffic, which bound the kernel wherever the weights had come early.  A unit's sums are reduced
+// over the warp together (6 shuffles for four rows of one sequence instead of 20) and a row's slices added in order, so results repeat bit for bit.
+// Weights do not depend on the previous kernel, so the pipelines are primed BEFORE griddepcontrol.wait, and the HBM pipe stays busy across the boundary.
+// What is left per launch: 0.7 us from one grid's end to the next one's wait, 0.7 for the activations' round trip to the L2 (a chain of kernels
+// that only do that takes 1.4 us each).  In a chain of its own kind, us, before / after: 4096 x 1024 4.0 / 3.5, 6144 x 1024 (gate / up) 5.4 / 4.3,
+// 12288 x 2048 10.6 / 9.3, 24576 x 4096 31.7 / 30.3.  (Two CTAs per SM, so that the next launch's sit there early, gained nothing and cost the long ones 10 %.)
 // Epilogue (all threads): store / residual add / SiLU*up on interleaved rows / logits + CTA argmax.
 // =====================================================================================
-#ifndef GV_WARPS
-#define GV_WARPS 32
-#endif
-#ifndef GV_DEPTH
-#define GV_DEPTH 2
-#endif
-#ifndef GV_MINB                    // CTAs per SM the GEMV is compiled for (2 lets the next launch's CTA prime its ring early)
-#define GV_MINB 1
-#endif
-constexpr int GV_SEG_CHUNKS = 4;                       // 512-byte chunks per pipeline slot (2 KB)
-constexpr int GV_SEG_BYTES = GV_SEG_CHUNKS * 512;
+constexpr int GV_WARPS = 16;
+constexpr int GV_ROWS = 4;                             // rows of a unit
+constexpr int GV_SLOT = GV_ROWS * 512;
 constexpr int GV_THREADS = GV_WARPS * 32;
-__host__ __device__ constexpr int gv_depth(int B) { return B == 1 ? GV_DEPTH : 1; }   // batched activations take the ring's shared memory
+__host__ __device__ constexpr int gv_depth(int B) { return B == 1 ? 4 : 2; }          // batched activations take the ring's shared memory
 
 __device__ __forceinline__ void cp_async16_cg(uint32_t dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
@@ -73,10 +66,10 @@ __device__ __forceinline__ float gemv_stage_streams(const GemvArgs& a, int b, fl
 
 // NORM: 0 the input as it is, 1 RMS norm folded in, 2 the norm of a sum of parallel streams
 template <int B, int EPI, int NORM>
-__global__ void __launch_bounds__(GV_THREADS, GV_MINB)
-gemv_kernel(GemvArgs a) {
+__global__ void __launch_bounds__(GV_THREADS, 1)
+gemv_kernel(GemvArgs a, int ns) {
     extern __shared__ __align__(1024) unsigned char gsm[];
-    // layout: [rings: GV_WARPS * GV_DEPTH * 2 KB][xs: B * K f32][acc: B * rpc f32]
+    // layout: [rings: GV_WARPS * depth * 2 KB][xs: B * K f32][sums: B * rpc * ns f32]
     const int K8 = a.K >> 3;
     constexpr int ROWS_PER_UNIT = (EPI == GEMV_SILU_MUL) ? 2 : 1;
     const int units = a.N / ROWS_PER_UNIT;
@@ -86,42 +79,43 @@ gemv_kernel(GemvArgs a) {
     const int r1 = min(a.N, r0 + rpc);
     const int nrows = max(0, r1 - r0);
     constexpr int DEPTH = gv_depth(B);
-    float4* xs = reinterpret_cast<float4*>(gsm + GV_WARPS * DEPTH * GV_SEG_BYTES);
+    float4* xs = reinterpret_cast<float4*>(gsm + GV_WARPS * DEPTH * GV_SLOT);
     float* acc_s = reinterpret_cast<float*>(xs) + (size_t)B * a.K;
-    __shared__ float red[32];
+    __shared__ float red[B][GV_WARPS];
     __shared__ float rstd_s[B];
     __shared__ float wbest_v[GV_WARPS][B];
     __shared__ int wbest_i[GV_WARPS][B];
     __shared__ int is_last_s;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // 32-bit chunk bookkeeping (chunk = 512 B = 256 elements; never straddles a row since K % 256 == 0)
-    const uint32_t cpr = (uint32_t)(a.K >> 8);                                     // chunks per row
-    const uint32_t total_chunks = (uint32_t)nrows * cpr;
-    const uint32_t total_segs = (total_chunks + GV_SEG_CHUNKS - 1) / GV_SEG_CHUNKS;
-    const uint32_t spw = (total_segs + GV_WARPS - 1) / GV_WARPS;                   // segments per warp
-    const uint32_t c_begin = min(total_chunks, (uint32_t)warp * spw * GV_SEG_CHUNKS);
-    const uint32_t c_end = min(total_chunks, ((uint32_t)warp + 1) * spw * GV_SEG_CHUNKS);
-    const uint32_t nseg = (c_end - c_begin + GV_SEG_CHUNKS - 1) / GV_SEG_CHUNKS;
-    const unsigned char* gsrc = reinterpret_cast<const unsigned char*>(a.W) + (size_t)r0 * a.K * 2 + (size_t)c_begin * 512 + lane * 16;
-    unsigned char* ring = gsm + (size_t)warp * DEPTH * GV_SEG_BYTES + lane * 16;
+    const int chunks = a.K >> 8, work = (nrows + GV_ROWS - 1) / GV_ROWS * ns;           // (K % 256 == 0)
+    // a walk over this warp's slots: unit u, column chunk c of [c0, c1)
+    struct Walk { int u, row, slice, c, c1; };
+    auto start = [&](Walk& w, int u) {
+        w.u = u;
+        if (u < work) { const int blk = u / ns; w.row = blk * GV_ROWS; w.slice = u - blk * ns; w.c = w.slice * chunks / ns; w.c1 = (w.slice + 1) * chunks / ns; }
+    };
+    const unsigned char* wbase = reinterpret_cast<const unsigned char*>(a.W) + (size_t)r0 * a.K * 2 + lane * 16;
+    unsigned char* ring = gsm + (size_t)warp * DEPTH * GV_SLOT + lane * 16;
     const uint32_t ring_u32 = smem_u32(ring);
-
-    auto issue = [&](uint32_t g) {                      // segment g of this warp -> slot g % GV_DEPTH
-        if (g < nseg) {
-            const uint32_t cb = g * GV_SEG_CHUNKS;
-            const uint32_t slot = g % DEPTH;
+    const size_t row_bytes = (size_t)a.K * 2;
+    Walk wi;
+    start(wi, warp);
+    uint32_t islot = 0;
+    auto issue = [&]() {
+        if (wi.u < work) {
+            const unsigned char* src = wbase + (size_t)wi.row * row_bytes + wi.c * 512;
 #pragma unroll
-            for (int c = 0; c < GV_SEG_CHUNKS; ++c)
-                if (c_begin + cb + c < c_end)
-                    cp_async16_cg(ring_u32 + slot * GV_SEG_BYTES + c * 512, gsrc + (size_t)(cb + c) * 512);
+            for (int i = 0; i < GV_ROWS; ++i)
+                if (wi.row + i < nrows) cp_async16_cg(ring_u32 + islot * GV_SLOT + i * 512, src + i * row_bytes);
+            if (++wi.c == wi.c1) start(wi, wi.u + GV_WARPS);
         }
+        islot = islot + 1 == DEPTH ? 0 : islot + 1;
         cp_async_commit_g();
     };
     // prime the pipeline: weights do not depend on the previous kernel
 #pragma unroll
-    for (int g = 0; g < DEPTH; ++g) issue((uint32_t)g);
-    for (int i = tid; i < B * rpc; i += GV_THREADS) acc_s[i] = 0.f;
+    for (int g = 0; g < DEPTH; ++g) issue();
     // RMSNorm weights are immutable (and cold in every cache): fetch this thread's first chunk before the dependency wait
     float4 nw0 = make_float4(0.f, 0.f, 0.f, 0.f), nw1 = nw0;
     if (NORM == 1 && tid < K8) { nw0 = reinterpret_cast<const float4*>(a.norm_w)[2 * tid]; nw1 = reinterpret_cast<const float4*>(a.norm_w)[2 * tid + 1]; }
@@ -129,6 +123,12 @@ gemv_kernel(GemvArgs a) {
     pdl_wait();
     pdl_launch_dependents();
 
+    // the residual's old values travel beside the activations: read in the epilogue they put another round trip to the L2 (0.5 us) behind the dot products
+    float old[B];
+    if constexpr (EPI == GEMV_RESID) {
+#pragma unroll
+        for (int b = 0; b < B; ++b) old[b] = tid < nrows ? a.y[(size_t)b * a.ldy + r0 + tid] : 0.f;
+    }
     // --- stage activations (f32) and, if NORM, fold the RMSNorm weight in and get 1/rms ---
 #pragma unroll
     for (int b = 0; b < B; ++b) {
@@ -161,12 +161,17 @@ gemv_kernel(GemvArgs a) {
             xs[(size_t)(b * 2 + 1) * K8 + i] = hi;
         }
         if (NORM) {
-            const float tot = block_sum(ssq, red);
-            const float ms = tot / (float)(a.norm_dim > 0 ? a.norm_dim : a.K) + a.eps;
-            if (tid == 0) rstd_s[b] = NORM == 2 ? 1.f / sqrtf(ms) : rsqrtf(ms);
+            ssq = warp_sum(ssq);
+            if (lane == 0) red[b][warp] = ssq;
         }
     }
     __syncthreads();
+    // 1 / rms is first read behind the next barrier: a warp per sequence adds the warps' shares while the others start on their rows
+    if (NORM && warp < B) {
+        const float ms = warp_sum(lane < GV_WARPS ? red[warp][lane] : 0.f) / (float)(a.norm_dim > 0 ? a.norm_dim : a.K) + a.eps;
+        if (lane == 0) rstd_s[warp] = NORM == 2 ? 1.f / sqrtf(ms) : rsqrtf(ms);
+    }
+    if (NORM && a.norm_out != nullptr) __syncthreads();
     if (NORM && a.norm_out != nullptr && blockIdx.x == 0) {      // post-norm hidden state for callers that need it (TTS code predictor input)
 #pragma unroll
         for (int b = 0; b < B; ++b)
@@ -180,57 +185,62 @@ gemv_kernel(GemvArgs a) {
     }
 
     {
-        float accum[B], accum2[B];
+        constexpr int V = GV_ROWS * B;                      // sums of a unit: value i * B + b is row i of sequence b
+        Walk w;
+        uint32_t slot = 0;
+        for (start(w, warp); w.u < work; start(w, w.u + GV_WARPS)) {
+            float acc[V], acc2[V];
 #pragma unroll
-        for (int b = 0; b < B; ++b) { accum[b] = 0.f; accum2[b] = 0.f; }
-        int cur_row = -1;
-        auto flush = [&]() {
-            if (cur_row >= 0) {
+            for (int v = 0; v < V; ++v) { acc[v] = 0.f; acc2[v] = 0.f; }
+            for (; w.c < w.c1; ++w.c) {
+                cp_async_wait_g<DEPTH - 1>();               // this slot has landed (groups complete in order); a lane reads its own copies
+                uint4 q[GV_ROWS];
+#pragma unroll
+                for (int i = 0; i < GV_ROWS; ++i) q[i] = *reinterpret_cast<const uint4*>(ring + slot * GV_SLOT + i * 512);
+                const int idx = (w.c << 5) + lane;          // 8-element piece of the row
 #pragma unroll
                 for (int b = 0; b < B; ++b) {
-                    const float v = warp_sum(accum[b] + accum2[b]);
-                    if (lane == 0) atomicAdd(&acc_s[(size_t)b * rpc + cur_row], v);
-                    accum[b] = 0.f; accum2[b] = 0.f;
-                }
-            }
-        };
-        uint32_t row = c_begin / cpr, rem = c_begin - row * cpr;
-        for (uint32_t g = 0; g < nseg; ++g) {
-            cp_async_wait_g<DEPTH - 1>();               // segment g has landed (groups complete in order)
-            __syncwarp();
-            const unsigned char* sp = ring + (g % DEPTH) * GV_SEG_BYTES;
-            const uint32_t cb = c_begin + g * GV_SEG_CHUNKS;
-            uint4 w[GV_SEG_CHUNKS];
+                    const float4 xl = xs[(size_t)(b * 2 + 0) * K8 + idx];
+                    const float4 xh = xs[(size_t)(b * 2 + 1) * K8 + idx];
 #pragma unroll
-            for (int c = 0; c < GV_SEG_CHUNKS; ++c)
-                if (cb + c < c_end) w[c] = *reinterpret_cast<const uint4*>(sp + c * 512);
-#pragma unroll
-            for (int c = 0; c < GV_SEG_CHUNKS; ++c) {
-                if (cb + c < c_end) {
-                    const int idx = (int)(rem << 5) + lane;                     // 8-element chunk index in the row
-                    if ((int)row != cur_row) { flush(); cur_row = (int)row; }
-                    const float w0 = bf16lo(w[c].x), w1 = bf16hi(w[c].x), w2 = bf16lo(w[c].y), w3 = bf16hi(w[c].y);
-                    const float w4 = bf16lo(w[c].z), w5 = bf16hi(w[c].z), w6 = bf16lo(w[c].w), w7 = bf16hi(w[c].w);
-#pragma unroll
-                    for (int b = 0; b < B; ++b) {
-                        const float4 xl = xs[(size_t)(b * 2 + 0) * K8 + idx];
-                        const float4 xh = xs[(size_t)(b * 2 + 1) * K8 + idx];
-                        float t = accum[b], u = accum2[b];
-                        t = fmaf(w0, xl.x, t); u = fmaf(w4, xh.x, u);
-                        t = fmaf(w1, xl.y, t); u = fmaf(w5, xh.y, u);
-                        t = fmaf(w2, xl.z, t); u = fmaf(w6, xh.z, u);
-                        t = fmaf(w3, xl.w, t); u = fmaf(w7, xh.w, u);
-                        accum[b] = t; accum2[b] = u;
+                    for (int i = 0; i < GV_ROWS; ++i) {
+                        float t = acc[i * B + b], u = acc2[i * B + b];
+                        t = fmaf(bf16lo(q[i].x), xl.x, t); u = fmaf(bf16lo(q[i].z), xh.x, u);
+                        t = fmaf(bf16hi(q[i].x), xl.y, t); u = fmaf(bf16hi(q[i].z), xh.y, u);
+                        t = fmaf(bf16lo(q[i].y), xl.z, t); u = fmaf(bf16lo(q[i].w), xh.z, u);
+                        t = fmaf(bf16hi(q[i].y), xl.w, t); u = fmaf(bf16hi(q[i].w), xh.w, u);
+                        acc[i * B + b] = t; acc2[i * B + b] = u;
                     }
                 }
-                if (++rem == cpr) { rem = 0; ++row; }
+                issue();                                    // refill the slot just drained
+                slot = slot + 1 == DEPTH ? 0 : slot + 1;
             }
-            __syncwarp();                               // every lane has its slot data in registers
-            issue(g + DEPTH);                           // refill the slot just drained
+            // all V sums over the warp at once: each step halves the values a lane carries on
+#pragma unroll
+            for (int v = 0; v < V; ++v) acc[v] += acc2[v];
+            int id = 0, bit = 16;
+#pragma unroll
+            for (int n = V / 2; n >= 1; n >>= 1, bit >>= 1) {
+                const bool up = lane & bit;
+#pragma unroll
+                for (int v = 0; v < n; ++v) {
+                    const float give = up ? acc[v] : acc[v + n], keep = up ? acc[v + n] : acc[v];
+                    acc[v] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
+                }
+                id += up ? n : 0;
+            }
+            for (int m = bit; m > 0; m >>= 1) acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], m);
+            const int row = w.row + id / B, b = id % B;
+            if ((lane & (2 * bit - 1)) == 0 && row < nrows) acc_s[((size_t)b * rpc + row) * ns + w.slice] = acc[0];
         }
-        flush();
     }
     __syncthreads();
+    auto sum_of = [&](int b, int i) {                       // a row's slices, in order
+        const float* p = acc_s + ((size_t)b * rpc + i) * ns;
+        float v = p[0];
+        for (int k = 1; k < ns; ++k) v += p[k];
+        return v;
+    };
 
     // ------------------------------- epilogue (all threads) -------------------------------
     float bestv[B];
@@ -242,7 +252,7 @@ gemv_kernel(GemvArgs a) {
 #pragma unroll
             for (int b = 0; b < B; ++b) {
                 const float r = NORM ? rstd_s[b] : 1.f;
-                float g = acc_s[(size_t)b * rpc + 2 * u] * r, up = acc_s[(size_t)b * rpc + 2 * u + 1] * r;
+                float g = sum_of(b, 2 * u) * r, up = sum_of(b, 2 * u + 1) * r;
                 if (a.bias) { g += a.bias[r0 + 2 * u]; up += a.bias[r0 + 2 * u + 1]; }
                 a.y[(size_t)b * a.ldy + (r0 / 2 + u)] = glu_pair_f(g, up, a.glu_limit);
             }
@@ -251,13 +261,13 @@ gemv_kernel(GemvArgs a) {
         for (int i = tid; i < nrows; i += GV_THREADS) {
 #pragma unroll
             for (int b = 0; b < B; ++b) {
-                const float v = acc_s[(size_t)b * rpc + i] * (NORM ? rstd_s[b] : 1.f);
+                const float v = sum_of(b, i) * (NORM ? rstd_s[b] : 1.f);
                 float* yp = a.y + (size_t)b * a.ldy + r0 + i;
                 if constexpr (EPI == GEMV_RESID) {
                     float add = a.bias ? v + a.bias[r0 + i] : v;
                     if (a.out_scale) add *= a.out_scale[r0 + i];
                     if (a.gate) add *= 1.f / (1.f + expf(-(a.gate[(size_t)b * a.ldg + r0 + i] + (a.gate_bias ? a.gate_bias[r0 + i] : 0.f))));
-                    *yp += add;
+                    *yp = (i == tid ? old[b] : *yp) + add;
                 } else if constexpr (EPI == GEMV_RELU2) { const float p = fmaxf(v, 0.f); *yp = p * p; }
                 else *yp = v;
                 if constexpr (EPI == GEMV_LOGITS_ARGMAX) {
@@ -344,15 +354,25 @@ gemv_kernel(GemvArgs a) {
     }
 }
 
-static size_t gemv_smem_bytes(int B, int K, int N, int rows_per_unit, int grid) {
-    const int units = N / rows_per_unit;
-    const int rpc = (units + grid - 1) / grid * rows_per_unit;
-    return (size_t)GV_WARPS * gv_depth(B) * GV_SEG_BYTES + (size_t)B * K * 4 + (size_t)B * rpc * 4 + 16;
+static int gemv_rpc(int N, int rows_per_unit, int grid) { return (N / rows_per_unit + grid - 1) / grid * rows_per_unit; }
+static size_t gemv_smem_bytes(int B, int K, int rpc, int ns) { return (size_t)GV_WARPS * gv_depth(B) * GV_SLOT + (size_t)B * K * 4 + (size_t)B * rpc * ns * 4 + 16; }
+// Slices of K a CTA's rows are cut into: the fewest column chunks on the busiest warp (a unit's reduction and its first slot cost about another), while
+// the sums fit.  One slice wherever the rows are enough for the warps.
+static int gemv_slices(int B, int K, int rpc) {
+    const int chunks = K / 256, blocks = (rpc + GV_ROWS - 1) / GV_ROWS;
+    int best = 1, cost = 1 << 30;
+    for (int ns = 1; ns <= std::min(chunks, GV_WARPS); ++ns) {
+        if (ns > 1 && gemv_smem_bytes(B, K, rpc, ns) > 227 * 1024) break;
+        const int c = (blocks * ns + GV_WARPS - 1) / GV_WARPS * ((chunks + ns - 1) / ns + 1);
+        if (c < cost) { cost = c; best = ns; }
+    }
+    return best;
 }
 
 template <int B, int EPI, int NORM>
 static int gemv_launch_t(cudaStream_t st, const GemvArgs& a, int num_sms, bool pdl) {
-    const size_t smem = gemv_smem_bytes(B, a.K, a.N, EPI == GEMV_SILU_MUL ? 2 : 1, num_sms);
+    const int rpc = gemv_rpc(a.N, EPI == GEMV_SILU_MUL ? 2 : 1, num_sms), ns = gemv_slices(B, a.K, rpc);
+    const size_t smem = gemv_smem_bytes(B, a.K, rpc, ns);
     if (smem > 227 * 1024) return -1000;
     static SmemOptIn seen;
     if (const int e = ensure_dyn_smem(gemv_kernel<B, EPI, NORM>, smem, seen)) return e;
@@ -366,7 +386,7 @@ static int gemv_launch_t(cudaStream_t st, const GemvArgs& a, int num_sms, bool p
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
-    return (int)cudaLaunchKernelEx(&cfg, gemv_kernel<B, EPI, NORM>, a);
+    return (int)cudaLaunchKernelEx(&cfg, gemv_kernel<B, EPI, NORM>, a, ns);
 }
 
 template <int B>
@@ -390,7 +410,7 @@ static int gemv_launch_b(cudaStream_t st, int epi, bool norm, const GemvArgs& a,
 // Largest sequence group (4, 2 or 1) whose f32 activations fit next to the weight rings for an in_dim of K.
 int gemv_max_group(int K, int N, int num_sms) {
     for (int B : {4, 2})
-        if (gemv_smem_bytes(B, K, N, 1, num_sms) <= 227 * 1024) return B;
+        if (gemv_smem_bytes(B, K, gemv_rpc(N, 1, num_sms), 1) <= 227 * 1024) return B;
     return 1;
 }
 

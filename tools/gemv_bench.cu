@@ -1,5 +1,5 @@
 // Standalone GEMV micro-benchmark (compiled ON the GPU box so pipeline parameters can be swept in one call):
-//   nvcc -gencode arch=compute_100a,code=sm_100a -O3 -std=c++17 -DGV_WARPS=8 -DGV_DEPTH=5 tools/gemv_bench.cu crane_b200/csrc/tc.cu crane_b200/csrc/tc_scratch.cu -o /tmp/gb && /tmp/gb
+//   nvcc -gencode arch=compute_100a,code=sm_100a -O3 -std=c++17 tools/gemv_bench.cu crane_b200/csrc/tc.cu crane_b200/csrc/tc_scratch.cu -o /tmp/gb && /tmp/gb
 // 1) isolated kernels per shape (weights rotated through > L2 worth of copies), 2) the PDL-chained weight stream of a whole
 // Qwen3-VL-2B decode step (28 x [qkv, o, gate_up, down] + lm_head, attention omitted).
 #include "../crane_b200/csrc/decode.cu"
@@ -29,7 +29,7 @@ int main() {
     struct Shape { const char* name; int epi; bool norm; int N, K; };
     Shape shapes[] = {{"qkv", GEMV_STORE, true, QKV, H}, {"o", GEMV_RESID, false, H, H}, {"gate_up", GEMV_SILU_MUL, true, 2 * I, H},
                       {"down", GEMV_RESID, false, H, I}, {"lm_head", GEMV_LOGITS_ARGMAX, true, V, H}};
-    printf("GV_WARPS=%d GV_DEPTH=%d\n", GV_WARPS, GV_DEPTH);
+    printf("GV_WARPS=%d depth=%d\n", GV_WARPS, gv_depth(1));
     for (auto& s : shapes) {
         const size_t wsz = (size_t)s.N * s.K;
         const int copies = (int)std::max<size_t>(1, std::min<size_t>(total / wsz, 64));
