@@ -590,10 +590,11 @@ attn_decode_kernel(AttnDecArgs a) {
     __shared__ float q_s[NREP][D];
     __shared__ float knew_s[D], vnew_s[D];
     __shared__ float mm_s[NW][NREP], ml_s[NW][NREP];
-    __shared__ float cta_o[NREP][D];
-    __shared__ float cta_ml[NREP][2];
+    __shared__ float part_o[NREP * D + ATTN_NSPLIT];         // [split][this CTA's share of the outputs], written by the cluster's CTAs
+    __shared__ float part_ml[ATTN_NSPLIT][NREP][2];
 
     cg::cluster_group cluster = cg::this_cluster();
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");      // (waited for before the first write to another CTA's shared memory)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // a KV head whose query group is wider than NREP is served by `groups` CTA clusters of NREP query heads each (6 = 2 x 3,
     // 8 = 2 x 4, ...): kvv numbers those sub-groups, query head = kvv * NREP + h; only sub-group 0 appends the new K/V row
@@ -800,50 +801,84 @@ attn_decode_kernel(AttnDecArgs a) {
 #pragma unroll
         for (int j = 0; j < EPL; ++j) o[h][j] = 0.f;
     }
-    auto attend = [&](bool valid, const bf16* kp, const bf16* vp, const bf16* klp, const bf16* vlp) __attribute__((always_inline)) {
-        float kf[EPL], vf[EPL];
-        if (valid) {
-            const uint4 kr = *reinterpret_cast<const uint4*>(kp);
-            const uint4 vr = *reinterpret_cast<const uint4*>(vp);
-            kf[0] = bf16lo(kr.x); kf[1] = bf16hi(kr.x); kf[2] = bf16lo(kr.y); kf[3] = bf16hi(kr.y);
-            kf[4] = bf16lo(kr.z); kf[5] = bf16hi(kr.z); kf[6] = bf16lo(kr.w); kf[7] = bf16hi(kr.w);
-            vf[0] = bf16lo(vr.x); vf[1] = bf16hi(vr.x); vf[2] = bf16lo(vr.y); vf[3] = bf16hi(vr.y);
-            vf[4] = bf16lo(vr.z); vf[5] = bf16hi(vr.z); vf[6] = bf16lo(vr.w); vf[7] = bf16hi(vr.w);
-            if (split_kv) {
-                const uint4 kl = *reinterpret_cast<const uint4*>(klp);
-                const uint4 vl = *reinterpret_cast<const uint4*>(vlp);
-                kf[0] += bf16lo(kl.x); kf[1] += bf16hi(kl.x); kf[2] += bf16lo(kl.y); kf[3] += bf16hi(kl.y);
-                kf[4] += bf16lo(kl.z); kf[5] += bf16hi(kl.z); kf[6] += bf16lo(kl.w); kf[7] += bf16hi(kl.w);
-                vf[0] += bf16lo(vl.x); vf[1] += bf16hi(vl.x); vf[2] += bf16lo(vl.y); vf[3] += bf16hi(vl.y);
-                vf[4] += bf16lo(vl.z); vf[5] += bf16hi(vl.z); vf[6] += bf16lo(vl.w); vf[7] += bf16hi(vl.w);
-            }
-        } else {
-#pragma unroll
-            for (int j = 0; j < EPL; ++j) { kf[j] = 0.f; vf[j] = 0.f; }
-        }
-#pragma unroll
-        for (int h = 0; h < NREP; ++h) {
-            float s = 0.f;
-#pragma unroll
-            for (int j = 0; j < EPL; ++j) s = fmaf(qr[h][j], kf[j], s);
-#pragma unroll
-            for (int ofs = LPT / 2; ofs > 0; ofs >>= 1) s += __shfl_xor_sync(0xffffffffu, s, ofs);
-            if (valid) {
-                const float mn = fmaxf(m[h], s);
-                const float corr = __expf(m[h] - mn), p = __expf(s - mn);
-                l[h] = l[h] * corr + p;
-#pragma unroll
-                for (int j = 0; j < EPL; ++j) o[h][j] = o[h][j] * corr + p * vf[j];
-                m[h] = mn;
-            }
+    // U tokens of this lane's group at a time: their scores and shuffles are independent, and the running sums are rescaled once for all of them (token by
+    // token the chain of five dependent steps and the rescaling bound the kernel: 32 sequences
+    // of 500 tokens 38 us, 47 before; 1 of 4000 16.1 and 21.3)
+    constexpr int U = 2;
+    auto unpack = [&](float* f, const bf16* hp, const bf16* lp) __attribute__((always_inline)) {
+        const uint4 r = *reinterpret_cast<const uint4*>(hp);
+        f[0] = bf16lo(r.x); f[1] = bf16hi(r.x); f[2] = bf16lo(r.y); f[3] = bf16hi(r.y);
+        f[4] = bf16lo(r.z); f[5] = bf16hi(r.z); f[6] = bf16lo(r.w); f[7] = bf16hi(r.w);
+        if (split_kv) {
+            const uint4 q = *reinterpret_cast<const uint4*>(lp);
+            f[0] += bf16lo(q.x); f[1] += bf16hi(q.x); f[2] += bf16lo(q.y); f[3] += bf16hi(q.y);
+            f[4] += bf16lo(q.z); f[5] += bf16hi(q.z); f[6] += bf16lo(q.w); f[7] += bf16hi(q.w);
         }
     };
+    auto attend = [&](const bool* valid, const bf16* const* kp, const bf16* const* vp, int lo) __attribute__((always_inline)) {
+        float sc[U][NREP];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            float kf[EPL];
+#pragma unroll
+            for (int j = 0; j < EPL; ++j) kf[j] = 0.f;
+            if (valid[u]) unpack(kf, kp[u], kp[u] + lo);
+#pragma unroll
+            for (int h = 0; h < NREP; ++h) {
+                float s = 0.f;
+#pragma unroll
+                for (int j = 0; j < EPL; ++j) s = fmaf(qr[h][j], kf[j], s);
+                sc[u][h] = s;
+            }
+        }
+#pragma unroll
+        for (int ofs = LPT / 2; ofs > 0; ofs >>= 1)
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int h = 0; h < NREP; ++h) sc[u][h] += __shfl_xor_sync(0xffffffffu, sc[u][h], ofs);
+        if (!valid[0]) return;                          // (tokens ascend: the others are not there either)
+#pragma unroll
+        for (int h = 0; h < NREP; ++h) {
+            float mn = m[h];
+#pragma unroll
+            for (int u = 0; u < U; ++u) if (valid[u]) mn = fmaxf(mn, sc[u][h]);
+            const float corr = __expf(m[h] - mn);
+            l[h] *= corr;
+#pragma unroll
+            for (int j = 0; j < EPL; ++j) o[h][j] *= corr;
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                sc[u][h] = valid[u] ? __expf(sc[u][h] - mn) : 0.f;
+                l[h] += sc[u][h];
+            }
+            m[h] = mn;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (valid[u]) {
+                float vf[EPL];
+                unpack(vf, vp[u], vp[u] + lo);
+#pragma unroll
+                for (int h = 0; h < NREP; ++h)
+#pragma unroll
+                    for (int j = 0; j < EPL; ++j) o[h][j] = fmaf(sc[u][h], vf[j], o[h][j]);
+            }
+    };
+    bool valid[U];
+    const bf16 *kp[U], *vp[U];
     if constexpr (RING) {
-        for (int i = 0; i < n_it; ++i) {
-            asm volatile("cp.async.wait_group %0;" ::"n"(ATTN_DEPTH - 1) : "memory");
-            const bf16* p = reinterpret_cast<const bf16*>(ring + (i % ATTN_DEPTH) * 2048);
-            attend(w0 + i * NW * TPW + grp < t_end, p, p + 256, p + 512, p + 768);
-            ring_issue(i + ATTN_DEPTH);
+        static_assert(ATTN_DEPTH % U == 0, "a turn's slots are neighbours");
+        for (int i = 0; i < n_it; i += U) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(ATTN_DEPTH - U) : "memory");
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                valid[u] = w0 + (i + u) * NW * TPW + grp < t_end;
+                kp[u] = reinterpret_cast<const bf16*>(ring + ((i + u) % ATTN_DEPTH) * 2048); vp[u] = kp[u] + 256;
+            }
+            attend(valid, kp, vp, 512);
+#pragma unroll
+            for (int u = 0; u < U; ++u) ring_issue(i + u + ATTN_DEPTH);
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
     } else {
@@ -852,9 +887,13 @@ attn_decode_kernel(AttnDecArgs a) {
             asm volatile("cp.async.wait_group 0;" ::: "memory");
             __syncthreads();
             const int n = min(TILE, t_end - tb);
-            for (int r0 = warp * TPW; r0 < n; r0 += NW * TPW) {
-                const int o_ = (r0 + grp) * D + gl * EPL;
-                attend(r0 + grp < n, k_t + o_, v_t + o_, kl_t + o_, vl_t + o_);
+            for (int r0 = warp * TPW; r0 < n; r0 += U * NW * TPW) {
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int r = r0 + u * NW * TPW + grp, o_ = r * D + gl * EPL;
+                    valid[u] = r < n; kp[u] = k_t + o_; vp[u] = v_t + o_;
+                }
+                attend(valid, kp, vp, 2 * TILE * D);
             }
         }
     }
@@ -903,8 +942,13 @@ attn_decode_kernel(AttnDecArgs a) {
         }
     }
     __syncthreads();
-    // merge the warps -> this CTA's partial in shared memory
-    for (int idx = tid; idx < NREP * D; idx += 256) {
+    // merge the warps, and push the result to the CTAs that merge the splits: CTA r of the cluster finishes outputs [r * per, (r + 1) * per).  Written to where
+    // they are read, the partials take one barrier; read from where they were made they took two round trips and a second barrier (1 sequence of
+    // 128 tokens, D = 128: 4.6 us a launch among its like, 5.3 before).
+    constexpr int E = NREP * D;
+    const int per = (E + ns - 1) / ns;
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");        // every CTA of the cluster runs
+    for (int idx = tid; idx < E; idx += 256) {
         const int h = idx / D, i = idx % D;
         float M = -INFINITY;
 #pragma unroll
@@ -916,37 +960,32 @@ attn_decode_kernel(AttnDecArgs a) {
             L += ml_s[w][h] * c;
             O += mo_s[((size_t)w * NREP + h) * D + i] * c;
         }
-        cta_o[h][i] = O;
-        if (i == 0) { cta_ml[h][0] = M; cta_ml[h][1] = L; }
+        const int to = idx / per;
+        *cluster.map_shared_rank(&part_o[split * per + (idx - to * per)], to) = O;
+        if (i < ns) {                                    // (ns <= 8 < D: lane i of a head tells CTA i)
+            float* ml = cluster.map_shared_rank(&part_ml[split][h][0], i);
+            ml[0] = M; ml[1] = L;
+        }
     }
-    // ---- merge the splits of this KV group through distributed shared memory ----
     cluster.sync();
-    for (int idx = split * 256 + tid; idx < NREP * D; idx += ns * 256) {
-        const int h = idx / D, i = idx % D;
-        float ms[ATTN_NSPLIT];
+    for (int t = tid; t < per && split * per + t < E; t += 256) {
+        const int idx = split * per + t, h = idx / D, i = idx % D;
         float M = -INFINITY;
 #pragma unroll
-        for (int s = 0; s < ATTN_NSPLIT; ++s) {       // (every load issued, splits that are not there masked: a loop with an early end serialised them, 1.3 us)
-            const float* rml = cluster.map_shared_rank(&cta_ml[0][0], RING ? min(s, ns - 1) : s);
-            ms[s] = RING && s >= ns ? -INFINITY : rml[h * 2];
-            M = fmaxf(M, ms[s]);
-        }
+        for (int s = 0; s < ATTN_NSPLIT; ++s) if (!RING || s < ns) M = fmaxf(M, part_ml[s][h][0]);
         float L = 0.f, O = 0.f;
 #pragma unroll
-        for (int s = 0; s < ATTN_NSPLIT; ++s) {
-            const int rs = RING ? min(s, ns - 1) : s;
-            const float c = (ms[s] == -INFINITY) ? 0.f : __expf(ms[s] - M);
-            const float* rml = cluster.map_shared_rank(&cta_ml[0][0], rs);
-            const float* ro = cluster.map_shared_rank(&cta_o[0][0], rs);
-            L += rml[h * 2 + 1] * c;
-            O += ro[h * D + i] * c;
-        }
+        for (int s = 0; s < ATTN_NSPLIT; ++s)
+            if (!RING || s < ns) {
+                const float ms = part_ml[s][h][0], c = (ms == -INFINITY) ? 0.f : __expf(ms - M);
+                L += part_ml[s][h][1] * c;
+                O += part_o[s * per + t] * c;
+            }
         const int head = kvv * NREP + h;
         float r = O / L;
         if (a.gated) r *= 1.0f / (1.0f + expf(-qkv[head * a.q_stride + D + i]));   // y * sigmoid(gate), modeling.rs:516-523
         a.out[(size_t)b * q_dim + head * D + i] = r;
     }
-    cluster.sync();                                      // nobody exits while its shared memory is still being read
 }
 
 template <int D, int NREP, bool RING>
@@ -987,7 +1026,10 @@ int attn_decode_launch(cudaStream_t st, int B, int D, const AttnDecArgs& a_in, b
     const int nrep = a.nh / a.nkv;
     if (a.rot_half < 32 || (a.rot_half % 32) != 0 || 2 * a.rot_half > D) return -1000;
     // any group width: the widest instantiated sub-group (4, 3, 2, 1 query heads) that divides it
-    const int sub = nrep % 4 == 0 ? 4 : nrep % 3 == 0 ? 3 : nrep % 2 == 0 ? 2 : 1;
+    int sub = nrep % 4 == 0 ? 4 : nrep % 3 == 0 ? 3 : nrep % 2 == 0 ? 2 : 1;
+    // narrower ones while all their clusters still run at once: few clusters leave most of the chip idle, and a CTA's time goes with its heads, not with the
+    // bytes the sub-groups read again (1 sequence, 8 heads over 2 of D = 256: 1000 tokens 9.4 us, 12.2 before)
+    while (sub % 2 == 0 && B * a.nkv * (nrep / sub * 2) <= tc_max_clusters(ATTN_NSPLIT)) sub /= 2;
     a.groups = nrep / sub;
     // splits per (sequence, KV group): all eight while they leave SMs idle, fewer as the batch itself fills the chip (two CTAs per SM)
     const int pairs = B * a.nkv * a.groups;
