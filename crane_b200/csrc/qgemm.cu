@@ -132,23 +132,37 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
 
     // ------------------------------------------------------------------------------------------------ raw weights: 16-byte asynchronous copies
     if (warp >= W_RAW) {           // (the weights do not depend on the kernel ahead: no dependency wait)
+        // A thread's pieces sit at the same places of every super-block's 128 rows, and those of 32 rows repeat CPB pieces later: CPB offsets in registers and no
+        // arithmetic beside the copies.  (Worked out per piece, a division by CPB and a 64-bit product each, the single warp of the wide tiles took
+        // 2 us per super-block and paced the kernel: 24576 x 4096 at 64 rows Q4_K 51.5 us, 40.9 so; Q6_K at 512 rows 405 and 289.)
         const int t = threadIdx.x - W_RAW * 32;
-        constexpr uint32_t CPB = C::SB / 16;
-        const size_t row_bytes = (size_t)KB * C::SB;
-        int rs = 0; uint32_t rph = 0;
+        constexpr int CPB = C::SB / 16, T = C::RAW_WARPS * 32, GRP = 128 / T;
+        const uint32_t row_bytes = (uint32_t)KB * C::SB;
+        uint32_t off[CPB];
+#pragma unroll
+        for (int j = 0; j < CPB; ++j) { const uint32_t q = j * T + t, r = q / CPB; off[j] = r * row_bytes + (q - r * CPB) * 16; }
+        int rs = 0, kb = it_begin % KB, n0 = it_begin / KB / a.sc.tiles_m * 128, tile = it_begin / KB; uint32_t rph = 0;
         for (int it = it_begin; it < it_end; ++it) {
             wait(&raw_empty[rs], rph ^ 1);
-            const int n0 = (it / KB / a.sc.tiles_m) * 128;
-            const uint8_t* src = a.w + (size_t)n0 * row_bytes + (size_t)(it % KB) * C::SB;
+            const uint8_t* src = a.w + (size_t)n0 * row_bytes + (size_t)kb * C::SB;
             const uint32_t dst = smem_u32(sm + C::OFF_RAW + rs * C::RAW_BYTES) + t * 16;
+            if (n0 + 128 <= a.N) {
 #pragma unroll
-            for (uint32_t j = 0; j < CPB * 4 / C::RAW_WARPS; ++j) {
-                const uint32_t q = j * (C::RAW_WARPS * 32) + (uint32_t)t, r = q / CPB, c = q - r * CPB;
-                const bool in = n0 + (int)r < a.N;
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + j * (C::RAW_WARPS * 512)), "l"(src + (in ? r * row_bytes + c * 16 : 0)), "r"(in ? 16 : 0) : "memory");
+                for (int g = 0; g < GRP; ++g)
+#pragma unroll
+                    for (int j = 0; j < CPB; ++j)
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + (g * CPB + j) * (T * 16)), "l"(src + (size_t)g * T * row_bytes + off[j]) : "memory");
+            } else {                                    // the last tile: rows behind the last one are zeros
+#pragma unroll 1
+                for (int j = 0; j < CPB * GRP; ++j) {
+                    const uint32_t q = j * T + t, r = q / CPB;
+                    const bool in = n0 + (int)r < a.N;
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + j * (T * 16)), "l"(src + (in ? (size_t)r * row_bytes + (q - r * CPB) * 16 : 0)), "r"(in ? 16 : 0) : "memory");
+                }
             }
             asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&raw_full[rs])) : "memory");
             if (++rs == C::NR) { rs = 0; rph ^= 1; }
+            if (++kb == KB) { kb = 0; ++tile; n0 = tile / a.sc.tiles_m * 128; }
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
     // ------------------------------------------------------------------------------------------------ activation codes and their scales by TMA
@@ -156,9 +170,8 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
         if (lane == 0) {
             tma_prefetch_desc(&tmX);
             pdl_wait();
-            int st = 0, ds = 0; uint32_t ph = 0;
+            int st = 0, ds = 0, kb = it_begin % KB, tile = it_begin / KB, m0 = tile % a.sc.tiles_m * NT; uint32_t ph = 0;
             for (int it = it_begin; it < it_end; ++it) {
-                const int kb = it % KB, m0 = (it / KB % a.sc.tiles_m) * NT;
                 // Slot ds of the scales was last read for super-block it - 4.  Its successor's data may go in once the first stage of `it` is free: a stage
                 // at most two super-blocks back has been multiplied then, and the accumulators kept that one behind the readers of it - 4.
                 for (int g = 0; g < C::SPS; ++g) {
@@ -178,6 +191,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
                     if (mins) tma_load_2d(sm + C::OFF_B2 + (it & 1) * C::B2_BYTES, &tmS, &full[st], kb * 16, m0);
                     if (++st == C::NSTG) { st = 0; ph ^= 1; }
                 }
+                if (++kb == KB) { kb = 0; ++tile; m0 = tile % a.sc.tiles_m * NT; }
             }
             wait.drain();
         }
@@ -475,17 +489,17 @@ static int qgemm_launch_t(cudaStream_t st, const unsigned char* w, const QRows& 
 
 // Above 32 rows: tiles of 64 activation rows, or of 128 (K-quants only), which unpack a block of weights half as often but have two stages for their operands
 // instead of three and twice the partial tile to park and add for every CTA that shares one.  Estimated us of either: super-blocks on the busiest CTA,
-// CTAs per tile, a constant; fitted to 7 linears x 14 row counts (33 .. 512) at widths 1024, 2048, 4096, within 16 % (Q4_K) and 9 % (Q6_K) of each time.
+// CTAs per tile, a constant; fitted to 8 linears x 13 row counts (33 .. 512) at widths 1024, 2048, 4096: the choice is never more than 1.5 % off the better one.
 // us, 64 / 128 wide:
-//   Q4_K  6144 x 1024   128 rows 13.3 / 16.4, 256 17.7 / 21.5, 512 27.9 / 26.3    2048 x 2048   256 14.9 / 22.3, 512 21.3 / 27.0
-//         12288 x 2048  128 27.5 / 28.8, 192 36.8 / 37.0, 256 47.4 / 37.5          24576 x 4096  64 46.6 / 58.4, 65 86.1 / 58.3, 512 325 / 198
-//   Q6_K  2048 x 6144   256 35.1 / 55.9, 512 58.6 / 63.2                           4096 x 12288  192 85.4 / 101, 256 111 / 101, 512 212 / 175
+//   Q4_K  6144 x 1024   128 rows 15.5 / 23.6, 512 31.7 / 39.7                       2048 x 2048   256 13.5 / 22.1, 512 17.4 / 26.6
+//         12288 x 2048  256 44.0 / 52.2, 512 77.4 / 79.9                            24576 x 4096  65 66.8 / 70.3, 128 69.4 / 72.0, 193 126 / 120, 512 246 / 225
+//   Q6_K  2048 x 6144   256 32.9 / 57.4, 512 52.1 / 61.7                            4096 x 12288  192 74.6 / 91.4, 256 95.1 / 93.0, 512 180 / 147
 // (Q8_0 reads an accumulator per 32 elements; at width 4096 a layer took 475 us at 128 rows and 1224 at 512 with 64, 655 and 1328 with 128.)
 static float qgemm_estimate(int qt, int nt, int M, int N, int K) {
     const long long iters = (long long)((M + nt - 1) / nt) * ((N + 127) / 128) * (K / 256), G = std::max<long long>(1, std::min<long long>(tc_device_sms(), iters / 2));
     const float most = (float)((iters + G - 1) / G), sharing = (float)(K / 256) * (float)G / (float)iters;
-    if (qt == QT_Q4_K) return nt == 64 ? 2.0f * most + 0.7f * sharing + 4.6f : 2.5f * most + 2.8f * sharing + 6.2f;
-    return nt == 64 ? 2.5f * most + 0.9f * sharing + 4.6f : 4.3f * most + 6.5f * sharing - 3.6f;
+    if (qt == QT_Q4_K) return nt == 64 ? 1.32f * most + 0.39f * sharing + 7.1f : 2.34f * most + 1.5f * sharing + 12.9f;
+    return nt == 64 ? 2.13f * most + 0.5f * sharing + 7.5f : 3.36f * most + 5.f * sharing + 14.f;
 }
 
 template <int QT>
