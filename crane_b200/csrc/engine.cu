@@ -216,7 +216,7 @@ struct crane_b200_model {
     int wide_rows = 0, wide_xq_mode = -1;
     float* am_val = nullptr; int* am_idx = nullptr;
     void linear_wide(int epi, const bf16* w, const unsigned char* qw, int qt, int N, int K, const float* xin, int ldx, const float* norm_w, float* y, int ldy,
-                     int B, bool same_input = false);
+                     int B, bool same_input = false, const QSegs& segs = {});
     void enqueue_wide_step(int advance, int B);
     // ---- configuration ----
     int device = 0, num_sms = 148;
@@ -376,10 +376,10 @@ struct crane_b200_model {
     size_t last_decode_steps = 0;
     uint64_t launches = 0;
     uint64_t graph_launches[2][DECODE_GROUP_MAX + 1] = {};
-    unsigned char* xqr_buf = nullptr;  // activation rows quantised for the tensor-core linears (qrows_at), xqr_rows of them
-    int xqr_rows = 0, xqr_mode_last = -1;
     unsigned char* xq_buf = nullptr;   // activations quantised for the quantised GEMVs (xquant_launch)
     int xq_mode_last = -1;
+    unsigned char* xqr_buf = nullptr;  // activation rows quantised for the tensor-core linears (qrows_at), xqr_rows of them
+    int xqr_rows = 0, xqr_mode_last = -1;
     // Split precision (default): every bf16 activation operand / KV page has a low-order plane (x = hi + lo) so the prefill
     // tensor-core path carries ~16 mantissa bits; lo_* = element offset of that plane from the buffer base, 0 when off.
     bool split = true;
@@ -429,9 +429,25 @@ struct crane_b200_model {
     void load_gguf_file(const char* path, size_t* n_loaded, size_t* n_skipped);
     unsigned char* up_quant(int qt, const void* data, size_t rows, int K, unsigned char* dst = nullptr, size_t dst_row_pitch = 0);
     void linear_decode(int epi, bool norm, const bf16* w, const unsigned char* qw, int qt, int N, int K, const float* xin, int ldx,
-                       const float* norm_w, float* y, int ldy, const GemvArgs* extra = nullptr, int B = 1, bool reuse_xq = false);
+                       const float* norm_w, float* y, int ldy, const GemvArgs* extra = nullptr, int B = 1, bool same_input = false, const QSegs& segs = {});
     void qlinear_rows(int epi, const unsigned char* qw, int qt, int N, int K, const float* xin, int ldx, const float* norm_w, float* y, int ldy,
-                      int S, bool reuse_xq = false);
+                      int S, bool reuse_xq = false, const QSegs& segs = {});
+    // q, k and v of a quantised layer, one launch per run of neighbours of one type: f(weight, type, rows, first column, pieces, not the first)
+    template <typename F> void qkv_runs(const LayerW& l, F&& f) const {
+        const int n[3] = {nh * q_stride(), nkv * D, nkv * D}, t[3] = {l.qt_q, l.qt_k, l.qt_v};
+        const unsigned char* w[3] = {l.q_wq, l.q_wk, l.q_wv};
+        for (int i = 0, col = 0; i < 3;) {
+            int j = i + 1, rows = n[i];
+            QSegs sg;
+            for (; j < 3 && t[j] == t[i] && rows % 128 == 0; ++j) {
+                if (j == i + 1) { sg.w1 = sg.w2 = w[j]; sg.s1 = rows; sg.s2 = rows + n[j]; } else sg.w2 = w[j];
+                rows += n[j];
+            }
+            if (sg.s2 % 128 != 0) sg.s2 = (sg.s2 + 127) / 128 * 128;       // (two pieces: nothing lies behind the second)
+            f(w[i], t[i], rows, col, sg, i > 0);
+            col += rows; i = j;
+        }
+    }
     bool load_text_tensor(const std::string& n, int dt, const int64_t* shape, int ndim, const void* data);
     bool load_vision_tensor(const std::string& n, int dt, const int64_t* shape, int ndim, const void* data);
     void finalize();
@@ -1011,16 +1027,18 @@ void crane_b200_model::load_tensor_ggml(const std::string& name_in, int qt, cons
 
 // One decode-path linear: bf16 GEMV or quantised GEMV with the same fused epilogue.
 void crane_b200_model::linear_decode(int epi, bool norm, const bf16* w, const unsigned char* qw, int qt, int N, int K, const float* xin, int ldx,
-                                     const float* norm_w, float* y, int ldy, const GemvArgs* extra, int B, bool reuse_xq) {
+                                     const float* norm_w, float* y, int ldy, const GemvArgs* extra, int B, bool same_input, const QSegs& segs) {
     GemvArgs g = extra ? *extra : GemvArgs{};
     g.N = N; g.K = K; g.x = xin; g.ldx = ldx; g.norm_w = norm_w; g.eps = eps; g.y = y; g.ldy = ldy;
     if (qt) {
         QGemvArgs qa;
         g.W = reinterpret_cast<const bf16*>(qw);
-        qa.g = g; qa.qtype = qt; qa.epi = epi; qa.norm = norm ? 1 : 0; qa.xq = xq_buf;
+        if (!norm) g.norm_w = nullptr;
+        qa.g = g; qa.qtype = qt; qa.epi = epi; qa.segs = segs;
         const int xmode = xq_mode_for(qt);
-        if (!reuse_xq || xmode != xq_mode_last) {     // same input (norm, block rule) as the previous quantised linear: k and v after q
-            LAUNCH_OK(xquant_launch(stream, B, xin, ldx, K, norm ? norm_w : nullptr, eps, xmode, xq_buf, use_pdl));
+        qa.xq = xquant_apart(B, K) ? xq_buf : nullptr;
+        if (qa.xq && (!same_input || xmode != xq_mode_last)) {      // (same input, norm and block rule as the previous quantised linear: v after q and k)
+            LAUNCH_OK(xquant_launch(stream, B, xin, ldx, K, g.norm_w, eps, xmode, xq_buf, use_pdl));
             xq_mode_last = xmode;
             ++launches;
         }
@@ -1037,7 +1055,7 @@ void crane_b200_model::linear_decode(int epi, bool norm, const bf16* w, const un
 // tensor cores (qgemm.cu); fewer rows go through the decode kernels, up to four per pass over the quantised weights.
 // `reuse_xq`: the rows were quantised by the previous call (same input, same norm) -- still checked against the block rule it used.
 void crane_b200_model::qlinear_rows(int epi, const unsigned char* qw, int qt, int N, int K, const float* xin, int ldx, const float* norm_w,
-                                    float* y, int ldy, int S, bool reuse_xq) {
+                                    float* y, int ldy, int S, bool reuse_xq, const QSegs& segs) {
     if (S >= qrows_min(qt)) {
         const int mode = xq_mode_for(qt);
         const QRows xr = qrows_at(xqr_buf, xqr_rows, K);
@@ -1046,14 +1064,13 @@ void crane_b200_model::qlinear_rows(int epi, const unsigned char* qw, int qt, in
             xqr_mode_last = mode;
             ++launches;
         }
-        LAUNCH_OK(qgemm_launch(stream, qt, qw, xr, S, N, K, epi, y, ldy, use_pdl));
+        LAUNCH_OK(qgemm_launch(stream, qt, qw, xr, S, N, K, epi, y, ldy, use_pdl, segs));
         ++launches;
         return;
     }
     for (int s0 = 0; s0 < S;) {
         const int B = (S - s0 >= 4) ? 4 : (S - s0 >= 2) ? 2 : 1;
-        linear_decode(epi, norm_w != nullptr, nullptr, qw, qt, N, K, xin + (size_t)s0 * ldx, ldx, norm_w, y + (size_t)s0 * ldy, ldy, nullptr, B,
-                      reuse_xq && S <= 4);
+        linear_decode(epi, norm_w != nullptr, nullptr, qw, qt, N, K, xin + (size_t)s0 * ldx, ldx, norm_w, y + (size_t)s0 * ldy, ldy, nullptr, B, reuse_xq && S <= 4, segs);
         s0 += B;
     }
 }
@@ -1308,11 +1325,10 @@ void crane_b200_model::enqueue_decode_step(int advance, bool with_embed, int B) 
     for (int li = 0; li < L; ++li) {
         LayerW& l = layers[li];
         if (l.full) {
-            if (l.qt_q) {   // GGUF keeps q/k/v as separate quantised matrices (qwen3/modeling.rs:252-255): three GEMVs into one qkv row
-                const int qs = nh * q_stride(), kvd = nkv * D;
-                linear_decode(GEMV_STORE, true, nullptr, l.q_wq, l.qt_q, qs, H, x_dec, H, l.ln1, qkv_dec, qkv_dim(), nullptr, B);
-                linear_decode(GEMV_STORE, true, nullptr, l.q_wk, l.qt_k, kvd, H, x_dec, H, l.ln1, qkv_dec + qs, qkv_dim(), nullptr, B, true);
-                linear_decode(GEMV_STORE, true, nullptr, l.q_wv, l.qt_v, kvd, H, x_dec, H, l.ln1, qkv_dec + qs + kvd, qkv_dim(), nullptr, B, true);
+            if (l.qt_q) {   // GGUF keeps q/k/v as separate quantised matrices (qwen3/modeling.rs:252-255): GEMVs into one qkv row
+                qkv_runs(l, [&](const unsigned char* w, int t, int n, int col, const QSegs& sg, bool more) {
+                    linear_decode(GEMV_STORE, true, nullptr, w, t, n, H, x_dec, H, l.ln1, qkv_dec + col, qkv_dim(), nullptr, B, more, sg);
+                });
             } else {
                 linear_decode(GEMV_STORE, true, l.wqkv, nullptr, 0, qkv_dim(), H, x_dec, H, l.ln1, qkv_dec, qkv_dim(), nullptr, B);
             }
@@ -1443,7 +1459,7 @@ int crane_b200_model::decode_group(size_t left) const {
 // y = epi(W x) of a group's rows, f32 in and out: the rows as three bf16 planes (24 bits), or as Q8 codes in front of a quantised matrix.
 // `same_input`: the rows are as the previous call left them (same input and norm) -- still checked against the block rule it used.
 void crane_b200_model::linear_wide(int epi, const bf16* w, const unsigned char* qw, int qt, int N, int K, const float* xin, int ldx, const float* norm_w,
-                                   float* y, int ldy, int B, bool same_input) {
+                                   float* y, int ldy, int B, bool same_input, const QSegs& segs) {
     if (qt) {
         const int mode = xq_mode_for(qt);
         const QRows xr = qrows_at(xqd_buf, wide_rows, K);
@@ -1452,7 +1468,7 @@ void crane_b200_model::linear_wide(int epi, const bf16* w, const unsigned char* 
             wide_xq_mode = mode;
             ++launches;
         }
-        LAUNCH_OK(qgemm_launch(stream, qt, qw, xr, B, N, K, epi, y, ldy, use_pdl));
+        LAUNCH_OK(qgemm_launch(stream, qt, qw, xr, B, N, K, epi, y, ldy, use_pdl, segs));
     } else {
         if (!same_input) {
             LAUNCH_OK(rows_split3_launch(stream, xin, ldx, B, K, norm_w, eps, w3_buf, (long long)w3_plane, use_pdl));
@@ -1469,10 +1485,9 @@ void crane_b200_model::enqueue_wide_step(int advance, int B) {
     for (int li = 0; li < L; ++li) {
         LayerW& l = layers[li];
         if (l.qt_q) {
-            const int qs = nh * q_stride(), kvd = nkv * D;
-            linear_wide(GEMV_STORE, nullptr, l.q_wq, l.qt_q, qs, H, x_dec, H, l.ln1, qkv_dec, qkv_dim(), B);
-            linear_wide(GEMV_STORE, nullptr, l.q_wk, l.qt_k, kvd, H, x_dec, H, l.ln1, qkv_dec + qs, qkv_dim(), B, true);
-            linear_wide(GEMV_STORE, nullptr, l.q_wv, l.qt_v, kvd, H, x_dec, H, l.ln1, qkv_dec + qs + kvd, qkv_dim(), B, true);
+            qkv_runs(l, [&](const unsigned char* w, int t, int n, int col, const QSegs& sg, bool more) {
+                linear_wide(GEMV_STORE, nullptr, w, t, n, H, x_dec, H, l.ln1, qkv_dec + col, qkv_dim(), B, more, sg);
+            });
         } else {
             linear_wide(GEMV_STORE, l.wqkv, nullptr, 0, qkv_dim(), H, x_dec, H, l.ln1, qkv_dec, qkv_dim(), B);
         }
@@ -1667,15 +1682,14 @@ void crane_b200_model::prefill(const uint32_t* ids, const float* embeds, size_t 
         if (l.full) {
             spans.mark(SP_ATTN_QKV);
             if (q_qkv) {   // GGUF keeps q / k / v separate and quantised (qwen3/modeling.rs:252-255): integer dots
-                const int qs = nh * q_stride(), kvd = nkv * D;
                 const bool all = S >= std::max(qrows_min(l.qt_q), std::max(qrows_min(l.qt_k), qrows_min(l.qt_v)));
-                for (int s0 = 0; s0 < S;) {               // (a few rows: groups of up to four, the three linears of a group share their codes)
+                for (int s0 = 0; s0 < S;) {               // (a few rows: groups of up to four)
                     const int left = S - s0, B = all ? left : left >= 4 ? 4 : left >= 2 ? 2 : 1;
                     const float* xr = x + (size_t)s0 * H;
                     float* yr = qkv + (size_t)s0 * qkv_dim();
-                    qlinear_rows(GEMV_STORE, l.q_wq, l.qt_q, qs, H, xr, H, l.ln1, yr, qkv_dim(), B);
-                    qlinear_rows(GEMV_STORE, l.q_wk, l.qt_k, kvd, H, xr, H, l.ln1, yr + qs, qkv_dim(), B, true);
-                    qlinear_rows(GEMV_STORE, l.q_wv, l.qt_v, kvd, H, xr, H, l.ln1, yr + qs + kvd, qkv_dim(), B, true);
+                    qkv_runs(l, [&](const unsigned char* w, int t, int n, int col, const QSegs& sg, bool more) {
+                        qlinear_rows(GEMV_STORE, w, t, n, H, xr, H, l.ln1, yr + col, qkv_dim(), B, more, sg);
+                    });
                     s0 += B;
                 }
             } else {
@@ -2766,10 +2780,13 @@ int crane_b200_op_qlinear(int device, const float* x, size_t m, size_t k, const 
             LAUNCH_OK(qgemm_launch(nullptr, ggml_type, dw, xr, (int)m, (int)n, (int)k, GEMV_STORE, dy, (int)n, false));
         } else for (size_t s0 = 0; s0 < m;) {
             const int B = (m - s0 >= 4) ? 4 : (m - s0 >= 2) ? 2 : 1;
-            LAUNCH_OK(xquant_launch(nullptr, B, dx + s0 * k, (int)k, (int)k, dn, eps, xq_mode_for(ggml_type), dxq, false));
             QGemvArgs qa = {};
             qa.g.W = reinterpret_cast<const bf16*>(dw); qa.g.N = (int)n; qa.g.K = (int)k; qa.g.y = dy + s0 * n; qa.g.ldy = (int)n; qa.g.eps = eps;
-            qa.qtype = ggml_type; qa.epi = GEMV_STORE; qa.norm = dn ? 1 : 0; qa.xq = dxq;
+            qa.g.x = dx + s0 * k; qa.g.ldx = (int)k; qa.g.norm_w = dn; qa.qtype = ggml_type; qa.epi = GEMV_STORE;
+            if (xquant_apart(B, (int)k)) {
+                LAUNCH_OK(xquant_launch(nullptr, B, dx + s0 * k, (int)k, (int)k, dn, eps, xq_mode_for(ggml_type), dxq, false));
+                qa.xq = dxq;
+            }
             LAUNCH_OK(qgemv_launch(nullptr, B, qa, prop.multiProcessorCount, false));
             s0 += B;
         }

@@ -193,130 +193,132 @@ __device__ __forceinline__ void warp_reduce_scatter(float (&v)[N], int lane, int
 }
 
 // ------------------------------------------------------------------------------------------------ activation quantiser
-// One CTA per sequence: the (optionally RMS-normalised) activation row -> int8 blocks in exactly the shared-memory image the
-// GEMV consumes (see xq_swz), written once to global so the 148 GEMV CTAs fetch 1.5 B/element with one bulk copy each instead
-// of re-reading and re-quantising 4 B/element.  The block rule is the one candle's CPU `QMatMul::forward` applies to the
-// activations before its integer dots (`LinearLayer::Quantized`, crane-core/src/ops/linear.rs:23-48):
+// The block rule is the one candle's CPU `QMatMul::forward` applies to the activations before its integer dots (`LinearLayer::Quantized`,
+// crane-core/src/ops/linear.rs:23-48):
 //   XQ_Q8_K (Q4_K / Q6_K weights): BlockQ8K::from_float -- 256 elements; max = first element of largest magnitude, sign kept;
 //                                  iscale = -128 / max; q = min(127, round(iscale * x)); d = 1 / iscale
 //   XQ_Q8_0 (Q8_0 weights)       : BlockQ8_0::from_float -- 32 elements; d = amax / 127; q = round(x * (1 / d)); the dot uses f16(d)
 // (round = half away from zero, Rust's f32::round).  RMSNorm is applied BEFORE quantising, as the reference does
-// (rms_norm -> linear), so the GEMV epilogue has nothing left to scale.
+// (rms_norm -> linear), so the epilogues have nothing left to scale.
 constexpr int XQ_THREADS = 1024;
 __host__ __device__ inline size_t xq_seq_bytes(int K) { return (size_t)K + (size_t)(K / 32) * 8 + (size_t)(K / 16) * 4; }
 
-// ROWS: the codes leave as f16 rows for the tensor cores (quant.cuh, QRows) instead of the GEMV's shared-memory image
-template <bool ROWS>
-__global__ void __launch_bounds__(XQ_THREADS, 1)
-xquant_kernel(const float* __restrict__ x, int ldx, int K, const float* __restrict__ norm_w, float eps, int B, int mode, unsigned char* __restrict__ out, QRows rows) {
-    __shared__ float red[32];
-    const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    unsigned char* xq = out + (size_t)b * xq_seq_bytes(K);
+// A warp's 256-element super-block g of the row: the lane's eight codes; returns their scale.  norm_w: nullable.
+__device__ __forceinline__ float xq_block(int mode, const float* xrow, const float* norm_w, float rstd, int g, int lane, int (&q)[8]) {
+    const int e = g * 256 + lane * 8;
+    float v[8];
+    {
+        const float4 a0 = *reinterpret_cast<const float4*>(xrow + e), a1 = *reinterpret_cast<const float4*>(xrow + e + 4);
+        v[0] = a0.x; v[1] = a0.y; v[2] = a0.z; v[3] = a0.w; v[4] = a1.x; v[5] = a1.y; v[6] = a1.z; v[7] = a1.w;
+    }
+    if (norm_w) {
+        const float4 w0 = *reinterpret_cast<const float4*>(norm_w + e), w1 = *reinterpret_cast<const float4*>(norm_w + e + 4);
+        const float wv[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = (v[j] * rstd) * wv[j];
+    }
+    float am = 0.f, mx = 0.f;
+    int ai = 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+        if (fabsf(v[j]) > am) { am = fabsf(v[j]); mx = v[j]; ai = j; }       // strict: the first occurrence wins
+    if (mode == XQ_Q8_K) {
+        int idx = lane * 8 + ai;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float oa = __shfl_xor_sync(0xffffffffu, am, o), om = __shfl_xor_sync(0xffffffffu, mx, o);
+            const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
+            if (oa > am || (oa == am && oi < idx)) { am = oa; mx = om; idx = oi; }
+        }
+        if (am > 0.f) {
+            const float iscale = -128.f / mx;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) q[j] = (int)fminf(roundf(iscale * v[j]), 127.f);
+            return 1.f / iscale;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) q[j] = 0;
+        return 0.f;
+    }
+    am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 1));
+    am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 2));
+    const float df = am / 127.f;
+    const float id = df != 0.f ? 1.f / df : 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) q[j] = (int)roundf(v[j] * id);
+    return __half2float(__float2half_rn(df));
+}
+
+// ... of the row into the image the GEMV reads: codes (xq_swz), {d, d * sum} per 32, sums per 16
+__device__ __forceinline__ void xq_image(int mode, const float* xrow, const float* norm_w, float rstd, int K, int g, int lane, unsigned char* xq) {
     float2* dsp = reinterpret_cast<float2*>(xq + K);
     int* isp = reinterpret_cast<int*>(xq + K + (K / 32) * 8);
+    const int e = g * 256 + lane * 8;
+    int q[8];
+    const float d = xq_block(mode, xrow, norm_w, rstd, g, lane, q);
+    const uint32_t p0 = (uint32_t)(q[0] & 0xff) | ((uint32_t)(q[1] & 0xff) << 8) | ((uint32_t)(q[2] & 0xff) << 16) | ((uint32_t)(q[3] & 0xff) << 24);
+    const uint32_t p1 = (uint32_t)(q[4] & 0xff) | ((uint32_t)(q[5] & 0xff) << 8) | ((uint32_t)(q[6] & 0xff) << 16) | ((uint32_t)(q[7] & 0xff) << 24);
+    *reinterpret_cast<uint2*>(xq + xq_swz(e)) = make_uint2(p0, p1);
+    const int s8 = q[0] + q[1] + q[2] + q[3] + q[4] + q[5] + q[6] + q[7];
+    const int s16 = s8 + __shfl_xor_sync(0xffffffffu, s8, 1);
+    const int s32 = s16 + __shfl_xor_sync(0xffffffffu, s16, 2);
+    if ((lane & 1) == 0) isp[e >> 4] = s16;
+    if ((lane & 3) == 0) dsp[e >> 5] = make_float2(d, d * (float)s32);
+}
+__device__ __forceinline__ float xq_rstd(const float* xrow, int K, float eps, float* red) {
+    float ssq = 0.f;
+    for (int i = threadIdx.x * 4; i < K; i += XQ_THREADS * 4) {
+        const float4 v = *reinterpret_cast<const float4*>(xrow + i);
+        ssq += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+    }
+    return rsqrtf(block_sum(ssq, red) / (float)K + eps);
+}
+
+// One CTA per sequence: the image, written once to global for the GEMV's CTAs to fetch with one bulk copy each.
+__global__ void __launch_bounds__(XQ_THREADS, 1)
+xquant_kernel(const float* __restrict__ x, int ldx, int K, const float* __restrict__ norm_w, float eps, int mode, unsigned char* __restrict__ out) {
+    __shared__ float red[32];
+    pdl_wait();
+    pdl_launch_dependents();
+    const float* xrow = x + (size_t)blockIdx.x * ldx;
+    const float rstd = norm_w ? xq_rstd(xrow, K, eps, red) : 1.f;
+    for (int g = threadIdx.x >> 5; g < K / 256; g += XQ_THREADS / 32) xq_image(mode, xrow, norm_w, rstd, K, g, threadIdx.x & 31, out + blockIdx.x * xq_seq_bytes(K));
+}
+size_t xquant_bytes(int B, int K) { return (size_t)B * xq_seq_bytes(K); }
+int xquant_launch(cudaStream_t st, int B, const float* x, int ldx, int K, const float* norm_w, float eps, int mode, unsigned char* out, bool pdl) {
+    if ((K % 256) != 0 || B < 1 || B > 4 || (ldx % 4) != 0) return -1000;
+    return launch_k(xquant_kernel, dim3(B), dim3(XQ_THREADS), 0, st, pdl, x, ldx, K, norm_w, eps, mode, out);
+}
+
+// One CTA per row: the codes as f16 rows for the tensor cores (quant.cuh, QRows).
+__global__ void __launch_bounds__(XQ_THREADS, 1)
+xquant_rows_kernel(const float* __restrict__ x, int ldx, int K, const float* __restrict__ norm_w, float eps, int mode, QRows rows) {
+    __shared__ float red[32];
+    const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     pdl_wait();
     pdl_launch_dependents();
     const float* xrow = x + (size_t)b * ldx;
-    float rstd = 1.f;
-    if (norm_w) {
-        float ssq = 0.f;
-        for (int i = tid * 4; i < K; i += XQ_THREADS * 4) {
-            const float4 v = *reinterpret_cast<const float4*>(xrow + i);
-            ssq += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-        }
-        rstd = rsqrtf(block_sum(ssq, red) / (float)K + eps);
-    }
-    for (int g = warp; g < K / 256; g += XQ_THREADS / 32) {           // one 256-element super-block per warp pass, 8 elements per lane
+    const float rstd = norm_w ? xq_rstd(xrow, K, eps, red) : 1.f;
+    for (int g = warp; g < K / 256; g += XQ_THREADS / 32) {
         const int e = g * 256 + lane * 8;
-        float v[8];
-        {
-            const float4 a0 = *reinterpret_cast<const float4*>(xrow + e), a1 = *reinterpret_cast<const float4*>(xrow + e + 4);
-            v[0] = a0.x; v[1] = a0.y; v[2] = a0.z; v[3] = a0.w; v[4] = a1.x; v[5] = a1.y; v[6] = a1.z; v[7] = a1.w;
-        }
-        if (norm_w) {
-            const float4 w0 = *reinterpret_cast<const float4*>(norm_w + e), w1 = *reinterpret_cast<const float4*>(norm_w + e + 4);
-            const float wv[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-#pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = (v[j] * rstd) * wv[j];
-        }
-        float am = 0.f, mx = 0.f;
-        int ai = 0;
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-            if (fabsf(v[j]) > am) { am = fabsf(v[j]); mx = v[j]; ai = j; }       // strict: the first occurrence wins
         int q[8];
-        float d;
+        const float d = xq_block(mode, xrow, norm_w, rstd, g, lane, q);
+        auto pair = [&](int i, int j) { return (uint32_t)__half_as_ushort(__int2half_rn(q[i])) | ((uint32_t)__half_as_ushort(__int2half_rn(q[j])) << 16); };
+        *reinterpret_cast<uint4*>(rows.codes + (size_t)b * K + e) = make_uint4(pair(0, 2), pair(1, 3), pair(4, 6), pair(5, 7));
+        int s32 = q[0] + q[1] + q[2] + q[3] + q[4] + q[5] + q[6] + q[7];
+        s32 += __shfl_xor_sync(0xffffffffu, s32, 1);
+        s32 += __shfl_xor_sync(0xffffffffu, s32, 2);
         if (mode == XQ_Q8_K) {
-            int idx = lane * 8 + ai;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const float oa = __shfl_xor_sync(0xffffffffu, am, o), om = __shfl_xor_sync(0xffffffffu, mx, o);
-                const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-                if (oa > am || (oa == am && oi < idx)) { am = oa; mx = om; idx = oi; }
+            if (lane == 0) rows.dx[(size_t)g * rows.ldd + b] = d;
+            if ((lane & 3) == 0) {
+                unsigned short* bs = rows.bsum + (size_t)b * (K / 16) + g * 16 + (lane >> 2);
+                bs[0] = __half_as_ushort(__int2half_rn(s32 & 63));
+                bs[8] = __half_as_ushort(__int2half_rn(s32 >> 6));
             }
-            if (am > 0.f) {
-                const float iscale = -128.f / mx;
-#pragma unroll
-                for (int j = 0; j < 8; ++j) q[j] = (int)fminf(roundf(iscale * v[j]), 127.f);
-                d = 1.f / iscale;
-            } else {
-                d = 0.f;
-#pragma unroll
-                for (int j = 0; j < 8; ++j) q[j] = 0;
-            }
-        } else {
-            am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 1));
-            am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 2));
-            const float df = am / 127.f;
-            const float id = df != 0.f ? 1.f / df : 0.f;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) q[j] = (int)roundf(v[j] * id);
-            d = __half2float(__float2half_rn(df));
+        } else if ((lane & 3) == 0) {
+            rows.dx[(size_t)(e >> 5) * rows.ldd + b] = d;
         }
-        if constexpr (ROWS) {
-            auto pair = [&](int i, int j) { return (uint32_t)__half_as_ushort(__int2half_rn(q[i])) | ((uint32_t)__half_as_ushort(__int2half_rn(q[j])) << 16); };
-            *reinterpret_cast<uint4*>(rows.codes + (size_t)b * K + e) = make_uint4(pair(0, 2), pair(1, 3), pair(4, 6), pair(5, 7));
-            int s32 = q[0] + q[1] + q[2] + q[3] + q[4] + q[5] + q[6] + q[7];
-            s32 += __shfl_xor_sync(0xffffffffu, s32, 1);
-            s32 += __shfl_xor_sync(0xffffffffu, s32, 2);
-            if (mode == XQ_Q8_K) {
-                if (lane == 0) rows.dx[(size_t)g * rows.ldd + b] = d;
-                if ((lane & 3) == 0) {
-                    unsigned short* bs = rows.bsum + (size_t)b * (K / 16) + g * 16 + (lane >> 2);
-                    bs[0] = __half_as_ushort(__int2half_rn(s32 & 63));
-                    bs[8] = __half_as_ushort(__int2half_rn(s32 >> 6));
-                }
-            } else if ((lane & 3) == 0) {
-                rows.dx[(size_t)(e >> 5) * rows.ldd + b] = d;
-            }
-            continue;
-        }
-        const uint32_t p0 = (uint32_t)(q[0] & 0xff) | ((uint32_t)(q[1] & 0xff) << 8) | ((uint32_t)(q[2] & 0xff) << 16) | ((uint32_t)(q[3] & 0xff) << 24);
-        const uint32_t p1 = (uint32_t)(q[4] & 0xff) | ((uint32_t)(q[5] & 0xff) << 8) | ((uint32_t)(q[6] & 0xff) << 16) | ((uint32_t)(q[7] & 0xff) << 24);
-        *reinterpret_cast<uint2*>(xq + xq_swz(e)) = make_uint2(p0, p1);
-        const int s8 = q[0] + q[1] + q[2] + q[3] + q[4] + q[5] + q[6] + q[7];
-        const int s16 = s8 + __shfl_xor_sync(0xffffffffu, s8, 1);
-        const int s32 = s16 + __shfl_xor_sync(0xffffffffu, s16, 2);
-        if ((lane & 1) == 0) isp[e >> 4] = s16;
-        if ((lane & 3) == 0) dsp[e >> 5] = make_float2(d, d * (float)s32);
     }
-    if (!ROWS && tid == 0) reinterpret_cast<float*>(out + (size_t)B * xq_seq_bytes(K))[b] = 1.f;      // the rows are already normalised
-}
-
-size_t xquant_bytes(int B, int K) { return (size_t)B * xq_seq_bytes(K) + 16; }
-
-int xquant_launch(cudaStream_t st, int B, const float* x, int ldx, int K, const float* norm_w, float eps, int mode, unsigned char* out, bool pdl) {
-    if ((K % 256) != 0 || B < 1 || B > 4 || (ldx % 4) != 0) return -1000;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(B);
-    cfg.blockDim = dim3(XQ_THREADS);
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    return (int)cudaLaunchKernelEx(&cfg, xquant_kernel<false>, x, ldx, K, norm_w, eps, B, mode, out, QRows{});
 }
 
 // the scales' rows are read 128 columns at a time whatever the number of rows
@@ -333,7 +335,7 @@ QRows qrows_at(unsigned char* buf, int rows, int K) {
 }
 int xquant_rows_launch(cudaStream_t st, int M, const float* x, int ldx, int K, const float* norm_w, float eps, int mode, const QRows& out, bool pdl) {
     if ((K % 256) != 0 || M < 1 || M > out.ldd || (ldx % 4) != 0) return -1000;
-    return launch_k(xquant_kernel<true>, dim3(M), dim3(XQ_THREADS), 0, st, pdl, x, ldx, K, norm_w, eps, M, mode, (unsigned char*)nullptr, out);
+    return launch_k(xquant_rows_kernel, dim3(M), dim3(XQ_THREADS), 0, st, pdl, x, ldx, K, norm_w, eps, mode, out);
 }
 
 #ifndef QG_R_DEF                    // tools/qgemv_bench.cu sweeps these
@@ -362,7 +364,7 @@ qgemv_kernel(QGemvArgs qa) {
     constexpr int SLOT = QG_R * ROWB;                  // bytes per ring slot
     const GemvArgs& a = qa.g;
     extern __shared__ __align__(1024) unsigned char qsm[];
-    // layout: [rings: QG_WARPS * DEPTH * SLOT][per b: xq K | {d, d*sum} K/32 float2 | isum16 K/16 i32][1/rms B f32, 16 B][acc B * rpc f32]
+    // layout: [rings: QG_WARPS * DEPTH * SLOT][per b: xq K | {d, d*sum} K/32 float2 | isum16 K/16 i32][acc B * rpc f32]
     const int K = a.K;
     const size_t xb = (size_t)K + (size_t)(K / 32) * 8 + (size_t)(K / 16) * 4;       // bytes of quantised activation per sequence
     unsigned char* xbase = qsm + (size_t)QG_WARPS * QG_DEPTH * SLOT;
@@ -372,8 +374,9 @@ qgemv_kernel(QGemvArgs qa) {
     const int rpc = upc * rows_per_unit;
     const int r0 = blockIdx.x * rpc;
     const int nrows = max(0, min(a.N, r0 + rpc) - r0);
-    float* acc_s = reinterpret_cast<float*>(xbase + (size_t)B * xb + 16);
+    float* acc_s = reinterpret_cast<float*>(xbase + (size_t)B * xb);
     __shared__ uint64_t xbar;
+    __shared__ float red[B][QG_MAXW];
     __shared__ float wbest_v[QG_MAXW][B];
     __shared__ int wbest_i[QG_MAXW][B];
     __shared__ int is_last_s;
@@ -389,7 +392,13 @@ qgemv_kernel(QGemvArgs qa) {
     const uint32_t tpw = (ntile + QG_WARPS - 1) / QG_WARPS;
     const uint32_t t_begin = min(ntile, (uint32_t)warp * tpw), t_end = min(ntile, ((uint32_t)warp + 1) * tpw);
     const uint32_t nt = t_end - t_begin;
-    const unsigned char* wbase = reinterpret_cast<const unsigned char*>(a.W) + (size_t)r0 * spr * TR::SB;
+    const unsigned char* wbase = reinterpret_cast<const unsigned char*>(a.W);
+    const size_t row_bytes = (size_t)spr * TR::SB;
+    auto row_at = [&](uint32_t i) {                     // row i of this CTA, in whichever piece of the weight it lies
+        const int r = r0 + (int)i;
+        if (qa.segs.s1 == 0 || r < qa.segs.s1) return wbase + (size_t)r * row_bytes;
+        return r < qa.segs.s2 ? qa.segs.w1 + (size_t)(r - qa.segs.s1) * row_bytes : qa.segs.w2 + (size_t)(r - qa.segs.s2) * row_bytes;
+    };
     unsigned char* ring = qsm + (size_t)warp * QG_DEPTH * SLOT;
     const uint32_t ring_u32 = smem_u32(ring);
 
@@ -400,7 +409,7 @@ qgemv_kernel(QGemvArgs qa) {
             const uint32_t cpr = min((uint32_t)QG_KT, spr - kt * QG_KT) * (TR::SB / 16);      // 16-byte chunks per tile row
             const uint32_t dst = ring_u32 + (p % QG_DEPTH) * SLOT;
             for (uint32_t r = 0; r < nr; ++r) {
-                const unsigned char* src = wbase + ((size_t)(rg * R + r) * spr + (size_t)kt * QG_KT) * TR::SB;
+                const unsigned char* src = row_at(rg * R + r) + (size_t)kt * QG_KT * TR::SB;
                 for (uint32_t c = lane; c < cpr; c += 32)
                     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + r * ROWB + c * 16), "l"(src + (size_t)c * 16) : "memory");
             }
@@ -416,14 +425,39 @@ qgemv_kernel(QGemvArgs qa) {
     pdl_wait();
     pdl_launch_dependents();
 
-    // ---- fetch the activations quantised by xquant_kernel: one bulk copy of the ready-made shared-memory image ----
-    const uint32_t xbytes = (uint32_t)(B * xb) + 16u;
-    if (tid == 0) {
-        mbar_arrive_expect_tx(&xbar, xbytes);
-        bulk_load(xbase, qa.xq, xbytes, &xbar);
+    float old[B];                                       // (beside the activations, not behind the dots)
+    if (qa.epi == GEMV_RESID)
+#pragma unroll
+        for (int b = 0; b < B; ++b) old[b] = tid < nrows ? a.y[(size_t)b * a.ldy + r0 + tid] : 0.f;
+    // ---- the quantised activations: one bulk copy of the ready-made image, or every CTA for itself (xquant_apart) ----
+    if (qa.xq) {
+        if (tid == 0) {
+            mbar_arrive_expect_tx(&xbar, (uint32_t)(B * xb));
+            bulk_load(xbase, qa.xq, (uint32_t)(B * xb), &xbar);
+        }
+        mbar_wait(&xbar, 0);
+    } else {
+        if (a.norm_w) {
+#pragma unroll
+            for (int b = 0; b < B; ++b) {
+                float ssq = 0.f;
+                for (int i = tid * 4; i < K; i += QG_THREADS * 4) {
+                    const float4 v = *reinterpret_cast<const float4*>(a.x + (size_t)b * a.ldx + i);
+                    ssq += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+                }
+                ssq = warp_sum(ssq);
+                if (lane == 0) red[b][warp] = ssq;
+            }
+            __syncthreads();
+        }
+#pragma unroll 1
+        for (int w = warp; w < B * (int)spr; w += QG_WARPS) {
+            const int b = w / (int)spr;
+            const float rstd = a.norm_w ? rsqrtf(warp_sum(lane < QG_WARPS ? red[b][lane] : 0.f) / (float)K + a.eps) : 1.f;
+            xq_image(xq_mode_for(QT), a.x + (size_t)b * a.ldx, a.norm_w, rstd, K, w - b * (int)spr, lane, xbase + (size_t)b * xb);
+        }
+        __syncthreads();
     }
-    mbar_wait(&xbar, 0);
-    const float* rstd_s = reinterpret_cast<const float*>(xbase + (size_t)B * xb);
 
     // ---- stream this warp's tiles ----
     {
@@ -477,17 +511,14 @@ qgemv_kernel(QGemvArgs qa) {
     if (qa.epi == GEMV_SILU_MUL) {
         for (int u = tid; u < nrows / 2; u += QG_THREADS)
 #pragma unroll
-            for (int b = 0; b < B; ++b) {
-                const float r = qa.norm ? rstd_s[b] : 1.f;
-                a.y[(size_t)b * a.ldy + (r0 / 2 + u)] = silu_f(acc_s[(size_t)b * rpc + 2 * u] * r) * (acc_s[(size_t)b * rpc + 2 * u + 1] * r);
-            }
+            for (int b = 0; b < B; ++b) a.y[(size_t)b * a.ldy + (r0 / 2 + u)] = silu_f(acc_s[(size_t)b * rpc + 2 * u]) * acc_s[(size_t)b * rpc + 2 * u + 1];
     } else {
         for (int i = tid; i < nrows; i += QG_THREADS)
 #pragma unroll
             for (int b = 0; b < B; ++b) {
-                const float v = acc_s[(size_t)b * rpc + i] * (qa.norm ? rstd_s[b] : 1.f);
+                const float v = acc_s[(size_t)b * rpc + i];
                 float* yp = a.y + (size_t)b * a.ldy + r0 + i;
-                if (qa.epi == GEMV_RESID) *yp += v; else *yp = v;
+                if (qa.epi == GEMV_RESID) *yp = (i == tid ? old[b] : *yp) + v; else *yp = v;
                 if (qa.epi == GEMV_LOGITS_ARGMAX && v > bestv[b]) { bestv[b] = v; besti[b] = r0 + i; }
             }
     }
@@ -561,7 +592,7 @@ static int qgemv_launch_t(cudaStream_t st, const QGemvArgs& qa, int num_sms, boo
     const int rpu = qa.epi == GEMV_SILU_MUL ? 2 : 1;
     const int rpc = ((a.N / rpu) + num_sms - 1) / num_sms * rpu;
     const size_t xb = (size_t)a.K + (size_t)(a.K / 32) * 8 + (size_t)(a.K / 16) * 4;
-    const size_t fixed = (size_t)B * xb + 16 + (size_t)B * rpc * 4 + 16, slot = (size_t)QG_DEPTH * QG_R * QG_KT * TR::SB;
+    const size_t fixed = (size_t)B * xb + (size_t)B * rpc * 4 + 16, slot = (size_t)QG_DEPTH * QG_R * QG_KT * TR::SB;
     int QG_WARPS = qg_warps(B);
     while (QG_WARPS > 4 && fixed + QG_WARPS * slot > 226 * 1024) --QG_WARPS;
     const int QG_THREADS = QG_WARPS * 32;
@@ -593,7 +624,7 @@ static int qgemv_launch_b(cudaStream_t st, const QGemvArgs& qa, int num_sms, boo
 }
 
 int qgemv_launch(cudaStream_t st, int B, const QGemvArgs& qa, int num_sms, bool pdl) {
-    if ((qa.g.K % 256) != 0 || qa.g.N <= 0) return -1000;
+    if ((qa.g.K % 256) != 0 || qa.g.N <= 0 || (qa.g.ldx % 4) != 0) return -1000;
     if (qa.epi == GEMV_SILU_MUL && (qa.g.N % 2) != 0) return -1000;
     switch (B) {
         case 1: return qgemv_launch_b<1>(st, qa, num_sms, pdl);

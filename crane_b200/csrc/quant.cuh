@@ -21,20 +21,29 @@ inline int q_src_block_elems(int qt) { return qt == QT_Q8_0 ? 32 : 256; }
 // Host: repack `rows` rows of K elements from the ggml byte layout into the device layout (dst sized rows * K/256 * q_sb_bytes).
 void q_repack_rows(int qt, const unsigned char* src, unsigned char* dst, size_t rows, int K);
 
+// Rows of a weight that lies in up to three pieces: rows [0, s1) in the launch's own `w`, [s1, s2) in w1, the others in w2 (q, k and v of one quantised type
+// are one launch).  s1 = 0: one piece.
+struct QSegs { const unsigned char *w1 = nullptr, *w2 = nullptr; int s1 = 0, s2 = 0; };
+
 struct QGemvArgs {
-    GemvArgs g;        // W is reinterpreted as the quantised bytes; epilogue fields as for the bf16 GEMV; g.x / g.norm_w unused
+    GemvArgs g;        // W is reinterpreted as the quantised bytes; g.x, g.ldx, and (nullable) g.norm_w with g.eps: the activation rows; epilogue fields as for the bf16 GEMV
     int qtype;
     int epi;           // GemvEpi
-    int norm;          // (kept for the epilogue contract) xquant_launch already normalised the rows: the stored scale is 1
-    const unsigned char* xq;   // activations of the B sequences, quantised by xquant_launch (xquant_bytes(B, K) bytes)
+    QSegs segs;
+    const unsigned char* xq;   // the rows quantised by xquant_launch (norm included), or nullptr: the kernel quantises them itself
 };
 
-// Quantise B activation rows (f32, row stride ldx; RMS-normalised with norm_w first when non-null) for qgemv_launch, with the
-// activation block rule candle pairs with the weight type: XQ_Q8_K for Q4_K / Q6_K, XQ_Q8_0 for Q8_0 (see xquant_kernel).
+// The activation block rule candle pairs with the weight type: XQ_Q8_K for Q4_K / Q6_K, XQ_Q8_0 for Q8_0 (see xq_block).
 enum XQMode : int { XQ_Q8_0 = 0, XQ_Q8_K = 1 };
-inline int xq_mode_for(int qt) { return qt == QT_Q8_0 ? XQ_Q8_0 : XQ_Q8_K; }
+__host__ __device__ constexpr int xq_mode_for(int qt) { return qt == QT_Q8_0 ? XQ_Q8_0 : XQ_Q8_K; }
+
+// Quantise B activation rows (f32, row stride ldx; RMS-normalised with norm_w first when non-null) for qgemv_launch.
 size_t xquant_bytes(int B, int K);
 int xquant_launch(cudaStream_t st, int B, const float* x, int ldx, int K, const float* norm_w, float eps, int mode, unsigned char* out, bool pdl);
+// Does a launch of its own quantise the rows?  Up to 32 super-blocks (two per warp) every CTA of the GEMV does it for itself: the launch takes 3 - 4 us.  Beyond, 148
+// CTAs repeating it take longer.  us a call, in the GEMV / apart: two layers of width 2048 in Q8_0, four tokens 521 / 588; one layer of width 4096 in Q4_K_M,
+// four rows 192 / 156, two steps of four sequences 434 / 353.
+constexpr bool xquant_apart(int B, int K) { return B * (K / 256) > 32; }
 
 int qgemv_launch(cudaStream_t st, int B, const QGemvArgs& a, int num_sms, bool pdl);
 
@@ -50,8 +59,9 @@ struct QRows { unsigned short* codes; float* dx; unsigned short* bsum; int ldd; 
 size_t qrows_bytes(int rows, int K);
 QRows qrows_at(unsigned char* buf, int rows, int K);
 int xquant_rows_launch(cudaStream_t st, int M, const float* x, int ldx, int K, const float* norm_w, float eps, int mode, const QRows& out, bool pdl);
-// y[m, n] = epi(sum_k W[n, k] x[m, k]); epi: GEMV_STORE, GEMV_RESID or GEMV_SILU_MUL (rows of W interleaved); x quantised for W's type
-int qgemm_launch(cudaStream_t st, int qt, const unsigned char* w, const QRows& x, int M, int N, int K, int epi, float* y, int ldy, bool pdl);
+// y[m, n] = epi(sum_k W[n, k] x[m, k]); epi: GEMV_STORE, GEMV_RESID or GEMV_SILU_MUL (rows of W interleaved); x quantised for W's type.  Pieces of W end at
+// multiples of 128 rows.
+int qgemm_launch(cudaStream_t st, int qt, const unsigned char* w, const QRows& x, int M, int N, int K, int epi, float* y, int ldy, bool pdl, const QSegs& segs = {});
 // rows x K quantised -> bf16 row-major
 int q_dequant_bf16_launch(cudaStream_t st, int qt, const unsigned char* w, size_t rows, int K, bf16* out);
 // gather + dequantise rows of a quantised embedding table to f32: ids[rows] (prefill) or, with ids == nullptr, state[r].token
