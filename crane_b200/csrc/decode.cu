@@ -461,7 +461,7 @@ copy_list_kernel(const __grid_constant__ CopyList list) {
         uint4 v[4], o[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-            if (i + j * step < n) { v[j] = s[i + j * step]; if (k) o[j] = d[i + j * step]; }
+            if (i + j * step < n) { v[j] = s ? s[i + j * step] : make_uint4(0u, 0u, 0u, 0u); if (k) o[j] = d[i + j * step]; }
 #pragma unroll
         for (int j = 0; j < 4; ++j)
             if (i + j * step < n) { if (k) k[i + j * step] = o[j]; d[i + j * step] = v[j]; }

@@ -117,7 +117,7 @@ constexpr int SEQ_PACK = 64;
 struct SeqPack { SeqState s[SEQ_PACK]; };
 int set_state_launch(cudaStream_t st, SeqState* state, const SeqState* snapshots, int n);
 // Device copies of one call, a launch for up to COPY_LIST of them (56 copies of a fork took 250 us one by one: 4 us each, whatever their size).
-// dst[i] <- src[i]; with `park`, park[i] <- the old dst[i] first (src and park may be the same memory only if dst is another).  Pointers and bytes in units of 16.
+// dst[i] <- src[i], or zeros without a src; with `park`, park[i] <- the old dst[i] first (src and park may be the same memory only if dst is another).  Pointers and bytes in units of 16.
 constexpr int COPY_LIST = 64;
 struct CopySeg { void* dst; const void* src; void* park; size_t bytes; };
 struct CopyList { CopySeg s[COPY_LIST]; int n; };

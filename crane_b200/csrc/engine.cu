@@ -696,6 +696,25 @@ static void want_shape(const std::string& name, const int64_t* shape, int ndim, 
     }
 }
 
+// Copies (zeros where there is no src) of one call: pieces of 16 bytes go on the list, others (odd sizes of small models) one by one.
+struct SegList {
+    cudaStream_t stream;
+    CopyList l = {};
+    void add(void* dst, const void* src, size_t bytes, void* park = nullptr) {
+        if (((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(park) | bytes) & 15) != 0) {
+            if (park) CUDA_OK(cudaMemcpyAsync(park, dst, bytes, cudaMemcpyDeviceToDevice, stream));
+            CUDA_OK(src ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, stream) : cudaMemsetAsync(dst, 0, bytes, stream));
+            return;
+        }
+        if (l.n == COPY_LIST) flush();
+        l.s[l.n++] = CopySeg{dst, src, park, bytes};
+    }
+    void flush() {
+        LAUNCH_OK(copy_list_launch(stream, l));
+        l.n = 0;
+    }
+};
+
 #include "engine_fosovik.inc"
 
 bool crane_b200_model::load_text_tensor(const std::string& n, int dt, const int64_t* shape, int ndim, const void* data) {
@@ -1360,25 +1379,6 @@ void crane_b200_model::gdn_args(GdnArgs& g, const LayerW& l, int S, const float*
     g.conv_w = l.conv_w; g.conv_state = l.conv_state; g.neg_exp_a = l.neg_exp_a; g.dt_bias = l.dt_bias; g.norm_w = l.gnorm; g.eps = eps;
     g.rec_state = l.rec_state; g.conv_out = conv; g.qn = qn; g.kn = kn; g.gb = gb; g.y = y;
 }
-
-// Copies of one call: pieces of 16 bytes go on the list, others (odd sizes of small models) one by one.
-struct SegList {
-    cudaStream_t stream;
-    CopyList l = {};
-    void add(void* dst, const void* src, size_t bytes, void* park = nullptr) {
-        if (((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(park) | bytes) & 15) != 0) {
-            if (park) CUDA_OK(cudaMemcpyAsync(park, dst, bytes, cudaMemcpyDeviceToDevice, stream));
-            CUDA_OK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, stream));
-            return;
-        }
-        if (l.n == COPY_LIST) flush();
-        l.s[l.n++] = CopySeg{dst, src, park, bytes};
-    }
-    void flush() {
-        LAUNCH_OK(copy_list_launch(stream, l));
-        l.n = 0;
-    }
-};
 
 void crane_b200_model::select_seq(int s) {
     if (s == cur) return;

@@ -3,7 +3,8 @@
 // B200 design: a persistent kernel, one CTA per SM, stream-K over the (128 x BN output tile, 64-wide k-step) iteration space; A and W
 // tiles stream HBM/L2 -> shared memory by TMA (cp.async.bulk.tensor, SWIZZLE_128B) through a multi-stage mbarrier ring; one elected
 // thread issues tcgen05.mma (UMMA 128 x BN x 16, bf16 x bf16 -> f32) into a double-buffered TMEM accumulator; eight epilogue warps
-// pull it back with tcgen05.ld, apply the fused epilogue (bias / residual add / SiLU*up / GELU / dtype cast) and hand it to TMA stores and adds, or park a partial tile for the tile's last contributor to sum in a fixed order (see gemm.cu).
+// pull it back with tcgen05.ld, apply the fused epilogue (bias / residual add / SiLU*up / GELU / dtype cast) and hand it to TMA stores and
+// adds, or park a partial tile for the tile's last contributor to sum in a fixed order (see gemm.cu).
 //
 // Replaces the cuBLAS GEMMs Candle launches for every `Linear` on the reference's GPU path and the
 // f32 gemm on its CPU path (crane-core/src/models/qwen3/modeling.rs:318-329,532,608-642;

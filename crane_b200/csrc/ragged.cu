@@ -659,12 +659,17 @@ __global__ void conv_window_kernel(RaggedBatch rb, Mamba2Args a, int C, int col0
     }
 }
 
-// Selective scan.  Block = (entry, head, slice of SSD_COLS value columns); thread (p, ns) owns state rows n = ns, ns + 8, ... of
-// column p in registers for the whole portion.  The recurrence itself is one FMA deep per token; what would serialise it is the
+// Selective scan.  Block = (entry, head, slice of SSD_COLS value columns); thread (p, ns) owns a run of state rows of
+// columns p and p + 16 in registers for the whole portion.  The recurrence itself is one FMA deep per token; what would serialise it is the
 // operand fetch, so the step inputs (x slice, B, C, dt) of SSD_CH tokens at a time are staged in shared memory with cp.async,
 // double-buffered: chunk c + 1 is in flight while chunk c is consumed.  dt = softplus(.) and the decay exp(-exp(A) dt) are
 // computed once per token, in f32, when its chunk lands.
-constexpr int SSD_NS = 8, SSD_MAXR = 32, SSD_COLS = 16, SSD_CH = 16;      // N <= 256; 16 columns x 8 = 128 threads per block: one warp per scheduler, many blocks
+// What bounds it: the instructions between one token and the next in the one warp a scheduler has.  A thread owns its state rows of SSD_CPT columns, so that B
+// and C, most of what a token reads from shared memory, are read once for both, and the outputs of four tokens are summed over the lanes together.
+// us, 16 heads of 128 x 128, one column and three shuffles a token / so: steps with a portion of 256 tokens 98 / 74, five entries 42 / 29.  (Segments from
+// 64 rows on gained nothing more for such portions: their second pass and the prefix take what they save.)
+constexpr int SSD_NS = 8, SSD_MAXR = 32, SSD_CPT = 2, SSD_COLS = 16 * SSD_CPT, SSD_CH = 16;      // N <= 256
+constexpr int SSD_TH = SSD_COLS / SSD_CPT * SSD_NS;         // 128 threads: one warp per scheduler, many blocks
 // Staged layout of one token: x slice [SSD_COLS] | B | C | dt, pad.  Thread ns owns the CONTIGUOUS state rows ns * R .. ns * R + R - 1,
 // so it reads its B and C values as float4; every R-run is followed by 4 pad floats, which spreads the eight runs of a warp over
 // all banks.
@@ -675,33 +680,39 @@ __host__ __device__ inline int ssd_npad(int N, int R) { (void)N; return 8 * (R +
 //   S_end(segment) = (product of the segment's decays) * S_start + S_local(segment run from zero).
 // MODE 1 runs every segment from zero and leaves S_local and the decay product; ssd_seg_prefix_kernel turns them into each segment's
 // start state (and the sequence's new state); MODE 2 is the scan proper from those start states.  MODE 0 = one segment, everything.
-constexpr int SSD_SEGS = 4, SSD_SEG_MIN = 512;              // segmented from this many rows in the longest entry
+constexpr int SSD_SEGS = 4, SSD_SEG_MIN = 512;              // an entry is segmented from this many rows on
 __host__ __device__ inline int ssd_seg_len(int len) { return ((len + SSD_SEGS - 1) / SSD_SEGS + SSD_CH - 1) / SSD_CH * SSD_CH; }
 template <int SSD_R, int MODE>                               // state rows per thread: ceil(N / 8) rounded up to 4, 8, 16 or 32
-__global__ void __launch_bounds__(SSD_COLS * SSD_NS) ssd_scan_kernel(RaggedBatch rb, Mamba2Args a, int C) {
+__global__ void __launch_bounds__(SSD_TH) ssd_scan_kernel(RaggedBatch rb, Mamba2Args a, int C) {
     extern __shared__ __align__(16) float ssm_s[];
     const int e = MODE == 0 ? blockIdx.x : blockIdx.x / SSD_SEGS, seg = MODE == 0 ? 0 : blockIdx.x % SSD_SEGS;
     const int h = blockIdx.y, ns = threadIdx.x & (SSD_NS - 1), pl = threadIdx.x / SSD_NS;
-    const int p0 = blockIdx.z * SSD_COLS, p = p0 + pl;
+    const int p0 = blockIdx.z * SSD_COLS;
     const int P = a.P, N = a.N, inner = a.heads * P, g = h / (a.heads / a.groups);
-    const bool live = p < P;
+    bool live[SSD_CPT];
+#pragma unroll
+    for (int j = 0; j < SSD_CPT; ++j) live[j] = p0 + pl + 16 * j < P;
     const int full_len = rb.ent_len[e], slot = rb.ent_slot[e];
-    const int seg_len = MODE == 0 ? full_len : ssd_seg_len(full_len), seg0 = seg * seg_len;
-    if (seg0 >= full_len) return;                             // (a short entry has fewer segments)
+    const bool whole = MODE == 0 || full_len < SSD_SEG_MIN;   // (a short entry beside long ones: as by itself, all of it in MODE 2)
+    if (MODE == 1 && whole) return;
+    const int seg_len = whole ? full_len : ssd_seg_len(full_len), seg0 = seg * seg_len;
+    if (seg0 >= full_len) return;                             // (fewer segments than SSD_SEGS)
     const int len = min(seg_len, full_len - seg0), r0 = rb.ent_row0[e] + seg0;
     const int ncol = min(SSD_COLS, P - p0);
     const int NP = ssd_npad(N, SSD_R), per_tok = SSD_COLS + 2 * NP + 4;
     float* stage[2] = {ssm_s, ssm_s + SSD_CH * per_tok};
     float* sdt = ssm_s + 2 * SSD_CH * per_tok;                // [SSD_CH] dt, [SSD_CH] decay
-    float* S = MODE == 0 ? a.ssm_state + (((size_t)slot * a.heads + h) * N) * P
+    float* S = whole ? a.ssm_state + (((size_t)slot * a.heads + h) * N) * P
                          : a.seg_state + ((((size_t)e * SSD_SEGS + seg) * a.heads + h) * N) * P;
     const int n0 = ns * SSD_R;
     // rows past N and tokens past the portion's end multiply zeros: the stages start zeroed and only real values are ever copied in
     for (int i = threadIdx.x; i < 2 * SSD_CH * per_tok; i += blockDim.x) ssm_s[i] = 0.f;
     __syncthreads();
-    float s[SSD_R];
+    float s[SSD_CPT][SSD_R];
 #pragma unroll
-    for (int i = 0; i < SSD_R; ++i) s[i] = (MODE != 1 && n0 + i < N && live) ? S[(size_t)(n0 + i) * P + p] : 0.f;
+    for (int i = 0; i < SSD_R; ++i)
+#pragma unroll
+        for (int j = 0; j < SSD_CPT; ++j) s[j][i] = (MODE != 1 && n0 + i < N && live[j]) ? S[(size_t)(n0 + i) * P + p0 + pl + 16 * j] : 0.f;
     float dprod = 1.f;                                        // MODE 1, thread 0: product of the segment's decays
     const float negA = -__expf(a.A_log[h]), Dh = a.D[h], dtb = a.dt_bias[h];
     const int dtcol = 2 * inner + 2 * a.groups * N + h;
@@ -753,57 +764,86 @@ __global__ void __launch_bounds__(SSD_COLS * SSD_NS) ssd_scan_kernel(RaggedBatch
         __syncthreads();
         if (MODE == 1 && threadIdx.x == 0) for (int t = 0; t < nt; ++t) dprod *= sdt[SSD_CH + t];
         const int tmax = (nt + 3) & ~3;                       // whole groups of four: the padding tokens leave the state as it is
-#pragma unroll 4
-        for (int t = 0; t < tmax; ++t) {
-            const float* tk = st + t * per_tok;
-            const float dt = sdt[t], decay = sdt[SSD_CH + t];
-            const float xv = live ? tk[pl] : 0.f;
-            const float4* B4 = reinterpret_cast<const float4*>(tk + SSD_COLS + ssd_idx(n0, SSD_R));
-            const float4* C4 = reinterpret_cast<const float4*>(tk + SSD_COLS + NP + ssd_idx(n0, SSD_R));
-            const float dx = dt * xv;
-            if (MODE == 1) {                                  // state only
+#pragma unroll 1
+        for (int t4 = 0; t4 < tmax; t4 += 4) {                // four tokens: their outputs' sums over the eight lanes are formed together (7 shuffles, not 3 each)
+            float y[4 * SSD_CPT];                             // value tt * SSD_CPT + j: token t4 + tt, column j
+#pragma unroll
+            for (int tt = 0; tt < 4; ++tt) {
+                const int t = t4 + tt;
+                const float* tk = st + t * per_tok;
+                const float dt = sdt[t], decay = sdt[SSD_CH + t];
+                float dx[SSD_CPT];
+#pragma unroll
+                for (int j = 0; j < SSD_CPT; ++j) dx[j] = dt * (live[j] ? tk[pl + 16 * j] : 0.f);
+                const float4* B4 = reinterpret_cast<const float4*>(tk + SSD_COLS + ssd_idx(n0, SSD_R));
+                const float4* C4 = reinterpret_cast<const float4*>(tk + SSD_COLS + NP + ssd_idx(n0, SSD_R));
+                float y0[SSD_CPT], y1[SSD_CPT];
+#pragma unroll
+                for (int j = 0; j < SSD_CPT; ++j) y0[j] = y1[j] = 0.f;
 #pragma unroll
                 for (int i = 0; i < SSD_R / 4; ++i) {
                     const float4 b = B4[i];
-                    s[4 * i] = fmaf(decay, s[4 * i], b.x * dx); s[4 * i + 1] = fmaf(decay, s[4 * i + 1], b.y * dx);
-                    s[4 * i + 2] = fmaf(decay, s[4 * i + 2], b.z * dx); s[4 * i + 3] = fmaf(decay, s[4 * i + 3], b.w * dx);
+#pragma unroll
+                    for (int j = 0; j < SSD_CPT; ++j) {
+                        s[j][4 * i] = fmaf(decay, s[j][4 * i], b.x * dx[j]); s[j][4 * i + 1] = fmaf(decay, s[j][4 * i + 1], b.y * dx[j]);
+                        s[j][4 * i + 2] = fmaf(decay, s[j][4 * i + 2], b.z * dx[j]); s[j][4 * i + 3] = fmaf(decay, s[j][4 * i + 3], b.w * dx[j]);
+                    }
+                    if constexpr (MODE != 1) {                // (MODE 1: state only)
+                        const float4 cc = C4[i];
+#pragma unroll
+                        for (int j = 0; j < SSD_CPT; ++j) {
+                            y0[j] = fmaf(s[j][4 * i], cc.x, y0[j]); y1[j] = fmaf(s[j][4 * i + 1], cc.y, y1[j]);
+                            y0[j] = fmaf(s[j][4 * i + 2], cc.z, y0[j]); y1[j] = fmaf(s[j][4 * i + 3], cc.w, y1[j]);
+                        }
+                    }
                 }
-                continue;
-            }
-            float y0 = 0.f, y1 = 0.f;
 #pragma unroll
-            for (int i = 0; i < SSD_R / 4; ++i) {
-                const float4 b = B4[i], cc = C4[i];
-                { s[4 * i]     = fmaf(decay, s[4 * i],     b.x * dx); y0 = fmaf(s[4 * i],     cc.x, y0); }
-                { s[4 * i + 1] = fmaf(decay, s[4 * i + 1], b.y * dx); y1 = fmaf(s[4 * i + 1], cc.y, y1); }
-                { s[4 * i + 2] = fmaf(decay, s[4 * i + 2], b.z * dx); y0 = fmaf(s[4 * i + 2], cc.z, y0); }
-                { s[4 * i + 3] = fmaf(decay, s[4 * i + 3], b.w * dx); y1 = fmaf(s[4 * i + 3], cc.w, y1); }
+                for (int j = 0; j < SSD_CPT; ++j) y[tt * SSD_CPT + j] = y0[j] + y1[j];
             }
-            float y = y0 + y1;
+            if constexpr (MODE != 1) {
+                static_assert(4 * SSD_CPT == SSD_NS, "a value per lane");
+                int id = 0;
 #pragma unroll
-            for (int o = SSD_NS / 2; o > 0; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
-            if (ns == 0 && live && t < nt) a.y[(size_t)(r0 + c * SSD_CH + t) * inner + h * P + p] = y + Dh * xv;
+                for (int n = SSD_NS / 2; n >= 1; n >>= 1) {
+                    const bool up = ns & n;
+#pragma unroll
+                    for (int v = 0; v < n; ++v) {
+                        const float give = up ? y[v] : y[v + n], keep = up ? y[v + n] : y[v];
+                        y[v] = keep + __shfl_xor_sync(0xffffffffu, give, n);
+                    }
+                    id += up ? n : 0;
+                }
+                const int t = t4 + id / SSD_CPT, col = pl + 16 * (id % SSD_CPT);
+                if (p0 + col < P && t < nt) a.y[(size_t)(r0 + c * SSD_CH + t) * inner + h * P + p0 + col] = y[0] + Dh * st[t * per_tok + col];
+            }
         }
         __syncthreads();                                      // the stage is free for chunk c + 2
     }
-    if (MODE == 2) return;                                    // the prefix kernel already wrote the sequence's new state
+    if (MODE == 2 && !whole) return;                          // the prefix kernel already wrote the sequence's new state
 #pragma unroll
-    for (int i = 0; i < SSD_R; ++i) if (n0 + i < N && live) S[(size_t)(n0 + i) * P + p] = s[i];
+    for (int i = 0; i < SSD_R; ++i)
+#pragma unroll
+        for (int j = 0; j < SSD_CPT; ++j) if (n0 + i < N && live[j]) S[(size_t)(n0 + i) * P + p0 + pl + 16 * j] = s[j][i];
     if (MODE == 1 && threadIdx.x == 0 && blockIdx.z == 0) a.seg_decay[((size_t)e * SSD_SEGS + seg) * a.heads + h] = dprod;
 }
 // Start state of every segment, in order: seg_state[k] holds S_local on entry and S_start(k) on exit; the slot gets the end state.
 __global__ void ssd_seg_prefix_kernel(RaggedBatch rb, Mamba2Args a) {
     const int e = blockIdx.x, h = blockIdx.y, np = a.N * a.P;
-    const int len = rb.ent_len[e], slot = rb.ent_slot[e], nseg = (len + ssd_seg_len(len) - 1) / ssd_seg_len(len);
+    const int len = rb.ent_len[e], slot = rb.ent_slot[e];
+    if (len < SSD_SEG_MIN) return;
+    const int nseg = (len + ssd_seg_len(len) - 1) / ssd_seg_len(len);
     float* S = a.ssm_state + ((size_t)slot * a.heads + h) * np;
     for (int i = blockIdx.z * blockDim.x + threadIdx.x; i < np; i += gridDim.z * blockDim.x) {
-        float cur = S[i];
-        for (int k = 0; k < nseg; ++k) {
-            float* loc = a.seg_state + (((size_t)e * SSD_SEGS + k) * a.heads + h) * np + i;
-            const float l = *loc;
-            *loc = cur;
-            cur = fmaf(a.seg_decay[((size_t)e * SSD_SEGS + k) * a.heads + h], cur, l);
-        }
+        float cur = S[i], l[SSD_SEGS], d[SSD_SEGS];
+        const size_t at = ((size_t)e * SSD_SEGS * a.heads + h) * np + i, step = (size_t)a.heads * np;
+#pragma unroll
+        for (int k = 0; k < SSD_SEGS; ++k) if (k < nseg) { l[k] = a.seg_state[at + k * step]; d[k] = a.seg_decay[((size_t)e * SSD_SEGS + k) * a.heads + h]; }      // in flight together
+#pragma unroll
+        for (int k = 0; k < SSD_SEGS; ++k)
+            if (k < nseg) {
+                a.seg_state[at + k * step] = cur;
+                cur = fmaf(d[k], cur, l[k]);
+            }
         S[i] = cur;
     }
 }
@@ -1330,7 +1370,7 @@ int mamba2_mixer_launch(cudaStream_t st, const RaggedBatch& rb, const Mamba2Args
         }
     }
     const dim3 sgrid(rb.E, a.heads, (a.P + SSD_COLS - 1) / SSD_COLS);
-    const int nr = (a.N + SSD_NS - 1) / SSD_NS, sthreads = SSD_COLS * SSD_NS;
+    const int nr = (a.N + SSD_NS - 1) / SSD_NS, sthreads = SSD_TH;
     const int rr = nr <= 4 ? 4 : nr <= 8 ? 8 : nr <= 16 ? 16 : 32;
     const size_t ssm = (size_t)(2 * SSD_CH * (SSD_COLS + 2 * ssd_npad(a.N, rr) + 4) + 2 * SSD_CH) * sizeof(float);      // <= 78 KB at N = 256
     const bool segs = a.seg_state != nullptr && a.max_len >= SSD_SEG_MIN;
@@ -1348,7 +1388,7 @@ int mamba2_mixer_launch(cudaStream_t st, const RaggedBatch& rb, const Mamba2Args
     } else {
         const dim3 ggrid(rb.E * SSD_SEGS, a.heads, sgrid.z);
         if ((e = scan(ssd_scan_kernel<4, 1>, ssd_scan_kernel<8, 1>, ssd_scan_kernel<16, 1>, ssd_scan_kernel<32, 1>, seen1, ggrid))) return e;
-        ssd_seg_prefix_kernel<<<dim3(rb.E, a.heads, 8), 256, 0, st>>>(rb, a);
+        ssd_seg_prefix_kernel<<<dim3(rb.E, a.heads, std::min(32, (a.N * a.P + 255) / 256)), 256, 0, st>>>(rb, a);
         if ((e = last_err())) return e;
         if ((e = scan(ssd_scan_kernel<4, 2>, ssd_scan_kernel<8, 2>, ssd_scan_kernel<16, 2>, ssd_scan_kernel<32, 2>, seen2, ggrid))) return e;
     }
