@@ -560,7 +560,7 @@ static GemmPlan gemm_plan(int mode, int M, int N, int K, bool split, int sms) {
         const double whole = fixed + (double)per * KB * tk;
         const double it = std::max((double)tiles * KB / sms, (double)g_gemm_minit);
         const double contrib = KB / it + 1.0;
-        const double sk = fixed + it * (split && bn == 256 ? 0.66 : tk) + contrib * (bn == 256 ? 2.3 : bn == 128 ? 1.9 : 1.3);
+        const double sk = fixed + it * (bn == 256 ? (split ? 0.66 : 0.42) : tk) + contrib * (bn == 256 ? 2.3 : bn == 128 ? 1.9 : 1.3);
         if (g_mode != 2 && whole < best.cost) best = GemmPlan{bn, false, whole};
         // stream-K only below one wave of whole tiles: above it the extra partial-tile traffic costs more than the idle SMs
         if (g_mode != 1 && (tiles < sms || g_mode == 2) && tiles * KB >= 2LL * sms && sk < best.cost) best = GemmPlan{bn, true, sk};
