@@ -265,14 +265,19 @@ __device__ __forceinline__ void xq_image(int mode, const float* xrow, const floa
     if ((lane & 1) == 0) isp[e >> 4] = s16;
     if ((lane & 3) == 0) dsp[e >> 5] = make_float2(d, d * (float)s32);
 }
-__device__ __forceinline__ float xq_rstd(const float* xrow, int K, float eps, float* red) {
+// Sum of squares of a row, in ONE order whatever the launch: thread t of XQ_THREADS adds its pieces of four, a warp its lanes, 32 warps' sums last.  The scale of a row
+// decides which of two codes a value on their border takes, and a flipped code moves an output by 1 / 128 of its block: another order (the warps a GEMV happens to
+// have) gave a row other codes alone than in a group or a prompt.  Threads with 4 t >= K have nothing to add.
+__device__ __forceinline__ float xq_ssq(const float* xrow, int K, int t) {
     float ssq = 0.f;
-    for (int i = threadIdx.x * 4; i < K; i += XQ_THREADS * 4) {
+    for (int i = t * 4; i < K; i += XQ_THREADS * 4) {
         const float4 v = *reinterpret_cast<const float4*>(xrow + i);
         ssq += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
     }
-    return rsqrtf(block_sum(ssq, red) / (float)K + eps);
+    return ssq;
 }
+__device__ __forceinline__ float xq_rstd_of(float total, int K, float eps) { return rsqrtf(total / (float)K + eps); }
+__device__ __forceinline__ float xq_rstd(const float* xrow, int K, float eps, float* red) { return xq_rstd_of(block_sum(xq_ssq(xrow, K, threadIdx.x), red), K, eps); }
 
 // One CTA per sequence: the image, written once to global for the GEMV's CTAs to fetch with one bulk copy each.
 __global__ void __launch_bounds__(XQ_THREADS, 1)
@@ -376,7 +381,7 @@ qgemv_kernel(QGemvArgs qa) {
     const int nrows = max(0, min(a.N, r0 + rpc) - r0);
     float* acc_s = reinterpret_cast<float*>(xbase + (size_t)B * xb);
     __shared__ uint64_t xbar;
-    __shared__ float red[B][QG_MAXW];
+    __shared__ float red[B][32];
     __shared__ float wbest_v[QG_MAXW][B];
     __shared__ int wbest_i[QG_MAXW][B];
     __shared__ int is_last_s;
@@ -437,23 +442,25 @@ qgemv_kernel(QGemvArgs qa) {
         }
         mbar_wait(&xbar, 0);
     } else {
+        const int nvw = min(32, (K + 127) / 128);           // of xq_ssq's 32 warps, those with anything to add
         if (a.norm_w) {
+#pragma unroll 1
+            for (int vw = warp; vw < nvw; vw += QG_WARPS) {
+                float ssq[B];
 #pragma unroll
-            for (int b = 0; b < B; ++b) {
-                float ssq = 0.f;
-                for (int i = tid * 4; i < K; i += QG_THREADS * 4) {
-                    const float4 v = *reinterpret_cast<const float4*>(a.x + (size_t)b * a.ldx + i);
-                    ssq += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+                for (int b = 0; b < B; ++b) ssq[b] = xq_ssq(a.x + (size_t)b * a.ldx, K, vw * 32 + lane);
+#pragma unroll
+                for (int b = 0; b < B; ++b) {
+                    ssq[b] = warp_sum(ssq[b]);
+                    if (lane == 0) red[b][vw] = ssq[b];
                 }
-                ssq = warp_sum(ssq);
-                if (lane == 0) red[b][warp] = ssq;
             }
             __syncthreads();
         }
 #pragma unroll 1
         for (int w = warp; w < B * (int)spr; w += QG_WARPS) {
             const int b = w / (int)spr;
-            const float rstd = a.norm_w ? rsqrtf(warp_sum(lane < QG_WARPS ? red[b][lane] : 0.f) / (float)K + a.eps) : 1.f;
+            const float rstd = a.norm_w ? xq_rstd_of(warp_sum(lane < nvw ? red[b][lane] : 0.f), K, a.eps) : 1.f;
             xq_image(xq_mode_for(QT), a.x + (size_t)b * a.ldx, a.norm_w, rstd, K, w - b * (int)spr, lane, xbase + (size_t)b * xb);
         }
         __syncthreads();

@@ -101,3 +101,23 @@ def test_prompts_at_the_line(recipe):
 def test_wide_row_tiles(qt, m, n, k):
     """Enough work for every block that tiles of 128 rows are taken."""
     test_rows_against_integer_dots(qt, m, n, k)
+
+
+@pytest.mark.parametrize("qt", ["Q4_K", "Q6_K", "Q8_0"])
+@pytest.mark.parametrize("k", [256, 1280, 2048, 4096])
+def test_codes_of_a_row_are_its_own(qt, k):
+    """A row behind a folded-in norm has the same 8-bit codes alone, in groups of two and four, and in a prompt.  Every value lies on the border of two codes, so a
+    last bit of 1 / rms decides for many at once; one code the other way moves a result by (1 / 128) / (0.58 sqrt(k)) of its size, 2e-4 at k = 4096, while
+    the order of the additions alone keeps within BAR."""
+    import crane_b200
+    rng = np.random.default_rng(k + len(qt))
+    top, blk = (127.0, 32) if qt == "Q8_0" else (128.0, 256)
+    x = (rng.integers(0, int(top) - 1, (12, k)) + 0.5).astype(np.float32) * rng.choice([-1.0, 1.0], (12, k)).astype(np.float32)
+    x[:, ::blk] = top
+    x *= rng.uniform(0.1, 1.0, (12, 1)).astype(np.float32)      # (so that squares round)
+    raw = blocks(rng, 384, k, qt)
+    run = lambda rows: crane_b200.op_qlinear(rows, raw, gq.GGML_TYPE_ID[qt], 384, norm_w=np.ones(k, np.float32))  # noqa: E731
+    prompt = run(x)                                     # 12 rows: tensor cores
+    for n in (1, 2, 4):
+        got = np.concatenate([run(x[i:i + n]) for i in range(0, 12, n)])
+        assert (np.abs(got - prompt).max(1) <= BAR * np.abs(prompt).max(1)).all(), n
