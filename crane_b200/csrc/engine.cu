@@ -216,7 +216,7 @@ struct crane_b200_model {
     int wide_rows = 0, wide_xq_mode = -1;
     float* am_val = nullptr; int* am_idx = nullptr;
     void linear_wide(int epi, const bf16* w, const unsigned char* qw, int qt, int N, int K, const float* xin, int ldx, const float* norm_w, float* y, int ldy,
-                     int B, bool same_input = false, const QSegs& segs = {});
+                     int B, bool same_input = false);
     void enqueue_wide_step(int advance, int B);
     // ---- configuration ----
     int device = 0, num_sms = 148;
@@ -429,23 +429,20 @@ struct crane_b200_model {
     void load_gguf_file(const char* path, size_t* n_loaded, size_t* n_skipped);
     unsigned char* up_quant(int qt, const void* data, size_t rows, int K, unsigned char* dst = nullptr, size_t dst_row_pitch = 0);
     void linear_decode(int epi, bool norm, const bf16* w, const unsigned char* qw, int qt, int N, int K, const float* xin, int ldx,
-                       const float* norm_w, float* y, int ldy, const GemvArgs* extra = nullptr, int B = 1, bool same_input = false, const QSegs& segs = {});
+                       const float* norm_w, float* y, int ldy, const GemvArgs* extra = nullptr, int B = 1, bool same_input = false, const QMore& more = {});
     void qlinear_rows(int epi, const unsigned char* qw, int qt, int N, int K, const float* xin, int ldx, const float* norm_w, float* y, int ldy,
-                      int S, bool reuse_xq = false, const QSegs& segs = {});
-    // q, k and v of a quantised layer, one launch per run of neighbours of one type: f(weight, type, rows, first column, pieces, not the first)
-    template <typename F> void qkv_runs(const LayerW& l, F&& f) const {
+                      int S, bool reuse_xq = false);
+    // q, k and v of a quantised layer: f(weight, type, rows, first column, further matrices, not the first).  As GEMVs neighbours of one type share a launch; on the
+    // tensor cores each has its own (dealt out along K together, their sums would be grouped otherwise).
+    template <typename F> void qkv_linears(const LayerW& l, bool gemv, F&& f) const {
         const int n[3] = {nh * q_stride(), nkv * D, nkv * D}, t[3] = {l.qt_q, l.qt_k, l.qt_v};
         const unsigned char* w[3] = {l.q_wq, l.q_wk, l.q_wv};
         for (int i = 0, col = 0; i < 3;) {
-            int j = i + 1, rows = n[i];
-            QSegs sg;
-            for (; j < 3 && t[j] == t[i] && rows % 128 == 0; ++j) {
-                if (j == i + 1) { sg.w1 = sg.w2 = w[j]; sg.s1 = rows; sg.s2 = rows + n[j]; } else sg.w2 = w[j];
-                rows += n[j];
-            }
-            if (sg.s2 % 128 != 0) sg.s2 = (sg.s2 + 127) / 128 * 128;       // (two pieces: nothing lies behind the second)
-            f(w[i], t[i], rows, col, sg, i > 0);
-            col += rows; i = j;
+            QMore more;
+            int j = i + 1, end = col + n[i];
+            for (; gemv && j < 3 && t[j] == t[i]; end += n[j++]) { more.w[j - i - 1] = w[j]; more.n[j - i - 1] = n[j]; }
+            f(w[i], t[i], n[i], col, more, i > 0);
+            col = end; i = j;
         }
     }
     bool load_text_tensor(const std::string& n, int dt, const int64_t* shape, int ndim, const void* data);
@@ -1046,14 +1043,14 @@ void crane_b200_model::load_tensor_ggml(const std::string& name_in, int qt, cons
 
 // One decode-path linear: bf16 GEMV or quantised GEMV with the same fused epilogue.
 void crane_b200_model::linear_decode(int epi, bool norm, const bf16* w, const unsigned char* qw, int qt, int N, int K, const float* xin, int ldx,
-                                     const float* norm_w, float* y, int ldy, const GemvArgs* extra, int B, bool same_input, const QSegs& segs) {
+                                     const float* norm_w, float* y, int ldy, const GemvArgs* extra, int B, bool same_input, const QMore& more) {
     GemvArgs g = extra ? *extra : GemvArgs{};
     g.N = N; g.K = K; g.x = xin; g.ldx = ldx; g.norm_w = norm_w; g.eps = eps; g.y = y; g.ldy = ldy;
     if (qt) {
         QGemvArgs qa;
         g.W = reinterpret_cast<const bf16*>(qw);
         if (!norm) g.norm_w = nullptr;
-        qa.g = g; qa.qtype = qt; qa.epi = epi; qa.segs = segs;
+        qa.g = g; qa.qtype = qt; qa.epi = epi; qa.more = more;
         const int xmode = xq_mode_for(qt);
         qa.xq = xquant_apart(B, K) ? xq_buf : nullptr;
         if (qa.xq && (!same_input || xmode != xq_mode_last)) {      // (same input, norm and block rule as the previous quantised linear: v after q and k)
@@ -1074,7 +1071,7 @@ void crane_b200_model::linear_decode(int epi, bool norm, const bf16* w, const un
 // tensor cores (qgemm.cu); fewer rows go through the decode kernels, up to four per pass over the quantised weights.
 // `reuse_xq`: the rows were quantised by the previous call (same input, same norm) -- still checked against the block rule it used.
 void crane_b200_model::qlinear_rows(int epi, const unsigned char* qw, int qt, int N, int K, const float* xin, int ldx, const float* norm_w,
-                                    float* y, int ldy, int S, bool reuse_xq, const QSegs& segs) {
+                                    float* y, int ldy, int S, bool reuse_xq) {
     if (S >= qrows_min(qt)) {
         const int mode = xq_mode_for(qt);
         const QRows xr = qrows_at(xqr_buf, xqr_rows, K);
@@ -1083,13 +1080,13 @@ void crane_b200_model::qlinear_rows(int epi, const unsigned char* qw, int qt, in
             xqr_mode_last = mode;
             ++launches;
         }
-        LAUNCH_OK(qgemm_launch(stream, qt, qw, xr, S, N, K, epi, y, ldy, use_pdl, segs));
+        LAUNCH_OK(qgemm_launch(stream, qt, qw, xr, S, N, K, epi, y, ldy, use_pdl));
         ++launches;
         return;
     }
     for (int s0 = 0; s0 < S;) {
         const int B = (S - s0 >= 4) ? 4 : (S - s0 >= 2) ? 2 : 1;
-        linear_decode(epi, norm_w != nullptr, nullptr, qw, qt, N, K, xin + (size_t)s0 * ldx, ldx, norm_w, y + (size_t)s0 * ldy, ldy, nullptr, B, reuse_xq && S <= 4, segs);
+        linear_decode(epi, norm_w != nullptr, nullptr, qw, qt, N, K, xin + (size_t)s0 * ldx, ldx, norm_w, y + (size_t)s0 * ldy, ldy, nullptr, B, reuse_xq && S <= 4);
         s0 += B;
     }
 }
@@ -1345,8 +1342,8 @@ void crane_b200_model::enqueue_decode_step(int advance, bool with_embed, int B) 
         LayerW& l = layers[li];
         if (l.full) {
             if (l.qt_q) {   // GGUF keeps q/k/v as separate quantised matrices (qwen3/modeling.rs:252-255): GEMVs into one qkv row
-                qkv_runs(l, [&](const unsigned char* w, int t, int n, int col, const QSegs& sg, bool more) {
-                    linear_decode(GEMV_STORE, true, nullptr, w, t, n, H, x_dec, H, l.ln1, qkv_dec + col, qkv_dim(), nullptr, B, more, sg);
+                qkv_linears(l, true, [&](const unsigned char* w, int t, int n, int col, const QMore& more, bool again) {
+                    linear_decode(GEMV_STORE, true, nullptr, w, t, n, H, x_dec, H, l.ln1, qkv_dec + col, qkv_dim(), nullptr, B, again, more);
                 });
             } else {
                 linear_decode(GEMV_STORE, true, l.wqkv, nullptr, 0, qkv_dim(), H, x_dec, H, l.ln1, qkv_dec, qkv_dim(), nullptr, B);
@@ -1459,7 +1456,7 @@ int crane_b200_model::decode_group(size_t left) const {
 // y = epi(W x) of a group's rows, f32 in and out: the rows as three bf16 planes (24 bits), or as Q8 codes in front of a quantised matrix.
 // `same_input`: the rows are as the previous call left them (same input and norm) -- still checked against the block rule it used.
 void crane_b200_model::linear_wide(int epi, const bf16* w, const unsigned char* qw, int qt, int N, int K, const float* xin, int ldx, const float* norm_w,
-                                   float* y, int ldy, int B, bool same_input, const QSegs& segs) {
+                                   float* y, int ldy, int B, bool same_input) {
     if (qt) {
         const int mode = xq_mode_for(qt);
         const QRows xr = qrows_at(xqd_buf, wide_rows, K);
@@ -1468,7 +1465,7 @@ void crane_b200_model::linear_wide(int epi, const bf16* w, const unsigned char* 
             wide_xq_mode = mode;
             ++launches;
         }
-        LAUNCH_OK(qgemm_launch(stream, qt, qw, xr, B, N, K, epi, y, ldy, use_pdl, segs));
+        LAUNCH_OK(qgemm_launch(stream, qt, qw, xr, B, N, K, epi, y, ldy, use_pdl));
     } else {
         if (!same_input) {
             LAUNCH_OK(rows_split3_launch(stream, xin, ldx, B, K, norm_w, eps, w3_buf, (long long)w3_plane, use_pdl));
@@ -1485,8 +1482,8 @@ void crane_b200_model::enqueue_wide_step(int advance, int B) {
     for (int li = 0; li < L; ++li) {
         LayerW& l = layers[li];
         if (l.qt_q) {
-            qkv_runs(l, [&](const unsigned char* w, int t, int n, int col, const QSegs& sg, bool more) {
-                linear_wide(GEMV_STORE, nullptr, w, t, n, H, x_dec, H, l.ln1, qkv_dec + col, qkv_dim(), B, more, sg);
+            qkv_linears(l, false, [&](const unsigned char* w, int t, int n, int col, const QMore&, bool again) {
+                linear_wide(GEMV_STORE, nullptr, w, t, n, H, x_dec, H, l.ln1, qkv_dec + col, qkv_dim(), B, again);
             });
         } else {
             linear_wide(GEMV_STORE, l.wqkv, nullptr, 0, qkv_dim(), H, x_dec, H, l.ln1, qkv_dec, qkv_dim(), B);
@@ -1687,8 +1684,9 @@ void crane_b200_model::prefill(const uint32_t* ids, const float* embeds, size_t 
                     const int left = S - s0, B = all ? left : left >= 4 ? 4 : left >= 2 ? 2 : 1;
                     const float* xr = x + (size_t)s0 * H;
                     float* yr = qkv + (size_t)s0 * qkv_dim();
-                    qkv_runs(l, [&](const unsigned char* w, int t, int n, int col, const QSegs& sg, bool more) {
-                        qlinear_rows(GEMV_STORE, w, t, n, H, xr, H, l.ln1, yr + col, qkv_dim(), B, more, sg);
+                    qkv_linears(l, !all, [&](const unsigned char* w, int t, int n, int col, const QMore& more, bool again) {
+                        if (all) qlinear_rows(GEMV_STORE, w, t, n, H, xr, H, l.ln1, yr + col, qkv_dim(), B, again);
+                        else linear_decode(GEMV_STORE, true, nullptr, w, t, n, H, xr, H, l.ln1, yr + col, qkv_dim(), nullptr, B, again, more);
                     });
                     s0 += B;
                 }

@@ -67,7 +67,6 @@ struct QCfg {
 
 struct QGemmArgs {
     const unsigned char* w;        // [N, K / 256] blocks
-    QSegs segs;                    // (pieces end at multiples of 128 rows)
     int M, N, K, epi;              // activation rows, weight rows
     float* y; int ldy;             // [M, ldy] (GEMV_SILU_MUL: [M, N / 2])
     const float* dx;               // [GROUPS * K / 256][ldd] activation scales
@@ -145,8 +144,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
         int rs = 0, kb = it_begin % KB, n0 = it_begin / KB / a.sc.tiles_m * 128, tile = it_begin / KB; uint32_t rph = 0;
         for (int it = it_begin; it < it_end; ++it) {
             wait(&raw_empty[rs], rph ^ 1);
-            const uint8_t* src = (a.segs.s1 == 0 || n0 < a.segs.s1 ? a.w + (size_t)n0 * row_bytes : n0 < a.segs.s2 ? a.segs.w1 + (size_t)(n0 - a.segs.s1) * row_bytes
-                                                                        : a.segs.w2 + (size_t)(n0 - a.segs.s2) * row_bytes) + (size_t)kb * C::SB;
+            const uint8_t* src = a.w + (size_t)n0 * row_bytes + (size_t)kb * C::SB;
             const uint32_t dst = smem_u32(sm + C::OFF_RAW + rs * C::RAW_BYTES) + t * 16;
             if (n0 + 128 <= a.N) {
 #pragma unroll
@@ -467,7 +465,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
 }
 
 template <int QT, int NT>
-static int qgemm_launch_t(cudaStream_t st, const unsigned char* w, const QRows& x, int M, int N, int K, int epi, float* y, int ldy, bool pdl, const QSegs& segs) {
+static int qgemm_launch_t(cudaStream_t st, const unsigned char* w, const QRows& x, int M, int N, int K, int epi, float* y, int ldy, bool pdl) {
     using C = QCfg<QT, NT>;
     CUtensorMap tmX, tmS;
     if (!tc_tmap_16(&tmX, x.codes, (uint64_t)M, (uint64_t)K, (uint64_t)K, NT, 64, CU_TENSOR_MAP_SWIZZLE_128B)) return -1001;
@@ -475,7 +473,7 @@ static int qgemm_launch_t(cudaStream_t st, const unsigned char* w, const QRows& 
     static SmemOptIn seen;
     if (const int e = ensure_dyn_smem(qgemm_kernel<QT, NT>, (size_t)C::SMEM, seen)) return e;
     QGemmArgs a = {};
-    a.w = w; a.segs = segs; a.M = M; a.N = N; a.K = K; a.epi = epi; a.y = y; a.ldy = ldy; a.dx = x.dx; a.ldd = x.ldd;
+    a.w = w; a.M = M; a.N = N; a.K = K; a.epi = epi; a.y = y; a.ldy = ldy; a.dx = x.dx; a.ldd = x.ldd;
     TcSched& sc = a.sc;
     sc.tiles_m = (M + NT - 1) / NT; sc.tiles_n = (N + 127) / 128; sc.KB = K / 256;
     const long long tiles = (long long)sc.tiles_m * sc.tiles_n, iters = tiles * sc.KB;
@@ -505,21 +503,21 @@ static float qgemm_estimate(int qt, int nt, int M, int N, int K) {
 }
 
 template <int QT>
-static int qgemm_launch_q(cudaStream_t st, const unsigned char* w, const QRows& x, int M, int N, int K, int epi, float* y, int ldy, bool pdl, const QSegs& segs) {
-    if (M <= 16) return qgemm_launch_t<QT, 16>(st, w, x, M, N, K, epi, y, ldy, pdl, segs);
-    if (M <= 32) return qgemm_launch_t<QT, 32>(st, w, x, M, N, K, epi, y, ldy, pdl, segs);
+static int qgemm_launch_q(cudaStream_t st, const unsigned char* w, const QRows& x, int M, int N, int K, int epi, float* y, int ldy, bool pdl) {
+    if (M <= 16) return qgemm_launch_t<QT, 16>(st, w, x, M, N, K, epi, y, ldy, pdl);
+    if (M <= 32) return qgemm_launch_t<QT, 32>(st, w, x, M, N, K, epi, y, ldy, pdl);
     if constexpr (QT != QT_Q8_0) {
-        if (qgemm_estimate(QT, 128, M, N, K) < qgemm_estimate(QT, 64, M, N, K)) return qgemm_launch_t<QT, 128>(st, w, x, M, N, K, epi, y, ldy, pdl, segs);
+        if (qgemm_estimate(QT, 128, M, N, K) < qgemm_estimate(QT, 64, M, N, K)) return qgemm_launch_t<QT, 128>(st, w, x, M, N, K, epi, y, ldy, pdl);
     }
-    return qgemm_launch_t<QT, 64>(st, w, x, M, N, K, epi, y, ldy, pdl, segs);
+    return qgemm_launch_t<QT, 64>(st, w, x, M, N, K, epi, y, ldy, pdl);
 }
 
-int qgemm_launch(cudaStream_t st, int qt, const unsigned char* w, const QRows& x, int M, int N, int K, int epi, float* y, int ldy, bool pdl, const QSegs& segs) {
-    if (M <= 0 || N <= 0 || K <= 0 || (K % 256) != 0 || (epi == GEMV_SILU_MUL && (N % 2) != 0) || M > x.ldd || (segs.s1 % 128) != 0 || (segs.s2 % 128) != 0) return -1000;
+int qgemm_launch(cudaStream_t st, int qt, const unsigned char* w, const QRows& x, int M, int N, int K, int epi, float* y, int ldy, bool pdl) {
+    if (M <= 0 || N <= 0 || K <= 0 || (K % 256) != 0 || (epi == GEMV_SILU_MUL && (N % 2) != 0) || M > x.ldd) return -1000;
     switch (qt) {
-        case QT_Q4_K: return qgemm_launch_q<QT_Q4_K>(st, w, x, M, N, K, epi, y, ldy, pdl, segs);
-        case QT_Q6_K: return qgemm_launch_q<QT_Q6_K>(st, w, x, M, N, K, epi, y, ldy, pdl, segs);
-        case QT_Q8_0: return qgemm_launch_q<QT_Q8_0>(st, w, x, M, N, K, epi, y, ldy, pdl, segs);
+        case QT_Q4_K: return qgemm_launch_q<QT_Q4_K>(st, w, x, M, N, K, epi, y, ldy, pdl);
+        case QT_Q6_K: return qgemm_launch_q<QT_Q6_K>(st, w, x, M, N, K, epi, y, ldy, pdl);
+        case QT_Q8_0: return qgemm_launch_q<QT_Q8_0>(st, w, x, M, N, K, epi, y, ldy, pdl);
         default: return -1000;
     }
 }

@@ -358,7 +358,8 @@ __host__ __device__ constexpr int qg_warps(int B) { return B >= 4 ? QG_W4_DEF : 
 // a contiguous range of tiles (k fastest), streams each through its private cp.async ring, keeps its activation slice in
 // registers and one f32 accumulator per (row, sequence), and flushes them to the CTA's shared row accumulators when it
 // moves on to another row group.
-template <int B, int QT>
+// MORE: q, k and v share the launch (QMore)
+template <int B, int QT, bool MORE>
 __global__ void __launch_bounds__(qg_warps(B) * 32, 1)
 qgemv_kernel(QGemvArgs qa) {
     using TR = QTraits<QT>;
@@ -374,11 +375,7 @@ qgemv_kernel(QGemvArgs qa) {
     const size_t xb = (size_t)K + (size_t)(K / 32) * 8 + (size_t)(K / 16) * 4;       // bytes of quantised activation per sequence
     unsigned char* xbase = qsm + (size_t)QG_WARPS * QG_DEPTH * SLOT;
     const int rows_per_unit = (qa.epi == GEMV_SILU_MUL) ? 2 : 1;
-    const int units = a.N / rows_per_unit;
-    const int upc = (units + gridDim.x - 1) / gridDim.x;
-    const int rpc = upc * rows_per_unit;
-    const int r0 = blockIdx.x * rpc;
-    const int nrows = max(0, min(a.N, r0 + rpc) - r0);
+    const int mats = !MORE ? 1 : qa.more.n[1] ? 3 : 2;
     float* acc_s = reinterpret_cast<float*>(xbase + (size_t)B * xb);
     __shared__ uint64_t xbar;
     __shared__ float red[B][32];
@@ -389,47 +386,71 @@ qgemv_kernel(QGemvArgs qa) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t spr = (uint32_t)(K >> 8);                                          // super-blocks per row
     const uint32_t nkt = (spr + QG_KT - 1) / QG_KT;                                   // k-tiles per row
-    // rows per tile: QG_R when that leaves every warp at least two tiles, fewer for short row blocks (q/k/v/o projections)
-    uint32_t R = QG_R;
-    while (R > 1 && (((uint32_t)nrows + R - 1) / R) * nkt < 2u * (uint32_t)QG_WARPS) R >>= 1;
-    const uint32_t nrg = ((uint32_t)nrows + R - 1) / R;                               // row groups
-    const uint32_t ntile = nrg * nkt;
-    const uint32_t tpw = (ntile + QG_WARPS - 1) / QG_WARPS;
-    const uint32_t t_begin = min(ntile, (uint32_t)warp * tpw), t_end = min(ntile, ((uint32_t)warp + 1) * tpw);
-    const uint32_t nt = t_end - t_begin;
-    const unsigned char* wbase = reinterpret_cast<const unsigned char*>(a.W);
     const size_t row_bytes = (size_t)spr * TR::SB;
-    auto row_at = [&](uint32_t i) {                     // row i of this CTA, in whichever piece of the weight it lies
-        const int r = r0 + (int)i;
-        if (qa.segs.s1 == 0 || r < qa.segs.s1) return wbase + (size_t)r * row_bytes;
-        return r < qa.segs.s2 ? qa.segs.w1 + (size_t)(r - qa.segs.s1) * row_bytes : qa.segs.w2 + (size_t)(r - qa.segs.s2) * row_bytes;
+    // The matrix at hand and this CTA's rows of it.  Every matrix is dealt out as in a launch of its own, so that its rows' sums are formed in the same order, and
+    // the codes of the next linear are the same, whether q, k and v share a launch or not.
+    struct Mat { const unsigned char* w; int rpc, r0, nrows, out, acc0; };             // (out, acc0: what the matrices ahead take of y and of the sums)
+    auto mat = [&](int k) {
+        Mat m{reinterpret_cast<const unsigned char*>(a.W), qa.rpc[0], 0, a.N, 0, 0};
+        if (MORE && k >= 1) m = Mat{qa.more.w[0], qa.rpc[1], 0, qa.more.n[0], a.N, B * qa.rpc[0]};
+        if (MORE && k >= 2) m = Mat{qa.more.w[1], qa.rpc[2], 0, qa.more.n[1], a.N + qa.more.n[0], B * (qa.rpc[0] + qa.rpc[1])};
+        m.r0 = (int)blockIdx.x * m.rpc;
+        m.nrows = max(0, min(m.nrows, m.r0 + m.rpc) - m.r0);
+        return m;
     };
+    // this warp's tiles [t, end) of it, of R rows; `turn`: the warp that takes the first ones, as short matrices leave warps without any.  (Worked out ahead of the
+    // dependency wait: the divisions are 0.3 us.)
+    struct Deal { uint32_t R, t, end; };
+    uint32_t turn = 0;
+    auto deal = [&](int nrows) {
+        Deal d{QG_R};
+        // rows per tile: QG_R when that leaves every warp at least two tiles, fewer for short row blocks (q/k/v/o projections)
+        while (d.R > 1 && (((uint32_t)nrows + d.R - 1) / d.R) * nkt < 2u * (uint32_t)QG_WARPS) d.R >>= 1;
+        const uint32_t ntile = ((uint32_t)nrows + d.R - 1) / d.R * nkt, tpw = (ntile + QG_WARPS - 1) / QG_WARPS;
+        const uint32_t u = (uint32_t)warp >= turn ? warp - turn : warp + QG_WARPS - turn;
+        d.t = min(ntile, u * tpw);
+        d.end = min(ntile, (u + 1) * tpw);
+        if (MORE) {
+            turn += ntile ? (ntile + tpw - 1) / tpw : 0u;
+            if (turn >= (uint32_t)QG_WARPS) turn -= QG_WARPS;
+        }
+        return d;
+    };
+    const Deal d0 = deal(mat(0).nrows), d1 = MORE ? deal(mat(1).nrows) : d0, d2 = MORE && mats > 2 ? deal(mat(2).nrows) : d0;
+    auto dealt = [&](int k) { return !MORE || k == 0 ? d0 : k == 1 ? d1 : d2; };
     unsigned char* ring = qsm + (size_t)warp * QG_DEPTH * SLOT;
     const uint32_t ring_u32 = smem_u32(ring);
 
-    auto issue = [&](uint32_t p) {
-        if (p < nt) {
-            const uint32_t t = t_begin + p, rg = t / nkt, kt = t - rg * nkt;
-            const uint32_t nr = min(R, (uint32_t)nrows - rg * R);
+    Mat mi = mat(0);                                    // the tiles requested so far
+    Deal di = d0;
+    int ki = 0;
+    uint32_t islot = 0;
+    auto issue = [&]() {
+        while (di.t == di.end && ki + 1 < mats) { ++ki; mi = mat(ki); di = dealt(ki); }
+        if (di.t < di.end) {
+            const uint32_t rg = di.t / nkt, kt = di.t - rg * nkt;
+            const uint32_t nr = min(di.R, (uint32_t)mi.nrows - rg * di.R);
             const uint32_t cpr = min((uint32_t)QG_KT, spr - kt * QG_KT) * (TR::SB / 16);      // 16-byte chunks per tile row
-            const uint32_t dst = ring_u32 + (p % QG_DEPTH) * SLOT;
-            for (uint32_t r = 0; r < nr; ++r) {
-                const unsigned char* src = row_at(rg * R + r) + (size_t)kt * QG_KT * TR::SB;
+            const uint32_t dst = ring_u32 + islot * SLOT;
+            const unsigned char* src = mi.w + (size_t)(mi.r0 + rg * di.R) * row_bytes + (size_t)kt * QG_KT * TR::SB;
+            for (uint32_t r = 0; r < nr; ++r, src += row_bytes)
                 for (uint32_t c = lane; c < cpr; c += 32)
                     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + r * ROWB + c * 16), "l"(src + (size_t)c * 16) : "memory");
-            }
+            ++di.t;
         }
+        islot = islot + 1 == QG_DEPTH ? 0 : islot + 1;
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
 #pragma unroll
-    for (int p = 0; p < QG_DEPTH; ++p) issue((uint32_t)p);
-    for (int i = tid; i < B * rpc; i += QG_THREADS) acc_s[i] = 0.f;
+    for (int p = 0; p < QG_DEPTH; ++p) issue();
+    for (int i = tid; i < B * (qa.rpc[0] + (mats > 1 ? qa.rpc[1] : 0) + (mats > 2 ? qa.rpc[2] : 0)); i += QG_THREADS) acc_s[i] = 0.f;
     if (tid == 0) { mbar_init(&xbar, 1); fence_barrier_init(); }
     __syncthreads();
 
     pdl_wait();
     pdl_launch_dependents();
 
+    const int r0 = mat(0).r0, nrows = mat(0).nrows, rpc = qa.rpc[0];
     float old[B];                                       // (beside the activations, not behind the dots)
     if (qa.epi == GEMV_RESID)
 #pragma unroll
@@ -445,15 +466,21 @@ qgemv_kernel(QGemvArgs qa) {
         const int nvw = min(32, (K + 127) / 128);           // of xq_ssq's 32 warps, those with anything to add
         if (a.norm_w) {
 #pragma unroll 1
-            for (int vw = warp; vw < nvw; vw += QG_WARPS) {
-                float ssq[B];
-#pragma unroll
-                for (int b = 0; b < B; ++b) ssq[b] = xq_ssq(a.x + (size_t)b * a.ldx, K, vw * 32 + lane);
+            for (int vw = warp; vw < nvw; vw += 2 * QG_WARPS) {      // two of them at once: their loads are in flight together
+                const int second = vw + QG_WARPS < nvw ? vw + QG_WARPS : -1;
+                float ssq[2][B];
 #pragma unroll
                 for (int b = 0; b < B; ++b) {
-                    ssq[b] = warp_sum(ssq[b]);
-                    if (lane == 0) red[b][vw] = ssq[b];
+                    ssq[0][b] = xq_ssq(a.x + (size_t)b * a.ldx, K, vw * 32 + lane);
+                    ssq[1][b] = second < 0 ? 0.f : xq_ssq(a.x + (size_t)b * a.ldx, K, second * 32 + lane);
                 }
+#pragma unroll
+                for (int b = 0; b < B; ++b)
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        const float v = warp_sum(ssq[j][b]);
+                        if (lane == 0 && (j == 0 || second >= 0)) red[b][j ? second : vw] = v;
+                    }
             }
             __syncthreads();
         }
@@ -473,44 +500,56 @@ qgemv_kernel(QGemvArgs qa) {
         float acc[QG_R * B];
 #pragma unroll
         for (int i = 0; i < QG_R * B; ++i) acc[i] = 0.f;
-        uint32_t cur_rg = 0xffffffffu, cur_kt = 0xffffffffu;
-        auto flush = [&]() {
-            int idx;
-            warp_reduce_scatter<QG_R * B>(acc, lane, idx);
-            const int r = idx / B, b = idx % B;
-            const uint32_t row = cur_rg * R + r;
-            if ((lane & (32 / (QG_R * B) - 1)) == 0 && (uint32_t)r < R && row < (uint32_t)nrows) atomicAdd(&acc_s[(size_t)b * rpc + row], acc[0]);
+        uint32_t cur_kt = 0xffffffffu, slot = 0;
+        for (int k = 0; k < mats; ++k) {
+            const Mat m = mat(k);
+            const Deal d = dealt(k);
+            uint32_t cur_rg = 0xffffffffu;
+            auto flush = [&]() {
+                int idx;
+                warp_reduce_scatter<QG_R * B>(acc, lane, idx);
+                const int r = idx / B, b = idx % B;
+                const uint32_t row = cur_rg * d.R + r;
+                if ((lane & (32 / (QG_R * B) - 1)) == 0 && (uint32_t)r < d.R && row < (uint32_t)m.nrows) atomicAdd(&acc_s[m.acc0 + (size_t)b * m.rpc + row], acc[0]);
 #pragma unroll
-            for (int i = 0; i < QG_R * B; ++i) acc[i] = 0.f;
-        };
-        for (uint32_t p = 0; p < nt; ++p) {
-            asm volatile("cp.async.wait_group %0;" ::"n"(QG_DEPTH - 1) : "memory");
-            __syncwarp();
-            const uint32_t t = t_begin + p, rg = t / nkt, kt = t - rg * nkt;
-            if (rg != cur_rg) {
-                if (cur_rg != 0xffffffffu) flush();
-                cur_rg = rg;
-            }
-            const bool active = kt * QG_KT + sbk < spr;
-            if (kt != cur_kt) {
-                if (active) xs.load(xbase, xb, K, (int)(kt * QG_KT) + sbk, qq);
-                cur_kt = kt;
-            }
-            const uint32_t nr = min(R, (uint32_t)nrows - rg * R);
-            const unsigned char* sb = ring + (p % QG_DEPTH) * SLOT + sbk * TR::SB;
-            if (active) {
+                for (int i = 0; i < QG_R * B; ++i) acc[i] = 0.f;
+            };
+            for (uint32_t t = d.t; t < d.end; ++t) {
+                asm volatile("cp.async.wait_group %0;" ::"n"(QG_DEPTH - 1) : "memory");
+                __syncwarp();
+                const uint32_t rg = t / nkt, kt = t - rg * nkt;
+                if (rg != cur_rg) {
+                    if (cur_rg != 0xffffffffu) flush();
+                    cur_rg = rg;
+                }
+                const bool active = kt * QG_KT + sbk < spr;
+                if (kt != cur_kt) {
+                    if (active) xs.load(xbase, xb, K, (int)(kt * QG_KT) + sbk, qq);
+                    cur_kt = kt;
+                }
+                const uint32_t nr = min(d.R, (uint32_t)m.nrows - rg * d.R);
+                const unsigned char* sb = ring + slot * SLOT + sbk * TR::SB;
+                if (active) {
 #pragma unroll
-                for (int r = 0; r < QG_R; ++r)
-                    if ((uint32_t)r < nr) sb_quarter_dot<QT, B>(sb + r * ROWB, qq, xs, acc + r * B);
+                    for (int r = 0; r < QG_R; ++r)
+                        if ((uint32_t)r < nr) sb_quarter_dot<QT, B>(sb + r * ROWB, qq, xs, acc + r * B);
+                }
+                __syncwarp();
+                issue();
+                slot = slot + 1 == QG_DEPTH ? 0 : slot + 1;
             }
-            __syncwarp();
-            issue(p + QG_DEPTH);
+            if (cur_rg != 0xffffffffu) flush();
         }
-        if (cur_rg != 0xffffffffu) flush();
     }
     __syncthreads();
 
     // ---- epilogue (same contracts as the bf16 GEMV) ----
+    for (int k = 1; k < mats; ++k) {
+        const Mat m = mat(k);
+        for (int i = tid; i < m.nrows; i += QG_THREADS)
+#pragma unroll
+            for (int b = 0; b < B; ++b) a.y[(size_t)b * a.ldy + m.out + m.r0 + i] = acc_s[m.acc0 + b * m.rpc + i];
+    }
     float bestv[B];
     int besti[B];
 #pragma unroll
@@ -593,31 +632,43 @@ qgemv_kernel(QGemvArgs qa) {
 }
 
 template <int B, int QT>
-static int qgemv_launch_t(cudaStream_t st, const QGemvArgs& qa, int num_sms, bool pdl) {
+static int qgemv_launch_t(cudaStream_t st, const QGemvArgs& args, int num_sms, bool pdl) {
     using TR = QTraits<QT>;
+    QGemvArgs qa = args;
     const GemvArgs& a = qa.g;
     const int rpu = qa.epi == GEMV_SILU_MUL ? 2 : 1;
-    const int rpc = ((a.N / rpu) + num_sms - 1) / num_sms * rpu;
+    auto rpc = [&](int n) { return (size_t)((n / rpu + num_sms - 1) / num_sms * rpu); };
     const size_t xb = (size_t)a.K + (size_t)(a.K / 32) * 8 + (size_t)(a.K / 16) * 4;
-    const size_t fixed = (size_t)B * xb + (size_t)B * rpc * 4 + 16, slot = (size_t)QG_DEPTH * QG_R * QG_KT * TR::SB;
-    int QG_WARPS = qg_warps(B);
-    while (QG_WARPS > 4 && fixed + QG_WARPS * slot > 226 * 1024) --QG_WARPS;
+    const size_t fixed = (size_t)B * xb + 32, slot = (size_t)QG_DEPTH * QG_R * QG_KT * TR::SB, most = 226 * 1024;
+    auto warps = [&](int n) {                           // what fits beside n rows' sums
+        int w = qg_warps(B);
+        while (w > 4 && fixed + B * rpc(n) * 4 + w * slot > most) --w;
+        return w;
+    };
+    const int QG_WARPS = warps(a.N);
+    size_t smem = fixed + B * rpc(a.N) * 4 + QG_WARPS * slot;
+    if (qa.more.n[0]) {
+        if (qa.epi != GEMV_STORE) return -1000;
+        bool one = true;
+        for (int n : qa.more.n) if (n) { one = one && warps(n) == QG_WARPS; smem += B * rpc(n) * 4; }
+        if (!one || smem > most) {                      // launches of their own: the same sums
+            QGemvArgs q = qa;
+            q.more = QMore{};
+            int e = qgemv_launch_t<B, QT>(st, q, num_sms, pdl);
+            for (int i = 0; i < 2 && qa.more.n[i] && !e; ++i) {
+                q.g.y += q.g.N; q.g.N = qa.more.n[i]; q.g.W = reinterpret_cast<const bf16*>(qa.more.w[i]);
+                e = qgemv_launch_t<B, QT>(st, q, num_sms, pdl);
+            }
+            return e;
+        }
+    }
     const int QG_THREADS = QG_WARPS * 32;
-    const size_t smem = fixed + QG_WARPS * slot;
-    if (smem > 226 * 1024) return -1000;
-    static SmemOptIn seen;
-    if (const int e = ensure_dyn_smem(qgemv_kernel<B, QT>, smem, seen)) return e;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(num_sms);
-    cfg.blockDim = dim3(QG_THREADS);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    return (int)cudaLaunchKernelEx(&cfg, qgemv_kernel<B, QT>, qa);
+    if (smem > most) return -1000;
+    for (int i = 0; i < 3; ++i) qa.rpc[i] = (int)rpc(i ? qa.more.n[i - 1] : a.N);
+    static SmemOptIn seen[2];
+    auto* kern = qa.more.n[0] ? qgemv_kernel<B, QT, true> : qgemv_kernel<B, QT, false>;
+    if (const int e = ensure_dyn_smem(kern, smem, seen[qa.more.n[0] != 0])) return e;
+    return launch_k(kern, dim3(num_sms), dim3(QG_THREADS), smem, st, pdl, qa);
 }
 
 template <int B>

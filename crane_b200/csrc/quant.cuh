@@ -21,15 +21,15 @@ inline int q_src_block_elems(int qt) { return qt == QT_Q8_0 ? 32 : 256; }
 // Host: repack `rows` rows of K elements from the ggml byte layout into the device layout (dst sized rows * K/256 * q_sb_bytes).
 void q_repack_rows(int qt, const unsigned char* src, unsigned char* dst, size_t rows, int K);
 
-// Rows of a weight that lies in up to three pieces: rows [0, s1) in the launch's own `w`, [s1, s2) in w1, the others in w2 (q, k and v of one quantised type
-// are one launch).  s1 = 0: one piece.
-struct QSegs { const unsigned char *w1 = nullptr, *w2 = nullptr; int s1 = 0, s2 = 0; };
+// Further matrices of a GEMV launch (k and v of q's type beside q): n[i] rows of w[i], results one behind the other's.  n = 0: none.
+struct QMore { const unsigned char* w[2] = {nullptr, nullptr}; int n[2] = {0, 0}; };
 
 struct QGemvArgs {
     GemvArgs g;        // W is reinterpreted as the quantised bytes; g.x, g.ldx, and (nullable) g.norm_w with g.eps: the activation rows; epilogue fields as for the bf16 GEMV
     int qtype;
     int epi;           // GemvEpi
-    QSegs segs;
+    QMore more;        // (GEMV_STORE only)
+    int rpc[3];        // rows of each matrix per CTA (set by the launch)
     const unsigned char* xq;   // the rows quantised by xquant_launch (norm included), or nullptr: the kernel quantises them itself
 };
 
@@ -59,9 +59,8 @@ struct QRows { unsigned short* codes; float* dx; unsigned short* bsum; int ldd; 
 size_t qrows_bytes(int rows, int K);
 QRows qrows_at(unsigned char* buf, int rows, int K);
 int xquant_rows_launch(cudaStream_t st, int M, const float* x, int ldx, int K, const float* norm_w, float eps, int mode, const QRows& out, bool pdl);
-// y[m, n] = epi(sum_k W[n, k] x[m, k]); epi: GEMV_STORE, GEMV_RESID or GEMV_SILU_MUL (rows of W interleaved); x quantised for W's type.  Pieces of W end at
-// multiples of 128 rows.
-int qgemm_launch(cudaStream_t st, int qt, const unsigned char* w, const QRows& x, int M, int N, int K, int epi, float* y, int ldy, bool pdl, const QSegs& segs = {});
+// y[m, n] = epi(sum_k W[n, k] x[m, k]); epi: GEMV_STORE, GEMV_RESID or GEMV_SILU_MUL (rows of W interleaved); x quantised for W's type
+int qgemm_launch(cudaStream_t st, int qt, const unsigned char* w, const QRows& x, int M, int N, int K, int epi, float* y, int ldy, bool pdl);
 // rows x K quantised -> bf16 row-major
 int q_dequant_bf16_launch(cudaStream_t st, int qt, const unsigned char* w, size_t rows, int K, bf16* out);
 // gather + dequantise rows of a quantised embedding table to f32: ids[rows] (prefill) or, with ids == nullptr, state[r].token
