@@ -801,9 +801,9 @@ attn_decode_kernel(AttnDecArgs a) {
 #pragma unroll
         for (int j = 0; j < EPL; ++j) o[h][j] = 0.f;
     }
-    // U tokens of this lane's group at a time: their scores and shuffles are independent, and the running sums are rescaled once for all of them (token by
-    // token the chain of five dependent steps and the rescaling bound the kernel: 32 sequences
-    // of 500 tokens 38 us, 47 before; 1 of 4000 16.1 and 21.3)
+    // U tokens of this lane's group at a time: their scores, shuffles and exponentials are independent, where token by token they were a chain of five dependent
+    // steps.  The running sums take them one after the other all the same: rescaled once for both they were rounded otherwise, and what a quantised model's codes
+    // make of that is 1e-2 of its logits.  (32 sequences of 45 .. 300 tokens, 32 heads over 8 of D = 128: 30.1 us, 34.1 token by token, 28.9 rescaled once.)
     constexpr int U = 2;
     auto unpack = [&](float* f, const bf16* hp, const bf16* lp) __attribute__((always_inline)) {
         const uint4 r = *reinterpret_cast<const uint4*>(hp);
@@ -838,32 +838,28 @@ attn_decode_kernel(AttnDecArgs a) {
 #pragma unroll
                 for (int h = 0; h < NREP; ++h) sc[u][h] += __shfl_xor_sync(0xffffffffu, sc[u][h], ofs);
         if (!valid[0]) return;                          // (tokens ascend: the others are not there either)
+        float c[U][NREP];
 #pragma unroll
-        for (int h = 0; h < NREP; ++h) {
-            float mn = m[h];
+        for (int h = 0; h < NREP; ++h)
 #pragma unroll
-            for (int u = 0; u < U; ++u) if (valid[u]) mn = fmaxf(mn, sc[u][h]);
-            const float corr = __expf(m[h] - mn);
-            l[h] *= corr;
-#pragma unroll
-            for (int j = 0; j < EPL; ++j) o[h][j] *= corr;
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
+            for (int u = 0; u < U; ++u) {               // (a token that is not there: factor 1, weight 0)
+                const float mn = valid[u] ? fmaxf(m[h], sc[u][h]) : m[h];
+                c[u][h] = __expf(m[h] - mn);
                 sc[u][h] = valid[u] ? __expf(sc[u][h] - mn) : 0.f;
-                l[h] += sc[u][h];
+                l[h] = l[h] * c[u][h] + sc[u][h];
+                m[h] = mn;
             }
-            m[h] = mn;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            float vf[EPL];
+#pragma unroll
+            for (int j = 0; j < EPL; ++j) vf[j] = 0.f;
+            if (valid[u]) unpack(vf, vp[u], vp[u] + lo);
+#pragma unroll
+            for (int h = 0; h < NREP; ++h)
+#pragma unroll
+                for (int j = 0; j < EPL; ++j) o[h][j] = o[h][j] * c[u][h] + sc[u][h] * vf[j];
         }
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-            if (valid[u]) {
-                float vf[EPL];
-                unpack(vf, vp[u], vp[u] + lo);
-#pragma unroll
-                for (int h = 0; h < NREP; ++h)
-#pragma unroll
-                    for (int j = 0; j < EPL; ++j) o[h][j] = fmaf(sc[u][h], vf[j], o[h][j]);
-            }
     };
     bool valid[U];
     const bf16 *kp[U], *vp[U];

@@ -2,7 +2,8 @@
 
 A quantised linear rounds its input to 8-bit codes.  A value on the border of two goes the other way when one addition ahead of it is done in another order, and the
 logits move by up to 1e-2 of their size where f32 sums alone would move them by 1e-6.  So the order of every sum ahead of the codes -- the rows' 1 / rms, the sums of
-q, k and v wherever their launches end -- is part of what a quantised model answers, and these checksums hold it: they were recorded with one launch per linear.  A change that moves one has to say why the new order is the better one."""
+q, k and v wherever their launches end, decode attention over its tokens -- is part of what a quantised model answers, and these checksums hold it: they were
+recorded with one launch per linear and attention token after token.  A change that moves one has to say why the new order is the better one."""
 import zlib
 
 import numpy as np
@@ -66,12 +67,12 @@ def _batch(m, n, past):
 
 CASES = {
     "three rows": lambda m: _prompt(m, 3), "forty rows": lambda m: _prompt(m, 40),
-    "token behind 4": lambda m: _tokens(m, 4),
-    "pair": lambda m: _batch(m, 2, 12), "24 short": lambda m: _batch(m, 24, 12),
+    "token behind 4": lambda m: _tokens(m, 4), "token behind 300": lambda m: _tokens(m, 300),
+    "pair": lambda m: _batch(m, 2, 12), "24 short": lambda m: _batch(m, 24, 12), "24 long": lambda m: _batch(m, 24, 300),
 }
 BITS = {
-    "q8_0": {"three rows": 860423412, "forty rows": 2319047176, "token behind 4": 915047249, "pair": 2572308134, "24 short": 351940177},
-    "q4_k_m": {"three rows": 2799229761, "forty rows": 133175824, "token behind 4": 3687851847, "pair": 14193225, "24 short": 2683411286},
+    "q8_0": {"three rows": 860423412, "forty rows": 2319047176, "token behind 4": 915047249, "token behind 300": 70435833, "pair": 2572308134, "24 short": 351940177, "24 long": 908247942},
+    "q4_k_m": {"three rows": 2799229761, "forty rows": 133175824, "token behind 4": 3687851847, "token behind 300": 2366858767, "pair": 14193225, "24 short": 2683411286, "24 long": 151590533},
 }
 
 
