@@ -356,13 +356,15 @@ gemv_kernel(GemvArgs a, int ns) {
 
 static int gemv_rpc(int N, int rows_per_unit, int grid) { return (N / rows_per_unit + grid - 1) / grid * rows_per_unit; }
 static size_t gemv_smem_bytes(int B, int K, int rpc, int ns) { return (size_t)GV_WARPS * gv_depth(B) * GV_SLOT + (size_t)B * K * 4 + (size_t)B * rpc * ns * 4 + 16; }
+// Shared memory that a launch may ask for: 227 KB a block has, less the norm's own arrays where there is one (with the alignment of what follows them, 1 KB).
+constexpr size_t gemv_most(bool norm) { return (norm ? 226 : 227) * 1024; }
 // Slices of K a CTA's rows are cut into: the fewest column chunks on the busiest warp (a unit's reduction and its first slot cost about another), while
 // the sums fit.  One slice wherever the rows are enough for the warps.
-static int gemv_slices(int B, int K, int rpc) {
+static int gemv_slices(int B, int K, int rpc, bool norm) {
     const int chunks = K / 256, blocks = (rpc + GV_ROWS - 1) / GV_ROWS;
     int best = 1, cost = 1 << 30;
     for (int ns = 1; ns <= std::min(chunks, GV_WARPS); ++ns) {
-        if (ns > 1 && gemv_smem_bytes(B, K, rpc, ns) > 227 * 1024) break;
+        if (ns > 1 && gemv_smem_bytes(B, K, rpc, ns) > gemv_most(norm)) break;
         const int c = (blocks * ns + GV_WARPS - 1) / GV_WARPS * ((chunks + ns - 1) / ns + 1);
         if (c < cost) { cost = c; best = ns; }
     }
@@ -371,9 +373,9 @@ static int gemv_slices(int B, int K, int rpc) {
 
 template <int B, int EPI, int NORM>
 static int gemv_launch_t(cudaStream_t st, const GemvArgs& a, int num_sms, bool pdl) {
-    const int rpc = gemv_rpc(a.N, EPI == GEMV_SILU_MUL ? 2 : 1, num_sms), ns = gemv_slices(B, a.K, rpc);
+    const int rpc = gemv_rpc(a.N, EPI == GEMV_SILU_MUL ? 2 : 1, num_sms), ns = gemv_slices(B, a.K, rpc, NORM != 0);
     const size_t smem = gemv_smem_bytes(B, a.K, rpc, ns);
-    if (smem > 227 * 1024) return -1000;
+    if (smem > gemv_most(NORM != 0)) return -1000;
     static SmemOptIn seen;
     if (const int e = ensure_dyn_smem(gemv_kernel<B, EPI, NORM>, smem, seen)) return e;
     cudaLaunchConfig_t cfg = {};
@@ -410,7 +412,7 @@ static int gemv_launch_b(cudaStream_t st, int epi, bool norm, const GemvArgs& a,
 // Largest sequence group (4, 2 or 1) whose f32 activations fit next to the weight rings for an in_dim of K.
 int gemv_max_group(int K, int N, int num_sms) {
     for (int B : {4, 2})
-        if (gemv_smem_bytes(B, K, gemv_rpc(N, 1, num_sms), 1) <= 227 * 1024) return B;
+        if (gemv_smem_bytes(B, K, gemv_rpc(N, 1, num_sms), 1) <= gemv_most(true)) return B;
     return 1;
 }
 

@@ -10,6 +10,7 @@ import pytest
 from conftest import rel_err
 import crane_b200
 from crane_b200 import synth
+from oracle import ggml_quant as gq
 from oracle.qwen3 import Qwen3Oracle
 
 pytestmark = pytest.mark.gpu
@@ -51,6 +52,45 @@ def test_groups_of_sequences(n):
     _, got = m.decode_batch(slots, [int(t[-1]) for t in ids], 1, want_logits=True)
     for row, k, t in zip(got, lens, ids):
         orc = Qwen3Oracle(cfg, w)
+        orc.forward(t[:k], 0)
+        assert rel_err(row, orc.forward(t[k:], k).numpy()) < TOL
+    m.close()
+
+
+@pytest.mark.parametrize("cfg", [
+    # 3, 5 and 6 column chunks in several slices; 9 and 18 rows a CTA, a head of 1003
+    dict(hidden_size=768, intermediate_size=1280, num_attention_heads=6, num_hidden_layers=2, vocab_size=1003),
+    # 4864 rows of 10240 columns: five slices would be the fastest, and take the shared memory that the folded-in norm needs for itself
+    dict(hidden_size=10240, intermediate_size=256, num_attention_heads=34, num_hidden_layers=1, vocab_size=257)], ids=["odd", "wide"])
+def test_four_sequences_through_the_gemv(cfg):
+    """A quantised embedding sends groups of four, and with them every bf16 linear, past the tensor cores: the GEMV of four sequences, against the oracle."""
+    cfg = dict(synth.TINY_QWEN3_UNTIED, **dict(cfg, num_key_value_heads=2))
+    m = crane_b200.Qwen3Model(cfg, device=0, max_seq_len=160, max_batch=4)
+    w = {}
+    for name, shape, kind in synth.text_tensor_specs(cfg):
+        rng = np.random.default_rng(len(w))
+        t = rng.standard_normal((min(shape[0], 97),) + tuple(shape[1:]) if len(shape) > 1 else shape, dtype=np.float32)
+        t = t * shape[1] ** -0.5 if kind == "linear" else t if kind == "embed" else 1 + 0.02 * t
+        t = np.resize(t, shape).astype(np.float32)       # (97 rows again and again)
+        if kind == "embed":
+            raw = gq.quantize(t, "Q8_0")
+            m.load_tensor_ggml(name, gq.GGML_TYPE_ID["Q8_0"], shape, raw)
+            w[name] = gq.dequantize(raw, "Q8_0", shape[1])
+        else:
+            bits = synth.f32_to_bf16_bits(t)
+            m.load_tensor(name, bits)
+            w[name] = synth.bf16_bits_to_f32(bits)
+    m.finalize()
+    lens = [3, 130, 17, 66]
+    slots = [0] + [m.seq_create() for _ in range(3)]
+    ids = [synth.synth_token_ids(k + 1, cfg["vocab_size"], f"q{k}") for k in lens]
+    for s, k, t in zip(slots, lens, ids):
+        m.seq_select(s)
+        m.forward_step(t[:k], 0)
+    _, got = m.decode_batch(slots, [int(t[-1]) for t in ids], 1, want_logits=True)
+    orc = Qwen3Oracle(cfg, w)
+    for row, k, t in zip(got, lens, ids):
+        orc.clear_kv_cache()
         orc.forward(t[:k], 0)
         assert rel_err(row, orc.forward(t[k:], k).numpy()) < TOL
     m.close()
