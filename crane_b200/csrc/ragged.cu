@@ -7,6 +7,7 @@
 #include "ragged.cuh"
 #include "ragged_dev.cuh"
 #include "decode.cuh"
+#include "tc.cuh"
 
 #include <algorithm>
 
@@ -659,8 +660,8 @@ __global__ void conv_window_kernel(RaggedBatch rb, Mamba2Args a, int C, int col0
     }
 }
 
-// Selective scan.  Block = (entry, head, slice of SSD_COLS value columns); thread (p, ns) owns a run of state rows of
-// columns p and p + 16 in registers for the whole portion.  The recurrence itself is one FMA deep per token; what would serialise it is the
+// Selective scan.  Block = (entry, head, slice of 16 SSD_CPT value columns); thread (p, ns) owns a run of state rows of
+// columns p and p + 16 (SSD_CPT = 2; p alone with 1) in registers for the whole portion.  The recurrence itself is one FMA deep per token; what would serialise it is the
 // operand fetch, so the step inputs (x slice, B, C, dt) of SSD_CH tokens at a time are staged in shared memory with cp.async,
 // double-buffered: chunk c + 1 is in flight while chunk c is consumed.  dt = softplus(.) and the decay exp(-exp(A) dt) are
 // computed once per token, in f32, when its chunk lands.
@@ -668,9 +669,9 @@ __global__ void conv_window_kernel(RaggedBatch rb, Mamba2Args a, int C, int col0
 // and C, most of what a token reads from shared memory, are read once for both, and the outputs of four tokens are summed over the lanes together.
 // us, 16 heads of 128 x 128, one column and three shuffles a token / so: steps with a portion of 256 tokens 98 / 74, five entries 42 / 29.  (Segments from
 // 64 rows on gained nothing more for such portions: their second pass and the prefix take what they save.)
-constexpr int SSD_NS = 8, SSD_MAXR = 32, SSD_CPT = 2, SSD_COLS = 16 * SSD_CPT, SSD_CH = 16;      // N <= 256
-constexpr int SSD_TH = SSD_COLS / SSD_CPT * SSD_NS;         // 128 threads: one warp per scheduler, many blocks
-// Staged layout of one token: x slice [SSD_COLS] | B | C | dt, pad.  Thread ns owns the CONTIGUOUS state rows ns * R .. ns * R + R - 1,
+constexpr int SSD_NS = 8, SSD_MAXR = 32, SSD_CH = 16;      // N <= 256
+constexpr int SSD_TH = 16 * SSD_NS;                         // 128 threads: one warp per scheduler, many blocks
+// Staged layout of one token: x slice [16 SSD_CPT] | B | C | dt, pad.  Thread ns owns the CONTIGUOUS state rows ns * R .. ns * R + R - 1,
 // so it reads its B and C values as float4; every R-run is followed by 4 pad floats, which spreads the eight runs of a warp over
 // all banks.
 __host__ __device__ inline int ssd_idx(int n, int R) { return n + 4 * (n / R); }
@@ -682,8 +683,9 @@ __host__ __device__ inline int ssd_npad(int N, int R) { (void)N; return 8 * (R +
 // start state (and the sequence's new state); MODE 2 is the scan proper from those start states.  MODE 0 = one segment, everything.
 constexpr int SSD_SEGS = 4, SSD_SEG_MIN = 512;              // an entry is segmented from this many rows on
 __host__ __device__ inline int ssd_seg_len(int len) { return ((len + SSD_SEGS - 1) / SSD_SEGS + SSD_CH - 1) / SSD_CH * SSD_CH; }
-template <int SSD_R, int MODE>                               // state rows per thread: ceil(N / 8) rounded up to 4, 8, 16 or 32
+template <int SSD_R, int MODE, int SSD_CPT = 2>              // state rows per thread: ceil(N / 8) rounded up to 4, 8, 16 or 32
 __global__ void __launch_bounds__(SSD_TH) ssd_scan_kernel(RaggedBatch rb, Mamba2Args a, int C) {
+    constexpr int SSD_COLS = 16 * SSD_CPT;
     extern __shared__ __align__(16) float ssm_s[];
     const int e = MODE == 0 ? blockIdx.x : blockIdx.x / SSD_SEGS, seg = MODE == 0 ? 0 : blockIdx.x % SSD_SEGS;
     const int h = blockIdx.y, ns = threadIdx.x & (SSD_NS - 1), pl = threadIdx.x / SSD_NS;
@@ -801,20 +803,20 @@ __global__ void __launch_bounds__(SSD_TH) ssd_scan_kernel(RaggedBatch rb, Mamba2
                 for (int j = 0; j < SSD_CPT; ++j) y[tt * SSD_CPT + j] = y0[j] + y1[j];
             }
             if constexpr (MODE != 1) {
-                static_assert(4 * SSD_CPT == SSD_NS, "a value per lane");
-                int id = 0;
+                int id = 0, bit = SSD_NS / 2;
 #pragma unroll
-                for (int n = SSD_NS / 2; n >= 1; n >>= 1) {
-                    const bool up = ns & n;
+                for (int n = 2 * SSD_CPT; n >= 1; n >>= 1, bit >>= 1) {
+                    const bool up = ns & bit;
 #pragma unroll
                     for (int v = 0; v < n; ++v) {
                         const float give = up ? y[v] : y[v + n], keep = up ? y[v + n] : y[v];
-                        y[v] = keep + __shfl_xor_sync(0xffffffffu, give, n);
+                        y[v] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
                     }
                     id += up ? n : 0;
                 }
+                if (SSD_CPT == 1) y[0] += __shfl_xor_sync(0xffffffffu, y[0], 1);
                 const int t = t4 + id / SSD_CPT, col = pl + 16 * (id % SSD_CPT);
-                if (p0 + col < P && t < nt) a.y[(size_t)(r0 + c * SSD_CH + t) * inner + h * P + p0 + col] = y[0] + Dh * st[t * per_tok + col];
+                if ((SSD_CPT == 2 || !(ns & 1)) && p0 + col < P && t < nt) a.y[(size_t)(r0 + c * SSD_CH + t) * inner + h * P + p0 + col] = y[0] + Dh * st[t * per_tok + col];
             }
         }
         __syncthreads();                                      // the stage is free for chunk c + 2
@@ -1369,11 +1371,16 @@ int mamba2_mixer_launch(cudaStream_t st, const RaggedBatch& rb, const Mamba2Args
             if ((e = last_err())) return e;
         }
     }
-    const dim3 sgrid(rb.E, a.heads, (a.P + SSD_COLS - 1) / SSD_COLS);
+    const bool segs = a.seg_state != nullptr && a.max_len >= SSD_SEG_MIN;
     const int nr = (a.N + SSD_NS - 1) / SSD_NS, sthreads = SSD_TH;
     const int rr = nr <= 4 ? 4 : nr <= 8 ? 8 : nr <= 16 ? 16 : 32;
-    const size_t ssm = (size_t)(2 * SSD_CH * (SSD_COLS + 2 * ssd_npad(a.N, rr) + 4) + 2 * SSD_CH) * sizeof(float);      // <= 78 KB at N = 256
-    const bool segs = a.seg_state != nullptr && a.max_len >= SSD_SEG_MIN;
+    // Columns of a block.  States of more than 128 rows hold 64 values of two columns per thread and spill; with one column a thread has half the work per token, which
+    // is the shorter way while blocks of 16 columns have an SM each.  us, 16 / 32 columns, 16 heads of state 256 x 128: one entry of 1 token 8.4 / 9.6, of 64 24.8 / 29.9,
+    // of 500 136 / 186; two entries of 64 32.7 / 30.5, of 500 200 / 188.
+    const bool narrow = rr == 32 && !segs && rb.E * a.heads * ((a.P + 15) / 16) <= tc_device_sms();
+    const int cols = narrow ? 16 : 32;
+    const dim3 sgrid(rb.E, a.heads, (a.P + cols - 1) / cols);
+    const size_t ssm = (size_t)(2 * SSD_CH * (cols + 2 * ssd_npad(a.N, rr) + 4) + 2 * SSD_CH) * sizeof(float);      // <= 80 KB at N = 256
     auto run = [&](auto kern, SmemOptIn& seen, dim3 grid) -> int {
         if (const int er = ensure_dyn_smem(kern, ssm, seen)) return er;
         kern<<<grid, sthreads, ssm, st>>>(rb, a, C);
@@ -1382,8 +1389,10 @@ int mamba2_mixer_launch(cudaStream_t st, const RaggedBatch& rb, const Mamba2Args
     auto scan = [&](auto k4, auto k8, auto k16, auto k32, SmemOptIn* seen, dim3 grid) -> int {
         return nr <= 4 ? run(k4, seen[0], grid) : nr <= 8 ? run(k8, seen[1], grid) : nr <= 16 ? run(k16, seen[2], grid) : run(k32, seen[3], grid);
     };
-    static SmemOptIn seen0[4], seen1[4], seen2[4];
-    if (!segs) {
+    static SmemOptIn seen0[4], seen1[4], seen2[4], seen_n;
+    if (narrow) {
+        if ((e = run(ssd_scan_kernel<32, 0, 1>, seen_n, sgrid))) return e;
+    } else if (!segs) {
         if ((e = scan(ssd_scan_kernel<4, 0>, ssd_scan_kernel<8, 0>, ssd_scan_kernel<16, 0>, ssd_scan_kernel<32, 0>, seen0, sgrid))) return e;
     } else {
         const dim3 ggrid(rb.E * SSD_SEGS, a.heads, sgrid.z);

@@ -595,6 +595,28 @@ def test_widest_heads_largest_state_many_experts(precision, tol):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("state", [129, 192, 256])
+def test_large_states_in_blocks_of_16_and_32_columns(state):
+    """One entry takes blocks of 16 value columns (16 heads x 3 of 40), four entries blocks of 32: portions around the scan's turns of 4 and stages of 16 tokens."""
+    ssm = {"type": "mamba2", "mixer": {"heads": 16, "vdim": 40, "state": state, "groups": 2, "conv": 4, "norm_groups": 2}}
+    cfg = config([dict(ssm, mlp=DENSE)], width=128)
+    m, o = make(cfg, seed=37, precision="f32", max_tokens=512, max_batch=4)
+    ids = [tokens(60 + i, cfg["vocab"], 70 + i) for i in range(4)]
+    want = [o.forward(t, o.new_state()).numpy() for t in ids]
+    slots = [0] + [m.seq_create() for _ in range(3)]
+    at = 0
+    for n in (1, 3, 16, 17):                                                           # alone
+        assert rel(m.step_batch([(0, ids[0][at:at + n], all_rows(n))]), want[0][at:at + n]) < F32_TOL
+        at += n
+    for s, t, w in zip(slots[1:], ids[1:], want[1:]):
+        assert rel(m.step_batch([(s, t[:5], all_rows(5))]), w[:5]) < F32_TOL
+    ends = [(0, at, at + 19), (1, 5, 22), (2, 5, 6), (3, 5, 40)]                       # side by side
+    got = m.step_batch([(slots[i], ids[i][b:e], all_rows(e - b)) for i, b, e in ends])
+    assert rel(got, np.concatenate([want[i][b:e] for i, b, e in ends])) < F32_TOL
+    m.close()
+
+
+@pytest.mark.gpu
 def test_step_batch_rejects_bad_requests_and_stays_usable():
     import crane_b200
     m, o = make(SINGLE["dense"], 91, precision="f32", max_tokens=128, max_batch=2)
