@@ -135,6 +135,9 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
         // A thread's pieces sit at the same places of every super-block's 128 rows, and those of 32 rows repeat CPB pieces later: CPB offsets in registers and no
         // arithmetic beside the copies.  (Worked out per piece, a division by CPB and a 64-bit product each, the single warp of the wide tiles took
         // 2 us per super-block and paced the kernel: 24576 x 4096 at 64 rows Q4_K 51.5 us, 40.9 so; Q6_K at 512 rows 405 and 289.)
+        // Q8_0 at up to 32 rows works them out all the same: its four warps have the time, and with 17 copies of 16 bytes at once the HBM took longer (24576 x 4096: 16
+        // rows 53.6 us, 51.2 so; 32 rows 64.6 and 59.8; K-quants, of 9 and 14 pieces, 33.7 / 34.0 and 53.7 / 55.1).
+        constexpr bool PER_PIECE = QT == QT_Q8_0 && C::RAW_WARPS > 1;
         const int t = threadIdx.x - W_RAW * 32;
         constexpr int CPB = C::SB / 16, T = C::RAW_WARPS * 32, GRP = 128 / T;
         const uint32_t row_bytes = (uint32_t)KB * C::SB;
@@ -146,14 +149,14 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
             wait(&raw_empty[rs], rph ^ 1);
             const uint8_t* src = a.w + (size_t)n0 * row_bytes + (size_t)kb * C::SB;
             const uint32_t dst = smem_u32(sm + C::OFF_RAW + rs * C::RAW_BYTES) + t * 16;
-            if (n0 + 128 <= a.N) {
+            if (!PER_PIECE && n0 + 128 <= a.N) {
 #pragma unroll
                 for (int g = 0; g < GRP; ++g)
 #pragma unroll
                     for (int j = 0; j < CPB; ++j)
                         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + (g * CPB + j) * (T * 16)), "l"(src + (size_t)g * T * row_bytes + off[j]) : "memory");
-            } else {                                    // the last tile: rows behind the last one are zeros
-#pragma unroll 1
+            } else {                                    // (the last tile: rows behind the last one are zeros)
+#pragma unroll (PER_PIECE ? CPB * GRP : 1)
                 for (int j = 0; j < CPB * GRP; ++j) {
                     const uint32_t q = j * T + t, r = q / CPB;
                     const bool in = n0 + (int)r < a.N;
@@ -162,7 +165,8 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
             }
             asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&raw_full[rs])) : "memory");
             if (++rs == C::NR) { rs = 0; rph ^= 1; }
-            if (++kb == KB) { kb = 0; ++tile; n0 = tile / a.sc.tiles_m * 128; }
+            if constexpr (PER_PIECE) { kb = (it + 1) % KB; n0 = (it + 1) / KB / a.sc.tiles_m * 128; }
+            else if (++kb == KB) { kb = 0; ++tile; n0 = tile / a.sc.tiles_m * 128; }
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
     // ------------------------------------------------------------------------------------------------ activation codes and their scales by TMA
