@@ -1,6 +1,6 @@
-"""GPU (-m gpu): the decode chain where its splits can go wrong: contexts around the turns, tiles and splits of the attention kernel, query groups of every
-width a launch narrows or keeps, matrices whose rows and column chunks do not fill the GEMV's units and slices, groups of 1, 2 and 4 sequences, and forks
-of more segments than one launch copies.
+"""GPU (-m gpu): the decode chain where its splits can go wrong: contexts around the turns, tiles and splits of the attention kernel in both its forms, rings that
+come round several times, query groups of every width a launch narrows or keeps, matrices whose rows and column chunks do not fill the GEMV's units and slices,
+groups of 1, 2 and 4 sequences, and forks of more segments than one launch copies.
 
 Tolerance: cached keys and values carry two bf16 planes (2^-17 of each), everything else 24 bits; three layers, logits relative to the largest: 1e-4
 (measured 1e-5)."""
@@ -40,7 +40,7 @@ def test_one_sequence(heads, past):
 
 @pytest.mark.parametrize("n", [2, 4])
 def test_groups_of_sequences(n):
-    """Groups that go through the GEMVs (two sequences, and what a batch leaves over) against one sequence at a time."""
+    """Two sequences, which go through the GEMVs, and four, which share a pass over the tensor cores, each against the oracle."""
     cfg = dict(synth.TINY_QWEN3, intermediate_size=1280)
     m, w = _model(cfg, max_seq_len=320, max_batch=n)
     lens = [3, 130, 17, 66][:n]
@@ -54,6 +54,33 @@ def test_groups_of_sequences(n):
         orc = Qwen3Oracle(cfg, w)
         orc.forward(t[:k], 0)
         assert rel_err(row, orc.forward(t[k:], k).numpy()) < TOL
+    m.close()
+
+
+@pytest.mark.parametrize("n,kv_heads,dim,precision", [(20, 2, 128, "split"), (20, 2, 128, "bf16"), (20, 2, 256, "split"), (40, 4, 128, "split")],
+                         ids=["128 split", "128 bf16", "256 split", "two splits"])
+def test_rings_that_come_round(n, kv_heads, dim, precision):
+    """More (sequence, KV head) pairs than the tile form takes: a warp's ring has six places of two tokens (one at D = 256), and comes round behind 96 (48) tokens of each
+    of the four splits, or two of 160 pairs.  Contexts around once, twice and three times round, and around a turn, against each sequence alone in the tile form.
+    In plain bf16 a new key or value whose sums came in another order may round to the neighbouring bf16, 2^-8 of it; the results average over such values: 2^-9."""
+    tol = TOL if precision == "split" else 2.0 ** -9
+    cfg = dict(synth.TINY_QWEN3, num_hidden_layers=2, head_dim=dim, num_key_value_heads=kv_heads, num_attention_heads=2 * kv_heads)
+    m, _ = _model(cfg, max_seq_len=1216, max_batch=n, precision=precision)
+    turn = (4 if n == 20 else 2) * (16 if dim == 128 else 8)          # tokens that all splits' warps take at once
+    lens = [1, turn - 1, turn, turn + 1, 2 * turn + 1, 3 * turn] + [k * 6 * turn + d for k in (1, 2, 3) for d in (-1, 0, 1)]
+    lens = [min(k, 1200) for k in lens] + [int(k) for k in np.random.default_rng(dim).integers(2, 1200, n - len(lens))]
+    slots = [0] + [m.seq_create() for _ in range(n - 1)]
+    ids = [synth.synth_token_ids(k + 2, cfg["vocab_size"], f"r{i}") for i, k in enumerate(lens)]
+    want = []
+    for s, k, t in zip(slots, lens, ids):
+        m.seq_select(s)
+        m.forward_step(t[:k], 0)
+        want.append([m.forward_step(t[k + i:k + i + 1], k + i) for i in range(2)])
+        m.set_kv_caches([], k)
+    for i in range(2):
+        _, got = m.decode_batch(slots, [int(t[k + i]) for k, t in zip(lens, ids)], 1, want_logits=True)
+        for row, w, k in zip(got, want, lens):
+            assert rel_err(row, w[i]) < tol, k
     m.close()
 
 
