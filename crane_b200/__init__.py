@@ -25,7 +25,7 @@ F32, BF16, F16 = 0, 1, 2
 OK, INVALID_ARG, OOM, CUDA_ERROR, UNSUPPORTED, NOT_LOADED = 0, -1, -2, -3, -4, -5
 
 # cb::GemmEpiMode (crane_b200/csrc/gemm.cuh)
-EPI_STORE_F32, EPI_STORE_BF16, EPI_RESID_F32, EPI_SILU_MUL_BF16, EPI_GELU_ERF_BF16, EPI_GELU_TANH_BF16 = range(6)
+EPI_STORE_F32, EPI_STORE_BF16, EPI_RESID_F32, EPI_SILU_MUL_BF16, EPI_GELU_ERF_BF16, EPI_GELU_TANH_BF16, EPI_RELU2_BF16 = range(7)
 
 
 class CraneB200Error(RuntimeError):
@@ -127,6 +127,7 @@ _SIGNATURES = {
     "crane_b200_decode_path": (C.c_int, [C.c_void_p]),
     "crane_b200_prof_enable": (C.c_int, [C.c_void_p, C.c_int]),
     "crane_b200_prof_report": (C.c_int, [C.c_void_p, C.c_char_p, C.c_size_t, C.POINTER(C.c_size_t)]),
+    "crane_b200_op_gemm_epi": (C.c_int, [C.c_int] + [C.c_void_p] * 3 + [C.c_int] * 4 + [C.c_void_p] * 4 + [C.c_float] + [C.c_void_p] * 2),
     "crane_b200_op_gemm": (C.c_int, [C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p,
                                      C.c_void_p, C.c_int]),
 }
@@ -735,6 +736,24 @@ def op_gemm(a_bits: np.ndarray, w_bits: np.ndarray, mode: int, bias=None, out_in
     if rc != OK:
         raise CraneB200Error(rc, (lib.crane_b200_last_error(None) or b"").decode("utf-8", "replace"))
     return out
+
+
+def op_gemm_epi(a_bits, w_bits, mode: int, a_lo_bits=None, bias=None, col_scale=None, gate=None, gate_bias=None, glu_limit=0.0, out_init=None, lo=False, device=0):
+    """Kernel-level test hook: op_gemm with every part of the epilogue -> result (bf16 bits or f32), with `lo` beside the low-order plane's bits."""
+    lib = load_library()
+    M, K = a_bits.shape
+    N = w_bits.shape[0]
+    cols = N // 2 if mode == EPI_SILU_MUL_BF16 else N
+    half = mode not in (EPI_STORE_F32, EPI_RESID_F32)
+    out = np.zeros((M, cols), np.uint16 if half else np.float32) if out_init is None else np.ascontiguousarray(out_init).copy()
+    low = np.zeros((M, cols), np.uint16) if lo else None
+    ins = [np.ascontiguousarray(x) if x is not None else None for x in (a_bits, a_lo_bits, w_bits)]
+    f = [np.ascontiguousarray(x, dtype=np.float32) if x is not None else None for x in (bias, col_scale, gate, gate_bias)]
+    ptr = lambda x: None if x is None else _ptr(x)  # noqa: E731
+    rc = lib.crane_b200_op_gemm_epi(device, *map(ptr, ins), M, N, K, mode, *map(ptr, f), glu_limit, _ptr(out), ptr(low))
+    if rc != OK:
+        raise CraneB200Error(rc, (lib.crane_b200_last_error(None) or b"").decode("utf-8", "replace"))
+    return (out, low) if lo else out
 
 
 def op_topk(logits: np.ndarray, k: int, device=0) -> np.ndarray:

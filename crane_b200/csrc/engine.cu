@@ -2866,6 +2866,46 @@ int crane_b200_last_timing(const crane_b200_model* m, float* prefill_ms, float* 
     return CRANE_B200_OK;
 }
 
+int crane_b200_op_gemm_epi(int device, const uint16_t* a, const uint16_t* a_lo, const uint16_t* w, int M, int N, int K, int mode, const float* bias,
+                           const float* col_scale, const float* gate, const float* gate_bias, float glu_limit, void* out_inout, uint16_t* out_lo) {
+    if (!a || !w || !out_inout || M <= 0 || N <= 0 || K <= 0 || mode < EPI_STORE_F32 || mode > EPI_RELU2_BF16) return CRANE_B200_INVALID_ARG;
+    if (cudaSetDevice(device) != cudaSuccess) return CRANE_B200_CUDA_ERROR;
+    const bool half_out = mode != EPI_STORE_F32 && mode != EPI_RESID_F32;
+    const int cols = mode == EPI_SILU_MUL_BF16 ? N / 2 : N;
+    const size_t mk = (size_t)M * K, out_n = (size_t)M * cols;
+    int rc = CRANE_B200_OK;
+    std::vector<void*> bufs;
+    auto up = [&](const void* src, size_t bytes) -> void* {
+        if (!src) return nullptr;
+        void* p = nullptr;
+        CUDA_OK(cudaMalloc(&p, bytes));
+        bufs.push_back(p);
+        CUDA_OK(cudaMemcpy(p, src, bytes, cudaMemcpyHostToDevice));
+        return p;
+    };
+    try {
+        bf16 *da = (bf16*)up(a, mk * 2), *dl = (bf16*)up(a_lo, mk * 2), *dw = (bf16*)up(w, (size_t)N * K * 2);
+        void *dout = up(out_inout, out_n * (half_out ? 2 : 4)), *dlo = half_out ? up(out_lo, out_n * 2) : nullptr;
+        GemmEpi ep{dout, dlo, cols, (float*)up(bias, (size_t)N * 4), mode};
+        ep.col_scale = (float*)up(col_scale, (size_t)N * 4);
+        ep.gate = (float*)up(gate, (size_t)M * N * 4); ep.ldg = N;
+        ep.gate_bias = (float*)up(gate_bias, (size_t)N * 4);
+        ep.glu_limit = glu_limit;
+        const int r = gemm_bf16_launch(nullptr, da, dl, K, dw, M, N, K, ep, false);
+        if (r == -1000) fail(CRANE_B200_UNSUPPORTED, "op_gemm_epi: shape");
+        LAUNCH_OK(r);
+        CUDA_OK(cudaDeviceSynchronize());
+        check_waits(nullptr);
+        CUDA_OK(cudaMemcpy(out_inout, dout, out_n * (half_out ? 2 : 4), cudaMemcpyDeviceToHost));
+        if (dlo) CUDA_OK(cudaMemcpy(out_lo, dlo, out_n * 2, cudaMemcpyDeviceToHost));
+    } catch (const EngineError& e) {
+        g_create_error = e.msg;
+        rc = e.code;
+    }
+    for (void* p : bufs) cudaFree(p);
+    return rc;
+}
+
 int crane_b200_op_gemm(int device, const uint16_t* a, const uint16_t* a_lo, const uint16_t* w, int M, int N, int K, int mode, const float* bias,
                        void* out_inout, int use_simt) {
     if (!a || !w || !out_inout) return CRANE_B200_INVALID_ARG;

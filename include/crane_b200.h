@@ -317,6 +317,11 @@ CRANE_B200_API int crane_b200_decode_path(const crane_b200_model* m);
  * (NULL: plain bf16); mode = cb::GemmEpiMode; out dtype follows the mode. */
 CRANE_B200_API int crane_b200_op_gemm(int device, const uint16_t* a, const uint16_t* a_lo, const uint16_t* w, int M, int N, int K, int mode,
                        const float* bias, void* out_inout, int use_simt);
+/* The same with every part of the epilogue: col_scale [N], gate [M, N] with gate_bias [N], the gated unit's limit (all nullable / 0), and out_lo [M, out cols], the
+ * low-order plane of a bf16 result (NULL: none).  Tensor cores only. */
+CRANE_B200_API int crane_b200_op_gemm_epi(int device, const uint16_t* a, const uint16_t* a_lo, const uint16_t* w, int M, int N, int K, int mode,
+                                          const float* bias, const float* col_scale, const float* gate, const float* gate_bias, float glu_limit,
+                                          void* out_inout, uint16_t* out_lo);
 
 /* y[m, n] = quantised linear of x[m, k] (host f32) through the engine's kernels (xquant + qgemv up to 4 rows, Q8_0 6, qgemm above): `raw` = n rows
  * of ggml blocks (ggml_type 8 / 12 / 14), optional RMSNorm weight norm_w[k] applied first (eps).  = candle's CPU `QMatMul::forward`

@@ -113,6 +113,7 @@ extern "C" {
     pub fn crane_b200_prof_report(m: *const crane_b200_model, buf: *mut c_char, cap: usize, needed: *mut usize) -> c_int;
     pub fn crane_b200_decode_path(m: *const crane_b200_model) -> c_int;
     pub fn crane_b200_op_gemm(device: c_int, a: *const u16, a_lo: *const u16, w: *const u16, M: c_int, N: c_int, K: c_int, mode: c_int, bias: *const f32, out_inout: *mut c_void, use_simt: c_int) -> c_int;
+    pub fn crane_b200_op_gemm_epi(device: c_int, a: *const u16, a_lo: *const u16, w: *const u16, M: c_int, N: c_int, K: c_int, mode: c_int, bias: *const f32, col_scale: *const f32, gate: *const f32, gate_bias: *const f32, glu_limit: f32, out_inout: *mut c_void, out_lo: *mut u16) -> c_int;
     pub fn crane_b200_op_qlinear(device: c_int, x: *const f32, m: usize, k: usize, raw: *const c_void, raw_bytes: usize, ggml_type: c_int, n: usize, norm_w: *const f32, eps: f32, y: *mut f32) -> c_int;
     pub fn crane_b200_op_topk(device: c_int, logits: *const f32, vocab: usize, k: usize, idx_out: *mut u32) -> c_int;
     pub fn crane_b200_op_sample(device: c_int, logits: *const f32, vocab: usize, p: *const crane_b200_sampling, token_out: *mut u32, logits_after: *mut f32) -> c_int;
