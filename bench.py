@@ -1,11 +1,11 @@
 #!/usr/bin/env python
-"""bench.py -- Qwen3-VL-2B decode tok/s + prefill TFLOP/s on N x B200 (BASELINE.json `metric`), with the
+"""bench.py -- Qwen3-VL-2B decode tok/s + prefill TFLOP/s on N x B200 , with the
 kernel roofline and the reference-equivalent CPU path timed beside it.
 
     python bench.py --gpus N --steps K --warmup W            # this repo's CUDA path (C ABI)
     python bench.py --impl reference --steps K --warmup W    # the reference's CPU arithmetic (oracle) on host cores
 
-A *step* is one request of BASELINE.json configs[1]: one 448x448 image + 256 prompt tokens
+A *step* is one request: one 448x448 image + 256 prompt tokens
 (ViT -> splice -> prefill of 454 positions) followed by 256 greedy decode tokens.  Weights are the seeded
 synthetic checkpoint of crane_b200/synth.py (no checkpoints offline); per-GPU work is fixed as N grows
 (independent requests per rank, no data-path collective): "scaling": "weak".
@@ -36,7 +36,7 @@ IMAGE_HW = (448, 448)
 
 
 # --------------------------------------------------------------------------------------------------
-# workload + algorithmic cost model (SURVEY.md section 8d)
+# workload + algorithmic cost model
 # --------------------------------------------------------------------------------------------------
 def make_request(cfg, tag="bench"):
     image = synth.synth_image(*IMAGE_HW, tag=tag)
@@ -193,11 +193,11 @@ def run_cpu(cfg, weights, n_decode, steps, warmup, budget_s=None, keep_logits=Fa
 
 
 def bench_config4(args, rank, world, local_rank):
-    """BASELINE.json configs[3]: Qwen3-8B with a Q4_K_M-like GGUF recipe, 32 sequences decoded in lock-step, sharded over the N
+    """Qwen3-8B with a Q4_K_M-like GGUF recipe, 32 sequences decoded in lock-step, sharded over the N
     GPUs of the box (32 / N per rank: the total batch is fixed, "scaling": "strong"); every round ends with the NCCL all-gather of
     the 32 logits rows and greedy tokens (crane_b200_decode_batch_gather).  A step = one decode round of the whole batch.
     Weights are syntactically valid random ggml blocks (tools/bench_configs.py fake_blocks: timing only, parity of the quantised
-    path is tests/test_gpu_parity.py); the CPU arm of this config is not part of the driver's contract and is not run."""
+    path is tests/test_gpu_parity.py); the CPU arm of this config is not run."""
     import torch
     import crane_b200
     sys.path.insert(0, os.path.join(ROOT, "tools"))
@@ -298,7 +298,7 @@ def bench_config4(args, rank, world, local_rank):
 
 
 def bench_config2(args, rank, world, local_rank):
-    """BASELINE.json configs[2]: Qwen3.5-0.8B (3 Gated-Delta-Net layers per gated full-attention layer) bf16, one request =
+    """Qwen3.5-0.8B (3 Gated-Delta-Net layers per gated full-attention layer) bf16, one request =
     4096-token prefill + 512 greedy decode tokens on one GPU; N > 1 = N independent replicas ("scaling": "weak").  A step = one request.
     `value` = decode tok/s (CUDA events around the on-device loop), `prefill_*` from the events around the prefill pass, `e2e` =
     decode tokens / wall time of the whole request through the generate call (host token ids in, host token ids out).
@@ -974,7 +974,7 @@ def bench_rupulix(args, rank, world, local_rank):
 
 
 def other_config_summary(config, steps=2, timeout_s=120):
-    """One more BASELINE config measured by THIS script in a child process (`bench.py --config <config>`), condensed for the headline
+    """One more workload measured by THIS script in a child process (`bench.py --config <config>`), condensed for the headline
     line's `other_configs` field.  A child, so that nothing it does -- a failure, a hang (killed at the timeout) -- can keep the
     headline line from being printed; whatever goes wrong comes back as {"error": ...}."""
     try:
@@ -1228,7 +1228,7 @@ def main():
                          "min_top2_margin_rel": min(margins), "min_top2_margin_at_step": int(np.argmin(margins)),
                          "against": "oracle (torch f32) on the same full-size request; rel = max|d| / max|ref|"}
     if world == 1 and args.config == "qwen3_vl_2b" and not args.no_cpu_baseline and not args.no_other_configs and os.environ.get("CRANE_B200_BENCH_EXTRA", "1") != "0":
-        # BASELINE configs[2] beside the headline: Qwen3.5-0.8B, 4096-token prefill (chunkwise Gated-Delta-Net) + 512 decode tokens
+        # beside the headline: Qwen3.5-0.8B, 4096-token prefill (chunkwise Gated-Delta-Net) + 512 decode tokens
         out["other_configs"] = {"qwen3_5_0_8b": other_config_summary("qwen3_5_0_8b")}
     print(json.dumps(out))
     model.close()

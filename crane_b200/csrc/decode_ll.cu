@@ -3,7 +3,7 @@
 //
 // Why.  A batch-1 decode step of Qwen3-VL-2B is 141 dependent bandwidth-bound phases (113 weight matrices + 28 attentions) of
 // 1.3-96 us of HBM time each.  As separate kernels every phase boundary costs ~2.5 us during which the HBM pipe is idle
-// (round 1: 50 % of the HBM roofline); a grid barrier per phase costs about the same.  Here:
+// (50 % of the HBM roofline, measured); a grid barrier per phase costs about the same.  Here:
 //   * one CTA per SM stays resident; each of its 8 warps owns a fixed column range of every weight matrix and streams it, in
 //     tiles of 16 rows x 64 columns, through a private cp.async ring (12 x 2 KB per warp, 192 KB per SM).  The prefetch cursor
 //     is independent of the consumption cursor and runs ahead across phase, layer and token boundaries: while a warp waits

@@ -1,8 +1,8 @@
 // Chunkwise (WY / UT-transform) evaluation of the Gated-Delta-Net recurrence for prefill: 64 tokens per step instead of one.
 //
 // The reference evaluates  S <- S e^{g_t};  d = beta_t (v_t - S^T k_t);  S <- S + k_t d^T;  y_t = S^T q_t  token by token
-// (crane-core/src/ops/gdn/backend.rs:90-156, kernels/cuda/gdn.cu:29-153 -- 2 x __syncthreads per token) and so did round 1 of this
-// engine (gdn.cu: gdn_recur_kernel, 1.26 ms per layer at 4 096 tokens, latency-bound on 64 CTAs).  The same recurrence in chunk
+// (crane-core/src/ops/gdn/backend.rs:90-156, kernels/cuda/gdn.cu:29-153 -- 2 x __syncthreads per token) and so does
+// gdn_recur_kernel (gdn.cu; 1.26 ms per layer at 4 096 tokens, latency-bound on 64 CTAs).  The same recurrence in chunk
 // form is three launches, two of them parallel over all chunks and the serial one 64x shorter; kernels and algebra are in
 // gdn_chunk_kernels.inc, the numpy restatement the tests use is oracle/gdn_chunked.py.
 #include "gdn.cuh"

@@ -8,8 +8,8 @@
 
 namespace cb {
 
-// CRANE_B200_GEMM_BN=64|128|256 pins the tile width (sweeps).  (Round 1 also had 2x2 TMA-multicast clusters; measured on B200 they
-// did not pay -- the L2 already merges concurrent requests for a line from a few CTAs -- and they are gone.)
+// CRANE_B200_GEMM_BN=64|128|256 pins the tile width (sweeps).  (Clusters of 2 x 2 that share their loads
+// did not pay on B200: the L2 already merges concurrent requests for a line from a few CTAs.)
 static const int g_gemm_bn = [] { const char* e = getenv("CRANE_B200_GEMM_BN"); return e ? atoi(e) : 0; }();
 
 // =====================================================================================

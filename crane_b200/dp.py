@@ -1,6 +1,6 @@
 """Data-parallel plumbing for N replicas (one process per GPU): request sharding and the max-over-ranks timing rule.
 
-The hot path shards across independent sequences only (SURVEY.md section 8e): rank r owns requests {i : i mod N == r},
+The hot path shards across independent sequences only: rank r owns requests {i : i mod N == r},
 runs them on its own full-weight replica with no data-path collective, and the job throughput is
 (sum of units over ranks) / (max time over ranks).  `torch.distributed` (nccl on GPUs, gloo in the CPU tests) carries only
 these scalars.

@@ -22,7 +22,7 @@ import numpy as np
 SEED = 20260923
 
 # --------------------------------------------------------------------------------------
-# Configurations.  Starred values in SURVEY.md section 8 are pinned by the reference,
+# Configurations.  Values that the reference's code pins are its own,
 # the rest are the public HF config.json values of each checkpoint.
 # --------------------------------------------------------------------------------------
 
@@ -809,7 +809,7 @@ def synth_token_ids(n: int, vocab: int, tag: str = "ids", forbid=()) -> np.ndarr
 
 
 def synth_image(h: int, w: int, tag: str = "image") -> np.ndarray:
-    """uint8 HWC image (SURVEY.md section 8d)."""
+    """uint8 HWC image."""
     return _rng(tag).integers(0, 256, size=(h, w, 3), dtype=np.uint8)
 
 

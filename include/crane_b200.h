@@ -2,7 +2,7 @@
  * crane_b200 -- C ABI of the B200-native forward-pass engine that sits behind crane-core's model API.
  *
  * Every entry point below is what the reference's Rust side would bind through `extern "C"` for this
- * path; the reference interface each one replaces is cited as file:line under /root/reference.
+ * path; the reference interface each one replaces is cited as file:line of its project.
  * The Rust-side binding a Crane maintainer would add is shown in INTEGRATION.md.
  *
  * Conventions
@@ -96,7 +96,7 @@ CRANE_B200_API int crane_b200_load_tensor(crane_b200_model* m, const char* name,
  * crane-core/src/ops/linear.rs:23-48): decode streams the quantised bytes, prefill dequantises one matrix at a time. */
 CRANE_B200_API int crane_b200_load_tensor_ggml(crane_b200_model* m, const char* name, int ggml_type, const int64_t* shape, int ndim,
                                                const void* data, size_t nbytes);
-/* Whole-file readers (SURVEY 8f N1): every tensor of a .safetensors file (`VarBuilder::from_mmaped_safetensors`,
+/* Whole-file readers: every tensor of a .safetensors file (`VarBuilder::from_mmaped_safetensors`,
  * crane-core/src/models/qwen3/model.rs:91-92) or of a GGUF v2/v3 file (`gguf_file::Content::read` + `Qwen3Model::from_gguf`,
  * crane-core/src/models/qwen3/modeling.rs:821-935) is registered under its own name; quantised GGUF tensors keep their blocks.
  * Tensors the engine has no use for are skipped and counted in *n_skipped (both counters optional).  The model config still
@@ -206,7 +206,7 @@ CRANE_B200_API int crane_b200_step_batch(crane_b200_model* m, const crane_b200_s
 /* Tokens sequence `seq` holds in the cache. */
 CRANE_B200_API int crane_b200_seq_len(const crane_b200_model* m, int seq, size_t* len_out);
 
-/* ---- multi-GPU batch decode (32 sequences over 8 x B200) ----------------------------------------------
+/* ---- multi-GPU batch decode (32 sequences over 8 x B200, say) -----------------------------------------------------------
  * One process and one handle per GPU, every rank holding the full weights and its share of the sequences; the only data-path
  * exchange is the all-gather of each round's results (NCCL over NVLink, enqueued on the engine stream behind the lm_head).
  * NCCL (libnccl.so.2) is bound at run time by the first of these calls; a single-GPU deployment never loads it.
@@ -223,7 +223,7 @@ CRANE_B200_API int crane_b200_decode_batch_gather(crane_b200_model* m, const int
 /* Host copy of the rows gathered by the last decode_batch_gather that asked for logits ([world * n, V] f32; tests, host samplers). */
 CRANE_B200_API int crane_b200_copy_gathered_logits(crane_b200_model* m, float* host_out, size_t n_floats);
 
-/* ---- device-side sampling (crane-serve/src/engine/sampling.rs:169-480) ------------------------------------------ */
+/* ---- device-side sampling (crane-serve/src/engine/sampling.rs:169-480) ------------------------------------------------------- */
 /* Per-sequence sampling request = the fields of `Sequence` that `sampling::sample` reads.  The draw needs uniforms in
  * (1e-7, 0.999) (`rand_like(1e-7, 0.999)`, sampling.rs:387): the reference takes them from candle's device RNG, whose stream no
  * test pins, so they are an input here -- `uniforms` (host, top_k values, or vocab values when neither top-k nor top-p applies), or

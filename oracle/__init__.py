@@ -2,5 +2,5 @@
 
 Only tests/, __graft_entry__.smoke() and bench.py's cpu_baseline / --impl reference legs
 import this package.  The product (crane_b200/) never does and fails loudly without its
-CUDA library.  Parity status per component is recorded in DESIGN.md section "Oracle".
+CUDA library.  Each module says what its component's parity is pinned to.
 """

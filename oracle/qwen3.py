@@ -220,7 +220,7 @@ class Qwen3Oracle:
 
 
 def argmax_first(logits: torch.Tensor) -> int:
-    """Greedy rule of the oracle: lowest index among maxima (SURVEY.md A20)."""
+    """Greedy rule of the oracle: lowest index among maxima."""
     m = logits.max()
     return int(torch.nonzero(logits == m)[0, 0])
 

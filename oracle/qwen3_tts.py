@@ -12,7 +12,7 @@ pre-norm, per-head QK-norm before half-split RoPE, SwiGLU) -- arithmetic shared 
 Parity status: the decoder stack is pinned (via Qwen3Oracle vs HF); the TTS glue is restated from the reference only, and the
 reference's sampler (`LogitsProcessor::from_sampling(42, TopKThenTopP{k: 50})`, candle-transformers, un-vendored) is NOT
 pinned: the oracle takes a `pick(logits, kind, index)` callback (default: first maximum) or forced codes, so parity is
-checked on logits given forced tokens and on greedy codes (SURVEY.md section 8c).
+checked on logits given forced tokens and on greedy codes.
 """
 from __future__ import annotations
 

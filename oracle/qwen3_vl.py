@@ -1,8 +1,8 @@
 """CPU oracle for the Qwen3-VL prefix (ViT + splice + interleaved MRoPE + DeepStack)
 -- TEST INFRASTRUCTURE ONLY (see oracle/qwen3.py for the rules and the pinning story).
 
-The reference's `qwen3_vl` module is dead code (crane-core/src/models/mod.rs:19); per
-SURVEY.md F4 the arithmetic to follow is (all crane-core/src/models/):
+The reference's `qwen3_vl` module is dead code (crane-core/src/models/mod.rs:19); the
+arithmetic to follow is (all crane-core/src/models/):
   ViT .............................. qwen3_5/vision.rs (whole file; identical to qwen3_vl/vision.rs)
   text decoder ..................... qwen3/modeling.rs (oracle/qwen3.py)
   interleaved MRoPE cos/sin ........ qwen3_5/modeling.rs:172-245
@@ -12,7 +12,7 @@ SURVEY.md F4 the arithmetic to follow is (all crane-core/src/models/):
   DeepStack injection .............. qwen3_vl/text.rs:252-270,280-333
 Second opinion: HF `Qwen3VLForConditionalGeneration` (oracle/make_golden.py).
 
-Activation note (SURVEY.md A18): the reference maps the ViT MLP's `gelu_pytorch_tanh` to
+Activation note: the reference maps the ViT MLP's `gelu_pytorch_tanh` to
 candle `Activation::Gelu`, which is the ERF gelu (qwen3_5/config.rs:160-172), and the patch
 mergers call `xs.gelu()`, candle's TANH approximation (qwen3_5/vision.rs:276).  HF does the
 opposite.  `vit_act` / `merger_act` default to the reference's choice; the HF cross-check

@@ -1,6 +1,6 @@
 """GPU (-m gpu): the CUDA path, called through the C ABI, against the oracle and the committed fixtures.
 
-Tolerances ("rel" = max|a-b| / max|b| over a logits vector; BASELINE.json's bar is <=1e-3 rel against the f32 CPU path;
+Tolerances ("rel" = max|a-b| / max|b| over a logits vector; the bar is <=1e-3 rel against the f32 CPU path;
 the measured values are printed):
   * kernel-level GEMM, f32 output ...... 1e-5  (same bf16 inputs, f32 accumulation, different order)
   * default engine (split precision: hi+lo bf16 operands and KV pages) ... 1e-3 everywhere (measured ~1e-5 .. 3e-5)
@@ -20,7 +20,7 @@ from oracle.qwen3_vl import Qwen3VLOracle
 
 pytestmark = pytest.mark.gpu
 
-DECODE_TOL = 1e-3          # default (split-precision) engine
+DECODE_TOL = 1e-3          # default (split-precision) engine: the bar against the f32 path
 PREFILL_TOL = 1e-3
 FAST_DECODE_TOL = 1e-2     # "precision": "bf16"
 FAST_PREFILL_TOL = 2e-2
@@ -89,7 +89,7 @@ def test_gemm_epilogues(simt):
 @pytest.mark.parametrize("shape", [(454, 2048, 6144), (784, 1024, 4096), (454, 12288, 2048), (300, 1184, 512), (1, 2048, 64), (2000, 4096, 1024)],
                          ids=["down", "vit-fc2", "gate-up", "ragged-n", "one-row-one-kstep", "multi-wave"])
 def test_gemm_stream_k_full_width(shape):
-    """The persistent stream-K schedule at the widths of the BASELINE models: tiles shared by 2..5 CTAs (partials parked and summed
+    """The persistent stream-K schedule at the widths of the full-size models: tiles shared by 2..5 CTAs (partials parked and summed
     in contributor order), CTAs spanning several tiles (double-buffered accumulator), a ragged last column tile, every fused
     epilogue -- against float64, and bitwise equal from run to run."""
     M, N, K = shape
@@ -415,7 +415,7 @@ def test_gdn_chunkwise_recurrence_against_sequential_and_oracle(dk):
 @pytest.mark.parametrize("nh,nkv", [(6, 2), (12, 2), (16, 2), (10, 2), (24, 4)], ids=["nrep3", "nrep6", "nrep8", "nrep5", "nrep6-24over4"])
 def test_decode_attention_any_group_width(nh, nkv):
     """Query groups wider than the attention kernel's sub-group (4 heads) are served by several CTA clusters per KV head: 6 = 2 x 3,
-    8 = 2 x 4, 5 = 5 x 1 -- the north star's "4 KV heads broadcast to 24 Q heads" is the last case."""
+    8 = 2 x 4, 5 = 5 x 1 -- 4 KV heads broadcast to 24 Q heads is the last case."""
     cfg = dict(synth.TINY_QWEN3, num_attention_heads=nh, num_key_value_heads=nkv, num_hidden_layers=2)
     m, w = _model(cfg, persistent=False)
     orc = Qwen3Oracle(cfg, w)
@@ -432,7 +432,7 @@ def test_decode_attention_any_group_width(nh, nkv):
     m.close()
 
 
-# ---- full-width geometries of the BASELINE models (few layers, small vocabulary: seconds on the CPU oracle) -----------------------
+# ---- full-width geometries of the full-size models (few layers, small vocabulary: seconds on the CPU oracle) -----------------------
 
 WIDE_QWEN3_8B = dict(synth.QWEN3_8B, num_hidden_layers=2, vocab_size=4096, max_position_embeddings=4096)
 WIDE_QWEN3_5 = dict(synth.QWEN3_5_0_8B, num_hidden_layers=4, vocab_size=4096, max_position_embeddings=4096)
@@ -542,7 +542,7 @@ ALL_Q8_0 = {k: "Q8_0" for k in Q4_K_M_LIKE} | {"embed_tokens.weight": "Q8_0"}
 @pytest.mark.parametrize("qt", ["Q8_0", "Q4_K", "Q6_K"])
 @pytest.mark.parametrize("shape", [(5, 256, 96), (4, 4096, 300), (7, 12288, 148 * 2 + 3)], ids=["k256", "k4096-b4", "k12288"])
 def test_quantised_linear_kernel_against_integer_dot_oracle(qt, shape):
-    """xquant + qgemv on one linear at the widths of the BASELINE models (K = 4096: Qwen3-8B hidden, 12288: its MLP) and with the
+    """xquant + qgemv on one linear at the widths of the full-size models (K = 4096: Qwen3-8B hidden, 12288: its MLP) and with the
     4-row groups of batched decode, against ggml's integer dots (oracle/ggml_quant.py `qmatmul`): identical activation blocks and
     integer sums, so only the order of the f32 additions differs."""
     from oracle import ggml_quant as gq
@@ -597,12 +597,12 @@ def test_quantised_linears_against_integer_dot_oracle(recipe_name):
       3. the engine end to end on the 3-layer model: an activation that sits within ~1e-5 (the f32 / split-bf16 noise between two
          correct implementations) of a rounding boundary takes the neighbouring int8 code, and one flipped code moves an output
          by ~1e-3; a few of them per pass leave the logits within the scale of the quantisation noise itself, which is what is
-         asserted, with the distance to the un-quantised-activation semantics (round 1's oracle) printed beside it."""
+         asserted, with the distance to the un-quantised-activation semantics printed beside it."""
     cfg = synth.TINY_QWEN3_UNTIED if recipe_name == "q4_k_m_like" else synth.TINY_QWEN3
     recipe = Q4_K_M_LIKE if recipe_name == "q4_k_m_like" else ALL_Q8_0
     m, wq, qd = _quantised_model(cfg, recipe)
     orc = Qwen3Oracle(cfg, wq, quantised=qd)
-    plain = Qwen3Oracle(cfg, wq)                                  # y = x_f32 . dequant(W)^T: what round 1 compared against
+    plain = Qwen3Oracle(cfg, wq)                                  # y = x_f32 . dequant(W)^T
     ids = synth.synth_token_ids(70, cfg["vocab_size"], "quant")
     ref = orc.forward(ids, 0).numpy()
     # 1. kernels on the oracle's activations
@@ -889,7 +889,7 @@ def test_tts_frame_loop_against_oracle():
     m.close()
 
 
-# ---- native checkpoint readers (SURVEY 8f N1): a .safetensors file and a GGUF file read by the library itself ---------------------
+# ---- native checkpoint readers: a .safetensors file and a GGUF file read by the library itself ---------------------
 
 HF_TO_GGUF = {"input_layernorm.weight": "attn_norm.weight", "post_attention_layernorm.weight": "ffn_norm.weight",
               "self_attn.q_proj.weight": "attn_q.weight", "self_attn.k_proj.weight": "attn_k.weight", "self_attn.v_proj.weight": "attn_v.weight",
@@ -1110,7 +1110,7 @@ def test_qwen3_5_gguf_file(tmp_path):
     mq.close()
 
 
-# ---- device-side sampler (SURVEY 8f N2 / A20): top-k total order, penalties, top-p, Gumbel-max ----------------------------------------
+# ---- device-side sampler: top-k total order, penalties, top-p, Gumbel-max ----------------------------------------
 
 def test_topk_kernel_known_answers_and_host_order():
     """The reference's own top-k cases (crane-core/tests/rocm_kernels.rs:96-198) through the kernel: indices are compared bit for bit."""

@@ -1,5 +1,5 @@
 """CPU: the oracle against (a) the committed HF-generated fixtures and (b) every literal known answer /
-property the reference's own tests hold for this path (SURVEY.md section 8c)."""
+property the reference's own tests hold for this path."""
 import math
 
 import numpy as np

@@ -83,7 +83,7 @@ def _write_gguf(path, arch):
 
 @pytest.mark.parametrize("arch", ["qwen3", "qwen35"])
 def test_gguf_config_survives_mutated_files(tmp_path, arch):
-    """Found by this test in round 2 and fixed: a mutated `block_count` drove a 4-billion-entry `layer_types` loop (hang) or overflowed
+    """What this test found once: a mutated `block_count` drove a 4-billion-entry `layer_types` loop (hang) or overflowed
     the fixed 12 KB text buffer (truncated JSON returned as success); an architecture name with a quote in it produced invalid JSON;
     64-bit counts were cast to signed integers unchecked."""
     path = str(tmp_path / "meta.gguf")

@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Device timings for the other BASELINE.json configs (the headline config 1 is bench.py):
+"""Device timings for workloads beside bench.py's headline:
   c0  Qwen3-0.6B bf16          128-token prefill + 128 greedy decode steps
   c2  Qwen3.5-0.8B hybrid      4096-token prefill + 512 decode steps
   c3  Qwen3-8B Q4_K_M-like     4 sequences x (128-token prompt, 256 batched decode steps)  [the per-GPU share of batch 32 on 8 GPUs]
