@@ -1159,12 +1159,10 @@ def main():
 
     peaks = load_peaks()
     traffic = None           # DRAM bytes of one decode launch measured by ncu (tools/summarize_ncu.py traffic)
-    for tf in ("r02_traffic.json", "r01_traffic.json"):
-        try:
-            traffic = json.load(open(os.path.join(ROOT, "profiles", tf)))
-            break
-        except Exception:
-            pass
+    try:
+        traffic = json.load(open(os.path.join(ROOT, "profiles", "traffic.json")))
+    except Exception:
+        pass
     persistent = model.decode_path() == "persistent"
     # one launch of the dominant kernel: the persistent decode kernel runs all N_DECODE steps (contexts S .. S + N_DECODE - 1) in one
     # launch; the kernel-chain path replays one graph per step

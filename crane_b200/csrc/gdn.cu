@@ -37,7 +37,7 @@ gdn_conv_kernel(GdnArgs a) {
 
 // The same convolution for the usual 4-tap kernel over many rows: one thread per channel walks GDN_CONV_TT consecutive timesteps with
 // the tap window in registers, so every input element is loaded once (the per-element kernel above loads it ck times and, at
-// 4 096 rows, spends its time on 200 K tiny CTAs: 205 us per layer measured, profiles/r02_launches_gdn_chunk.csv).
+// 4 096 rows, spends its time on 200 K tiny CTAs: 205 us per layer measured).
 constexpr int GDN_CONV_TT = 32;
 __global__ void __launch_bounds__(128)
 gdn_conv4_rows_kernel(GdnArgs a) {

@@ -1,7 +1,7 @@
 #!/usr/bin/env python
 """tcgen05 GEMM timeline probe (run on the GPU box): for the prefill shapes of Qwen3-VL-2B, back-to-back event timing plus the
 per-CTA timeline (setup / first operands / main loop / accumulator wait / epilogue) written by the kernel's globaltimer stamps.
-  CRANE_B200_GEMM_CLUSTERS=0 python tools/gemm_probe.py      # without the multicast clusters"""
+  python tools/gemm_probe.py"""
 import os
 import sys
 

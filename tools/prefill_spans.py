@@ -1,7 +1,7 @@
 #!/usr/bin/env python
 """Stage spans of the headline request (ViT + prefill of 454 positions + 256 decode steps) through crane_b200_prof_enable /
 crane_b200_prof_report: device and host-submission time per stage, named as crane-core/src/ops/prof.rs names them.
-    python tools/prefill_spans.py [--reps 5] [--precision split|bf16] [--out profiles/r02_spans.json]"""
+    python tools/prefill_spans.py [--reps 5] [--precision split|bf16] [--out FILE]"""
 import argparse
 import json
 import os
