@@ -1052,7 +1052,7 @@ void crane_b200_model::linear_decode(int epi, bool norm, const bf16* w, const un
         if (!norm) g.norm_w = nullptr;
         qa.g = g; qa.qtype = qt; qa.epi = epi; qa.more = more;
         const int xmode = xq_mode_for(qt);
-        qa.xq = xquant_apart(B, K) ? xq_buf : nullptr;
+        qa.xq = xquant_apart(B, K, qt) ? xq_buf : nullptr;
         if (qa.xq && (!same_input || xmode != xq_mode_last)) {      // (same input, norm and block rule as the previous quantised linear: v after q and k)
             LAUNCH_OK(xquant_launch(stream, B, xin, ldx, K, g.norm_w, eps, xmode, xq_buf, use_pdl));
             xq_mode_last = xmode;
@@ -2781,7 +2781,7 @@ int crane_b200_op_qlinear(int device, const float* x, size_t m, size_t k, const 
             QGemvArgs qa = {};
             qa.g.W = reinterpret_cast<const bf16*>(dw); qa.g.N = (int)n; qa.g.K = (int)k; qa.g.y = dy + s0 * n; qa.g.ldy = (int)n; qa.g.eps = eps;
             qa.g.x = dx + s0 * k; qa.g.ldx = (int)k; qa.g.norm_w = dn; qa.qtype = ggml_type; qa.epi = GEMV_STORE;
-            if (xquant_apart(B, (int)k)) {
+            if (xquant_apart(B, (int)k, ggml_type)) {
                 LAUNCH_OK(xquant_launch(nullptr, B, dx + s0 * k, (int)k, (int)k, dn, eps, xq_mode_for(ggml_type), dxq, false));
                 qa.xq = dxq;
             }

@@ -378,7 +378,7 @@ qgemv_kernel(QGemvArgs qa) {
     const int mats = !MORE ? 1 : qa.more.n[1] ? 3 : 2;
     float* acc_s = reinterpret_cast<float*>(xbase + (size_t)B * xb);
     __shared__ uint64_t xbar;
-    __shared__ float red[B][32];
+    __shared__ float red[32];
     __shared__ float wbest_v[QG_MAXW][B];
     __shared__ int wbest_i[QG_MAXW][B];
     __shared__ int is_last_s;
@@ -456,39 +456,33 @@ qgemv_kernel(QGemvArgs qa) {
 #pragma unroll
         for (int b = 0; b < B; ++b) old[b] = tid < nrows ? a.y[(size_t)b * a.ldy + r0 + tid] : 0.f;
     // ---- the quantised activations: one bulk copy of the ready-made image, or every CTA for itself (xquant_apart) ----
-    if (qa.xq) {
+    constexpr bool INSIDE = B == 1 && QT == QT_Q8_0;
+    if (!INSIDE || qa.xq) {
         if (tid == 0) {
             mbar_arrive_expect_tx(&xbar, (uint32_t)(B * xb));
             bulk_load(xbase, qa.xq, (uint32_t)(B * xb), &xbar);
         }
         mbar_wait(&xbar, 0);
-    } else {
+    } else if constexpr (INSIDE) {
         const int nvw = min(32, (K + 127) / 128);           // of xq_ssq's 32 warps, those with anything to add
         if (a.norm_w) {
 #pragma unroll 1
-            for (int vw = warp; vw < nvw; vw += 2 * QG_WARPS) {      // two of them at once: their loads are in flight together
-                const int second = vw + QG_WARPS < nvw ? vw + QG_WARPS : -1;
-                float ssq[2][B];
+            for (int vw = warp; vw < nvw; vw += 4 * QG_WARPS) {      // four of them at once: their loads are in flight together
+                float ssq[4];
 #pragma unroll
-                for (int b = 0; b < B; ++b) {
-                    ssq[0][b] = xq_ssq(a.x + (size_t)b * a.ldx, K, vw * 32 + lane);
-                    ssq[1][b] = second < 0 ? 0.f : xq_ssq(a.x + (size_t)b * a.ldx, K, second * 32 + lane);
+                for (int j = 0; j < 4; ++j) ssq[j] = vw + j * QG_WARPS < nvw ? xq_ssq(a.x, K, (vw + j * QG_WARPS) * 32 + lane) : 0.f;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    ssq[j] = warp_sum(ssq[j]);
+                    if (lane == 0 && vw + j * QG_WARPS < nvw) red[vw + j * QG_WARPS] = ssq[j];
                 }
-#pragma unroll
-                for (int b = 0; b < B; ++b)
-#pragma unroll
-                    for (int j = 0; j < 2; ++j) {
-                        const float v = warp_sum(ssq[j][b]);
-                        if (lane == 0 && (j == 0 || second >= 0)) red[b][j ? second : vw] = v;
-                    }
             }
             __syncthreads();
         }
 #pragma unroll 1
-        for (int w = warp; w < B * (int)spr; w += QG_WARPS) {
-            const int b = w / (int)spr;
-            const float rstd = a.norm_w ? xq_rstd_of(warp_sum(lane < nvw ? red[b][lane] : 0.f), K, a.eps) : 1.f;
-            xq_image(xq_mode_for(QT), a.x + (size_t)b * a.ldx, a.norm_w, rstd, K, w - b * (int)spr, lane, xbase + (size_t)b * xb);
+        for (int g = warp; g < (int)spr; g += QG_WARPS) {
+            const float rstd = a.norm_w ? xq_rstd_of(warp_sum(lane < nvw ? red[lane] : 0.f), K, a.eps) : 1.f;
+            xq_image(xq_mode_for(QT), a.x, a.norm_w, rstd, K, g, lane, xbase);
         }
         __syncthreads();
     }
@@ -684,6 +678,7 @@ static int qgemv_launch_b(cudaStream_t st, const QGemvArgs& qa, int num_sms, boo
 int qgemv_launch(cudaStream_t st, int B, const QGemvArgs& qa, int num_sms, bool pdl) {
     if ((qa.g.K % 256) != 0 || qa.g.N <= 0 || (qa.g.ldx % 4) != 0) return -1000;
     if (qa.epi == GEMV_SILU_MUL && (qa.g.N % 2) != 0) return -1000;
+    if (!qa.xq && xquant_apart(B, qa.g.K, qa.qtype)) return -1000;
     switch (B) {
         case 1: return qgemv_launch_b<1>(st, qa, num_sms, pdl);
         case 2: return qgemv_launch_b<2>(st, qa, num_sms, pdl);

@@ -21,7 +21,7 @@ inline int q_src_block_elems(int qt) { return qt == QT_Q8_0 ? 32 : 256; }
 // Host: repack `rows` rows of K elements from the ggml byte layout into the device layout (dst sized rows * K/256 * q_sb_bytes).
 void q_repack_rows(int qt, const unsigned char* src, unsigned char* dst, size_t rows, int K);
 
-// Further matrices of a GEMV launch (k and v of q's type beside q): n[i] rows of w[i], results one behind the other's.  n = 0: none.
+// Further matrices of a GEMV launch (k and v of q's type beside q, which saves two launches a layer): n[i] rows of w[i], results one behind the other's.  n = 0: none.
 struct QMore { const unsigned char* w[2] = {nullptr, nullptr}; int n[2] = {0, 0}; };
 
 struct QGemvArgs {
@@ -40,10 +40,12 @@ __host__ __device__ constexpr int xq_mode_for(int qt) { return qt == QT_Q8_0 ? X
 // Quantise B activation rows (f32, row stride ldx; RMS-normalised with norm_w first when non-null) for qgemv_launch.
 size_t xquant_bytes(int B, int K);
 int xquant_launch(cudaStream_t st, int B, const float* x, int ldx, int K, const float* norm_w, float eps, int mode, unsigned char* out, bool pdl);
-// Does a launch of its own quantise the rows?  Up to 32 super-blocks (two per warp) every CTA of the GEMV does it for itself: the launch takes 3 - 4 us.  Beyond, 148
-// CTAs repeating it take longer.  us a call, in the GEMV / apart: two layers of width 2048 in Q8_0, four tokens 521 / 588; one layer of width 4096 in Q4_K_M,
-// four rows 192 / 156, two steps of four sequences 434 / 353.
-constexpr bool xquant_apart(int B, int K) { return B * (K / 256) > 32; }
+// Does a launch of its own quantise the rows?  One row in front of Q8_0 weights is quantised by every CTA of the GEMV for itself, up to 32 super-blocks (two per
+// warp); more rows, and the K-quants' blocks, whose largest value is looked for over the whole warp, are the shorter way apart.
+// us a call of four steps, two layers, in the GEMV / apart: Q8_0 one token of width 1024 (4 - 12 super-blocks) 392 / 405, 2048 (8 - 24) 458 / 492, 4096 (16, 48) 715 / 712;
+// two of 1024 (8 - 24) 482 / 485, of 2048 (16, 48) 583 / 544; four of 1024 (16 - 48) 608 / 560, of 2048 (32, 96) 706 / 642.  Q4_K_M one of 1024 443 / 432, of 2048 485 / 470, of
+// 4096 (16, 48) 738 / 715; two of 2048 616 / 578; four of 2048 815 / 691.
+constexpr bool xquant_apart(int B, int K, int qt) { return B > 1 || qt != QT_Q8_0 || K / 256 > 32; }
 
 int qgemv_launch(cudaStream_t st, int B, const QGemvArgs& a, int num_sms, bool pdl);
 
