@@ -1006,11 +1006,12 @@ static int attn_decode_launch_t(cudaStream_t st, int B, const AttnDecArgs& a, bo
     return (int)cudaLaunchKernelEx(&cfg, attn_decode_kernel<D, NREP, RING>, a);
 }
 // Tile form (a CTA requests its whole range ahead of the dependency wait) while its clusters of eight, one per (sequence, KV group), run at once: in split
-// precision a tile takes an SM, in plain bf16 a third of one.  Rings beyond.  us, tile / rings, contexts of 1000 tokens:
-//   split, D = 128, 8 KV heads   1 sequence 8.6 / 8.6, 2 16.8 / 9.7, 4 25.5 / 11.5         2 KV groups of 2   3 sequences (12 clusters) 11.8 / 11.7, 4 (16) 22.1 / 13.4
-//   split, D = 256, 2 KV heads   1 sequence 13.6 / 19.1, 5 14.5 / 19.4, 8 28.1 / 23.1      8 KV heads         1 sequence 12.8 / 14.3, 2 24.7 / 17.0
-//   plain, D = 128, 8 KV heads   4 sequences 11.0 / 10.3, in groups of two (64 heads) 2 sequences (32 clusters) 13.3 / 13.9, 3 (48) 24.8 / 20.7
-//   plain, D = 256               2 KV heads, 8 sequences 17.5 / 21.6; 8 KV heads, 4 17.2 / 17.2
+// precision a tile takes an SM, in plain bf16 a third of one.  Rings beyond.  us, tile / rings, contexts of 1000 tokens, single launches with cold caches (C: clusters):
+//   split, D = 128   2 KV heads of 2: 3 sequences (12 C) 10.1 / 10.5, 6 (12 C) 11.7 / 12.0, 9 (18 C) 19.6 / 13.7     4 heads: 3 (12 C) 11.9 / 12.7, 4 (16 C) 19.5 / 13.5
+//                    8 KV heads: 2 sequences (16 C) 19.0 / 13.1, 4 28.2 / 15.1
+//   split, D = 256   2 KV heads: 1 sequence 15.7 / 15.5, 5 (10 C) 18.0 / 17.7, 8 (16 C) 31.6 / 20.6     8 heads: 1 16.9 / 17.3, 2 (16 C) 31.6 / 20.9
+//   plain, D = 128   8 KV heads: 4 sequences (32 C) 12.4 / 12.8, 5 (40 C) 15.0 / 16.3; 64 heads over 8: 2 (32 C) 15.6 / 16.0, 3 (48 C) 26.2 / 21.4
+//   plain, D = 256   2 KV heads: 8 sequences 18.0 / 18.4; 8 heads: 4 (32 C) 19.8 / 19.7
 static bool attn_tile_form(const AttnDecArgs& a, int pairs) { return a.kv_bits || pairs <= (a.kv_lo_off ? tc_max_clusters(ATTN_NSPLIT) : 32); }
 
 template <int D, int NREP>

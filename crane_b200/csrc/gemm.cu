@@ -540,7 +540,8 @@ static int launch_tc(cudaStream_t stream, const bf16* A, const bf16* A_lo, int l
 
 // Tile width and schedule from a cost model fitted on B200 (microseconds; 42 shapes of 77 - 4096 rows, every width and schedule):
 //   a k-step costs t_k: 64- and 128-wide tiles wait for their operands, 128 x 256 ones for shared memory, which MMAs read at 96 bytes a cycle while TMA writes
-//   64 (two planes) or 96 (one) into it: 128 is the limit;
+//   64 (two planes) or 96 (one) into it: 128 is the limit.  (Split, 256 wide, us a step: 0.565 - 0.57 with 24 - 64 tiles at once, 0.57 - 0.58 with 80 - 112, 0.615 with 128 and 144, 0.70
+//   with 148, where the chip's power and the L2 begin to tell; hence 0.565, 0.60 above 96 and 0.66 with every SM busy.)
 //   whole tiles: each CTA runs ceil(tiles / CTAs) tiles, the epilogue of all but the last hidden under the next tile's MMAs;
 //   stream-K:    tiles x k-steps dealt evenly to all SMs, and the last of a tile's c contributors adding the others' parts.
 struct GemmPlan { int bn; bool stream_k; double cost; };

@@ -327,12 +327,16 @@ static int rows_cluster(int tiles_n, int steps, int sms) {
 // Is this kernel the faster one of the two for up to 128 rows?  Both stream the weights at about the same rate; the tiles of gemm.cu pay for 128 rows whatever M
 // is, while here the activations' traffic and the epilogue grow with the rows.  us, here / gemm.cu (planes x rows: weights):
 //   f32, a cluster per tile    always, but for 1 x 96 - 128 of K = 1024: 4096 x 1024 8.3 / 8.0 (1 x 77: 8.0 / 7.9; 4096 x 2048 11.3 / 12.0; 2 x 128: 4096 x 1024 10.0 / 10.2)
-//   f32, one CTA per tile      1 x 64: 12288 x 2048 13.2 / 15.4, 24576 x 4096 41.3 / 41.8; 1 x 96: 14.5 / 15.5, 46.4 / 42.5; 2 x 64: 18.0 / 18.2, 46.0 / 49.6; 2 x 96: 16384 x 2048 20.0 / 19.5
+//   f32, one CTA per tile      1 x 80: 12288 x 2048 10.9 / 12.9, 24576 x 4096 41.3 / 41.4; 1 x 96: 11.2 / 12.9, 43.3 / 41.8; 2 x 64: 16.7 / 17.7, 44.2 / 53.9; 2 x 96: 16384 x 2048
+//                              17.7 / 17.8, 24576 x 4096 47.1 / 54.1; 2 x 128: 18.3 / 18.1, 52.3 / 54.5
 //   gate / up, one plane       a cluster: 64 rows 6144 x 1024 7.9 / 9.0, 7168 x 1024 8.4 / 9.4; 77: 9.3 / 9.0, 10.0 / 10.1.  One CTA: 77 12288 x 2048 14.7 / 16.1, 24576 x 4096
 //                              43.2 / 44.4; 96: 15.4 / 16.2, 45.5 / 45.0
 //   gate / up, two planes      96 rows: 6144 x 1024 11.0 / 11.1, 12288 x 2048 19.9 / 20.6; 112: 11.6 / 11.2, 21.2 / 20.7; more tiles than SMs: 128 24576 x 4096 63.2 / 63.9
 //   other bf16 results         a cluster: 1 x 96 4096 x 1024 9.3 / 9.5, 112 10.2 / 9.6, 128 4096 x 2048 11.9 / 12.2; 2 x 128: 4096 x 1024 11.8 / 12.5
-//                              one CTA: 1 x 48: 12288 x 2048 15.1 / 14.7; 2 x 48: 15.9 / 18.3; 2 x 64: 21.0 / 18.8
+//                              one CTA: 1 x 48: 12288 x 2048 10.9 / 12.8, 24576 x 4096 38.8 / 40.5; 1 x 64: 11.1 / 12.8, 39.6 / 40.9; 1 x 80: 11.7 / 12.9, 41.7 / 40.9; 2 x 48:
+//                              12.1 / 17.6, 40.4 / 51.9; 2 x 64: 17.3 / 17.8, 45.0 / 52.0; 2 x 80: 18.2 / 17.9, 46.9 / 52.1
+// (One CTA per tile: measured back to back after either kernel got eight epilogue warps and the tiles lost their divisions.  The lines are those from before and lie on
+// the safe side: two f32 planes could go to 96 rows, other bf16 results to 64.)
 bool gemm_rows_pays(int mode, int P, int M, int N, int K) {
     if (M > 128) return false;
     const bool f32 = mode == EPI_STORE_F32 || mode == EPI_RESID_F32, glu = mode == EPI_SILU_MUL_BF16;

@@ -493,11 +493,13 @@ static int qgemm_launch_t(cudaStream_t st, const unsigned char* w, const QRows& 
 
 // Above 32 rows: tiles of 64 activation rows, or of 128 (K-quants only), which unpack a block of weights half as often but have two stages for their operands
 // instead of three and twice the partial tile to park and add for every CTA that shares one.  Estimated us of either: super-blocks on the busiest CTA,
-// CTAs per tile, a constant; fitted to 8 linears x 13 row counts (33 .. 512) at widths 1024, 2048, 4096: the choice is never more than 1.5 % off the better one.
-// us, 64 / 128 wide:
-//   Q4_K  6144 x 1024   128 rows 15.5 / 23.6, 512 31.7 / 39.7                       2048 x 2048   256 13.5 / 22.1, 512 17.4 / 26.6
-//         12288 x 2048  256 44.0 / 52.2, 512 77.4 / 79.9                            24576 x 4096  65 66.8 / 70.3, 128 69.4 / 72.0, 193 126 / 120, 512 246 / 225
-//   Q6_K  2048 x 6144   256 32.9 / 57.4, 512 52.1 / 61.7                            4096 x 12288  192 74.6 / 91.4, 256 95.1 / 93.0, 512 180 / 147
+// CTAs per tile, a constant; fitted to launches back to back, 8 linears x 13 row counts (33 .. 512) at widths 1024, 2048, 4096.
+// us of a prompt through one layer of Q4_K_M, every linear 64 wide / 128 wide / as estimated: width 4096  65 rows 292 / 392 / 287, 128 301 / 402 / 297, 256 447 / 500 / 427,
+// 384 611 / 601 / 561, 512 770 / 724 / 697; width 2048  256 242 / 321 / 234, 512 341 / 385 / 337; width 1024  512 220 / 280 / 221.
+// Launches by themselves with cold caches and a rested chip, 64 / 128 wide, where the wide form does better:
+//   Q4_K  6144 x 1024   128 rows 15.8 / 19.6, 512 26.5 / 28.9                       2048 x 2048   256 16.7 / 23.8, 512 21.0 / 29.1
+//         12288 x 2048  256 40.3 / 41.2, 512 69.2 / 63.9                            24576 x 4096  65 67.1 / 61.0, 128 68.9 / 63.2, 193 124 / 108, 512 238 / 198
+//   Q6_K  2048 x 6144   256 37.1 / 55.1, 512 58.7 / 60.6                            4096 x 12288  192 83.1 / 94.4, 256 105 / 95.5, 512 196 / 153
 // (Q8_0 reads an accumulator per 32 elements; at width 4096 a layer took 475 us at 128 rows and 1224 at 512 with 64, 655 and 1328 with 128.)
 static float qgemm_estimate(int qt, int nt, int M, int N, int K) {
     const long long iters = (long long)((M + nt - 1) / nt) * ((N + 127) / 128) * (K / 256), G = std::max<long long>(1, std::min<long long>(tc_device_sms(), iters / 2));
