@@ -278,8 +278,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     if (warp == 0) {
         if (lane == 0) {
             // A step takes the tensor pipe 130 to 530 ns and the issuing thread should take far less: the tile's coordinates are divided out once per
-            // segment, not per step.  (Four integer divisions a step made a step cost 325 - 420 ns whatever the tile's width: 1111 x 2048 x 6144 in
-            // plain bf16 took 39.9 us, 31.2 without them.)
+            // segment, not per step.  (Four integer divisions a step made a step of plain bf16 cost 325 - 420 ns whatever the tile's width; without them 250 with 64 columns, 267
+            // with 128, 340 - 420 with 256.)
             constexpr int B_OFF = Cfg::A_BYTES * (SPLIT ? 2 : 1);
             // weights do not depend on the predecessor kernel: their first tiles go out before the dependency wait
             const int npre = ep.w_dynamic ? 0 : min(it_end - it_begin, STAGES);

@@ -268,12 +268,10 @@ __device__ __forceinline__ void xq_image(int mode, const float* xrow, const floa
 // Sum of squares of a row, in ONE order whatever the launch: thread t of XQ_THREADS adds its pieces of four, a warp its lanes, 32 warps' sums last.  The scale of a row
 // decides which of two codes a value on their border takes, and a flipped code moves an output by 1 / 128 of its block: another order (the warps a GEMV happens to
 // have) gave a row other codes alone than in a group or a prompt.  Threads with 4 t >= K have nothing to add.
+__device__ __forceinline__ void xq_square(float& ssq, const float4& v) { ssq += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w; }
 __device__ __forceinline__ float xq_ssq(const float* xrow, int K, int t) {
     float ssq = 0.f;
-    for (int i = t * 4; i < K; i += XQ_THREADS * 4) {
-        const float4 v = *reinterpret_cast<const float4*>(xrow + i);
-        ssq += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-    }
+    for (int i = t * 4; i < K; i += XQ_THREADS * 4) xq_square(ssq, *reinterpret_cast<const float4*>(xrow + i));
     return ssq;
 }
 __device__ __forceinline__ float xq_rstd_of(float total, int K, float eps) { return rsqrtf(total / (float)K + eps); }
@@ -357,7 +355,8 @@ __host__ __device__ constexpr int qg_warps(int B) { return B >= 4 ? QG_W4_DEF : 
 // One CTA per SM owns a contiguous block of output rows.  Work unit = tile of QG_R rows x QG_KT super-blocks; a warp takes
 // a contiguous range of tiles (k fastest), streams each through its private cp.async ring, keeps its activation slice in
 // registers and one f32 accumulator per (row, sequence), and flushes them to the CTA's shared row accumulators when it
-// moves on to another row group.
+// moves on to another row group.  The flush is an atomic add: two warps' shares of a row give the same sum in either order; three or more, which short
+// row blocks of more than 4096 columns can have (512 x 6144), may differ in the last bit from run to run.
 // MORE: q, k and v share the launch (QMore)
 template <int B, int QT, bool MORE>
 __global__ void __launch_bounds__(qg_warps(B) * 32, 1)
@@ -398,8 +397,7 @@ qgemv_kernel(QGemvArgs qa) {
         m.nrows = max(0, min(m.nrows, m.r0 + m.rpc) - m.r0);
         return m;
     };
-    // this warp's tiles [t, end) of it, of R rows; `turn`: the warp that takes the first ones, as short matrices leave warps without any.  (Worked out ahead of the
-    // dependency wait: the divisions are 0.3 us.)
+    // this warp's tiles [t, end) of it, of R rows; `turn`: the warp that takes the first ones, as short matrices leave warps without any.
     struct Deal { uint32_t R, t, end; };
     uint32_t turn = 0;
     auto deal = [&](int nrows) {
@@ -416,7 +414,8 @@ qgemv_kernel(QGemvArgs qa) {
         }
         return d;
     };
-    const Deal d0 = deal(mat(0).nrows), d1 = MORE ? deal(mat(1).nrows) : d0, d2 = MORE && mats > 2 ? deal(mat(2).nrows) : d0;
+    const Deal d0 = deal(mat(0).nrows);
+    Deal d1 = d0, d2 = d0;
     auto dealt = [&](int k) { return !MORE || k == 0 ? d0 : k == 1 ? d1 : d2; };
     unsigned char* ring = qsm + (size_t)warp * QG_DEPTH * SLOT;
     const uint32_t ring_u32 = smem_u32(ring);
@@ -441,8 +440,13 @@ qgemv_kernel(QGemvArgs qa) {
         islot = islot + 1 == QG_DEPTH ? 0 : islot + 1;
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-#pragma unroll
-    for (int p = 0; p < QG_DEPTH; ++p) issue();
+    int primed = 0;
+    if (MORE) {                                         // (the first requests leave ahead of the other matrices' divisions)
+        for (; primed < QG_DEPTH && di.t < di.end; ++primed) issue();
+        d1 = deal(mat(1).nrows);
+        if (mats > 2) d2 = deal(mat(2).nrows);
+    }
+    for (; primed < QG_DEPTH; ++primed) issue();
     for (int i = tid; i < B * (qa.rpc[0] + (mats > 1 ? qa.rpc[1] : 0) + (mats > 2 ? qa.rpc[2] : 0)); i += QG_THREADS) acc_s[i] = 0.f;
     if (tid == 0) { mbar_init(&xbar, 1); fence_barrier_init(); }
     __syncthreads();
@@ -467,14 +471,22 @@ qgemv_kernel(QGemvArgs qa) {
         const int nvw = min(32, (K + 127) / 128);           // of xq_ssq's 32 warps, those with anything to add
         if (a.norm_w) {
 #pragma unroll 1
-            for (int vw = warp; vw < nvw; vw += 4 * QG_WARPS) {      // four of them at once: their loads are in flight together
-                float ssq[4];
+            for (int vw = warp; vw < nvw; vw += 4 * QG_WARPS) {      // four of them at once, of one or two pieces each (xquant_apart): all loads are in flight together
+                float4 v[4][2];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) ssq[j] = vw + j * QG_WARPS < nvw ? xq_ssq(a.x, K, (vw + j * QG_WARPS) * 32 + lane) : 0.f;
+                for (int j = 0; j < 4; ++j)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int w = vw + j * QG_WARPS, i = (w * 32 + lane + h * XQ_THREADS) * 4;
+                        v[j][h] = w < nvw && i < K ? *reinterpret_cast<const float4*>(a.x + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    }
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    ssq[j] = warp_sum(ssq[j]);
-                    if (lane == 0 && vw + j * QG_WARPS < nvw) red[vw + j * QG_WARPS] = ssq[j];
+                    float ssq = 0.f;
+                    xq_square(ssq, v[j][0]);
+                    xq_square(ssq, v[j][1]);            // (what is not there adds nothing)
+                    ssq = warp_sum(ssq);
+                    if (lane == 0 && vw + j * QG_WARPS < nvw) red[vw + j * QG_WARPS] = ssq;
                 }
             }
             __syncthreads();

@@ -42,7 +42,7 @@ size_t xquant_bytes(int B, int K);
 int xquant_launch(cudaStream_t st, int B, const float* x, int ldx, int K, const float* norm_w, float eps, int mode, unsigned char* out, bool pdl);
 // Does a launch of its own quantise the rows?  One row in front of Q8_0 weights is quantised by every CTA of the GEMV for itself, up to 32 super-blocks (two per
 // warp); more rows, and the K-quants' blocks, whose largest value is looked for over the whole warp, are the shorter way apart.
-// us a call of four steps, two layers, in the GEMV / apart: Q8_0 one token of width 1024 (4 - 12 super-blocks) 392 / 405, 2048 (8 - 24) 458 / 492, 4096 (16, 48) 715 / 712;
+// us a call of four steps, two layers, in the GEMV / apart: Q8_0 one token of width 1024 (4 - 12 super-blocks) 390 / 405, 2048 (8 - 24) 449 / 492, 4096 (16, 48) 679 / 712;
 // two of 1024 (8 - 24) 482 / 485, of 2048 (16, 48) 583 / 544; four of 1024 (16 - 48) 608 / 560, of 2048 (32, 96) 706 / 642.  Q4_K_M one of 1024 443 / 432, of 2048 485 / 470, of
 // 4096 (16, 48) 738 / 715; two of 2048 616 / 578; four of 2048 815 / 691.
 constexpr bool xquant_apart(int B, int K, int qt) { return B > 1 || qt != QT_Q8_0 || K / 256 > 32; }
