@@ -123,6 +123,8 @@ _SIGNATURES = {
     "crane_b200_vl_decode_step_argmax": (C.c_int, [C.c_void_p, C.c_uint32, C.c_size_t, C.POINTER(C.c_uint32)]),
     "crane_b200_next_mrope_pos": (C.c_uint32, [C.c_void_p]),
     "crane_b200_last_timing": (C.c_int, [C.c_void_p, C.POINTER(C.c_float), C.POINTER(C.c_float), C.POINTER(C.c_size_t)]),
+    "crane_b200_host_alloc": (C.c_int, [C.c_size_t, C.POINTER(C.c_void_p)]),
+    "crane_b200_host_free": (C.c_int, [C.c_void_p]),
     "crane_b200_kernel_launches": (C.c_uint64, [C.c_void_p]),
     "crane_b200_decode_path": (C.c_int, [C.c_void_p]),
     "crane_b200_prof_enable": (C.c_int, [C.c_void_p, C.c_int]),
@@ -170,6 +172,27 @@ def load_library():
 
 def _ptr(a: np.ndarray):
     return a.ctypes.data_as(C.c_void_p)
+
+
+class _Pinned:
+    """Owner of one buffer of the library's pinned pool; the arrays over it keep it alive."""
+
+    def __init__(self, address: int, shape, dtype):
+        self.__array_interface__ = {"data": (address, False), "shape": tuple(shape), "typestr": dtype.str, "version": 3}
+        self._address, self._free = address, load_library().crane_b200_host_free
+
+    def __del__(self):
+        self._free(self._address)
+
+
+def _result(shape, dtype=np.float32) -> np.ndarray:
+    """An uninitialised array for a call's results, in pinned memory while the pool has any (small ones: ordinary memory, a copy of a few KB is no faster there)."""
+    shape, dtype = tuple(int(n) for n in shape), np.dtype(dtype)
+    n = int(np.prod(shape, dtype=np.int64)) * dtype.itemsize
+    p = C.c_void_p()
+    if n < 4096 or load_library().crane_b200_host_alloc(n, C.byref(p)) != OK:
+        return np.empty(shape, dtype)
+    return np.asarray(_Pinned(p.value, shape, dtype))
 
 
 class Engine:
@@ -259,7 +282,7 @@ class Engine:
         return int(tok.value)
 
     def copy_logits(self) -> np.ndarray:
-        out = np.empty(self.vocab, dtype=np.float32)
+        out = _result((self.vocab,))
         self._ck(self.lib.crane_b200_copy_logits(self.h, _ptr(out), out.size))
         return out
 
@@ -323,7 +346,7 @@ class Engine:
         if not want_logits:
             return out, None
         rows, V = int(lg.rows), int(lg.vocab)
-        host = np.empty((rows, V), dtype=np.float32)
+        host = _result((rows, V))
         self._ck(self.lib.crane_b200_copy_gathered_logits(self.h, _ptr(host), host.size))
         return out, host
 
@@ -385,7 +408,7 @@ class Engine:
         self._ck(self.lib.crane_b200_step_batch(self.h, arr, len(entries), C.byref(lg)))
         if not rows or not copy:
             return None
-        out = np.empty((rows, self.vocab), dtype=np.float32)
+        out = _result((rows, self.vocab))
         self._ck(self.lib.crane_b200_copy_logits(self.h, _ptr(out), out.size))
         return out
 
@@ -399,7 +422,7 @@ class Engine:
         sq = np.ascontiguousarray(seqs, dtype=np.int32)
         tk = np.ascontiguousarray(tokens, dtype=np.uint32)
         out = np.empty((sq.size, n_steps), dtype=np.uint32)
-        lg = np.empty((sq.size, self.vocab), dtype=np.float32) if want_logits else None
+        lg = _result((sq.size, self.vocab)) if want_logits else None
         self._ck(self.lib.crane_b200_decode_batch(self.h, _ptr(sq), _ptr(tk), sq.size, n_steps, _ptr(out), None if lg is None else _ptr(lg)))
         return out, lg
 
@@ -448,8 +471,8 @@ class Engine:
         g = np.ascontiguousarray(grid_thw, dtype=np.uint32).reshape(-1, 3)
         merge = self.config["vision_config"]["spatial_merge_size"]
         n_tok = int(sum(int(t) * int(h) * int(w) for t, h, w in g) // (merge * merge))
-        out = np.empty((n_tok, self.hidden), dtype=np.float32)
-        ds = np.empty((want_deepstack, n_tok, self.hidden), dtype=np.float32) if want_deepstack else None
+        out = _result((n_tok, self.hidden))
+        ds = _result((want_deepstack, n_tok, self.hidden)) if want_deepstack else None
         self._ck(self.lib.crane_b200_encode_images(self.h, _ptr(pv), _ptr(g), g.shape[0], _ptr(out), None if ds is None else _ptr(ds)))
         return out, ds
 

@@ -19,6 +19,7 @@
 
 #include "decode.cuh"
 #include "decode_ll.cuh"
+#include "host_pool.h"
 #include "gdn.cuh"
 #include "gemm.cuh"
 #include "tc.cuh"
@@ -1963,6 +1964,11 @@ uint32_t crane_b200_model::fsv_greedy_rows(size_t rows, uint32_t* out) {
 // =================================================================================================
 // C ABI
 // =================================================================================================
+// A call that failed half way leaves no copy into the caller's memory behind: it may be another call's from now on.
+static void settle(crane_b200_model* m) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(m->stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) cudaStreamSynchronize(m->stream);
+}
 #define API_BEGIN(m)                                   \
     if (!(m)) return CRANE_B200_INVALID_ARG;           \
     try {                                              \
@@ -1971,6 +1977,7 @@ uint32_t crane_b200_model::fsv_greedy_rows(size_t rows, uint32_t* out) {
     }                                                  \
     catch (const EngineError& e) {                     \
         (m)->last_error = e.msg;                       \
+        if (e.code == CRANE_B200_CUDA_ERROR) settle(m);\
         return e.code;                                 \
     }                                                  \
     catch (const std::exception& e) {                  \
@@ -2024,6 +2031,7 @@ int crane_b200_create(const char* config_json, int device_ordinal, crane_b200_mo
                 CUDA_OK(cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking));
                 m->fsv->stream = m->stream;
                 *out = m.release();
+                HostPool::get().opened();
                 return CRANE_B200_OK;
             }
         }
@@ -2052,6 +2060,7 @@ int crane_b200_create(const char* config_json, int device_ordinal, crane_b200_mo
         return CRANE_B200_INVALID_ARG;
     }
     *out = m.release();
+    HostPool::get().opened();
     return CRANE_B200_OK;
 }
 
@@ -2074,8 +2083,19 @@ void crane_b200_destroy(crane_b200_model* m) {
     m->sampler.release();
     m->spans.release();
     for (cudaEvent_t e : {m->pev0, m->pev1, m->dev0, m->dev1}) if (e) cudaEventDestroy(e);
-    if (m->stream && m->owns_stream) { tc_scratch_release(m->stream); cudaStreamDestroy(m->stream); }
+    const bool own = m->owns_stream;
+    if (m->stream && own) { tc_scratch_release(m->stream); cudaStreamDestroy(m->stream); }
     delete m;
+    if (own) HostPool::get().closed();       // (a code predictor borrows its talker's stream and is no handle of its own)
+}
+
+int crane_b200_host_alloc(size_t bytes, void** out) {
+    if (!out || bytes == 0) return CRANE_B200_INVALID_ARG;
+    try { *out = HostPool::get().take(bytes); } catch (const std::exception&) { *out = nullptr; }
+    return *out ? CRANE_B200_OK : CRANE_B200_OOM;
+}
+int crane_b200_host_free(void* p) {
+    try { return HostPool::get().give(p) ? CRANE_B200_OK : CRANE_B200_INVALID_ARG; } catch (const std::exception&) { return CRANE_B200_OOM; }
 }
 
 const char* crane_b200_last_error(const crane_b200_model* m) { return m ? m->last_error.c_str() : g_create_error.c_str(); }

@@ -108,6 +108,8 @@ extern "C" {
     pub fn crane_b200_tts_prefill(m: *mut crane_b200_model, embeds: *const f32, prefill_len: usize, trailing_text: *const f32, n_trailing: usize, tts_pad_embed: *const f32) -> c_int;
     pub fn crane_b200_tts_generate(m: *mut crane_b200_model, max_frames: usize, repetition_penalty: f32, forced_frames: *const u32, frames_out: *mut u32, n_frames_out: *mut usize, first_logits_out: *mut f32, group_logits_out: *mut f32) -> c_int;
     pub fn crane_b200_last_timing(m: *const crane_b200_model, prefill_ms: *mut f32, decode_ms: *mut f32, decode_steps: *mut usize) -> c_int;
+    pub fn crane_b200_host_alloc(bytes: usize, out: *mut *mut c_void) -> c_int;
+    pub fn crane_b200_host_free(p: *mut c_void) -> c_int;
     pub fn crane_b200_kernel_launches(m: *const crane_b200_model) -> u64;
     pub fn crane_b200_prof_enable(m: *mut crane_b200_model, on: c_int) -> c_int;
     pub fn crane_b200_prof_report(m: *const crane_b200_model, buf: *mut c_char, cap: usize, needed: *mut usize) -> c_int;
