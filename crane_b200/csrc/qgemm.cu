@@ -45,14 +45,15 @@ struct QCfg {
     static constexpr int D_COLS = (MINS ? 2 : DG) * NT;         // TMEM: two such sets,
     static constexpr int UPS = QT == QT_Q6_K ? 2 : 1;           // then units of unpacked weights, this many to a super-block
     static constexpr int U_COLS = 128 * PLANES / UPS, NU = (512 - 2 * D_COLS) / U_COLS > 3 ? 3 : (512 - 2 * D_COLS) / U_COLS;
-    static constexpr int RAW_BYTES = 128 * SB;
+    static constexpr int RAW_BYTES = 128 * SB, RAW_REGS = QT == QT_Q4_K ? 5 : QT == QT_Q6_K ? 6 : 8;      // (16-byte pieces a thread reads per unit)
     static constexpr int NR = QT == QT_Q4_K ? (NT > 32 ? 5 : NT > 16 ? 6 : 8) : QT == QT_Q6_K ? (NT > 32 ? 5 : 6) : (NT > 32 ? 3 : 4);
     static constexpr int NB = QT == QT_Q6_K || NT < 64 ? 4 : 3;  // ring of codes, one unit each
     static constexpr int B2_BYTES = MINS ? NT * 32 : 0, B_BYTES = NT * 512 / UPS, STG_BYTES = B_BYTES + B2_BYTES;
     static constexpr int A2_BYTES = MINS ? 128 * 32 : 0;        // [NU]
-    // rings of scales, in super-blocks: who writes the scales of `it` has seen the MMAs of it - NU (weights) or it - NB (activations) done, so the
-    // accumulators of two super-blocks before that have been read
-    static constexpr int NS = NU > 2 && UPS == 1 ? 8 : 4, ND = NB + 2;
+    // rings of scales, in super-blocks.  Who writes the scales of `it` has seen the MMAs of an older one done, so the accumulators two hand-overs before that have
+    // been read.  Weights: in Q4_K it - NU (NU + 2 places); in Q6_K, written a unit ahead, the first half of it - 2 (4); in Q8_0, a super-block ahead, it - 3, of
+    // which at 16 rows only the super-block before it - 3 is known to have been read (NU + 3).  Activations: it - NB.
+    static constexpr int NS = (QT == QT_Q4_K && NU > 2) || (QT == QT_Q8_0 && NT == 16) ? 8 : 4, ND = NB + 2;
     static constexpr int SCW_BYTES = GROUPS * 128 * (MINS ? 8 : 4);
     static constexpr int DX_BYTES = GROUPS * NT * 4;
     static constexpr int EPI_WARPS = NT > 32 ? 8 : 4;
@@ -63,7 +64,7 @@ struct QCfg {
     static constexpr int OFF_A2 = NB * STG_PITCH, OFF_RAW = OFF_A2 + NU * A2_BYTES, OFF_SCW = OFF_RAW + NR * RAW_BYTES, OFF_DX = OFF_SCW + NS * SCW_BYTES,
                          OFF_BAR = OFF_DX + ND * DX_BYTES, SMEM = OFF_BAR + 512 + 1024;
     static_assert(SMEM <= 227 * 1024, "rings do not fit");
-    static_assert(NU >= 2 && 2 * D_COLS + NU * U_COLS <= 512 && NS >= (NU + UPS - 1) / UPS + 2, "TMEM");
+    static_assert(NU >= 2 && 2 * D_COLS + NU * U_COLS <= 512, "TMEM");
     static_assert(OFF_A2 % 1024 == 0 && OFF_RAW % 128 == 0 && OFF_DX % 16 == 0 && OFF_BAR % 8 == 0, "alignment");
 };
 
@@ -106,11 +107,22 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* v) {
           "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]),
           "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31]), "r"(taddr) : "memory");
 }
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* v) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
+        ::"r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
+          "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(taddr) : "memory");
+}
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {     // A from TMEM
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
                  ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
+
+// pairs of f32
+__device__ __forceinline__ uint64_t f2(float a, float b) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ void f2_split(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) { uint64_t r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) { uint64_t r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
 
 template <int QT, int NT>
 __global__ void __launch_bounds__(QCfg<QT, NT>::THREADS, 1)
@@ -245,33 +257,60 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
         }
     // ------------------------------------------------------------------------------------------------ weights: blocks -> f16 integers
     } else if (warp >= W_DEQ) {
-        // A lane has a row, the two warps of its 32 rows a half of every super-block each (Q6_K: of every unit), 64 elements at a time.
+        // A lane has a row, the two warps of its 32 rows a half of every super-block each (Q6_K: of every unit).  The raw bytes of the next unit are read into
+        // registers before this one's stores are waited for, so that only the instructions stand between two units.
         const int dw = warp - W_DEQ, half = dw >> 2, row = (dw & 3) * 32 + lane;
         const uint32_t lanes = (uint32_t)((dw & 3) * 32) << 16;
+        const int units = (it_end - it_begin) * C::UPS;
         int rs = 0, us = 0; uint32_t rph = 0, uph = 0;
-        for (int it = it_begin; it < it_end; ++it) {
-            wait(&raw_full[rs], rph);
-            uint8_t* scw = sm + C::OFF_SCW + (it & (C::NS - 1)) * C::SCW_BYTES;
+        uint4 raw[C::RAW_REGS];
+        uint32_t raw1 = 0;
+        auto fetch = [&](int u) {               // unit u: raw blocks of slot rs -> registers
+            const int n = C::UPS == 1 ? 0 : u % C::UPS;
+            if (n == 0) wait(&raw_full[rs], rph);
             const uint8_t* sb = sm + C::OFF_RAW + rs * C::RAW_BYTES + row * C::SB;
-#pragma unroll 1
-            for (int n = 0; n < C::UPS; ++n) {
+            if constexpr (QT == QT_Q4_K) {
+                raw[0] = *reinterpret_cast<const uint4*>(sb);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) raw[1 + j] = *reinterpret_cast<const uint4*>(sb + 16 + 64 * half + 16 * j);
+            } else if constexpr (QT == QT_Q6_K) {       // elements 128 n + 64 half ..: half n of the block, low or high nibbles
+#pragma unroll
+                for (int e = 0; e < 2; ++e) raw[e] = *reinterpret_cast<const uint4*>(sb + 128 + 32 * n + 16 * e);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) raw[2 + j] = *reinterpret_cast<const uint4*>(sb + 64 * n + 16 * j);
+                raw1 = *reinterpret_cast<const uint32_t*>(sb + 192 + 8 * n + 4 * half);       // scales: byte 2 * quarter + (element / 16)
+                if (n == 0 && half == 0)
+                    reinterpret_cast<float*>(sm + C::OFF_SCW + ((it_begin + u / C::UPS) & (C::NS - 1)) * C::SCW_BYTES)[row] =
+                        4.f * __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short*>(sb + 208)));
+            } else {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) raw[j] = *reinterpret_cast<const uint4*>(sb + 128 * half + 16 * j);
+                const uint2 d = *reinterpret_cast<const uint2*>(sb + 256 + 8 * half);
+                float* scw = reinterpret_cast<float*>(sm + C::OFF_SCW + ((it_begin + u) & (C::NS - 1)) * C::SCW_BYTES) + (4 * half) * 128 + row;
+                scw[0] = __half2float(__ushort_as_half((unsigned short)(d.x & 0xffffu))); scw[128] = __half2float(__ushort_as_half((unsigned short)(d.x >> 16)));
+                scw[256] = __half2float(__ushort_as_half((unsigned short)(d.y & 0xffffu))); scw[384] = __half2float(__ushort_as_half((unsigned short)(d.y >> 16)));
+            }
+            if (n == C::UPS - 1) {
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&raw_empty[rs]);
+                if (++rs == C::NR) { rs = 0; rph ^= 1; }
+            }
+        };
+        if (units > 0) fetch(0);
+        for (int u = 0; u < units; ++u) {
+            const uint32_t ta = tmem + lanes + (uint32_t)(2 * C::D_COLS + us * C::U_COLS);
+            const bool more = u + 1 < units;
+            if constexpr (QT == QT_Q4_K) {
+                const uint4 hdr = raw[0];
                 wait(&a_empty[us], uph ^ 1);
                 tc_fence_after();
-                const uint32_t ta = tmem + lanes + (uint32_t)(2 * C::D_COLS + us * C::U_COLS);
-#pragma unroll 1
-                for (int rr = 0; rr < 2 / C::UPS; ++rr) {
-                const int g = C::UPS == 1 ? 2 * half + rr : 2 * n + half;        // which 64 of the 256 elements
-                const uint32_t tg = ta + (uint32_t)(C::UPS == 1 ? g : half) * 32;
-                uint32_t o[32];
-                if constexpr (QT == QT_Q4_K) {
-                    const uint4 hdr = *reinterpret_cast<const uint4*>(sb);
-                    const uint4 w0 = *reinterpret_cast<const uint4*>(sb + 16 + 32 * g), w1 = *reinterpret_cast<const uint4*>(sb + 32 + 32 * g);
-                    // scales of sub-blocks 2g (low nibbles) and 2g + 1 (high): ggml get_scale_min_k4
-                    const int sh = 16 * (g & 1);
-                    const uint32_t y = hdr.y >> sh, z = hdr.w >> sh;
-                    const uint32_t sa = g < 2 ? y & 63 : (z & 0xF) | (((y >> 6) & 3) << 4), sb2 = g < 2 ? (y >> 8) & 63 : ((z >> 8) & 0xF) | (((y >> 14) & 3) << 4);
+#pragma unroll
+                for (int rr = 0; rr < 2; ++rr) {           // 64 elements: sub-blocks 4 half + 2 rr (low nibbles) and the one behind it (high); ggml get_scale_min_k4
+                    const uint32_t y = hdr.y >> (16 * rr), z = hdr.w >> (16 * rr);
+                    const uint32_t sa = half == 0 ? y & 63 : (z & 0xF) | (((y >> 6) & 3) << 4), sb2 = half == 0 ? (y >> 8) & 63 : ((z >> 8) & 0xF) | (((y >> 14) & 3) << 4);
                     const uint32_t s_lo = h2_int(sa), o_lo = h2_mul(s_lo, h2_const(0xE400)), t = h2_int(sb2), s_hi = h2_mul(t, h2_const(0x2C00)), o_hi = h2_mul(t, h2_const(0xD400));
-                    const uint32_t ww[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+                    const uint32_t ww[8] = {raw[1 + 2 * rr].x, raw[1 + 2 * rr].y, raw[1 + 2 * rr].z, raw[1 + 2 * rr].w, raw[2 + 2 * rr].x, raw[2 + 2 * rr].y, raw[2 + 2 * rr].z, raw[2 + 2 * rr].w};
+                    uint32_t o[32];
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {          // (1024 + q) * s - 1024 * s and (1024 + 16 q) * s / 16 - 64 * s: one rounding, exact
                         const uint32_t v = ww[i], v8 = v >> 8;
@@ -280,62 +319,68 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
                         o[16 + 2 * i] = h2_fma((v & 0x00F000F0u) | 0x64006400u, s_hi, o_hi);
                         o[16 + 2 * i + 1] = h2_fma((v8 & 0x00F000F0u) | 0x64006400u, s_hi, o_hi);
                     }
-                    tmem_st32(tg, o);
-                    if (g == 3) {                          // offsets m_0 .. m_7, 64 times them; d and dmin for the accumulators' readers
-                        uint32_t m[4], m64[4];
+                    tmem_st32(ta + (uint32_t)(2 * half + rr) * 32, o);
+                }
+                if (half == 1) {                           // offsets m_0 .. m_7, 64 times them; d and dmin for the accumulators' readers
+                    uint32_t m[4], m64[4];
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            uint32_t mj[2];
+                    for (int j = 0; j < 4; ++j) {
+                        uint32_t mj[2];
 #pragma unroll
-                            for (int e = 0; e < 2; ++e) {
-                                const int q = 2 * j + e, b = 8 * (q & 3);
-                                mj[e] = q < 4 ? (hdr.z >> b) & 63 : ((hdr.w >> (b + 4)) & 0xF) | (((hdr.z >> (b + 6)) & 3) << 4);
-                            }
-                            m[j] = h2_add((mj[0] | (mj[1] << 16)) + 0x64006400u, h2_const(0xE400));
-                            m64[j] = h2_mul(m[j], h2_const(0x5400));
+                        for (int e = 0; e < 2; ++e) {
+                            const int q = 2 * j + e, b = 8 * (q & 3);
+                            mj[e] = q < 4 ? (hdr.z >> b) & 63 : ((hdr.w >> (b + 4)) & 0xF) | (((hdr.z >> (b + 6)) & 3) << 4);
                         }
-                        uint8_t* a2 = sm + C::OFF_A2 + us * C::A2_BYTES + row * 32;
-                        const int sw = ((row >> 2) & 1) << 4;
-                        *reinterpret_cast<uint4*>(a2 + sw) = make_uint4(m[0], m[1], m[2], m[3]);
-                        *reinterpret_cast<uint4*>(a2 + (sw ^ 16)) = make_uint4(m64[0], m64[1], m64[2], m64[3]);
-                        reinterpret_cast<float2*>(scw)[row] = make_float2(__half2float(__ushort_as_half((unsigned short)(hdr.x & 0xffffu))), __half2float(__ushort_as_half((unsigned short)(hdr.x >> 16))));
+                        m[j] = h2_add((mj[0] | (mj[1] << 16)) + 0x64006400u, h2_const(0xE400));
+                        m64[j] = h2_mul(m[j], h2_const(0x5400));
                     }
-                } else if constexpr (QT == QT_Q6_K) {
-                    const int h = g >> 1, p = g & 1;       // p = 0: low nibbles, quarters q1 | q2 of half h; p = 1: high nibbles, q3 | q4
-                    if (g == 0) reinterpret_cast<float*>(scw)[row] = 4.f * __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short*>(sb + 208)));
-                    const uint32_t sw = *reinterpret_cast<const uint32_t*>(sb + 192 + 8 * h + 4 * p);       // scales: byte 2 * quarter + (element / 16)
-                    const uint32_t lmul = p ? h2_const(0x2400) : h2_const(0x3400), lofs = p ? h2_const(0xCC00) : h2_const(0xDC00);    // 1/64, 1/4; -16, -256
-                    const uint32_t lm = p ? 0x00F000F0u : 0x000F000Fu;
-                    uint32_t oh[32];
+                    uint8_t* a2 = sm + C::OFF_A2 + us * C::A2_BYTES + row * 32;
+                    const int sw = ((row >> 2) & 1) << 4;
+                    *reinterpret_cast<uint4*>(a2 + sw) = make_uint4(m[0], m[1], m[2], m[3]);
+                    *reinterpret_cast<uint4*>(a2 + (sw ^ 16)) = make_uint4(m64[0], m64[1], m64[2], m64[3]);
+                    reinterpret_cast<float2*>(sm + C::OFF_SCW + ((it_begin + u) & (C::NS - 1)) * C::SCW_BYTES)[row] =
+                        make_float2(__half2float(__ushort_as_half((unsigned short)(hdr.x & 0xffffu))), __half2float(__ushort_as_half((unsigned short)(hdr.x >> 16))));
+                    fence_proxy_async();                   // (the offsets' tile is in shared memory)
+                }
+                if (more) fetch(u + 1);
+            } else if constexpr (QT == QT_Q6_K) {
+                // half = 0: low nibbles, quarters q1 | q2 of the block's half; 1: high nibbles, q3 | q4
+                const uint32_t lmul = half ? h2_const(0x2400) : h2_const(0x3400), lofs = half ? h2_const(0xCC00) : h2_const(0xDC00);    // 1/64, 1/4; -16, -256
+                const uint32_t lm = half ? 0x00F000F0u : 0x000F000Fu;
+                wait(&a_empty[us], uph ^ 1);
+                tc_fence_after();
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {              // q: which of the two quarters, elements [32 q, 32 q + 32) of the 64
+                    uint32_t lo[16], hi[16];
+                    // high plane: two bits at 2 q (after the shift by 4 half): (1024 + 4^q v - 1024 - 2 * 4^q) * 4 f / 4^q
+                    const uint32_t hm = q ? 0x000C000Cu : 0x00030003u, hsub = q ? h2_const(0xE408) : h2_const(0xE402);
 #pragma unroll
                     for (int e = 0; e < 2; ++e) {          // e: elements [16 e, 16 e + 16) of a quarter
-                        const uint4 qh = *reinterpret_cast<const uint4*>(sb + 128 + 32 * h + 16 * e);
-                        const uint32_t wh[4] = {qh.x >> (4 * p), qh.y >> (4 * p), qh.z >> (4 * p), qh.w >> (4 * p)};
+                        const uint32_t f = h2_byte(raw1 >> (16 * q + 8 * e)), ls = h2_mul(f, lmul), lo_o = h2_mul(f, lofs), hs = q ? f : h2_mul(f, h2_const(0x4400));
+                        const uint32_t wl[4] = {raw[2 + 2 * q + e].x, raw[2 + 2 * q + e].y, raw[2 + 2 * q + e].z, raw[2 + 2 * q + e].w};
+                        const uint32_t wh[4] = {raw[e].x >> (4 * half), raw[e].y >> (4 * half), raw[e].z >> (4 * half), raw[e].w >> (4 * half)};
 #pragma unroll
-                        for (int q = 0; q < 2; ++q) {      // q: which of the two quarters, elements [32 q, 32 q + 32) of the step
-                            const uint4 ql = *reinterpret_cast<const uint4*>(sb + 64 * h + 32 * q + 16 * e);
-                            const uint32_t f = h2_byte(sw >> (16 * q + 8 * e)), ls = h2_mul(f, lmul), lo_o = h2_mul(f, lofs);
-                            // high plane: two bits at 2 q (after the shift by 4 p): (1024 + 4^q v - 1024 - 2 * 4^q) * 4 f / 4^q
-                            const uint32_t hm = q ? 0x000C000Cu : 0x00030003u, hsub = q ? h2_const(0xE408) : h2_const(0xE402), hs = q ? f : h2_mul(f, h2_const(0x4400));
-                            const uint32_t wl[4] = {ql.x, ql.y, ql.z, ql.w};
-                            uint32_t *lo = o + 16 * q + 8 * e, *hi = oh + 16 * q + 8 * e;
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                const uint32_t v = wl[i], v8 = v >> 8, u = wh[i], u8 = u >> 8;
-                                lo[2 * i] = h2_fma((v & lm) | 0x64006400u, ls, lo_o);
-                                lo[2 * i + 1] = h2_fma((v8 & lm) | 0x64006400u, ls, lo_o);
-                                hi[2 * i] = h2_mul(h2_add((u & hm) | 0x64006400u, hsub), hs);
-                                hi[2 * i + 1] = h2_mul(h2_add((u8 & hm) | 0x64006400u, hsub), hs);
-                            }
+                        for (int i = 0; i < 4; ++i) {
+                            const uint32_t v = wl[i], v8 = v >> 8, w = wh[i], w8 = w >> 8;
+                            lo[8 * e + 2 * i] = h2_fma((v & lm) | 0x64006400u, ls, lo_o);
+                            lo[8 * e + 2 * i + 1] = h2_fma((v8 & lm) | 0x64006400u, ls, lo_o);
+                            hi[8 * e + 2 * i] = h2_mul(h2_add((w & hm) | 0x64006400u, hsub), hs);
+                            hi[8 * e + 2 * i + 1] = h2_mul(h2_add((w8 & hm) | 0x64006400u, hsub), hs);
                         }
                     }
-                    tmem_st32(tg, o);
-                    tmem_st32(tg + C::U_COLS / 2, oh);
-                } else {
-                    const uint32_t d2 = *reinterpret_cast<const uint32_t*>(sb + 256 + 4 * g);
+                    tmem_st16(ta + (uint32_t)(32 * half + 16 * q), lo);
+                    tmem_st16(ta + (uint32_t)(C::U_COLS / 2 + 32 * half + 16 * q), hi);
+                }
+                if (more) fetch(u + 1);
+            } else {
+                wait(&a_empty[us], uph ^ 1);
+                tc_fence_after();
+#pragma unroll
+                for (int rr = 0; rr < 2; ++rr) {
+                    uint32_t o[32];
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
-                        const uint4 qv = *reinterpret_cast<const uint4*>(sb + 64 * g + 16 * c);
+                        const uint4 qv = raw[4 * rr + c];
                         const uint32_t ww[4] = {qv.x ^ 0x80808080u, qv.y ^ 0x80808080u, qv.z ^ 0x80808080u, qv.w ^ 0x80808080u};   // + 128: 0 .. 255
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
@@ -343,19 +388,15 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
                             o[8 * c + 2 * i + 1] = h2_add(((ww[i] >> 8) & 0x00FF00FFu) | 0x64006400u, h2_const(0xE480));
                         }
                     }
-                    tmem_st32(tg, o);
-                    reinterpret_cast<float*>(scw)[(2 * g) * 128 + row] = __half2float(__ushort_as_half((unsigned short)(d2 & 0xffffu)));
-                    reinterpret_cast<float*>(scw)[(2 * g + 1) * 128 + row] = __half2float(__ushort_as_half((unsigned short)(d2 >> 16)));
+                    tmem_st32(ta + (uint32_t)(2 * half + rr) * 32, o);
                 }
+                if (more) fetch(u + 1);
             }
-                tmem_st_wait();
-                tc_fence_before();
-                if (C::MINS && half == 1) fence_proxy_async();            // (the offsets' tile is in shared memory)
-                __syncwarp();
-                if (lane == 0) { mbar_arrive(&a_full[us]); if (n == C::UPS - 1) mbar_arrive(&raw_empty[rs]); }
-                if (++us == C::NU) { us = 0; uph ^= 1; }
-            }
-            if (++rs == C::NR) { rs = 0; rph ^= 1; }
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&a_full[us]);
+            if (++us == C::NU) { us = 0; uph ^= 1; }
         }
     // ------------------------------------------------------------------------------------------------ accumulators -> f32 sums -> epilogue
     } else {
@@ -393,10 +434,10 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
                             const float4 x = *reinterpret_cast<const float4*>(dx + g * NT + c + j);
                             const float xv[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-                            for (int e = 0; e < 4; ++e) {
-                                float v = dw * __uint_as_float(r[j + e]);
-                                if (C::MINS) v = fmaf(-dm, __uint_as_float(s[j + e]), v);
-                                acc[c + j + e] = fmaf(v, xv[e], acc[c + j + e]);
+                            for (int e = 0; e < 4; e += 2) {         // two columns an instruction, each rounded as by itself
+                                uint64_t v = f2_mul(f2(dw, dw), f2(__uint_as_float(r[j + e]), __uint_as_float(r[j + e + 1])));
+                                if (C::MINS) v = f2_fma(f2(-dm, -dm), f2(__uint_as_float(s[j + e]), __uint_as_float(s[j + e + 1])), v);
+                                f2_split(f2_fma(v, f2(xv[e], xv[e + 1]), f2(acc[c + j + e], acc[c + j + e + 1])), acc[c + j + e], acc[c + j + e + 1]);
                             }
                         }
                     }
@@ -424,13 +465,17 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
                     __threadfence();
 #pragma unroll
                     for (int j = 0; j < C::ACC; ++j) acc[j] = 0.f;
-                    for (int cc = c_first; cc <= c_last; ++cc) {
-                        const float* p = a.sc.ws + (size_t)(2 * cc + (sched_start(a.sc, cc) < t * KB ? 1 : 0)) * TILE_F + (size_t)col0 * 128 + row;
+                    // a contributor's columns are on their way while the one's before it are added
+                    auto part = [&](int cc) { return a.sc.ws + (size_t)(2 * cc + (sched_start(a.sc, cc) < t * KB ? 1 : 0)) * TILE_F + (size_t)col0 * 128 + row; };
+                    float x[C::ACC];
+                    const float* p = part(c_first);
 #pragma unroll
-                        for (int j = 0; j < C::ACC; ++j) {
-                            acc[j] += __ldcg(p + j * 128);
-                            if ((j & 15) == 15) asm volatile("" ::: "memory");     // 16 loads in flight, not all: registers
-                        }
+                    for (int j = 0; j < C::ACC; ++j) x[j] = __ldcg(p + j * 128);
+#pragma unroll 1
+                    for (int cc = c_first; cc <= c_last; ++cc) {
+                        p = part(min(cc + 1, c_last));
+#pragma unroll
+                        for (int j = 0; j < C::ACC; ++j) { acc[j] += x[j]; x[j] = __ldcg(p + j * 128); }
                     }
                     if (threadIdx.x == 0) a.sc.counters[t] = 0;
                 }
@@ -439,12 +484,14 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
             if (finish) {
                 const int n = n0 + row, cols = min(C::ACC, a.M - m0 - col0);
                 if (a.epi == GEMV_SILU_MUL) {                       // rows interleaved (gate_j, up_j): neighbouring lanes
-                    float* y = a.y + (size_t)(m0 + col0) * a.ldy + (n >> 1);
-                    const bool mine = !(lane & 1) && n < a.N;
+                    // the even lane takes the even columns, the odd lane the odd ones
+                    const int odd = lane & 1;
+                    float* y = a.y + (size_t)(m0 + col0 + odd) * a.ldy + (n >> 1);
 #pragma unroll
-                    for (int j = 0; j < C::ACC; ++j, y += a.ldy) {
-                        const float up = __shfl_xor_sync(0xffffffffu, acc[j], 1);
-                        if (mine && j < cols) *y = silu_f(acc[j]) * up;
+                    for (int j = 0; j < C::ACC; j += 2, y += 2 * a.ldy) {
+                        const float other = __shfl_xor_sync(0xffffffffu, odd ? acc[j] : acc[j + 1], 1);
+                        const float v = silu_f(odd ? other : acc[j]) * (odd ? acc[j + 1] : other);
+                        if (n < a.N && j + odd < cols) *y = v;
                     }
                 } else if (n < a.N) {
                     float* y = a.y + (size_t)(m0 + col0) * a.ldy + n;
