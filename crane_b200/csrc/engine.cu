@@ -214,10 +214,10 @@ struct crane_b200_model {
     bf16* w3_buf = nullptr;                 // three bf16 planes of a group's activations, w3_plane elements apart
     size_t w3_plane = 0;
     unsigned char* xqd_buf = nullptr;       // ... quantised (qrows_at, wide_rows rows)
-    int wide_rows = 0, wide_xq_mode = -1;
+    int wide_rows = 0;
     float* am_val = nullptr; int* am_idx = nullptr;
     void linear_wide(int epi, const bf16* w, const unsigned char* qw, int qt, int N, int K, const float* xin, int ldx, const float* norm_w, float* y, int ldy,
-                     int B, bool same_input = false);
+                     int B);
     void enqueue_wide_step(int advance, int B);
     // ---- configuration ----
     int device = 0, num_sms = 148;
@@ -380,7 +380,7 @@ struct crane_b200_model {
     unsigned char* xq_buf = nullptr;   // activations quantised for the quantised GEMVs (xquant_launch)
     int xq_mode_last = -1;
     unsigned char* xqr_buf = nullptr;  // activation rows quantised for the tensor-core linears (qrows_at), xqr_rows of them
-    int xqr_rows = 0, xqr_mode_last = -1;
+    int xqr_rows = 0;
     // Split precision (default): every bf16 activation operand / KV page has a low-order plane (x = hi + lo) so the prefill
     // tensor-core path carries ~16 mantissa bits; lo_* = element offset of that plane from the buffer base, 0 when off.
     bool split = true;
@@ -432,16 +432,17 @@ struct crane_b200_model {
     void linear_decode(int epi, bool norm, const bf16* w, const unsigned char* qw, int qt, int N, int K, const float* xin, int ldx,
                        const float* norm_w, float* y, int ldy, const GemvArgs* extra = nullptr, int B = 1, bool same_input = false, const QMore& more = {});
     void qlinear_rows(int epi, const unsigned char* qw, int qt, int N, int K, const float* xin, int ldx, const float* norm_w, float* y, int ldy,
-                      int S, bool reuse_xq = false);
-    // q, k and v of a quantised layer: f(weight, type, rows, first column, further matrices, not the first).  As GEMVs neighbours of one type share a launch; on the
-    // tensor cores each has its own (dealt out along K together, their sums would be grouped otherwise).
-    template <typename F> void qkv_linears(const LayerW& l, bool gemv, F&& f) const {
+                      int S);
+    // q, k and v of a quantised layer on the tensor cores: one set of codes where their types share a block rule, launches shared where they fit the chip
+    void qkv_rows(const LayerW& l, unsigned char* buf, int cap, const float* xin, float* y, int S);
+    // ... as GEMVs, through f(weight, type, rows, first column, further matrices, not the first): neighbours of one type share a launch
+    template <typename F> void qkv_linears(const LayerW& l, F&& f) const {
         const int n[3] = {nh * q_stride(), nkv * D, nkv * D}, t[3] = {l.qt_q, l.qt_k, l.qt_v};
         const unsigned char* w[3] = {l.q_wq, l.q_wk, l.q_wv};
         for (int i = 0, col = 0; i < 3;) {
             QMore more;
             int j = i + 1, end = col + n[i];
-            for (; gemv && j < 3 && t[j] == t[i]; end += n[j++]) { more.w[j - i - 1] = w[j]; more.n[j - i - 1] = n[j]; }
+            for (; j < 3 && t[j] == t[i]; end += n[j++]) { more.w[j - i - 1] = w[j]; more.n[j - i - 1] = n[j]; }
             f(w[i], t[i], n[i], col, more, i > 0);
             col = end; i = j;
         }
@@ -1070,25 +1071,34 @@ void crane_b200_model::linear_decode(int epi, bool norm, const bf16* w, const un
 // Prefill through a quantised linear: candle's `QMatMul::forward` quantises every activation ROW to Q8_K / Q8_0 blocks and takes
 // ggml integer dots whatever the number of rows (crane-core/src/ops/linear.rs:23-48).  From qrows_min rows on the integer dots run on the
 // tensor cores (qgemm.cu); fewer rows go through the decode kernels, up to four per pass over the quantised weights.
-// `reuse_xq`: the rows were quantised by the previous call (same input, same norm) -- still checked against the block rule it used.
 void crane_b200_model::qlinear_rows(int epi, const unsigned char* qw, int qt, int N, int K, const float* xin, int ldx, const float* norm_w,
-                                    float* y, int ldy, int S, bool reuse_xq) {
+                                    float* y, int ldy, int S) {
     if (S >= qrows_min(qt)) {
         const int mode = xq_mode_for(qt);
         const QRows xr = qrows_at(xqr_buf, xqr_rows, K);
-        if (!reuse_xq || mode != xqr_mode_last) {
-            LAUNCH_OK(xquant_rows_launch(stream, S, xin, ldx, K, norm_w, eps, mode, xr, use_pdl));
-            xqr_mode_last = mode;
-            ++launches;
-        }
+        LAUNCH_OK(xquant_rows_launch(stream, S, xin, ldx, K, norm_w, eps, mode, xr, use_pdl));
         LAUNCH_OK(qgemm_launch(stream, qt, qw, xr, S, N, K, epi, y, ldy, use_pdl));
-        ++launches;
+        launches += 2;
         return;
     }
     for (int s0 = 0; s0 < S;) {
         const int B = (S - s0 >= 4) ? 4 : (S - s0 >= 2) ? 2 : 1;
-        linear_decode(epi, norm_w != nullptr, nullptr, qw, qt, N, K, xin + (size_t)s0 * ldx, ldx, norm_w, y + (size_t)s0 * ldy, ldy, nullptr, B, reuse_xq && S <= 4);
+        linear_decode(epi, norm_w != nullptr, nullptr, qw, qt, N, K, xin + (size_t)s0 * ldx, ldx, norm_w, y + (size_t)s0 * ldy, ldy, nullptr, B);
         s0 += B;
+    }
+}
+
+void crane_b200_model::qkv_rows(const LayerW& l, unsigned char* buf, int cap, const float* xin, float* y, int S) {
+    const QMany m[3] = {{l.qt_q, l.q_wq, nh * q_stride(), y, qkv_dim()}, {l.qt_k, l.q_wk, nkv * D, y + nh * q_stride(), qkv_dim()},
+                        {l.qt_v, l.q_wv, nkv * D, y + nh * q_stride() + nkv * D, qkv_dim()}};
+    const QRows xr = qrows_at(buf, cap, H);
+    for (int i = 0, j; i < 3; i = j) {
+        const int mode = xq_mode_for(m[i].qt);
+        for (j = i + 1; j < 3 && xq_mode_for(m[j].qt) == mode; ++j) {}
+        LAUNCH_OK(xquant_rows_launch(stream, S, xin, H, H, l.ln1, eps, mode, xr, use_pdl));
+        int n = 0;
+        LAUNCH_OK(qgemm_many_launch(stream, m + i, j - i, xr, S, H, use_pdl, &n));
+        launches += 1 + n;
     }
 }
 
@@ -1343,7 +1353,7 @@ void crane_b200_model::enqueue_decode_step(int advance, bool with_embed, int B) 
         LayerW& l = layers[li];
         if (l.full) {
             if (l.qt_q) {   // GGUF keeps q/k/v as separate quantised matrices (qwen3/modeling.rs:252-255): GEMVs into one qkv row
-                qkv_linears(l, true, [&](const unsigned char* w, int t, int n, int col, const QMore& more, bool again) {
+                qkv_linears(l, [&](const unsigned char* w, int t, int n, int col, const QMore& more, bool again) {
                     linear_decode(GEMV_STORE, true, nullptr, w, t, n, H, x_dec, H, l.ln1, qkv_dec + col, qkv_dim(), nullptr, B, again, more);
                 });
             } else {
@@ -1455,37 +1465,27 @@ int crane_b200_model::decode_group(size_t left) const {
 }
 
 // y = epi(W x) of a group's rows, f32 in and out: the rows as three bf16 planes (24 bits), or as Q8 codes in front of a quantised matrix.
-// `same_input`: the rows are as the previous call left them (same input and norm) -- still checked against the block rule it used.
 void crane_b200_model::linear_wide(int epi, const bf16* w, const unsigned char* qw, int qt, int N, int K, const float* xin, int ldx, const float* norm_w,
-                                   float* y, int ldy, int B, bool same_input) {
+                                   float* y, int ldy, int B) {
     if (qt) {
         const int mode = xq_mode_for(qt);
         const QRows xr = qrows_at(xqd_buf, wide_rows, K);
-        if (!same_input || mode != wide_xq_mode) {
-            LAUNCH_OK(xquant_rows_launch(stream, B, xin, ldx, K, norm_w, eps, mode, xr, use_pdl));
-            wide_xq_mode = mode;
-            ++launches;
-        }
+        LAUNCH_OK(xquant_rows_launch(stream, B, xin, ldx, K, norm_w, eps, mode, xr, use_pdl));
         LAUNCH_OK(qgemm_launch(stream, qt, qw, xr, B, N, K, epi, y, ldy, use_pdl));
     } else {
-        if (!same_input) {
-            LAUNCH_OK(rows_split3_launch(stream, xin, ldx, B, K, norm_w, eps, w3_buf, (long long)w3_plane, use_pdl));
-            ++launches;
-        }
+        LAUNCH_OK(rows_split3_launch(stream, xin, ldx, B, K, norm_w, eps, w3_buf, (long long)w3_plane, use_pdl));
         const bf16* planes[3] = {w3_buf, w3_buf + w3_plane, w3_buf + 2 * w3_plane};
         GemmEpi ep{y, nullptr, ldy, nullptr, epi == GEMV_RESID ? EPI_RESID_F32 : epi == GEMV_SILU_MUL ? EPI_SILU_MUL_F32 : EPI_STORE_F32};
         LAUNCH_OK(gemm_rows_launch(stream, planes, 3, K, w, B, N, K, ep, use_pdl));
     }
-    ++launches;
+    launches += 2;
 }
 
 void crane_b200_model::enqueue_wide_step(int advance, int B) {
     for (int li = 0; li < L; ++li) {
         LayerW& l = layers[li];
         if (l.qt_q) {
-            qkv_linears(l, false, [&](const unsigned char* w, int t, int n, int col, const QMore&, bool again) {
-                linear_wide(GEMV_STORE, nullptr, w, t, n, H, x_dec, H, l.ln1, qkv_dec + col, qkv_dim(), B, again);
-            });
+            qkv_rows(l, xqd_buf, wide_rows, x_dec, qkv_dec, B);
         } else {
             linear_wide(GEMV_STORE, l.wqkv, nullptr, 0, qkv_dim(), H, x_dec, H, l.ln1, qkv_dec, qkv_dim(), B);
         }
@@ -1681,13 +1681,13 @@ void crane_b200_model::prefill(const uint32_t* ids, const float* embeds, size_t 
             spans.mark(SP_ATTN_QKV);
             if (q_qkv) {   // GGUF keeps q / k / v separate and quantised (qwen3/modeling.rs:252-255): integer dots
                 const bool all = S >= std::max(qrows_min(l.qt_q), std::max(qrows_min(l.qt_k), qrows_min(l.qt_v)));
-                for (int s0 = 0; s0 < S;) {               // (a few rows: groups of up to four)
-                    const int left = S - s0, B = all ? left : left >= 4 ? 4 : left >= 2 ? 2 : 1;
+                if (all) qkv_rows(l, xqr_buf, xqr_rows, x, qkv, S);
+                for (int s0 = 0; s0 < S && !all;) {       // (a few rows: groups of up to four)
+                    const int left = S - s0, B = left >= 4 ? 4 : left >= 2 ? 2 : 1;
                     const float* xr = x + (size_t)s0 * H;
                     float* yr = qkv + (size_t)s0 * qkv_dim();
-                    qkv_linears(l, !all, [&](const unsigned char* w, int t, int n, int col, const QMore& more, bool again) {
-                        if (all) qlinear_rows(GEMV_STORE, w, t, n, H, xr, H, l.ln1, yr + col, qkv_dim(), B, again);
-                        else linear_decode(GEMV_STORE, true, nullptr, w, t, n, H, xr, H, l.ln1, yr + col, qkv_dim(), nullptr, B, again, more);
+                    qkv_linears(l, [&](const unsigned char* w, int t, int n, int col, const QMore& more, bool again) {
+                        linear_decode(GEMV_STORE, true, nullptr, w, t, n, H, xr, H, l.ln1, yr + col, qkv_dim(), nullptr, B, again, more);
                     });
                     s0 += B;
                 }

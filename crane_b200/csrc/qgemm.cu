@@ -11,7 +11,7 @@
 //   Q8_0  A = q, one accumulator per 32-element block (both sides have a scale per 32)
 // and the block scales are applied in f32 when the accumulator is read, once per block: acc += (d_w D - dmin_w D2) d_x.
 //
-// The weight rows are the MMA's M = 128 rows and the activation rows its N (NT = 16 .. 64), so a decode batch pays for the columns it has.
+// The weight rows are the MMA's M = 128 rows and the activation rows its N (16 .. 64), so a decode batch pays for the columns it has.
 //
 // The unpacked weights go from registers to TMEM, the MMA's A operand there: 128 f16 columns of a super-block are 128 lanes x 64 columns, a lane's row being the row that
 // its thread unpacks.  Through shared memory (an f16 tile written by the unpacking warps, a proxy fence, read back by the MMAs) a super-block of 128 x 64 cost
@@ -33,10 +33,11 @@
 namespace cb {
 
 constexpr int QT_MAX_CTAS = 160;
-constexpr int DEQ_WARPS = 8;
 
-template <int QT, int NT>
+// TM activation rows per tile.  128 (K-quants): two MMAs' halves of 64 rows, each with one of the two sets of accumulators, so that the weights are unpacked once for both.
+template <int QT, int TM>
 struct QCfg {
+    static constexpr int NH = TM > 64 ? 2 : 1, NT = TM / NH;    // halves, columns per MMA
     static constexpr int SB = QT == QT_Q4_K ? 144 : QT == QT_Q6_K ? 224 : 272;
     static constexpr int PLANES = QT == QT_Q6_K ? 2 : 1;
     static constexpr int GROUPS = QT == QT_Q8_0 ? 8 : 1;        // accumulators per super-block
@@ -45,19 +46,22 @@ struct QCfg {
     static constexpr int D_COLS = (MINS ? 2 : DG) * NT;         // TMEM: two such sets,
     static constexpr int UPS = QT == QT_Q6_K ? 2 : 1;           // then units of unpacked weights, this many to a super-block
     static constexpr int U_COLS = 128 * PLANES / UPS, NU = (512 - 2 * D_COLS) / U_COLS > 3 ? 3 : (512 - 2 * D_COLS) / U_COLS;
-    static constexpr int RAW_BYTES = 128 * SB, RAW_REGS = QT == QT_Q4_K ? 5 : QT == QT_Q6_K ? 6 : 8;      // (16-byte pieces a thread reads per unit)
-    static constexpr int NR = QT == QT_Q4_K ? (NT > 32 ? 5 : NT > 16 ? 6 : 8) : QT == QT_Q6_K ? (NT > 32 ? 5 : 6) : (NT > 32 ? 3 : 4);
-    static constexpr int NB = QT == QT_Q6_K || NT < 64 ? 4 : 3;  // ring of codes, one unit each
+    static constexpr int DEQ_WARPS = 8, PARTS = DEQ_WARPS / 4, RR = 4 / PARTS;      // warps that unpack; a warp's share of a super-block: RR x 64 elements
+    static constexpr int RAW_BYTES = 128 * SB, RAW_REGS = QT == QT_Q4_K ? 1 + 2 * RR : QT == QT_Q6_K ? 2 + 2 * RR : 4 * RR;      // (16-byte pieces a thread reads per unit)
+    static constexpr int NR = QT == QT_Q4_K ? (TM > 64 ? 3 : TM > 32 ? 5 : TM > 16 ? 6 : 8) : QT == QT_Q6_K ? (TM > 32 ? 5 : 6) : (TM > 32 ? 3 : 4);
+    static constexpr int NB = QT == QT_Q6_K || TM != 64 ? 4 : 3;  // ring of codes: one unit of NT rows each
     static constexpr int B2_BYTES = MINS ? NT * 32 : 0, B_BYTES = NT * 512 / UPS, STG_BYTES = B_BYTES + B2_BYTES;
     static constexpr int A2_BYTES = MINS ? 128 * 32 : 0;        // [NU]
     // rings of scales, in super-blocks.  Who writes the scales of `it` has seen the MMAs of an older one done, so the accumulators two hand-overs before that have
     // been read.  Weights: in Q4_K it - NU (NU + 2 places); in Q6_K, written a unit ahead, the first half of it - 2 (4); in Q8_0, a super-block ahead, it - 3, of
-    // which at 16 rows only the super-block before it - 3 is known to have been read (NU + 3).  Activations: it - NB.
-    static constexpr int NS = (QT == QT_Q4_K && NU > 2) || (QT == QT_Q8_0 && NT == 16) ? 8 : 4, ND = NB + 2;
+    // which at 16 rows only the super-block before it - 3 is known to have been read (NU + 3).  Activations: it - NB / NH or it - NB / UPS.
+    static constexpr int NS = (QT == QT_Q4_K && NU > 2) || (QT == QT_Q8_0 && TM == 16) ? 8 : 4, ND = NB + 2;
     static constexpr int SCW_BYTES = GROUPS * 128 * (MINS ? 8 : 4);
-    static constexpr int DX_BYTES = GROUPS * NT * 4;
-    static constexpr int EPI_WARPS = NT > 32 ? 8 : 4;
-    static constexpr int ACC = NT / (EPI_WARPS / 4);            // columns per epilogue thread
+    static constexpr int DX_BYTES = GROUPS * TM * 4;
+    static constexpr int EPI_WARPS = TM > 16 ? 8 : 4;          // (a division of the gated unit takes a lane 160 cycles, and nothing overlaps it: the columns are spread)
+    static constexpr int ACC = TM / (EPI_WARPS / 4);            // columns per epilogue thread
+    static constexpr int CH = ACC > 32 ? 8 : 16;                // ... read at once
+    static constexpr int GATHER = TM > 64 ? 1 : TM > 32 ? 2 : TM > 16 ? 3 : 4;      // parts of a shared tile on their way at once, 16 columns each
     static constexpr int THREADS = (EPI_WARPS + DEQ_WARPS + 3) * 32;
     // offsets from a 1024-byte boundary; the swizzled tiles first
     static constexpr int STG_PITCH = (STG_BYTES + 1023) / 1024 * 1024;
@@ -65,6 +69,7 @@ struct QCfg {
                          OFF_BAR = OFF_DX + ND * DX_BYTES, SMEM = OFF_BAR + 512 + 1024;
     static_assert(SMEM <= 227 * 1024, "rings do not fit");
     static_assert(NU >= 2 && 2 * D_COLS + NU * U_COLS <= 512, "TMEM");
+    static_assert(NH == 1 || QT != QT_Q8_0, "two halves share the two sets");
     static_assert(OFF_A2 % 1024 == 0 && OFF_RAW % 128 == 0 && OFF_DX % 16 == 0 && OFF_BAR % 8 == 0, "alignment");
 };
 
@@ -124,10 +129,11 @@ __device__ __forceinline__ void f2_split(uint64_t v, float& a, float& b) { asm("
 __device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) { uint64_t r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
 __device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) { uint64_t r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
 
-template <int QT, int NT>
-__global__ void __launch_bounds__(QCfg<QT, NT>::THREADS, 1)
-qgemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmS, QGemmArgs a) {
-    using C = QCfg<QT, NT>;
+// One CTA's share (`cta` of a.sc.G) of one linear
+template <int QT, int TM>
+__device__ __forceinline__ void qgemm_body(const CUtensorMap& tmW, const CUtensorMap& tmX, const CUtensorMap& tmS, const QGemmArgs& a, const int cta) {
+    using C = QCfg<QT, TM>;
+    constexpr int NT = C::NT, NH = C::NH;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint64_t* bars = reinterpret_cast<uint64_t*>(sm + C::OFF_BAR);
@@ -140,16 +146,16 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
     const TcWait wait{gave_up, a.err};
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    constexpr int W_DEQ = C::EPI_WARPS, W_TMA = W_DEQ + DEQ_WARPS, W_MMA = W_TMA + 1, W_RAW = W_MMA + 1;
-    const int KB = a.sc.KB, it_begin = sched_start(a.sc, blockIdx.x), it_end = sched_start(a.sc, blockIdx.x + 1);
+    constexpr int W_DEQ = C::EPI_WARPS, W_TMA = W_DEQ + C::DEQ_WARPS, W_MMA = W_TMA + 1, W_RAW = W_MMA + 1;
+    const int KB = a.sc.KB, it_begin = sched_start(a.sc, cta), it_end = sched_start(a.sc, cta + 1);
 
     if (threadIdx.x == 0) {
         *gave_up = 0;
-        for (int i = 0; i < C::NR; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], DEQ_WARPS); }
-        for (int i = 0; i < C::NU; ++i) { mbar_init(&a_full[i], DEQ_WARPS); mbar_init(&a_empty[i], 1); }
+        for (int i = 0; i < C::NR; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], C::DEQ_WARPS); }
+        for (int i = 0; i < C::NU; ++i) { mbar_init(&a_full[i], C::DEQ_WARPS); mbar_init(&a_empty[i], 1); }
         for (int i = 0; i < C::NB; ++i) { mbar_init(&b_full[i], 1); mbar_init(&b_empty[i], 1); }
         for (int i = 0; i < C::ND; ++i) mbar_init(&dx_full[i], 1);
-        for (int i = 0; i < 2; ++i) { mbar_init(&d_full[i], 1); mbar_init(&d_empty[i], C::EPI_WARPS); }
+        for (int i = 0; i < 2; ++i) { mbar_init(&d_full[i], 1); mbar_init(&d_empty[i], C::EPI_WARPS / NH); }
         fence_barrier_init();
     }
     if (warp == W_MMA) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
@@ -178,26 +184,27 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
         if (lane == 0) {
             tma_prefetch_desc(&tmX);
             pdl_wait();
-            int st = 0, ds = 0, kb = it_begin % KB, tile = it_begin / KB, m0 = tile % a.sc.tiles_m * NT; uint32_t ph = 0;
+            int st = 0, ds = 0, kb = it_begin % KB, tile = it_begin / KB, m0 = tile % a.sc.tiles_m * TM; uint32_t ph = 0;
             for (int it = it_begin; it < it_end; ++it) {
 #pragma unroll 1
-                for (int g = 0; g < C::UPS; ++g) {
+                for (int g = 0; g < C::UPS * NH; ++g) {       // units, and the halves of each
+                    const int n = g / NH, m = m0 + g % NH * NT;
                     wait(&b_empty[st], ph ^ 1);
                     if (g == 0) {
                         mbar_arrive_expect_tx(&dx_full[ds], C::DX_BYTES);
 #pragma unroll
                         for (int q = 0; q < C::GROUPS; ++q)
-                            bulk_load(sm + C::OFF_DX + ds * C::DX_BYTES + q * NT * 4, a.dx + (size_t)(kb * C::GROUPS + q) * a.ldd + m0, NT * 4, &dx_full[ds]);
+                            bulk_load(sm + C::OFF_DX + ds * C::DX_BYTES + q * TM * 4, a.dx + (size_t)(kb * C::GROUPS + q) * a.ldd + m0, TM * 4, &dx_full[ds]);
                         if (++ds == C::ND) ds = 0;
                     }
                     mbar_arrive_expect_tx(&b_full[st], C::STG_BYTES);
                     uint8_t* dst = sm + st * C::STG_PITCH;
 #pragma unroll
-                    for (int c = 0; c < 4 / C::UPS; ++c) tma_load_2d(dst + c * NT * 128, &tmX, &b_full[st], kb * 256 + (g * (4 / C::UPS) + c) * 64, m0);
-                    if (C::MINS) tma_load_2d(dst + C::B_BYTES, &tmS, &b_full[st], kb * 16, m0);
+                    for (int c = 0; c < 4 / C::UPS; ++c) tma_load_2d(dst + c * NT * 128, &tmX, &b_full[st], kb * 256 + (n * (4 / C::UPS) + c) * 64, m);
+                    if (C::MINS) tma_load_2d(dst + C::B_BYTES, &tmS, &b_full[st], kb * 16, m);
                     if (++st == C::NB) { st = 0; ph ^= 1; }
                 }
-                if (++kb == KB) { kb = 0; ++tile; m0 = tile % a.sc.tiles_m * NT; }
+                if (++kb == KB) { kb = 0; ++tile; m0 = tile % a.sc.tiles_m * TM; }
             }
             wait.drain();
         }
@@ -208,14 +215,11 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
         for (int it = it_begin; it < it_end; ++it) {
 #pragma unroll 1
             for (int g = 0; g < C::UPS; ++g) {
-                if (QT != QT_Q8_0 && g == 0) wait(&d_empty[ds], dph ^ 1);
-                wait(&b_full[st], ph);
-                wait(&a_full[us], uph);
-                tc_fence_after();
                 const uint32_t ta = tmem + (uint32_t)(2 * C::D_COLS + us * C::U_COLS);
-                const uint32_t bb = smem_u32(sm + st * C::STG_PITCH);
-                const uint64_t bd = make_smem_desc_sw128(bb);
                 if constexpr (QT == QT_Q8_0) {
+                    wait(&b_full[st], ph);
+                    wait(&a_full[us], uph);
+                    const uint64_t bd = make_smem_desc_sw128(smem_u32(sm + st * C::STG_PITCH));
 #pragma unroll
                     for (int s = 0; s < C::GROUPS / C::DG; ++s) {
                         wait(&d_empty[ds], dph ^ 1);
@@ -233,33 +237,47 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
                         __syncwarp();
                         if (++ds == 2) { ds = 0; dph ^= 1; }
                     }
+                    if (++st == C::NB) { st = 0; ph ^= 1; }
                 } else {
-                    const uint32_t d = tmem + (uint32_t)(ds * C::D_COLS), acc0 = (uint32_t)(g != 0);
-                    if (elect_one()) {
+#pragma unroll 1
+                    for (int h = 0; h < NH; ++h) {
+                        if (g == 0) wait(&d_empty[ds], dph ^ 1);
+                        wait(&b_full[st], ph);
+                        if (h == 0) wait(&a_full[us], uph);
+                        tc_fence_after();
+                        const uint32_t bb = smem_u32(sm + st * C::STG_PITCH);
+                        const uint64_t bd = make_smem_desc_sw128(bb);
+                        const uint32_t d = tmem + (uint32_t)(ds * C::D_COLS), acc0 = (uint32_t)(g != 0);
+                        if (elect_one()) {
 #pragma unroll
-                        for (int k = 0; k < 16 / C::UPS; ++k) {
-                            const uint64_t bw = bd + (uint64_t)((k >> 2) * NT * 8 + 2 * (k & 3));
-                            umma_ts(d, ta + 8 * k, bw, idesc, k == 0 ? acc0 : 1u);
-                            if (C::PLANES == 2) umma_ts(d, ta + C::U_COLS / 2 + 8 * k, bw, idesc, 1u);
+                            for (int k = 0; k < 16 / C::UPS; ++k) {
+                                const uint64_t bw = bd + (uint64_t)((k >> 2) * NT * 8 + 2 * (k & 3));
+                                umma_ts(d, ta + 8 * k, bw, idesc, k == 0 ? acc0 : 1u);
+                                if (C::PLANES == 2) umma_ts(d, ta + C::U_COLS / 2 + 8 * k, bw, idesc, 1u);
+                            }
+                            if (C::MINS)
+                                umma_bf16(d + NT, make_smem_desc_sw32(smem_u32(sm + C::OFF_A2 + us * C::A2_BYTES)), make_smem_desc_sw32(bb + C::B_BYTES), idesc, 0u);
+                            if (h == NH - 1) umma_commit(&a_empty[us]);
+                            umma_commit(&b_empty[st]);
+                            if (g == C::UPS - 1) umma_commit(&d_full[ds]);
                         }
-                        if (C::MINS)
-                            umma_bf16(d + NT, make_smem_desc_sw32(smem_u32(sm + C::OFF_A2 + us * C::A2_BYTES)), make_smem_desc_sw32(bb + C::B_BYTES), idesc, 0u);
-                        umma_commit(&a_empty[us]);
-                        umma_commit(&b_empty[st]);
-                        if (g == C::UPS - 1) umma_commit(&d_full[ds]);
+                        __syncwarp();
+                        // one half: the sets take turns by super-block; two: each has its own
+                        if (NH == 1) { if (g == C::UPS - 1 && ++ds == 2) { ds = 0; dph ^= 1; } }
+                        else if (++ds == 2) { ds = 0; if (g == C::UPS - 1) dph ^= 1; }
+                        if (++st == C::NB) { st = 0; ph ^= 1; }
                     }
-                    __syncwarp();
-                    if (g == C::UPS - 1 && ++ds == 2) { ds = 0; dph ^= 1; }
                 }
-                if (++st == C::NB) { st = 0; ph ^= 1; }
                 if (++us == C::NU) { us = 0; uph ^= 1; }
             }
         }
     // ------------------------------------------------------------------------------------------------ weights: blocks -> f16 integers
     } else if (warp >= W_DEQ) {
-        // A lane has a row, the two warps of its 32 rows a half of every super-block each (Q6_K: of every unit).  The raw bytes of the next unit are read into
+        // A lane has a row, the PARTS warps of its 32 rows a part of every super-block each (Q6_K: of every unit).  The raw bytes of the next unit are read into
         // registers before this one's stores are waited for, so that only the instructions stand between two units.
-        const int dw = warp - W_DEQ, half = dw >> 2, row = (dw & 3) * 32 + lane;
+        const int dw = warp - W_DEQ, part = dw >> 2, row = (dw & 3) * 32 + lane;
+        const int half = part & 1, q_first = C::PARTS == 4 ? part >> 1 : 0;      // Q6_K: nibbles, and the first of a unit's two quarters
+        constexpr int RR = C::RR;
         const uint32_t lanes = (uint32_t)((dw & 3) * 32) << 16;
         const int units = (it_end - it_begin) * C::UPS;
         int rs = 0, us = 0; uint32_t rph = 0, uph = 0;
@@ -272,23 +290,26 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
             if constexpr (QT == QT_Q4_K) {
                 raw[0] = *reinterpret_cast<const uint4*>(sb);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) raw[1 + j] = *reinterpret_cast<const uint4*>(sb + 16 + 64 * half + 16 * j);
-            } else if constexpr (QT == QT_Q6_K) {       // elements 128 n + 64 half ..: half n of the block, low or high nibbles
+                for (int j = 0; j < 2 * RR; ++j) raw[1 + j] = *reinterpret_cast<const uint4*>(sb + 16 + 32 * RR * part + 16 * j);
+            } else if constexpr (QT == QT_Q6_K) {       // half n of the block
 #pragma unroll
                 for (int e = 0; e < 2; ++e) raw[e] = *reinterpret_cast<const uint4*>(sb + 128 + 32 * n + 16 * e);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) raw[2 + j] = *reinterpret_cast<const uint4*>(sb + 64 * n + 16 * j);
-                raw1 = *reinterpret_cast<const uint32_t*>(sb + 192 + 8 * n + 4 * half);       // scales: byte 2 * quarter + (element / 16)
-                if (n == 0 && half == 0)
+                for (int j = 0; j < 2 * RR; ++j) raw[2 + j] = *reinterpret_cast<const uint4*>(sb + 64 * n + 32 * q_first + 16 * j);
+                raw1 = *reinterpret_cast<const uint32_t*>(sb + 192 + 8 * n + 4 * half) >> (16 * q_first);       // scales: byte 2 * quarter + (element / 16)
+                if (n == 0 && part == 0)
                     reinterpret_cast<float*>(sm + C::OFF_SCW + ((it_begin + u / C::UPS) & (C::NS - 1)) * C::SCW_BYTES)[row] =
                         4.f * __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short*>(sb + 208)));
             } else {
 #pragma unroll
-                for (int j = 0; j < 8; ++j) raw[j] = *reinterpret_cast<const uint4*>(sb + 128 * half + 16 * j);
-                const uint2 d = *reinterpret_cast<const uint2*>(sb + 256 + 8 * half);
-                float* scw = reinterpret_cast<float*>(sm + C::OFF_SCW + ((it_begin + u) & (C::NS - 1)) * C::SCW_BYTES) + (4 * half) * 128 + row;
-                scw[0] = __half2float(__ushort_as_half((unsigned short)(d.x & 0xffffu))); scw[128] = __half2float(__ushort_as_half((unsigned short)(d.x >> 16)));
-                scw[256] = __half2float(__ushort_as_half((unsigned short)(d.y & 0xffffu))); scw[384] = __half2float(__ushort_as_half((unsigned short)(d.y >> 16)));
+                for (int j = 0; j < 4 * RR; ++j) raw[j] = *reinterpret_cast<const uint4*>(sb + 64 * RR * part + 16 * j);
+                float* scw = reinterpret_cast<float*>(sm + C::OFF_SCW + ((it_begin + u) & (C::NS - 1)) * C::SCW_BYTES) + (2 * RR * part) * 128 + row;
+#pragma unroll
+                for (int rr = 0; rr < RR; ++rr) {
+                    const uint32_t d = *reinterpret_cast<const uint32_t*>(sb + 256 + 4 * (RR * part + rr));
+                    scw[256 * rr] = __half2float(__ushort_as_half((unsigned short)(d & 0xffffu)));
+                    scw[256 * rr + 128] = __half2float(__ushort_as_half((unsigned short)(d >> 16)));
+                }
             }
             if (n == C::UPS - 1) {
                 __syncwarp();
@@ -299,15 +320,15 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
         if (units > 0) fetch(0);
         for (int u = 0; u < units; ++u) {
             const uint32_t ta = tmem + lanes + (uint32_t)(2 * C::D_COLS + us * C::U_COLS);
-            const bool more = u + 1 < units;
+            wait(&a_empty[us], uph ^ 1);
+            tc_fence_after();
             if constexpr (QT == QT_Q4_K) {
                 const uint4 hdr = raw[0];
-                wait(&a_empty[us], uph ^ 1);
-                tc_fence_after();
 #pragma unroll
-                for (int rr = 0; rr < 2; ++rr) {           // 64 elements: sub-blocks 4 half + 2 rr (low nibbles) and the one behind it (high); ggml get_scale_min_k4
-                    const uint32_t y = hdr.y >> (16 * rr), z = hdr.w >> (16 * rr);
-                    const uint32_t sa = half == 0 ? y & 63 : (z & 0xF) | (((y >> 6) & 3) << 4), sb2 = half == 0 ? (y >> 8) & 63 : ((z >> 8) & 0xF) | (((y >> 14) & 3) << 4);
+                for (int rr = 0; rr < RR; ++rr) {          // 64 elements: sub-blocks 2 g (low nibbles) and 2 g + 1 (high); ggml get_scale_min_k4
+                    const int g = RR * part + rr;
+                    const uint32_t y = hdr.y >> (16 * (g & 1)), z = hdr.w >> (16 * (g & 1));
+                    const uint32_t sa = g < 2 ? y & 63 : (z & 0xF) | (((y >> 6) & 3) << 4), sb2 = g < 2 ? (y >> 8) & 63 : ((z >> 8) & 0xF) | (((y >> 14) & 3) << 4);
                     const uint32_t s_lo = h2_int(sa), o_lo = h2_mul(s_lo, h2_const(0xE400)), t = h2_int(sb2), s_hi = h2_mul(t, h2_const(0x2C00)), o_hi = h2_mul(t, h2_const(0xD400));
                     const uint32_t ww[8] = {raw[1 + 2 * rr].x, raw[1 + 2 * rr].y, raw[1 + 2 * rr].z, raw[1 + 2 * rr].w, raw[2 + 2 * rr].x, raw[2 + 2 * rr].y, raw[2 + 2 * rr].z, raw[2 + 2 * rr].w};
                     uint32_t o[32];
@@ -319,9 +340,9 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
                         o[16 + 2 * i] = h2_fma((v & 0x00F000F0u) | 0x64006400u, s_hi, o_hi);
                         o[16 + 2 * i + 1] = h2_fma((v8 & 0x00F000F0u) | 0x64006400u, s_hi, o_hi);
                     }
-                    tmem_st32(ta + (uint32_t)(2 * half + rr) * 32, o);
+                    tmem_st32(ta + (uint32_t)g * 32, o);
                 }
-                if (half == 1) {                           // offsets m_0 .. m_7, 64 times them; d and dmin for the accumulators' readers
+                if (part == C::PARTS - 1) {                // offsets m_0 .. m_7, 64 times them; d and dmin for the accumulators' readers
                     uint32_t m[4], m64[4];
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
@@ -342,41 +363,35 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
                         make_float2(__half2float(__ushort_as_half((unsigned short)(hdr.x & 0xffffu))), __half2float(__ushort_as_half((unsigned short)(hdr.x >> 16))));
                     fence_proxy_async();                   // (the offsets' tile is in shared memory)
                 }
-                if (more) fetch(u + 1);
             } else if constexpr (QT == QT_Q6_K) {
                 // half = 0: low nibbles, quarters q1 | q2 of the block's half; 1: high nibbles, q3 | q4
                 const uint32_t lmul = half ? h2_const(0x2400) : h2_const(0x3400), lofs = half ? h2_const(0xCC00) : h2_const(0xDC00);    // 1/64, 1/4; -16, -256
                 const uint32_t lm = half ? 0x00F000F0u : 0x000F000Fu;
-                wait(&a_empty[us], uph ^ 1);
-                tc_fence_after();
 #pragma unroll
-                for (int q = 0; q < 2; ++q) {              // q: which of the two quarters, elements [32 q, 32 q + 32) of the 64
+                for (int r = 0; r < RR; ++r) {             // elements [32 q, 32 q + 32) of the 64
+                    const int q = q_first + r;
                     uint32_t lo[16], hi[16];
-                    // high plane: two bits at 2 q (after the shift by 4 half): (1024 + 4^q v - 1024 - 2 * 4^q) * 4 f / 4^q
-                    const uint32_t hm = q ? 0x000C000Cu : 0x00030003u, hsub = q ? h2_const(0xE408) : h2_const(0xE402);
 #pragma unroll
-                    for (int e = 0; e < 2; ++e) {          // e: elements [16 e, 16 e + 16) of a quarter
-                        const uint32_t f = h2_byte(raw1 >> (16 * q + 8 * e)), ls = h2_mul(f, lmul), lo_o = h2_mul(f, lofs), hs = q ? f : h2_mul(f, h2_const(0x4400));
-                        const uint32_t wl[4] = {raw[2 + 2 * q + e].x, raw[2 + 2 * q + e].y, raw[2 + 2 * q + e].z, raw[2 + 2 * q + e].w};
-                        const uint32_t wh[4] = {raw[e].x >> (4 * half), raw[e].y >> (4 * half), raw[e].z >> (4 * half), raw[e].w >> (4 * half)};
+                    for (int e = 0; e < 2; ++e) {          // e: elements [16 e, 16 e + 16) of a quarter; high plane: (1024 + v - 1024 - 2) * 4 f
+                        const uint32_t f = h2_byte(raw1 >> (16 * r + 8 * e)), ls = h2_mul(f, lmul), lo_o = h2_mul(f, lofs), hs = h2_mul(f, h2_const(0x4400));
+                        const uint32_t wl[4] = {raw[2 + 2 * r + e].x, raw[2 + 2 * r + e].y, raw[2 + 2 * r + e].z, raw[2 + 2 * r + e].w};
+                        const int sh = 4 * half + 2 * q;
+                        const uint32_t wh[4] = {raw[e].x >> sh, raw[e].y >> sh, raw[e].z >> sh, raw[e].w >> sh};
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
                             const uint32_t v = wl[i], v8 = v >> 8, w = wh[i], w8 = w >> 8;
                             lo[8 * e + 2 * i] = h2_fma((v & lm) | 0x64006400u, ls, lo_o);
                             lo[8 * e + 2 * i + 1] = h2_fma((v8 & lm) | 0x64006400u, ls, lo_o);
-                            hi[8 * e + 2 * i] = h2_mul(h2_add((w & hm) | 0x64006400u, hsub), hs);
-                            hi[8 * e + 2 * i + 1] = h2_mul(h2_add((w8 & hm) | 0x64006400u, hsub), hs);
+                            hi[8 * e + 2 * i] = h2_mul(h2_add((w & 0x00030003u) | 0x64006400u, h2_const(0xE402)), hs);
+                            hi[8 * e + 2 * i + 1] = h2_mul(h2_add((w8 & 0x00030003u) | 0x64006400u, h2_const(0xE402)), hs);
                         }
                     }
                     tmem_st16(ta + (uint32_t)(32 * half + 16 * q), lo);
                     tmem_st16(ta + (uint32_t)(C::U_COLS / 2 + 32 * half + 16 * q), hi);
                 }
-                if (more) fetch(u + 1);
             } else {
-                wait(&a_empty[us], uph ^ 1);
-                tc_fence_after();
 #pragma unroll
-                for (int rr = 0; rr < 2; ++rr) {
+                for (int rr = 0; rr < RR; ++rr) {
                     uint32_t o[32];
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
@@ -388,10 +403,10 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
                             o[8 * c + 2 * i + 1] = h2_add(((ww[i] >> 8) & 0x00FF00FFu) | 0x64006400u, h2_const(0xE480));
                         }
                     }
-                    tmem_st32(ta + (uint32_t)(2 * half + rr) * 32, o);
+                    tmem_st32(ta + (uint32_t)(RR * part + rr) * 32, o);
                 }
-                if (more) fetch(u + 1);
             }
+            if (u + 1 < units) fetch(u + 1);
             tmem_st_wait();
             tc_fence_before();
             __syncwarp();
@@ -402,12 +417,11 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
     } else {
         pdl_wait();
         const int q = warp & 3, col0 = (warp >> 2) * C::ACC, row = q * 32 + lane;
-        constexpr size_t TILE_F = (size_t)128 * NT;
-        constexpr int CH = 16;                                      // columns per read
-        int ds = 0, xs = 0; uint32_t dph = 0, xph = 0;
+        constexpr size_t TILE_F = (size_t)128 * TM;
+        int ds = NH == 2 ? warp >> 2 : 0, xs = 0; uint32_t dph = 0, xph = 0;
         for (int it = it_begin; it < it_end;) {
             const int seg_end = min(it_end, (it / KB + 1) * KB), t = it / KB;
-            const int n0 = (t / a.sc.tiles_m) * 128, m0 = (t % a.sc.tiles_m) * NT;
+            const int n0 = (t / a.sc.tiles_m) * 128, m0 = (t % a.sc.tiles_m) * TM;
             const bool sole = it % KB == 0 && seg_end - it == KB, head = it == it_begin;
             float acc[C::ACC];
 #pragma unroll
@@ -422,16 +436,16 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
                     float dw, dm = 0.f;
                     if constexpr (C::MINS) { const float2 s = reinterpret_cast<const float2*>(scw)[row]; dw = s.x; dm = s.y; }
                     else dw = reinterpret_cast<const float*>(scw)[g * 128 + row];
-                    const uint32_t d = tmem + (uint32_t)(ds * C::D_COLS + (g % C::DG) * NT + col0) + ((uint32_t)(q * 32) << 16);
+                    const uint32_t d = tmem + (uint32_t)(ds * C::D_COLS + (g % C::DG) * NT + (NH == 2 ? 0 : col0)) + ((uint32_t)(q * 32) << 16);
 #pragma unroll
-                    for (int c = 0; c < C::ACC; c += CH) {
-                        uint32_t r[CH], s[CH];
-                        tmem_ld16_async(d + c, r);
-                        if (C::MINS) tmem_ld16_async(d + NT + c, s);
+                    for (int c = 0; c < C::ACC; c += C::CH) {
+                        uint32_t r[C::CH], s[C::CH];
+                        if constexpr (C::CH == 16) { tmem_ld16_async(d + c, r); if (C::MINS) tmem_ld16_async(d + NT + c, s); }
+                        else { tmem_ld8_async(d + c, r); if (C::MINS) tmem_ld8_async(d + NT + c, s); }
                         tmem_ld_wait();
 #pragma unroll
-                        for (int j = 0; j < CH; j += 4) {
-                            const float4 x = *reinterpret_cast<const float4*>(dx + g * NT + c + j);
+                        for (int j = 0; j < C::CH; j += 4) {
+                            const float4 x = *reinterpret_cast<const float4*>(dx + g * TM + c + j);
                             const float xv[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
                             for (int e = 0; e < 4; e += 2) {         // two columns an instruction, each rounded as by itself
@@ -445,14 +459,15 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
                         tc_fence_before();
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&d_empty[ds]);
-                        if (++ds == 2) { ds = 0; dph ^= 1; }
+                        if (NH == 2) dph ^= 1;
+                        else if (++ds == 2) { ds = 0; dph ^= 1; }
                     }
                 }
                 if (++xs == C::ND) { xs = 0; xph ^= 1; }
             }
             bool finish = sole;
             if (!sole) {      // park the partial tile (column by column: a warp's store is 128 contiguous bytes); the last contributor adds them in order
-                float* mine = a.sc.ws + (size_t)(2 * blockIdx.x + (head ? 0 : 1)) * TILE_F + (size_t)col0 * 128 + row;
+                float* mine = a.sc.ws + (size_t)(2 * cta + (head ? 0 : 1)) * TILE_F + (size_t)col0 * 128 + row;
 #pragma unroll
                 for (int j = 0; j < C::ACC; ++j) mine[j * 128] = acc[j];
                 __threadfence();
@@ -463,19 +478,30 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
                 finish = *last_flag != 0;
                 if (finish) {
                     __threadfence();
-#pragma unroll
-                    for (int j = 0; j < C::ACC; ++j) acc[j] = 0.f;
-                    // a contributor's columns are on their way while the one's before it are added
                     auto part = [&](int cc) { return a.sc.ws + (size_t)(2 * cc + (sched_start(a.sc, cc) < t * KB ? 1 : 0)) * TILE_F + (size_t)col0 * 128 + row; };
-                    float x[C::ACC];
-                    const float* p = part(c_first);
 #pragma unroll
-                    for (int j = 0; j < C::ACC; ++j) x[j] = __ldcg(p + j * 128);
+                    for (int c = 0; c < C::ACC; c += 16) {
+                        float sum[16];
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) sum[j] = 0.f;
 #pragma unroll 1
-                    for (int cc = c_first; cc <= c_last; ++cc) {
-                        p = part(min(cc + 1, c_last));
+                        for (int cc = c_first; cc <= c_last; cc += C::GATHER) {
+                            float x[C::GATHER][16];
 #pragma unroll
-                        for (int j = 0; j < C::ACC; ++j) { acc[j] += x[j]; x[j] = __ldcg(p + j * 128); }
+                            for (int r = 0; r < C::GATHER; ++r) {
+                                const float* p = part(min(cc + r, c_last)) + c * 128;
+#pragma unroll
+                                for (int j = 0; j < 16; ++j) x[r][j] = __ldcg(p + j * 128);
+                            }
+#pragma unroll
+                            for (int r = 0; r < C::GATHER; ++r)
+                                if (cc + r <= c_last) {
+#pragma unroll
+                                    for (int j = 0; j < 16; ++j) sum[j] += x[r][j];
+                                }
+                        }
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) acc[c + j] = sum[j];
                     }
                     if (threadIdx.x == 0) a.sc.counters[t] = 0;
                 }
@@ -517,35 +543,87 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
     if (warp == W_MMA) { tc_fence_after(); tmem_dealloc(tmem, 512); }
 }
 
-template <int QT, int NT>
-static int qgemm_launch_t(cudaStream_t st, const unsigned char* w, const QRows& x, int M, int N, int K, int epi, float* y, int ldy, bool pdl) {
-    using C = QCfg<QT, NT>;
-    CUtensorMap tmW, tmX, tmS;
-    if (!tc_tmap_16(&tmW, w, (uint64_t)N, (uint64_t)K / 256 * (C::SB / 2), (uint64_t)K / 256 * (C::SB / 2), 128, C::SB / 2, CU_TENSOR_MAP_SWIZZLE_NONE)) return -1001;
-    if (!tc_tmap_16(&tmX, x.codes, (uint64_t)M, (uint64_t)K, (uint64_t)K, NT, 64, CU_TENSOR_MAP_SWIZZLE_128B)) return -1001;
-    if (!tc_tmap_16(&tmS, x.bsum, (uint64_t)M, (uint64_t)K / 16, (uint64_t)K / 16, NT, 16, CU_TENSOR_MAP_SWIZZLE_32B)) return -1001;
-    static SmemOptIn seen;
-    if (const int e = ensure_dyn_smem(qgemm_kernel<QT, NT>, (size_t)C::SMEM, seen)) return e;
-    QGemmArgs a = {};
+template <int QT, int TM>
+__global__ void __launch_bounds__(QCfg<QT, TM>::THREADS, 1)
+qgemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmS, const __grid_constant__ QGemmArgs a) {
+    qgemm_body<QT, TM>(tmW, tmX, tmS, a, blockIdx.x);
+}
+
+// Linears of the same rows side by side, each dealt out over its own CTAs as by itself: at width 4096 k and v of 32 rows are 64 CTAs each, 21 us one behind the other and 16
+// together; at width 1024 q, k and v are one launch.
+struct QJob { CUtensorMap w, x, s; QGemmArgs a; int qt, cta0; };
+struct QJobs { QJob j[3]; int n; };
+template <int TM>
+__global__ void __launch_bounds__(QCfg<QT_Q4_K, TM>::THREADS, 1)
+qgemm_jobs_kernel(const __grid_constant__ QJobs jobs) {
+    int i = jobs.n - 1;
+    while (i > 0 && (int)blockIdx.x < jobs.j[i].cta0) --i;
+    const QJob& j = jobs.j[i];
+    const int cta = blockIdx.x - j.cta0;
+    if (j.qt == QT_Q4_K) qgemm_body<QT_Q4_K, TM>(j.w, j.x, j.s, j.a, cta);
+    else if (j.qt == QT_Q6_K) qgemm_body<QT_Q6_K, TM>(j.w, j.x, j.s, j.a, cta);
+    else qgemm_body<QT_Q8_0, TM>(j.w, j.x, j.s, j.a, cta);
+}
+
+// maps, arguments and division of work of one linear; workspace and counters come later
+static int q_prepare(int qt, int TM, const unsigned char* w, const QRows& x, int M, int N, int K, int epi, float* y, int ldy, QJob* out) {
+    const int half = q_sb_bytes(qt) / 2, NT = std::min(TM, 64);
+    if (!tc_tmap_16(&out->w, w, (uint64_t)N, (uint64_t)K / 256 * half, (uint64_t)K / 256 * half, 128, half, CU_TENSOR_MAP_SWIZZLE_NONE)) return -1001;
+    if (!tc_tmap_16(&out->x, x.codes, (uint64_t)M, (uint64_t)K, (uint64_t)K, NT, 64, CU_TENSOR_MAP_SWIZZLE_128B)) return -1001;
+    if (!tc_tmap_16(&out->s, x.bsum, (uint64_t)M, (uint64_t)K / 16, (uint64_t)K / 16, NT, 16, CU_TENSOR_MAP_SWIZZLE_32B)) return -1001;
+    QGemmArgs& a = out->a;
+    a = {};
     a.M = M; a.N = N; a.K = K; a.epi = epi; a.y = y; a.ldy = ldy; a.dx = x.dx; a.ldd = x.ldd;
     TcSched& sc = a.sc;
-    sc.tiles_m = (M + NT - 1) / NT; sc.tiles_n = (N + 127) / 128; sc.KB = K / 256;
+    sc.tiles_m = (M + TM - 1) / TM; sc.tiles_n = (N + 127) / 128; sc.KB = K / 256;
     const long long tiles = (long long)sc.tiles_m * sc.tiles_n, iters = tiles * sc.KB;
     if (iters > 0x7fffffffLL) return -1000;
     sc.unit = 1;
     sc.G = (int)std::max<long long>(1, std::min<long long>(std::min(tc_device_sms(), QT_MAX_CTAS), iters / 2));     // two super-blocks pay for a CTA's setup
     sc.base = (int)(iters / sc.G); sc.rem = (int)(iters % sc.G);
+    out->qt = qt; out->cta0 = 0;
+    return 0;
+}
+
+template <int QT, int TM>
+static int qgemm_launch_t(cudaStream_t st, const unsigned char* w, const QRows& x, int M, int N, int K, int epi, float* y, int ldy, bool pdl) {
+    using C = QCfg<QT, TM>;
+    QJob j;
+    if (const int e = q_prepare(QT, TM, w, x, M, N, K, epi, y, ldy, &j)) return e;
+    static SmemOptIn seen;
+    if (const int e = ensure_dyn_smem(qgemm_kernel<QT, TM>, (size_t)C::SMEM, seen)) return e;
     TcScratch s;
-    if (const int e = tc_scratch_get(st, (int)tiles, &s)) return e;
-    sc.ws = s.ws; sc.counters = s.counters; a.err = s.err;
-    return launch_k(qgemm_kernel<QT, NT>, dim3(sc.G), dim3(C::THREADS), C::SMEM, st, pdl, tmW, tmX, tmS, a);
+    if (const int e = tc_scratch_get(st, j.a.sc.tiles_m * j.a.sc.tiles_n, &s)) return e;
+    j.a.sc.ws = s.ws; j.a.sc.counters = s.counters; j.a.err = s.err;
+    return launch_k(qgemm_kernel<QT, TM>, dim3(j.a.sc.G), dim3(C::THREADS), C::SMEM, st, pdl, j.w, j.x, j.s, j.a);
+}
+
+// Activation rows per tile.  Above 64, tiles of 64 or of 128 (K-quants), which unpack a block of weights half as often and read twice the accumulators behind one set of
+// MMAs.  Estimated us of either: super-blocks on the busiest CTA and a constant, fitted to launches behind one another in prompts of 65 .. 512 rows at widths
+// 1024, 2048 and 4096; 64 / 128 rows wide, where the wide form does better or nearly so:
+//   Q4_K  12288 x 2048  384 rows 43.1 / 43.2, 512 53.6 / 55.7     24576 x 4096  128 rows 52.1 / 52.2, 192 70.3 / 91.3, 256 92.2 / 87.1, 384 129 / 118, 512 169 / 155
+//   Q6_K  2048 x 6144   384 36.4 / 40.4, 512 46.1 / 49.3          4096 x 12288  192 65.1 / 76.3, 256 81.8 / 78.3, 384 115 / 101, 512 148 / 124
+static float qgemm_estimate(int qt, int TM, int M, int N, int K) {
+    const long long iters = (long long)((M + TM - 1) / TM) * ((N + 127) / 128) * (K / 256), G = std::max<long long>(1, std::min<long long>(tc_device_sms(), iters / 2));
+    const float most = (float)((iters + G - 1) / G);
+    if (qt == QT_Q4_K) return TM == 64 ? 1.0f * most + 9.f : 1.6f * most + 20.f;
+    return TM == 64 ? 1.57f * most + 16.f : 2.18f * most + 32.f;
+}
+static int qgemm_rows(int qt, int M, int N, int K) {
+    if (M <= 64) return M <= 16 ? 16 : M <= 32 ? 32 : 64;
+    return qt != QT_Q8_0 && qgemm_estimate(qt, 128, M, N, K) < qgemm_estimate(qt, 64, M, N, K) ? 128 : 64;
 }
 
 template <int QT>
 static int qgemm_launch_q(cudaStream_t st, const unsigned char* w, const QRows& x, int M, int N, int K, int epi, float* y, int ldy, bool pdl) {
-    if (M <= 16) return qgemm_launch_t<QT, 16>(st, w, x, M, N, K, epi, y, ldy, pdl);
-    if (M <= 32) return qgemm_launch_t<QT, 32>(st, w, x, M, N, K, epi, y, ldy, pdl);
-    return qgemm_launch_t<QT, 64>(st, w, x, M, N, K, epi, y, ldy, pdl);
+    switch (qgemm_rows(QT, M, N, K)) {
+        case 16: return qgemm_launch_t<QT, 16>(st, w, x, M, N, K, epi, y, ldy, pdl);
+        case 32: return qgemm_launch_t<QT, 32>(st, w, x, M, N, K, epi, y, ldy, pdl);
+        case 64: return qgemm_launch_t<QT, 64>(st, w, x, M, N, K, epi, y, ldy, pdl);
+        default:
+            if constexpr (QT != QT_Q8_0) return qgemm_launch_t<QT, 128>(st, w, x, M, N, K, epi, y, ldy, pdl);
+            return -1000;
+    }
 }
 
 int qgemm_launch(cudaStream_t st, int qt, const unsigned char* w, const QRows& x, int M, int N, int K, int epi, float* y, int ldy, bool pdl) {
@@ -556,6 +634,51 @@ int qgemm_launch(cudaStream_t st, int qt, const unsigned char* w, const QRows& x
         case QT_Q8_0: return qgemm_launch_q<QT_Q8_0>(st, w, x, M, N, K, epi, y, ldy, pdl);
         default: return -1000;
     }
+}
+
+template <int TM>
+static int qgemm_jobs_launch_t(cudaStream_t st, QJobs& jobs, int ctas, int tiles, bool pdl) {
+    constexpr size_t smem = std::max(QCfg<QT_Q4_K, TM>::SMEM, std::max(QCfg<QT_Q6_K, TM>::SMEM, QCfg<QT_Q8_0, TM>::SMEM));
+    static SmemOptIn seen;
+    if (const int e = ensure_dyn_smem(qgemm_jobs_kernel<TM>, smem, seen)) return e;
+    TcScratch s;
+    if (const int e = tc_scratch_get(st, tiles, &s)) return e;
+    int t = 0;
+    for (int i = 0; i < jobs.n; ++i) {        // partial tiles and counters of their own
+        TcSched& sc = jobs.j[i].a.sc;
+        sc.ws = s.ws + (size_t)2 * jobs.j[i].cta0 * 128 * TM; sc.counters = s.counters + t; jobs.j[i].a.err = s.err;
+        t += sc.tiles_m * sc.tiles_n;
+    }
+    return launch_k(qgemm_jobs_kernel<TM>, dim3(ctas), dim3(QCfg<QT_Q4_K, TM>::THREADS), smem, st, pdl, jobs);
+}
+
+int qgemm_many_launch(cudaStream_t st, const QMany* m, int n, const QRows& x, int M, int K, bool pdl, int* launches) {
+    *launches = 0;
+    for (int i = 0; i < n;) {
+        if (M <= 0 || m[i].N <= 0 || K <= 0 || (K % 256) != 0 || M > x.ldd) return -1000;
+        const int TM = qgemm_rows(m[i].qt, M, m[i].N, K);
+        QJobs jobs = {};
+        int ctas = 0, tiles = 0, e = 0;
+        while (TM <= 64 && i + jobs.n < n && jobs.n < 3 && qgemm_rows(m[i + jobs.n].qt, M, m[i + jobs.n].N, K) == TM) {
+            const QMany& k = m[i + jobs.n];
+            QJob& j = jobs.j[jobs.n];
+            if ((e = q_prepare(k.qt, TM, k.w, x, M, k.N, K, GEMV_STORE, k.y, k.ldy, &j))) return e;
+            if (ctas + j.a.sc.G > std::min(tc_device_sms(), QT_MAX_CTAS)) break;
+            j.cta0 = ctas;
+            ctas += j.a.sc.G; tiles += j.a.sc.tiles_m * j.a.sc.tiles_n;
+            ++jobs.n;
+        }
+        if (jobs.n < 2) {
+            if ((e = qgemm_launch(st, m[i].qt, m[i].w, x, M, m[i].N, K, GEMV_STORE, m[i].y, m[i].ldy, pdl))) return e;
+            ++i;
+        } else {
+            e = TM == 16 ? qgemm_jobs_launch_t<16>(st, jobs, ctas, tiles, pdl) : TM == 32 ? qgemm_jobs_launch_t<32>(st, jobs, ctas, tiles, pdl) : qgemm_jobs_launch_t<64>(st, jobs, ctas, tiles, pdl);
+            if (e) return e;
+            i += jobs.n;
+        }
+        ++*launches;
+    }
+    return 0;
 }
 
 }  // namespace cb

@@ -63,6 +63,9 @@ QRows qrows_at(unsigned char* buf, int rows, int K);
 int xquant_rows_launch(cudaStream_t st, int M, const float* x, int ldx, int K, const float* norm_w, float eps, int mode, const QRows& out, bool pdl);
 // y[m, n] = epi(sum_k W[n, k] x[m, k]); epi: GEMV_STORE, GEMV_RESID or GEMV_SILU_MUL (rows of W interleaved); x quantised for W's type
 int qgemm_launch(cudaStream_t st, int qt, const unsigned char* w, const QRows& x, int M, int N, int K, int epi, float* y, int ldy, bool pdl);
+// several matrices of the same codes (GEMV_STORE): those whose CTAs fit the chip together share a launch.  *launches = how many there were
+struct QMany { int qt; const unsigned char* w; int N; float* y; int ldy; };
+int qgemm_many_launch(cudaStream_t st, const QMany* m, int n, const QRows& x, int M, int K, bool pdl, int* launches);
 // rows x K quantised -> bf16 row-major
 int q_dequant_bf16_launch(cudaStream_t st, int qt, const unsigned char* w, size_t rows, int K, bf16* out);
 // gather + dequantise rows of a quantised embedding table to f32: ids[rows] (prefill) or, with ids == nullptr, state[r].token

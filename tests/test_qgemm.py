@@ -121,3 +121,56 @@ def test_codes_of_a_row_are_its_own(qt, k):
     for n in (1, 2, 4):
         got = np.concatenate([run(x[i:i + n]) for i in range(0, 12, n)])
         assert (np.abs(got - prompt).max(1) <= BAR * np.abs(prompt).max(1)).all(), n
+
+
+@pytest.mark.parametrize("qt,m", [("Q4_K", 1100), ("Q6_K", 700), ("Q6_K", 641)])
+def test_tiles_of_128_rows(qt, m):
+    """Enough work for tiles of 128 activation rows (a ragged last one among them): the same rows in calls of 64, whose tiles are held to the oracle above.  Only the
+    division along K, the order of the f32 additions, differs."""
+    import crane_b200
+    rng = np.random.default_rng(m)
+    raw = np.tile(blocks(rng, 512, 4096, qt), (8, 1))
+    x = rng.standard_normal((m, 4096)).astype(np.float32)
+    got = crane_b200.op_qlinear(x, raw, gq.GGML_TYPE_ID[qt], 4096)
+    for r in range(0, m, 64):
+        part = crane_b200.op_qlinear(x[r: r + 64], raw, gq.GGML_TYPE_ID[qt], 4096) if m - r >= 5 else None
+        assert part is None or np.abs(got[r: r + 64] - part).max() <= BAR * np.abs(part).max()
+    assert np.array_equal(got, crane_b200.op_qlinear(x, raw, gq.GGML_TYPE_ID[qt], 4096))
+
+
+@pytest.mark.parametrize("types", [("Q4_K", "Q4_K", "Q6_K"), ("Q6_K", "Q4_K", "Q4_K"), ("Q8_0", "Q8_0", "Q8_0"), ("Q4_K", "Q8_0", "Q6_K")])
+@pytest.mark.parametrize("hidden", [512, 2560])
+def test_q_k_v_side_by_side(types, hidden):
+    """q, k and v that share a launch (or two, or none: 2560 x 2560 takes all CTAs) give the bits each gives by itself."""
+    import ctypes
+    import crane_b200
+    from crane_b200 import synth
+    cfg = dict(synth.TINY_QWEN3_UNTIED, hidden_size=hidden, intermediate_size=256, num_attention_heads=hidden // 128, num_key_value_heads=hidden // 256, head_dim=128, num_hidden_layers=1,
+               vocab_size=300)
+    rng = np.random.default_rng(hidden)
+    m = crane_b200.Qwen3Model(cfg, max_seq_len=256)
+    raws, norm, table = {}, None, None
+    for name, shape, kind in synth.text_tensor_specs(cfg):
+        short = name.split(".")[-2]
+        qt = dict(zip(("q_proj", "k_proj", "v_proj"), types)).get(short, "Q8_0") if "proj" in name else None
+        if qt:
+            raw = blocks(rng, shape[0], shape[1], qt)
+            raws[short] = (raw, qt, shape[0])
+            m.load_tensor_ggml(name, gq.GGML_TYPE_ID[qt], shape, raw)
+        else:
+            bits = synth.f32_to_bf16_bits(rng.standard_normal(shape, dtype=np.float32))
+            value = (bits.astype(np.uint32) << 16).view(np.float32)
+            norm, table = (value if name.endswith("input_layernorm.weight") else norm), (value if "embed" in name else table)
+            m.load_tensor(name, bits)
+    m.finalize()
+    width = sum(raws[n][2] for n in ("q_proj", "k_proj", "v_proj"))
+    for rows in (7, 16, 17, 33, 64, 65, 130):
+        ids = rng.integers(0, 300, rows).astype(np.uint32)
+        m.clear_kv_cache()
+        m.forward_step(ids, 0)
+        got = np.empty((rows, width), np.float32)
+        assert m.lib.crane_b200_debug_peek(m.h, 1, got.ctypes.data_as(ctypes.c_void_p), ctypes.c_size_t(got.size)) == 0
+        want = np.concatenate([crane_b200.op_qlinear(table[ids], raws[n][0], gq.GGML_TYPE_ID[raws[n][1]], raws[n][2], norm_w=norm, eps=cfg["rms_norm_eps"])
+                               for n in ("q_proj", "k_proj", "v_proj")], 1)
+        assert np.array_equal(got, want), rows
+    m.close()
