@@ -10,6 +10,7 @@
 #include "tc.cuh"
 
 #include <algorithm>
+#include <utility>
 
 namespace cb {
 
@@ -18,6 +19,8 @@ namespace {
 // ---------------------------------------------------------------------------------------------------------------- rows
 __global__ void embed_scale_rows_kernel(const int* __restrict__ ids, int T, const bf16* __restrict__ embed, int W, float scale,
                                         float* __restrict__ x, int ldx) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int r = blockIdx.x;
     const bf16* e = embed + (size_t)ids[r] * W;
     for (int c = threadIdx.x; c < W; c += blockDim.x) x[(size_t)r * ldx + c] = __bfloat162float(e[c]) * scale;
@@ -25,6 +28,8 @@ __global__ void embed_scale_rows_kernel(const int* __restrict__ ids, int T, cons
 
 __global__ void embed_sinpos_rows_kernel(const int* __restrict__ ids, const int* __restrict__ row_pos, const bf16* __restrict__ embed, int W,
                                          const float* __restrict__ freq, float* __restrict__ x, int ldx) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int r = blockIdx.x;
     const bf16* e = embed + (size_t)ids[r] * W;
     const float pos = (float)row_pos[r];
@@ -38,6 +43,8 @@ __global__ void embed_sinpos_rows_kernel(const int* __restrict__ ids, const int*
 __global__ void __launch_bounds__(256) post_norm_add_kernel(const float* __restrict__ y1, int ld1, const float* __restrict__ b1, const float* __restrict__ w1,
                                                             const float* __restrict__ y2, int ld2, const float* __restrict__ w2,
                                                             const float* __restrict__ norm_w, float eps, float* __restrict__ x, int ldx, int W, ActOut planes, DytNorm dyt) {
+    pdl_wait();
+    pdl_launch_dependents();
     __shared__ float red[3][8];
     const int r = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const float* a = y1 + (size_t)r * ld1;
@@ -85,6 +92,8 @@ __global__ void __launch_bounds__(256) post_norm_add_kernel(const float* __restr
 
 __global__ void dyt_rows_kernel(const float* __restrict__ x, int ldx, const int* __restrict__ rows, int W, const float* __restrict__ alpha,
                                 const float* __restrict__ w, const float* __restrict__ b, ActOut out) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int r = blockIdx.x, src = rows ? rows[r] : r;
     const float a = *alpha;
     for (int c = threadIdx.x; c < W; c += blockDim.x) store_act(out, r, c, tanhf(a * x[(size_t)src * ldx + c]) * w[c] + b[c]);
@@ -95,6 +104,8 @@ __global__ void dyt_rows_kernel(const float* __restrict__ x, int ldx, const int*
 // is cut into that many equal consecutive parts and each part is divided by its own root mean square.
 __global__ void __launch_bounds__(256) rms_rows_kernel(const float* __restrict__ x, int ldx, const int* __restrict__ rows, int W, float eps,
                                                        const float* __restrict__ w1, ActOut out1, const float* __restrict__ w2, ActOut out2, int groups) {
+    pdl_wait();
+    pdl_launch_dependents();
     __shared__ float red[8];
     const int r = blockIdx.x, src = rows ? rows[r] : r, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const float* xr = x + (size_t)src * ldx;
@@ -120,11 +131,15 @@ __global__ void __launch_bounds__(256) rms_rows_kernel(const float* __restrict__
 }
 
 __global__ void store_rows_kernel(const float* __restrict__ src, int lds, int W, ActOut dst, int col0) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int r = blockIdx.x;
     for (int c = threadIdx.x; c < W; c += blockDim.x) store_act(dst, r, col0 + c, src[(size_t)r * lds + c]);
 }
 
 __global__ void gather_rows_kernel(const float* __restrict__ src, int lds, const int* __restrict__ rows, int W, float* __restrict__ dst, int ldd) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int r = blockIdx.x;
     for (int c = threadIdx.x; c < W; c += blockDim.x) dst[(size_t)r * ldd + c] = src[(size_t)rows[r] * lds + c];
 }
@@ -136,6 +151,7 @@ template <int MODE>
 __global__ void __launch_bounds__(256) linear_f32_kernel(const float* __restrict__ A, int lda, const bf16* __restrict__ Wt, int ldw, int M, int N,
                                                          int K, float* __restrict__ C, int ldc, const float* __restrict__ col_scale,
                                                          const float* __restrict__ gate, int ldg, const float* __restrict__ gate_bias, const float* __restrict__ bias) {
+    pdl_wait();
     __shared__ float sa[16][64 + 4], sw[16][64 + 4];
     const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     float acc[4][4] = {};
@@ -187,6 +203,8 @@ __global__ void __launch_bounds__(256) linear_f32_kernel(const float* __restrict
 // shared memory and leave as the mixed ones.
 template <typename KT>
 __global__ void attn_prep_kernel(RaggedBatch rb, AttnPrepArgs a) {
+    pdl_wait();
+    pdl_launch_dependents();
     extern __shared__ float rot_cs[];                    // [rot_dims / 2] cos, then sin; with `talk` [H * d] queries behind them
     __shared__ float whole[2][8];
     float* sq = rot_cs + a.rot_dims;
@@ -301,6 +319,8 @@ __global__ void attn_prep_kernel(RaggedBatch rb, AttnPrepArgs a) {
 constexpr int AC_WARPS = 4;
 template <typename KT, int NC, int TAPS>
 __global__ void __launch_bounds__(AC_WARPS * 32) attn_conv_prep_kernel(RaggedBatch rb, AttnPrepArgs a, int tile) {
+    pdl_wait();
+    pdl_launch_dependents();
     __shared__ float ys[AC_WARPS][32 * NC];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, hh = blockIdx.y * AC_WARPS + warp, r0 = blockIdx.x * tile, r1 = min(rb.T, r0 + tile);
     if (hh >= a.H + 2 * a.G) return;
@@ -386,6 +406,7 @@ __device__ __forceinline__ float attn_out_factor(const SinkAttnArgs& a, int r, i
 }
 template <typename KT, int REP, bool STAGE, int MAXC>
 __global__ void __launch_bounds__(ATT_WARPS * 32) sink_attention_kernel(RaggedBatch rb, SinkAttnArgs a) {
+    pdl_wait();
     constexpr bool stage = STAGE;
     extern __shared__ __align__(16) float smem[];
     const int d = a.d, dv = a.dv, rep = a.H / a.G, nb = (rep + REP - 1) / REP;
@@ -591,6 +612,8 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) sink_attention_kernel(RaggedBa
 }
 
 __global__ void sink_attention_merge_kernel(SinkAttnArgs a) {
+    pdl_wait();
+    pdl_launch_dependents();
     __shared__ float wgt[64];
     __shared__ float Ls;
     const int r = blockIdx.x, h = blockIdx.y, dv = a.dv, ns = a.nsplit;           // nsplit <= 64
@@ -620,6 +643,8 @@ __global__ void sink_attention_merge_kernel(SinkAttnArgs a) {
 // Causal depthwise convolution over the x | B | C columns + SiLU.  The taps that reach before the entry's first row read the
 // sequence's carried window (zeros for a new sequence).
 __global__ void conv_silu_kernel(RaggedBatch rb, Mamba2Args a, int C, int col0) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int r = blockIdx.y, c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= C) return;
     const int e = rb.row_entry[r], i = r - rb.ent_row0[e], slot = rb.ent_slot[e], taps = a.taps;
@@ -634,6 +659,8 @@ __global__ void conv_silu_kernel(RaggedBatch rb, Mamba2Args a, int C, int col0) 
 }
 // Every entry one token (decode): the convolution and the window shift in one pass; thread = (entry, channel) owns its window column.
 __global__ void conv_step_kernel(RaggedBatch rb, Mamba2Args a, int C, int col0) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int e = blockIdx.y, c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= C) return;
     const int r = rb.ent_row0[e], slot = rb.ent_slot[e], taps = a.taps;
@@ -650,6 +677,8 @@ __global__ void conv_step_kernel(RaggedBatch rb, Mamba2Args a, int C, int col0) 
 }
 // New window = the last taps-1 inputs of the sequence (older ones shift down when the entry is shorter than the window).
 __global__ void conv_window_kernel(RaggedBatch rb, Mamba2Args a, int C, int col0) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int e = blockIdx.y, c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= C) return;
     const int len = rb.ent_len[e], r0 = rb.ent_row0[e], slot = rb.ent_slot[e], nwin = a.taps - 1;
@@ -666,9 +695,10 @@ __global__ void conv_window_kernel(RaggedBatch rb, Mamba2Args a, int C, int col0
 // double-buffered: chunk c + 1 is in flight while chunk c is consumed.  dt = softplus(.) and the decay exp(-exp(A) dt) are
 // computed once per token, in f32, when its chunk lands.
 // What bounds it: the instructions between one token and the next in the one warp a scheduler has.  A thread owns its state rows of SSD_CPT columns, so that B
-// and C, most of what a token reads from shared memory, are read once for both, and the outputs of four tokens are summed over the lanes together.
-// us, 16 heads of 128 x 128, one column and three shuffles a token / so: steps with a portion of 256 tokens 98 / 74, five entries 42 / 29.  (Segments from
-// 64 rows on gained nothing more for such portions: their second pass and the prefix take what they save.)
+// and C, most of what a token reads from shared memory, are read once for both, two state rows go through an instruction, and the outputs of four tokens are
+// summed over the lanes together.  us, 16 heads of 128 x 128: one portion of 256 tokens 58 with one row an instruction and reads through generic addresses, 49 so.
+// (Neither sixteen lanes a column, two warps a scheduler, nor four columns a thread were faster: 54 to 57.  Segments from 64 rows on gained nothing for such
+// portions: their second pass and the prefix take what they save.)
 constexpr int SSD_NS = 8, SSD_MAXR = 32, SSD_CH = 16;      // N <= 256
 constexpr int SSD_TH = 16 * SSD_NS;                         // 128 threads: one warp per scheduler, many blocks
 // Staged layout of one token: x slice [16 SSD_CPT] | B | C | dt, pad.  Thread ns owns the CONTIGUOUS state rows ns * R .. ns * R + R - 1,
@@ -685,11 +715,22 @@ constexpr int SSD_SEGS = 4, SSD_SEG_MIN = 512;              // an entry is segme
 __host__ __device__ inline int ssd_seg_len(int len) { return ((len + SSD_SEGS - 1) / SSD_SEGS + SSD_CH - 1) / SSD_CH * SSD_CH; }
 template <int SSD_R, int MODE, int SSD_CPT = 2>              // state rows per thread: ceil(N / 8) rounded up to 4, 8, 16 or 32
 __global__ void __launch_bounds__(SSD_TH) ssd_scan_kernel(RaggedBatch rb, Mamba2Args a, int C) {
+    pdl_wait();
     constexpr int SSD_COLS = 16 * SSD_CPT;
     extern __shared__ __align__(16) float ssm_s[];
-    const int e = MODE == 0 ? blockIdx.x : blockIdx.x / SSD_SEGS, seg = MODE == 0 ? 0 : blockIdx.x % SSD_SEGS;
-    const int h = blockIdx.y, ns = threadIdx.x & (SSD_NS - 1), pl = threadIdx.x / SSD_NS;
-    const int p0 = blockIdx.z * SSD_COLS;
+    // Entries in order of length, the longest first, and the slowest index of the grid: blocks of long portions that follow one another land on different SMs, those of
+    // single tokens beside them.  (Entries as they come, fastest: a step of two long portions and two tokens 107 us, so 50.)
+    __shared__ int s_entry;
+    const int rank = MODE == 0 ? blockIdx.z : blockIdx.z / SSD_SEGS, seg = MODE == 0 ? 0 : blockIdx.z % SSD_SEGS;
+    for (int i = threadIdx.x; i < rb.E; i += SSD_TH) {
+        const int li = rb.ent_len[i];
+        int ahead = 0;
+        for (int j = 0; j < rb.E; ++j) { const int lj = rb.ent_len[j]; ahead += lj > li || (lj == li && j < i); }
+        if (ahead == rank) s_entry = i;
+    }
+    __syncthreads();
+    const int e = s_entry, h = blockIdx.x, ns = threadIdx.x & (SSD_NS - 1), pl = threadIdx.x / SSD_NS;
+    const int p0 = blockIdx.y * SSD_COLS;
     const int P = a.P, N = a.N, inner = a.heads * P, g = h / (a.heads / a.groups);
     bool live[SSD_CPT];
 #pragma unroll
@@ -702,7 +743,7 @@ __global__ void __launch_bounds__(SSD_TH) ssd_scan_kernel(RaggedBatch rb, Mamba2
     const int len = min(seg_len, full_len - seg0), r0 = rb.ent_row0[e] + seg0;
     const int ncol = min(SSD_COLS, P - p0);
     const int NP = ssd_npad(N, SSD_R), per_tok = SSD_COLS + 2 * NP + 4;
-    float* stage[2] = {ssm_s, ssm_s + SSD_CH * per_tok};
+    auto stage = [&](int c) { return ssm_s + (c & 1) * SSD_CH * per_tok; };      // (computed: out of an array of pointers the reads are generic ones)
     float* sdt = ssm_s + 2 * SSD_CH * per_tok;                // [SSD_CH] dt, [SSD_CH] decay
     float* S = whole ? a.ssm_state + (((size_t)slot * a.heads + h) * N) * P
                          : a.seg_state + ((((size_t)e * SSD_SEGS + seg) * a.heads + h) * N) * P;
@@ -710,11 +751,14 @@ __global__ void __launch_bounds__(SSD_TH) ssd_scan_kernel(RaggedBatch rb, Mamba2
     // rows past N and tokens past the portion's end multiply zeros: the stages start zeroed and only real values are ever copied in
     for (int i = threadIdx.x; i < 2 * SSD_CH * per_tok; i += blockDim.x) ssm_s[i] = 0.f;
     __syncthreads();
-    float s[SSD_CPT][SSD_R];
+    uint64_t s[SSD_CPT][SSD_R / 2];                           // pairs of state rows
 #pragma unroll
-    for (int i = 0; i < SSD_R; ++i)
+    for (int i = 0; i < SSD_R / 2; ++i)
 #pragma unroll
-        for (int j = 0; j < SSD_CPT; ++j) s[j][i] = (MODE != 1 && n0 + i < N && live[j]) ? S[(size_t)(n0 + i) * P + p0 + pl + 16 * j] : 0.f;
+        for (int j = 0; j < SSD_CPT; ++j) {
+            auto at = [&](int n) { return (MODE != 1 && n < N && live[j]) ? S[(size_t)n * P + p0 + pl + 16 * j] : 0.f; };
+            s[j][i] = f2(at(n0 + 2 * i), at(n0 + 2 * i + 1));
+        }
     float dprod = 1.f;                                        // MODE 1, thread 0: product of the segment's decays
     const float negA = -__expf(a.A_log[h]), Dh = a.D[h], dtb = a.dt_bias[h];
     const int dtcol = 2 * inner + 2 * a.groups * N + h;
@@ -751,12 +795,12 @@ __global__ void __launch_bounds__(SSD_TH) ssd_scan_kernel(RaggedBatch rb, Mamba2
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     const int nch = (len + SSD_CH - 1) / SSD_CH;
-    fetch(0, stage[0]);
+    fetch(0, stage(0));
     for (int c = 0; c < nch; ++c) {
-        if (c + 1 < nch) { fetch(c + 1, stage[(c + 1) & 1]); asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+        if (c + 1 < nch) { fetch(c + 1, stage(c + 1)); asm volatile("cp.async.wait_group 1;" ::: "memory"); }
         else asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
-        const float* st = stage[c & 1];
+        const float* st = stage(c);
         const int nt = min(SSD_CH, len - c * SSD_CH);
         if (threadIdx.x < SSD_CH) {
             const float z = st[threadIdx.x * per_tok + SSD_COLS + 2 * NP] + dtb;
@@ -777,30 +821,29 @@ __global__ void __launch_bounds__(SSD_TH) ssd_scan_kernel(RaggedBatch rb, Mamba2
                 float dx[SSD_CPT];
 #pragma unroll
                 for (int j = 0; j < SSD_CPT; ++j) dx[j] = dt * (live[j] ? tk[pl + 16 * j] : 0.f);
-                const float4* B4 = reinterpret_cast<const float4*>(tk + SSD_COLS + ssd_idx(n0, SSD_R));
-                const float4* C4 = reinterpret_cast<const float4*>(tk + SSD_COLS + NP + ssd_idx(n0, SSD_R));
-                float y0[SSD_CPT], y1[SSD_CPT];
+                const ulonglong2* B4 = reinterpret_cast<const ulonglong2*>(tk + SSD_COLS + ssd_idx(n0, SSD_R));
+                const ulonglong2* C4 = reinterpret_cast<const ulonglong2*>(tk + SSD_COLS + NP + ssd_idx(n0, SSD_R));
+                // two state rows an instruction (each rounded as by itself): a state pair is decayed and fed, then multiplied with C
+                uint64_t yp[SSD_CPT], dxp[SSD_CPT];
+                const uint64_t dp = f2(decay, decay);
 #pragma unroll
-                for (int j = 0; j < SSD_CPT; ++j) y0[j] = y1[j] = 0.f;
+                for (int j = 0; j < SSD_CPT; ++j) { yp[j] = 0; dxp[j] = f2(dx[j], dx[j]); }
 #pragma unroll
                 for (int i = 0; i < SSD_R / 4; ++i) {
-                    const float4 b = B4[i];
+                    const ulonglong2 b = B4[i];
 #pragma unroll
                     for (int j = 0; j < SSD_CPT; ++j) {
-                        s[j][4 * i] = fmaf(decay, s[j][4 * i], b.x * dx[j]); s[j][4 * i + 1] = fmaf(decay, s[j][4 * i + 1], b.y * dx[j]);
-                        s[j][4 * i + 2] = fmaf(decay, s[j][4 * i + 2], b.z * dx[j]); s[j][4 * i + 3] = fmaf(decay, s[j][4 * i + 3], b.w * dx[j]);
+                        s[j][2 * i] = f2_fma(dp, s[j][2 * i], f2_mul(b.x, dxp[j]));
+                        s[j][2 * i + 1] = f2_fma(dp, s[j][2 * i + 1], f2_mul(b.y, dxp[j]));
                     }
                     if constexpr (MODE != 1) {                // (MODE 1: state only)
-                        const float4 cc = C4[i];
+                        const ulonglong2 cc = C4[i];
 #pragma unroll
-                        for (int j = 0; j < SSD_CPT; ++j) {
-                            y0[j] = fmaf(s[j][4 * i], cc.x, y0[j]); y1[j] = fmaf(s[j][4 * i + 1], cc.y, y1[j]);
-                            y0[j] = fmaf(s[j][4 * i + 2], cc.z, y0[j]); y1[j] = fmaf(s[j][4 * i + 3], cc.w, y1[j]);
-                        }
+                        for (int j = 0; j < SSD_CPT; ++j) { yp[j] = f2_fma(s[j][2 * i], cc.x, yp[j]); yp[j] = f2_fma(s[j][2 * i + 1], cc.y, yp[j]); }
                     }
                 }
 #pragma unroll
-                for (int j = 0; j < SSD_CPT; ++j) y[tt * SSD_CPT + j] = y0[j] + y1[j];
+                for (int j = 0; j < SSD_CPT; ++j) { float y0, y1; f2_split(yp[j], y0, y1); y[tt * SSD_CPT + j] = y0 + y1; }
             }
             if constexpr (MODE != 1) {
                 int id = 0, bit = SSD_NS / 2;
@@ -821,15 +864,23 @@ __global__ void __launch_bounds__(SSD_TH) ssd_scan_kernel(RaggedBatch rb, Mamba2
         }
         __syncthreads();                                      // the stage is free for chunk c + 2
     }
+    pdl_launch_dependents();                                  // (not earlier: blocks that wait beside a scan slow it down)
     if (MODE == 2 && !whole) return;                          // the prefix kernel already wrote the sequence's new state
 #pragma unroll
-    for (int i = 0; i < SSD_R; ++i)
+    for (int i = 0; i < SSD_R / 2; ++i)
 #pragma unroll
-        for (int j = 0; j < SSD_CPT; ++j) if (n0 + i < N && live[j]) S[(size_t)(n0 + i) * P + p0 + pl + 16 * j] = s[j][i];
-    if (MODE == 1 && threadIdx.x == 0 && blockIdx.z == 0) a.seg_decay[((size_t)e * SSD_SEGS + seg) * a.heads + h] = dprod;
+        for (int j = 0; j < SSD_CPT; ++j) {
+            float v[2];
+            f2_split(s[j][i], v[0], v[1]);
+#pragma unroll
+            for (int k = 0; k < 2; ++k) if (n0 + 2 * i + k < N && live[j]) S[(size_t)(n0 + 2 * i + k) * P + p0 + pl + 16 * j] = v[k];
+        }
+    if (MODE == 1 && threadIdx.x == 0 && blockIdx.y == 0) a.seg_decay[((size_t)e * SSD_SEGS + seg) * a.heads + h] = dprod;
 }
 // Start state of every segment, in order: seg_state[k] holds S_local on entry and S_start(k) on exit; the slot gets the end state.
 __global__ void ssd_seg_prefix_kernel(RaggedBatch rb, Mamba2Args a) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int e = blockIdx.x, h = blockIdx.y, np = a.N * a.P;
     const int len = rb.ent_len[e], slot = rb.ent_slot[e];
     if (len < SSD_SEG_MIN) return;
@@ -852,6 +903,8 @@ __global__ void ssd_seg_prefix_kernel(RaggedBatch rb, Mamba2Args a) {
 
 // out = unit_rms_per_group(y * silu(z)) * w : block per (row, group)
 __global__ void gated_group_rms_kernel(Mamba2Args a) {
+    pdl_wait();
+    pdl_launch_dependents();
     __shared__ float scratch[32];
     const int r = blockIdx.x, gi = blockIdx.y, inner = a.heads * a.P, gs = inner / a.norm_groups;
     const float* y = a.y + (size_t)r * inner + gi * gs;
@@ -868,6 +921,8 @@ __global__ void gated_group_rms_kernel(Mamba2Args a) {
 
 // ---------------------------------------------------------------------------------------------------------------- feed-forwards
 __global__ void clamped_glu_kernel(const float* __restrict__ gu, int ld, int stride, int up_off, int F, float limit, ActOut out) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int r = blockIdx.y, j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= F) return;
     const float g = fminf(gu[(size_t)r * ld + (size_t)j * stride], limit);
@@ -876,6 +931,8 @@ __global__ void clamped_glu_kernel(const float* __restrict__ gu, int ld, int str
 }
 
 __global__ void silu_glu_kernel(const float* __restrict__ gu, int ld, int F, ActOut out, float limit, const float* __restrict__ bias) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int r = blockIdx.y, j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= F) return;
     store_act(out, r, j, glu_pair_f(gu[(size_t)r * ld + 2 * j] + (bias ? bias[2 * j] : 0.f), gu[(size_t)r * ld + 2 * j + 1] + (bias ? bias[2 * j + 1] : 0.f), limit < 0.f ? limit : 0.f));
@@ -918,6 +975,7 @@ __device__ __forceinline__ bool router_vec_ok(int W, int ldw, int ldh) { return 
 
 // Many rows: one warp per row, four experts per pass over the row (which stays in L1).
 __global__ void __launch_bounds__(256) router_logits_kernel(MoeArgs a, const bf16* __restrict__ w_router, int ldw) {
+    pdl_wait();
     const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (r >= a.T) return;
     const float* h = a.h + (size_t)r * a.ldh;
@@ -994,6 +1052,8 @@ __device__ __forceinline__ void choose_experts(const MoeArgs& a, const float* z,
 
 // One warp per row, logits from global memory.
 __global__ void __launch_bounds__(128) route_kernel(MoeArgs a) {
+    pdl_wait();
+    pdl_launch_dependents();
     __shared__ float scr[4][3][256];
     const int warp = threadIdx.x >> 5, r = blockIdx.x * 4 + warp, lane = threadIdx.x & 31;
     if (r >= a.T) return;
@@ -1004,6 +1064,8 @@ __global__ void __launch_bounds__(128) route_kernel(MoeArgs a) {
 // Few rows (decode): router logits and the choice in one block per row.  Warp w computes the logits of experts w, w + 8, ...
 // (f32 products of the f32 row with the bf16 router rows, lanes striding the width), warp 0 then selects as route_kernel does.
 __global__ void __launch_bounds__(256) route_rows_kernel(MoeArgs a, const bf16* __restrict__ w_router, int ldw) {
+    pdl_wait();
+    pdl_launch_dependents();
     __shared__ float z[256 + 4];
     __shared__ float scr[3][256];
     const int r = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1022,6 +1084,8 @@ __global__ void __launch_bounds__(256) route_rows_kernel(MoeArgs a, const bf16* 
 
 // Counting sort of the (row, choice) pairs by expert + the tile map of the grouped linears (32 pairs per tile).  One block.
 __global__ void moe_sort_kernel(MoeArgs a) {
+    pdl_wait();
+    pdl_launch_dependents();
     extern __shared__ int sh[];
     int* cnt = sh; int* off = sh + a.E; int* fill = sh + 2 * a.E;
     const int n = a.T * a.top;
@@ -1050,6 +1114,7 @@ __global__ void moe_sort_kernel(MoeArgs a) {
 // Grouped linear: tile = 32 pairs of one expert x 64 output columns.  UP: act[pair] = gelu_erf(up_e h[row of pair]); else y[pair] = down_e act[pair].
 template <bool UP>
 __global__ void __launch_bounds__(256) moe_linear_kernel(MoeArgs a) {
+    pdl_wait();
     __shared__ float sa[16][32 + 1], sw[16][64 + 4];
     __shared__ int spair[32];
     const int tile = blockIdx.y;
@@ -1102,6 +1167,8 @@ __global__ void __launch_bounds__(256) moe_linear_kernel(MoeArgs a) {
 // the weight is 1 where it already multiplied the expert's input.  Optionally, before the add: an every-token expert's output times a
 // per-row scalar joins the sum, a per-column scale applies, and a sigmoid gate per element multiplies the whole.
 __global__ void moe_combine_kernel(MoeArgs a, int y_sorted) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int r = blockIdx.y, c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= a.W) return;
     float s = 0.f;
@@ -1115,6 +1182,8 @@ __global__ void moe_combine_kernel(MoeArgs a, int y_sorted) {
     a.x[(size_t)r * a.ldx + c] += s;
 }
 __global__ void moe_gather_kernel(MoeArgs a, ActOut src, ActOut dst) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int i = blockIdx.x, r = a.sorted[i] / a.top;
     if (a.scale_input) {                                    // the expert's input is weight * h, rounded as the planes round it
         const float ws = a.sel_w[a.sorted[i]];
@@ -1142,6 +1211,8 @@ __global__ void moe_gather_kernel(MoeArgs a, ActOut src, ActOut dst) {
 constexpr int ARGMAX_PARTS = 64;
 __device__ __forceinline__ void argmax_merge(float& bv, int& bi, float ov, int oi) { if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; } }
 __global__ void __launch_bounds__(256) argmax_parts_kernel(const float* __restrict__ logits, int V, float* __restrict__ pv, int* __restrict__ pi) {
+    pdl_wait();
+    pdl_launch_dependents();
     __shared__ float sv[8];
     __shared__ int si[8];
     const int e = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1160,6 +1231,8 @@ __global__ void __launch_bounds__(256) argmax_parts_kernel(const float* __restri
 // one warp per row finishes the argmax (lowest index among maxima), feeds the token back and moves the positions on
 __global__ void greedy_advance_kernel(const float* __restrict__ pv, const int* __restrict__ pi, int E, int* ids, int* row_pos, int* ent_pos0,
                                       uint32_t* out, int out_stride, int* step) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int t = *step;
     for (int e = warp; e < E; e += nw) {
@@ -1180,6 +1253,7 @@ __global__ void greedy_advance_kernel(const float* __restrict__ pv, const int* _
 // shared memory and every warp streams two weight rows with 16-byte loads (padded row widths are multiples of 256).
 template <bool UP>
 __global__ void __launch_bounds__(256) moe_gemv_kernel(MoeArgs a) {
+    pdl_wait();
     extern __shared__ float xs[];
     const int pr = blockIdx.y, e = a.sel_e[pr], lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int N = UP ? a.F : a.W, K = UP ? a.W : a.F, ldw = UP ? a.ldwu : a.ldwd;
@@ -1215,62 +1289,68 @@ __global__ void __launch_bounds__(256) moe_gemv_kernel(MoeArgs a) {
 }
 
 inline int last_err() { return (int)cudaGetLastError(); }
+// Every kernel of this file begins with the dependency wait and lets the next one in, so it is launched as a programmatic dependent: its launch and the fetch of
+// its first instructions run under the tail of the kernel ahead (2 to 3 us from one grid's end to the next one's start before).  A failure is left for last_err.
+template <typename... KArgs, typename... Args>
+inline void go(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
+    (void)launch_k(kernel, grid, block, smem, st, prefill_pdl(), std::forward<Args>(args)...);
+}
 
 }  // namespace
 
 // ---------------------------------------------------------------------------------------------------------------- launchers
 int embed_scale_rows_launch(cudaStream_t st, const int* ids, int T, const bf16* embed, int W, float scale, float* x, int ldx) {
-    embed_scale_rows_kernel<<<T, 128, 0, st>>>(ids, T, embed, W, scale, x, ldx);
+    go(embed_scale_rows_kernel, T, 128, 0, st, ids, T, embed, W, scale, x, ldx);
     return last_err();
 }
 int embed_sinpos_rows_launch(cudaStream_t st, const int* ids, const int* row_pos, int T, const bf16* embed, int W, const float* freq, float* x, int ldx) {
-    embed_sinpos_rows_kernel<<<T, 128, 0, st>>>(ids, row_pos, embed, W, freq, x, ldx);
+    go(embed_sinpos_rows_kernel, T, 128, 0, st, ids, row_pos, embed, W, freq, x, ldx);
     return last_err();
 }
 int post_norm_add_launch(cudaStream_t st, const float* y1, int ld1, const float* b1, const float* w1, const float* y2, int ld2, const float* w2,
                          const float* norm_w, float eps, float* x, int ldx, int T, int W, const ActOut& planes, const DytNorm& dyt) {
     if (!y1 || !norm_w || (planes.f && !dyt.w)) return -1000;
-    post_norm_add_kernel<<<T, 256, 0, st>>>(y1, ld1, b1, w1, y2, ld2, w2, norm_w, eps, x, ldx, W, planes, dyt);
+    go(post_norm_add_kernel, T, 256, 0, st, y1, ld1, b1, w1, y2, ld2, w2, norm_w, eps, x, ldx, W, planes, dyt);
     return last_err();
 }
 int dyt_rows_launch(cudaStream_t st, const float* x, int ldx, const int* rows, int R, int W, const float* alpha, const float* w, const float* b,
                     const ActOut& out) {
-    dyt_rows_kernel<<<R, 128, 0, st>>>(x, ldx, rows, W, alpha, w, b, out);
+    go(dyt_rows_kernel, R, 128, 0, st, x, ldx, rows, W, alpha, w, b, out);
     return last_err();
 }
 int greedy_advance_launch(cudaStream_t st, const float* logits, int V, int E, float* part_val, int* part_idx, int* ids, int* row_pos,
                           int* ent_pos0, uint32_t* out, int out_stride, int* step) {
-    argmax_parts_kernel<<<dim3(ARGMAX_PARTS, E), 256, 0, st>>>(logits, V, part_val, part_idx);
+    go(argmax_parts_kernel, dim3(ARGMAX_PARTS, E), 256, 0, st, logits, V, part_val, part_idx);
     int e = last_err();
     if (e) return e;
-    greedy_advance_kernel<<<1, 256, 0, st>>>(part_val, part_idx, E, ids, row_pos, ent_pos0, out, out_stride, step);
+    go(greedy_advance_kernel, 1, 256, 0, st, part_val, part_idx, E, ids, row_pos, ent_pos0, out, out_stride, step);
     return last_err();
 }
 int gather_rows_launch(cudaStream_t st, const float* src, int lds, const int* rows, int R, int W, float* dst, int ldd) {
-    gather_rows_kernel<<<R, 128, 0, st>>>(src, lds, rows, W, dst, ldd);
+    go(gather_rows_kernel, R, 128, 0, st, src, lds, rows, W, dst, ldd);
     return last_err();
 }
 int linear_f32_launch(cudaStream_t st, const float* A, int lda, const bf16* W, int ldw, int M, int N, int K, int mode, float* C, int ldc,
                       const float* col_scale, const float* gate, int ldg, const float* gate_bias, const float* bias) {
     if (M <= 0 || N <= 0 || K <= 0) return -1000;
     const dim3 grid((N + 63) / 64, (M + 63) / 64);
-    if (mode == LIN_RELU2) linear_f32_kernel<LIN_RELU2><<<grid, 256, 0, st>>>(A, lda, W, ldw, M, N, K, C, ldc, nullptr, nullptr, 0, nullptr, nullptr);
-    else if (mode == LIN_RESID) linear_f32_kernel<LIN_RESID><<<grid, 256, 0, st>>>(A, lda, W, ldw, M, N, K, C, ldc, col_scale, gate, ldg, gate_bias, bias);
-    else linear_f32_kernel<LIN_STORE><<<grid, 256, 0, st>>>(A, lda, W, ldw, M, N, K, C, ldc, nullptr, nullptr, 0, nullptr, nullptr);
+    if (mode == LIN_RELU2) go(linear_f32_kernel<LIN_RELU2>, grid, 256, 0, st, A, lda, W, ldw, M, N, K, C, ldc, nullptr, nullptr, 0, nullptr, nullptr);
+    else if (mode == LIN_RESID) go(linear_f32_kernel<LIN_RESID>, grid, 256, 0, st, A, lda, W, ldw, M, N, K, C, ldc, col_scale, gate, ldg, gate_bias, bias);
+    else go(linear_f32_kernel<LIN_STORE>, grid, 256, 0, st, A, lda, W, ldw, M, N, K, C, ldc, nullptr, nullptr, 0, nullptr, nullptr);
     return last_err();
 }
 int rms_rows_launch(cudaStream_t st, const float* x, int ldx, const int* rows, int R, int W, float eps, const float* w1, const ActOut& out1,
                     const float* w2, const ActOut& out2, int groups) {
     if (groups < 1 || W % groups) return -1000;
-    rms_rows_kernel<<<R, 256, 0, st>>>(x, ldx, rows, W, eps, w1, out1, w2, out2, groups);
+    go(rms_rows_kernel, R, 256, 0, st, x, ldx, rows, W, eps, w1, out1, w2, out2, groups);
     return last_err();
 }
 int store_rows_launch(cudaStream_t st, const float* src, int lds, int T, int W, const ActOut& dst, int col0) {
-    store_rows_kernel<<<T, 128, 0, st>>>(src, lds, W, dst, col0);
+    go(store_rows_kernel, T, 128, 0, st, src, lds, W, dst, col0);
     return last_err();
 }
 int silu_glu_launch(cudaStream_t st, const float* gu, int ld, int T, int F, const ActOut& out, float limit, const float* bias) {
-    silu_glu_kernel<<<dim3((F + 127) / 128, T), 128, 0, st>>>(gu, ld, F, out, limit, bias);
+    go(silu_glu_kernel, dim3((F + 127) / 128, T), 128, 0, st, gu, ld, F, out, limit, bias);
     return last_err();
 }
 template <typename KT>
@@ -1280,7 +1360,7 @@ static int attn_conv_prep_launch(cudaStream_t st, const RaggedBatch& rb, const A
     const dim3 grid((rb.T + tile - 1) / tile, (units + AC_WARPS - 1) / AC_WARPS);
     auto run = [&](auto k0, auto k1, auto k2, auto k3, auto k4) {
         auto k = a.conv_taps == 1 ? k1 : a.conv_taps == 2 ? k2 : a.conv_taps == 3 ? k3 : a.conv_taps == 4 ? k4 : k0;
-        k<<<grid, AC_WARPS * 32, 0, st>>>(rb, a, tile);
+        go(k, grid, AC_WARPS * 32, 0, st, rb, a, tile);
     };
     if (w <= 64) run(attn_conv_prep_kernel<KT, 2, 0>, attn_conv_prep_kernel<KT, 2, 1>, attn_conv_prep_kernel<KT, 2, 2>, attn_conv_prep_kernel<KT, 2, 3>, attn_conv_prep_kernel<KT, 2, 4>);
     else if (w <= 128) run(attn_conv_prep_kernel<KT, 4, 0>, attn_conv_prep_kernel<KT, 4, 1>, attn_conv_prep_kernel<KT, 4, 2>, attn_conv_prep_kernel<KT, 4, 3>, attn_conv_prep_kernel<KT, 4, 4>);
@@ -1299,8 +1379,8 @@ int attn_prep_launch(cudaStream_t st, const RaggedBatch& rb, const AttnPrepArgs&
         static SmemOptIn seen_f, seen_b;
         if (const int e = a.kv_f32 ? ensure_dyn_smem(attn_prep_kernel<float>, sm, seen_f) : ensure_dyn_smem(attn_prep_kernel<bf16>, sm, seen_b)) return e;
     }
-    if (a.kv_f32) attn_prep_kernel<float><<<rb.T, 256, sm, st>>>(rb, a);
-    else attn_prep_kernel<bf16><<<rb.T, 256, sm, st>>>(rb, a);
+    if (a.kv_f32) go(attn_prep_kernel<float>, rb.T, 256, sm, st, rb, a);
+    else go(attn_prep_kernel<bf16>, rb.T, 256, sm, st, rb, a);
     return last_err();
 }
 template <typename KT, int REP, int MAXC>
@@ -1318,11 +1398,11 @@ static int sink_attention_launch_t(cudaStream_t st, const RaggedBatch& rb, const
     static SmemOptIn seen, seen_staged;
     if (stage) {
         if (const int e = ensure_dyn_smem(sink_attention_kernel<KT, REP, true, MAXC>, smem, seen_staged)) return e;
-        sink_attention_kernel<KT, REP, true, MAXC><<<dim3(rb.T, a.G * nb, a.nsplit), ATT_WARPS * 32, smem, st>>>(rb, a);
+        go(sink_attention_kernel<KT, REP, true, MAXC>, dim3(rb.T, a.G * nb, a.nsplit), ATT_WARPS * 32, smem, st, rb, a);
         return last_err();
     }
     if (const int e = ensure_dyn_smem(sink_attention_kernel<KT, REP, false, MAXC>, smem, seen)) return e;
-    sink_attention_kernel<KT, REP, false, MAXC><<<dim3(rb.T, a.G * nb, a.nsplit), ATT_WARPS * 32, smem, st>>>(rb, a);
+    go(sink_attention_kernel<KT, REP, false, MAXC>, dim3(rb.T, a.G * nb, a.nsplit), ATT_WARPS * 32, smem, st, rb, a);
     return last_err();
 }
 template <typename KT>
@@ -1350,7 +1430,7 @@ int sink_attention_launch(cudaStream_t st, const RaggedBatch& rb, const SinkAttn
 }
 int sink_attention_merge_launch(cudaStream_t st, const RaggedBatch& rb, const SinkAttnArgs& a) {
     if (a.nsplit > 64) return -1000;
-    sink_attention_merge_kernel<<<dim3(rb.T, a.H), 128, 0, st>>>(a);
+    go(sink_attention_merge_kernel, dim3(rb.T, a.H), 128, 0, st, a);
     return last_err();
 }
 int mamba2_launch_count(bool single_rows, int max_len) { return single_rows ? 3 : max_len >= SSD_SEG_MIN ? 6 : 4; }
@@ -1361,13 +1441,13 @@ int mamba2_mixer_launch(cudaStream_t st, const RaggedBatch& rb, const Mamba2Args
     if (a.N > SSD_NS * SSD_MAXR || a.heads % a.groups || inner % a.norm_groups || a.taps < 1) return -1000;
     int e;
     if (a.single_rows) {
-        conv_step_kernel<<<dim3((C + 127) / 128, rb.E), 128, 0, st>>>(rb, a, C, inner);
+        go(conv_step_kernel, dim3((C + 127) / 128, rb.E), 128, 0, st, rb, a, C, inner);
         if ((e = last_err())) return e;
     } else {
-        conv_silu_kernel<<<dim3((C + 127) / 128, rb.T), 128, 0, st>>>(rb, a, C, inner);
+        go(conv_silu_kernel, dim3((C + 127) / 128, rb.T), 128, 0, st, rb, a, C, inner);
         if ((e = last_err())) return e;
         if (a.taps > 1) {
-            conv_window_kernel<<<dim3((C + 127) / 128, rb.E), 128, 0, st>>>(rb, a, C, inner);
+            go(conv_window_kernel, dim3((C + 127) / 128, rb.E), 128, 0, st, rb, a, C, inner);
             if ((e = last_err())) return e;
         }
     }
@@ -1376,14 +1456,17 @@ int mamba2_mixer_launch(cudaStream_t st, const RaggedBatch& rb, const Mamba2Args
     const int rr = nr <= 4 ? 4 : nr <= 8 ? 8 : nr <= 16 ? 16 : 32;
     // Columns of a block.  States of more than 128 rows hold 64 values of two columns per thread and spill; with one column a thread has half the work per token, which
     // is the shorter way while blocks of 16 columns have an SM each.  us, 16 / 32 columns, 16 heads of state 256 x 128: one entry of 1 token 8.4 / 9.6, of 64 24.8 / 29.9,
-    // of 500 136 / 186; two entries of 64 32.7 / 30.5, of 500 200 / 188.
+    // of 500 136 / 186; two entries of 64 32.7 / 30.5, of 500 200 / 188 (one state row an instruction on either side).
     const bool narrow = rr == 32 && !segs && rb.E * a.heads * ((a.P + 15) / 16) <= tc_device_sms();
     const int cols = narrow ? 16 : 32;
-    const dim3 sgrid(rb.E, a.heads, (a.P + cols - 1) / cols);
+    const dim3 sgrid(a.heads, (a.P + cols - 1) / cols, rb.E);
     const size_t ssm = (size_t)(2 * SSD_CH * (cols + 2 * ssd_npad(a.N, rr) + 4) + 2 * SSD_CH) * sizeof(float);      // <= 80 KB at N = 256
+    // While there is an SM for every block, none shares one (more than half of its shared memory each): the scheduler otherwise puts pairs on some SMs, and two blocks of
+    // 256 tokens on one take 65 us, alone 50.
     auto run = [&](auto kern, SmemOptIn& seen, dim3 grid) -> int {
-        if (const int er = ensure_dyn_smem(kern, ssm, seen)) return er;
-        kern<<<grid, sthreads, ssm, st>>>(rb, a, C);
+        const size_t bytes = (long long)grid.x * grid.y * grid.z <= tc_device_sms() ? std::max<size_t>(ssm, 116 * 1024) : ssm;
+        if (const int er = ensure_dyn_smem(kern, bytes, seen)) return er;
+        go(kern, grid, sthreads, bytes, st, rb, a, C);
         return last_err();
     };
     auto scan = [&](auto k4, auto k8, auto k16, auto k32, SmemOptIn* seen, dim3 grid) -> int {
@@ -1395,18 +1478,18 @@ int mamba2_mixer_launch(cudaStream_t st, const RaggedBatch& rb, const Mamba2Args
     } else if (!segs) {
         if ((e = scan(ssd_scan_kernel<4, 0>, ssd_scan_kernel<8, 0>, ssd_scan_kernel<16, 0>, ssd_scan_kernel<32, 0>, seen0, sgrid))) return e;
     } else {
-        const dim3 ggrid(rb.E * SSD_SEGS, a.heads, sgrid.z);
+        const dim3 ggrid(sgrid.x, sgrid.y, rb.E * SSD_SEGS);
         if ((e = scan(ssd_scan_kernel<4, 1>, ssd_scan_kernel<8, 1>, ssd_scan_kernel<16, 1>, ssd_scan_kernel<32, 1>, seen1, ggrid))) return e;
-        ssd_seg_prefix_kernel<<<dim3(rb.E, a.heads, std::min(32, (a.N * a.P + 255) / 256)), 256, 0, st>>>(rb, a);
+        go(ssd_seg_prefix_kernel, dim3(rb.E, a.heads, std::min(32, (a.N * a.P + 255) / 256)), 256, 0, st, rb, a);
         if ((e = last_err())) return e;
         if ((e = scan(ssd_scan_kernel<4, 2>, ssd_scan_kernel<8, 2>, ssd_scan_kernel<16, 2>, ssd_scan_kernel<32, 2>, seen2, ggrid))) return e;
     }
     if ((e = last_err())) return e;
-    gated_group_rms_kernel<<<dim3(rb.T, a.norm_groups), 128, 0, st>>>(a);
+    go(gated_group_rms_kernel, dim3(rb.T, a.norm_groups), 128, 0, st, a);
     return last_err();
 }
 int clamped_glu_launch(cudaStream_t st, const float* gu, int ld, int stride, int up_off, int T, int F, float limit, const ActOut& out) {
-    clamped_glu_kernel<<<dim3((F + 127) / 128, T), 128, 0, st>>>(gu, ld, stride, up_off, F, limit, out);
+    go(clamped_glu_kernel, dim3((F + 127) / 128, T), 128, 0, st, gu, ld, stride, up_off, F, limit, out);
     return last_err();
 }
 static bool moe_few_pairs(const MoeArgs& a) {
@@ -1417,41 +1500,41 @@ int moe_route_launch(cudaStream_t st, const MoeArgs& a, const bf16* w_router, in
     if (a.n_groups > 1 && (a.E % a.n_groups || a.keep < 1 || a.keep > a.n_groups || a.top > a.keep * (a.E / a.n_groups))) return -1000;
     int e;
     if (a.T <= 64) {          // few rows: logits + selection in one launch
-        route_rows_kernel<<<a.T, 256, 0, st>>>(a, w_router, ldw);
+        go(route_rows_kernel, a.T, 256, 0, st, a, w_router, ldw);
         e = last_err();
     } else {
-        router_logits_kernel<<<(a.T + 7) / 8, 256, 0, st>>>(a, w_router, ldw);
+        go(router_logits_kernel, (a.T + 7) / 8, 256, 0, st, a, w_router, ldw);
         if ((e = last_err())) return e;
-        route_kernel<<<(a.T + 3) / 4, 128, 0, st>>>(a);
+        go(route_kernel, (a.T + 3) / 4, 128, 0, st, a);
         e = last_err();
     }
     if (e || moe_few_pairs(a)) return e;                  // (a handful of pairs go through moe_gemv, which reads the choices as they are)
-    moe_sort_kernel<<<1, 1024, (size_t)3 * a.E * sizeof(int), st>>>(a);
+    go(moe_sort_kernel, 1, 1024, (size_t)3 * a.E * sizeof(int), st, a);
     return last_err();
 }
 int moe_experts_launch(cudaStream_t st, const MoeArgs& a) {
     if (moe_few_pairs(a)) {
-        moe_gemv_kernel<true><<<dim3(((a.gated ? 2 * a.F : a.F) + 15) / 16, a.T * a.top), 256, (size_t)a.ldwu * 4, st>>>(a);
+        go(moe_gemv_kernel<true>, dim3(((a.gated ? 2 * a.F : a.F) + 15) / 16, a.T * a.top), 256, (size_t)a.ldwu * 4, st, a);
         int e = last_err();
         if (e) return e;
-        moe_gemv_kernel<false><<<dim3((a.W + 15) / 16, a.T * a.top), 256, (size_t)a.ldwd * 4, st>>>(a);
+        go(moe_gemv_kernel<false>, dim3((a.W + 15) / 16, a.T * a.top), 256, (size_t)a.ldwd * 4, st, a);
         if ((e = last_err())) return e;
         return moe_combine_launch(st, a, false);
     }
-    moe_linear_kernel<true><<<dim3(((a.gated ? 2 * a.F : a.F) + 63) / 64, a.max_tiles), 256, 0, st>>>(a);
+    go(moe_linear_kernel<true>, dim3(((a.gated ? 2 * a.F : a.F) + 63) / 64, a.max_tiles), 256, 0, st, a);
     int e = last_err();
     if (e) return e;
-    moe_linear_kernel<false><<<dim3((a.W + 63) / 64, a.max_tiles), 256, 0, st>>>(a);
+    go(moe_linear_kernel<false>, dim3((a.W + 63) / 64, a.max_tiles), 256, 0, st, a);
     if ((e = last_err())) return e;
     return moe_combine_launch(st, a, false);
 }
 int moe_gather_launch(cudaStream_t st, const MoeArgs& a, const ActOut& src, const ActOut& dst) {
     if (!src.hi || !dst.hi || src.ldb != dst.ldb || (src.ldb & 7)) return -1000;
-    moe_gather_kernel<<<a.T * a.top, 128, 0, st>>>(a, src, dst);
+    go(moe_gather_kernel, a.T * a.top, 128, 0, st, a, src, dst);
     return last_err();
 }
 int moe_combine_launch(cudaStream_t st, const MoeArgs& a, bool y_sorted) {
-    moe_combine_kernel<<<dim3((a.W + 127) / 128, a.T), 128, 0, st>>>(a, y_sorted ? 1 : 0);
+    go(moe_combine_kernel, dim3((a.W + 127) / 128, a.T), 128, 0, st, a, y_sorted ? 1 : 0);
     return last_err();
 }
 

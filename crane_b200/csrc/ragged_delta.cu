@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(DR_COLS * DR_NS) delta_scan_kernel(RaggedBatch
     const int d = a.d, dv = a.dv, H = a.H, Hk = a.Hk, hk = h / (H / Hk), DPD = dr_pad(R), PT = NV * DPD + DR_COLS + 4;
     const bool live = p < dv;
     const int len = rb.ent_len[e], slot = rb.ent_slot[e], r0 = rb.ent_row0[e], ncol = min(DR_COLS, dv - p0), n0 = ns * R;
-    float* stage[2] = {sm, sm + DR_CH * PT};
+    auto stage = [&](int c) { return sm + (c & 1) * DR_CH * PT; };      // (computed: out of an array of pointers the reads are generic ones)
     float* sy = sm + 2 * DR_CH * PT;                          // [CH][COLS]
     for (int i = threadIdx.x; i < 2 * DR_CH * PT; i += blockDim.x) sm[i] = 0.f;       // rows past d, columns past dv stay zero
     float* S = a.state + ((size_t)slot * H + h) * d * dv + (live ? p : 0);
@@ -188,12 +188,12 @@ __global__ void __launch_bounds__(DR_COLS * DR_NS) delta_scan_kernel(RaggedBatch
         }
     };
     const int nch = (len + DR_CH - 1) / DR_CH;
-    fetch(0, stage[0]);
+    fetch(0, stage(0));
     for (int ch = 0; ch < nch; ++ch) {
-        if (ch + 1 < nch) { fetch(ch + 1, stage[(ch + 1) & 1]); asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+        if (ch + 1 < nch) { fetch(ch + 1, stage(ch + 1)); asm volatile("cp.async.wait_group 1;" ::: "memory"); }
         else asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
-        const float* st = stage[ch & 1];
+        const float* st = stage(ch);
         const int nt = min(DR_CH, len - ch * DR_CH);
         for (int tg = 0; tg < nt; tg += 4) {
             float o[4];

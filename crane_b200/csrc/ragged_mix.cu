@@ -486,7 +486,7 @@ __global__ void __launch_bounds__(GLA_COLS * GLA_NS) gla_scan_kernel(RaggedBatch
     const int len = min(seg_len, full_len - seg0), r0 = rb.ent_row0[e] + seg0;
     const int ncol = min(GLA_COLS, dv - p0);
     const int NP = gla_npad(R), per_tok = GLA_COLS + 3 * NP;
-    float* stage[2] = {gla_s, gla_s + GLA_CH * per_tok};
+    auto stage = [&](int c) { return gla_s + (c & 1) * GLA_CH * per_tok; };      // (computed: out of an array of pointers the reads are generic ones)
     float* S = MODE == 0 ? a.state + (((size_t)slot * a.H + h) * d) * dv : a.seg_state + ((((size_t)e * GLA_SEGS + seg) * a.H + h) * d) * dv;
     const int n0 = ns * R;
     for (int i = threadIdx.x; i < 2 * GLA_CH * per_tok; i += blockDim.x) gla_s[i] = 0.f;
@@ -538,12 +538,12 @@ __global__ void __launch_bounds__(GLA_COLS * GLA_NS) gla_scan_kernel(RaggedBatch
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     const int nch = (len + GLA_CH - 1) / GLA_CH;
-    fetch(0, stage[0]);
+    fetch(0, stage(0));
     for (int c = 0; c < nch; ++c) {
-        if (c + 1 < nch) { fetch(c + 1, stage[(c + 1) & 1]); asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+        if (c + 1 < nch) { fetch(c + 1, stage(c + 1)); asm volatile("cp.async.wait_group 1;" ::: "memory"); }
         else asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
-        const float* st = stage[c & 1];
+        const float* st = stage(c);
         const int nt = min(GLA_CH, len - c * GLA_CH);
         for (int t = 0; t < nt; ++t) {
             const float* tk = st + t * per_tok;

@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(SC_COLS * SC_NS) mamba1_scan_kernel(RaggedBatc
     const bool last_seg = seg0 + seg_len >= full_len;
     if (MODE == 1 && last_seg) return;                        // nothing follows the last segment: its end state is MODE 2's to leave
     const int len = min(seg_len, full_len - seg0), r0 = rb.ent_row0[e] + seg0;
-    float* stage[2] = {sm, sm + SC_CH * PT};
+    auto stage = [&](int c) { return sm + (c & 1) * SC_CH * PT; };      // (computed: out of an array of pointers the reads are generic ones)
     float* sy = sm + 2 * SC_CH * PT;                                    // [CH][COLS]
     const int n0 = ns * R, ncol = min(SC_COLS, a.inner - c0);
     for (int i = threadIdx.x; i < 2 * SC_CH * PT; i += blockDim.x) sm[i] = 0.f;       // entries past N, channels past the last stay zero
@@ -138,12 +138,12 @@ __global__ void __launch_bounds__(SC_COLS * SC_NS) mamba1_scan_kernel(RaggedBatc
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     const int nch = (len + SC_CH - 1) / SC_CH;
-    fetch(0, stage[0]);
+    fetch(0, stage(0));
     for (int ch = 0; ch < nch; ++ch) {
-        if (ch + 1 < nch) { fetch(ch + 1, stage[(ch + 1) & 1]); asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+        if (ch + 1 < nch) { fetch(ch + 1, stage(ch + 1)); asm volatile("cp.async.wait_group 1;" ::: "memory"); }
         else asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
-        const float* st = stage[ch & 1];
+        const float* st = stage(ch);
         const int nt = min(SC_CH, len - ch * SC_CH);
         const int tmax = (nt + 3) & ~3;                       // whole groups of four: a token past the end leaves the state as it is
 #pragma unroll 4
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(SC_COLS * SC_NS) mlstm_scan_kernel(RaggedBatch
     const bool last_seg = seg0 + seg_len >= full_len;
     if (MODE == 1 && last_seg) return;                        // nothing follows the last segment: its end state is MODE 2's to leave
     const int len = min(seg_len, full_len - seg0), r0 = rb.ent_row0[e] + seg0;
-    float* stage[2] = {sm, sm + SC_CH * PT};
+    auto stage = [&](int c) { return sm + (c & 1) * SC_CH * PT; };      // (computed: out of an array of pointers the reads are generic ones)
     float* sy = sm + 2 * SC_CH * PT;                        // [CH][COLS]
     for (int i = threadIdx.x; i < 2 * SC_CH * PT; i += blockDim.x) sm[i] = 0.f;        // rows past d and columns past dv stay zero
     const int n0 = ns * R;
@@ -316,12 +316,12 @@ __global__ void __launch_bounds__(SC_COLS * SC_NS) mlstm_scan_kernel(RaggedBatch
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     const int nch = (len + SC_CH - 1) / SC_CH;
-    fetch(0, stage[0]);
+    fetch(0, stage(0));
     for (int ch = 0; ch < nch; ++ch) {
-        if (ch + 1 < nch) { fetch(ch + 1, stage[(ch + 1) & 1]); asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+        if (ch + 1 < nch) { fetch(ch + 1, stage(ch + 1)); asm volatile("cp.async.wait_group 1;" ::: "memory"); }
         else asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
-        const float* st = stage[ch & 1];
+        const float* st = stage(ch);
         const int nt = min(SC_CH, len - ch * SC_CH);
         const int tmax = (nt + 3) & ~3;                       // whole groups of four: a token past the end leaves the memory as it is
 #pragma unroll 4
