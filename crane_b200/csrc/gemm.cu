@@ -8,7 +8,7 @@
 
 namespace cb {
 
-// CRANE_B200_GEMM_BN=64|128|256 pins the tile width (sweeps).  (Clusters of 2 x 2 that share their loads
+// CRANE_B200_GEMM_BN=64|128|256 pins the tile width, 512 the tiles of CTA pairs (sweeps).  (Clusters of 2 x 2 that share their loads
 // did not pay on B200: the L2 already merges concurrent requests for a line from a few CTAs.)
 static const int g_gemm_bn = [] { const char* e = getenv("CRANE_B200_GEMM_BN"); return e ? atoi(e) : 0; }();
 
@@ -226,6 +226,93 @@ struct GemmCfg {
     static constexpr int TMEM_COLS = 2 * BN;
 };
 
+// What the epilogue warps do with the accumulators of a CTA's segments.  `cta`: the CTA's place in the schedule, with PER = 2 the pair's, of which this is CTA `rank`;
+// every CTA has 128 rows of a tile, partial tiles and counters of its own.
+template <int MODE, int BN, int PER, typename Ready, typename Drained>
+__device__ __forceinline__ void gemm_epilogue(const GemmEpi& ep, const CUtensorMap& tmO, const CUtensorMap& tmOlo, EpiPatch& patch, uint8_t* ring, int M, int N, const TcSched& sc, int cta,
+                                              int rank, int it_begin, int it_end, uint32_t tmem_base, uint64_t* tmem_full_bar, const TcWait& wait, int* last_flag, int q, int part,
+                                              int lane, Ready&& first_ready, Drained&& drained) {
+    const int KB = sc.KB;
+    constexpr int CHUNKS = BN / 32;
+    constexpr size_t TILE_F = (size_t)GEMM_BM * BN;
+    int seg = 0;
+    for (int it = it_begin; it < it_end; ++seg) {
+        const int seg_end = min(it_end, (it / KB + 1) * KB);
+        const int t = it / KB, kb0 = it % KB, kb1 = kb0 + (seg_end - it);
+        const int m0 = ((t % sc.tiles_m) * PER + rank) * GEMM_BM + q * 32, n0 = (t / sc.tiles_m) * BN;
+        const int b = seg & 1;
+        const uint32_t acc = tmem_base + (uint32_t)(b * BN) + ((uint32_t)(q * 32) << 16);
+        const bool sole = kb0 == 0 && kb1 == KB;
+        const int c_first = sched_owner(sc, t * KB), c_last = sched_owner(sc, t * KB + KB - 1);
+        // a shared tile whose other contributors have all arrived already is finished without parking this part (read while the MMAs run)
+        if (!sole && threadIdx.x == 128) *last_flag = ld_acquire(&sc.counters[t * PER + rank]) == c_last - c_first;
+        wait(&tmem_full_bar[b], (seg >> 1) & 1);
+        tc_fence_after();
+        if (threadIdx.x == 128 && seg == 0) first_ready();
+        bool finish = sole;
+        if (!sole) {
+            named_bar_sync(1, 32 * EPI_WARPS);
+            finish = *last_flag;
+            if (!finish) {
+                // park it.  A 32 x 32 block of (row = lane, column j) is stored as 8 rows of 32 float4: the float4
+                // of lane l in row k holds columns 4k .. 4k+3 of row l, so every store / reload instruction moves 512 contiguous bytes
+                float* mine = sc.ws + (size_t)((2 * cta + (it == it_begin ? 0 : 1)) * PER + rank) * TILE_F + (size_t)q * CHUNKS * 1024;
+#pragma unroll 1
+                for (int c = part; c < CHUNKS; c += EPI_WARPS / 4) {
+                    uint32_t r[32];
+                    tmem_ld32(acc + (uint32_t)(c * 32), r);
+                    float4* dst = reinterpret_cast<float4*>(mine + c * 1024) + lane;
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)
+                        dst[k * 32] = make_float4(__uint_as_float(r[4 * k]), __uint_as_float(r[4 * k + 1]), __uint_as_float(r[4 * k + 2]), __uint_as_float(r[4 * k + 3]));
+                }
+                // arrive at the tile; the last of its contributors finishes it
+                __threadfence();
+                named_bar_sync(1, 32 * EPI_WARPS);
+                if (threadIdx.x == 128) *last_flag = atomicAdd(&sc.counters[t * PER + rank], 1) == c_last - c_first;
+                named_bar_sync(1, 32 * EPI_WARPS);
+                finish = *last_flag;
+            }
+            if (finish) {
+                __threadfence();
+                if (threadIdx.x == 128) sc.counters[t * PER + rank] = 0;       // clean for the next launch on this stream
+            }
+        }
+        if (seg_end == it_end) { patch.base = ring; patch.ring = true; }      // every MMA of this CTA has read its operands
+        if (finish && m0 < M)
+            epi_rows<MODE, BN>(ep, tmO, tmOlo, patch, m0, M, n0, N, part, lane, [&](int c, float* v) {
+                tmem_ld32(acc + (uint32_t)(c * 32), reinterpret_cast<uint32_t*>(v));
+                if (sole) return;
+                // a shared tile: contributor order, whoever came last
+                float sum[32];
+#pragma unroll
+                for (int j = 0; j < 32; ++j) sum[j] = 0.f;
+#pragma unroll 1
+                for (int cc = c_first; cc <= c_last; ++cc) {
+                    if (cc == cta) {
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) sum[j] += v[j];
+                        continue;
+                    }
+                    const float4* p = reinterpret_cast<const float4*>(sc.ws + (size_t)((2 * cc + (sched_start(sc, cc) < t * KB ? 1 : 0)) * PER + rank) * TILE_F +
+                                                                      (size_t)(q * CHUNKS + c) * 1024) + lane;
+                    float4 x[8];
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) x[k] = __ldcg(p + k * 32);
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) { sum[4 * k] += x[k].x; sum[4 * k + 1] += x[k].y; sum[4 * k + 2] += x[k].z; sum[4 * k + 3] += x[k].w; }
+                }
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] = sum[j];
+            });
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) drained(b);
+        if (!sole) named_bar_sync(1, 32 * EPI_WARPS);             // last_flag is rewritten by the next segment
+        it = seg_end;
+    }
+}
+
 // SPLIT: the activation operand comes as two bf16 planes A = hi + lo (lo = bf16(x - hi), ~16 mantissa bits together); the
 // weight tile is fetched once and multiplied by both, accumulating into the same TMEM columns: D = hi.W^T + lo.W^T.
 // (Bounds: 384 threads, but no more registers than 512 would leave each: the row kernels beside a linear need some too.)
@@ -350,84 +437,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         pdl_wait();                                 // the epilogue reads / overwrites activations of the predecessor too
         const int q = warp & 3, part = (warp - 4) >> 2;
         EpiPatch patch{epi_smem + (warp - 4) * EPI_PATCH, false};
-        constexpr int CHUNKS = BN / 32;
-        constexpr size_t TILE_F = (size_t)GEMM_BM * BN;
-        int seg = 0;
-        for (int it = it_begin; it < it_end; ++seg) {
-            const int seg_end = min(it_end, (it / KB + 1) * KB);
-            const int t = it / KB, kb0 = it % KB, kb1 = kb0 + (seg_end - it);
-            const int m0 = (t % sc.tiles_m) * GEMM_BM + q * 32, n0 = (t / sc.tiles_m) * BN;
-            const int b = seg & 1;
-            const uint32_t acc = tmem_base + (uint32_t)(b * BN) + ((uint32_t)(q * 32) << 16);
-            const bool sole = kb0 == 0 && kb1 == KB;
-            const int c_first = sched_owner(sc, t * KB), c_last = sched_owner(sc, t * KB + KB - 1);
-            // a shared tile whose other contributors have all arrived already is finished without parking this part (read while the MMAs run)
-            if (!sole && threadIdx.x == 128) *last_flag = ld_acquire(&sc.counters[t]) == c_last - c_first;
-            wait(&tmem_full_bar[b], (seg >> 1) & 1);
-            tc_fence_after();
-            if (threadIdx.x == 128 && seg == 0) stamp(4);   // first accumulator ready
-            bool finish = sole;
-            if (!sole) {
-                named_bar_sync(1, 32 * EPI_WARPS);
-                finish = *last_flag;
-                if (!finish) {
-                    // park it.  A 32 x 32 block of (row = lane, column j) is stored as 8 rows of 32 float4: the float4
-                    // of lane l in row k holds columns 4k .. 4k+3 of row l, so every store / reload instruction moves 512 contiguous bytes
-                    float* mine = sc.ws + (size_t)(2 * cta + (it == it_begin ? 0 : 1)) * TILE_F + (size_t)q * CHUNKS * 1024;
-#pragma unroll 1
-                    for (int c = part; c < CHUNKS; c += EPI_WARPS / 4) {
-                        uint32_t r[32];
-                        tmem_ld32(acc + (uint32_t)(c * 32), r);
-                        float4* dst = reinterpret_cast<float4*>(mine + c * 1024) + lane;
-#pragma unroll
-                        for (int k = 0; k < 8; ++k)
-                            dst[k * 32] = make_float4(__uint_as_float(r[4 * k]), __uint_as_float(r[4 * k + 1]), __uint_as_float(r[4 * k + 2]), __uint_as_float(r[4 * k + 3]));
-                    }
-                    // arrive at the tile; the last of its contributors finishes it
-                    __threadfence();
-                    named_bar_sync(1, 32 * EPI_WARPS);
-                    if (threadIdx.x == 128) *last_flag = atomicAdd(&sc.counters[t], 1) == c_last - c_first;
-                    named_bar_sync(1, 32 * EPI_WARPS);
-                    finish = *last_flag;
-                }
-                if (finish) {
-                    __threadfence();
-                    if (threadIdx.x == 128) sc.counters[t] = 0;       // clean for the next launch on this stream
-                }
-            }
-            if (seg_end == it_end) { patch.base = smem + (warp - 4) * 4 * EPI_PATCH; patch.ring = true; }      // every MMA of this CTA has read its operands
-            if (finish && m0 < M)
-                epi_rows<MODE, BN>(ep, tmO, tmOlo, patch, m0, M, n0, N, part, lane, [&](int c, float* v) {
-                    tmem_ld32(acc + (uint32_t)(c * 32), reinterpret_cast<uint32_t*>(v));
-                    if (sole) return;
-                    // a shared tile: contributor order, whoever came last
-                    float sum[32];
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) sum[j] = 0.f;
-#pragma unroll 1
-                    for (int cc = c_first; cc <= c_last; ++cc) {
-                        if (cc == cta) {
-#pragma unroll
-                            for (int j = 0; j < 32; ++j) sum[j] += v[j];
-                            continue;
-                        }
-                        const float4* p = reinterpret_cast<const float4*>(sc.ws + (size_t)(2 * cc + (sched_start(sc, cc) < t * KB ? 1 : 0)) * TILE_F +
-                                                                          (size_t)(q * CHUNKS + c) * 1024) + lane;
-                        float4 x[8];
-#pragma unroll
-                        for (int k = 0; k < 8; ++k) x[k] = __ldcg(p + k * 32);
-#pragma unroll
-                        for (int k = 0; k < 8; ++k) { sum[4 * k] += x[k].x; sum[4 * k + 1] += x[k].y; sum[4 * k + 2] += x[k].z; sum[4 * k + 3] += x[k].w; }
-                    }
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) v[j] = sum[j];
-                });
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&tmem_empty_bar[b]);
-            if (!sole) named_bar_sync(1, 32 * EPI_WARPS);             // last_flag is rewritten by the next segment
-            it = seg_end;
-        }
+        gemm_epilogue<MODE, BN, 1>(ep, tmO, tmOlo, patch, smem + (warp - 4) * 4 * EPI_PATCH, M, N, sc, cta, 0, it_begin, it_end, tmem_base, tmem_full_bar, wait, last_flag, q, part, lane,
+                                   [&] { stamp(4); }, [&](int b) { mbar_arrive(&tmem_empty_bar[b]); });      // (stamp: first accumulator ready)
         if (lane == 0) tma_store_wait_read<0>();        // (the writes themselves are complete when the grid is)
         if (threadIdx.x == 128) stamp(5);               // this CTA's rows stored
     }
@@ -435,6 +446,146 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     __syncthreads();
     if (threadIdx.x == 0) stamp(6);                 // whole CTA done
     if (warp == 2) { tc_fence_after(); tmem_dealloc(tmem_base, Cfg::TMEM_COLS); if (lane == 0) stamp(7); }
+}
+
+// =====================================================================================
+// The same over pairs of CTAs: a tile is 256 x 256, each CTA has 128 of its rows, loads its own rows of A and HALF of the weight rows, and the even CTA issues
+// tcgen05.mma.cta_group::2 for both, which reads either half from where it lies.  An SM takes in about 64 bytes a cycle: a 64-wide k-step of a 128 x 256 tile brings 48 KB
+// (plain bf16) for 512 cycles of MMAs, 64 KB (two planes) for 1024; half of the weights' 32 KB comes off that here.
+// One schedule over pairs ("cta" of TcSched); epilogue, parking and fix-up are each CTA's own, for its 128 rows: counters and partial tiles are per CTA.
+// =====================================================================================
+template <bool SPLIT>
+struct Gemm2Cfg {
+    static constexpr int BN = 256;
+    static constexpr int A_BYTES = GEMM_BM * GEMM_BK * 2;
+    static constexpr int B_BYTES = BN / 2 * GEMM_BK * 2;
+    static constexpr int STAGE_BYTES = A_BYTES * (SPLIT ? 2 : 1) + B_BYTES;     // [A hi | A lo (SPLIT) | half of B]
+    static constexpr int STAGES = GEMM_STAGE_BUDGET / STAGE_BYTES;
+    static constexpr int EPI_BYTES = EPI_WARPS * EPI_PATCH;
+    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_BYTES + 1024 /*align*/ + 256 /*barriers*/;
+    static_assert((2 * STAGES + 4) * 8 + 12 <= 256, "barrier area");
+};
+template <int MODE, bool SPLIT>
+__global__ void __launch_bounds__(512, 1) __cluster_dims__(2, 1, 1)
+gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmAlo, const __grid_constant__ CUtensorMap tmB,
+                const __grid_constant__ CUtensorMap tmO, const __grid_constant__ CUtensorMap tmOlo, GemmEpi ep, int M, int N, int K, TcSched sc, int* err) {
+    using Cfg = Gemm2Cfg<SPLIT>;
+    constexpr int STAGES = Cfg::STAGES, BN = Cfg::BN;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t* epi_smem = smem + STAGES * Cfg::STAGE_BYTES;
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(epi_smem + Cfg::EPI_BYTES);      // of the even CTA: both CTAs' operands of a stage
+    uint64_t* empty_bar = full_bar + STAGES;           // of each CTA
+    uint64_t* tmem_full_bar = empty_bar + STAGES;      // [2] of each CTA: accumulator b complete
+    uint64_t* tmem_empty_bar = tmem_full_bar + 2;      // [2] of the even CTA: accumulator b drained by the epilogue warps of both
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty_bar + 2);
+    int* last_flag = reinterpret_cast<int*>(tmem_slot + 1);
+    int* gave_up = last_flag + 1;
+    const TcWait wait{gave_up, err};
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = (int)cluster_rank(), pair = blockIdx.x >> 1;
+    const int KB = sc.KB;
+    const int it_begin = sched_start(sc, pair), it_end = sched_start(sc, pair + 1);
+
+    if (warp == 0 && lane == 0) {
+        tma_prefetch_desc(&tmA);
+        if (SPLIT) tma_prefetch_desc(&tmAlo);
+        tma_prefetch_desc(&tmB);
+        for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+        for (int b = 0; b < 2; ++b) { mbar_init(&tmem_full_bar[b], 1); mbar_init(&tmem_empty_bar[b], 2 * EPI_WARPS); }
+        *gave_up = 0;
+        fence_barrier_init();
+    }
+    if (warp == 2) { tmem_alloc_pair(tmem_slot, 2 * BN); tmem_relinquish_pair(); }
+    tc_fence_before();
+    __syncthreads();
+    __syncwarp();
+    cluster_sync_all();                             // the pair's barriers are initialised before either CTA signals the other's
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    pdl_launch_dependents();
+    if (warp == 0) {
+        if (lane == 0) {
+            constexpr int B_OFF = Cfg::A_BYTES * (SPLIT ? 2 : 1);
+            const int npre = ep.w_dynamic ? 0 : min(it_end - it_begin, STAGES);
+            int t = it_begin / KB, kb = it_begin - t * KB, n0 = t / sc.tiles_m * BN + rank * (BN / 2);
+            for (int i = 0; i < npre; ++i) {        // the weights' first tiles go out before the dependency wait
+                if (rank == 0) mbar_arrive_expect_tx(&full_bar[i], 2 * Cfg::STAGE_BYTES);
+                tma_load_2d_pair(smem + i * Cfg::STAGE_BYTES + B_OFF, &tmB, peer_smem(&full_bar[i], 0), kb * GEMM_BK, n0);
+                if (++kb == KB) { kb = 0; ++t; n0 = t / sc.tiles_m * BN + rank * (BN / 2); }
+            }
+            pdl_wait();
+            int s = 0, left = npre; uint32_t ph = 0;
+            for (int it = it_begin; it < it_end;) {
+                t = it / KB;
+                const int seg_end = min(it_end, (t + 1) * KB), nt = t / sc.tiles_m, m0 = (t - nt * sc.tiles_m) * (2 * GEMM_BM) + rank * GEMM_BM;
+                n0 = nt * BN + rank * (BN / 2);
+                int kc = (it - t * KB) * GEMM_BK;
+                for (; it < seg_end; ++it, kc += GEMM_BK) {
+                    uint8_t* a_dst = smem + s * Cfg::STAGE_BYTES;
+                    const uint32_t bar = peer_smem(&full_bar[s], 0);
+                    if (left > 0) --left;
+                    else {
+                        wait(&empty_bar[s], ph ^ 1);
+                        if (rank == 0) mbar_arrive_expect_tx(&full_bar[s], 2 * Cfg::STAGE_BYTES);
+                        tma_load_2d_pair(a_dst + B_OFF, &tmB, bar, kc, n0);
+                    }
+                    tma_load_2d_pair(a_dst, &tmA, bar, kc, m0);
+                    if (SPLIT) tma_load_2d_pair(a_dst + Cfg::A_BYTES, &tmAlo, bar, kc, m0);
+                    if (++s == STAGES) { s = 0; ph ^= 1; }
+                }
+            }
+            wait.drain();
+        }
+    } else if (warp == 1) {
+        if (rank == 0) {
+            constexpr uint32_t idesc = make_idesc_bf16(2 * GEMM_BM, BN);
+            int s = 0; uint32_t ph = 0;
+            int seg = 0;
+            for (int it = it_begin; it < it_end; ++seg) {
+                const int seg_end = min(it_end, (it / KB + 1) * KB);
+                const int b = seg & 1;
+                wait(&tmem_empty_bar[b], ((seg >> 1) & 1) ^ 1);       // both epilogues have drained this accumulator (first two: free)
+                tc_fence_after();
+                const uint32_t acc = tmem_base + (uint32_t)(b * BN);
+                for (int i = it; i < seg_end; ++i) {
+                    wait(&full_bar[s], ph);
+                    tc_fence_after();
+                    const uint32_t a_addr = smem_u32(smem + s * Cfg::STAGE_BYTES);
+                    const uint64_t adesc = make_smem_desc_sw128(a_addr);
+                    const uint64_t aldesc = make_smem_desc_sw128(a_addr + Cfg::A_BYTES);
+                    const uint64_t bdesc = make_smem_desc_sw128(a_addr + Cfg::A_BYTES * (SPLIT ? 2 : 1));
+                    if (elect_one()) {
+#pragma unroll
+                        for (int k = 0; k < GEMM_BK / 16; ++k) {
+                            umma_bf16_pair(acc, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc, (uint32_t)((i != it) | (k != 0)));
+                            if (SPLIT) umma_bf16_pair(acc, aldesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc, 1u);
+                        }
+                        umma_commit_pair(&empty_bar[s]);
+                        if (i == seg_end - 1) umma_commit_pair(&tmem_full_bar[b]);
+                    }
+                    __syncwarp();
+                    if (++s == STAGES) { s = 0; ph ^= 1; }
+                }
+                it = seg_end;
+            }
+        }
+    } else if (warp >= 4) {
+        if (threadIdx.x == 128) { tma_prefetch_desc(&tmO); tma_prefetch_desc(&tmOlo); }
+        pdl_wait();
+        const int q = warp & 3, part = (warp - 4) >> 2;
+        EpiPatch patch{epi_smem + (warp - 4) * EPI_PATCH, false};
+        gemm_epilogue<MODE, BN, 2>(ep, tmO, tmOlo, patch, smem + (warp - 4) * 4 * EPI_PATCH, M, N, sc, pair, rank, it_begin, it_end, tmem_base, tmem_full_bar, wait, last_flag, q, part, lane,
+                                   [] {}, [&](int b) { mbar_arrive_peer(peer_smem(&tmem_empty_bar[b], 0)); });
+        if (lane == 0) tma_store_wait_read<0>();
+    }
+    tc_fence_before();
+    __syncthreads();
+    __syncwarp();
+    cluster_sync_all();                             // neither CTA leaves while the other's MMAs read its operands or its warps signal here
+    if (warp == 2) { tc_fence_after(); tmem_dealloc_pair(tmem_base, 2 * BN); }
 }
 
 // =====================================================================================
@@ -483,6 +634,17 @@ gemm_simt_kernel(const bf16* __restrict__ A, const bf16* __restrict__ A_lo, int 
 // parking and re-reading partial tiles -- outweighs the parallelism)
 static const int g_gemm_minit = [] { const char* e = getenv("CRANE_B200_GEMM_MINIT"); const int v = e ? atoi(e) : 0; return v > 0 ? v : 8; }();
 
+// maps of the results: patches of 32 rows (see epi_rows)
+template <int MODE>
+static bool out_maps(const GemmEpi& epi, int M, int N, CUtensorMap* tmO, CUtensorMap* tmOlo) {
+    constexpr bool F32 = MODE == EPI_STORE_F32 || MODE == EPI_RESID_F32, GLU = MODE == EPI_SILU_MUL_BF16;
+    const uint64_t out_cols = GLU ? N / 2 : N;
+    const CUtensorMapDataType ot = F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+    constexpr CUtensorMapSwizzle osw = GLU ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B;
+    return tc_tmap(tmO, epi.out, ot, (uint64_t)M, out_cols, (uint64_t)epi.ldo, 32, F32 || GLU ? 16 : 32, osw) &&
+           tc_tmap(tmOlo, !F32 && epi.out_lo ? epi.out_lo : epi.out, ot, (uint64_t)M, out_cols, (uint64_t)epi.ldo, 32, F32 || GLU ? 16 : 32, osw);
+}
+
 template <int BN, int MODE, bool SPLIT>
 static int launch_tc(cudaStream_t stream, const bf16* A, const bf16* A_lo, int lda, const bf16* W, int M, int N, int K, const GemmEpi& epi,
                      bool stream_k) {
@@ -491,14 +653,8 @@ static int launch_tc(cudaStream_t stream, const bf16* A, const bf16* A_lo, int l
     if (!tc_tmap_bf16(&tmA, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, GEMM_BM)) return -1001;
     if (!tc_tmap_bf16(&tmAlo, SPLIT ? A_lo : A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, GEMM_BM)) return -1001;
     if (!tc_tmap_bf16(&tmB, W, (uint64_t)N, (uint64_t)K, (uint64_t)K, BN)) return -1001;
-    constexpr bool F32 = MODE == EPI_STORE_F32 || MODE == EPI_RESID_F32;
     CUtensorMap tmO, tmOlo;
-    const uint64_t out_cols = MODE == EPI_SILU_MUL_BF16 ? N / 2 : N;
-    const CUtensorMapDataType ot = F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-    constexpr bool GLU = MODE == EPI_SILU_MUL_BF16;
-    constexpr CUtensorMapSwizzle osw = GLU ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B;
-    if (!tc_tmap(&tmO, epi.out, ot, (uint64_t)M, out_cols, (uint64_t)epi.ldo, 32, F32 || GLU ? 16 : 32, osw)) return -1001;
-    if (!tc_tmap(&tmOlo, !F32 && epi.out_lo ? epi.out_lo : epi.out, ot, (uint64_t)M, out_cols, (uint64_t)epi.ldo, 32, F32 || GLU ? 16 : 32, osw)) return -1001;
+    if (!out_maps<MODE>(epi, M, N, &tmO, &tmOlo)) return -1001;
     int* err = nullptr;
     if (const int e = tc_err_word(stream, &err)) return e;
     static SmemOptIn seen;
@@ -538,12 +694,52 @@ static int launch_tc(cudaStream_t stream, const bf16* A, const bf16* A_lo, int l
     return (int)cudaLaunchKernelEx(&cfg, gemm_tc_kernel<BN, MODE, SPLIT>, tmA, tmAlo, tmB, tmO, tmOlo, epi, M, N, K, sc, err);
 }
 
+template <int MODE, bool SPLIT>
+static int launch_tc2(cudaStream_t stream, const bf16* A, const bf16* A_lo, int lda, const bf16* W, int M, int N, int K, const GemmEpi& epi, bool stream_k) {
+    using Cfg = Gemm2Cfg<SPLIT>;
+    CUtensorMap tmA, tmAlo, tmB, tmO, tmOlo;
+    if (!tc_tmap_bf16(&tmA, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, GEMM_BM)) return -1001;
+    if (!tc_tmap_bf16(&tmAlo, SPLIT ? A_lo : A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, GEMM_BM)) return -1001;
+    if (!tc_tmap_bf16(&tmB, W, (uint64_t)N, (uint64_t)K, (uint64_t)K, Cfg::BN / 2)) return -1001;
+    if (!out_maps<MODE>(epi, M, N, &tmO, &tmOlo)) return -1001;
+    int* err = nullptr;
+    if (const int e = tc_err_word(stream, &err)) return e;
+    static SmemOptIn seen;
+    if (const int e = ensure_dyn_smem(gemm_tc2_kernel<MODE, SPLIT>, (size_t)Cfg::SMEM_BYTES, seen)) return e;
+    TcSched sc = {};
+    sc.tiles_m = (M + 2 * GEMM_BM - 1) / (2 * GEMM_BM);
+    sc.tiles_n = (N + Cfg::BN - 1) / Cfg::BN;
+    sc.KB = K / GEMM_BK;
+    const long long tiles = (long long)sc.tiles_m * sc.tiles_n, iters = tiles * sc.KB;
+    if (iters > 0x7fffffffLL) return -1000;
+    const int cap = std::min(tc_max_clusters(2), GEMM_MAX_CTAS / 2);
+    sc.unit = stream_k ? 1 : sc.KB;
+    const long long units = iters / sc.unit;
+    sc.G = (int)std::max<long long>(1, std::min<long long>(cap, stream_k ? iters / g_gemm_minit : tiles));
+    sc.base = (int)(units / sc.G);
+    sc.rem = (int)(units % sc.G);
+    if (sc.unit != sc.KB) {
+        TcScratch scratch;
+        if (const int e = tc_scratch_get(stream, (int)tiles * 2, &scratch)) return e;
+        sc.ws = scratch.ws;
+        sc.counters = scratch.counters;
+    }
+    return launch_k(gemm_tc2_kernel<MODE, SPLIT>, dim3(2 * sc.G), dim3(128 + 32 * EPI_WARPS), Cfg::SMEM_BYTES, stream, prefill_pdl(), tmA, tmAlo, tmB, tmO, tmOlo, epi, M, N, K, sc, err);
+}
+
 // Tile width and schedule from a cost model fitted on B200 (microseconds; 42 shapes of 77 - 4096 rows, every width and schedule):
 //   a k-step costs t_k: 64- and 128-wide tiles wait for their operands, 128 x 256 ones for shared memory, which MMAs read at 96 bytes a cycle while TMA writes
 //   64 (two planes) or 96 (one) into it: 128 is the limit.  (Split, 256 wide, us a step: 0.565 - 0.57 with 24 - 64 tiles at once, 0.57 - 0.58 with 80 - 112, 0.615 with 128 and 144, 0.70
 //   with 148, where the chip's power and the L2 begin to tell; hence 0.565, 0.60 above 96 and 0.66 with every SM busy.)
 //   whole tiles: each CTA runs ceil(tiles / CTAs) tiles, the epilogue of all but the last hidden under the next tile's MMAs;
 //   stream-K:    tiles x k-steps dealt evenly to all SMs, and the last of a tile's c contributors adding the others' parts.
+// Tiles of pairs (256 x 256): a k-step 0.31 us plain and 0.62 split with few tiles, 0.36 and 0.63 with every SM busy on the scale that gives the single tiles 0.42 and 0.66, two or three
+// us more of setup and hand-over.  Worth it where the operands are what takes the time; not where a gated or GELU tile's epilogue does (9 us), nor with rows that fill 256 badly.  Their
+// stream-K pays above one wave too, while all operands stay in the L2 (CTAs at different k-steps share nothing of what they read): 4096 x 12288 at 2048 rows 187 us, whole tiles 141.
+//   us, single / pairs, plain: 24576 x 4096 at 256 rows 78.8 / 55.3, 512 108 / 87, 2048 392 / 327, 4096 822 / 657    6144 x 4096 at 784 64.4 / 44.9, 4096 170 / 142
+//   12288 x 2048 at 784 59.7 / 44.4, 1111 48.4 / 55.3, 4096 152 / 136                                                4096 x 12288 at 512 69.6 / 52.6, 4096 318 / 284
+//   split: 24576 x 4096 at 512 153 / 144, 4096 1204 / 1100    6144 x 4096 at 4096 283 / 263    4096 x 4096 193 / 179    8256 x 1024 103 / 97    7168 x 1024 92 / 88
+constexpr int GEMM_PAIR = 512;          // GemmPlan::bn: 256 x 256 tiles of two CTAs
 struct GemmPlan { int bn; bool stream_k; double cost; };
 static GemmPlan gemm_plan(int mode, int M, int N, int K, bool split, int sms) {
     static const int g_mode = [] { const char* e = getenv("CRANE_B200_GEMM_SCHED"); return e ? atoi(e) : 0; }();   // 1: whole tiles, 2: stream-K
@@ -551,7 +747,7 @@ static GemmPlan gemm_plan(int mode, int M, int N, int K, bool split, int sms) {
     const bool light = mode == EPI_STORE_F32 || mode == EPI_RESID_F32 || mode == EPI_STORE_BF16 || mode == EPI_RELU2_BF16;
     GemmPlan best{64, false, 1e30};
     for (int bn : {256, 128, 64}) {
-        if (g_gemm_bn && bn != g_gemm_bn) continue;
+        if (g_gemm_bn && bn != g_gemm_bn && !(g_gemm_bn == GEMM_PAIR && (M <= GEMM_BM || N < 256))) continue;
         if (!g_gemm_bn && bn > 64 && N < bn) continue;
         const long long tiles = (long long)tm * ((N + bn - 1) / bn);
         const long long per = (tiles + std::min<long long>(tiles, sms) - 1) / std::min<long long>(tiles, sms);
@@ -566,6 +762,19 @@ static GemmPlan gemm_plan(int mode, int M, int N, int K, bool split, int sms) {
         // stream-K only below one wave of whole tiles: above it the extra partial-tile traffic costs more than the idle SMs
         if (g_mode != 1 && (tiles < sms || g_mode == 2) && tiles * KB >= 2LL * sms && sk < best.cost) best = GemmPlan{bn, true, sk};
     }
+    const int pairs = std::min(tc_max_clusters(2), sms / 2);
+    if (pairs > 0 && M > GEMM_BM && N >= 256 && (!g_gemm_bn || g_gemm_bn == GEMM_PAIR)) {
+        const long long tiles = (long long)((M + 255) / 256) * ((N + 255) / 256), per = (tiles + pairs - 1) / pairs;
+        const double tk = split ? (per > 1 ? 0.63 : 0.62) : (per > 1 ? 0.36 : 0.31), fixed = light ? 8.9 : 13.2;
+        if (light || KB * tk >= 9. || g_gemm_bn) {
+            const double whole = fixed + (double)per * KB * tk;
+            if (g_mode != 2 && whole < best.cost) best = GemmPlan{GEMM_PAIR, false, whole};
+            const double it = std::max((double)tiles * KB / pairs, (double)g_gemm_minit);
+            const double sk = fixed + 6. + it * (split ? 0.63 : 0.36) + (KB / it + 1.0) * 2.3;
+            const double operands = 2. * K * ((double)N + (double)M * (split ? 2 : 1));
+            if (g_mode != 1 && operands <= 126e6 && tiles * KB >= 2LL * pairs && sk < best.cost) best = GemmPlan{GEMM_PAIR, true, sk};
+        }
+    }
     return best;
 }
 
@@ -578,6 +787,7 @@ static int launch_mode(cudaStream_t stream, const bf16* A, const bf16* A_lo, int
         return (int)cudaGetLastError();
     }
     const GemmPlan p = gemm_plan(MODE, M, N, K, A_lo != nullptr, std::min(tc_device_sms(), GEMM_MAX_CTAS));
+    if (p.bn == GEMM_PAIR) return A_lo != nullptr ? launch_tc2<MODE, true>(stream, A, A_lo, lda, W, M, N, K, epi, p.stream_k) : launch_tc2<MODE, false>(stream, A, nullptr, lda, W, M, N, K, epi, p.stream_k);
     if (A_lo != nullptr) {
         switch (p.bn) {
             case 256: return launch_tc<256, MODE, true>(stream, A, A_lo, lda, W, M, N, K, epi, p.stream_k);

@@ -1,0 +1,54 @@
+"""GPU (-m gpu): GEMM tiles of CTA pairs (256 x 256, gemm_tc2_kernel) at their edges: one row more than a CTA's 128, one more than a pair's 256, rows that leave the odd CTA
+without any, column tiles of 32, 160 and 288 columns, one k-step, whole tiles and tiles shared along K.  The width is pinned in a process of its own (the plan takes pairs
+for large shapes only); two shapes that the plan gives to pairs by itself beside it.  Against float64: f32 results to 1e-5 (test_gemm_edges.py derives the bounds), bf16 results
+with their low-order plane to 2^-14 (its 2^-15, and up to 4096 products added in one accumulator instead of several)."""
+import os
+import subprocess
+import sys
+
+import numpy as np
+import pytest
+
+import crane_b200
+from crane_b200 import synth
+
+pytestmark = pytest.mark.gpu
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+def check(M, N, K, split):
+    rng = np.random.default_rng(M * 3 + N + K)
+    a = rng.standard_normal((M, K), dtype=np.float32)
+    bits = synth.f32_to_bf16_bits(a)
+    lo = synth.f32_to_bf16_bits(a - synth.bf16_round(a)) if split else None
+    val = synth.bf16_round(a).astype(np.float64) + (synth.bf16_round(a - synth.bf16_round(a)).astype(np.float64) if split else 0.0)
+    wf = rng.standard_normal((N, K), dtype=np.float32) / np.sqrt(K)
+    ref = val @ synth.bf16_round(wf).astype(np.float64).T
+    w = synth.f32_to_bf16_bits(wf)
+    bias, init = rng.standard_normal(N).astype(np.float32), rng.standard_normal((M, N)).astype(np.float32)
+    err = lambda got, want: np.abs(got - want).max() / np.abs(want).max()  # noqa: E731
+    for _ in range(2):
+        one = crane_b200.op_gemm(bits, w, crane_b200.EPI_STORE_F32, a_lo_bits=lo, bias=bias)
+        two = crane_b200.op_gemm(bits, w, crane_b200.EPI_STORE_F32, a_lo_bits=lo, bias=bias)
+        assert np.array_equal(one, two) and err(one, ref + bias) < 1e-5
+    assert err(crane_b200.op_gemm(bits, w, crane_b200.EPI_RESID_F32, a_lo_bits=lo, out_init=init), init + ref) < 1e-5
+    g, u = ref[:, 0::2], ref[:, 1::2]
+    hi, low = crane_b200.op_gemm_epi(bits, w, crane_b200.EPI_SILU_MUL_BF16, a_lo_bits=lo, lo=True)
+    assert err(synth.bf16_bits_to_f32(hi).astype(np.float64) + synth.bf16_bits_to_f32(low), g / (1 + np.exp(-g)) * u) < 2.0 ** -14
+    hi, low = crane_b200.op_gemm_epi(bits, w, crane_b200.EPI_STORE_BF16, a_lo_bits=lo, lo=True)
+    assert err(synth.bf16_bits_to_f32(hi).astype(np.float64) + synth.bf16_bits_to_f32(low), ref) < 2.0 ** -14
+
+
+EDGES = [(129, 256, 64), (256, 288, 192), (257, 416, 512), (300, 544, 1024), (385, 1056, 128), (640, 256, 4096)]
+
+
+@pytest.mark.parametrize("schedule", ["1", "2"], ids=["whole", "shared"])
+def test_edges(schedule):
+    code = "import sys; sys.path[:0] = [%r, %r]; import test_gemm_pairs as t\nfor e in t.EDGES:\n    for s in (False, True): t.check(*e, s)" % (ROOT, os.path.join(ROOT, "tests"))
+    r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, CRANE_B200_GEMM_BN="512", CRANE_B200_GEMM_SCHED=schedule), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("shape,split", [((2000, 6176, 2048), False), ((770, 6176, 4096), False), ((2200, 4128, 2048), True)], ids=["whole", "shared", "split"])
+def test_shapes_of_the_plan(shape, split):
+    check(*shape, split)
