@@ -1,9 +1,15 @@
 // Flash attention forward on tcgen05 (prefill and vision tower): 128 query rows x one head per CTA, scores and output in TMEM.
 //
 // What bounds it: in split precision (hi + lo bf16 planes, three products kept of each) the MMAs -- per 128 keys at D = 128 24 of 128 columns for the scores
-// and 24 for the output, 3.1 k cycles -- and, just below, the 128 KB of K / V planes a tile brings from L2 (about 64 KB per us and SM).  The
-// softmax of a tile, one row per thread, runs under the MMAs of the next scores.  Tiles are 128 keys (64 at D = 256, where output, scores
-// and probabilities fill TMEM): 64-key tiles were bound by the hand-overs, 2.9 us each, 662 us for 4096 rows x 32 heads, D = 128, causal, split
+// and 24 for the output, 3.1 k cycles, 3.9 k measured: the scores' operands, both in shared memory, take its 128 bytes a cycle, and K / V come in beside them -- and, just
+// below, the 128 KB of K / V planes a tile brings from L2 and the softmax's exponentials and conversions.  Probabilities replace the scores they come from (two buffers
+// in turn, two planes in the 32 columns of 32 scores), so the softmax of a tile, one row per thread, runs under the output's MMAs of the tile before: it waits
+// for them only where the output has to be rescaled.  With columns of their own the probabilities of a tile waited for every one of those MMAs: us a launch
+// before / so, 4096 rows x 32 heads D = 128 split 357 / 338, 4096 x 8 heads D = 256 split 227 / 197, 784 rows x 16 heads D = 64 split 21.2 / 19.7, 1111 x 16
+// D = 128 plain 21.5 / 19.2.  Short calls are bound by latencies and by code that comes out of a cold instruction cache, so the loops over a
+// tile's columns are loops (77 rows behind 1 500 keys, 16 heads: 27.6 / 24.5).
+// (A second softmax group on alternate tiles, with three buffers, gained nothing: 3.9 k of its 4.9 k cycles a tile were MMAs, and short calls got 3 % longer.)
+// Tiles are 128 keys (64 at D = 256): 64-key tiles were bound by the hand-overs, 2.9 us each, 662 us for 4096 rows x 32 heads, D = 128, causal, split
 // (mma.sync, flash.cuh: 1690).
 //
 // One TMA producer, one MMA issuer, four softmax / epilogue warps (TMEM lane = query row = thread).  K and V stream through ONE ring of slots in
@@ -34,8 +40,8 @@ struct FtcCfg {
     static constexpr int Q_BYTES = P * 128 * D * 2;
     static constexpr int NSLOT = (208 * 1024 - Q_BYTES) / SLOT;
     static constexpr int SMEM = Q_BYTES + NSLOT * SLOT + 1024;
-    static constexpr int C_S = D, C_P = D + 2 * BN;                 // TMEM columns: O [0, D), two score buffers of BN, P planes of BN / 2
-    static_assert(NVS * R == BN && R >= 16 && NSLOT >= 4 && C_P + BN / 2 * P <= 512, "");
+    static constexpr int C_S = D;                                   // TMEM columns: O [0, D), two buffers of BN that scores arrive in and probabilities replace
+    static_assert(NVS * R == BN && R >= 16 && NSLOT >= 4 && C_S + 2 * BN <= 512, "");
 };
 
 __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {     // A from TMEM
@@ -92,7 +98,7 @@ flash_tc_kernel(const __grid_constant__ FtcMaps maps, FlashArgs a, int ns, int* 
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint8_t* ring = sm + C::Q_BYTES;
-    __shared__ uint64_t full[C::NSLOT], empty[C::NSLOT], q_full, s_full[2], s_empty[2], p_full, pv_done;
+    __shared__ uint64_t full[C::NSLOT], empty[C::NSLOT], q_full, s_full[2], p_full[2], pv_done[4];
     __shared__ uint32_t tmem_slot;
     __shared__ int gave_up;
     const TcWait wait{&gave_up, err};
@@ -100,8 +106,9 @@ flash_tc_kernel(const __grid_constant__ FtcMaps maps, FlashArgs a, int ns, int* 
     if (threadIdx.x == 0) {
         gave_up = 0;
         for (int i = 0; i < C::NSLOT; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
-        mbar_init(&q_full, 4); mbar_init(&p_full, 4); mbar_init(&pv_done, 1);
-        for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&s_empty[i], 4); }
+        mbar_init(&q_full, 4);
+        for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 4); }
+        for (int i = 0; i < 4; ++i) mbar_init(&pv_done[i], 1);
         fence_barrier_init();
     }
     if (warp == 2) { tmem_alloc(&tmem_slot, 512); tmem_relinquish(); }
@@ -149,6 +156,7 @@ flash_tc_kernel(const __grid_constant__ FtcMaps maps, FlashArgs a, int ns, int* 
         }
     };
 
+    float m_row = -INFINITY, l_row = 0.f;              // softmax warps: a row's reference and sum, for the cluster's merge
     if (warp == 0) {
         if (lane == 0 && n_walk > 0) {
             int st = 0; uint32_t ph = 0;
@@ -214,11 +222,10 @@ flash_tc_kernel(const __grid_constant__ FtcMaps maps, FlashArgs a, int ns, int* 
         int st = 0; uint32_t ph = 0;
         wait(&q_full, 0);
         auto scores = [&](int i) {
-            const uint32_t d = tmem + C::C_S + (uint32_t)(i & 1) * BN;
-            wait(&s_empty[i & 1], ((i >> 1) & 1) ^ 1);
-            tc_fence_after();
+            const uint32_t d = tmem + C::C_S + (uint32_t)(i & 1) * BN;      // (the probabilities of tile i - 2 that were there: their MMAs are ahead of these)
             for (int s = 0; s < C::NKS; ++s) {
                 wait(&full[st], ph);
+                tc_fence_after();
                 const uint64_t kd = make_smem_desc_sw128(smem_u32(ring + st * C::SLOT));
                 if (elect_one()) {
 #pragma unroll
@@ -244,7 +251,7 @@ flash_tc_kernel(const __grid_constant__ FtcMaps maps, FlashArgs a, int ns, int* 
         if (n_walk > 0) scores(0);
         for (int i = 0; i < n_walk; ++i) {
             if (i + 1 < n_walk) scores(i + 1);
-            wait(&p_full, i & 1);
+            wait(&p_full[i & 1], (i >> 1) & 1);
             tc_fence_after();
             for (int s = 0; s < C::NVS; ++s) {
                 wait(&full[st], ph);
@@ -253,16 +260,17 @@ flash_tc_kernel(const __grid_constant__ FtcMaps maps, FlashArgs a, int ns, int* 
                 if (elect_one()) {
 #pragma unroll
                     for (int k = 0; k < C::R / 16; ++k) {
-                        const uint32_t pa = tmem + C::C_P + (uint32_t)(s * (C::R / 2) + k * 8);
+                        const int key = s * C::R + k * 16;
+                        const uint32_t pa = tmem + C::C_S + (uint32_t)((i & 1) * BN + (key >> 5) * 32 + ((key >> 4) & 1) * 8);
                         const uint32_t acc = (uint32_t)((i | s | k) != 0);
                         if constexpr (SPLIT) {
-                            umma_ts(tmem, pa + BN / 2, vd + (uint64_t)(k * 128), id_o, acc);
+                            umma_ts(tmem, pa + 16, vd + (uint64_t)(k * 128), id_o, acc);
                             umma_ts(tmem, pa, vl + (uint64_t)(k * 128), id_o, 1u);
                             umma_ts(tmem, pa, vd + (uint64_t)(k * 128), id_o, 1u);
                         } else umma_ts(tmem, pa, vd + (uint64_t)(k * 128), id_o, acc);
                     }
                     umma_commit(&empty[st]);
-                    if (s == C::NVS - 1) umma_commit(&pv_done);
+                    if (s == C::NVS - 1) umma_commit(&pv_done[i & 3]);
                 }
                 __syncwarp();
                 if (++st == C::NSLOT) { st = 0; ph ^= 1; }
@@ -298,7 +306,6 @@ flash_tc_kernel(const __grid_constant__ FtcMaps maps, FlashArgs a, int ns, int* 
             const int kv0 = tile_at(i) * BN;
             wait(&s_full[i & 1], (i >> 1) & 1);
             tc_fence_after();
-            uint32_t u[BN];
             const uint32_t sa = tmem + lanes + C::C_S + (uint32_t)(i & 1) * BN;
             if (mods) {                 // cap, then the distance terms, in f32 on the scaled score, in place (one copy of this code for 16 columns: unrolled over
 #pragma unroll 1                        // the tile it outgrew the instruction cache and a tile took 64 k cycles)
@@ -322,31 +329,44 @@ flash_tc_kernel(const __grid_constant__ FtcMaps maps, FlashArgs a, int ns, int* 
                 }
                 tmem_st_wait();
             }
-#pragma unroll
-            for (int c = 0; c < BN; c += 16) tmem_ld16_async(sa + c, u + c);
-            tmem_ld_wait();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&s_empty[i & 1]);
-            float* s = reinterpret_cast<float*>(u);
             // every key of the tile visible to every row of this warp?  (the warp's first row sees the fewest new keys, its last the fewest old ones)
             const bool whole = kv0 + BN <= T && (!CAUSAL || (kv0 + BN - 1 <= kv_off + q0 + q * 32 && (a.window <= 0 || kv_off + q0 + q * 32 + 31 - kv0 < a.window)));
-            if (!whole) {               // the row sees columns [lo, hi) of the tile and those below kp
+            if (!whole) {               // the row sees columns [lo, hi) of the tile and those below kp (in place, for the code's size)
                 const int hi = (CAUSAL ? min(T, qpos + 1) : T) - kv0, lo = (CAUSAL && a.window > 0) ? qpos - a.window + 1 - kv0 : -1, kp = keep - kv0;
+#pragma unroll 1
+                for (int c = 0; c < BN; c += 16) {
+                    uint32_t w[16];
+                    tmem_ld16_async(sa + c, w);
+                    tmem_ld_wait();
 #pragma unroll
-                for (int c = 0; c < BN; ++c) s[c] = (c < hi && (c >= lo || c < kp)) ? s[c] : -INFINITY;
+                    for (int j = 0; j < 16; ++j) if (!(c + j < hi && (c + j >= lo || c + j < kp))) w[j] = 0xff800000u;
+                    tmem_st16(sa + c, w);
+                }
+                tmem_st_wait();
             }
+            // Both passes over the scores are loops over 64 columns that read them from TMEM: code that a CTA with two or three tiles runs once or twice comes out of a cold
+            // instruction cache (unrolled over 128 columns, its first exponentials took 6 k cycles and the next tile's 2.2 k).
+            constexpr int CH = 64;
             float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};      // (four chains: a warp has its scheduler to itself)
+#pragma unroll 1
+            for (int c0 = 0; c0 < BN; c0 += CH) {
+                uint32_t u[CH];
 #pragma unroll
-            for (int c = 0; c < BN; ++c) mx4[c & 3] = fmaxf(mx4[c & 3], s[c]);
+                for (int c = 0; c < CH; c += 16) tmem_ld16_async(sa + c0 + c, u + c);
+                tmem_ld_wait();
+#pragma unroll
+                for (int c = 0; c < CH; ++c) mx4[c & 3] = fmaxf(mx4[c & 3], __uint_as_float(u[c]));
+            }
             const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * mul;
-            if (i > 0) { wait(&pv_done, (i - 1) & 1); tc_fence_after(); }      // O is whole and the P columns are free
             const bool grow = mx > m + 8.f || (m == -INFINITY && mx > -INFINITY);
             if (__any_sync(0xffffffffu, grow)) {
                 const float mn = fmaxf(m, mx), f = m == -INFINITY ? 0.f : exp2f(m - mn);
                 l *= f;
                 m = mn;
                 if (i > 0) {
+                    // O is whole.  (Four barriers in turn: when the scores of tile i are there, the MMAs of tile i - 2 are done, so a parity cannot stand for an older use.)
+                    wait(&pv_done[(i - 1) & 3], ((i - 1) >> 2) & 1);
+                    tc_fence_after();
 #pragma unroll 1
                     for (int c = 0; c < D; c += 16) {
                         uint32_t o[16];
@@ -360,23 +380,32 @@ flash_tc_kernel(const __grid_constant__ FtcMaps maps, FlashArgs a, int ns, int* 
             }
             const float ref = m == -INFINITY ? 0.f : m;
             float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+            for (int c0 = 0; c0 < BN; c0 += CH) {
+                uint32_t u[CH];
 #pragma unroll
-            for (int c = 0; c < BN; c += 32) {
-                uint32_t hi[16], lo[16];
+                for (int c = 0; c < CH; c += 16) tmem_ld16_async(sa + c0 + c, u + c);
+                tmem_ld_wait();
+                const float* s = reinterpret_cast<const float*>(u);
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const float p0 = ex2(fmaf(s[c + 2 * j], mul, -ref)), p1 = ex2(fmaf(s[c + 2 * j + 1], mul, -ref));
-                    sum[(2 * j) & 3] += p0; sum[(2 * j + 1) & 3] += p1;
-                    split_bf16x2(p0, p1, hi[j], lo[j]);
+                for (int c = 0; c < CH; c += 32) {
+                    uint32_t hi[16], lo[16];
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        const float p0 = ex2(fmaf(s[c + 2 * j], mul, -ref)), p1 = ex2(fmaf(s[c + 2 * j + 1], mul, -ref));
+                        sum[(2 * j) & 3] += p0; sum[(2 * j + 1) & 3] += p1;
+                        split_bf16x2(p0, p1, hi[j], lo[j]);
+                    }
+                    tmem_st16(sa + c0 + c, hi);                           // in place of the 32 scores: 16 columns of either plane
+                    if (SPLIT) tmem_st16(sa + c0 + c + 16, lo);
                 }
-                tmem_st16(tmem + lanes + C::C_P + c / 2, hi);
-                if (SPLIT) tmem_st16(tmem + lanes + C::C_P + BN / 2 + c / 2, lo);
             }
             l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
             tmem_st_wait();
             tc_fence_before();
             if (kv0 + BN > T) {       // the rows behind the last key are a page's never written rest or the next sequence's: zero times whatever is there must stay zero
                 const int seq = n_walk * C::NKS + (n_walk - 1) * C::NVS;
+                if (i > 0) wait(&pv_done[(i - 1) & 3], ((i - 1) >> 2) & 1);      // (every slot's use before its last has been filled: the parities below cannot stand for an older one)
                 for (int j = 0; j < C::NVS; ++j) {
                     const int slot = (seq + j) % C::NSLOT, lo_r = max(0, T - kv0 - j * C::R);
                     if (lo_r >= C::R) continue;
@@ -388,53 +417,65 @@ flash_tc_kernel(const __grid_constant__ FtcMaps maps, FlashArgs a, int ns, int* 
                 fence_proxy_async();
             }
             __syncwarp();
-            if (lane == 0) mbar_arrive(&p_full);
+            if (lane == 0) mbar_arrive(&p_full[i & 1]);
         }
-        if (n_walk > 0) { wait(&pv_done, (n_walk - 1) & 1); tc_fence_after(); }
-        if (ns > 1) {                   // output columns [column][row], reference and sum into shared memory, in place of the operands (all read by now)
-            float* o_s = reinterpret_cast<float*>(sm) + r;
-            if (n_walk > 0) {
-#pragma unroll 1
-                for (int c = 0; c < D; c += 16) {
-                    uint32_t w[16];
-                    tmem_ld16_async(tmem + lanes + c, w);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) o_s[(c + j) * 128] = __uint_as_float(w[j]);
-                }
-            }
-            o_s[D * 128] = m; o_s[(D + 1) * 128] = l;
-        } else store(0, 16, m, l, r, [&](int c, float* v) {
+        if (n_walk > 0) { wait(&pv_done[(n_walk - 1) & 3], ((n_walk - 1) >> 2) & 1); tc_fence_after(); }
+        m_row = m; l_row = l;
+        if (ns == 1) store(0, 16, m, l, r, [&](int c, float* v) {
             uint32_t* w = reinterpret_cast<uint32_t*>(v);
             tmem_ld16_async(tmem + lanes + c, w);
             tmem_ld_wait();
         });
     }
     if (ns > 1) {
+        // CTA k merges and stores the groups of 16 columns k, k + ns ..; every CTA pushes its part of them, its references and its sums there, over the operands, which nobody
+        // needs any more behind the first barrier: [source][group][column][row].  (Pulled by the merging CTA, peer by peer, they took 14 k cycles of a short turn's 48.)
         cg::cluster_group cluster = cg::this_cluster();
+        const int groups = (D / 16 + ns - 1) / ns, r = (warp & 3) * 32 + lane;
+        float* part = reinterpret_cast<float*>(sm);
+        float* stat = part + ns * groups * 2048;                     // [source][reference, sum][row]
         cluster.sync();
         if (warp >= 4) {
-            const int r = (warp & 3) * 32 + lane;
-            const float* peer[8];
-            float f[8], M = -INFINITY, L = 0.f;
+            if (n_walk > 0) {
+#pragma unroll 1
+                for (int c = 0, to = 0, g = 0; c < D; c += 16) {
+                    uint32_t w[16];
+                    tmem_ld16_async(tmem + ((uint32_t)((warp & 3) * 32) << 16) + c, w);
+                    float* dst = cluster.map_shared_rank(part, to) + (rank * groups + g) * 2048 + r;
+                    tmem_ld_wait();
 #pragma unroll
-            for (int k = 0; k < 8; ++k)
-                if (k < ns) { peer[k] = cluster.map_shared_rank(reinterpret_cast<const float*>(sm), k) + r; f[k] = peer[k][D * 128]; M = fmaxf(M, f[k]); }
-#pragma unroll
-            for (int k = 0; k < 8; ++k)
-                if (k < ns) { f[k] = f[k] == -INFINITY ? 0.f : exp2f(f[k] - M); L += peer[k][(D + 1) * 128] * f[k]; }
+                    for (int j = 0; j < 16; ++j) dst[j * 128] = __uint_as_float(w[j]);
+                    if (++to == ns) { to = 0; ++g; }
+                }
+            }
+#pragma unroll 1
+            for (int k = 0; k < ns; ++k) {
+                float* dst = cluster.map_shared_rank(stat, k) + rank * 256 + r;
+                dst[0] = m_row; dst[128] = l_row;
+            }
+        }
+        cluster.sync();
+        if (warp >= 4) {
+            float M = -INFINITY, L = 0.f;
+#pragma unroll 1
+            for (int k = 0; k < ns; ++k) M = fmaxf(M, stat[k * 256 + r]);
+            auto factor = [&](int k) { const float m = stat[k * 256 + r]; return m == -INFINITY ? 0.f : exp2f(m - M); };
+#pragma unroll 1
+            for (int k = 0; k < ns; ++k) L += stat[k * 256 + 128 + r] * factor(k);
             store(rank * 16, 16 * ns, M, L, r, [&](int c, float* v) {
+                const float* p = part + (c / 16) / ns * 2048 + r;
 #pragma unroll
                 for (int j = 0; j < 16; ++j) v[j] = 0.f;
+#pragma unroll 1
+                for (int k = 0; k < ns; ++k, p += groups * 2048) {
+                    const float f = factor(k);
+                    if (f > 0.f) {
 #pragma unroll
-                for (int k = 0; k < 8; ++k)
-                    if (k < ns && f[k] > 0.f) {
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) v[j] = fmaf(peer[k][(c + j) * 128], f[k], v[j]);
+                        for (int j = 0; j < 16; ++j) v[j] = fmaf(p[j * 128], f, v[j]);
                     }
+                }
             });
         }
-        cluster.sync();                 // nobody leaves while its shared memory is still being read
     }
     tc_fence_before();
     __syncthreads();
