@@ -23,6 +23,13 @@ __global__ void embed_scale_rows_kernel(const int* __restrict__ ids, int T, cons
     pdl_launch_dependents();
     const int r = blockIdx.x;
     const bf16* e = embed + (size_t)ids[r] * W;
+    if (((W | ldx) & 3) == 0 && (((uintptr_t)embed & 7) | ((uintptr_t)x & 15)) == 0) {       // four columns a thread
+        for (int c = 4 * threadIdx.x; c < W; c += 4 * blockDim.x) {
+            const uint2 v = *reinterpret_cast<const uint2*>(e + c);
+            *reinterpret_cast<float4*>(x + (size_t)r * ldx + c) = make_float4(bf16lo(v.x) * scale, bf16hi(v.x) * scale, bf16lo(v.y) * scale, bf16hi(v.y) * scale);
+        }
+        return;
+    }
     for (int c = threadIdx.x; c < W; c += blockDim.x) x[(size_t)r * ldx + c] = __bfloat162float(e[c]) * scale;
 }
 
@@ -96,6 +103,16 @@ __global__ void dyt_rows_kernel(const float* __restrict__ x, int ldx, const int*
     pdl_launch_dependents();
     const int r = blockIdx.x, src = rows ? rows[r] : r;
     const float a = *alpha;
+    // four columns a thread, all their operands in flight together (one after the other, 5 rows of 1024 took 5.4 us of a decode step's layer)
+    const float* xr = x + (size_t)src * ldx;
+    if ((((long long)W | ldx | out.ldf | out.ldb | out.lo_off) & 3) == 0 && ((((uintptr_t)x | (uintptr_t)w | (uintptr_t)b | (uintptr_t)out.f) & 15) | ((uintptr_t)out.hi & 7)) == 0) {
+        for (int c = 4 * threadIdx.x; c < W; c += 4 * blockDim.x) {
+            const float4 xv = *reinterpret_cast<const float4*>(xr + c), wv = *reinterpret_cast<const float4*>(w + c), bv = *reinterpret_cast<const float4*>(b + c);
+            const float v[4] = {tanhf(a * xv.x) * wv.x + bv.x, tanhf(a * xv.y) * wv.y + bv.y, tanhf(a * xv.z) * wv.z + bv.z, tanhf(a * xv.w) * wv.w + bv.w};
+            store_act4(out, r, c, v);
+        }
+        return;
+    }
     for (int c = threadIdx.x; c < W; c += blockDim.x) store_act(out, r, c, tanhf(a * x[(size_t)src * ldx + c]) * w[c] + b[c]);
 }
 
@@ -748,9 +765,7 @@ __global__ void __launch_bounds__(SSD_TH) ssd_scan_kernel(RaggedBatch rb, Mamba2
     float* S = whole ? a.ssm_state + (((size_t)slot * a.heads + h) * N) * P
                          : a.seg_state + ((((size_t)e * SSD_SEGS + seg) * a.heads + h) * N) * P;
     const int n0 = ns * SSD_R;
-    // rows past N and tokens past the portion's end multiply zeros: the stages start zeroed and only real values are ever copied in
-    for (int i = threadIdx.x; i < 2 * SSD_CH * per_tok; i += blockDim.x) ssm_s[i] = 0.f;
-    __syncthreads();
+    const int nch = (len + SSD_CH - 1) / SSD_CH;
     uint64_t s[SSD_CPT][SSD_R / 2];                           // pairs of state rows
 #pragma unroll
     for (int i = 0; i < SSD_R / 2; ++i)
@@ -759,6 +774,9 @@ __global__ void __launch_bounds__(SSD_TH) ssd_scan_kernel(RaggedBatch rb, Mamba2
             auto at = [&](int n) { return (MODE != 1 && n < N && live[j]) ? S[(size_t)n * P + p0 + pl + 16 * j] : 0.f; };
             s[j][i] = f2(at(n0 + 2 * i), at(n0 + 2 * i + 1));
         }
+    // rows past N and tokens past the portion's end multiply zeros: the stages in use start zeroed and only real values are ever copied in (the state is on its way meanwhile)
+    for (int i = threadIdx.x; i < min(nch, 2) * SSD_CH * per_tok / 4; i += blockDim.x) reinterpret_cast<float4*>(ssm_s)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    __syncthreads();
     float dprod = 1.f;                                        // MODE 1, thread 0: product of the segment's decays
     const float negA = -__expf(a.A_log[h]), Dh = a.D[h], dtb = a.dt_bias[h];
     const int dtcol = 2 * inner + 2 * a.groups * N + h;
@@ -794,7 +812,6 @@ __global__ void __launch_bounds__(SSD_TH) ssd_scan_kernel(RaggedBatch rb, Mamba2
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    const int nch = (len + SSD_CH - 1) / SSD_CH;
     fetch(0, stage(0));
     for (int c = 0; c < nch; ++c) {
         if (c + 1 < nch) { fetch(c + 1, stage(c + 1)); asm volatile("cp.async.wait_group 1;" ::: "memory"); }
@@ -1300,7 +1317,7 @@ inline void go(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cud
 
 // ---------------------------------------------------------------------------------------------------------------- launchers
 int embed_scale_rows_launch(cudaStream_t st, const int* ids, int T, const bf16* embed, int W, float scale, float* x, int ldx) {
-    go(embed_scale_rows_kernel, T, 128, 0, st, ids, T, embed, W, scale, x, ldx);
+    go(embed_scale_rows_kernel, T, 256, 0, st, ids, T, embed, W, scale, x, ldx);
     return last_err();
 }
 int embed_sinpos_rows_launch(cudaStream_t st, const int* ids, const int* row_pos, int T, const bf16* embed, int W, const float* freq, float* x, int ldx) {
@@ -1315,7 +1332,7 @@ int post_norm_add_launch(cudaStream_t st, const float* y1, int ld1, const float*
 }
 int dyt_rows_launch(cudaStream_t st, const float* x, int ldx, const int* rows, int R, int W, const float* alpha, const float* w, const float* b,
                     const ActOut& out) {
-    go(dyt_rows_kernel, R, 128, 0, st, x, ldx, rows, W, alpha, w, b, out);
+    go(dyt_rows_kernel, R, 256, 0, st, x, ldx, rows, W, alpha, w, b, out);
     return last_err();
 }
 int greedy_advance_launch(cudaStream_t st, const float* logits, int V, int E, float* part_val, int* part_idx, int* ids, int* row_pos,
