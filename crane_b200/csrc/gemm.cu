@@ -239,7 +239,9 @@ __device__ __forceinline__ void gemm_epilogue(const GemmEpi& ep, const CUtensorM
     for (int it = it_begin; it < it_end; ++seg) {
         const int seg_end = min(it_end, (it / KB + 1) * KB);
         const int t = it / KB, kb0 = it % KB, kb1 = kb0 + (seg_end - it);
-        const int m0 = ((t % sc.tiles_m) * PER + rank) * GEMM_BM + q * 32, n0 = (t / sc.tiles_m) * BN;
+        int mt, nt;
+        sched_place(sc, cta, t, mt, nt);
+        const int m0 = (mt * PER + rank) * GEMM_BM + q * 32, n0 = nt * BN;
         const int b = seg & 1;
         const uint32_t acc = tmem_base + (uint32_t)(b * BN) + ((uint32_t)(q * 32) << 16);
         const bool sole = kb0 == 0 && kb1 == KB;
@@ -370,17 +372,20 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             constexpr int B_OFF = Cfg::A_BYTES * (SPLIT ? 2 : 1);
             // weights do not depend on the predecessor kernel: their first tiles go out before the dependency wait
             const int npre = ep.w_dynamic ? 0 : min(it_end - it_begin, STAGES);
-            int t = it_begin / KB, kb = it_begin - t * KB, n0 = t / sc.tiles_m * BN;
+            int t = it_begin / KB, kb = it_begin - t * KB, mt, nt;
+            sched_place(sc, cta, t, mt, nt);
+            int n0 = nt * BN;
             for (int i = 0; i < npre; ++i) {
                 mbar_arrive_expect_tx(&full_bar[i], Cfg::STAGE_BYTES);
                 tma_load_2d(smem + i * Cfg::STAGE_BYTES + B_OFF, &tmB, &full_bar[i], kb * GEMM_BK, n0);
-                if (++kb == KB) { kb = 0; ++t; n0 = t / sc.tiles_m * BN; }
+                if (++kb == KB && i + 1 < npre) { kb = 0; sched_place(sc, cta, ++t, mt, nt); n0 = nt * BN; }
             }
             pdl_wait();
             int s = 0, left = npre; uint32_t ph = 0;
             for (int it = it_begin; it < it_end;) {
                 t = it / KB;
-                const int seg_end = min(it_end, (t + 1) * KB), nt = t / sc.tiles_m, m0 = (t - nt * sc.tiles_m) * GEMM_BM;
+                sched_place(sc, cta, t, mt, nt);
+                const int seg_end = min(it_end, (t + 1) * KB), m0 = mt * GEMM_BM;
                 n0 = nt * BN;
                 int kc = (it - t * KB) * GEMM_BK;
                 for (; it < seg_end; ++it, kc += GEMM_BK) {
@@ -510,17 +515,20 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         if (lane == 0) {
             constexpr int B_OFF = Cfg::A_BYTES * (SPLIT ? 2 : 1);
             const int npre = ep.w_dynamic ? 0 : min(it_end - it_begin, STAGES);
-            int t = it_begin / KB, kb = it_begin - t * KB, n0 = t / sc.tiles_m * BN + rank * (BN / 2);
+            int t = it_begin / KB, kb = it_begin - t * KB, mt, nt;
+            sched_place(sc, pair, t, mt, nt);
+            int n0 = nt * BN + rank * (BN / 2);
             for (int i = 0; i < npre; ++i) {        // the weights' first tiles go out before the dependency wait
                 if (rank == 0) mbar_arrive_expect_tx(&full_bar[i], 2 * Cfg::STAGE_BYTES);
                 tma_load_2d_pair(smem + i * Cfg::STAGE_BYTES + B_OFF, &tmB, peer_smem(&full_bar[i], 0), kb * GEMM_BK, n0);
-                if (++kb == KB) { kb = 0; ++t; n0 = t / sc.tiles_m * BN + rank * (BN / 2); }
+                if (++kb == KB && i + 1 < npre) { kb = 0; sched_place(sc, pair, ++t, mt, nt); n0 = nt * BN + rank * (BN / 2); }
             }
             pdl_wait();
             int s = 0, left = npre; uint32_t ph = 0;
             for (int it = it_begin; it < it_end;) {
                 t = it / KB;
-                const int seg_end = min(it_end, (t + 1) * KB), nt = t / sc.tiles_m, m0 = (t - nt * sc.tiles_m) * (2 * GEMM_BM) + rank * GEMM_BM;
+                sched_place(sc, pair, t, mt, nt);
+                const int seg_end = min(it_end, (t + 1) * KB), m0 = mt * (2 * GEMM_BM) + rank * GEMM_BM;
                 n0 = nt * BN + rank * (BN / 2);
                 int kc = (it - t * KB) * GEMM_BK;
                 for (; it < seg_end; ++it, kc += GEMM_BK) {
@@ -634,6 +642,11 @@ gemm_simt_kernel(const bf16* __restrict__ A, const bf16* __restrict__ A_lo, int 
 // parking and re-reading partial tiles -- outweighs the parallelism)
 static const int g_gemm_minit = [] { const char* e = getenv("CRANE_B200_GEMM_MINIT"); const int v = e ? atoi(e) : 0; return v > 0 ? v : 8; }();
 
+// Whole tiles are dealt in turn, eight rows of tiles wide: the CTAs at work at one time then read 8 strips of A and about 9 of the weights between them.  Each CTA a run of
+// its own (one strip of the weights per CTA, all of A, 200 MB in use) read 5.0 GB for 24576 x 4096 at 4096 rows in split mode, 1174 us under the power limit; so 0.70 GB,
+// 980 us.  Bands of 4 and of all 16 rows: within 1 % of that.  Tiles shared along K stay in runs: their order is part of the results.
+static int sched_band(const TcSched& sc, bool stream_k) { return stream_k ? sc.tiles_m : std::min(8, sc.tiles_m); }
+
 // maps of the results: patches of 32 rows (see epi_rows)
 template <int MODE>
 static bool out_maps(const GemmEpi& epi, int M, int N, CUtensorMap* tmO, CUtensorMap* tmOlo) {
@@ -667,6 +680,7 @@ static int launch_tc(cudaStream_t stream, const bf16* A, const bf16* A_lo, int l
     if (iters > 0x7fffffffLL) return -1000;
     const int cap = std::min(tc_device_sms(), GEMM_MAX_CTAS);
     sc.unit = stream_k ? 1 : sc.KB;
+    sc.band = sched_band(sc, stream_k);
     const long long units = iters / sc.unit;
     sc.G = (int)std::max<long long>(1, std::min<long long>(cap, stream_k ? iters / g_gemm_minit : tiles));
     sc.base = (int)(units / sc.G);
@@ -714,6 +728,7 @@ static int launch_tc2(cudaStream_t stream, const bf16* A, const bf16* A_lo, int 
     if (iters > 0x7fffffffLL) return -1000;
     const int cap = std::min(tc_max_clusters(2), GEMM_MAX_CTAS / 2);
     sc.unit = stream_k ? 1 : sc.KB;
+    sc.band = sched_band(sc, stream_k);
     const long long units = iters / sc.unit;
     sc.G = (int)std::max<long long>(1, std::min<long long>(cap, stream_k ? iters / g_gemm_minit : tiles));
     sc.base = (int)(units / sc.G);
@@ -736,7 +751,7 @@ static int launch_tc2(cudaStream_t stream, const bf16* A, const bf16* A_lo, int 
 // Tiles of pairs (256 x 256): a k-step 0.31 us plain and 0.62 split with few tiles, 0.36 and 0.63 with every SM busy on the scale that gives the single tiles 0.42 and 0.66, two or three
 // us more of setup and hand-over.  Worth it where the operands are what takes the time; not where a gated or GELU tile's epilogue does (9 us), nor with rows that fill 256 badly.  Their
 // stream-K pays above one wave too, while all operands stay in the L2 (CTAs at different k-steps share nothing of what they read): 4096 x 12288 at 2048 rows 187 us, whole tiles 141.
-//   us, single / pairs, plain: 24576 x 4096 at 256 rows 78.8 / 55.3, 512 108 / 87, 2048 392 / 327, 4096 822 / 657    6144 x 4096 at 784 64.4 / 44.9, 4096 170 / 142
+//   us, single / pairs (with whole tiles in runs, before they were dealt in turn: sched_band), plain: 24576 x 4096 at 256 rows 78.8 / 55.3, 512 108 / 87, 2048 392 / 327, 4096 822 / 657    6144 x 4096 at 784 64.4 / 44.9, 4096 170 / 142
 //   12288 x 2048 at 784 59.7 / 44.4, 1111 48.4 / 55.3, 4096 152 / 136                                                4096 x 12288 at 512 69.6 / 52.6, 4096 318 / 284
 //   split: 24576 x 4096 at 512 153 / 144, 4096 1204 / 1100    6144 x 4096 at 4096 283 / 263    4096 x 4096 193 / 179    8256 x 1024 103 / 97    7168 x 1024 92 / 88
 constexpr int GEMM_PAIR = 512;          // GemmPlan::bn: 256 x 256 tiles of two CTAs

@@ -216,11 +216,11 @@ int tc_max_clusters(int cl);
 
 // ---- work dealt out along K ------------------------------------------------------------------
 // G CTAs share tiles x KB iterations; CTA c owns the iterations [unit * (c * base + min(c, rem)), ...): base or base + 1 units of `unit`
-// iterations -- unit = KB deals out whole tiles (nothing is split), unit = 1 is stream-K
+// iterations -- unit = KB deals out whole tiles (nothing is split; where a CTA's j-th lies: sched_place), unit = 1 is stream-K
 struct TcSched {
-    int tiles_m, tiles_n, KB;      // output tiles and iterations per tile; tile t = n_tile * tiles_m + m_tile (the CTAs working at the
-                                   // same time share their weight rows: the L2 merges those requests)
+    int tiles_m, tiles_n, KB;      // output tiles and iterations per tile; tile t: sched_place (a linear of few rows, gemm_rows.cu: one row of tiles)
     int G, unit, base, rem;
+    int band;                      // rows of tiles that sched_place walks together (tiles_m: all of them)
     float* ws;                     // [2 * G] partial tiles
     int* counters;                 // [tiles] arrivals per tile, zero between launches (the finisher resets its tile)
 };
@@ -228,6 +228,14 @@ __host__ __device__ inline int sched_start(const TcSched& s, int c) { return s.u
 __host__ __device__ inline int sched_owner(const TcSched& s, int it) {       // CTA whose range holds iteration `it`
     const int u = it / s.unit, big = s.rem * (s.base + 1);
     return u < big ? u / (s.base + 1) : s.rem + (u - big) / s.base;
+}
+// Where tile t of CTA c's range lies.  Whole tiles: the CTA's j-th is number c + j * G, so that the G tiles of a turn are neighbours (a CTA has base tiles, the first rem one
+// more: every number below G * base + rem once); numbers run along the rows of a band, then along n, then to the next band.
+__host__ __device__ inline void sched_place(const TcSched& s, int c, int t, int& mt, int& nt) {
+    if (s.unit == s.KB) t = c + (t - (c * s.base + (c < s.rem ? c : s.rem))) * s.G;
+    const int per = s.band * s.tiles_n, b = t / per, r = t - b * per, left = s.tiles_m - b * s.band, w = left < s.band ? left : s.band;
+    nt = r / w;
+    mt = b * s.band + r - nt * w;
 }
 
 }  // namespace cb

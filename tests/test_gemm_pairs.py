@@ -49,6 +49,16 @@ def test_edges(schedule):
     assert r.returncode == 0, r.stderr[-2000:]
 
 
+TURNS = [(2400, 2336, 128), (2050, 4640, 64), (1100, 9472, 192)]        # several tiles a CTA; rows of tiles that 8 does not divide
+
+
+@pytest.mark.parametrize("width", ["64", "256", "512"])
+def test_whole_tiles_in_turns(width):
+    code = "import sys; sys.path[:0] = [%r, %r]; import test_gemm_pairs as t\nfor e in t.TURNS: t.check(*e, e[0] == 2050)" % (ROOT, os.path.join(ROOT, "tests"))
+    r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, CRANE_B200_GEMM_BN=width, CRANE_B200_GEMM_SCHED="1"), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
 @pytest.mark.parametrize("shape,split", [((2000, 6176, 2048), False), ((770, 6176, 4096), False), ((2200, 4128, 2048), True)], ids=["whole", "shared", "split"])
 def test_shapes_of_the_plan(shape, split):
     check(*shape, split)
