@@ -2837,6 +2837,11 @@ extern "C" CRANE_B200_API int crane_b200_debug_expire_wait(crane_b200_model* m) 
     if (m) cudaSetDevice(m->device);
     return tc_expire_wait(m ? m->stream : nullptr) == 0 ? CRANE_B200_OK : CRANE_B200_CUDA_ERROR;
 }
+/* ... of one CTA of a pair, whose other CTA waits for what never comes either, with a kernel's own limit of 4 s */
+extern "C" CRANE_B200_API int crane_b200_debug_expire_wait_pair(crane_b200_model* m) {
+    if (m) cudaSetDevice(m->device);
+    return tc_expire_wait_pair(m ? m->stream : nullptr) == 0 ? CRANE_B200_OK : CRANE_B200_CUDA_ERROR;
+}
 
 static int op_sampler(int device, const float* logits, size_t vocab, size_t k, const crane_b200_sampling* p, uint32_t* out, float* logits_after) {
     if (!logits || !out || vocab == 0 || vocab > (size_t)INT32_MAX) return CRANE_B200_INVALID_ARG;

@@ -486,10 +486,9 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty_bar + 2);
     int* last_flag = reinterpret_cast<int*>(tmem_slot + 1);
     int* gave_up = last_flag + 1;
-    const TcWait wait{gave_up, err};
-
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rank = (int)cluster_rank(), pair = blockIdx.x >> 1;
+    const TcWait wait{gave_up, err, peer_smem(gave_up, rank ^ 1)};
     const int KB = sc.KB;
     const int it_begin = sched_start(sc, pair), it_end = sched_start(sc, pair + 1);
 
@@ -545,7 +544,6 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     if (++s == STAGES) { s = 0; ph ^= 1; }
                 }
             }
-            wait.drain();
         }
     } else if (warp == 1) {
         if (rank == 0) {
@@ -593,6 +591,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     __syncthreads();
     __syncwarp();
     cluster_sync_all();                             // neither CTA leaves while the other's MMAs read its operands or its warps signal here
+    wait.drain();                                   // (a wait of either CTA ran out: copies and MMAs in flight reach into both)
     if (warp == 2) { tc_fence_after(); tmem_dealloc_pair(tmem_base, 2 * BN); }
 }
 

@@ -87,6 +87,29 @@ int tc_expire_wait(cudaStream_t st) {
     return (int)cudaGetLastError();
 }
 
+__global__ void __cluster_dims__(2, 1, 1) expire_wait_pair_kernel(int* err) {
+    __shared__ uint64_t bar;
+    __shared__ int gave_up;
+    const uint32_t rank = cluster_rank();
+    gave_up = 0;
+    mbar_init(&bar, 1);
+    fence_barrier_init();
+    cluster_sync_all();
+    const uint32_t peer = peer_smem(&gave_up, rank ^ 1);
+    if (rank == 1) { const TcWaitT<2000000> wait{&gave_up, err, peer}; wait(&bar, 0); }
+    else { const TcWait wait{&gave_up, err, peer}; wait(&bar, 0); }        // (4 s by itself; the partner's word ends it)
+    cluster_sync_all();
+    const TcWait both{&gave_up, err, peer};
+    both(&bar, 0);                  // (given up: returns at once in either)
+    both.drain();
+}
+int tc_expire_wait_pair(cudaStream_t st) {
+    int* err = nullptr;
+    if (const int e = tc_err_word(st, &err)) return e;
+    expire_wait_pair_kernel<<<2, 1, 0, st>>>(err);
+    return (int)cudaGetLastError();
+}
+
 __global__ void __launch_bounds__(256, 1) cluster_probe_kernel() {}
 int tc_max_clusters(int cl) {
     static std::mutex mu;

@@ -9,15 +9,17 @@
 namespace cb {
 
 // ---- bounded waits ---------------------------------------------------------------------
-// A wait that runs out (4 s at 1.9 GHz: a wait in these kernels is for a copy or an MMA of its own CTA, or for the end of the kernel ahead)
-// raises the CTA's `gave_up` word in shared memory and the stream's error word in pinned host memory; every later wait of the CTA
-// returns at once, the kernel runs to its end with its results discarded, and every call that hands results to the caller reads the word first
+// A wait that runs out (4 s at 1.9 GHz: a wait in these kernels is for a copy or an MMA of its own CTA, or of either CTA of a pair, or for the end of the kernel ahead)
+// raises the CTA's `gave_up` word in shared memory, with it that of the other CTA of a pair, and the stream's error word in pinned host memory; every later wait of the
+// CTA, or of both, returns at once, the kernel runs to its end with its results discarded, and every call that hands results to the caller reads the word first
 // (sync_results in engine.cu) and reports the error.  Results that are left on the device are covered by the call that reads them.
 constexpr long long TC_WAIT_CYCLES = 8000000000LL;
+constexpr uint32_t TC_NO_PEER = 0xffffffffu;
 template <long long LIMIT>
 struct TcWaitT {
     volatile int* gave_up;      // shared memory, zeroed before the first wait
     int* err;                   // pinned host memory (tc_err_word), written only when a wait runs out
+    uint32_t peer = TC_NO_PEER; // the word of the pair's other CTA (a cluster address), which leaves behind a barrier of both only
     __device__ __forceinline__ void operator()(uint64_t* bar, uint32_t parity) const {
         const uint32_t addr = smem_u32(bar);
         long long t0 = 0;
@@ -32,11 +34,17 @@ struct TcWaitT {
             if ((n & 255u) == 255u) {
                 if (*gave_up) return;
                 if (!t0) t0 = clock64();
-                else if (clock64() - t0 > LIMIT) { *gave_up = 1; *reinterpret_cast<volatile int*>(err) = 1; return; }
+                else if (clock64() - t0 > LIMIT) {
+                    *gave_up = 1;
+                    if (peer != TC_NO_PEER) asm volatile("st.relaxed.cluster.shared::cluster.u32 [%0], 1;" ::"r"(peer) : "memory");
+                    *reinterpret_cast<volatile int*>(err) = 1;
+                    return;
+                }
             }
         }
     }
-    // the issuing thread's last act when a wait ran out: copies still in flight must not land in a successor's shared memory
+    // the issuing thread's last act when a wait ran out (in a pair: every thread's of both, behind their last barrier): copies still in flight must not land in a
+    // successor's shared memory
     __device__ __forceinline__ void drain() const {
         if (!*gave_up) return;
         const long long t0 = clock64();
@@ -210,6 +218,7 @@ inline bool tc_tmap_bf16(CUtensorMap* map, const void* base, uint64_t rows, uint
 }
 // launches a kernel whose wait runs out after about a millisecond (for tests of what follows)
 int tc_expire_wait(cudaStream_t st);
+int tc_expire_wait_pair(cudaStream_t st);      // ... one CTA's of a pair, while the other waits for what never comes
 int tc_device_sms();
 // clusters of `cl` (2 .. 8) CTAs that the device runs at the same time when a CTA takes a whole SM
 int tc_max_clusters(int cl);

@@ -132,3 +132,25 @@ def test_speech_calls():
     m.load_checkpoint(synth.synth_checkpoint(cfg))
     reported(m, lambda: [m.text_project([1, 2, 3])])
     m.close()
+
+
+def test_pair_gives_up_together():
+    """One CTA of a pair gives up after a millisecond; the other, whose wait would run for 4 s, is released by it, and the error is reported once."""
+    import time
+    import crane_b200
+    cfg = synth.TINY_QWEN3_UNTIED
+    m = crane_b200.Qwen3Model(cfg, max_seq_len=64)
+    m.load_checkpoint(synth.synth_checkpoint(cfg))
+    ids = synth.synth_token_ids(20, cfg["vocab_size"], "wp")
+    want = m.forward_step(ids, 0)
+    fn = crane_b200.load_library().crane_b200_debug_expire_wait_pair
+    fn.restype, fn.argtypes = C.c_int, [C.c_void_p]
+    t = time.perf_counter()
+    assert fn(m.h) == 0
+    m.clear_kv_cache()
+    with pytest.raises(crane_b200.CraneB200Error, match="wait ran out"):
+        m.forward_step(ids, 0)
+    assert time.perf_counter() - t < 2.0
+    m.clear_kv_cache()
+    assert np.array_equal(m.forward_step(ids, 0), want)
+    m.close()
