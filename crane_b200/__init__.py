@@ -175,7 +175,7 @@ def _ptr(a: np.ndarray):
 
 
 class _Pinned:
-    """Owner of one buffer of the library's pinned pool; the arrays over it keep it alive."""
+    """Owner of one piece of the library's pinned range; the arrays over it keep it alive."""
 
     def __init__(self, address: int, shape, dtype):
         self.__array_interface__ = {"data": (address, False), "shape": tuple(shape), "typestr": dtype.str, "version": 3}
@@ -186,7 +186,12 @@ class _Pinned:
 
 
 def _result(shape, dtype=np.float32) -> np.ndarray:
-    """An uninitialised array for a call's results, in pinned memory while the pool has any (small ones: ordinary memory, a copy of a few KB is no faster there)."""
+    """An uninitialised array for a call's results, in pinned memory while the pool has any (small ones: ordinary memory, a copy of a few KB is no faster there).
+
+    It is writeable, contiguous and its caller's for good, as one of ordinary memory is, but its memory is the pool's: `owndata` is False and an in-place `resize`
+    is refused (`copy()` gives an array that owns its data).  Programs that keep results keep their pieces of the pool's 64 MiB; when it is used up, results come
+    in ordinary memory.
+    """
     shape, dtype = tuple(int(n) for n in shape), np.dtype(dtype)
     n = int(np.prod(shape, dtype=np.int64)) * dtype.itemsize
     p = C.c_void_p()
@@ -209,6 +214,7 @@ class Engine:
         if rc != OK:
             raise CraneB200Error(rc, (self.lib.crane_b200_last_error(None) or b"").decode("utf-8", "replace"))
         self.h = h
+        _result((1024,))                         # the pinned range is made here, not in the first call with results
         self.vocab = self.lib.crane_b200_vocab_size(h)
         self.hidden = self.lib.crane_b200_hidden_size(h)
 

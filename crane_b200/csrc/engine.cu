@@ -2031,7 +2031,7 @@ int crane_b200_create(const char* config_json, int device_ordinal, crane_b200_mo
                 CUDA_OK(cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking));
                 m->fsv->stream = m->stream;
                 *out = m.release();
-                HostPool::get().opened();
+                HostPool::get().opened(device_ordinal);
                 return CRANE_B200_OK;
             }
         }
@@ -2060,7 +2060,7 @@ int crane_b200_create(const char* config_json, int device_ordinal, crane_b200_mo
         return CRANE_B200_INVALID_ARG;
     }
     *out = m.release();
-    HostPool::get().opened();
+    HostPool::get().opened(device_ordinal);
     return CRANE_B200_OK;
 }
 

@@ -1,68 +1,97 @@
-// Pinned host memory for results (crane_b200_host_alloc / _free): copies into it run at the link's rate and need no second copy by the host.
-// A copy of 1 MB into pageable memory took 20 us on the link and another 80 to 100 in the driver's staging.  us a call, pageable / pinned: two decode rounds of 32
-// sequences over 8192 logits 949 / 848 (dense, two layers), 625 / 532 (Q4_K_M, one); four tokens over 151 936 logits 2740 / 2597; the features
-// of an image, 6.4 MB, 3668 / 3367.  Pinning costs 50 us and more, so returned buffers are kept, in powers of two; what is out and what is kept together stay under
-// CAP, whatever programs hold on to, and the kept ones go back when the last handle is destroyed.
+// Pinned host memory for results (crane_b200_host_alloc / _free): copies into it run at the link's rate and need no second copy by the host.  us of a copy into pinned /
+// pageable memory on the GPU box: 64 KB 11 / 18, 1 MB 29 / 83, 8 MB 157 / 472, 32 MB 601 / 1980 and more.
+// Pinning itself takes far longer than it saves one call (cudaHostAlloc of 1 MB 2.2 ms, of 16 MB 12 ms, freeing 0.4 to 1.8 ms), so no call pins: ONE range of SIZE bytes, in
+// huge pages where the system has them (32 MB registered in 2.2 ms, from cudaHostAlloc 18 ms), is registered by the first request while a handle is open -- the Python
+// engine makes it as it opens -- and results are pieces of it, the smallest free stretch that holds them.  What does not fit gets ordinary memory from the caller, as does what
+// comes when programs have kept the whole range.  us of a new handle's first pass / of later ones: 32 sequences' round over 8192 logits 940 / 862 (ordinary memory 1030 / 965, buffers
+// pinned one by one 3400 to 10 000 / 865), one token over 151 936 four times 3300 / 2595 (3540 / 2748, 5000 to 8000 / 2600), an image's features 8300 / 3380 (9200 / 3880, 18 000 / 3350).  It goes back with the last handle or, where pieces are still out, with the last of those.
 #pragma once
 
 #include <cuda_runtime.h>
+#include <sys/mman.h>
 
 #include <cstddef>
+#include <map>
 #include <mutex>
-#include <unordered_map>
-#include <vector>
+#include <thread>
 
 namespace cb {
 
 class HostPool {
 public:
-    static constexpr int MIN_LOG = 12, MAX_LOG = 25;                    // 4 KB .. 32 MB
-    static constexpr size_t CAP = (size_t)64 << 20;
+    static constexpr size_t SIZE = (size_t)64 << 20, PIECE = 4096;
     static HostPool& get() { static HostPool* p = new HostPool; return *p; }       // (never destroyed: arrays may outlive static objects)
 
     void* take(size_t bytes) {
-        int c = MIN_LOG;
-        while (((size_t)1 << c) < bytes) if (++c > MAX_LOG) return nullptr;
+        if (bytes == 0 || bytes > SIZE) return nullptr;
+        const size_t n = (bytes + PIECE - 1) / PIECE * PIECE;
         std::lock_guard<std::mutex> g(mu_);
         if (handles_ == 0) return nullptr;
-        void* p = nullptr;
-        if (!free_[c - MIN_LOG].empty()) { p = free_[c - MIN_LOG].back(); free_[c - MIN_LOG].pop_back(); }
-        else {
-            if (held_ + ((size_t)1 << c) > CAP) trim();
-            if (held_ + ((size_t)1 << c) > CAP) return nullptr;
-            if (cudaHostAlloc(&p, (size_t)1 << c, cudaHostAllocPortable) != cudaSuccess) { cudaGetLastError(); return nullptr; }
-            held_ += (size_t)1 << c;
-        }
-        out_[p] = c;
-        return p;
+        if (!base_ && !tried_) { tried_ = true; reserve(); }
+        auto best = free_.end();
+        for (auto it = free_.begin(); it != free_.end(); ++it)
+            if (it->second >= n && (best == free_.end() || it->second < best->second)) best = it;
+        if (best == free_.end()) return nullptr;
+        const size_t at = best->first, left = best->second - n;
+        out_[at] = n;
+        free_.erase(best);
+        if (left) free_[at + n] = left;
+        return base_ + at;
     }
     bool give(void* p) {
         std::lock_guard<std::mutex> g(mu_);
-        auto it = out_.find(p);
+        const char* c = static_cast<const char*>(p);
+        if (!base_ || c < base_ || c >= base_ + SIZE) return false;
+        auto it = out_.find((size_t)(c - base_));
         if (it == out_.end()) return false;
-        const int c = it->second;
+        auto f = free_.emplace(it->first, it->second).first;
         out_.erase(it);
-        if (handles_ > 0) free_[c - MIN_LOG].push_back(p);
-        else drop(p, c);
+        auto next = std::next(f);
+        if (next != free_.end() && f->first + f->second == next->first) { f->second += next->second; free_.erase(next); }
+        if (f != free_.begin()) {
+            auto prev = std::prev(f);
+            if (prev->first + prev->second == f->first) { prev->second += f->second; free_.erase(f); }
+        }
+        if (handles_ == 0 && out_.empty()) release();
         return true;
     }
-    void opened() { std::lock_guard<std::mutex> g(mu_); ++handles_; }
-    void closed() { std::lock_guard<std::mutex> g(mu_); if (--handles_ == 0) trim(); }
-    size_t held() { std::lock_guard<std::mutex> g(mu_); return held_; }
+    void opened(int device) { std::lock_guard<std::mutex> g(mu_); ++handles_; device_ = device; tried_ = false; }
+    void closed() { std::lock_guard<std::mutex> g(mu_); if (--handles_ == 0 && out_.empty()) release(); }
 
 private:
-    void drop(void* p, int c) { cudaFreeHost(p); held_ -= (size_t)1 << c; }
-    void trim() {
-        for (int i = 0; i <= MAX_LOG - MIN_LOG; ++i) {
-            for (void* p : free_[i]) drop(p, i + MIN_LOG);
-            free_[i].clear();
-        }
+    // On a thread of its own, with a handle's device: the caller's has its current device and context left as they are (a new thread's are GPU 0 and none), and a stream
+    // that another thread is capturing does not forbid it.
+    template <typename F> static void aside(int device, F&& f) {
+        std::thread([&] {
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+            if (cudaThreadExchangeStreamCaptureMode(&mode) == cudaSuccess && cudaSetDevice(device) == cudaSuccess) f();
+        }).join();
+    }
+    void reserve() {
+        void* p = mmap(nullptr, SIZE, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+        if (p == MAP_FAILED) return;
+        madvise(p, SIZE, MADV_HUGEPAGE);
+        bool ok = false;
+        try { aside(device_, [&] { ok = cudaHostRegister(p, SIZE, cudaHostRegisterPortable) == cudaSuccess; }); } catch (const std::exception&) {}
+        if (!ok) { munmap(p, SIZE); return; }
+        base_ = static_cast<char*>(p);
+        reserved_on_ = device_;
+        free_[0] = SIZE;
+    }
+    void release() {
+        if (!base_) return;
+        bool ok = false;
+        try { aside(reserved_on_, [&] { ok = cudaHostUnregister(base_) == cudaSuccess; }); } catch (const std::exception&) {}
+        if (!ok) return;                 // (kept, registered, for the next handle)
+        munmap(base_, SIZE);
+        base_ = nullptr;
+        free_.clear();
     }
     std::mutex mu_;
-    std::vector<void*> free_[MAX_LOG - MIN_LOG + 1];
-    std::unordered_map<void*, int> out_;
-    size_t held_ = 0;       // bytes out and kept
-    int handles_ = 0;
+    char* base_ = nullptr;
+    std::map<size_t, size_t> free_, out_;       // offset -> length; free stretches have pieces that are out between them
+    int handles_ = 0, device_ = 0, reserved_on_ = 0;
+    bool tried_ = false;                        // one attempt per handle opened
 };
 
 }  // namespace cb

@@ -2,6 +2,9 @@
 out without a handle."""
 import ctypes as C
 import gc
+import os
+import subprocess
+import sys
 import threading
 
 import numpy as np
@@ -9,6 +12,8 @@ import pytest
 
 import crane_b200
 from crane_b200 import synth
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def test_without_a_handle_there_is_none():
@@ -73,3 +78,80 @@ def test_threads_share_the_pool():
         t.join()
     m.close()
     assert not bad
+
+
+@pytest.mark.gpu
+def test_pieces_of_one_range():
+    """Every piece lies in one range of 64 MiB, whatever was asked for before: rounds of 32 rows over 151 936 logits (19.4 MB) with the last one still held, beside a row at
+    a time, never leave it; a program that keeps everything ends in ordinary memory; and what was given back in any order is whole again.  (In a process of its own: the
+    range is a process's.)"""
+    r = subprocess.run([sys.executable, "-c", "import sys; sys.path[:0] = [%r, %r]; import test_host_pool as t; t.pieces()" % (ROOT, os.path.join(ROOT, "tests"))],
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
+def pieces():
+    m = crane_b200.Qwen3Model(synth.TINY_QWEN3, max_seq_len=64)
+    span = []
+
+    def take(*shape):
+        a = crane_b200._result(shape)
+        a[...] = len(span)
+        if a.base is not None:
+            span.extend((a.ctypes.data, a.ctypes.data + a.nbytes))
+        return a
+    for _ in range(4):
+        out = None                                          # (a first round; those behind it hold the one before)
+        for _ in range(5):
+            out = take(32, 151936)
+            row = take(151936)
+            assert out.base is not None and row.base is not None
+        del out, row
+    rng = np.random.default_rng(0)
+    kept = [take(int(rng.integers(1024, 1 << 20))) for _ in range(100)]
+    marks = [k.flat[0] for k in kept]
+    assert any(k.base is None for k in kept) and all((k == v).all() for k, v in zip(kept, marks))
+    while kept:
+        kept.pop(int(rng.integers(len(kept))))
+    whole = take(16 << 20)
+    assert whole.base is not None and max(span) - min(span) <= 64 << 20
+    m.close()
+    assert (whole == whole.flat[0]).all()
+    m = crane_b200.Qwen3Model(synth.TINY_QWEN3, max_seq_len=64)          # the range lives on with its piece; the next handle finds it used up
+    assert crane_b200._result((1024,)).base is None
+    del whole
+    assert crane_b200._result((1024,)).base is not None
+    m.close()
+
+
+@pytest.mark.gpu
+def test_a_thread_keeps_its_context():
+    """Taking and giving back results opens no context in a thread that has none, the range's making and release included."""
+    cu = C.CDLL("libcuda.so.1")
+    seen = []
+
+    def current():
+        c = C.c_void_p()
+        assert cu.cuCtxGetCurrent(C.byref(c)) == 0
+        seen.append(c.value)
+
+    def work():
+        current()
+        lib, p = crane_b200.load_library(), C.c_void_p()
+        assert lib.crane_b200_host_alloc(1 << 20, C.byref(p)) == crane_b200.OK
+        current()
+        assert lib.crane_b200_host_free(p) == crane_b200.OK
+        current()
+
+    m = crane_b200.Qwen3Model(synth.TINY_QWEN3, max_seq_len=64)
+    t = threading.Thread(target=work)
+    t.start()
+    t.join()
+    last = crane_b200._result((5000,))
+    m.close()
+    box = [last]
+    del last
+    t = threading.Thread(target=lambda: (current(), box.clear(), gc.collect(), current()))
+    t.start()
+    t.join()
+    assert seen == [None] * 5
