@@ -14,6 +14,7 @@
 #include <cstdarg>
 #include <cstring>
 #include <memory>
+#include <numeric>
 #include <string>
 #include <vector>
 

@@ -732,32 +732,25 @@ constexpr int SSD_SEGS = 4, SSD_SEG_MIN = 512;              // an entry is segme
 __host__ __device__ inline int ssd_seg_len(int len) { return ((len + SSD_SEGS - 1) / SSD_SEGS + SSD_CH - 1) / SSD_CH * SSD_CH; }
 template <int SSD_R, int MODE, int SSD_CPT = 2>              // state rows per thread: ceil(N / 8) rounded up to 4, 8, 16 or 32
 __global__ void __launch_bounds__(SSD_TH) ssd_scan_kernel(RaggedBatch rb, Mamba2Args a, int C) {
-    pdl_wait();
     constexpr int SSD_COLS = 16 * SSD_CPT;
     extern __shared__ __align__(16) float ssm_s[];
     // Entries in order of length, the longest first, and the slowest index of the grid: blocks of long portions that follow one another land on different SMs, those of
-    // single tokens beside them.  (Entries as they come, fastest: a step of two long portions and two tokens 107 us, so 50.)
-    __shared__ int s_entry;
+    // single tokens beside them.  (Entries as they come, fastest: a step of two long portions and two tokens 107 us, so 50.)  The order comes with the step's descriptors;
+    // single tokens alone go as they come.  (Worked out by every block from the lengths, 64 tokens took 64.7 us, so 57.2; 16 portions of 20 tokens 31.4 / 28.7; one token 7.1 / 7.2.)
     const int rank = MODE == 0 ? blockIdx.z : blockIdx.z / SSD_SEGS, seg = MODE == 0 ? 0 : blockIdx.z % SSD_SEGS;
-    for (int i = threadIdx.x; i < rb.E; i += SSD_TH) {
-        const int li = rb.ent_len[i];
-        int ahead = 0;
-        for (int j = 0; j < rb.E; ++j) { const int lj = rb.ent_len[j]; ahead += lj > li || (lj == li && j < i); }
-        if (ahead == rank) s_entry = i;
-    }
-    __syncthreads();
-    const int e = s_entry, h = blockIdx.x, ns = threadIdx.x & (SSD_NS - 1), pl = threadIdx.x / SSD_NS;
+    const int e = MODE == 0 && a.single_rows ? rank : rb.ent_order[rank], full_len = rb.ent_len[e], slot = rb.ent_slot[e], row0 = rb.ent_row0[e];
+    pdl_wait();                                               // (what a step's descriptors say is there before its first kernel, and none changes it)
+    const int h = blockIdx.x, ns = threadIdx.x & (SSD_NS - 1), pl = threadIdx.x / SSD_NS;
     const int p0 = blockIdx.y * SSD_COLS;
     const int P = a.P, N = a.N, inner = a.heads * P, g = h / (a.heads / a.groups);
     bool live[SSD_CPT];
 #pragma unroll
     for (int j = 0; j < SSD_CPT; ++j) live[j] = p0 + pl + 16 * j < P;
-    const int full_len = rb.ent_len[e], slot = rb.ent_slot[e];
     const bool whole = MODE == 0 || full_len < SSD_SEG_MIN;   // (a short entry beside long ones: as by itself, all of it in MODE 2)
     if (MODE == 1 && whole) return;
     const int seg_len = whole ? full_len : ssd_seg_len(full_len), seg0 = seg * seg_len;
     if (seg0 >= full_len) return;                             // (fewer segments than SSD_SEGS)
-    const int len = min(seg_len, full_len - seg0), r0 = rb.ent_row0[e] + seg0;
+    const int len = min(seg_len, full_len - seg0), r0 = row0 + seg0;
     const int ncol = min(SSD_COLS, P - p0);
     const int NP = ssd_npad(N, SSD_R), per_tok = SSD_COLS + 2 * NP + 4;
     auto stage = [&](int c) { return ssm_s + (c & 1) * SSD_CH * per_tok; };      // (computed: out of an array of pointers the reads are generic ones)

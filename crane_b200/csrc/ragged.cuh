@@ -30,6 +30,7 @@ struct RaggedBatch {
     const int* ent_len;     // [E] rows of the entry
     const int* ent_pos0;    // [E] tokens the sequence held before this step
     const int* ent_slot;    // [E] sequence slot: block-table row and recurrent-state slot
+    const int* ent_order;   // [E] the entries from the longest to the shortest, those of one length as they come
     int T, E;
 };
 
