@@ -2985,14 +2985,17 @@ int crane_b200_op_gemm(int device, const uint16_t* a, const uint16_t* a_lo, cons
                 //  so that stamp is the ARRIVAL of the producer warp; the TMEM dealloc stamp 7 is the real end of the CTA)
                 fprintf(stderr, "   isolated launch: first CTA start -> last CTA end %.2f us\n", ((double)t7 - (double)t0) / 1e3);
                 double acc[6] = {0, 0, 0, 0, 0, 0}, start_max = 0;
+                size_t have[6] = {0, 0, 0, 0, 0, 0};              // (the odd CTA of a pair issues no MMAs: it has neither of their stamps)
                 for (size_t i = 0; i < max_tiles; ++i) if (hp[8 * i]) {
-                    for (int j = 0; j < 6; ++j) acc[j] += (double)((long long)hp[8 * i + j + 1] - (long long)hp[8 * i + j]);
+                    for (int j = 0; j < 6; ++j)
+                        if (hp[8 * i + j + 1] && hp[8 * i + j]) { acc[j] += (double)((long long)hp[8 * i + j + 1] - (long long)hp[8 * i + j]); ++have[j]; }
                     start_max = std::max(start_max, (double)(hp[8 * i] - t0));
                 }
                 fprintf(stderr, "gemm_prof M=%d N=%d K=%d split=%d: %.2f us/launch back-to-back (%.1f TFLOP/s); one launch: %zu CTAs, span %.2f us, last CTA start +%.2f us; "
                         "per-CTA mean ns: setup %.0f | first operands %.0f | mainloop issue %.0f | accumulator wait %.0f | epilogue %.0f\n",
                         M, N, K, a_lo ? 1 : 0, ms * 1e3 / 20, 2.0 * M * N * K / (ms * 1e-3 / 20) / 1e12, n, (t1 - t0) / 1e3, start_max / 1e3,
-                        acc[0] / n, acc[1] / n, acc[2] / n, acc[3] / n, acc[4] / n, acc[5] / n);
+                        acc[0] / std::max<size_t>(have[0], 1), acc[1] / std::max<size_t>(have[1], 1), acc[2] / std::max<size_t>(have[2], 1), acc[3] / std::max<size_t>(have[3], 1),
+                        acc[4] / std::max<size_t>(have[4], 1));
                 {   // the same launch 8 times back to back, each with its own stamp block: where the time BETWEEN kernels goes
                     const int NB = 8;
                     cudaMemset(dprof, 0, max_tiles * 8 * sizeof(unsigned long long));

@@ -491,6 +491,11 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     const TcWait wait{gave_up, err, peer_smem(gave_up, rank ^ 1)};
     const int KB = sc.KB;
     const int it_begin = sched_start(sc, pair), it_end = sched_start(sc, pair + 1);
+    unsigned long long* prof = ep.prof ? ep.prof + 8 * (size_t)blockIdx.x : nullptr;       // (stamps 2 and 3, the MMAs': the even CTA's)
+    auto stamp = [&](int i) {
+        if (prof) { unsigned long long t; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t)); prof[i] = t; }
+    };
+    if (threadIdx.x == 0) stamp(0);
 
     if (warp == 0 && lane == 0) {
         tma_prefetch_desc(&tmA);
@@ -509,6 +514,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
+    if (threadIdx.x == 0) stamp(1);
     pdl_launch_dependents();
     if (warp == 0) {
         if (lane == 0) {
@@ -558,6 +564,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 const uint32_t acc = tmem_base + (uint32_t)(b * BN);
                 for (int i = it; i < seg_end; ++i) {
                     wait(&full_bar[s], ph);
+                    if (i == it_begin && lane == 0) stamp(2);
                     tc_fence_after();
                     const uint32_t a_addr = smem_u32(smem + s * Cfg::STAGE_BYTES);
                     const uint64_t adesc = make_smem_desc_sw128(a_addr);
@@ -577,6 +584,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 }
                 it = seg_end;
             }
+            if (lane == 0) stamp(3);
         }
     } else if (warp >= 4) {
         if (threadIdx.x == 128) { tma_prefetch_desc(&tmO); tma_prefetch_desc(&tmOlo); }
@@ -584,15 +592,17 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         const int q = warp & 3, part = (warp - 4) >> 2;
         EpiPatch patch{epi_smem + (warp - 4) * EPI_PATCH, false};
         gemm_epilogue<MODE, BN, 2>(ep, tmO, tmOlo, patch, smem + (warp - 4) * 4 * EPI_PATCH, M, N, sc, pair, rank, it_begin, it_end, tmem_base, tmem_full_bar, wait, last_flag, q, part, lane,
-                                   [] {}, [&](int b) { mbar_arrive_peer(peer_smem(&tmem_empty_bar[b], 0)); });
+                                   [&] { stamp(4); }, [&](int b) { mbar_arrive_peer(peer_smem(&tmem_empty_bar[b], 0)); });
         if (lane == 0) tma_store_wait_read<0>();
+        if (threadIdx.x == 128) stamp(5);
     }
     tc_fence_before();
     __syncthreads();
     __syncwarp();
+    if (threadIdx.x == 0) stamp(6);
     cluster_sync_all();                             // neither CTA leaves while the other's MMAs read its operands or its warps signal here
     wait.drain();                                   // (a wait of either CTA ran out: copies and MMAs in flight reach into both)
-    if (warp == 2) { tc_fence_after(); tmem_dealloc_pair(tmem_base, 2 * BN); }
+    if (warp == 2) { tc_fence_after(); tmem_dealloc_pair(tmem_base, 2 * BN); if (lane == 0) stamp(7); }
 }
 
 // =====================================================================================

@@ -39,7 +39,7 @@ struct GemmEpi {
     const float* gate = nullptr; int ldg = 0; const float* gate_bias = nullptr;   // nullable [M, ldg] (+ [N]): the accumulator of (m, n) is multiplied by
                                         // sigmoid(gate[m, n] + gate_bias[n]) after bias and col_scale, before the mode's store / add
     float glu_limit = 0.f;    // EPI_SILU_MUL_BF16 only: 0 = SiLU(gate) * up; > 0 = the clamped gated unit with this limit
-    unsigned long long* prof = nullptr;   // optional: 8 globaltimer stamps per CTA (tile timeline, tools/gemm_probe.py)
+    unsigned long long* prof = nullptr;   // optional: 8 globaltimer stamps per CTA (tile timeline, tools/gemm_probe.py; tensor-core tiles, of one CTA or two)
 };
 
 struct TmaEncoder;  // host: resolves cuTensorMapEncodeTiled once

@@ -3,6 +3,7 @@ without any, column tiles of 32, 160 and 288 columns, one k-step, whole tiles an
 for large shapes only); two shapes that the plan gives to pairs by itself beside it.  Against float64: f32 results to 1e-5 (test_gemm_edges.py derives the bounds), bf16 results
 with their low-order plane to 2^-14 (its 2^-15, and up to 4096 products added in one accumulator instead of several)."""
 import os
+import re
 import subprocess
 import sys
 
@@ -62,3 +63,16 @@ def test_whole_tiles_in_turns(width):
 @pytest.mark.parametrize("shape,split", [((2000, 6176, 2048), False), ((770, 6176, 4096), False), ((2200, 4128, 2048), True)], ids=["whole", "shared", "split"])
 def test_shapes_of_the_plan(shape, split):
     check(*shape, split)
+
+
+def test_timeline():
+    """The timeline of a launch (tools/gemm_probe.py) where the plan takes pairs: every stage has a time, and none is longer than the launch."""
+    code = ("import sys; sys.path[:0] = [%r]; import numpy as np, crane_b200; r = np.random.default_rng(0).integers(0x3c00, 0x3c80, (2, 1024, 2048)).astype(np.uint16);"
+            "crane_b200.op_gemm(r[0], r[1], crane_b200.EPI_STORE_F32)" % ROOT)
+    r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, CRANE_B200_GEMM_BN="512", CRANE_B200_GEMM_SCHED="1", CRANE_B200_GEMM_PROF="1"), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    line = next(x for x in r.stderr.splitlines() if x.startswith("gemm_prof"))
+    assert "one launch: 32 CTAs" in line
+    span = float(re.search(r"span ([0-9.]+) us", line).group(1))
+    stages = [float(x) for x in re.findall(r"(?:setup|operands|issue|wait|epilogue) ([0-9.+-]+)", line)]
+    assert len(stages) == 5 and 1.0 < span < 1e4 and all(0.0 < x <= 1e3 * span for x in stages), line
