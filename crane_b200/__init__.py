@@ -189,8 +189,8 @@ def _result(shape, dtype=np.float32) -> np.ndarray:
     """An uninitialised array for a call's results, in pinned memory while the pool has any (small ones: ordinary memory, a copy of a few KB is no faster there).
 
     It is writeable, contiguous and its caller's for good, as one of ordinary memory is, but its memory is the pool's: `owndata` is False and an in-place `resize`
-    is refused (`copy()` gives an array that owns its data).  Programs that keep results keep their pieces of the pool's 64 MiB; when it is used up, results come
-    in ordinary memory.
+    is refused (`copy()` gives an array that owns its data).  Programs that keep results keep their pieces of the pool; when it is used up, results come in
+    ordinary memory.
     """
     shape, dtype = tuple(int(n) for n in shape), np.dtype(dtype)
     n = int(np.prod(shape, dtype=np.int64)) * dtype.itemsize

@@ -2004,6 +2004,9 @@ static void check_room(crane_b200_model* m, size_t start_pos, size_t n) {
 
 extern "C" {
 
+// bytes of results that a handle's programs hold at a time: sixteen calls' logits of every sequence; two large images' features
+static size_t results_held(const crane_b200_model* m) { return std::max((size_t)16 * m->max_batch * m->V * sizeof(float), m->is_vl ? (size_t)32 << 20 : 0); }
+
 int crane_b200_create(const char* config_json, int device_ordinal, crane_b200_model** out) {
     if (!config_json || !out) { g_create_error = "null argument"; return CRANE_B200_INVALID_ARG; }
     *out = nullptr;
@@ -2031,8 +2034,9 @@ int crane_b200_create(const char* config_json, int device_ordinal, crane_b200_mo
                 m->use_persistent = false;
                 CUDA_OK(cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking));
                 m->fsv->stream = m->stream;
+                const size_t held = results_held(m.get());
                 *out = m.release();
-                HostPool::get().opened(device_ordinal);
+                HostPool::get().opened(device_ordinal, held);
                 return CRANE_B200_OK;
             }
         }
@@ -2060,8 +2064,9 @@ int crane_b200_create(const char* config_json, int device_ordinal, crane_b200_mo
         if (m->fsv) { m->fsv->release(); delete m->fsv; }
         return CRANE_B200_INVALID_ARG;
     }
+    const size_t held = results_held(m.get());
     *out = m.release();
-    HostPool::get().opened(device_ordinal);
+    HostPool::get().opened(device_ordinal, held);
     return CRANE_B200_OK;
 }
 

@@ -298,10 +298,10 @@ CRANE_B200_API int crane_b200_tts_generate(crane_b200_model* m, size_t max_frame
 /* ---- profiling (crane-core/src/ops/prof.rs:37-243 `CRANE_PROF`) ----------------------------------- */
 /* Device time (ms, CUDA events on the engine stream) of the last prefill pass and last decode run. */
 CRANE_B200_API int crane_b200_last_timing(const crane_b200_model* m, float* prefill_ms, float* decode_ms, size_t* decode_steps);
-/* Pinned host memory for results, pieces of one range of 64 MiB that the handles of a process share: every call above that writes results to host memory takes any
- * pointer, and copies into these at the link's rate.  The first request while a handle is open makes the range (a few milliseconds, on that handle's device; the calling
- * thread's current device stays as it is), later ones call nothing of CUDA's.  CRANE_B200_OOM when no free stretch of it holds the request or no handle
- * exists: use ordinary memory then.  The range is given back with the last handle; pieces that are out stay valid until freed, and the range with them. */
+/* Pinned host memory for results, pieces of one range that the handles of a process share: every call above that writes results to host memory takes any pointer, and
+ * copies into these at the link's rate.  The first request while a handle is open makes the range, of 2 to 64 MiB by what the handle's results need (0.8 to 9 ms, on that
+ * handle's device; the calling thread's current device stays as it is); later ones call nothing of CUDA's.  CRANE_B200_OOM when no free stretch of it holds the request
+ * or no handle exists: use ordinary memory then.  The range is given back with the last handle; pieces that are out stay valid until freed, and the range with them. */
 CRANE_B200_API int crane_b200_host_alloc(size_t bytes, void** out);
 CRANE_B200_API int crane_b200_host_free(void* p);
 /* Kernels launched by this handle since creation (graph replays count their nodes). */

@@ -82,7 +82,7 @@ def test_threads_share_the_pool():
 
 @pytest.mark.gpu
 def test_pieces_of_one_range():
-    """Every piece lies in one range of 64 MiB, whatever was asked for before: rounds of 32 rows over 151 936 logits (19.4 MB) with the last one still held, beside a row at
+    """Every piece lies in one range of up to 64 MiB, as far as the handles need it, whatever was asked for before: rounds of 32 rows over 151 936 logits (19.4 MB) with the last one still held, beside a row at
     a time, never leave it; a program that keeps everything ends in ordinary memory; and what was given back in any order is whole again.  (In a process of its own: the
     range is a process's.)"""
     r = subprocess.run([sys.executable, "-c", "import sys; sys.path[:0] = [%r, %r]; import test_host_pool as t; t.pieces()" % (ROOT, os.path.join(ROOT, "tests"))],
@@ -91,8 +91,14 @@ def test_pieces_of_one_range():
 
 
 def pieces():
-    m = crane_b200.Qwen3Model(synth.TINY_QWEN3, max_seq_len=64)
-    span = []
+    small = dict(synth.TINY_QWEN3)
+    large = dict(synth.TINY_QWEN3, vocab_size=151936)
+    m = crane_b200.Qwen3Model(small, max_seq_len=64)                    # 2 MiB are enough for it
+    assert crane_b200._result((1 << 18,)).base is not None and crane_b200._result((3 << 18,)).base is None
+    early = crane_b200._result((1024,))
+    n = crane_b200.Qwen3Model(large, max_seq_len=64, max_batch=32)      # ... and the rest for this one
+    m.close()
+    span = [early.ctypes.data, early.ctypes.data + early.nbytes]
 
     def take(*shape):
         a = crane_b200._result(shape)
@@ -113,14 +119,20 @@ def pieces():
     assert any(k.base is None for k in kept) and all((k == v).all() for k, v in zip(kept, marks))
     while kept:
         kept.pop(int(rng.integers(len(kept))))
-    whole = take(16 << 20)
-    assert whole.base is not None and max(span) - min(span) <= 64 << 20
-    m.close()
-    assert (whole == whole.flat[0]).all()
-    m = crane_b200.Qwen3Model(synth.TINY_QWEN3, max_seq_len=64)          # the range lives on with its piece; the next handle finds it used up
+    del early
+    assert take(62 << 18).base is not None and crane_b200._result((64 << 18,)).base is None       # (no piece lies across what was added)
+    first, rest = take(2 << 18), take(62 << 18)
+    assert first.base is not None and rest.base is not None and max(span) - min(span) == 64 << 20
+    n.close()
+    assert (rest == rest.flat[0]).all()
+    m = crane_b200.Qwen3Model(small, max_seq_len=64)                    # the range lives on with its pieces; the next handle finds it used up
     assert crane_b200._result((1024,)).base is None
-    del whole
+    del first
     assert crane_b200._result((1024,)).base is not None
+    m.close()
+    del rest
+    m = crane_b200.Qwen3Model(large, max_seq_len=64, max_batch=32)      # made anew, in one
+    assert crane_b200._result((64 << 18,)).base is not None
     m.close()
 
 
