@@ -2776,12 +2776,13 @@ int crane_b200_decode_batch_sample(crane_b200_model* m, const int* seqs, const u
     API_END(m)
 }
 
-int crane_b200_op_qlinear(int device, const float* x, size_t m, size_t k, const void* raw, size_t raw_bytes, int ggml_type, size_t n,
-                          const float* norm_w, float eps, float* y) {
+static int op_qlinear(int device, const float* x, size_t m, size_t k, const void* raw, size_t raw_bytes, int ggml_type, size_t n, const float* norm_w, float eps, int epi, float* y) {
     if (!x || !raw || !y || m == 0 || n == 0 || k == 0 || (k % 256) != 0) return CRANE_B200_INVALID_ARG;
     if (ggml_type != QT_Q4_K && ggml_type != QT_Q6_K && ggml_type != QT_Q8_0) return CRANE_B200_UNSUPPORTED;
     if (raw_bytes != n * (k / q_src_block_elems(ggml_type)) * q_src_block_bytes(ggml_type)) return CRANE_B200_INVALID_ARG;
+    if (epi != GEMV_STORE && (m < (size_t)qrows_min(ggml_type) || (epi == GEMV_SILU_MUL && (n & 1)))) return CRANE_B200_INVALID_ARG;
     if (cudaSetDevice(device) != cudaSuccess) return CRANE_B200_CUDA_ERROR;
+    const size_t n_out = epi == GEMV_SILU_MUL ? n / 2 : n;
     int rc = CRANE_B200_OK;
     float *dx = nullptr, *dy = nullptr, *dn = nullptr;
     unsigned char *dw = nullptr, *dxq = nullptr, *dxr = nullptr;
@@ -2795,13 +2796,14 @@ int crane_b200_op_qlinear(int device, const float* x, size_t m, size_t k, const 
         CUDA_OK(cudaMalloc((void**)&dxq, xquant_bytes(4, (int)k)));
         CUDA_OK(cudaMemcpy(dx, x, m * k * 4, cudaMemcpyHostToDevice));
         CUDA_OK(cudaMemcpy(dw, packed.data(), packed.size(), cudaMemcpyHostToDevice));
-        CUDA_OK(cudaMemset(dy, 0, m * n * 4));
+        if (epi == GEMV_STORE) CUDA_OK(cudaMemset(dy, 0, m * n * 4));
+        else CUDA_OK(cudaMemcpy(dy, y, m * n_out * 4, cudaMemcpyHostToDevice));
         if (norm_w) { CUDA_OK(cudaMalloc((void**)&dn, k * 4)); CUDA_OK(cudaMemcpy(dn, norm_w, k * 4, cudaMemcpyHostToDevice)); }
         if (m >= (size_t)qrows_min(ggml_type)) {
             CUDA_OK(cudaMalloc((void**)&dxr, qrows_bytes((int)m, (int)k)));
             const QRows xr = qrows_at(dxr, (int)m, (int)k);
             LAUNCH_OK(xquant_rows_launch(nullptr, (int)m, dx, (int)k, (int)k, dn, eps, xq_mode_for(ggml_type), xr, false));
-            LAUNCH_OK(qgemm_launch(nullptr, ggml_type, dw, xr, (int)m, (int)n, (int)k, GEMV_STORE, dy, (int)n, false));
+            LAUNCH_OK(qgemm_launch(nullptr, ggml_type, dw, xr, (int)m, (int)n, (int)k, epi, dy, (int)n_out, false));
         } else for (size_t s0 = 0; s0 < m;) {
             const int B = (m - s0 >= 4) ? 4 : (m - s0 >= 2) ? 2 : 1;
             QGemvArgs qa = {};
@@ -2816,7 +2818,7 @@ int crane_b200_op_qlinear(int device, const float* x, size_t m, size_t k, const 
         }
         CUDA_OK(cudaDeviceSynchronize());
         check_waits(nullptr);
-        CUDA_OK(cudaMemcpy(y, dy, m * n * 4, cudaMemcpyDeviceToHost));
+        CUDA_OK(cudaMemcpy(y, dy, m * n_out * 4, cudaMemcpyDeviceToHost));
     } catch (const EngineError& e) {
         g_create_error = e.msg;
         rc = e.code;
@@ -2824,6 +2826,19 @@ int crane_b200_op_qlinear(int device, const float* x, size_t m, size_t k, const 
     for (void* p : {(void*)dx, (void*)dy, (void*)dn, (void*)dw, (void*)dxq, (void*)dxr}) if (p) cudaFree(p);
     return rc;
 }
+int crane_b200_op_qlinear(int device, const float* x, size_t m, size_t k, const void* raw, size_t raw_bytes, int ggml_type, size_t n,
+                          const float* norm_w, float eps, float* y) {
+    return op_qlinear(device, x, m, k, raw, raw_bytes, ggml_type, n, norm_w, eps, GEMV_STORE, y);
+}
+
+/* debugging aids (not in the public header) for tests that say which form of a kernel they run.  A quantised linear on the tensor cores with its epilogue: 1 adds to y [m, n],
+ * 2 is silu(gate) * up of interleaved rows, y [m, n / 2] */
+extern "C" CRANE_B200_API int crane_b200_debug_qlinear(int device, const float* x, size_t m, size_t k, const void* raw, size_t raw_bytes, int ggml_type, size_t n, int epi, float* y) {
+    if (epi != 1 && epi != 2) return CRANE_B200_INVALID_ARG;
+    return op_qlinear(device, x, m, k, raw, raw_bytes, ggml_type, n, nullptr, 0.f, epi == 1 ? GEMV_RESID : GEMV_SILU_MUL, y);
+}
+/* ... the activation rows of its tiles (16, 32, 64 or 128) */
+extern "C" CRANE_B200_API int crane_b200_debug_qgemm_rows(int ggml_type, int m, int n, int k) { return qgemm_rows(ggml_type, m, n, k); }
 
 /* debugging aid (not in the public header): copy a prefill workspace to the host -- 0: residual stream x [S, H], 1: qkv [S, qkv_dim],
  * 2: the f32 rows in front of / behind a quantised linear [S, max(I, q_dim)] */

@@ -11,7 +11,8 @@
 //   Q8_0  A = q, one accumulator per 32-element block (both sides have a scale per 32)
 // and the block scales are applied in f32 when the accumulator is read, once per block: acc += (d_w D - dmin_w D2) d_x.
 //
-// The weight rows are the MMA's M = 128 rows and the activation rows its N (16 .. 64), so a decode batch pays for the columns it has.
+// The weight rows are the MMA's M = 128 rows and the activation rows its N (16 .. 64; a tile of TM = 128 activation rows is two MMAs of 64), so a decode batch pays for the columns it
+// has.
 //
 // The unpacked weights go from registers to TMEM, the MMA's A operand there: 128 f16 columns of a super-block are 128 lanes x 64 columns, a lane's row being the row that
 // its thread unpacks.  Through shared memory (an f16 tile written by the unpacking warps, a proxy fence, read back by the MMAs) a super-block of 128 x 64 cost
@@ -21,7 +22,7 @@
 // What bounds it: at few rows the quantised bytes (decode), at many the bytes of the activation codes, the MMAs and the instructions that turn nibbles into f16 (about
 // 1.2 per weight).  Hence the split of a CTA into roles that overlap: one thread that brings raw blocks by TMA, eight warps that unpack
 // them, one TMA producer for the activation codes, one MMA issuer, four or eight warps that
-// read accumulators.  Stream-K over (128 x NT tile, super-block): every SM has the same number of super-blocks whatever the shape; partial
+// read accumulators.  Stream-K over (128 x TM tile, super-block): every SM has the same number of super-blocks whatever the shape; partial
 // tiles are added in contributor order by the last to arrive, so a result does not depend on who that was.
 #include "quant.cuh"
 #include "tc.cuh"
@@ -29,6 +30,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <cstdlib>
 
 namespace cb {
 
@@ -603,7 +605,10 @@ static float qgemm_estimate(int qt, int TM, int M, int N, int K) {
     if (qt == QT_Q4_K) return TM == 64 ? 1.0f * most + 9.f : 1.6f * most + 20.f;
     return TM == 64 ? 1.57f * most + 16.f : 2.18f * most + 32.f;
 }
-static int qgemm_rows(int qt, int M, int N, int K) {
+// CRANE_B200_QGEMM_ROWS=16|32|64|128 pins it (tests, sweeps; 128: K-quants only)
+int qgemm_rows(int qt, int M, int N, int K) {
+    static const int pin = [] { const char* e = getenv("CRANE_B200_QGEMM_ROWS"); return e ? atoi(e) : 0; }();
+    if (pin) return pin;
     if (M <= 64) return M <= 16 ? 16 : M <= 32 ? 32 : 64;
     return qt != QT_Q8_0 && qgemm_estimate(qt, 128, M, N, K) < qgemm_estimate(qt, 64, M, N, K) ? 128 : 64;
 }

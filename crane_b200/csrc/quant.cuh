@@ -63,6 +63,8 @@ QRows qrows_at(unsigned char* buf, int rows, int K);
 int xquant_rows_launch(cudaStream_t st, int M, const float* x, int ldx, int K, const float* norm_w, float eps, int mode, const QRows& out, bool pdl);
 // y[m, n] = epi(sum_k W[n, k] x[m, k]); epi: GEMV_STORE, GEMV_RESID or GEMV_SILU_MUL (rows of W interleaved); x quantised for W's type
 int qgemm_launch(cudaStream_t st, int qt, const unsigned char* w, const QRows& x, int M, int N, int K, int epi, float* y, int ldy, bool pdl);
+// activation rows of a tile for such a linear (16, 32, 64 or 128)
+int qgemm_rows(int qt, int M, int N, int K);
 // several matrices of the same codes (GEMV_STORE): those whose CTAs fit the chip together share a launch.  *launches = how many there were
 struct QMany { int qt; const unsigned char* w; int N; float* y; int ldy; };
 int qgemm_many_launch(cudaStream_t st, const QMany* m, int n, const QRows& x, int M, int K, bool pdl, int* launches);

@@ -1,11 +1,16 @@
 """Quantised linears on the tensor cores (csrc/qgemm.cu) against the oracle's integer dots, at the edges of the kernel's tiles: 16 / 32 / 64 /
-128 activation columns, 128 weight rows, one and more super-blocks, work shared by several blocks and not."""
+128 activation rows, 128 weight rows, one and more super-blocks, work shared by several blocks and not."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
 from oracle import ggml_quant as gq
 
 pytestmark = pytest.mark.gpu
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 # The integer dots are exact on both sides; what differs is the order of the f32 additions over K / 256 (K-quants) or K / 32 (Q8_0) block terms
 # of either sign: under sqrt(blocks) * 2^-24 of the row's largest term, 2e-6 of the largest output at K = 4096.  Bound: five times that.
@@ -99,8 +104,53 @@ def test_prompts_at_the_line(recipe):
 @pytest.mark.parametrize("qt", ["Q4_K", "Q6_K"])
 @pytest.mark.parametrize("m,n,k", [(200, 12288, 512), (257, 12160, 512)])
 def test_wide_row_tiles(qt, m, n, k):
-    """Enough work for every block that tiles of 128 rows are taken."""
+    """Several tiles of 64 rows for every block (the plan's at 148 SMs)."""
+    assert rows_of(qt, m, n, k) == 64
     test_rows_against_integer_dots(qt, m, n, k)
+
+
+def rows_of(qt, m, n, k):
+    """Activation rows of the tiles that the plan takes."""
+    import crane_b200
+    return crane_b200.load_library().crane_b200_debug_qgemm_rows(gq.GGML_TYPE_ID[qt], m, n, k)
+
+
+# one row of a second half, a half less one, whole halves and tiles, one row of a third half and tile; weight rows that 128 does not divide; one super-block and many, a block's
+# own and shared
+EDGES = [(5, 128, 256), (65, 130, 512), (64, 384, 768), (127, 700, 1024), (128, 256, 4096), (129, 130, 2560), (191, 640, 512), (193, 2080, 1024), (256, 128, 2048), (257, 1000, 256)]
+
+
+def edges(qt, height):
+    """At tiles of `height` rows, pinned: every edge against the integer dots, the residual and the gated epilogue beside the plain one."""
+    import ctypes
+    import crane_b200
+    fn = crane_b200.load_library().crane_b200_debug_qlinear
+    ptr = lambda a: a.ctypes.data_as(ctypes.c_void_p)  # noqa: E731
+    for m, n, k in EDGES:
+        m = max(m, 7)                                       # (fewer rows are GEMVs)
+        assert rows_of(qt, m, n, k) == height
+        test_rows_against_integer_dots(qt, m, n, k)
+        rng = np.random.default_rng(m + n + k)
+        raw, x = blocks(rng, n, k, qt), rng.standard_normal((m, k)).astype(np.float32)
+        want = gq.qmatmul(x, raw, qt)
+        for epi, y in ((1, rng.standard_normal((m, n)).astype(np.float32)), (2, np.full((m, n // 2), 9.0, np.float32))):
+            if epi == 1:
+                ref = y + want.astype(np.float64)
+            else:
+                g, u = want[:, 0::2].astype(np.float64), want[:, 1::2].astype(np.float64)
+                ref = g / (1.0 + np.exp(-g)) * u
+            # (the gated unit: 1.1 |u| of a gate's error and |g| of an up's, both below 4 deviations here; expf and the division add a few units of 2^-24)
+            bar = BAR * (np.abs(ref).max() if epi == 1 else 2.1 * np.abs(want).max() ** 2)
+            rc = fn(0, ptr(x), ctypes.c_size_t(m), ctypes.c_size_t(k), ptr(raw), ctypes.c_size_t(raw.nbytes), gq.GGML_TYPE_ID[qt], ctypes.c_size_t(n), epi, ptr(y))
+            assert rc == 0 and np.abs(y - ref).max() <= bar, (m, n, k, epi)
+
+
+@pytest.mark.parametrize("qt,height", [(q, h) for q in ("Q4_K", "Q6_K", "Q8_0") for h in (16, 32, 64, 128) if q != "Q8_0" or h < 128])
+def test_edges_of_every_tile(qt, height):
+    """In a process of its own: the pin is read once."""
+    code = "import sys; sys.path[:0] = [%r, %r]; import test_qgemm as t; t.edges(%r, %d)" % (ROOT, os.path.join(ROOT, "tests"), qt, height)
+    r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, CRANE_B200_QGEMM_ROWS=str(height)), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
 
 
 @pytest.mark.parametrize("qt", ["Q4_K", "Q6_K", "Q8_0"])
@@ -123,19 +173,24 @@ def test_codes_of_a_row_are_its_own(qt, k):
         assert (np.abs(got - prompt).max(1) <= BAR * np.abs(prompt).max(1)).all(), n
 
 
-@pytest.mark.parametrize("qt,m", [("Q4_K", 1100), ("Q6_K", 700), ("Q6_K", 641)])
-def test_tiles_of_128_rows(qt, m):
-    """Enough work for tiles of 128 activation rows (a ragged last one among them): the same rows in calls of 64, whose tiles are held to the oracle above.  Only the
-    division along K, the order of the f32 additions, differs."""
+@pytest.mark.parametrize("qt,m,n", [("Q4_K", 1100, 8192), ("Q6_K", 700, 8192), ("Q6_K", 641, 8192)])
+def test_tiles_of_128_rows(qt, m, n):
+    """Enough work that the plan takes tiles of 128 activation rows (a ragged last one among them): the same rows in calls of 64, which do not.  Only the division along K, the
+    order of the f32 additions, differs; the first rows and the last against the oracle."""
     import crane_b200
+    assert rows_of(qt, m, n, 4096) == 128 and rows_of(qt, 64, n, 4096) == 64
     rng = np.random.default_rng(m)
-    raw = np.tile(blocks(rng, 512, 4096, qt), (8, 1))
+    few = blocks(rng, 512, 4096, qt)
+    raw = np.tile(few, (n // 512, 1))
     x = rng.standard_normal((m, 4096)).astype(np.float32)
-    got = crane_b200.op_qlinear(x, raw, gq.GGML_TYPE_ID[qt], 4096)
-    for r in range(0, m, 64):
-        part = crane_b200.op_qlinear(x[r: r + 64], raw, gq.GGML_TYPE_ID[qt], 4096) if m - r >= 5 else None
-        assert part is None or np.abs(got[r: r + 64] - part).max() <= BAR * np.abs(part).max()
-    assert np.array_equal(got, crane_b200.op_qlinear(x, raw, gq.GGML_TYPE_ID[qt], 4096))
+    got = crane_b200.op_qlinear(x, raw, gq.GGML_TYPE_ID[qt], n)
+    for r in [*range(0, m - 64, 64), m - 64]:
+        part = crane_b200.op_qlinear(x[r: r + 64], raw, gq.GGML_TYPE_ID[qt], n)
+        assert np.abs(got[r: r + 64] - part).max() <= BAR * np.abs(part).max()
+    some = [0, 1, 63, 64, 127, 128, m - 2, m - 1]
+    want = np.tile(gq.qmatmul(x[some], few, qt), (1, n // 512))
+    assert np.abs(got[some] - want).max() <= BAR * np.abs(want).max()
+    assert np.array_equal(got, crane_b200.op_qlinear(x, raw, gq.GGML_TYPE_ID[qt], n))
 
 
 @pytest.mark.parametrize("types", [("Q4_K", "Q4_K", "Q6_K"), ("Q6_K", "Q4_K", "Q4_K"), ("Q8_0", "Q8_0", "Q8_0"), ("Q4_K", "Q8_0", "Q6_K")])
