@@ -2839,6 +2839,12 @@ extern "C" CRANE_B200_API int crane_b200_debug_qlinear(int device, const float* 
 }
 /* ... the activation rows of its tiles (16, 32, 64 or 128) */
 extern "C" CRANE_B200_API int crane_b200_debug_qgemm_rows(int ggml_type, int m, int n, int k) { return qgemm_rows(ggml_type, m, n, k); }
+/* ... columns of the tiles of a bf16 GEMM (0: gemm_rows.cu), 1000 more where they are shared along K */
+extern "C" CRANE_B200_API int crane_b200_debug_gemm_tiles(int mode, int m, int n, int k, int split) {
+    bool stream_k = false;
+    const int bn = gemm_tiles(mode, m, n, k, split != 0, &stream_k);
+    return bn ? bn + (stream_k ? 1000 : 0) : 0;
+}
 
 /* debugging aid (not in the public header): copy a prefill workspace to the host -- 0: residual stream x [S, H], 1: qkv [S, qkv_dim],
  * 2: the f32 rows in front of / behind a quantised linear [S, max(I, q_dim)] */

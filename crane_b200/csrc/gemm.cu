@@ -826,6 +826,14 @@ static int launch_mode(cudaStream_t stream, const bf16* A, const bf16* A_lo, int
     }
 }
 
+int gemm_tiles(int mode, int M, int N, int K, bool split, bool* stream_k) {
+    *stream_k = true;
+    if (gemm_rows_pays(mode, split ? 2 : 1, M, N, K)) return 0;
+    const GemmPlan p = gemm_plan(mode, M, N, K, split, std::min(tc_device_sms(), GEMM_MAX_CTAS));
+    *stream_k = p.stream_k;
+    return p.bn;
+}
+
 int gemm_bf16_launch(cudaStream_t stream, const bf16* A, const bf16* A_lo, int lda, const bf16* W, int M, int N, int K,
                      const GemmEpi& epi, bool use_simt) {
     if (M <= 0 || N <= 0 || K <= 0 || (K % GEMM_BK) != 0 || (N % 32) != 0 || (lda % 8) != 0) return -1000;

@@ -49,6 +49,8 @@ struct TmaEncoder;  // host: resolves cuTensorMapEncodeTiled once
 // `A_lo` (nullable): low-order plane of a split-precision activation operand, same shape/stride as A (see gemm.cu).
 int gemm_bf16_launch(cudaStream_t stream, const bf16* A, const bf16* A_lo, int lda, const bf16* W, int M, int N, int K,
                      const GemmEpi& epi, bool use_simt);
+// columns of the tiles that such a GEMM takes: 64, 128, 256, 512 for 256 x 256 over a pair of CTAs, 0 for gemm_rows.cu; and whether they are shared along K
+int gemm_tiles(int mode, int M, int N, int K, bool split, bool* stream_k);
 // Few activation rows, 1 .. 3 bf16 planes (gemm_rows.cu); planes share lda.  gemm_bf16_launch comes here by itself where gemm_rows_pays.
 bool gemm_rows_pays(int mode, int planes, int M, int N, int K);
 int gemm_rows_launch(cudaStream_t stream, const bf16* const* planes, int n_planes, int lda, const bf16* W, int M, int N, int K, const GemmEpi& epi, bool pdl);

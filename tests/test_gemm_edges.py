@@ -48,9 +48,12 @@ def test_epilogues_at_tile_edges(shape, split):
 @pytest.mark.parametrize("split", [False, True], ids=["plain", "split"])
 @pytest.mark.parametrize("shape", [(160, 288, 1024), (161, 544, 1024), (255, 1024, 64), (300, 160, 4096), (129, 6176, 512), (129, 4128, 4096), (257, 8224, 1024), (600, 4128, 4096)],
                          ids=["64", "64a", "64b", "64 shared", "128", "128 shared", "256", "256 shared"])
-def test_every_part_of_the_epilogue(shape, split):
+def test_every_part_of_the_epilogue(shape, split, request):
     """Bias, column scale, gate and both planes of every mode, in tiles of the width and schedule that the plan takes at 148 SMs."""
     M, N, K = shape
+    name = request.node.callspec.id.replace("split", "").replace("plain", "").strip("-")
+    plan = crane_b200.load_library().crane_b200_debug_gemm_tiles
+    assert {plan(mode, M, N, K, int(split)) for mode in range(7)} == {int(name.split()[0].rstrip("ab")) + (1000 if "shared" in name else 0)}
     rng = np.random.default_rng(M + N * 3 + K)
     a = rng.standard_normal((M, K), dtype=np.float32)
     hi = synth.bf16_round(a)

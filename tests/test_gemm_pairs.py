@@ -1,7 +1,8 @@
 """GPU (-m gpu): GEMM tiles of CTA pairs (256 x 256, gemm_tc2_kernel) at their edges: one row more than a CTA's 128, one more than a pair's 256, rows that leave the odd CTA
 without any, column tiles of 32, 160 and 288 columns, one k-step, whole tiles and tiles shared along K.  The width is pinned in a process of its own (the plan takes pairs
-for large shapes only); two shapes that the plan gives to pairs by itself beside it.  Against float64: f32 results to 1e-5 (test_gemm_edges.py derives the bounds), bf16 results
-with their low-order plane to 2^-14 (its 2^-15, and up to 4096 products added in one accumulator instead of several)."""
+for large shapes only); three shapes that the plan gives to pairs by itself beside it; every check asks the plan for the tiles that it means.  Against float64: f32 results to
+1e-5, bf16 results with their low-order plane to 2^-15 (test_gemm_edges.py derives the bounds).  One accumulator that takes all of K is off by an amount that grows with K: at
+4096 products of two planes f32 results by up to 1.0e-5, both planes by 0.9 of 2^-15, the same in tiles of 64, 256 and 512 columns."""
 import os
 import re
 import subprocess
@@ -17,7 +18,14 @@ pytestmark = pytest.mark.gpu
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
-def check(M, N, K, split):
+def tiles(M, N, K, split, modes=(crane_b200.EPI_STORE_F32, crane_b200.EPI_RESID_F32, crane_b200.EPI_SILU_MUL_BF16, crane_b200.EPI_STORE_BF16)):
+    """Columns of the tiles that the plan takes, 1000 more where they are shared along K: one answer for all modes."""
+    got = {crane_b200.load_library().crane_b200_debug_gemm_tiles(m, M, N, K, int(split)) for m in modes}
+    return got.pop() if len(got) == 1 else got
+
+
+def check(M, N, K, split, want):
+    assert tiles(M, N, K, split) == want
     rng = np.random.default_rng(M * 3 + N + K)
     a = rng.standard_normal((M, K), dtype=np.float32)
     bits = synth.f32_to_bf16_bits(a)
@@ -35,19 +43,24 @@ def check(M, N, K, split):
     assert err(crane_b200.op_gemm(bits, w, crane_b200.EPI_RESID_F32, a_lo_bits=lo, out_init=init), init + ref) < 1e-5
     g, u = ref[:, 0::2], ref[:, 1::2]
     hi, low = crane_b200.op_gemm_epi(bits, w, crane_b200.EPI_SILU_MUL_BF16, a_lo_bits=lo, lo=True)
-    assert err(synth.bf16_bits_to_f32(hi).astype(np.float64) + synth.bf16_bits_to_f32(low), g / (1 + np.exp(-g)) * u) < 2.0 ** -14
+    assert err(synth.bf16_bits_to_f32(hi).astype(np.float64) + synth.bf16_bits_to_f32(low), g / (1 + np.exp(-g)) * u) < 2.0 ** -15
     hi, low = crane_b200.op_gemm_epi(bits, w, crane_b200.EPI_STORE_BF16, a_lo_bits=lo, lo=True)
-    assert err(synth.bf16_bits_to_f32(hi).astype(np.float64) + synth.bf16_bits_to_f32(low), ref) < 2.0 ** -14
+    assert err(synth.bf16_bits_to_f32(hi).astype(np.float64) + synth.bf16_bits_to_f32(low), ref) < 2.0 ** -15
 
 
-EDGES = [(129, 256, 64), (256, 288, 192), (257, 416, 512), (300, 544, 1024), (385, 1056, 128), (640, 256, 4096)]
+EDGES = {"1": [(129, 256, 64), (256, 288, 192), (257, 416, 512), (300, 544, 1024), (385, 1056, 128), (640, 256, 4096)],
+         "2": [(129, 288, 4864), (256, 288, 4864), (257, 416, 2432), (300, 544, 2048), (385, 1056, 1024), (640, 256, 4096)]}      # (148 k-steps and more: two for each of 74 pairs)
+
+
+def run(code, **env):
+    r = subprocess.run([sys.executable, "-c", "import sys; sys.path[:0] = [%r, %r]; import test_gemm_pairs as t\n%s" % (ROOT, os.path.join(ROOT, "tests"), code)], env=dict(os.environ, **env),
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
 
 
 @pytest.mark.parametrize("schedule", ["1", "2"], ids=["whole", "shared"])
 def test_edges(schedule):
-    code = "import sys; sys.path[:0] = [%r, %r]; import test_gemm_pairs as t\nfor e in t.EDGES:\n    for s in (False, True): t.check(*e, s)" % (ROOT, os.path.join(ROOT, "tests"))
-    r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, CRANE_B200_GEMM_BN="512", CRANE_B200_GEMM_SCHED=schedule), capture_output=True, text=True, timeout=300)
-    assert r.returncode == 0, r.stderr[-2000:]
+    run("for e in t.EDGES[%r]:\n    for s in (False, True): t.check(*e, s, %d)" % (schedule, 512 if schedule == "1" else 1512), CRANE_B200_GEMM_BN="512", CRANE_B200_GEMM_SCHED=schedule)
 
 
 TURNS = [(2400, 2336, 128), (2050, 4640, 64), (1100, 9472, 192)]        # several tiles a CTA; rows of tiles that 8 does not divide
@@ -55,14 +68,12 @@ TURNS = [(2400, 2336, 128), (2050, 4640, 64), (1100, 9472, 192)]        # severa
 
 @pytest.mark.parametrize("width", ["64", "256", "512"])
 def test_whole_tiles_in_turns(width):
-    code = "import sys; sys.path[:0] = [%r, %r]; import test_gemm_pairs as t\nfor e in t.TURNS: t.check(*e, e[0] == 2050)" % (ROOT, os.path.join(ROOT, "tests"))
-    r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, CRANE_B200_GEMM_BN=width, CRANE_B200_GEMM_SCHED="1"), capture_output=True, text=True, timeout=300)
-    assert r.returncode == 0, r.stderr[-2000:]
+    run("for e in t.TURNS: t.check(*e, e[0] == 2050, %s)" % width, CRANE_B200_GEMM_BN=width, CRANE_B200_GEMM_SCHED="1")
 
 
-@pytest.mark.parametrize("shape,split", [((2000, 6176, 2048), False), ((770, 6176, 4096), False), ((2200, 4128, 2048), True)], ids=["whole", "shared", "split"])
-def test_shapes_of_the_plan(shape, split):
-    check(*shape, split)
+@pytest.mark.parametrize("shape,split,want", [((2000, 6176, 2048), False, 512), ((770, 6176, 4096), False, 1512), ((2200, 4128, 2048), True, 1512)], ids=["whole", "shared", "split"])
+def test_shapes_of_the_plan(shape, split, want):
+    check(*shape, split, want)
 
 
 def test_timeline():
