@@ -495,8 +495,7 @@ int vit_pos_embed_add_launch(cudaStream_t st, float* x, int N, int Hv, const flo
 
 // qkv f32 [N, 3, nh, hd] -> bf16 same layout; q and k rotated in f32 with the 2-D (row, col) table
 // cos/sin [N, hd/2] (full-width cat(emb, emb) of the reference collapses to a half-split rotation).
-// VEC: four pairs a thread, read and written as vectors (head widths and planes that are multiples of 8); else pair by pair
-template <bool VEC>
+// Four pairs a thread, read and written as vectors: head widths are multiples of 8 (784 rows of 16 heads of 64, split: 8.8 us a launch pair by pair, 3.9 so).
 __global__ void __launch_bounds__(256)
 vit_rope_kernel(const float* __restrict__ qkv, int nh, int hd, const float* __restrict__ cs, const float* __restrict__ sn,
                 bf16* __restrict__ out, long long lo_off) {
@@ -507,46 +506,25 @@ vit_rope_kernel(const float* __restrict__ qkv, int nh, int hd, const float* __re
     const int Hv = nh * hd;
     const float* row = qkv + (size_t)p * 3 * Hv;
     bf16* orow = out + (size_t)p * 3 * Hv;
-    if constexpr (VEC) {
-        auto put = [&](bf16* o, float4 v) {
-            uint32_t h0, h1, l0, l1;
-            split_bf16x2(v.x, v.y, h0, l0); split_bf16x2(v.z, v.w, h1, l1);
-            *reinterpret_cast<uint2*>(o) = make_uint2(h0, h1);
-            if (lo_off) *reinterpret_cast<uint2*>(o + lo_off) = make_uint2(l0, l1);
-        };
-        const int per = half / 4;
-        for (int i = threadIdx.x; i < 2 * nh * per; i += blockDim.x) {    // q and k: heads follow one another
-            const int h = i / per, j = (i - h * per) * 4;
-            const float4 c = *reinterpret_cast<const float4*>(cs + (size_t)p * half + j), s = *reinterpret_cast<const float4*>(sn + (size_t)p * half + j);
-            const float4 x1 = *reinterpret_cast<const float4*>(row + h * hd + j), x2 = *reinterpret_cast<const float4*>(row + h * hd + j + half);
-            put(orow + h * hd + j, make_float4(x1.x * c.x - x2.x * s.x, x1.y * c.y - x2.y * s.y, x1.z * c.z - x2.z * s.z, x1.w * c.w - x2.w * s.w));
-            put(orow + h * hd + j + half, make_float4(x2.x * c.x + x1.x * s.x, x2.y * c.y + x1.y * s.y, x2.z * c.z + x1.z * s.z, x2.w * c.w + x1.w * s.w));
-        }
-        for (int i = threadIdx.x; i < Hv / 4; i += blockDim.x) put(orow + 2 * Hv + 4 * i, *reinterpret_cast<const float4*>(row + 2 * Hv + 4 * i));
-        return;
-    }
-    auto put = [&](bf16* p, float v) {
-        const bf16 h = __float2bfloat16_rn(v);
-        *p = h;
-        if (lo_off) p[lo_off] = __float2bfloat16_rn(v - __bfloat162float(h));
+    auto put = [&](bf16* o, float4 v) {
+        uint32_t h0, h1, l0, l1;
+        split_bf16x2(v.x, v.y, h0, l0); split_bf16x2(v.z, v.w, h1, l1);
+        *reinterpret_cast<uint2*>(o) = make_uint2(h0, h1);
+        if (lo_off) *reinterpret_cast<uint2*>(o + lo_off) = make_uint2(l0, l1);
     };
-    for (int i = threadIdx.x; i < 2 * nh * half; i += blockDim.x) {   // q and k pairs
-        const int which = i / (nh * half), rem = i % (nh * half);
-        const int h = rem / half, j = rem % half;
-        const float c = cs[(size_t)p * half + j], s = sn[(size_t)p * half + j];
-        const float* v = row + which * Hv + h * hd;
-        const float x1 = v[j], x2 = v[j + half];
-        bf16* o = orow + which * Hv + h * hd;
-        put(o + j, x1 * c - x2 * s);
-        put(o + j + half, x2 * c + x1 * s);
+    const int per = half / 4;
+    for (int i = threadIdx.x; i < 2 * nh * per; i += blockDim.x) {    // q and k: heads follow one another
+        const int h = i / per, j = (i - h * per) * 4;
+        const float4 c = *reinterpret_cast<const float4*>(cs + (size_t)p * half + j), s = *reinterpret_cast<const float4*>(sn + (size_t)p * half + j);
+        const float4 x1 = *reinterpret_cast<const float4*>(row + h * hd + j), x2 = *reinterpret_cast<const float4*>(row + h * hd + j + half);
+        put(orow + h * hd + j, make_float4(x1.x * c.x - x2.x * s.x, x1.y * c.y - x2.y * s.y, x1.z * c.z - x2.z * s.z, x1.w * c.w - x2.w * s.w));
+        put(orow + h * hd + j + half, make_float4(x2.x * c.x + x1.x * s.x, x2.y * c.y + x1.y * s.y, x2.z * c.z + x1.z * s.z, x2.w * c.w + x1.w * s.w));
     }
-    for (int i = threadIdx.x; i < Hv; i += blockDim.x) put(orow + 2 * Hv + i, row[2 * Hv + i]);
+    for (int i = threadIdx.x; i < Hv / 4; i += blockDim.x) put(orow + 2 * Hv + 4 * i, *reinterpret_cast<const float4*>(row + 2 * Hv + 4 * i));
 }
 int vit_rope_launch(cudaStream_t st, const float* qkv, int N, int nh, int hd, const float* cos, const float* sin, bf16* out, long long lo_off) {
-    const bool vec = hd % 8 == 0 && lo_off % 4 == 0 && (((uintptr_t)qkv | (uintptr_t)cos | (uintptr_t)sin) & 15) == 0 && ((uintptr_t)out & 7) == 0;
-    // 784 rows of 16 heads of 64, split: 8.8 us a launch pair by pair
-    return vec ? launch_k(vit_rope_kernel<true>, dim3(N), dim3(256), 0, st, prefill_pdl(), qkv, nh, hd, cos, sin, out, lo_off)
-               : launch_k(vit_rope_kernel<false>, dim3(N), dim3(256), 0, st, prefill_pdl(), qkv, nh, hd, cos, sin, out, lo_off);
+    if (hd % 8 != 0 || lo_off % 4 != 0 || (((uintptr_t)qkv | (uintptr_t)cos | (uintptr_t)sin) & 15) != 0 || ((uintptr_t)out & 7) != 0) return -1000;      // (64 and 128 are what towers have)
+    return launch_k(vit_rope_kernel, dim3(N), dim3(256), 0, st, prefill_pdl(), qkv, nh, hd, cos, sin, out, lo_off);
 }
 
 }  // namespace cb
