@@ -2839,6 +2839,26 @@ extern "C" CRANE_B200_API int crane_b200_debug_qlinear(int device, const float* 
 }
 /* ... the activation rows of its tiles (16, 32, 64 or 128) */
 extern "C" CRANE_B200_API int crane_b200_debug_qgemm_rows(int ggml_type, int m, int n, int k) { return qgemm_rows(ggml_type, m, n, k); }
+/* ... the row norms in front of linears (b: layer norm), out and out_lo [rows, W] as bf16 bits */
+extern "C" CRANE_B200_API int crane_b200_debug_row_norm(const float* x, int rows, int W, const float* w, const float* b, float eps, uint16_t* out, uint16_t* out_lo) {
+    if (!x || !w || !out || !out_lo || rows < 1 || W < 1) return CRANE_B200_INVALID_ARG;
+    const size_t n = (size_t)rows * W;
+    float* d = nullptr;
+    bf16* o = nullptr;
+    int rc = CRANE_B200_CUDA_ERROR;
+    if (cudaMalloc((void**)&d, (n + 2 * (size_t)W + 8) * 4) == cudaSuccess && cudaMalloc((void**)&o, (2 * n + 8) * 2) == cudaSuccess) {
+        const size_t at_w = (n + 3) / 4 * 4, at_b = at_w + (size_t)(W + 3) / 4 * 4, lo = (n + 3) / 4 * 4;
+        cudaMemcpy(d, x, n * 4, cudaMemcpyHostToDevice);
+        cudaMemcpy(d + at_w, w, (size_t)W * 4, cudaMemcpyHostToDevice);
+        if (b) cudaMemcpy(d + at_b, b, (size_t)W * 4, cudaMemcpyHostToDevice);
+        const int r = b ? layernorm_rows_launch(nullptr, d, rows, W, d + at_w, d + at_b, eps, o, (long long)lo) : rmsnorm_rows_launch(nullptr, d, rows, W, d + at_w, eps, o, (long long)lo);
+        if (r == -1000) rc = CRANE_B200_UNSUPPORTED;
+        else if (r == 0 && cudaDeviceSynchronize() == cudaSuccess && cudaMemcpy(out, o, n * 2, cudaMemcpyDeviceToHost) == cudaSuccess &&
+                 cudaMemcpy(out_lo, o + lo, n * 2, cudaMemcpyDeviceToHost) == cudaSuccess) rc = CRANE_B200_OK;
+    }
+    cudaFree(d); cudaFree(o);
+    return rc;
+}
 /* ... columns of the tiles of a bf16 GEMM (0: gemm_rows.cu), 1000 more where they are shared along K */
 extern "C" CRANE_B200_API int crane_b200_debug_gemm_tiles(int mode, int m, int n, int k, int split) {
     bool stream_k = false;

@@ -130,6 +130,20 @@ def test_each_mechanism_alone(name):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("precision,tol", [("f32", F32_TOL), ("split", SPLIT_TOL)])
+@pytest.mark.parametrize("width", [150, 77])
+def test_widths_that_four_does_not_divide(width, precision, tol):
+    """Embedding and norm kernels column by column, in a prompt and in a token's step."""
+    cfg = config([layer(ATT_PLAIN, DENSE), layer(SSM1)], width=width, vocab=120)
+    m, o = make(cfg, 17, precision=precision)
+    ids = tokens(41, 120, 18)
+    want = o.forward(ids, o.new_state()).numpy()
+    got = np.concatenate([m.step_batch([(0, ids[:40], all_rows(40))]), m.step_batch([(0, ids[40:], [0])])])
+    assert rel(got, want) < tol
+    m.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision,tol", [("f32", F32_TOL), ("split", SPLIT_TOL)])
 def test_whole_model_prefill_and_token_by_token_decoding(precision, tol):
     m, o = make(FULL, 5, precision=precision)
     ids = tokens(150, FULL["vocab"], 6)

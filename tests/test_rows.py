@@ -244,3 +244,27 @@ def test_quantised_decode_batch_against_the_oracle(recipe, n):
                                    (97, 2048, 1024), (128, 2048, 2048), (128, 1024, 1088), (5, 19008, 64)])
 def test_few_rows_at_the_lines(m, n, k, split):
     test_few_rows(m, n, k, split)
+
+
+# f32 sums over W terms in some order: sqrt(W) * 2^-24 of the sum, below 4e-6 at 8192, half of it in 1 / rms; the two planes leave out 2^-17 of a value; the rest a few units of 2^-24.
+@pytest.mark.parametrize("width", [4, 64, 1020, 1024, 1028, 1152, 2048, 2052, 2560, 4092, 4096, 4100, 5120, 8192])
+@pytest.mark.parametrize("kind", ["rms", "layer"])
+def test_row_norms(width, kind):
+    """Rows held in registers (up to 1024, 2048 and 4096 columns), full and not, and the longer ones read again for every pass."""
+    import ctypes as C
+    import crane_b200 as cb
+    rng = np.random.default_rng(width)
+    x = (rng.standard_normal((7, width)) * rng.uniform(0.01, 30.0, (7, 1)) + (0.7 if kind == "layer" else 0.0)).astype(np.float32)
+    x[3] = 0.0
+    w, b = rng.uniform(0.5, 1.5, width).astype(np.float32), rng.standard_normal(width).astype(np.float32)
+    hi, lo = np.empty((7, width), np.uint16), np.empty((7, width), np.uint16)
+    ptr = lambda a: a.ctypes.data_as(C.c_void_p)  # noqa: E731
+    assert cb.load_library().crane_b200_debug_row_norm(ptr(x), 7, width, ptr(w), ptr(b) if kind == "layer" else None, C.c_float(1e-6), ptr(hi), ptr(lo)) == 0
+    x64 = x.astype(np.float64)
+    if kind == "layer":
+        d = x64 - x64.mean(1, keepdims=True)
+        want = d / np.sqrt((d * d).mean(1, keepdims=True) + 1e-6) * w + b
+    else:
+        want = x64 / np.sqrt((x64 * x64).mean(1, keepdims=True) + 1e-6) * w
+    got = synth.bf16_bits_to_f32(hi).astype(np.float64) + synth.bf16_bits_to_f32(lo)
+    assert np.abs(got - want).max() <= 2.0 ** -16 * np.abs(want).max()
