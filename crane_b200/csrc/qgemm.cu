@@ -48,7 +48,7 @@ struct QCfg {
     static constexpr int D_COLS = (MINS ? 2 : DG) * NT;         // TMEM: two such sets,
     static constexpr int UPS = QT == QT_Q6_K ? 2 : 1;           // then units of unpacked weights, this many to a super-block
     static constexpr int U_COLS = 128 * PLANES / UPS, NU = (512 - 2 * D_COLS) / U_COLS > 3 ? 3 : (512 - 2 * D_COLS) / U_COLS;
-    static constexpr int DEQ_WARPS = 8, PARTS = DEQ_WARPS / 4, RR = 4 / PARTS;      // warps that unpack; a warp's share of a super-block: RR x 64 elements
+    static constexpr int DEQ_WARPS = 8, RR = 2;                 // warps that unpack, two to 32 rows; a warp's share of a super-block: RR x 64 elements
     static constexpr int RAW_BYTES = 128 * SB, RAW_REGS = QT == QT_Q4_K ? 1 + 2 * RR : QT == QT_Q6_K ? 2 + 2 * RR : 4 * RR;      // (16-byte pieces a thread reads per unit)
     static constexpr int NR = QT == QT_Q4_K ? (TM > 64 ? 3 : TM > 32 ? 5 : TM > 16 ? 6 : 8) : QT == QT_Q6_K ? (TM > 32 ? 5 : 6) : (TM > 32 ? 3 : 4);
     static constexpr int NB = QT == QT_Q6_K || TM != 64 ? 4 : 3;  // ring of codes: one unit of NT rows each
@@ -104,26 +104,6 @@ __host__ __device__ constexpr uint32_t h2_const(uint32_t bits) { return bits | (
 __device__ __forceinline__ uint32_t h2_int(uint32_t v) { return h2_add(v * 0x00010001u + 0x64006400u, h2_const(0xE400)); }
 // ... a signed byte (v + 128 is unsigned)
 __device__ __forceinline__ uint32_t h2_byte(uint32_t v) { return h2_add(((v ^ 0x80u) & 0xffu) * 0x00010001u + 0x64006400u, h2_const(0xE480)); }
-
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* v) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31};"
-        ::"r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
-          "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]),
-          "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]),
-          "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31]), "r"(taddr) : "memory");
-}
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* v) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
-        ::"r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
-          "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(taddr) : "memory");
-}
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {     // A from TMEM
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-                 ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
 
 // One CTA's share (`cta` of a.sc.G) of one linear
 template <int QT, int TM>
@@ -269,10 +249,9 @@ __device__ __forceinline__ void qgemm_body(const CUtensorMap& tmW, const CUtenso
         }
     // ------------------------------------------------------------------------------------------------ weights: blocks -> f16 integers
     } else if (warp >= W_DEQ) {
-        // A lane has a row, the PARTS warps of its 32 rows a part of every super-block each (Q6_K: of every unit).  The raw bytes of the next unit are read into
+        // A lane has a row, the two warps of its 32 rows a half of every super-block each (Q6_K: the low or the high nibbles of every unit).  The raw bytes of the next unit are read into
         // registers before this one's stores are waited for, so that only the instructions stand between two units.
         const int dw = warp - W_DEQ, part = dw >> 2, row = (dw & 3) * 32 + lane;
-        const int half = part & 1, q_first = C::PARTS == 4 ? part >> 1 : 0;      // Q6_K: nibbles, and the first of a unit's two quarters
         constexpr int RR = C::RR;
         const uint32_t lanes = (uint32_t)((dw & 3) * 32) << 16;
         const int units = (it_end - it_begin) * C::UPS;
@@ -291,8 +270,8 @@ __device__ __forceinline__ void qgemm_body(const CUtensorMap& tmW, const CUtenso
 #pragma unroll
                 for (int e = 0; e < 2; ++e) raw[e] = *reinterpret_cast<const uint4*>(sb + 128 + 32 * n + 16 * e);
 #pragma unroll
-                for (int j = 0; j < 2 * RR; ++j) raw[2 + j] = *reinterpret_cast<const uint4*>(sb + 64 * n + 32 * q_first + 16 * j);
-                raw1 = *reinterpret_cast<const uint32_t*>(sb + 192 + 8 * n + 4 * half) >> (16 * q_first);       // scales: byte 2 * quarter + (element / 16)
+                for (int j = 0; j < 2 * RR; ++j) raw[2 + j] = *reinterpret_cast<const uint4*>(sb + 64 * n + 16 * j);
+                raw1 = *reinterpret_cast<const uint32_t*>(sb + 192 + 8 * n + 4 * part);       // scales: byte 2 * quarter + (element / 16)
                 if (n == 0 && part == 0)
                     reinterpret_cast<float*>(sm + C::OFF_SCW + ((it_begin + u / C::UPS) & (C::NS - 1)) * C::SCW_BYTES)[row] =
                         4.f * __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short*>(sb + 208)));
@@ -338,7 +317,7 @@ __device__ __forceinline__ void qgemm_body(const CUtensorMap& tmW, const CUtenso
                     }
                     tmem_st32(ta + (uint32_t)g * 32, o);
                 }
-                if (part == C::PARTS - 1) {                // offsets m_0 .. m_7, 64 times them; d and dmin for the accumulators' readers
+                if (part == 1) {                           // offsets m_0 .. m_7, 64 times them; d and dmin for the accumulators' readers
                     uint32_t m[4], m64[4];
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
@@ -360,18 +339,17 @@ __device__ __forceinline__ void qgemm_body(const CUtensorMap& tmW, const CUtenso
                     fence_proxy_async();                   // (the offsets' tile is in shared memory)
                 }
             } else if constexpr (QT == QT_Q6_K) {
-                // half = 0: low nibbles, quarters q1 | q2 of the block's half; 1: high nibbles, q3 | q4
-                const uint32_t lmul = half ? h2_const(0x2400) : h2_const(0x3400), lofs = half ? h2_const(0xCC00) : h2_const(0xDC00);    // 1/64, 1/4; -16, -256
-                const uint32_t lm = half ? 0x00F000F0u : 0x000F000Fu;
+                // part 0: low nibbles, quarters q1 | q2 of the block's half; 1: high nibbles, q3 | q4
+                const uint32_t lmul = part ? h2_const(0x2400) : h2_const(0x3400), lofs = part ? h2_const(0xCC00) : h2_const(0xDC00);    // 1/64, 1/4; -16, -256
+                const uint32_t lm = part ? 0x00F000F0u : 0x000F000Fu;
 #pragma unroll
-                for (int r = 0; r < RR; ++r) {             // elements [32 q, 32 q + 32) of the 64
-                    const int q = q_first + r;
+                for (int q = 0; q < RR; ++q) {             // elements [32 q, 32 q + 32) of the 64
                     uint32_t lo[16], hi[16];
 #pragma unroll
                     for (int e = 0; e < 2; ++e) {          // e: elements [16 e, 16 e + 16) of a quarter; high plane: (1024 + v - 1024 - 2) * 4 f
-                        const uint32_t f = h2_byte(raw1 >> (16 * r + 8 * e)), ls = h2_mul(f, lmul), lo_o = h2_mul(f, lofs), hs = h2_mul(f, h2_const(0x4400));
-                        const uint32_t wl[4] = {raw[2 + 2 * r + e].x, raw[2 + 2 * r + e].y, raw[2 + 2 * r + e].z, raw[2 + 2 * r + e].w};
-                        const int sh = 4 * half + 2 * q;
+                        const uint32_t f = h2_byte(raw1 >> (16 * q + 8 * e)), ls = h2_mul(f, lmul), lo_o = h2_mul(f, lofs), hs = h2_mul(f, h2_const(0x4400));
+                        const uint32_t wl[4] = {raw[2 + 2 * q + e].x, raw[2 + 2 * q + e].y, raw[2 + 2 * q + e].z, raw[2 + 2 * q + e].w};
+                        const int sh = 4 * part + 2 * q;
                         const uint32_t wh[4] = {raw[e].x >> sh, raw[e].y >> sh, raw[e].z >> sh, raw[e].w >> sh};
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
@@ -382,8 +360,8 @@ __device__ __forceinline__ void qgemm_body(const CUtensorMap& tmW, const CUtenso
                             hi[8 * e + 2 * i + 1] = h2_mul(h2_add((w8 & 0x00030003u) | 0x64006400u, h2_const(0xE402)), hs);
                         }
                     }
-                    tmem_st16(ta + (uint32_t)(32 * half + 16 * q), lo);
-                    tmem_st16(ta + (uint32_t)(C::U_COLS / 2 + 32 * half + 16 * q), hi);
+                    tmem_st16(ta + (uint32_t)(32 * part + 16 * q), lo);
+                    tmem_st16(ta + (uint32_t)(C::U_COLS / 2 + 32 * part + 16 * q), hi);
                 }
             } else {
 #pragma unroll
