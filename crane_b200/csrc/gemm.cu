@@ -759,10 +759,15 @@ static int launch_tc2(cudaStream_t stream, const bf16* A, const bf16* A_lo, int 
 //   stream-K:    tiles x k-steps dealt evenly to all SMs, and the last of a tile's c contributors adding the others' parts.
 // Tiles of pairs (256 x 256): a k-step 0.31 us plain and 0.62 split with few tiles, 0.36 and 0.63 with every SM busy on the scale that gives the single tiles 0.42 and 0.66, two or three
 // us more of setup and hand-over.  Worth it where the operands are what takes the time; not where a gated or GELU tile's epilogue does (9 us), nor with rows that fill 256 badly.  Their
-// stream-K pays above one wave too, while all operands stay in the L2 (CTAs at different k-steps share nothing of what they read): 4096 x 12288 at 2048 rows 187 us, whole tiles 141.
-//   us, single / pairs (with whole tiles in runs, before they were dealt in turn: sched_band), plain: 24576 x 4096 at 256 rows 78.8 / 55.3, 512 108 / 87, 2048 392 / 327, 4096 822 / 657    6144 x 4096 at 784 64.4 / 44.9, 4096 170 / 142
-//   12288 x 2048 at 784 59.7 / 44.4, 1111 48.4 / 55.3, 4096 152 / 136                                                4096 x 12288 at 512 69.6 / 52.6, 4096 318 / 284
-//   split: 24576 x 4096 at 512 153 / 144, 4096 1204 / 1100    6144 x 4096 at 4096 283 / 263    4096 x 4096 193 / 179    8256 x 1024 103 / 97    7168 x 1024 92 / 88
+// stream-K pays above one wave too, while all operands stay in the L2 (CTAs at different k-steps share nothing of what they read): 4096 x 12288 at 2048 rows 187 us, whole tiles 141; 6144 x 4096 at
+// 2500 rows, split, 161 and 178.
+//   The constants were fitted to whole tiles in runs; since they are dealt in turn (sched_band) both sides' whole tiles are faster.  us of launches by themselves, the best single tiles /
+//   the best pairs / as planned, plain: 24576 x 4096 at 200 rows 62 / 56 / 68, 300 64 / 76 / 64, 512 89 / 78 / 78, 1111 173 / 165 / 173, 1700 255 / 230 / 231, 4096 546 / 484 / 484
+//   6144 x 4096 at 784 44.4 / 45.7 / 45.7, 1111 53 / 52 / 52, 4096 159 / 142 / 143     4096 x 12288 at 512 65 / 54 / 70, 784 78 / 74 / 74, 1111 81 / 131 / 82, 4096 313 / 279 / 279
+//   12288 x 2048 at 784 46 / 44 / 44, 1111 48 / 55 / 48, 4096 149 / 135 / 135
+//   split: 24576 x 4096 at 512 148 / 142 / 142, 784 234 / 263 / 234, 4096 967 / 923 / 925     6144 x 4096 at 784 66 / 73 / 73, 1111 82 / 87 / 95, 4096 263 / 263 / 263
+//   4096 x 4096 at 4096 187 / 180 / 179     4096 x 12288 at 1700 239 / 260 / 260, 4096 538 / 528 / 528     8256 x 1024 at 4096 101 / 95 / 99     7168 x 1024 92 / 88 / 91
+//   13 shapes of these models at 8 row counts from 200 to 4096, either precision: within 4 % of the best of six pinned plans in 184 of 208, at most 1.30 of it.
 constexpr int GEMM_PAIR = 512;          // GemmPlan::bn: 256 x 256 tiles of two CTAs
 struct GemmPlan { int bn; bool stream_k; double cost; };
 static GemmPlan gemm_plan(int mode, int M, int N, int K, bool split, int sms) {
