@@ -14,6 +14,7 @@ from __future__ import annotations
 
 import ctypes as C
 import json
+import math
 import os
 
 import numpy as np
@@ -176,13 +177,14 @@ def _ptr(a: np.ndarray):
 
 class _Pinned:
     """Owner of one piece of the library's pinned range; the arrays over it keep it alive."""
+    __slots__ = ("__array_interface__", "_free")
 
-    def __init__(self, address: int, shape, dtype):
-        self.__array_interface__ = {"data": (address, False), "shape": tuple(shape), "typestr": dtype.str, "version": 3}
-        self._address, self._free = address, load_library().crane_b200_host_free
+    def __init__(self, address: int, shape, typestr: str, free):
+        self.__array_interface__ = {"data": (address, False), "shape": shape, "typestr": typestr, "version": 3}
+        self._free = free
 
     def __del__(self):
-        self._free(self._address)
+        self._free(self.__array_interface__["data"][0])
 
 
 def _result(shape, dtype=np.float32) -> np.ndarray:
@@ -192,12 +194,12 @@ def _result(shape, dtype=np.float32) -> np.ndarray:
     is refused (`copy()` gives an array that owns its data).  Programs that keep results keep their pieces of the pool; when it is used up, results come in
     ordinary memory.
     """
-    shape, dtype = tuple(int(n) for n in shape), np.dtype(dtype)
-    n = int(np.prod(shape, dtype=np.int64)) * dtype.itemsize
-    p = C.c_void_p()
-    if n < 4096 or load_library().crane_b200_host_alloc(n, C.byref(p)) != OK:
+    shape, dtype = tuple(map(int, shape)), np.dtype(dtype)
+    n = math.prod(shape) * dtype.itemsize
+    lib, p = load_library(), C.c_void_p()
+    if n < 4096 or lib.crane_b200_host_alloc(n, C.byref(p)) != OK:
         return np.empty(shape, dtype)
-    return np.asarray(_Pinned(p.value, shape, dtype))
+    return np.asarray(_Pinned(p.value, shape, dtype.str, lib.crane_b200_host_free))
 
 
 class Engine:
