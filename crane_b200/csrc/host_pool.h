@@ -1,5 +1,5 @@
 // Pinned host memory for results (crane_b200_host_alloc / _free): copies into it run at the link's rate and need no second copy by the host.  us of a copy into pinned /
-// pageable memory on the GPU box: 64 KB 11 / 18, 1 MB 29 / 83, 8 MB 157 / 472, 32 MB 601 / 1980 and more.
+// pageable memory: 64 KB 11 / 18, 1 MB 29 / 83, 8 MB 157 / 472, 32 MB 601 / 1980 and more (a Python call for a row of 8 KB 19 / 24, of 593 KB 30 / 66).
 // Pinning itself takes far longer than it saves one call (cudaHostAlloc of 1 MB 2.2 ms, of 16 MB 12 ms, freeing 0.4 to 1.8 ms), so no call pins.  ONE range of up to SIZE
 // bytes, in huge pages where the system has them, is registered by the first request while a handle is open -- the Python engine makes it as it opens -- as far as its
 // handles' results need (ms: 2 MB 0.8, 8 MB 1.7, 64 MB 9; to give them back 0.4 to 1.9), and further when a handle that needs more has opened.  Results are pieces of it, the
