@@ -4,7 +4,8 @@
 // bytes, in huge pages where the system has them, is registered by the first request while a handle is open -- the Python engine makes it as it opens -- as far as its
 // handles' results need (ms: 2 MB 0.8, 8 MB 1.7, 64 MB 9; to give them back 0.4 to 1.9), and further when a handle that needs more has opened.  Results are pieces of it, the
 // smallest free stretch that holds them.  What does not fit gets ordinary memory from the caller, as does what comes when programs have kept the whole range.  It goes back with
-// the last handle or, where pieces are still out, with the last of those.  us of a new handle's first pass / of later ones: 32 sequences' round over 8192 logits 940 / 862
+// the last handle or, where pieces are still out, with the last of those.  Its pages are private ones: a forked process has copies of its own, where pages of cudaHostAlloc are
+// shared and would show it what later calls of its parent write.  us of a new handle's first pass / of later ones: 32 sequences' round over 8192 logits 940 / 862
 // (ordinary memory 1030 / 965, buffers pinned one by one 3400 to 10 000 / 865), one token over 151 936 four times 3300 / 2595 (3540 / 2748, 5000 to 8000 / 2600), an image's
 // features 8300 / 3380 (9200 / 3880, 18 000 / 3350).
 #pragma once

@@ -167,3 +167,36 @@ def test_a_thread_keeps_its_context():
     t.start()
     t.join()
     assert seen == [None] * 5
+
+
+@pytest.mark.gpu
+def test_a_forked_process_keeps_what_it_had():
+    """A child's results are its own, as in ordinary memory, while its parent's later calls reuse their pieces, and the parent's later results are right although it has written
+    to pages that the child shares.  (The child calls nothing of CUDA's.)"""
+    r = subprocess.run([sys.executable, "-c", "import sys; sys.path[:0] = [%r, %r]; import test_host_pool as t; t.forked()" % (ROOT, os.path.join(ROOT, "tests"))],
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
+def forked():
+    cfg = dict(synth.TINY_QWEN3, vocab_size=40000)
+    m = crane_b200.Qwen3Model(cfg, max_seq_len=64)
+    m.load_checkpoint(synth.synth_checkpoint(cfg))
+    got = m.forward_step([1, 2, 3], 0)
+    was, at = got.copy(), got.ctypes.data
+    assert got.base is not None
+    to_child, go = os.pipe()
+    pid = os.fork()
+    if pid == 0:
+        os.read(to_child, 1)
+        os._exit(0 if np.array_equal(got, was) else 1)
+    got[:] = 0.0
+    del got
+    m.clear_kv_cache()
+    again = m.forward_step([1, 2, 3], 0)
+    assert again.ctypes.data == at and np.array_equal(again, was)
+    m.clear_kv_cache()
+    m.forward_step([4, 5], 0)
+    os.write(go, b"x")
+    assert os.waitstatus_to_exitcode(os.waitpid(pid, 0)[1]) == 0
+    m.close()
